@@ -178,6 +178,38 @@ cudaError_t launch_patchify(const ConvParams& p, const float* x, float* rows, cu
 cudaError_t launch_depthwise_conv(const ConvParams& p, const float* x, const float* w,
                                   const float* bias, float* out, cudaStream_t st);
 
+// Small convolutions (group 1) on the CUDA cores without a column buffer (conv_simt.cu). `wt` is the
+// filter matrix transposed by launch_pack_filter: [k][conv_simt_ldw(oc)]. `gate`: [n][c] factors of
+// the input channels (pointwise convolutions only), or null; `residual`: added last, or null.
+inline int64_t conv_simt_ldw(int64_t oc) { return (oc + 3) / 4 * 4; }
+bool conv_simt_supported(const ConvParams& p);
+cudaError_t launch_pack_filter(const float* w, float* wt, int64_t oc, int64_t k, cudaStream_t st);
+cudaError_t launch_conv_simt(const ConvParams& p, const float* x, const float* wt, const float* bias, const float* gate,
+                             const float* residual, float* out, cudaStream_t st);
+// Larger convolutions (group 1, no Gelu behind) on the tensor cores, 3xTF32, planes read in place
+// (conv_tc.cu). The filter is split and blocked once by launch_pack_filter_tc into
+// conv_tc_filter_elems floats; the other operands as above.
+bool conv_tc_supported(const ConvParams& p);
+int64_t conv_tc_filter_elems(const ConvParams& p);
+cudaError_t launch_pack_filter_tc(const ConvParams& p, const float* w, float* packed, cudaStream_t st);
+cudaError_t launch_conv_tc(const ConvParams& p, const float* x, const float* packed, const float* bias, const float* gate,
+                           const float* residual, float* out, int* err_word, cudaStream_t st);
+
+// Squeeze-and-excite gate in one kernel (squeeze_excite.cu):
+//   gate[n, :] = act2(W2 * act1(W1 * mean(x[n, :, plane]) + b1) + b2),  W1 [s, c], W2 [c, s].
+struct SqueezeExciteParams {
+  const float* x;
+  const float* w1; const float* b1;   // biases may be null
+  const float* w2; const float* b2;
+  float* gate;
+  int n, c, s;
+  int64_t hw;
+  int act1, act2;
+  float alpha1, beta1, alpha2, beta2;
+};
+bool squeeze_excite_supported(const SqueezeExciteParams& p);
+cudaError_t launch_squeeze_excite(const SqueezeExciteParams& p, cudaStream_t st);
+
 // ---- GEMM -------------------------------------------------------------------
 // C[b] = act(alpha * op(A[b]) * op(B[b]) + beta * Cin[b] + bias) (+ residual)
 // Row-major operands; trans_a: A stored [K, M]; trans_b: B stored [N, K].
@@ -220,6 +252,10 @@ struct GemmParams {
                             // through registers, 2 A taken pre-split from a16_hi / a16_lo by TMA
 };
 cudaError_t launch_gemm_simt(const GemmParams& p, cudaStream_t st);
+// Few rows (m <= kGemmRowsMax) against a [N, K] operand: one warp per output column (gemm_rows.cu).
+constexpr int64_t kGemmRowsMax = 32;
+bool gemm_rows_supported(const GemmParams& p);
+cudaError_t launch_gemm_rows(const GemmParams& p, cudaStream_t st);
 
 // tcgen05 / TMEM / TMA path. Needs A row-major with K contiguous (trans_a == 0)
 // and B stored [N, K] (trans_b == 1), 16-byte aligned bases and leading

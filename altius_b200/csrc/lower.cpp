@@ -113,7 +113,26 @@ struct Plan {
   std::map<int, int> reduce_sibling; // ReduceMean node -> ReduceMax node of the same rows computed with it
   struct SeGate { int x, gate; };
   std::map<int, SeGate> se_gate;    // pointwise Conv2d node -> squeeze-excite Mul folded into its input
+  struct Squeeze { int conv1, conv2, b1, b2, act1, act2, out; float alpha1, beta1, alpha2, beta2; };
+  std::map<int, Squeeze> squeeze;   // GlobalAveragePool node -> the two 1 x 1 convolutions behind it
 };
+
+// Sessions on a device refine the schedule with kernels that a plan_only session does not list: its
+// schedule, arena plan and launch count are those of the general kernels, whatever the device.
+bool on_device(const AcSession& s) { return !s.opt.plan_only; }
+// gemm_mode 1 promises exact ascending chains and 2 its own precision: both keep their kernels.
+bool fp32_level_mode(const AcSession& s) { return s.opt.gemm_mode == 0 || s.opt.gemm_mode == 3; }
+
+// Convolutions below the size from which the tensor cores take them (2^23 operations) run on the
+// small-convolution kernel: at 28 K products per SM or fewer they are bound by latency.
+constexpr double kTensorConvFloor = double(1 << 23);
+bool small_conv_applies(const AcSession& s, double flops) {
+  return on_device(s) && fp32_level_mode(s) && flops < kTensorConvFloor;
+}
+// The larger ones on the tensor-core kernel that reads the planes itself.
+bool tensor_conv_applies(const AcSession& s, double flops) {
+  return on_device(s) && fp32_level_mode(s) && flops >= kTensorConvFloor;
+}
 
 // Recognises `hs = HardSigmoid(t); m = Mul(t, hs)` hanging off value t whose only
 // uses are those two nodes. Returns the Mul node or -1.
@@ -513,11 +532,59 @@ void detect_se_gate(Ctx& c, Plan& plan) {
     for (int64_t k = 0; k < conv.ints[9]; ++k) nopad = nopad && conv.ints[10 + k] == 0;
     const double flops = 2.0 * xv.dims[0] * ov.dims[1] * hw * ch;
     // The conditions under which lower_conv / emit_gemm take the [K, N] tensor-core path.
-    if (!pointwise || !nopad || (hw % 4) != 0 || (ch % 4) != 0 || ch < 8 || flops < double(1 << 23) ||
+    // On a device the convolution kernels take a gate with any plane (lower_conv's conditions); the
+    // GEMM that reads the planes by TMA needs whole float4s and a size of its own.
+    const bool gelu = plan.epi.count(cn) && plan.epi[cn].act == ACT_GELU;
+    const bool direct = on_device(c.s) && fp32_level_mode(c.s) && ch <= 4096 && ov.dims[1] <= 16384 && !gelu &&
+                        xv.numel() < (1ll << 30);
+    const bool tensor = (hw % 4) == 0 && (ch % 4) == 0 && ch >= 8 && flops >= kTensorConvFloor;
+    if (!pointwise || !nopad || !(tensor || direct) ||
         xv.dims[0] > 65535 || !c.val(conv.inputs[1]).is_const)
       continue;
     plan.se_gate[cn] = Plan::SeGate{x, g};
     c.absorbed[nid] = 1;
+  }
+}
+
+// GlobalAveragePool -> pointwise Conv2d [+ act] -> pointwise Conv2d [+ act] on the 1 x 1 planes: the
+// squeeze-and-excite block up to its gate, one kernel.
+void detect_squeeze(Ctx& c, Plan& plan) {
+  if (!on_device(c.s) || !fp32_level_mode(c.s)) return;
+  auto plain_1x1 = [&](int nid) {
+    const Node& n = c.node(nid);
+    if (c.absorbed[nid] || n.op != AC_OP_CONV2D || n.ints[0] != 1 || n.ints[1] != 1 || n.ints[2] != 1 || n.ints[3] != 1 ||
+        n.ints[6] != 1 || n.ints[7] != 0 || n.ints[8] != 0 || !c.val(n.inputs[1]).is_const)
+      return false;
+    for (int64_t k = 0; k < n.ints[9]; ++k)
+      if (n.ints[10 + k] != 0) return false;
+    auto e = plan.epi.find(nid);
+    return e == plan.epi.end() || e->second.residual < 0;
+  };
+  for (int nid : c.s.order) {
+    const Node& n = c.node(nid);
+    if (c.absorbed[nid] || n.op != AC_OP_GLOBALAVERAGEPOOL || !c.single_use(n.outputs[0])) continue;
+    Plan::Squeeze q{};
+    int cur = n.outputs[0];
+    for (int k = 0; k < 2; ++k) {
+      const int cn = c.single_use(cur) ? c.only_consumer(cur) : -1;
+      if (cn < 0 || !plain_1x1(cn) || c.node(cn).inputs[0] != cur) { cur = -1; break; }
+      const Node& cv = c.node(cn);
+      auto e = plan.epi.find(cn);
+      const Epilogue ep = e == plan.epi.end() ? Epilogue{} : e->second;
+      const int bias = ep.bias >= 0 ? ep.bias : (cv.inputs.size() > 2 ? cv.inputs[2] : -1);
+      cur = ep.out >= 0 ? ep.out : cv.outputs[0];
+      if (k == 0) { q.conv1 = cn; q.b1 = bias; q.act1 = ep.act; q.alpha1 = ep.act_alpha; q.beta1 = ep.act_beta; }
+      else { q.conv2 = cn; q.b2 = bias; q.act2 = ep.act; q.alpha2 = ep.act_alpha; q.beta2 = ep.act_beta; }
+    }
+    if (cur < 0) continue;
+    q.out = cur;
+    const Value& xv = c.val(n.inputs[0]);
+    SqueezeExciteParams p{};
+    p.n = (int)xv.dims[0]; p.c = (int)xv.dims[1]; p.hw = xv.dims[2] * xv.dims[3];
+    p.s = (int)c.val(c.node(q.conv1).inputs[1]).dims[0];
+    if (c.val(c.node(q.conv2).inputs[1]).dims[0] != p.c || c.val(n.inputs[0]).is_const || !squeeze_excite_supported(p)) continue;
+    c.absorbed[q.conv1] = c.absorbed[q.conv2] = 1;
+    plan.squeeze[nid] = q;
   }
 }
 
@@ -683,11 +750,19 @@ int effective_pairs(const AcSession& s) {
   return s.opt.gemm_pairs == 0 ? 2 : (s.opt.gemm_pairs == 3 ? 0 : s.opt.gemm_pairs);
 }
 
+// Products of a few rows run in fp32 on the kernel that streams B (classifier heads at small batches).
+bool gemm_rows_applies(const AcSession& s, const GemmShape& g, bool b_const, int64_t a_off, int64_t b_off) {
+  return on_device(s) && fp32_level_mode(s) && g.batch == 1 && !g.ta && g.m <= kGemmRowsMax && g.k >= 4 && (g.k % 4) == 0 &&
+         (g.lda % 4) == 0 && (a_off % 4) == 0 &&
+         (g.tb ? (g.ldb % 4) == 0 && (b_off % 4) == 0 : b_const && b_off == 0);
+}
+
 // The static part of emit_gemm's decision to run a GEMM with a constant rhs on the CTA-pair
 // kernel that takes A pre-split (kept in one place: plan_presplit decides with it which
 // producers write split results before the GEMMs themselves are lowered).
 bool presplit_applies(const AcSession& s, const GemmShape& g, bool b_const, int64_t a_off, int64_t b_off) {
   const int mode = s.opt.gemm_mode;
+  if (gemm_rows_applies(s, g, b_const, a_off, b_off)) return false;
   if (mode != 0 || effective_pairs(s) != 2 || !b_const || g.batch != 1 || g.ta || b_off != 0) return false;
   const double flops = 2.0 * g.batch * g.m * g.n * g.k;
   const double tc_floor = (g.batch == 1 && g.m <= 128 && g.k >= 64) ? double(1 << 19) : double(1 << 23);
@@ -772,6 +847,34 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   double bytes = 4.0 * g.batch * (g.m * g.k + g.m * g.n) + 4.0 * (g.sb ? g.batch : 1) * g.k * g.n;
   if (res >= 0) bytes += 4.0 * g.batch * g.m * g.n;
   const double flops = 2.0 * g.batch * g.m * g.n * g.k;
+
+  if (bias_m < 0 && b_row_scale < 0 && gemm_rows_applies(*s, g, em.c.val(b).is_const, a_off, b_off)) {
+    int bt = b;
+    if (!g.tb) {
+      bt = new_value(em.c, g.k * g.n, true);
+      const int64_t kk = g.k, nn = g.n;
+      em.add("weight_transpose", op, {b}, {bt}, 8.0 * kk * nn, 0, [=](cudaStream_t st) {
+        return launch_transpose2d(s->fptr(b), s->fptr_mut(bt), 1, (int)kk, (int)nn, st);
+      });
+      g.tb = 1;
+      g.ldb = g.k;
+    }
+    const GemmShape q = g;
+    em.add("gemm_fp32_rows", op, {a, bt, c_in, bias_n, res}, {out}, bytes, flops, [=](cudaStream_t st) {
+      GemmParams p{};
+      p.m = q.m; p.n = q.n; p.k = q.k; p.batch = 1;
+      p.a = s->fptr(a) + a_off; p.lda = q.lda;
+      p.b = s->fptr(bt) + b_off; p.ldb = q.ldb; p.trans_b = 1;
+      p.c = s->fptr_mut(out) + c_off; p.ldc = q.ldc;
+      p.alpha = alpha; p.beta = c_in >= 0 ? beta : 0.f;
+      p.c_in = c_in >= 0 ? s->fptr(c_in) + c_off : nullptr; p.ldc_in = q.ldc;
+      p.bias_n = bias_n >= 0 ? s->fptr(bias_n) : nullptr; p.bias_scale = bias_scale;
+      p.act = act; p.act_alpha = aa; p.act_beta = ab;
+      p.residual = res >= 0 ? s->fptr(res) + c_off : nullptr; p.ld_res = q.ldc;
+      return gemm_rows_supported(p) ? launch_gemm_rows(p, st) : launch_gemm_simt(p, st);
+    });
+    return;
+  }
 
   // ---- tensor-core eligibility (static part; alignment is re-checked at launch) ----
   const int mode = s->opt.gemm_mode;
@@ -1069,6 +1172,31 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
   // GEMM form: out[n] (ocg x ohw) = W_g (ocg x k) * col[n, g] (k x ohw), bias per row.
   const bool pointwise = p.kh == 1 && p.kw == 1 && p.sh == 1 && p.sw == 1 && p.pad_t == 0 &&
                          p.pad_l == 0 && pads[2] == 0 && pads[3] == 0;
+  if (tensor_conv_applies(*s, flops) && !(pointwise && ohw == 1) && conv_tc_supported(p)) {
+    const int wt = new_value(em.c, conv_tc_filter_elems(p), em.c.val(w).is_const);
+    em.add("filter_pack", n.op, {w}, {wt}, 4.0 * p.oc * kdim * 3, 0,
+           [=](cudaStream_t st) { return launch_pack_filter_tc(p, s->fptr(w), s->fptr_mut(wt), st); });
+    const int res = ep.residual, gv = gate ? gate->gate : -1;
+    const double bytes = f32_bytes(xv) + f32_bytes(wv) + f32_bytes(ov) * (res >= 0 ? 2 : 1);
+    em.add("gemm_tf32x3_tcgen05", n.op, {x, wt, bias, gv, res}, {out}, bytes, flops, [=](cudaStream_t st) {
+      return launch_conv_tc(p, s->fptr(x), s->fptr(wt), bias >= 0 ? s->fptr(bias) : nullptr,
+                            gv >= 0 ? s->fptr(gv) : nullptr, res >= 0 ? s->fptr(res) : nullptr, s->fptr_mut(out), s->err_word, st);
+    });
+    return;
+  }
+  if (small_conv_applies(*s, flops) && !(pointwise && ohw == 1) && conv_simt_supported(p)) {
+    const int wt = new_value(em.c, conv_simt_ldw(p.oc) * kdim, em.c.val(w).is_const);
+    const int64_t oc = p.oc, kd = kdim;
+    em.add("filter_pack", n.op, {w}, {wt}, 8.0 * oc * kd, 0,
+           [=](cudaStream_t st) { return launch_pack_filter(s->fptr(w), s->fptr_mut(wt), oc, kd, st); });
+    const int res = ep.residual, gv = gate ? gate->gate : -1;
+    const double bytes = f32_bytes(xv) + f32_bytes(wv) + f32_bytes(ov) * (res >= 0 ? 2 : 1);
+    em.add("conv_fp32_simt", n.op, {x, wt, bias, gv, res}, {out}, bytes, flops, [=](cudaStream_t st) {
+      return launch_conv_simt(p, s->fptr(x), s->fptr(wt), bias >= 0 ? s->fptr(bias) : nullptr,
+                              gv >= 0 ? s->fptr(gv) : nullptr, res >= 0 ? s->fptr(res) : nullptr, s->fptr_mut(out), st);
+    });
+    return;
+  }
   int bsrc = x;
   if (!pointwise) {
     // Scratch column buffer col[n, c, kh, kw, oh, ow] (conv2d.rs:81-143).
@@ -1527,6 +1655,25 @@ void lower_node(Emit& em, Plan& plan, int nid) {
       const Value& xv = V(x);
       require_f32(xv, "GlobalAveragePool");
       const int64_t planes = xv.dims[0] * xv.dims[1], hw = xv.dims[2] * xv.dims[3];
+      auto sq = plan.squeeze.find(nid);
+      if (sq != plan.squeeze.end()) {
+        const Plan::Squeeze q = sq->second;
+        const int w1 = c.node(q.conv1).inputs[1], w2 = c.node(q.conv2).inputs[1];
+        const int64_t ch = xv.dims[1], hid = V(w1).dims[0], nb = xv.dims[0];
+        const double bytes = f32_bytes(xv) + f32_bytes(V(w1)) + f32_bytes(V(w2)) + 4.0 * planes;
+        em.add("squeeze_excite", n.op, {x, w1, q.b1, w2, q.b2}, {q.out}, bytes, 4.0 * nb * ch * hid, [=](cudaStream_t st) {
+          SqueezeExciteParams p{};
+          p.x = s->fptr(x);
+          p.w1 = s->fptr(w1); p.b1 = q.b1 >= 0 ? s->fptr(q.b1) : nullptr;
+          p.w2 = s->fptr(w2); p.b2 = q.b2 >= 0 ? s->fptr(q.b2) : nullptr;
+          p.gate = s->fptr_mut(q.out);
+          p.n = (int)nb; p.c = (int)ch; p.s = (int)hid; p.hw = hw;
+          p.act1 = q.act1; p.act2 = q.act2;
+          p.alpha1 = q.alpha1; p.beta1 = q.beta1; p.alpha2 = q.alpha2; p.beta2 = q.beta2;
+          return launch_squeeze_excite(p, st);
+        });
+        return;
+      }
       em.add("global_avg_pool", n.op, {x}, {o}, 4.0 * planes * hw + 4.0 * planes, 0,
              [=](cudaStream_t st) { return launch_gavg_pool(s->fptr(x), s->fptr_mut(o), planes, hw, st); });
       return;
@@ -1804,6 +1951,7 @@ void lower_graph(AcSession& s) {
       detect_layer_norm(c, plan);
       detect_hardswish(c, plan);
       detect_se_gate(c, plan);
+      detect_squeeze(c, plan);
       detect_reduce_siblings(c, plan);
       // Debug toggle: ALTIUS_CUDA_NO_FUSED_SPLIT=1 keeps a split kernel in front of every pair GEMM.
       if (!std::getenv("ALTIUS_CUDA_NO_FUSED_SPLIT")) plan_presplit(c, plan);

@@ -1,0 +1,183 @@
+// The squeeze-and-excite block of the MobileNets up to its gate,
+//   GlobalAveragePool -> 1 x 1 Conv + act -> 1 x 1 Conv + act,
+// in one kernel. As three launches (pool, and two products of a few rows against up to 960 x 240
+// weights) it took 20 to 145 us per block of the network at a batch of one: one or two blocks of a
+// GEMM walked K alone. The work is 0.5 MFLOP and 2 MB of weights per image, so it is bound by
+// latency: a cluster of eight blocks shares one to four images; every block pools its eighth of the
+// channels and leaves the means in the shared memory of all eight, computes an eighth of the hidden
+// units from them and exchanges those in the same way, then finishes its eighth of the gate.
+// Several images per cluster (from a batch of 17 on, when the clusters of one image no longer fit
+// the SMs at once) read the weights once for all of them.
+#include <cooperative_groups.h>
+
+#include "kernels.h"
+#include "pdl.cuh"
+#include "ref_math.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace ac {
+namespace {
+
+constexpr int kCluster = 8, kThreads = 1024, kWarps = kThreads / 32;
+
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ __forceinline__ float sum8(float v) {   // over eight neighbouring lanes
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ __forceinline__ float dot4(float4 a, float4 b, float acc) {
+  return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, acc))));
+}
+__device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+template <int G>
+__global__ void __launch_bounds__(kThreads) squeeze_excite_kernel(const SqueezeExciteParams p) {
+  extern __shared__ __align__(16) float smem[];
+  float* mean = smem;                 // [G][c]
+  float* hid = smem + G * p.c;        // [G][s]
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = blockIdx.z, n0 = blockIdx.x * G;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7, quarter = lane >> 3;
+  const int c = p.c, s = p.s, hw = (int)p.hw;
+  const int cper = (c + kCluster - 1) / kCluster, c0 = rank * cper, c1 = min(c, c0 + cper), cn = max(c1 - c0, 0);
+  cl.barrier_arrive();
+  // The warp's first row of W1 is requested before anything else; eight loads of a lane cover 1024 inputs.
+  const int j0 = rank + kCluster * warp;
+  float4 w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int k = lane * 4 + i * 128;
+    w[i] = j0 < s && k < c ? ldg4(p.w1 + (long long)j0 * c + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  pdl_trigger();
+  pdl_wait();
+  cl.barrier_wait();                  // every block of the cluster runs: its shared memory may be written
+
+  // ---- means of this block's channels: eight lanes each ----
+  const bool v4 = (hw & 3) == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0;
+  for (int i = warp * 4; i < G * cn; i += kWarps * 4) {
+    const int item = i + quarter, g = min(item / max(cn, 1), G - 1), ch = c0 + item - g * cn;
+    const bool ok = item < G * cn && n0 + g < p.n;
+    float acc = 0.f;
+    if (ok) {
+      const float* row = p.x + ((long long)(n0 + g) * c + ch) * hw;
+      if (v4) {
+#pragma unroll 8
+        for (int j = sub * 4; j < hw; j += 32) {
+          const float4 v = *reinterpret_cast<const float4*>(row + j);
+          acc = __fadd_rn(acc, __fadd_rn(__fadd_rn(v.x, v.y), __fadd_rn(v.z, v.w)));
+        }
+      } else {
+#pragma unroll 8
+        for (int j = sub; j < hw; j += 8) acc = __fadd_rn(acc, row[j]);
+      }
+    }
+    acc = __fdiv_rn(sum8(acc), (float)hw);
+    if (item < G * cn) cl.map_shared_rank(mean, sub)[g * c + ch] = acc;
+  }
+  cl.sync();
+
+  // ---- hidden units rank, rank + 8, ...: a warp each, all G images at once ----
+  for (int j = j0; j < s; j += kCluster * kWarps) {
+    float acc[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) acc[g] = 0.f;
+    const float* row = p.w1 + (long long)j * c;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = lane * 4 + i * 128;
+      if (k >= c) continue;
+      const float4 wv = j == j0 ? w[i] : ldg4(row + k);
+#pragma unroll
+      for (int g = 0; g < G; ++g) acc[g] = dot4(wv, lds4(mean + g * c + k), acc[g]);
+    }
+    for (int k = 1024 + lane * 4; k < c; k += 128) {
+      const float4 wv = ldg4(row + k);
+#pragma unroll
+      for (int g = 0; g < G; ++g) acc[g] = dot4(wv, lds4(mean + g * c + k), acc[g]);
+    }
+    float v = 0.f;                    // lane g * 8 + q sends image g to block q
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const float u = warp_sum(acc[g]);
+      if (quarter == g) v = u;
+    }
+    if (p.b1) v = __fadd_rn(v, __ldg(p.b1 + j));
+    v = apply_act(p.act1, v, p.alpha1, p.beta1);
+    if (quarter < G) cl.map_shared_rank(hid, sub)[quarter * s + j] = v;
+  }
+  // The lane's part of its first row of W2: eight loads cover 256 hidden units.
+  const int ch0 = c0 + warp * 4 + quarter;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int k = sub * 4 + i * 32;
+    w[i] = ch0 < c1 && k < s ? ldg4(p.w2 + (long long)ch0 * s + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  cl.sync();
+
+  // ---- gate: eight lanes per channel ----
+  for (int ch = ch0; ch - quarter < c1; ch += kWarps * 4) {
+    float acc[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) acc[g] = 0.f;
+    if (ch < c1) {
+      const float* row = p.w2 + (long long)ch * s;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = sub * 4 + i * 32;
+        if (k >= s) continue;
+        const float4 wv = ch == ch0 ? w[i] : ldg4(row + k);
+#pragma unroll
+        for (int g = 0; g < G; ++g) acc[g] = dot4(wv, lds4(hid + g * s + k), acc[g]);
+      }
+      for (int k = 256 + sub * 4; k < s; k += 32) {
+        const float4 wv = ldg4(row + k);
+#pragma unroll
+        for (int g = 0; g < G; ++g) acc[g] = dot4(wv, lds4(hid + g * s + k), acc[g]);
+      }
+    }
+    float v = 0.f;                    // lane sub == g finishes image g
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const float u = sum8(acc[g]);
+      if (sub == g) v = u;
+    }
+    if (ch < c1 && sub < G && n0 + sub < p.n) {
+      if (p.b2) v = __fadd_rn(v, __ldg(p.b2 + ch));
+      p.gate[(long long)(n0 + sub) * c + ch] = apply_act(p.act2, v, p.alpha2, p.beta2);
+    }
+  }
+}
+
+template <int G>
+cudaError_t launch_g(const SqueezeExciteParams& p, cudaStream_t st) {
+  return launch_pdl(squeeze_excite_kernel<G>, dim3((unsigned)((p.n + G - 1) / G), 1, kCluster), dim3(kThreads),
+                    (size_t)G * (p.c + p.s) * sizeof(float), st, kCluster, p);
+}
+
+inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
+
+}  // namespace
+
+bool squeeze_excite_supported(const SqueezeExciteParams& p) {
+  // Rows of the weights (and of the vectors in shared memory) are read as float4s; four images'
+  // vectors fit the 48 KB every kernel may use.
+  return p.c >= 8 && (p.c % 4) == 0 && p.s >= 4 && (p.s % 4) == 0 && p.c + p.s <= 3072 && p.n >= 1 && p.hw >= 1 &&
+         p.hw < (1 << 28);
+}
+
+cudaError_t launch_squeeze_excite(const SqueezeExciteParams& p, cudaStream_t st) {
+  if (!squeeze_excite_supported(p) || !al16(p.w1) || !al16(p.w2)) return cudaErrorInvalidValue;
+  const int per_wave = 16;            // clusters of eight that run at once: two in each part of the chip that can hold one
+  if (p.n <= per_wave) return launch_g<1>(p, st);
+  return p.n <= 2 * per_wave ? launch_g<2>(p, st) : launch_g<4>(p, st);
+}
+
+}  // namespace ac

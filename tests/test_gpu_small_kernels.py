@@ -1,0 +1,125 @@
+"""Kernels for small problems against float64: convolutions below the tensor cores' size, the
+squeeze-and-excite block, products of a few rows. All are fp32 dot products of K terms in another
+order than the oracle's; each of the at most K + 8 roundings of a partial sum is off by at most
+2^-24 of sum |a||b|, so (K + 8) * 2^-24 * sum |a||b| bounds the error whatever the order."""
+import numpy as np
+import pytest
+import torch
+
+from altius_b200 import ir
+from altius_b200.session import CudaSessionBuilder
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -24
+
+
+def _run(build, inputs, kinds=None):
+    g = ir.Graph()
+    vals = [g.add_input(f"in{i}", a.shape) for i, a in enumerate(inputs)]
+    g.outputs.append(build(g, *vals))
+    sess = CudaSessionBuilder(ir.Model(g, 13)).build()
+    try:
+        if kinds:
+            assert [e["kind"] for e in sess.schedule()] == kinds
+        return sess.run(list(inputs))[0]
+    finally:
+        sess.close()
+
+
+def _conv(g, x, w, b, k=1, s=1, p=0):
+    return g.op("Conv2d", x, g.new_init(w), g.new_init(b), kernel_shape=[k, k], strides=[s, s], padding=[p] * 4,
+                dilations=[1, 1], group=1, auto_pad="")
+
+
+# n, c, h, oc, kernel, stride, pad, gate: one K step and several (cluster split), channel counts off
+# the tile, planes whose rows are not whole float4s, columns across images, more than 148 tiles
+@pytest.mark.parametrize("n,c,h,oc,k,s,p,gate", [
+    (1, 16, 8, 16, 1, 1, 0, False), (1, 240, 14, 80, 1, 1, 0, True), (3, 61, 7, 37, 1, 1, 0, True),
+    (2, 960, 3, 5, 1, 1, 0, False), (1, 3, 33, 16, 3, 2, 1, False), (2, 7, 9, 12, 5, 1, 2, False),
+    (1, 16, 112, 16, 1, 1, 0, False), (5, 9, 31, 33, 1, 1, 0, True), (1, 33, 17, 40, 1, 2, 0, False)])
+def test_small_convolution(cuda_lib, n, c, h, oc, k, s, p, gate):
+    rng = np.random.default_rng(c * h + oc)
+    x = rng.standard_normal((n, c, h, h)).astype(np.float32)
+    w = rng.standard_normal((oc, c, k, k)).astype(np.float32)
+    b = rng.standard_normal(oc).astype(np.float32)
+    gt = rng.random((n, c, 1, 1)).astype(np.float32)
+    oh = (h + 2 * p - k) // s + 1
+    r = rng.standard_normal((n, oc, oh, oh)).astype(np.float32)
+
+    def build(g, xi, ri, gi=None):
+        y = _conv(g, g.op("Mul", xi, gi) if gate else xi, w, b, k, s, p)
+        return g.op("Add", g.op("ReLU", y), ri)
+    got = _run(build, [x, r] + ([gt] if gate else []), ["conv_fp32_simt"])
+    xg = torch.from_numpy(x * gt if gate else x).double()
+    conv = lambda a, f, bias: torch.nn.functional.conv2d(a, f, bias, stride=s, padding=p)
+    want = torch.relu(conv(xg, torch.from_numpy(w).double(), torch.from_numpy(b).double())).numpy() + r
+    mass = conv(xg.abs(), torch.from_numpy(w).double().abs(), torch.from_numpy(b).double().abs()).numpy() + np.abs(r)
+    assert (np.abs(got - want) <= (c * k * k + 8) * EPS * mass).all()
+
+
+# one, two and four images per cluster, with a remainder; planes with and without whole float4s
+@pytest.mark.parametrize("n,c,h,s", [(1, 72, 28, 24), (3, 960, 7, 240), (19, 120, 14, 32), (41, 36, 5, 4), (1, 8, 1, 8)])
+def test_squeeze_excite_block(cuda_lib, n, c, h, s):
+    rng = np.random.default_rng(c + h)
+    x = rng.standard_normal((n, c, h, h)).astype(np.float32) + 0.5
+    w1, w2 = (rng.standard_normal(d).astype(np.float32) / 4 for d in ((s, c, 1, 1), (c, s, 1, 1)))
+    b1, b2 = rng.standard_normal(s).astype(np.float32), rng.standard_normal(c).astype(np.float32)
+
+    def build(g, xi):
+        z = g.op("ReLU", _conv(g, g.op("GlobalAveragePool", xi), w1, b1))
+        return g.op("HardSigmoid", _conv(g, z, w2, b2), alpha=0.2, beta=0.5)
+    got = _run(build, [x], ["squeeze_excite"])[:, :, 0, 0]
+    x64, a1, a2 = x.astype(np.float64), w1[:, :, 0, 0].astype(np.float64), w2[:, :, 0, 0].astype(np.float64)
+    mean = x64.mean((2, 3))
+    hid = np.maximum(mean @ a1.T + b1, 0)
+    z = hid @ a2.T + b2
+    # errors of the means and of the first product pass through |W| with slope at most one
+    e_mean = (h * h + 8) * EPS * np.abs(x64).mean((2, 3))
+    e_hid = e_mean @ np.abs(a1).T + (c + 8) * EPS * (np.abs(mean) @ np.abs(a1).T + np.abs(b1))
+    e_z = e_hid @ np.abs(a2).T + (s + 8) * EPS * (hid @ np.abs(a2).T + np.abs(b2))
+    assert (np.abs(got - np.clip(0.2 * z + 0.5, 0, 1)) <= 0.2 * e_z + 4 * EPS).all()
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 4, 3), (1, 768, 1000), (2, 132, 17), (3, 256, 10), (4, 60, 33), (9, 1280, 65), (32, 960, 1280)])
+def test_product_of_a_few_rows(cuda_lib, m, k, n):
+    rng = np.random.default_rng(m + k + n)
+    a = rng.standard_normal((m, k)).astype(np.float32)
+    w = rng.standard_normal((n, k)).astype(np.float32)
+    b = rng.standard_normal(n).astype(np.float32)
+    got = _run(lambda g, x: g.op("ReLU", g.op("Gemm", x, g.new_init(w), g.new_init(b), alpha=0.5, beta=2.0, trans_a=False,
+                                              trans_b=True)), [a], ["gemm_fp32_rows"])
+    a64, w64 = a.astype(np.float64), w.astype(np.float64)
+    want = np.maximum(0.5 * (a64 @ w64.T) + 2.0 * b, 0)
+    assert (np.abs(got - want) <= (k + 8) * EPS * (0.5 * (np.abs(a64) @ np.abs(w64).T) + 2.0 * np.abs(b))).all()
+    w2 = np.ascontiguousarray(w.T)     # stored [K, N]: transposed once at create
+    got = _run(lambda g, x: g.op("MatMul", x, g.new_init(w2)), [a], ["gemm_fp32_rows"])
+    assert (np.abs(got - a64 @ w64.T) <= (k + 8) * EPS * (np.abs(a64) @ np.abs(w64).T)).all()
+
+
+# 3xTF32 with a tensor-memory accumulator that truncates after every MMA step of 8 products: two
+# operands of 22 bits and K / 8 * 3 truncations of at most 2^-23 each of the partial sum, with
+# the bound the other tensor-core tests use for the latter: 1e-5 |want| + 5e-6 sum |a||b|.
+# Channel counts off the 16s, K off the 8s and 32s, planes of odd size, K cut over a cluster of
+# eight, several channel tiles, windows, a gate; residual and bias always.
+@pytest.mark.parametrize("n,c,h,oc,k,s,p,gate", [
+    (3, 21, 57, 27, 1, 1, 0, True), (2, 960, 7, 160, 1, 1, 0, True), (1, 672, 14, 112, 1, 1, 0, False),
+    (5, 40, 28, 241, 1, 1, 0, False), (2, 3, 97, 33, 3, 2, 1, False), (1, 72, 14, 80, 5, 1, 2, False),
+    (2, 1, 512, 16, 1, 1, 0, True), (1, 4096, 5, 300, 1, 1, 0, False), (32, 16, 40, 64, 1, 1, 0, False)])
+def test_tensor_core_convolution(cuda_lib, n, c, h, oc, k, s, p, gate):
+    rng = np.random.default_rng(c * h + oc)
+    x = rng.standard_normal((n, c, h, h)).astype(np.float32)
+    w = rng.standard_normal((oc, c, k, k)).astype(np.float32)
+    b = rng.standard_normal(oc).astype(np.float32)
+    gt = rng.random((n, c, 1, 1)).astype(np.float32)
+    oh = (h + 2 * p - k) // s + 1
+    r = rng.standard_normal((n, oc, oh, oh)).astype(np.float32)
+
+    def build(g, xi, ri, gi=None):
+        y = _conv(g, g.op("Mul", xi, gi) if gate else xi, w, b, k, s, p)
+        return g.op("Add", g.op("ReLU", y), ri)
+    got = _run(build, [x, r] + ([gt] if gate else []), ["gemm_tf32x3_tcgen05"])
+    xg = torch.from_numpy(x * gt if gate else x).double()
+    conv = lambda a, f, bias: torch.nn.functional.conv2d(a, f, bias, stride=s, padding=p)
+    want = torch.relu(conv(xg, torch.from_numpy(w).double(), torch.from_numpy(b).double())).numpy() + r
+    mass = conv(xg.abs(), torch.from_numpy(w).double().abs(), torch.from_numpy(b).double().abs()).numpy() + np.abs(r)
+    assert (np.abs(got - want) <= 1e-5 * np.abs(want) + 5e-6 * mass).all()
