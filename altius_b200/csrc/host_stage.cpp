@@ -1,0 +1,144 @@
+#include "host_stage.h"
+
+#include <algorithm>
+#include <cstring>
+#include <map>
+
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
+
+namespace ac {
+namespace {
+inline void relax() {
+#if defined(__x86_64__)
+  _mm_pause();
+#else
+  std::this_thread::yield();
+#endif
+}
+}  // namespace
+
+std::shared_ptr<HostStage> HostStage::of_device(int device) {
+  static std::mutex m;
+  static std::map<int, std::weak_ptr<HostStage>> made;
+  std::lock_guard<std::mutex> lock(m);
+  if (std::shared_ptr<HostStage> s = made[device].lock()) return s;
+  std::shared_ptr<HostStage> s(new HostStage());
+  if (!s->init()) return nullptr;
+  made[device] = s;
+  return s;
+}
+
+bool HostStage::init() {
+  if (cudaHostAlloc(reinterpret_cast<void**>(&ring_), kChunk * kSlots, cudaHostAllocPortable) != cudaSuccess) {
+    (void)cudaGetLastError();
+    ring_ = nullptr;
+    return false;
+  }
+  for (cudaEvent_t& e : left_)
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+  const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
+  for (int i = 0; i < std::min(6, cores / 2); ++i) threads_.emplace_back([this] { worker(); });
+  return true;
+}
+
+HostStage::~HostStage() {
+  {
+    std::lock_guard<std::mutex> lock(m_);
+    stop_ = true;
+  }
+  cv_.notify_all();
+  for (std::thread& t : threads_) t.join();
+  for (cudaEvent_t e : left_)
+    if (e) cudaEventDestroy(e);
+  if (ring_) cudaFreeHost(ring_);
+}
+
+// Copies the next chunk below `limit` whose slot is free; false if there is none now.
+bool HostStage::copy_next(int limit) {
+  int c = next_.load(std::memory_order_relaxed);
+  if (c >= limit || c >= allowed_.load(std::memory_order_acquire)) return false;
+  if (!next_.compare_exchange_strong(c, c + 1)) return false;
+  const size_t at = (size_t)c * kChunk;
+  std::memcpy(ring_ + (size_t)(c % kSlots) * kChunk, src_ + at, std::min(kChunk, bytes_ - at));
+  done_[c].store(1, std::memory_order_release);
+  return true;
+}
+
+void HostStage::worker() {
+  uint64_t seen = 0;
+  for (;;) {
+    {
+      std::unique_lock<std::mutex> lock(m_);
+      cv_.wait(lock, [&] { return stop_ || job_ != seen; });
+      if (stop_) return;
+      seen = job_;
+      ++busy_;
+    }
+    while (next_.load(std::memory_order_relaxed) < chunks_)
+      if (!copy_next(chunks_)) relax();
+    std::lock_guard<std::mutex> lock(m_);
+    --busy_;
+  }
+}
+
+cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  std::lock_guard<std::mutex> use(use_);
+  const int n = (int)((bytes + kChunk - 1) / kChunk);
+  for (cudaEvent_t e : left_)                 // slots an earlier upload may still occupy
+    if (cudaError_t err = cudaEventSynchronize(e)) return err;
+  {
+    // Workers that have not left the previous job yet (all its chunks are taken: soon).
+    std::unique_lock<std::mutex> lock(m_);
+    while (busy_ > 0) {
+      lock.unlock();
+      relax();
+      lock.lock();
+    }
+    if (done_size_ < n) {
+      done_.reset(new std::atomic<char>[n]);
+      done_size_ = n;
+    }
+    for (int i = 0; i < n; ++i) done_[i].store(0, std::memory_order_relaxed);
+    src_ = static_cast<const char*>(src);
+    bytes_ = bytes;
+    chunks_ = n;
+    next_.store(0);
+    allowed_.store(std::min(n, kSlots));
+    ++job_;
+  }
+  cv_.notify_all();
+  cudaError_t err = cudaSuccess;
+  int allowed = std::min(n, kSlots);
+  for (int c = 0; c < n && err == cudaSuccess; ++c) {
+    do {
+      // Chunk allowed - kSlots is on its way (it is below c): once it has left, its slot is free.
+      while (allowed < n && allowed - kSlots < c) {
+        if (cudaEventQuery(left_[allowed % kSlots]) != cudaSuccess) {
+          (void)cudaGetLastError();
+          break;
+        }
+        allowed_.store(++allowed, std::memory_order_release);
+      }
+      if (!copy_next(c + 1)) relax();         // this chunk itself, if no worker has taken it yet
+    } while (!done_[c].load(std::memory_order_acquire));
+    const size_t at = (size_t)c * kChunk;
+    err = cudaMemcpyAsync(static_cast<char*>(dst) + at, ring_ + (size_t)(c % kSlots) * kChunk, std::min(kChunk, bytes - at),
+                          cudaMemcpyHostToDevice, st);
+    if (err == cudaSuccess) err = cudaEventRecord(left_[c % kSlots], st);
+  }
+  if (err != cudaSuccess) {                   // nobody may go on reading the caller's memory
+    next_.store(n);
+    for (;;) {
+      std::lock_guard<std::mutex> lock(m_);
+      if (busy_ == 0) break;
+    }
+  }
+  return err;
+}
+
+}  // namespace ac

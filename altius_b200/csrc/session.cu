@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <set>
 
 #include "session.h"
 
@@ -175,9 +176,147 @@ void upload_weights(AcSession& s, const AcGraphDesc& g) {
     if (v.is_init) v.host = v.host_owned.empty() ? nullptr : v.host_owned.data();
 }
 
-cudaError_t replay(AcSession* s, cudaStream_t st) {
-  for (Step& step : s->steps) {
-    cudaError_t e = step.fn(st);
+cudaError_t replay(AcSession* s, cudaStream_t st, int first, int last) {
+  for (int i = first; i < last; ++i) {
+    cudaError_t e = s->steps[i].fn(st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+cudaError_t replay(AcSession* s, cudaStream_t st) { return replay(s, st, 0, (int)s->steps.size()); }
+
+cudaError_t capture(AcSession* s, int first, int last, cudaGraph_t* graph, cudaGraphExec_t* exec) {
+  cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return e;
+  e = replay(s, s->stream, first, last);
+  const cudaError_t e2 = cudaStreamEndCapture(s->stream, graph);
+  if (e != cudaSuccess) return e;
+  if (e2 != cudaSuccess) return e2;
+  return cudaGraphInstantiate(exec, *graph, 0);
+}
+
+cudaError_t launch_all(AcSession* s) { return s->graph_exec ? cudaGraphLaunch(s->graph_exec, s->stream) : replay(s, s->stream); }
+
+// A run on device buffers need not copy them in and out of the arena (115 of the 200 us that the
+// tensor-op micrograph spent on the GPU): the kernels that read a graph input or write a graph
+// output take the caller's pointers. Their launches cannot be in a graph then, so this is done where
+// they are few and together: at most six segments, at most eight such steps (a launch
+// costs the host about 3 us, a graph of any size 1 us).
+void plan_segments(AcSession& s) {
+  std::vector<char> io(s.storages.size(), 0);
+  std::set<int> seen;
+  auto bindable = [&](int v) {
+    const int sid = s.values[v].storage;
+    if (s.values[v].is_const || s.storages[sid].weight || !seen.insert(sid).second) return false;
+    io[sid] = 1;
+    return true;
+  };
+  for (int v : s.inputs)
+    if (!bindable(v)) return;
+  for (int v : s.outputs)
+    if (!bindable(v)) return;
+  for (const Step& st : s.init_steps)
+    for (int w : st.writes)
+      if (io[w]) return;
+  int direct = 0;
+  std::vector<Segment> segs;
+  for (int i = 0; i < (int)s.steps.size(); ++i) {
+    bool touches = false;
+    for (int r : s.steps[i].reads) touches = touches || io[r];
+    for (int w : s.steps[i].writes) touches = touches || io[w];
+    direct += touches;
+    // A graph segment is marked by last < 0 until its end is known.
+    if (segs.empty() || touches != (segs.back().graph == nullptr)) {
+      Segment g;
+      g.first = i;
+      g.graph = touches ? nullptr : reinterpret_cast<cudaGraph_t>(1);
+      segs.push_back(g);
+    }
+    segs.back().last = i + 1;
+  }
+  if (segs.size() > 6 || direct > 8) return;
+  for (Segment& g : segs) {
+    if (!g.graph) continue;
+    g.graph = nullptr;
+    if (cudaError_t e = capture(&s, g.first, g.last, &g.graph, &g.exec)) {
+      s.segments = segs;               // destroyed with the session
+      fail(AC_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
+    }
+  }
+  s.segments = segs;
+}
+
+// Kernels read and write with 16-byte accesses; a result may not land on a buffer that a later
+// kernel still reads.
+bool can_bind(const AcSession* s, const void* const* ins, void* const* outs) {
+  if (s->segments.empty()) return false;
+  std::vector<std::pair<uintptr_t, uintptr_t>> in, out;
+  for (size_t i = 0; i < s->inputs.size(); ++i) {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(ins[i]);
+    if (p & 15) return false;
+    in.push_back({p, p + s->values[s->inputs[i]].bytes()});
+  }
+  for (size_t i = 0; i < s->outputs.size(); ++i) {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(outs[i]);
+    if (p & 15) return false;
+    out.push_back({p, p + s->values[s->outputs[i]].bytes()});
+  }
+  for (size_t i = 0; i < out.size(); ++i) {
+    for (auto& q : in)
+      if (out[i].first < q.second && q.first < out[i].second) return false;
+    for (size_t j = i + 1; j < out.size(); ++j)
+      if (out[i].first < out[j].second && out[j].first < out[i].second) return false;
+  }
+  return true;
+}
+
+// The schedule with device buffers in place of the arena slots of the graph's inputs (and outputs,
+// unless outs is null).
+cudaError_t launch_bound(AcSession* s, const void* const* ins, void* const* outs) {
+  auto bind = [&](bool on) {
+    for (size_t i = 0; i < s->inputs.size(); ++i)
+      s->storages[s->values[s->inputs[i]].storage].bound = on ? const_cast<void*>(ins[i]) : nullptr;
+    for (size_t i = 0; outs && i < s->outputs.size(); ++i)
+      s->storages[s->values[s->outputs[i]].storage].bound = on ? outs[i] : nullptr;
+  };
+  bind(true);
+  cudaError_t e = cudaSuccess;
+  for (const Segment& g : s->segments) {
+    e = g.exec ? cudaGraphLaunch(g.exec, s->stream) : replay(s, s->stream, g.first, g.last);
+    if (e != cudaSuccess) break;
+  }
+  bind(false);
+  return e;
+}
+
+cudaError_t use_device(int device) {
+  int cur = -1;
+  if (cudaGetDevice(&cur) == cudaSuccess && cur == device) return cudaSuccess;
+  return cudaSetDevice(device);
+}
+
+constexpr size_t kSmallIo = size_t(1) << 20;   // inputs (outputs) up to this go through the session's staging block
+
+// Host inputs into the arena. Small ones are gathered in the page-locked block first: the driver's own
+// path from pageable memory costs a call of up to 35 us there, the copy into the block 1 to 13.
+cudaError_t upload_inputs(AcSession* s, const void* const* ins) {
+  size_t at = 0;
+  for (size_t i = 0; i < s->inputs.size(); ++i) {
+    const size_t bytes = s->values[s->inputs[i]].bytes();
+    void* dst = s->ptr(s->inputs[i]);
+    cudaError_t e;
+    if (s->stage_in) {
+      std::memcpy(s->stage_in + at, ins[i], bytes);
+      e = cudaMemcpyAsync(dst, s->stage_in + at, bytes, cudaMemcpyHostToDevice, s->stream);
+      at += align_up(bytes, 256);
+    } else {
+      cudaPointerAttributes pa{};
+      bool pageable = bytes > kSmallIo;
+      if (pageable && cudaPointerGetAttributes(&pa, ins[i]) == cudaSuccess) pageable = pa.type == cudaMemoryTypeUnregistered;
+      if (pageable && !s->host_stage) s->host_stage = HostStage::of_device(s->device);
+      e = pageable && s->host_stage ? s->host_stage->upload(dst, ins[i], bytes, s->stream)
+                                    : cudaMemcpyAsync(dst, ins[i], bytes, cudaMemcpyHostToDevice, s->stream);
+    }
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -261,9 +400,7 @@ int create_fallback(AcSession* s) {
 int check_err_word(AcSession* s) {
   const int code = *s->err_host;
   if (code == 0) return AC_OK;
-  cudaMemsetAsync(s->err_word, 0, sizeof(int), s->stream);
-  cudaStreamSynchronize(s->stream);
-  *s->err_host = 0;
+  *s->err_host = 0;      // the stream has been drained: no kernel writes it now
   if (code == kGemmRangeCode && s->opt.gemm_mode == 0) {
     const int rc = create_fallback(s);
     if (rc != AC_OK) return rc;
@@ -289,18 +426,21 @@ int run_common(AcSession* s, const void* const* ins, void* const* outs, bool dev
     if (rc != AC_OK) s->err = s->fallback->err;
     return rc;
   }
-  cudaError_t e = cudaSetDevice(s->device);
+  cudaError_t e = use_device(s->device);
   if (e != cudaSuccess) return set_err(s, AC_ERR_CUDA, cudaGetErrorString(e));
-  const cudaMemcpyKind in_kind = device_io ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  const cudaMemcpyKind out_kind = device_io ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   // An error after this point drains the stream before returning, for the same reason.
   auto fail_cuda = [&](const std::string& what, cudaError_t err) {
     cudaStreamSynchronize(s->stream);
     return set_err(s, AC_ERR_CUDA, what + cudaGetErrorString(err));
   };
-  for (size_t i = 0; i < s->inputs.size(); ++i) {
-    const Value& v = s->values[s->inputs[i]];
-    e = cudaMemcpyAsync(s->ptr(s->inputs[i]), ins[i], v.bytes(), in_kind, s->stream);
+  const bool bound = device_io && can_bind(s, ins, outs);
+  if (!bound) {
+    if (device_io) {
+      for (size_t i = 0; i < s->inputs.size() && e == cudaSuccess; ++i)
+        e = cudaMemcpyAsync(s->ptr(s->inputs[i]), ins[i], s->values[s->inputs[i]].bytes(), cudaMemcpyDeviceToDevice, s->stream);
+    } else {
+      e = upload_inputs(s, ins);
+    }
     if (e != cudaSuccess) return fail_cuda("input copy: ", e);
   }
   if (s->opt.enable_profiling) {
@@ -314,22 +454,30 @@ int run_common(AcSession* s, const void* const* ins, void* const* outs, bool dev
       if (e != cudaSuccess) return fail_cuda(s->steps[i].kind + ": ", e);
       cudaEventRecord(s->events[2 * i + 1], s->stream);
     }
-  } else if (s->graph_exec) {
-    e = cudaGraphLaunch(s->graph_exec, s->stream);
-    if (e != cudaSuccess) return fail_cuda("graph launch: ", e);
   } else {
-    e = replay(s, s->stream);
+    e = bound ? launch_bound(s, ins, outs) : launch_all(s);
     if (e != cudaSuccess) return fail_cuda("kernel launch: ", e);
   }
-  for (size_t i = 0; i < s->outputs.size(); ++i) {
-    const Value& v = s->values[s->outputs[i]];
-    e = cudaMemcpyAsync(outs[i], s->ptr(s->outputs[i]), v.bytes(), out_kind, s->stream);
+  size_t at = 0;
+  for (size_t i = 0; i < s->outputs.size() && !bound; ++i) {
+    const size_t bytes = s->values[s->outputs[i]].bytes();
+    const bool staged = !device_io && s->stage_out;
+    e = cudaMemcpyAsync(staged ? s->stage_out + at : outs[i], s->ptr(s->outputs[i]), bytes,
+                        device_io ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s->stream);
     if (e != cudaSuccess) return fail_cuda("output copy: ", e);
+    at += align_up(bytes, 256);
   }
-  cudaMemcpyAsync(s->err_host, s->err_word, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
   e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) return set_err(s, AC_ERR_CUDA, std::string("run: ") + cudaGetErrorString(e));
   if (const int rc = check_err_word(s)) return rc == 1 ? run_common(s, ins, outs, device_io) : rc;
+  if (!device_io && s->stage_out) {
+    at = 0;
+    for (size_t i = 0; i < s->outputs.size(); ++i) {
+      const size_t bytes = s->values[s->outputs[i]].bytes();
+      std::memcpy(outs[i], s->stage_out + at, bytes);
+      at += align_up(bytes, 256);
+    }
+  }
   if (s->opt.enable_profiling) {
     for (size_t i = 0; i < s->steps.size(); ++i) {
       float ms = 0.f;
@@ -376,25 +524,33 @@ int create_session(const AcGraphDesc* graph, const AcOptions* options, AcSession
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
       fail(AC_ERR_NO_DEVICE, "no CUDA device is visible: this backend has no CPU fallback");
     if (s->device < 0 || s->device >= ndev) fail(AC_ERR_NO_DEVICE, "device ordinal out of range");
-    cudaDeviceProp prop;
-    AC_CUDA(cudaGetDeviceProperties(&prop, s->device));
-    if (prop.major != 10)
+    int major = 0;
+    AC_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, s->device));
+    if (major != 10)
       fail(AC_ERR_NO_DEVICE, "device is not sm_100 (the kernels are built for sm_100a only)");
     AC_CUDA(cudaSetDevice(s->device));
     AC_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-    AC_CUDA(cudaMalloc(&s->err_word, sizeof(int)));
-    AC_CUDA(cudaMemset(s->err_word, 0, sizeof(int)));
-    AC_CUDA(cudaHostAlloc(&s->err_host, sizeof(int), cudaHostAllocDefault));
-    *s->err_host = 0;
     parse_graph(*s, *graph);
     infer_shapes(*s);
+    {
+      size_t in = 0, out = 0;
+      for (int v : s->inputs) in += align_up(s->values[v].bytes(), 256);
+      for (int v : s->outputs) out += align_up(s->values[v].bytes(), 256);
+      if (in > kSmallIo) in = 0;
+      if (out > kSmallIo) out = 0;
+      AC_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&s->host_block), 256 + in + out, cudaHostAllocMapped));
+      s->err_host = reinterpret_cast<int*>(s->host_block);
+      *s->err_host = 0;
+      AC_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->err_word), s->host_block, 0));
+      if (in) s->stage_in = s->host_block + 256;
+      if (out) s->stage_out = s->host_block + 256 + in;
+    }
     lower_graph(*s);
     plan_arena(*s);
     AC_CUDA(cudaMalloc(&s->arena, s->arena_bytes));
     upload_weights(*s, *graph);
     for (Step& st : s->init_steps) AC_CUDA(st.fn(s->stream));
     AC_CUDA(cudaStreamSynchronize(s->stream));
-    AC_CUDA(cudaMemcpy(s->err_host, s->err_word, sizeof(int), cudaMemcpyDeviceToHost));
     if (*s->err_host == kGemmRangeCode) fail(-kGemmRangeCode, "a constant operand exceeds the fp16 range");
     if (*s->err_host != 0) fail(AC_ERR_CUDA, "a kernel gave up a bounded wait while preparing constants");
     if (s->opt.gemm_mode == 0) s->desc = copy_graph(*graph);
@@ -406,12 +562,9 @@ int create_session(const AcGraphDesc* graph, const AcOptions* options, AcSession
         AC_CUDA(cudaMemset(s->sweep_buf, 0, kSweepBytes));
       }
     } else if (!s->opt.disable_cuda_graph && !s->steps.empty()) {
-      AC_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-      cudaError_t e = replay(s, s->stream);
-      cudaError_t e2 = cudaStreamEndCapture(s->stream, &s->graph);
+      const cudaError_t e = capture(s, 0, (int)s->steps.size(), &s->graph, &s->graph_exec);
       if (e != cudaSuccess) fail(AC_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-      AC_CUDA(e2);
-      AC_CUDA(cudaGraphInstantiate(&s->graph_exec, s->graph, 0));
+      plan_segments(*s);
     }
   } catch (const BuildError& e) {
     set_err(nullptr, e.status, e.msg);
@@ -469,7 +622,7 @@ int altius_cuda_run_batches(AcSession* s, int32_t n_batches, const void* const* 
     }
     return AC_OK;
   }
-  cudaError_t e = cudaSetDevice(s->device);
+  cudaError_t e = use_device(s->device);
   if (e == cudaSuccess && !s->copy_stream) {
     e = cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking);
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
@@ -489,19 +642,23 @@ int altius_cuda_run_batches(AcSession* s, int32_t n_batches, const void* const* 
       e = cudaMemcpyAsync(s->staging[k][i], src, s->values[s->inputs[i]].bytes(), cudaMemcpyHostToDevice, s->copy_stream);
     }
     if (e == cudaSuccess) e = cudaEventRecord(s->staged[k], s->copy_stream);
-    // compute stream: staging -> arena (device copy), schedule, outputs to the host
+    // compute stream: the schedule on the staging set, or staging -> arena and the schedule; outputs to the host
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s->stream, s->staged[k], 0);
-    for (size_t i = 0; i < ni && e == cudaSuccess; ++i)
-      e = cudaMemcpyAsync(s->ptr(s->inputs[i]), s->staging[k][i], s->values[s->inputs[i]].bytes(),
-                          cudaMemcpyDeviceToDevice, s->stream);
-    if (e == cudaSuccess) e = cudaEventRecord(s->consumed[k], s->stream);
-    if (e == cudaSuccess) e = s->graph_exec ? cudaGraphLaunch(s->graph_exec, s->stream) : replay(s, s->stream);
+    if (!s->segments.empty()) {
+      if (e == cudaSuccess) e = launch_bound(s, s->staging[k].data(), nullptr);
+      if (e == cudaSuccess) e = cudaEventRecord(s->consumed[k], s->stream);
+    } else {
+      for (size_t i = 0; i < ni && e == cudaSuccess; ++i)
+        e = cudaMemcpyAsync(s->ptr(s->inputs[i]), s->staging[k][i], s->values[s->inputs[i]].bytes(),
+                            cudaMemcpyDeviceToDevice, s->stream);
+      if (e == cudaSuccess) e = cudaEventRecord(s->consumed[k], s->stream);
+      if (e == cudaSuccess) e = launch_all(s);
+    }
     for (size_t i = 0; i < no && e == cudaSuccess; ++i) {
       void* dst = outs[(size_t)b * no + i];
       e = cudaMemcpyAsync(dst, s->ptr(s->outputs[i]), s->values[s->outputs[i]].bytes(), cudaMemcpyDeviceToHost, s->stream);
     }
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(s->err_host, s->err_word, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) {
     // Whatever was enqueued before the failure finishes before the caller gets its buffers back.
@@ -531,22 +688,26 @@ int altius_cuda_time_device_runs(AcSession* s, const void* const* d_ins, void* c
     if (rc != AC_OK) s->err = s->fallback->err;
     return rc;
   }
-  cudaError_t e = cudaSetDevice(s->device);
+  cudaError_t e = use_device(s->device);
+  const bool bound = can_bind(s, d_ins, d_outs);
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   if (e == cudaSuccess) e = cudaEventCreate(&t0);
   if (e == cudaSuccess) e = cudaEventCreate(&t1);
   if (e == cudaSuccess) e = cudaEventRecord(t0, s->stream);
   for (int it = 0; it < iters && e == cudaSuccess; ++it) {
+    if (bound) {
+      e = launch_bound(s, d_ins, d_outs);
+      continue;
+    }
     for (size_t i = 0; i < s->inputs.size() && e == cudaSuccess; ++i)
       e = cudaMemcpyAsync(s->ptr(s->inputs[i]), d_ins[i], s->values[s->inputs[i]].bytes(),
                           cudaMemcpyDeviceToDevice, s->stream);
-    if (e == cudaSuccess) e = s->graph_exec ? cudaGraphLaunch(s->graph_exec, s->stream) : replay(s, s->stream);
+    if (e == cudaSuccess) e = launch_all(s);
     for (size_t i = 0; i < s->outputs.size() && e == cudaSuccess; ++i)
       e = cudaMemcpyAsync(d_outs[i], s->ptr(s->outputs[i]), s->values[s->outputs[i]].bytes(),
                           cudaMemcpyDeviceToDevice, s->stream);
   }
   if (e == cudaSuccess) e = cudaEventRecord(t1, s->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(s->err_host, s->err_word, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   if (e == cudaSuccess && *s->err_host != 0) {
     if (t0) cudaEventDestroy(t0);
@@ -644,7 +805,10 @@ void altius_cuda_destroy(AcSession* s) {
   if (s->graph) cudaGraphDestroy(s->graph);
   for (cudaEvent_t ev : s->events)
     if (ev) cudaEventDestroy(ev);
-  if (s->err_word) cudaFree(s->err_word);
+  for (ac::Segment& g : s->segments) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    if (g.graph) cudaGraphDestroy(g.graph);
+  }
   if (s->sweep_buf) cudaFree(s->sweep_buf);
   for (int k = 0; k < 2; ++k) {
     for (void* p : s->staging[k])
@@ -653,7 +817,7 @@ void altius_cuda_destroy(AcSession* s) {
     if (s->consumed[k]) cudaEventDestroy(s->consumed[k]);
   }
   if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
-  if (s->err_host) cudaFreeHost(s->err_host);
+  if (s->host_block) cudaFreeHost(s->host_block);
   if (s->arena) cudaFree(s->arena);
   if (s->weights) cudaFree(s->weights);
   if (s->stream) cudaStreamDestroy(s->stream);

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/altius_session_cuda.h"
+#include "host_stage.h"
 #include "kernels.h"
 
 namespace ac {
@@ -51,6 +52,7 @@ struct Storage {
   bool weight = false;   // lives in the weight blob, not the arena
   bool pinned_live = false;  // graph input/output or constant: live for the whole run
   size_t offset = 0;     // byte offset inside its region
+  void* bound = nullptr; // set while steps are enqueued on a caller's device buffer in place of the arena slot
 };
 
 struct Step {
@@ -61,6 +63,14 @@ struct Step {
   double bytes = 0, flops = 0;     // algorithmic work
   int launches = 1;
   bool const_only = false;         // all inputs constant: executed once at create()
+};
+
+// Consecutive steps of the schedule for runs on bound buffers: those that touch a graph input or
+// output are launched one by one on the caller's pointers, the others replay a graph.
+struct Segment {
+  int first = 0, last = 0;         // steps [first, last)
+  cudaGraph_t graph = nullptr;     // null: launched one by one
+  cudaGraphExec_t exec = nullptr;
 };
 
 struct ProfileAcc {
@@ -105,8 +115,16 @@ struct AcSession {
   size_t arena_bytes = 0;
   char* weights = nullptr;
   size_t weight_bytes = 0;
-  int* err_word = nullptr;             // device word written by kernels whose bounded waits expire
-  int* err_host = nullptr;             // page-locked mirror
+  // One page-locked, device-mapped block: the error word (written by kernels whose bounded waits expire
+  // or whose operands leave their range, read by the host after a run without a copy), then
+  // staging for small inputs and outputs of host runs (0 bytes where they are large).
+  char* host_block = nullptr;
+  int* err_word = nullptr;             // its device address
+  volatile int* err_host = nullptr;
+  char* stage_in = nullptr;
+  char* stage_out = nullptr;
+  std::shared_ptr<ac::HostStage> host_stage;   // uploads of large pageable inputs, from the first one on
+  std::vector<ac::Segment> segments;   // empty: this schedule does not run on bound buffers
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
@@ -132,6 +150,7 @@ struct AcSession {
 
   void* ptr(int value) const {
     const ac::Storage& st = storages[values[value].storage];
+    if (st.bound) return st.bound;
     return (st.weight ? weights : arena) + st.offset;
   }
   const float* fptr(int value) const { return static_cast<const float*>(ptr(value)); }
