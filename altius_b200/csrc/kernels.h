@@ -327,5 +327,9 @@ bool attention_tc16_shape_ok(int head_dim, int tokens, int64_t ld16, int64_t q_c
                              int64_t out_row_stride, int64_t out_batch_stride);
 bool attention_tc16_supported(const Attention16Params& p);
 cudaError_t launch_attention_tc16(const Attention16Params& p, cudaStream_t st);
+// The same operands and result for any number of tokens: keys in blocks with a running maximum.
+bool attention_flash16_shape_ok(int head_dim, int tokens, int64_t ld16, int64_t q_col, int64_t k_col, int64_t v_col,
+                                int64_t out_row_stride, int64_t out_batch_stride);
+cudaError_t launch_attention_flash16(const Attention16Params& p, cudaStream_t st);
 
 }  // namespace ac

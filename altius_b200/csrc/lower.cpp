@@ -201,6 +201,19 @@ bool trace_head_view(Ctx& c, int v, HeadView* out, std::vector<int>* nodes) {
   return true;
 }
 
+int effective_pairs(const AcSession& s) {
+  // AcOptions.gemm_pairs: 0 (default) and 2 -> CTA pairs with A pre-split for TMA where the
+  // cost model prefers them, 1 -> pairs that stage A through registers, 3 -> no pairs.
+  return s.opt.gemm_pairs == 0 ? 2 : (s.opt.gemm_pairs == 3 ? 0 : s.opt.gemm_pairs);
+}
+
+bool flash_attention_applies(const AcSession& s, const AttentionFusion& f) {
+  return on_device(s) && s.opt.gemm_mode == 0 && effective_pairs(s) == 2 && !std::getenv("ALTIUS_CUDA_NO_ATTENTION_TMA") &&
+         f.q.src == f.k.src && f.q.src == f.v.src && !s.values[f.q.src].is_const && s.values[f.q.src].elem_ty == AC_F32 &&
+         attention_flash16_shape_ok((int)f.q.hd, (int)f.q.T, f.q.C, f.q.col, f.k.col, f.v.col, f.q.H * f.q.hd,
+                                    f.q.T * f.q.H * f.q.hd);
+}
+
 // MatMul(q, Transpose(k)) -> [Mul|Div scalar] -> Softmax -> MatMul(., v) -> Reshape ->
 // Transpose[0,2,1,3] -> Reshape, with q, k, v head views of [B,T,C] tensors.
 void detect_attention(Ctx& c, Plan& plan) {
@@ -251,7 +264,9 @@ void detect_attention(Ctx& c, Plan& plan) {
     if (f.q.B != f.k.B || f.q.B != f.v.B || f.q.H != f.k.H || f.q.H != f.v.H || f.q.T != f.k.T ||
         f.q.T != f.v.T || f.q.hd != f.k.hd || f.q.hd != f.v.hd || f.q.C != f.k.C || f.q.C != f.v.C)
       continue;
-    if (f.q.hd != 64 || f.q.T > 256 || f.q.B * f.q.H > 65535 || (f.q.C % 4) || (f.q.col % 4) ||
+    // Beyond 256 tokens only the kernel that takes keys in blocks, from the fp16 halves of one projection.
+    if (f.q.T > 256 && !flash_attention_applies(c.s, f)) continue;
+    if (f.q.hd != 64 || f.q.B * f.q.H > 65535 || (f.q.C % 4) || (f.q.col % 4) ||
         (f.k.col % 4) || (f.v.col % 4))
       continue;
     // O [BH,T,hd] -> Reshape [B,H,T,hd] -> Transpose [0,2,1,3] -> Reshape [B,T,D]
@@ -744,12 +759,6 @@ int new_value(Ctx& c, int64_t numel, bool is_const) {
   return (int)c.s.values.size() - 1;
 }
 
-int effective_pairs(const AcSession& s) {
-  // AcOptions.gemm_pairs: 0 (default) and 2 -> CTA pairs with A pre-split for TMA where the
-  // cost model prefers them, 1 -> pairs that stage A through registers, 3 -> no pairs.
-  return s.opt.gemm_pairs == 0 ? 2 : (s.opt.gemm_pairs == 3 ? 0 : s.opt.gemm_pairs);
-}
-
 // Products of a few rows run in fp32 on the kernel that streams B (classifier heads at small batches).
 bool gemm_rows_applies(const AcSession& s, const GemmShape& g, bool b_const, int64_t a_off, int64_t b_off) {
   return on_device(s) && fp32_level_mode(s) && g.batch == 1 && !g.ta && g.m <= kGemmRowsMax && g.k >= 4 && (g.k % 4) == 0 &&
@@ -819,7 +828,7 @@ void plan_presplit(Ctx& c, Plan& plan) {
       const int src = f.q.src;
       if (src != f.k.src || src != f.v.src || split_users.count(src) || c.val(src).is_const) continue;
       if (!attention_tc16_shape_ok((int)f.q.hd, (int)f.q.T, f.q.C, f.q.col, f.k.col, f.v.col, f.q.H * f.q.hd,
-                                   f.q.T * f.q.H * f.q.hd))
+                                   f.q.T * f.q.H * f.q.hd) && !flash_attention_applies(c.s, f))
         continue;
       split_users[src] = 1;
     }
@@ -1472,11 +1481,29 @@ void lower_node(Emit& em, Plan& plan, int nid) {
         const double flops = 4.0 * B * H * T * T * hd;
         // gemm_mode 1 asks for exact fp32 FMA chains: it keeps the CUDA-core kernel.
         const bool tc_attn = s->opt.gemm_mode != 1 && hd == 64 && T > 64 && T <= 256;
+        // The projection as halves on the fixed scale: written by its GEMM, else (only where no other
+        // kernel takes this many tokens) by a split kernel.
+        auto si = c.split.find(f.q.src);
+        bool halves = si != c.split.end() && f.q.src == f.k.src && f.q.src == f.v.src;
+        const bool flash_ok = halves && flash_attention_applies(*s, f);
+        if (halves && !si->second.produced) {
+          halves = flash_ok && T > 256;
+          if (halves) {
+            const int src = f.q.src, hi = si->second.hi, lo = si->second.lo;
+            em.add("act_f16_split", n.op, {src}, {hi, lo}, 8.0 * B * T * C, 0, [=](cudaStream_t st) {
+              return launch_f16_split(s->fptr(src), s->fptr_mut(hi), s->fptr_mut(lo), B * T, C, C, C, s->err_word, nullptr, nullptr, 1, st);
+            });
+            si->second.produced = true;
+          }
+        }
+        const bool tc16 = halves && tc_attn &&
+                          attention_tc16_shape_ok((int)hd, (int)T, C, f.q.col, f.k.col, f.v.col, H * hd, T * H * hd);
+        const bool flash = halves && flash_ok && !tc16;
         int o16_hi = -1, o16_lo = -1;
         bool o_fp32 = true;
         {
           auto so = c.split.find(f.out);
-          if (so != c.split.end() && !so->second.produced && tc_attn) {
+          if (so != c.split.end() && !so->second.produced && (tc_attn || flash)) {
             o16_hi = so->second.hi; o16_lo = so->second.lo;
             o_fp32 = so->second.fp32_needed;
             so->second.produced = true;
@@ -1485,12 +1512,10 @@ void lower_node(Emit& em, Plan& plan, int nid) {
         std::vector<int> awrites;
         if (o_fp32) awrites.push_back(f.out);
         if (o16_hi >= 0) { awrites.push_back(o16_hi); awrites.push_back(o16_lo); }
-        // The projection was written on the fixed scale by its GEMM: the TMA-fed kernel.
-        auto si = c.split.find(f.q.src);
-        if (tc_attn && si != c.split.end() && si->second.produced && f.q.src == f.k.src && f.q.src == f.v.src &&
-            attention_tc16_shape_ok((int)hd, (int)T, C, f.q.col, f.k.col, f.v.col, H * hd, T * H * hd)) {
+        if (tc16 || flash) {
           const int in_hi = si->second.hi, in_lo = si->second.lo;
-          em.add("attention_tma_tcgen05", n.op, {in_hi, in_lo, f.scale}, awrites, bytes, flops, [=](cudaStream_t st) {
+          em.add(tc16 ? "attention_tma_tcgen05" : "attention_flash_tcgen05", n.op, {in_hi, in_lo, f.scale}, awrites, bytes, flops,
+                 [=](cudaStream_t st) {
             Attention16Params p{};
             p.qkv16_hi = s->ptr(in_hi); p.qkv16_lo = s->ptr(in_lo);
             p.ld16 = C; p.q_col = f.q.col; p.k_col = f.k.col; p.v_col = f.v.col;
@@ -1500,7 +1525,7 @@ void lower_node(Emit& em, Plan& plan, int nid) {
             p.batch = (int)B; p.heads = (int)H; p.tokens = (int)T; p.head_dim = (int)hd;
             p.scale = f.scale >= 0 ? s->fptr(f.scale) : nullptr; p.scale_mode = f.scale_mode;
             p.err_word = s->err_word;
-            return launch_attention_tc16(p, st);
+            return tc16 ? launch_attention_tc16(p, st) : launch_attention_flash16(p, st);
           });
           return;
         }
