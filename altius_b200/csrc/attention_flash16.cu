@@ -174,7 +174,14 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
           }
         }
         idle = did ? 0 : idle + 1;
-        if (idle > kPollLimit) { atomicExch(p.err, 51); break; }
+        if (idle > kPollLimit) {
+          atomicExch(p.err, 51);
+          for (int g = 0; g < 2; ++g) {         // copies in flight land
+            if (kn[g] > 0) (void)mbar_wait(&bar.k_full[g], (uint32_t)((kn[g] - 1) & 1));
+            if (vn[g] > 0) (void)mbar_wait(&bar.v_full[g], (uint32_t)((vn[g] - 1) & 1));
+          }
+          break;
+        }
       }
     }
   } else if (warp == kMmaWarp) {

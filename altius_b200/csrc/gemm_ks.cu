@@ -1,0 +1,291 @@
+// fp16-split GEMM for few rows (a small batch of a transformer): C = epilogue(A * B^T) with both operands
+// as fp16 halves by TMA (A on the fixed scale, written by the kernel in front; B prepared once), three
+// kind::f16 MMAs per product into one accumulator -- the operand formats of the CTA-pair kernel
+// (gemm_tc.cu), which takes the larger problems.
+//
+// What bounds it: 197 rows against 768 x 2304 are 2.1 GFLOP and 7 MB of weights, 1.2 us of either, so what
+// counts is latency. On 256 x 256 tiles such a product has 9 tiles for 74 pairs; cut along K its
+// partial sums went through memory to a second kernel, 20 us in all. Here a cluster of S blocks
+// shares one 128 x BN tile: each takes a range of K (two to eight K-blocks), and the accumulators
+// meet in distributed shared memory: every block sends each peer that peer's columns of its
+// accumulator, and after one cluster barrier finishes its own BN / S columns (sum in rank order, so
+// the result does not depend on timing; bias, activation, residual; whole-line stores). The weights
+// of the first stages are requested while the kernel in front still runs.
+//
+// Per block: warps 0-7 move the accumulator and run the epilogue, warp 8 issues TMA, warp 9 MMAs.
+#include <cooperative_groups.h>
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "kernels.h"
+#include "pdl.cuh"
+#include "ref_math.cuh"
+#include "tc_common.cuh"
+#include "tensor_map.h"
+
+namespace cg = cooperative_groups;
+
+namespace ac {
+namespace {
+
+using namespace tc;
+
+constexpr int BM = 128, KB = 64, kEpiThreads = 256, kTmaWarp = 8, kMmaWarp = 9, kThreads = 320, kMaxStages = 4;
+constexpr int kAHalf = BM * KB * 2;           // bytes of A's hi (or lo) tile
+
+struct KsDev {
+  int m, n, k;
+  int bn, stages, kper;                       // columns of a tile, ring entries, K-blocks per block of the cluster
+  int pitch;                                  // float4s per row of the exchange buffer (odd: no bank conflicts)
+  float* c; long long ldc;                    // may be null when c16_hi / c16_lo are given
+  uint2* c16_hi; uint2* c16_lo; long long ldc16;
+  const float* bias; const float* res; long long ldres;
+  const float* acc_scale;                     // device scalar or null
+  int* err;
+};
+
+__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
+         (uint64_t)2 << 61;
+}
+
+template <int ACT>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
+               const __grid_constant__ CUtensorMap tb_hi, const __grid_constant__ CUtensorMap tb_lo, const KsDev p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full;
+  __shared__ uint32_t tmem_slot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int bn = p.bn, S = p.stages, parts = gridDim.z, share = bn / parts, rank = blockIdx.z;
+  const int bhalf = bn * KB * 2, stage_bytes = 2 * kAHalf + 2 * bhalf;
+  float4* part = reinterpret_cast<float4*>(smem + S * stage_bytes);   // [parts][BM][pitch]
+  const int nkb = (p.k + KB - 1) / KB, kb0 = rank * p.kper, kbs = min(nkb, kb0 + p.kper) - kb0;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * bn;
+  const uint32_t cols = bn <= 32 ? 32 : bn <= 64 ? 64 : 128;
+  cg::cluster_group cl = cg::this_cluster();
+  if (parts > 1) cl.barrier_arrive();         // answered before the first write to another block's memory
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    mbar_init(&acc_full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(cols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  pdl_trigger();
+
+  auto load_b = [&](int it) {
+    uint8_t* b = smem + (it % S) * stage_bytes + 2 * kAHalf;
+    mbar_arrive_expect_tx(&full[it % S], (uint32_t)stage_bytes);
+    tma_load_3d(b, &tb_hi, &full[it % S], (kb0 + it) * KB, n0, 0);
+    tma_load_3d(b + bhalf, &tb_lo, &full[it % S], (kb0 + it) * KB, n0, 0);
+  };
+  auto load_a = [&](int it) {
+    uint8_t* a = smem + (it % S) * stage_bytes;
+    tma_load_3d(a, &ta_hi, &full[it % S], (kb0 + it) * KB, m0, 0);
+    tma_load_3d(a + kAHalf, &ta_lo, &full[it % S], (kb0 + it) * KB, m0, 0);
+  };
+  if (warp == kTmaWarp && lane == 0)
+    for (int it = 0; it < S && it < kbs; ++it) load_b(it);   // constants: ahead of pdl_wait
+  pdl_wait();
+  if (parts > 1) cl.barrier_wait();           // every block of the cluster runs
+
+  unsigned seen = 0;
+  if (warp == kTmaWarp) {
+    if (lane == 0) {
+      for (int it = 0; it < kbs; ++it) {
+        if (it >= S) {
+          if (!mbar_wait(&empty[it % S], (uint32_t)((it / S) & 1) ^ 1)) {
+            atomicExch(p.err, 61);
+            for (int s = 0; s < S; ++s) (void)mbar_wait(&full[s], (uint32_t)((it - 1) / S) & 1);   // copies in flight land
+            break;
+          }
+          load_b(it);
+        }
+        load_a(it);
+      }
+    }
+  } else if (warp == kMmaWarp) {
+    if (lane == 0) {
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      for (int it = 0; it < kbs; ++it) {
+        const int s = it % S;
+        if (!mbar_wait(&full[s], (uint32_t)(it / S) & 1)) { atomicExch(p.err, 62); break; }
+        tc_fence_after();
+        const uint32_t a = smem_u32(smem + s * stage_bytes);
+        const uint64_t da = desc_sw128(a), dal = desc_sw128(a + kAHalf);
+        const uint64_t db = desc_sw128(a + 2 * kAHalf), dbl = desc_sw128(a + 2 * kAHalf + bhalf);
+        const int steps = min(4, (p.k - (kb0 + it) * KB + 15) / 16);
+        for (int kk = 0; kk < steps; ++kk) {
+          const uint64_t off = (uint64_t)(kk * 32 >> 4);
+          tc_mma_f16(tmem, dal + off, db + off, idesc, (it > 0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
+          tc_mma_f16(tmem, da + off, dbl + off, idesc, 1u);                             // a_hi * b_lo
+          tc_mma_f16(tmem, da + off, db + off, idesc, 1u);                              // a_hi * b_hi
+        }
+        tc_commit(&empty[s]);
+      }
+      tc_commit(&acc_full);
+    }
+  } else {
+    if (!mbar_wait(&acc_full, 0)) atomicExch(p.err, 63);
+    tc_fence_after();
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    for (int c = (warp >> 2) * 16; c < bn; c += 32) {
+      uint32_t u[16];
+      tc_ld_32x16_nowait(base + (uint32_t)c, u);
+      tc_wait_ld();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int col = c + 4 * i, owner = col / share;
+        float4* dst = parts > 1 ? cl.map_shared_rank(part, owner) : part;
+        dst[(rank * BM + row) * p.pitch + (col - owner * share) / 4] =
+            make_float4(__uint_as_float(u[4 * i]), __uint_as_float(u[4 * i + 1]), __uint_as_float(u[4 * i + 2]),
+                        __uint_as_float(u[4 * i + 3]));
+      }
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  if (parts > 1) cl.sync();
+  else __syncthreads();
+
+  // ---- this block's columns of the tile ----
+  if (warp < 8) {
+    const float sc = p.acc_scale ? __fmul_rn(__ldg(p.acc_scale), kFixedUnscale) : kFixedUnscale;
+    const int quads = share / 4, total = BM * quads;
+    float most = 0.f;
+#pragma unroll 2
+    for (int e = tid; e < total; e += kEpiThreads) {
+      const int row = e / quads, q = e - row * quads;
+      const int r = m0 + row, col = n0 + rank * share + 4 * q;
+      if (r >= p.m || col >= p.n) continue;   // n % 4 == 0: the four columns exist together
+      float4 rs = make_float4(0.f, 0.f, 0.f, 0.f), b = rs;
+      if (p.res) rs = *reinterpret_cast<const float4*>(p.res + (long long)r * p.ldres + col);
+      if (p.bias) b = __ldg(reinterpret_cast<const float4*>(p.bias + col));
+      float4 x = part[row * p.pitch + q];
+      for (int s = 1; s < parts; ++s) {
+        const float4 u = part[(s * BM + row) * p.pitch + q];
+        x.x = __fadd_rn(x.x, u.x); x.y = __fadd_rn(x.y, u.y); x.z = __fadd_rn(x.z, u.z); x.w = __fadd_rn(x.w, u.w);
+      }
+      x.x = __fmul_rn(x.x, sc); x.y = __fmul_rn(x.y, sc); x.z = __fmul_rn(x.z, sc); x.w = __fmul_rn(x.w, sc);
+      if (p.bias) { x.x = __fadd_rn(x.x, b.x); x.y = __fadd_rn(x.y, b.y); x.z = __fadd_rn(x.z, b.z); x.w = __fadd_rn(x.w, b.w); }
+      if (ACT == ACT_GELU) {
+        const float2 lo = gelu_ref2(make_float2(x.x, x.y)), hi = gelu_ref2(make_float2(x.z, x.w));
+        x = make_float4(lo.x, lo.y, hi.x, hi.y);
+      } else if (ACT == ACT_RELU) {
+        x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f);
+      }
+      if (p.res) { x.x = __fadd_rn(x.x, rs.x); x.y = __fadd_rn(x.y, rs.y); x.z = __fadd_rn(x.z, rs.z); x.w = __fadd_rn(x.w, rs.w); }
+      if (p.c) *reinterpret_cast<float4*>(p.c + (long long)r * p.ldc + col) = x;
+      if (p.c16_hi) {
+        uint2 h, l;
+        f16_split_fixed(x, h, l);
+        const long long at = ((long long)r * p.ldc16 + col) >> 2;
+        p.c16_hi[at] = h;
+        p.c16_lo[at] = l;
+        most = split_track(most, x);
+      }
+    }
+    if (p.c16_hi) seen = split_seen_fixed_of_max(most);
+  }
+  // Out of range, or nothing but tiny values in this block's 128 x share results.
+  const int over = __syncthreads_or((int)(seen & 1u)), fine = __syncthreads_or((int)(seen & 2u)), tiny = __syncthreads_or((int)(seen & 4u));
+  if (tid == 0 && (over || (tiny && !fine))) atomicCAS(p.err, 0, kRangeCode);
+  if (warp == kMmaWarp) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
+  }
+}
+
+constexpr size_t kSmemMax = 231000;
+
+struct Shape {
+  int bn = 0, split = 0, kper = 0, stages = 0, pitch = 0;
+  size_t smem = 0;
+  double clocks = 1e30;
+};
+
+// Tile width and K split by clocks: a K-block costs its twelve MMAs (about 110 clocks each up to 128
+// columns) or its bytes at 28 a clock, whichever is more; start, first loads, exchange and epilogue
+// about 5000 (and 250 per block of a cluster).
+Shape pick_shape(int64_t m, int64_t n, int64_t k, int sms) {
+  Shape best;
+  const int nkb = (int)((k + KB - 1) / KB);
+  const long long mt = (m + BM - 1) / BM;
+  for (int bn : {32, 64, 96, 128}) {
+    for (int split : {1, 2, 4, 8}) {
+      const int kper = (nkb + split - 1) / split;
+      if ((split - 1) * kper >= nkb || (bn % (4 * split)) != 0) continue;
+      const int quads = bn / split / 4, pitch = quads | 1;
+      const size_t stage = 2 * (size_t)kAHalf + (size_t)bn * KB * 4, ex = (size_t)split * BM * pitch * 16;
+      const int stages = (int)std::min<size_t>(std::min(kper, kMaxStages), (kSmemMax - 1024 - ex) / stage);
+      if (stages < std::min(2, kper)) continue;
+      const double ctas = (double)mt * ((n + bn - 1) / bn) * split, waves = std::ceil(ctas / sms);
+      const double kb = std::max(12 * 110.0, (double)stage / 28.0);
+      const double t = waves * (kper * kb + 5000.0 + 250.0 * split + 10.0 * bn);
+      if (t < best.clocks) {
+        best.bn = bn; best.split = split; best.kper = kper; best.stages = stages; best.pitch = pitch;
+        best.smem = stages * stage + ex + 1024;
+        best.clocks = t;
+      }
+    }
+  }
+  return best;
+}
+
+template <int ACT>
+cudaError_t launch_act(const CUtensorMap& ah, const CUtensorMap& al, const CUtensorMap& bh, const CUtensorMap& bl,
+                       const KsDev& d, const Shape& sh, cudaStream_t st) {
+  static unsigned long long done = 0;
+  if (cudaError_t e = ensure_dynamic_smem(gemm_ks_kernel<ACT>, (int)kSmemMax, &done)) return e;
+  const dim3 grid((unsigned)((d.n + sh.bn - 1) / sh.bn), (unsigned)((d.m + BM - 1) / BM), (unsigned)sh.split);
+  return launch_pdl(gemm_ks_kernel<ACT>, grid, dim3(kThreads), sh.smem, st, sh.split, ah, al, bh, bl, d);
+}
+
+inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
+
+}  // namespace
+
+double gemm_ks_clocks(int64_t m, int64_t n, int64_t k) {
+  if (m < 1 || n < 4 || (n % 4) || k < 64 || (k % 8) || m > (1 << 20) || n > (1 << 20)) return 1e30;
+  return pick_shape(m, n, k, device_sm_count()).clocks;
+}
+
+bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bias_scale) {
+  return (act == ACT_NONE || act == ACT_GELU || act == ACT_RELU) && !bias_m && !c_in && alpha == 1.f && bias_scale == 1.f;
+}
+
+cudaError_t launch_gemm_ks(const GemmParams& q, int* err_word, cudaStream_t st) {
+  if (!q.a16_hi || !q.a16_lo || !q.b16_hi || !q.b16_lo || !q.a16_fixed || !q.b16_plain || q.batch != 1 || (q.n % 4) ||
+      (q.k % 8) || (q.lda16 % 8) || (q.ldb16 % 8) || !al16(q.a16_hi) || !al16(q.a16_lo) || !al16(q.b16_hi) || !al16(q.b16_lo) ||
+      (q.c && (!al16(q.c) || (q.ldc % 4))) || (q.residual && (!al16(q.residual) || (q.ld_res % 4))) || (q.bias_n && !al16(q.bias_n)) ||
+      (q.c16_hi && (q.ldc16 % 4)) || !gemm_ks_epilogue_ok(q.act, q.bias_m != nullptr, q.beta != 0.f && q.c_in, q.alpha, q.bias_scale))
+    return cudaErrorInvalidValue;
+  const Shape sh = pick_shape(q.m, q.n, q.k, device_sm_count());
+  KsDev d{};
+  d.m = (int)q.m; d.n = (int)q.n; d.k = (int)q.k;
+  d.bn = sh.bn; d.stages = sh.stages; d.kper = sh.kper; d.pitch = sh.pitch;
+  d.c = q.c; d.ldc = q.ldc;
+  d.c16_hi = static_cast<uint2*>(q.c16_hi); d.c16_lo = static_cast<uint2*>(q.c16_lo); d.ldc16 = q.ldc16;
+  d.bias = q.bias_n; d.res = q.residual; d.ldres = q.ld_res;
+  d.acc_scale = q.b16_inv_scale;
+  d.err = err_word;
+  CUtensorMap ah, al, bh, bl;
+  if (!make_map16(&ah, q.a16_hi, q.k, q.m, 1, q.lda16, q.m * q.lda16, BM) || !make_map16(&al, q.a16_lo, q.k, q.m, 1, q.lda16, q.m * q.lda16, BM) ||
+      !make_map16(&bh, q.b16_hi, q.k, q.n, 1, q.ldb16, q.n * q.ldb16, sh.bn) || !make_map16(&bl, q.b16_lo, q.k, q.n, 1, q.ldb16, q.n * q.ldb16, sh.bn))
+    return cudaErrorInvalidValue;
+  if (q.act == ACT_GELU) return launch_act<ACT_GELU>(ah, al, bh, bl, d, sh, st);
+  if (q.act == ACT_RELU) return launch_act<ACT_RELU>(ah, al, bh, bl, d, sh, st);
+  return launch_act<ACT_NONE>(ah, al, bh, bl, d, sh, st);
+}
+
+}  // namespace ac

@@ -1708,6 +1708,17 @@ bool gemm_tc_wants_presplit(int64_t m, int64_t n, int64_t k, int64_t batch) {
   return pick_shape(m, n, k, batch, 2, 2).pair;
 }
 
+// A K-block of a 256 x 256 tile takes 1950 clocks, launch, first operands and last epilogue 20000, the
+// K-slice pass behind it 9000 (ViT-B/16's four GEMMs at 1 to 96 images, within 15 %).
+double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k) {
+  const int pairs = pair_count();
+  if (pairs <= 0) return 1e30;
+  const TcPlan pl = make_plan(m, n, k, 1, 256, 2, 64, pairs);
+  double blocks = (double)((pl.sc.dp_tiles + pairs - 1) / pairs) * pl.sc.num_kb;
+  if (pl.sc.tail_parts >= 2) blocks += (double)pl.sc.num_kb / pl.sc.tail_parts;
+  return blocks * 1950.0 + 20000.0 + (pl.sc.tail_parts >= 2 ? 9000.0 : 0.0);
+}
+
 size_t gemm_tc_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, int allow_pairs) {
   const TcShape sh = pick_shape(m, n, k, batch, variant, allow_pairs);
   const int kbf = sh.pair && allow_pairs == 2 ? 64 : (variant == 2 ? BK16 : BK);   // pre-split A: K-blocks of 64 halves

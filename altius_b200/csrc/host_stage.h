@@ -1,7 +1,7 @@
 // Uploads of large pageable host buffers. cudaMemcpyAsync from pageable memory copies through the
 // driver's own page-locked buffer on the calling thread: 16-19 GB/s on the host measured, a third of
 // the link (19 MB: 1080 us, against 359 us from page-locked memory). Here a few threads copy chunks
-// into a page-locked ring (45 GB/s with four, 95 with eight) while the chunks in front are on the
+// into a page-locked ring (past the caches, see the copy) while the chunks in front are on the
 // link, so the upload runs at the link's rate after the first chunk.
 //
 // One stage per device, shared by the sessions that need it and freed with the last of them; one
@@ -28,8 +28,8 @@ class HostStage {
   cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st);
 
  private:
-  static constexpr size_t kChunk = size_t(512) << 10;
-  static constexpr int kSlots = 16;
+  static constexpr size_t kChunk = size_t(1) << 20;
+  static constexpr int kSlots = 12;
   HostStage() = default;
   bool init();
   void worker();

@@ -272,6 +272,13 @@ size_t gemm_tc_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t batch, i
 // (a16_hi / a16_lo): the producer of A, or a split kernel in front, then writes the halves.
 bool gemm_tc_wants_presplit(int64_t m, int64_t n, int64_t k, int64_t batch);
 constexpr int kGemmRangeCode = 21;
+// Clocks of the pre-split GEMM of this shape on CTA pairs (its K-slice pass included), by the same plan the
+// launch uses; and of the kernel for few rows (gemm_ks.cu: clusters that share a tile along K; 1e30
+// where it does not apply), which takes the operands of the pair kernel.
+double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k);
+double gemm_ks_clocks(int64_t m, int64_t n, int64_t k);
+bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bias_scale);
+cudaError_t launch_gemm_ks(const GemmParams& p, int* err_word, cudaStream_t st);
 // fp16 split of a constant [rows, k] operand (row stride ld) into [rows, k8] halves
 // (k8 >= k, a multiple of 8, padding zero); leaves kGemmRangeCode in *err_word when an
 // element exceeds the fp16 range.

@@ -35,7 +35,7 @@ struct Ctx {
   // that computes the value, or a split kernel); `fp32_needed`: someone still reads the value
   // itself, so its producer writes it as well.
   // The halves are on the fixed scale (f16_split_fixed): X = x * 2^8, hi = rn(X), lo = rn(X - hi).
-  struct Split { int hi = -1, lo = -1; bool produced = false, fp32_needed = true; };
+  struct Split { int hi = -1, lo = -1; bool produced = false, fp32_needed = true, by_producer = false; };
   std::map<int, Split> split;
   explicit Ctx(AcSession& s_) : s(s_) {}
 
@@ -780,6 +780,17 @@ bool presplit_applies(const AcSession& s, const GemmShape& g, bool b_const, int6
   return gemm_tc_wants_presplit(g.m, g.n, g.k, g.batch);
 }
 
+// The same operands on the kernel for few rows, where it is the faster one (only for an A whose
+// producer writes the halves: a split kernel in front would cost what it saves).
+bool gemm_ks_applies(const AcSession& s, const GemmShape& g, bool b_const, int64_t a_off, int64_t b_off) {
+  if (!on_device(s) || s.opt.gemm_mode != 0 || effective_pairs(s) != 2 || !b_const || g.batch != 1 || g.ta || a_off != 0 ||
+      b_off != 0 || g.lda != g.k || gemm_rows_applies(s, g, b_const, a_off, b_off))
+    return false;
+  if (g.tb ? (g.ldb % 4) != 0 : (g.k % 4) != 0) return false;
+  if (2.0 * g.m * g.n * g.k < double(1 << 20)) return false;
+  return gemm_ks_clocks(g.m, g.n, g.k) < gemm_tc_pair_clocks(g.m, g.n, g.k);
+}
+
 GemmShape matmul_shape(Ctx& c, const Node& n, bool trans_b_folded) {
   const Value& av = c.val(n.inputs[0]);
   const Value& ov = c.val(n.outputs[0]);
@@ -807,8 +818,15 @@ GemmShape matmul_shape(Ctx& c, const Node& n, bool trans_b_folded) {
 // presplit_applies to. Their scratch halves are created here.
 void plan_presplit(Ctx& c, Plan& plan) {
   std::map<int, int> split_users;   // value -> MatMul nodes that take it pre-split
+  std::set<int> writable;           // results whose producers can write the halves
+  for (auto& kv : plan.attention) writable.insert(kv.second.out);
   for (int nid : c.s.order) {
     const Node& n = c.node(nid);
+    if (n.op == AC_OP_LAYERNORMALIZATION && !c.absorbed[nid]) {
+      const Value& v = c.val(n.outputs[0]);
+      const int64_t len = v.dims[v.rank - 1];
+      if ((len % 8) == 0 && len <= 1024) writable.insert(n.outputs[0]);
+    }
     if (c.absorbed[nid] || n.op != AC_OP_MATMUL) continue;
     const int a = n.inputs[0];
     if (c.val(a).is_const || c.val(a).elem_ty != AC_F32 || c.val(a).rank < 2) continue;
@@ -816,8 +834,13 @@ void plan_presplit(Ctx& c, Plan& plan) {
     const bool folded_t = it != plan.epi.end() && it->second.trans_b_src >= 0;
     const int b = folded_t ? it->second.trans_b_src : n.inputs[1];
     const GemmShape g = matmul_shape(c, n, folded_t);
-    if (!presplit_applies(c.s, g, c.val(b).is_const, 0, 0)) continue;
+    const bool b_const = c.val(b).is_const;
+    const int act = it == plan.epi.end() ? (int)ACT_NONE : it->second.act;
+    if (!presplit_applies(c.s, g, b_const, 0, 0) &&
+        !(writable.count(a) && gemm_ks_applies(c.s, g, b_const, 0, 0) && gemm_ks_epilogue_ok(act, false, false, 1.f, 1.f)))
+      continue;
     split_users[a]++;
+    if ((g.n % 8) == 0) writable.insert(it == plan.epi.end() ? n.outputs[0] : it->second.out);
   }
   // The [B, T, 3D] projection in front of a fused attention core: its GEMM writes it on the fixed
   // scale and the TMA-fed attention kernel reads Q, K and V from there (the Split node between
@@ -840,6 +863,7 @@ void plan_presplit(Ctx& c, Plan& plan) {
     Ctx::Split sp;
     sp.hi = new_value(c, floats, false);
     sp.lo = new_value(c, floats, false);
+    sp.by_producer = writable.count(a) != 0;
     sp.fp32_needed = c.is_output[a] || (int)c.consumers[a].size() != kv.second;
     c.split[a] = sp;
   }
@@ -921,7 +945,10 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   int b16_hi = -1, b16_lo = -1, b16_scale = -1;
   int64_t ldb16 = 0;
   const bool b16_ok = tc && mode == 0 && em.c.val(b_use).is_const && g.tb && g.batch == 1 && b_off == 0;
-  const bool pre = b16_ok && presplit_applies(*s, g, true, a_off, b_off);
+  const auto sp_a = em.c.split.find(a);
+  const bool use_ks = b16_ok && sp_a != em.c.split.end() && sp_a->second.by_producer && b_row_scale < 0 && gemm_ks_applies(*s, g, true, a_off, b_off) &&
+                      gemm_ks_epilogue_ok(act, bias_m >= 0, c_in >= 0, alpha, bias_scale) && c_off == 0 && g.ldc == g.n;
+  const bool pre = b16_ok && (use_ks || presplit_applies(*s, g, true, a_off, b_off));
   if (b16_ok) {
     ldb16 = (g.k + 7) / 8 * 8;
     const int64_t floats = g.n * ldb16 / 2;     // two halves per float of scratch
@@ -991,7 +1018,7 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   {
     auto so = em.c.split.find(out);
     if (so != em.c.split.end() && !so->second.produced && a16_hi >= 0 && c_off == 0 && g.ldc == g.n && (g.n % 8) == 0 &&
-        gemm_tc_can_split_output(act, bias_n >= 0, bias_m >= 0, c_in >= 0, alpha, bias_scale)) {
+        (use_ks || gemm_tc_can_split_output(act, bias_n >= 0, bias_m >= 0, c_in >= 0, alpha, bias_scale))) {
       c16_hi = so->second.hi; c16_lo = so->second.lo;
       c_fp32 = so->second.fp32_needed;
       c16_fixed = true;
@@ -1001,7 +1028,7 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   // Scratch for the K-sliced tail tiles of the persistent kernel (lives for this step only).
   int ws = -1;
   size_t ws_bytes = 0;
-  if (tc) {
+  if (tc && !use_ks) {
     ws_bytes = gemm_tc_workspace_bytes(g.m, g.n, g.k, g.batch, b16_hi >= 0 ? 2 : (b_lo >= 0 ? 0 : 1), pairs);
     if (ws_bytes) ws = new_value(em.c, (int64_t)(ws_bytes / 4), false);
   }
@@ -1011,7 +1038,8 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
                             c_in, bias_n, bias_m, res, b_row_scale};
   const char* kind = !tc ? "gemm_fp32_simt"
                      : (mode == 2 ? "gemm_tf32x1_tcgen05"
-                                  : (b16_hi >= 0 ? (a16_hi >= 0 ? "gemm_f16x3_pair_tcgen05" : "gemm_f16x3_tcgen05")
+                                  : (b16_hi >= 0 ? (use_ks ? "gemm_f16x3_cluster_tcgen05"
+                                                    : a16_hi >= 0 ? "gemm_f16x3_pair_tcgen05" : "gemm_f16x3_tcgen05")
                                                  : "gemm_tf32x3_tcgen05"));
   std::vector<int> writes;
   if (c_fp32) writes.push_back(out);
@@ -1049,6 +1077,7 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
     p.bias_scale = bias_scale;
     p.act = act; p.act_alpha = aa; p.act_beta = ab;
     p.residual = res >= 0 ? s->fptr(res) + c_off : nullptr; p.ld_res = g.ldc; p.stride_res = g.sc;
+    if (use_ks) return launch_gemm_ks(p, s->err_word, st);
     if (tc && gemm_tc_supported(p)) return launch_gemm_tc(p, mode, s->err_word, st);
     if (!p.a || !p.c || p.c16_hi || p.b_row_scale) return cudaErrorInvalidValue;   // operands exist for the tensor-core kernel only
     // The CUDA-core kernel multiplies the operand as given, not a TF32-rounded copy of it.

@@ -123,3 +123,31 @@ def test_tensor_core_convolution(cuda_lib, n, c, h, oc, k, s, p, gate):
     want = torch.relu(conv(xg, torch.from_numpy(w).double(), torch.from_numpy(b).double())).numpy() + r
     mass = conv(xg.abs(), torch.from_numpy(w).double().abs(), torch.from_numpy(b).double().abs()).numpy() + np.abs(r)
     assert (np.abs(got - want) <= 1e-5 * np.abs(want) + 5e-6 * mass).all()
+
+
+# An MLP behind a LayerNormalization: both products on clusters that share a tile along K, the first one
+# writing the halves the second one takes. Rows off the tiles, K off the K-blocks, N off the tile widths.
+# fp16-split products: 1e-5 |want| + 5e-6 sum |a||b| each (as in the other tests of the format); the first
+# one's error reaches the second through |w2| (Gelu has slope at most 1.13).
+@pytest.mark.parametrize("m,d,hidden", [(33, 192, 768), (197, 768, 3072), (129, 200, 328), (128, 1024, 64), (700, 384, 1536)])
+def test_few_row_products_on_clusters(cuda_lib, m, d, hidden):
+    rng = np.random.default_rng(m + d)
+    x = rng.standard_normal((m, d)).astype(np.float32)
+    gam, bet = (1 + 0.1 * rng.standard_normal(d)).astype(np.float32), (0.1 * rng.standard_normal(d)).astype(np.float32)
+    w1 = (rng.standard_normal((d, hidden)) / np.sqrt(d)).astype(np.float32)
+    w2 = (rng.standard_normal((hidden, d)) / np.sqrt(hidden)).astype(np.float32)
+    b1, b2 = rng.standard_normal(hidden).astype(np.float32), rng.standard_normal(d).astype(np.float32)
+
+    def build(g, xi):
+        h = g.op("LayerNormalization", xi, g.new_init(gam), g.new_init(bet), axis=-1, epsilon=1e-6, stash_type=1)
+        h = g.op("Gelu", g.op("Add", g.op("MatMul", h, g.new_init(w1)), g.new_init(b1)))
+        return g.op("Add", xi, g.op("Add", g.op("MatMul", h, g.new_init(w2)), g.new_init(b2)))
+    got = _run(build, [x], ["layer_norm", "gemm_f16x3_cluster_tcgen05", "gemm_f16x3_cluster_tcgen05"])
+    t = lambda a: torch.from_numpy(a).double()
+    h = torch.nn.functional.layer_norm(t(x), (d,), t(gam), t(bet), 1e-6)
+    z = h @ t(w1) + t(b1)
+    e1 = 1e-5 * z.abs() + 5e-6 * (h.abs() @ t(w1).abs()) + 1e-5 * (h.abs() @ t(w1).abs())   # LayerNorm itself: 1e-5
+    a = torch.nn.functional.gelu(z, approximate="tanh")
+    want = t(x) + a @ t(w2) + t(b2)
+    bound = 1.13 * e1 @ t(w2).abs() + 1e-5 * want.abs() + 6e-6 * (a.abs() @ t(w2).abs())
+    assert (np.abs(got - want.numpy()) <= bound.numpy()).all()
