@@ -46,6 +46,7 @@ struct ConvDev {
   int act;
   float act_alpha, act_beta;
   int kper;                 // K steps per block of the cluster
+  int early;                // the filter is a constant: read ahead of pdl_wait
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(T) conv_simt_kernel(const ConvDev p) {
   }
   const float* gcol = p.gate ? p.gate + (long long)cb * p.k : nullptr;
 
-  auto load_w = [&](int s, int kt) {      // constants: may run ahead of pdl_wait
+  auto load_w = [&](int s, int kt) {
     float* As = smem + s * C::STAGE;
     const int k0 = kt * BK;
 #pragma unroll
@@ -204,6 +205,7 @@ __global__ void __launch_bounds__(T) conv_simt_kernel(const ConvDev p) {
     }
   };
 
+  if (!p.early) pdl_wait();                // packed by a step in front
 #pragma unroll
   for (int s = 0; s < S - 1; ++s)
     if (s < kts) load_w(s, kt0 + s);
@@ -327,7 +329,7 @@ bool conv_simt_supported(const ConvParams& q) {
 }
 
 cudaError_t launch_conv_simt(const ConvParams& q, const float* x, const float* wt, const float* bias, const float* gate,
-                             const float* residual, float* out, cudaStream_t st) {
+                             const float* residual, float* out, bool constants, cudaStream_t st) {
   ConvDev p{};
   p.x = x; p.wt = wt; p.out = out; p.bias = bias; p.res = residual; p.gate = gate;
   p.ldw = (int)conv_simt_ldw(q.oc); p.m = q.oc; p.k = q.c * q.kh * q.kw; p.hw = q.oh * q.ow; p.n = q.n * p.hw;
@@ -335,6 +337,7 @@ cudaError_t launch_conv_simt(const ConvParams& q, const float* x, const float* w
   p.x_batch = (long long)q.c * q.ih * q.iw; p.out_batch = (long long)p.m * p.hw;
   p.ih = q.ih; p.iw = q.iw; p.ow = q.ow; p.kh = q.kh; p.kw = q.kw; p.sh = q.sh; p.sw = q.sw; p.dh = q.dh; p.dw = q.dw;
   p.pt = q.pad_t; p.pl = q.pad_l;
+  p.early = constants;
   p.act = q.act; p.act_alpha = q.act_alpha; p.act_beta = q.act_beta;
   const bool window = q.kh != 1 || q.kw != 1 || q.sh != 1 || q.sw != 1 || q.pad_t || q.pad_l || q.oh != q.ih || q.ow != q.iw;
   if (window && gate) return cudaErrorInvalidValue;

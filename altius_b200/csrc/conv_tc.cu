@@ -54,6 +54,7 @@ struct ConvTcDev {
   long long x_batch, out_batch;
   int ih, iw, ow, kh, kw, sh, sw, dh, dw, pt, pl;
   float act_alpha, act_beta;
+  int early;                // filter and bias are constants: read ahead of pdl_wait
   int* err;
 };
 
@@ -111,6 +112,7 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(cols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
+  if (!p.early) pdl_wait();                    // computed by a step in front
   const int m0 = blockIdx.y * bn, mlast = p.m - 1 - m0;   // first channel; last one that exists, relative to it
   if (tid < bn) bias_s[tid] = p.bias && tid <= mlast ? __ldg(p.bias + m0 + tid) : 0.f;
   if (WINDOW) {
@@ -133,7 +135,7 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
     mbar_arrive_expect_tx(&full[s], (uint32_t)bbytes);
     bulk_load(smem + s * stage_bytes + 2 * kABytes, wsrc + (size_t)(g % kbs) * (bbytes / 4), (uint32_t)bbytes, &full[s]);
   };
-  if (tid == 0) {                              // constants: may run ahead of pdl_wait
+  if (tid == 0) {                              // ahead of pdl_wait where these are constants
     if (p.resident) {
       mbar_arrive_expect_tx(&w_full, (uint32_t)(kbs * bbytes));
       bulk_load(wres, wsrc, (uint32_t)(kbs * bbytes), &w_full);
@@ -519,7 +521,7 @@ cudaError_t launch_pack_filter_tc(const ConvParams& q, const float* w, float* pa
 }
 
 cudaError_t launch_conv_tc(const ConvParams& q, const float* x, const float* packed, const float* bias, const float* gate,
-                           const float* residual, float* out, int* err_word, cudaStream_t st) {
+                           const float* residual, float* out, bool constants, int* err_word, cudaStream_t st) {
   const Shape sh = pick_shape(q, device_sm_count());
   ConvTcDev p{};
   p.x = x; p.w = packed; p.out = out; p.bias = bias; p.res = residual; p.gate = gate;
@@ -530,6 +532,7 @@ cudaError_t launch_conv_tc(const ConvParams& q, const float* x, const float* pac
   p.ih = q.ih; p.iw = q.iw; p.ow = q.ow; p.kh = q.kh; p.kw = q.kw; p.sh = q.sh; p.sw = q.sw; p.dh = q.dh; p.dw = q.dw;
   p.pt = q.pad_t; p.pl = q.pad_l;
   p.act_alpha = q.act_alpha; p.act_beta = q.act_beta;
+  p.early = constants;
   p.err = err_word;
   const bool window = q.kh != 1 || q.kw != 1 || q.sh != 1 || q.sw != 1 || q.pad_t || q.pad_l || q.oh != q.ih || q.ow != q.iw;
   if (window && gate) return cudaErrorInvalidValue;

@@ -95,6 +95,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   };
   if (warp == kTmaWarp && lane == 0)
     for (int it = 0; it < S && it < kbs; ++it) load_b(it);   // constants: ahead of pdl_wait
+  __syncwarp();
   pdl_wait();
   if (parts > 1) cl.barrier_wait();           // every block of the cluster runs
 

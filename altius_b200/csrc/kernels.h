@@ -185,7 +185,7 @@ inline int64_t conv_simt_ldw(int64_t oc) { return (oc + 3) / 4 * 4; }
 bool conv_simt_supported(const ConvParams& p);
 cudaError_t launch_pack_filter(const float* w, float* wt, int64_t oc, int64_t k, cudaStream_t st);
 cudaError_t launch_conv_simt(const ConvParams& p, const float* x, const float* wt, const float* bias, const float* gate,
-                             const float* residual, float* out, cudaStream_t st);
+                             const float* residual, float* out, bool constants, cudaStream_t st);
 // Larger convolutions (group 1, no Gelu behind) on the tensor cores, 3xTF32, planes read in place
 // (conv_tc.cu). The filter is split and blocked once by launch_pack_filter_tc into
 // conv_tc_filter_elems floats; the other operands as above.
@@ -193,7 +193,7 @@ bool conv_tc_supported(const ConvParams& p);
 int64_t conv_tc_filter_elems(const ConvParams& p);
 cudaError_t launch_pack_filter_tc(const ConvParams& p, const float* w, float* packed, cudaStream_t st);
 cudaError_t launch_conv_tc(const ConvParams& p, const float* x, const float* packed, const float* bias, const float* gate,
-                           const float* residual, float* out, int* err_word, cudaStream_t st);
+                           const float* residual, float* out, bool constants, int* err_word, cudaStream_t st);
 
 // Squeeze-and-excite gate in one kernel (squeeze_excite.cu):
 //   gate[n, :] = act2(W2 * act1(W1 * mean(x[n, :, plane]) + b1) + b2),  W1 [s, c], W2 [c, s].

@@ -1210,6 +1210,8 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
   // GEMM form: out[n] (ocg x ohw) = W_g (ocg x k) * col[n, g] (k x ohw), bias per row.
   const bool pointwise = p.kh == 1 && p.kw == 1 && p.sh == 1 && p.sw == 1 && p.pad_t == 0 &&
                          p.pad_l == 0 && pads[2] == 0 && pads[3] == 0;
+  // What the kernels may read while the one in front still runs.
+  const bool constants = em.c.val(w).is_const && (bias < 0 || em.c.val(bias).is_const);
   if (tensor_conv_applies(*s, flops) && !(pointwise && ohw == 1) && conv_tc_supported(p)) {
     const int wt = new_value(em.c, conv_tc_filter_elems(p), em.c.val(w).is_const);
     em.add("filter_pack", n.op, {w}, {wt}, 4.0 * p.oc * kdim * 3, 0,
@@ -1218,7 +1220,7 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
     const double bytes = f32_bytes(xv) + f32_bytes(wv) + f32_bytes(ov) * (res >= 0 ? 2 : 1);
     em.add("gemm_tf32x3_tcgen05", n.op, {x, wt, bias, gv, res}, {out}, bytes, flops, [=](cudaStream_t st) {
       return launch_conv_tc(p, s->fptr(x), s->fptr(wt), bias >= 0 ? s->fptr(bias) : nullptr,
-                            gv >= 0 ? s->fptr(gv) : nullptr, res >= 0 ? s->fptr(res) : nullptr, s->fptr_mut(out), s->err_word, st);
+                            gv >= 0 ? s->fptr(gv) : nullptr, res >= 0 ? s->fptr(res) : nullptr, s->fptr_mut(out), constants, s->err_word, st);
     });
     return;
   }
@@ -1231,7 +1233,7 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
     const double bytes = f32_bytes(xv) + f32_bytes(wv) + f32_bytes(ov) * (res >= 0 ? 2 : 1);
     em.add("conv_fp32_simt", n.op, {x, wt, bias, gv, res}, {out}, bytes, flops, [=](cudaStream_t st) {
       return launch_conv_simt(p, s->fptr(x), s->fptr(wt), bias >= 0 ? s->fptr(bias) : nullptr,
-                              gv >= 0 ? s->fptr(gv) : nullptr, res >= 0 ? s->fptr(res) : nullptr, s->fptr_mut(out), st);
+                              gv >= 0 ? s->fptr(gv) : nullptr, res >= 0 ? s->fptr(res) : nullptr, s->fptr_mut(out), constants, st);
     });
     return;
   }

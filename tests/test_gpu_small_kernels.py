@@ -125,6 +125,33 @@ def test_tensor_core_convolution(cuda_lib, n, c, h, oc, k, s, p, gate):
     assert (np.abs(got - want) <= 1e-5 * np.abs(want) + 5e-6 * mass).all()
 
 
+# Filter and bias computed by the steps in front: nothing of them may be read before these have finished.
+@pytest.mark.parametrize("n,c,h,oc,kinds", [
+    (1, 48, 12, 40, "conv_fp32_simt"), (2, 256, 28, 96, "gemm_tf32x3_tcgen05")])
+def test_convolution_with_computed_filter(cuda_lib, n, c, h, oc, kinds):
+    rng = np.random.default_rng(c)
+    x, w, b = (rng.standard_normal(d).astype(np.float32) for d in ((n, c, h, h), (oc, c, 1, 1), (oc,)))
+    w2, b2 = rng.standard_normal(w.shape).astype(np.float32), rng.standard_normal(b.shape).astype(np.float32)
+
+    def build(g, xi, wi, bi):
+        return g.op("Conv2d", xi, g.op("Mul", wi, g.new_init(w2)), g.op("Mul", bi, g.new_init(b2)), kernel_shape=[1, 1],
+                    strides=[1, 1], padding=[0] * 4, dilations=[1, 1], group=1, auto_pad="")
+    g = ir.Graph()
+    vals = [g.add_input(f"in{i}", a.shape) for i, a in enumerate((x, w, b))]
+    g.outputs.append(build(g, *vals))
+    sess = CudaSessionBuilder(ir.Model(g, 13)).build()
+    assert kinds in [e["kind"] for e in sess.schedule()]
+    t = lambda a: torch.from_numpy(a).double()
+    for i in range(3):       # other operands on each run
+        xs = [np.roll(a, i, 0) * np.float32(1 + i) for a in (x, w, b)]
+        got = sess.run(xs)[0]
+        wd, bd = t(xs[1] * w2), t(xs[2] * b2)
+        want = torch.nn.functional.conv2d(t(xs[0]), wd, bd).numpy()
+        mass = torch.nn.functional.conv2d(t(xs[0]).abs(), wd.abs(), bd.abs()).numpy()
+        assert (np.abs(got - want) <= 1e-5 * np.abs(want) + 5e-6 * mass).all()
+    sess.close()
+
+
 # An MLP behind a LayerNormalization: both products on clusters that share a tile along K, the first one
 # writing the halves the second one takes. Rows off the tiles, K off the K-blocks, N off the tile widths.
 # fp16-split products: 1e-5 |want| + 5e-6 sum |a||b| each (as in the other tests of the format); the first
