@@ -37,7 +37,7 @@ constexpr int kAHalf = BM * KB * 2;           // bytes of A's hi (or lo) tile
 struct KsDev {
   int m, n, k;
   int bn, stages, kper;                       // columns of a tile, ring entries, K-blocks per block of the cluster
-  int pitch;                                  // float4s per row of the exchange buffer (odd: no bank conflicts)
+  int inv;                                    // ceil(2^20 / quads), quads = float4s per row of a block's share: e / quads = e * inv >> 20
   float* c; long long ldc;                    // may be null when c16_hi / c16_lo are given
   uint2* c16_hi; uint2* c16_lo; long long ldc16;
   const float* bias; const float* res; long long ldres;
@@ -58,10 +58,11 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full;
   __shared__ uint32_t tmem_slot;
+  __shared__ unsigned seen;                   // what the block has seen of the values it split
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bn = p.bn, S = p.stages, parts = gridDim.z, share = bn / parts, rank = blockIdx.z;
   const int bhalf = bn * KB * 2, stage_bytes = 2 * kAHalf + 2 * bhalf;
-  float4* part = reinterpret_cast<float4*>(smem + S * stage_bytes);   // [parts][BM][pitch]
+  float4* part = reinterpret_cast<float4*>(smem + S * stage_bytes);   // [parts][quads][BM + 1]
   const int nkb = (p.k + KB - 1) / KB, kb0 = rank * p.kper, kbs = min(nkb, kb0 + p.kper) - kb0;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * bn;
   const uint32_t cols = bn <= 32 ? 32 : bn <= 64 ? 64 : 128;
@@ -70,6 +71,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   if (tid == 0) {
     for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(&acc_full, 1);
+    seen = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) {
@@ -99,7 +101,6 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   pdl_wait();
   if (parts > 1) cl.barrier_wait();           // every block of the cluster runs
 
-  unsigned seen = 0;
   if (warp == kTmaWarp) {
     if (lane == 0) {
       for (int it = 0; it < kbs; ++it) {
@@ -115,7 +116,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       }
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
       for (int it = 0; it < kbs; ++it) {
         const int s = it % S;
@@ -124,8 +125,10 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
         const uint32_t a = smem_u32(smem + s * stage_bytes);
         const uint64_t da = desc_sw128(a), dal = desc_sw128(a + kAHalf);
         const uint64_t db = desc_sw128(a + 2 * kAHalf), dbl = desc_sw128(a + 2 * kAHalf + bhalf);
-        const int steps = min(4, (p.k - (kb0 + it) * KB + 15) / 16);
-        for (int kk = 0; kk < steps; ++kk) {
+        // Always four steps (what lies beyond K arrives as zeros): with a run-time count an instruction
+        // took 113 clocks to issue, unrolled 57 (96 columns).
+#pragma unroll
+        for (int kk = 0; kk < KB / 16; ++kk) {
           const uint64_t off = (uint64_t)(kk * 32 >> 4);
           tc_mma_f16(tmem, dal + off, db + off, idesc, (it > 0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
           tc_mma_f16(tmem, da + off, dbl + off, idesc, 1u);                             // a_hi * b_lo
@@ -135,22 +138,53 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       }
       tc_commit(&acc_full);
     }
-  } else {
-    if (!mbar_wait(&acc_full, 0)) atomicExch(p.err, 63);
+  }
+  // ---- accumulator -> the blocks that finish its columns -> this block's columns of the tile ----
+  // Columns are handled in float4s: `quads` of them per row and block, float4 q of row r of rank s at
+  // [(s * quads + q) * (BM + 1) + r]: a warp's rows are neighbours when they are sent (512 bytes a
+  // store) and its columns lie in different banks when they are read.
+  const int quads = share / 4, total = BM * quads;
+  constexpr int CH = 4;                        // float4s a thread has in work at once
+  float4 rs[CH], bi[CH];
+  auto place = [&](int e, int* row, int* q) {
+    *row = (int)(((unsigned)e * (unsigned)p.inv) >> 20);
+    *q = e - *row * quads;
+    return e < total && m0 + *row < p.m && n0 + rank * share + 4 * *q < p.n;   // n % 4 == 0: the four columns exist together
+  };
+  auto fetch = [&](int e0) {
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      int row, q;
+      rs[i] = bi[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!place(e0 + i * kEpiThreads, &row, &q)) continue;
+      const int col = n0 + rank * share + 4 * q;
+      if (p.res) rs[i] = *reinterpret_cast<const float4*>(p.res + (long long)(m0 + row) * p.ldres + col);
+      if (p.bias) bi[i] = ld_plain(reinterpret_cast<const float4*>(p.bias + col));
+    }
+  };
+  if (warp < 8) {
+    fetch(tid);                                // under the products
+    if (!warp_mbar_wait(&acc_full, 0, lane)) atomicExch(p.err, 63);
     tc_fence_after();
     const int row = (warp & 3) * 32 + lane;
     const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    for (int c = (warp >> 2) * 16; c < bn; c += 32) {
-      uint32_t u[16];
-      tc_ld_32x16_nowait(base + (uint32_t)c, u);
+    for (int c = (warp >> 2) * 16; c < bn; c += 64) {
+      uint32_t u[2][16];
+      const bool two = c + 32 < bn;
+      tc_ld_32x16_nowait(base + (uint32_t)c, u[0]);
+      if (two) tc_ld_32x16_nowait(base + (uint32_t)(c + 32), u[1]);
       tc_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int col = c + 4 * i, owner = col / share;
-        float4* dst = parts > 1 ? cl.map_shared_rank(part, owner) : part;
-        dst[(rank * BM + row) * p.pitch + (col - owner * share) / 4] =
-            make_float4(__uint_as_float(u[4 * i]), __uint_as_float(u[4 * i + 1]), __uint_as_float(u[4 * i + 2]),
-                        __uint_as_float(u[4 * i + 3]));
+      for (int h = 0; h < 2; ++h) {
+        if (h == 1 && !two) break;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int cq = c / 4 + 8 * h + i, owner = (int)(((unsigned)cq * (unsigned)p.inv) >> 20);
+          float4* dst = part + ((rank * quads + cq - owner * quads) * (BM + 1) + row);
+          if (parts > 1) dst = cl.map_shared_rank(dst, owner);
+          *dst = make_float4(__uint_as_float(u[h][4 * i]), __uint_as_float(u[h][4 * i + 1]), __uint_as_float(u[h][4 * i + 2]),
+                             __uint_as_float(u[h][4 * i + 3]));
+        }
       }
     }
     tc_fence_before();
@@ -159,48 +193,64 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   if (parts > 1) cl.sync();
   else __syncthreads();
 
-  // ---- this block's columns of the tile ----
   if (warp < 8) {
-    const float sc = p.acc_scale ? __fmul_rn(__ldg(p.acc_scale), kFixedUnscale) : kFixedUnscale;
-    const int quads = share / 4, total = BM * quads;
+    const float sc = p.acc_scale ? __fmul_rn(ld_plain(p.acc_scale), kFixedUnscale) : kFixedUnscale;
     float most = 0.f;
-#pragma unroll 2
-    for (int e = tid; e < total; e += kEpiThreads) {
-      const int row = e / quads, q = e - row * quads;
-      const int r = m0 + row, col = n0 + rank * share + 4 * q;
-      if (r >= p.m || col >= p.n) continue;   // n % 4 == 0: the four columns exist together
-      float4 rs = make_float4(0.f, 0.f, 0.f, 0.f), b = rs;
-      if (p.res) rs = *reinterpret_cast<const float4*>(p.res + (long long)r * p.ldres + col);
-      if (p.bias) b = __ldg(reinterpret_cast<const float4*>(p.bias + col));
-      float4 x = part[row * p.pitch + q];
-      for (int s = 1; s < parts; ++s) {
-        const float4 u = part[(s * BM + row) * p.pitch + q];
-        x.x = __fadd_rn(x.x, u.x); x.y = __fadd_rn(x.y, u.y); x.z = __fadd_rn(x.z, u.z); x.w = __fadd_rn(x.w, u.w);
+    for (int e0 = tid; e0 < total; e0 += CH * kEpiThreads) {
+      if (e0 != tid) fetch(e0);
+      float4 x[CH];
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int e = e0 + i * kEpiThreads;
+        int row, q;
+        const bool ok = place(e, &row, &q);
+        const float4* src = part + (ok ? q * (BM + 1) + row : 0);
+        x[i] = src[0];
+        for (int s = 1; s < parts; ++s) {
+          const float4 u = src[s * quads * (BM + 1)];
+          x[i].x = __fadd_rn(x[i].x, u.x); x[i].y = __fadd_rn(x[i].y, u.y); x[i].z = __fadd_rn(x[i].z, u.z); x[i].w = __fadd_rn(x[i].w, u.w);
+        }
       }
-      x.x = __fmul_rn(x.x, sc); x.y = __fmul_rn(x.y, sc); x.z = __fmul_rn(x.z, sc); x.w = __fmul_rn(x.w, sc);
-      if (p.bias) { x.x = __fadd_rn(x.x, b.x); x.y = __fadd_rn(x.y, b.y); x.z = __fadd_rn(x.z, b.z); x.w = __fadd_rn(x.w, b.w); }
-      if (ACT == ACT_GELU) {
-        const float2 lo = gelu_ref2(make_float2(x.x, x.y)), hi = gelu_ref2(make_float2(x.z, x.w));
-        x = make_float4(lo.x, lo.y, hi.x, hi.y);
-      } else if (ACT == ACT_RELU) {
-        x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f);
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const float4 b = bi[i], r = rs[i];
+        float4 y = x[i];
+        y.x = __fmul_rn(y.x, sc); y.y = __fmul_rn(y.y, sc); y.z = __fmul_rn(y.z, sc); y.w = __fmul_rn(y.w, sc);
+        if (p.bias) { y.x = __fadd_rn(y.x, b.x); y.y = __fadd_rn(y.y, b.y); y.z = __fadd_rn(y.z, b.z); y.w = __fadd_rn(y.w, b.w); }
+        if (ACT == ACT_GELU) {
+          const float2 lo = gelu_ref2(make_float2(y.x, y.y)), hi = gelu_ref2(make_float2(y.z, y.w));
+          y = make_float4(lo.x, lo.y, hi.x, hi.y);
+        } else if (ACT == ACT_RELU) {
+          y.x = fmaxf(y.x, 0.f); y.y = fmaxf(y.y, 0.f); y.z = fmaxf(y.z, 0.f); y.w = fmaxf(y.w, 0.f);
+        }
+        if (p.res) { y.x = __fadd_rn(y.x, r.x); y.y = __fadd_rn(y.y, r.y); y.z = __fadd_rn(y.z, r.z); y.w = __fadd_rn(y.w, r.w); }
+        x[i] = y;
       }
-      if (p.res) { x.x = __fadd_rn(x.x, rs.x); x.y = __fadd_rn(x.y, rs.y); x.z = __fadd_rn(x.z, rs.z); x.w = __fadd_rn(x.w, rs.w); }
-      if (p.c) *reinterpret_cast<float4*>(p.c + (long long)r * p.ldc + col) = x;
-      if (p.c16_hi) {
-        uint2 h, l;
-        f16_split_fixed(x, h, l);
-        const long long at = ((long long)r * p.ldc16 + col) >> 2;
-        p.c16_hi[at] = h;
-        p.c16_lo[at] = l;
-        most = split_track(most, x);
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        int row, q;
+        if (!place(e0 + i * kEpiThreads, &row, &q)) continue;
+        const long long r = m0 + row;
+        const int col = n0 + rank * share + 4 * q;
+        if (p.c) *reinterpret_cast<float4*>(p.c + r * p.ldc + col) = x[i];
+        if (p.c16_hi) {
+          uint2 h, l;
+          f16_split_fixed(x[i], h, l);
+          const long long at = (r * p.ldc16 + col) >> 2;
+          p.c16_hi[at] = h;
+          p.c16_lo[at] = l;
+          most = split_track(most, x[i]);
+        }
       }
     }
-    if (p.c16_hi) seen = split_seen_fixed_of_max(most);
+    if (p.c16_hi) {
+      const unsigned all = __reduce_or_sync(0xffffffffu, split_seen_fixed_of_max(most));
+      if (lane == 0) atomicOr(&seen, all);
+    }
   }
+  __syncthreads();
   // Out of range, or nothing but tiny values in this block's 128 x share results.
-  const int over = __syncthreads_or((int)(seen & 1u)), fine = __syncthreads_or((int)(seen & 2u)), tiny = __syncthreads_or((int)(seen & 4u));
-  if (tid == 0 && (over || (tiny && !fine))) atomicCAS(p.err, 0, kRangeCode);
+  if (tid == 0 && ((seen & 1u) || ((seen & 4u) && !(seen & 2u)))) atomicCAS(p.err, 0, kRangeCode);
   if (warp == kMmaWarp) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
@@ -210,7 +260,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
 constexpr size_t kSmemMax = 231000;
 
 struct Shape {
-  int bn = 0, split = 0, kper = 0, stages = 0, pitch = 0;
+  int bn = 0, split = 0, kper = 0, stages = 0, inv = 0;
   size_t smem = 0;
   double clocks = 1e30;
 };
@@ -226,15 +276,15 @@ Shape pick_shape(int64_t m, int64_t n, int64_t k, int sms) {
     for (int split : {1, 2, 4, 8}) {
       const int kper = (nkb + split - 1) / split;
       if ((split - 1) * kper >= nkb || (bn % (4 * split)) != 0) continue;
-      const int quads = bn / split / 4, pitch = quads | 1;
-      const size_t stage = 2 * (size_t)kAHalf + (size_t)bn * KB * 4, ex = (size_t)split * BM * pitch * 16;
+      const int quads = bn / split / 4;
+      const size_t stage = 2 * (size_t)kAHalf + (size_t)bn * KB * 4, ex = (size_t)split * quads * (BM + 1) * 16;
       const int stages = (int)std::min<size_t>(std::min(kper, kMaxStages), (kSmemMax - 1024 - ex) / stage);
       if (stages < std::min(2, kper)) continue;
       const double ctas = (double)mt * ((n + bn - 1) / bn) * split, waves = std::ceil(ctas / sms);
       const double kb = std::max(12 * 110.0, (double)stage / 28.0);
       const double t = waves * (kper * kb + 5000.0 + 250.0 * split + 10.0 * bn);
       if (t < best.clocks) {
-        best.bn = bn; best.split = split; best.kper = kper; best.stages = stages; best.pitch = pitch;
+        best.bn = bn; best.split = split; best.kper = kper; best.stages = stages; best.inv = ((1 << 20) + quads - 1) / quads;
         best.smem = stages * stage + ex + 1024;
         best.clocks = t;
       }
@@ -274,7 +324,7 @@ cudaError_t launch_gemm_ks(const GemmParams& q, int* err_word, cudaStream_t st) 
   const Shape sh = pick_shape(q.m, q.n, q.k, device_sm_count());
   KsDev d{};
   d.m = (int)q.m; d.n = (int)q.n; d.k = (int)q.k;
-  d.bn = sh.bn; d.stages = sh.stages; d.kper = sh.kper; d.pitch = sh.pitch;
+  d.bn = sh.bn; d.stages = sh.stages; d.kper = sh.kper; d.inv = sh.inv;
   d.c = q.c; d.ldc = q.ldc;
   d.c16_hi = static_cast<uint2*>(q.c16_hi); d.c16_lo = static_cast<uint2*>(q.c16_lo); d.ldc16 = q.ldc16;
   d.bias = q.bias_n; d.res = q.residual; d.ldres = q.ld_res;

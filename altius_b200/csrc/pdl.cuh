@@ -13,7 +13,14 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // The dependent grid may be scheduled once all blocks have said so (or left).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// `cluster`: blocks per cluster along z (1: none).
+// Loads of what the schedule computes. Not __ldg: the read-only path is for memory that nobody writes
+// while the grid exists, and a grid launched this way exists while its predecessors write.
+template <typename T>
+__device__ __forceinline__ T ld_plain(const T* p) {
+  return *p;
+}
+
+// `cluster`: blocks per cluster along z (1: none; 0: none, and no overlap either).
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster,
                        Args... args) {
@@ -25,7 +32,7 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 0 ? 1 : 0;
   if (cluster > 1) {
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = (unsigned)cluster;

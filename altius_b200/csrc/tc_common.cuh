@@ -81,6 +81,14 @@ __device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, i
   return done != 0;
 }
 
+// One thread of a converged warp, in a form that lets ptxas keep the operands of the tensor-core
+// instructions behind it in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x,
                                             int y, int z) {
   asm volatile(
