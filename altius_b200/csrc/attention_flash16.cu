@@ -185,7 +185,7 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
       }
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       int sn[2] = {0, 0}, pn[2] = {0, 0};       // blocks whose scores / products have been issued
       const int n[2] = {items_of(0) * blocks, items_of(1) * blocks};
       uint32_t idle = 0;
@@ -200,10 +200,23 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
             const uint32_t id128 = (1u << 4) | (1u << 16) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(QM >> 4) << 24);   // B MN-major
             const uint32_t id64 = (1u << 4) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(QM >> 4) << 24);
             const uint64_t v = desc_mn128(base + 4 * kTile);
-            for (int c = 0; c < chunks; ++c)    // P_hi * [V_hi | V_lo]
+            auto hi = [&](int c) {              // P_hi * [V_hi | V_lo]
               mma_f16_ta(o_col, s_col + (uint32_t)(16 * c), v + (uint64_t)(c * 128), id128, (j > 0 || c > 0) ? 1u : 0u);
-            for (int c = 0; c < chunks; ++c)    // P_lo * V_hi
+            };
+            auto lo = [&](int c) {              // P_lo * V_hi
               mma_f16_ta(o_col, s_col + (uint32_t)(16 * c + 8), v + (uint64_t)(c * 128), id64, 1u);
+            };
+            if (chunks == KV / 16) {            // unrolled: half the time to issue an instruction
+#pragma unroll
+              for (int c = 0; c < KV / 16; ++c) hi(c);
+#pragma unroll
+              for (int c = 0; c < KV / 16; ++c) lo(c);
+            } else {
+#pragma unroll 1
+              for (int c = 0; c < chunks; ++c) hi(c);
+#pragma unroll 1
+              for (int c = 0; c < chunks; ++c) lo(c);
+            }
             tc_commit(&bar.pv_done[g]);
             ++pn[g];
             did = true;
@@ -243,7 +256,7 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
     const uint32_t scol = trow + (uint32_t)(g * 128 + hf * 64), ocol = trow + kOCol + (uint32_t)(g * 128 + hf * 32);
     // Scores arrive as (q * 2^8) . (k * 2^8); t = acc * c1 with c1 = 2^-16 * log2(e) (* | /) scale.
     const float kLog2e = 1.44269504088896341f;
-    const float sc = SMODE ? __ldg(p.scale) : 1.f;
+    const float sc = SMODE ? ld_plain(p.scale) : 1.f;
     const float c1 = __fmul_rn(SMODE == 1 ? __fmul_rn(sc, kLog2e) : (SMODE == 2 ? __fdiv_rn(kLog2e, sc) : kLog2e),
                                kFixedUnscale * kFixedUnscale);
     float seen_max = 0.f;

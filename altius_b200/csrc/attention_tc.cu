@@ -45,6 +45,7 @@
 #include <type_traits>
 
 #include "kernels.h"
+#include "pdl.cuh"
 #include "ref_math.cuh"
 #include "tc_common.cuh"
 
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(kAtLaunch, 1) attention_tc_kernel(AttnTcDev p)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();
   if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(kTmemCols));
@@ -259,7 +261,7 @@ __global__ void __launch_bounds__(kAtLaunch, 1) attention_tc_kernel(AttnTcDev p)
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int idx = tid + kAtThreads * i, row = idx >> 4, c4 = idx & 15;
-        if (FIRST) qv[i] = __ldg(reinterpret_cast<const float4*>(qg + (long long)min(q0 + row, T - 1) * p.row_stride + c4 * 4));
+        if (FIRST) qv[i] = ld_plain(reinterpret_cast<const float4*>(qg + (long long)min(q0 + row, T - 1) * p.row_stride + c4 * 4));
         else qv[i] = qnext[i];
       }
       if constexpr (FIRST) {
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(kAtLaunch, 1) attention_tc_kernel(AttnTcDev p)
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
           const int idx = tid + kAtThreads * i, row = idx >> 4, c4 = idx & 15;
-          kvv[i] = __ldg(reinterpret_cast<const float4*>(kg + (long long)min(row, T - 1) * p.row_stride + c4 * 4));
+          kvv[i] = ld_plain(reinterpret_cast<const float4*>(kg + (long long)min(row, T - 1) * p.row_stride + c4 * 4));
         }
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
@@ -289,7 +291,7 @@ __global__ void __launch_bounds__(kAtLaunch, 1) attention_tc_kernel(AttnTcDev p)
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int t = 16 * i + 4 * vtg + u;
-            vv[i][u] = __ldg(vg + (long long)min(t, T - 1) * p.row_stride + vd);   // masked when stored
+            vv[i][u] = ld_plain(vg + (long long)min(t, T - 1) * p.row_stride + vd);   // masked when stored
           }
       }
     }
@@ -360,7 +362,7 @@ __global__ void __launch_bounds__(kAtLaunch, 1) attention_tc_kernel(AttnTcDev p)
       // e = 2^(t - max t) is one FFMA and one ex2.approx per score (2 ulp; the CUDA-core kernel
       // keeps the reference's polynomial).
       const float kLog2e = 1.44269504088896341f;
-      const float sc = SMODE ? __ldg(p.scale) : 1.f;
+      const float sc = SMODE ? ld_plain(p.scale) : 1.f;
       const float c1 = SMODE == 1 ? __fmul_rn(sc, kLog2e) : (SMODE == 2 ? __fdiv_rn(kLog2e, sc) : kLog2e);
       float m = CUDART_NAN_F;
 #pragma unroll 1
@@ -427,7 +429,7 @@ __global__ void __launch_bounds__(kAtLaunch, 1) attention_tc_kernel(AttnTcDev p)
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int idx = tid + kAtThreads * i, r2 = idx >> 4, c4 = idx & 15;
-          qnext[i] = __ldg(reinterpret_cast<const float4*>(qg + (long long)min(q0 + QM + r2, T - 1) * p.row_stride + c4 * 4));
+          qnext[i] = ld_plain(reinterpret_cast<const float4*>(qg + (long long)min(q0 + QM + r2, T - 1) * p.row_stride + c4 * 4));
         }
       }
       xch[hf * QM + row] = sum;
@@ -530,8 +532,7 @@ cudaError_t launch_nb_mode(const AttnTcDev& d, int bh, cudaStream_t st) {
   cudaError_t e = ensure_dynamic_smem(attention_tc_kernel<NB, SMODE, kResident>, kDyn, &attr_done);
   if (e != cudaSuccess) return e;
   dim3 grid(kResident ? 1 : (d.tokens + QM - 1) / QM, bh);
-  attention_tc_kernel<NB, SMODE, kResident><<<grid, kAtLaunch, kDyn, st>>>(d);
-  return cudaGetLastError();
+  return launch_pdl(attention_tc_kernel<NB, SMODE, kResident>, grid, dim3(kAtLaunch), kDyn, st, 1, d);
 }
 
 template <int NB>

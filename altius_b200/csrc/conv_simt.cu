@@ -88,7 +88,7 @@ __device__ __forceinline__ float finish(const ConvDev& p, float v, float bias) {
 template <int LOAD>
 __device__ __forceinline__ void store_quad(const ConvDev& p, int row, int col, float4 v) {
   if (row >= p.m || col >= p.n) return;
-  const float bias = p.bias ? __ldg(p.bias + row) : 0.f;
+  const float bias = p.bias ? ld_plain(p.bias + row) : 0.f;
   v.x = finish(p, v.x, bias); v.y = finish(p, v.y, bias); v.z = finish(p, v.z, bias); v.w = finish(p, v.w, bias);
   if (LOAD == LOAD_VEC) {   // planes are whole float4s: the four columns lie in one image
     const int b = col / p.hw;

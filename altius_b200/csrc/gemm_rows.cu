@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kWarps * 32) gemm_rows_kernel(const GemmParams
   for (int k = lane * 4; k < K; k += 128) {
     float4 bv[NW];
 #pragma unroll
-    for (int j = 0; j < NW; ++j) bv[j] = __ldg(reinterpret_cast<const float4*>(b[j] + k));
+    for (int j = 0; j < NW; ++j) bv[j] = ld_plain(reinterpret_cast<const float4*>(b[j] + k));
 #pragma unroll
     for (int i = 0; i < MT; ++i) {
       const float4 av = *reinterpret_cast<const float4*>(a[i] + k);

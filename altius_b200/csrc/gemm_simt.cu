@@ -13,6 +13,7 @@
 // conflict-free float4), operands staged through double-buffered shared memory
 // with the next K step prefetched into registers during the math.
 #include "kernels.h"
+#include "pdl.cuh"
 #include "ref_math.cuh"
 
 namespace ac {
@@ -247,20 +248,24 @@ __global__ void __launch_bounds__(256) depthwise_kernel(const float* __restrict_
 // pixels. Per output the taps are visited in the same order as above and out-of-range taps are
 // skipped, so the results are bit-identical to the generic kernel.
 template <int K, int S, int ACT>
-__global__ void __launch_bounds__(256) depthwise_rows_kernel(const float* __restrict__ x,
+__global__ void __launch_bounds__(256) depthwise_rows_kernel(const float* x,
                                                              const float* __restrict__ w,
                                                              const float* __restrict__ bias,
-                                                             float* __restrict__ out, ConvParams p,
+                                                             float* out, ConvParams p,
                                                              unsigned owg, unsigned items) {
   const unsigned item = blockIdx.x * 256u + threadIdx.x;
-  if (item >= items) return;
-  const unsigned xg = item % owg, t = item / owg;
+  const bool live = item < items;
+  const unsigned xg = item % owg, t = (live ? item : 0u) / owg;
   const unsigned oy = t % (unsigned)p.oh, plane = t / (unsigned)p.oh;   // plane = n * c + ch
   const int ch = (int)(plane % (unsigned)p.c);
   const float* in = x + (long long)plane * p.ih * p.iw;
   float wk[K * K];
 #pragma unroll
-  for (int i = 0; i < K * K; ++i) wk[i] = __ldg(w + ch * (K * K) + i);
+  for (int i = 0; i < K * K; ++i) wk[i] = __ldg(w + ch * (K * K) + i);   // constants where the launch overlaps
+  const float bv = bias ? __ldg(bias + ch) : 0.f;
+  pdl_trigger();
+  pdl_wait();
+  if (!live) return;
   constexpr int SEG = 3 * S + K;
   const int ox0 = (int)xg * 4;
   const int y0 = (int)oy * S - p.pad_t, x0 = ox0 * S - p.pad_l;
@@ -274,7 +279,7 @@ __global__ void __launch_bounds__(256) depthwise_rows_kernel(const float* __rest
 #pragma unroll
     for (int j = 0; j < SEG; ++j) {
       const int ix = x0 + j;
-      seg[j] = (ix >= 0 && ix < p.iw) ? __ldg(row + ix) : 0.f;
+      seg[j] = (ix >= 0 && ix < p.iw) ? ld_plain(row + ix) : 0.f;
     }
 #pragma unroll
     for (int fx = 0; fx < K; ++fx)
@@ -284,7 +289,6 @@ __global__ void __launch_bounds__(256) depthwise_rows_kernel(const float* __rest
         if (ix >= 0 && ix < p.iw) acc[o] = fmaf(wk[fy * K + fx], seg[o * S + fx], acc[o]);
       }
   }
-  const float bv = bias ? __ldg(bias + ch) : 0.f;
   float* dst = out + ((long long)plane * p.oh + oy) * p.ow + ox0;
 #pragma unroll
   for (int o = 0; o < 4; ++o) {
@@ -297,12 +301,12 @@ __global__ void __launch_bounds__(256) depthwise_rows_kernel(const float* __rest
 
 template <int K, int S>
 bool launch_depthwise_rows(const ConvParams& p, const float* x, const float* w, const float* bias, float* out,
-                           unsigned owg, unsigned items, cudaStream_t st) {
+                           unsigned owg, unsigned items, int overlap, cudaError_t* e, cudaStream_t st) {
   const unsigned blocks = (items + 255u) / 256u;
   switch (p.act) {
-    case ACT_NONE: depthwise_rows_kernel<K, S, ACT_NONE><<<blocks, 256, 0, st>>>(x, w, bias, out, p, owg, items); return true;
-    case ACT_RELU: depthwise_rows_kernel<K, S, ACT_RELU><<<blocks, 256, 0, st>>>(x, w, bias, out, p, owg, items); return true;
-    case ACT_HARDSWISH: depthwise_rows_kernel<K, S, ACT_HARDSWISH><<<blocks, 256, 0, st>>>(x, w, bias, out, p, owg, items); return true;
+    case ACT_NONE: *e = launch_pdl(depthwise_rows_kernel<K, S, ACT_NONE>, dim3(blocks), dim3(256), 0, st, overlap, x, w, bias, out, p, owg, items); return true;
+    case ACT_RELU: *e = launch_pdl(depthwise_rows_kernel<K, S, ACT_RELU>, dim3(blocks), dim3(256), 0, st, overlap, x, w, bias, out, p, owg, items); return true;
+    case ACT_HARDSWISH: *e = launch_pdl(depthwise_rows_kernel<K, S, ACT_HARDSWISH>, dim3(blocks), dim3(256), 0, st, overlap, x, w, bias, out, p, owg, items); return true;
     default: return false;
   }
 }
@@ -333,18 +337,20 @@ cudaError_t launch_gemm_simt(const GemmParams& q, cudaStream_t st) {
 }
 
 cudaError_t launch_depthwise_conv(const ConvParams& p, const float* x, const float* w,
-                                  const float* bias, float* out, cudaStream_t st) {
+                                  const float* bias, float* out, bool constants, cudaStream_t st) {
   const long long total = (long long)p.n * p.oc * p.oh * p.ow;
   if (total == 0) return cudaSuccess;
   const long long owg = (p.ow + 3) / 4, items = (long long)p.n * p.oc * p.oh * owg;
   if (p.kh == p.kw && p.sh == p.sw && p.dh == 1 && p.dw == 1 && items < (1ll << 31) &&
       (long long)p.ih * p.iw < (1ll << 31)) {
     bool done = false;
-    if (p.kh == 3 && p.sh == 1) done = launch_depthwise_rows<3, 1>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, st);
-    else if (p.kh == 3 && p.sh == 2) done = launch_depthwise_rows<3, 2>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, st);
-    else if (p.kh == 5 && p.sh == 1) done = launch_depthwise_rows<5, 1>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, st);
-    else if (p.kh == 5 && p.sh == 2) done = launch_depthwise_rows<5, 2>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, st);
-    if (done) return cudaGetLastError();
+    cudaError_t e = cudaSuccess;
+    const int overlap = constants ? 1 : 0;
+    if (p.kh == 3 && p.sh == 1) done = launch_depthwise_rows<3, 1>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, overlap, &e, st);
+    else if (p.kh == 3 && p.sh == 2) done = launch_depthwise_rows<3, 2>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, overlap, &e, st);
+    else if (p.kh == 5 && p.sh == 1) done = launch_depthwise_rows<5, 1>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, overlap, &e, st);
+    else if (p.kh == 5 && p.sh == 2) done = launch_depthwise_rows<5, 2>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, overlap, &e, st);
+    if (done) return e;
   }
   depthwise_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(x, w, bias, out, p, total);
   return cudaGetLastError();

@@ -49,6 +49,7 @@
 #include <mutex>
 
 #include "kernels.h"
+#include "pdl.cuh"
 #include "ref_math.cuh"
 #include "tc_common.cuh"
 
@@ -154,7 +155,7 @@ __device__ __forceinline__ void load_acc(uint32_t taddr, uint32_t (&v)[32], floa
   }
 }
 __device__ __forceinline__ float acc_scale_of(const TcEpilogue& ep) {
-  return ep.acc_scale ? __fmul_rn(__ldg(ep.acc_scale), ep.acc_scale_const) : ep.acc_scale_const;
+  return ep.acc_scale ? __fmul_rn(ld_plain(ep.acc_scale), ep.acc_scale_const) : ep.acc_scale_const;
 }
 
 // Epilogue of one warp's 32 rows. The accumulator chunk arrives with one thread
@@ -191,12 +192,12 @@ __device__ __noinline__ void epilogue_generic(const TcEpilogue& ep, float4* stag
         const int col = col0 + 4 * c4;
         float4 bn = make_float4(0.f, 0.f, 0.f, 0.f);
         if (ep.bias_n) {
-          if (vec_ok && col + 3 < ep.n) bn = __ldg(reinterpret_cast<const float4*>(ep.bias_n + col));
+          if (vec_ok && col + 3 < ep.n) bn = ld_plain(reinterpret_cast<const float4*>(ep.bias_n + col));
           else {
-            if (col < ep.n) bn.x = __ldg(ep.bias_n + col);
-            if (col + 1 < ep.n) bn.y = __ldg(ep.bias_n + col + 1);
-            if (col + 2 < ep.n) bn.z = __ldg(ep.bias_n + col + 2);
-            if (col + 3 < ep.n) bn.w = __ldg(ep.bias_n + col + 3);
+            if (col < ep.n) bn.x = ld_plain(ep.bias_n + col);
+            if (col + 1 < ep.n) bn.y = ld_plain(ep.bias_n + col + 1);
+            if (col + 2 < ep.n) bn.z = ld_plain(ep.bias_n + col + 2);
+            if (col + 3 < ep.n) bn.w = ld_plain(ep.bias_n + col + 3);
           }
           if (ep.bias_scale != 1.f) {
             bn.x = __fmul_rn(ep.bias_scale, bn.x); bn.y = __fmul_rn(ep.bias_scale, bn.y);
@@ -214,24 +215,24 @@ __device__ __noinline__ void epilogue_generic(const TcEpilogue& ep, float4* stag
           float cv[4] = {0.f, 0.f, 0.f, 0.f}, rv[4] = {0.f, 0.f, 0.f, 0.f};
           if (cin) {
             if (full4) {
-              const float4 t4 = __ldg(reinterpret_cast<const float4*>(cin + (long long)row * ep.ldcin + col));
+              const float4 t4 = ld_plain(reinterpret_cast<const float4*>(cin + (long long)row * ep.ldcin + col));
               cv[0] = t4.x; cv[1] = t4.y; cv[2] = t4.z; cv[3] = t4.w;
             } else {
               for (int e = 0; e < 4; ++e)
-                if (col + e < ep.n) cv[e] = __ldg(cin + (long long)row * ep.ldcin + col + e);
+                if (col + e < ep.n) cv[e] = ld_plain(cin + (long long)row * ep.ldcin + col + e);
             }
           }
           if (res) {
             if (full4) {
-              const float4 t4 = __ldg(reinterpret_cast<const float4*>(res + (long long)row * ep.ldres + col));
+              const float4 t4 = ld_plain(reinterpret_cast<const float4*>(res + (long long)row * ep.ldres + col));
               rv[0] = t4.x; rv[1] = t4.y; rv[2] = t4.z; rv[3] = t4.w;
             } else {
               for (int e = 0; e < 4; ++e)
-                if (col + e < ep.n) rv[e] = __ldg(res + (long long)row * ep.ldres + col + e);
+                if (col + e < ep.n) rv[e] = ld_plain(res + (long long)row * ep.ldres + col + e);
             }
           }
-          const float bm = ep.bias_m ? (ep.bias_scale == 1.f ? __ldg(ep.bias_m + row)
-                                                             : __fmul_rn(ep.bias_scale, __ldg(ep.bias_m + row)))
+          const float bm = ep.bias_m ? (ep.bias_scale == 1.f ? ld_plain(ep.bias_m + row)
+                                                             : __fmul_rn(ep.bias_scale, ld_plain(ep.bias_m + row)))
                                      : 0.f;
           const float bnv[4] = {bn.x, bn.y, bn.z, bn.w};
 #pragma unroll
@@ -278,7 +279,7 @@ __device__ __forceinline__ bool epilogue_fast(const TcEpilogue& ep, float4* stag
   float bm[8];
   if (BIAS == 2) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) bm[i] = row_base + 4 * i < ep.m ? __ldg(ep.bias_m + row_base + 4 * i) : 0.f;
+    for (int i = 0; i < 8; ++i) bm[i] = row_base + 4 * i < ep.m ? ld_plain(ep.bias_m + row_base + 4 * i) : 0.f;
   }
 #pragma unroll 1
   for (int cc = cc0; cc < cc1; ++cc) {
@@ -297,7 +298,7 @@ __device__ __forceinline__ bool epilogue_fast(const TcEpilogue& ep, float4* stag
     const int col = col0 + 4 * c4;
     const bool col_ok = col < ep.n;   // n % 4 == 0: the whole float4 is in range
     float4 bn = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (BIAS == 1 && col_ok) bn = __ldg(reinterpret_cast<const float4*>(ep.bias_n + col));
+    if (BIAS == 1 && col_ok) bn = ld_plain(reinterpret_cast<const float4*>(ep.bias_n + col));
     float4 a[8], r[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -306,7 +307,7 @@ __device__ __forceinline__ bool epilogue_fast(const TcEpilogue& ep, float4* stag
       if (HAS_RES) {
         const int row = row_base + 4 * i;
         r[i] = (col_ok && row < ep.m)
-                   ? __ldg(reinterpret_cast<const float4*>(res + (long long)row * ep.ldres + col))
+                   ? ld_plain(reinterpret_cast<const float4*>(res + (long long)row * ep.ldres + col))
                    : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
@@ -410,7 +411,7 @@ __device__ __forceinline__ bool epilogue_parked(const TcEpilogue& ep, float4* bu
     const int col = n0 + chunk * 32 + 4 * c8;
     const bool col_ok = col < ep.n;                 // n % 4 == 0: the whole float4 is in range
     float4 bn = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (BIAS == 1 && col_ok) bn = __ldg(reinterpret_cast<const float4*>(ep.bias_n + col));
+    if (BIAS == 1 && col_ok) bn = ld_plain(reinterpret_cast<const float4*>(ep.bias_n + col));
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
       const int row_base = m0 + q * 32 + 16 * pass + r4;
@@ -421,10 +422,10 @@ __device__ __forceinline__ bool epilogue_parked(const TcEpilogue& ep, float4* bu
         const int rl = 16 * pass + 4 * i + r4;
         a[i] = buf[rl * 8 + epi_slot(rl, c8)];
         const int row = row_base + 4 * i;
-        if (BIAS == 2) bm[i] = row < ep.m ? __ldg(ep.bias_m + row) : 0.f;
+        if (BIAS == 2) bm[i] = row < ep.m ? ld_plain(ep.bias_m + row) : 0.f;
         if (HAS_RES) {
           r[i] = (col_ok && row < ep.m)
-                     ? __ldg(reinterpret_cast<const float4*>(res + (long long)row * ep.ldres + col))
+                     ? ld_plain(reinterpret_cast<const float4*>(res + (long long)row * ep.ldres + col))
                      : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
@@ -522,19 +523,19 @@ __device__ __forceinline__ void fixup_apply(const TcEpilogue& ep, int row, int c
     float y = x[e];
     if (ep.alpha != 1.f) y = __fmul_rn(ep.alpha, y);
     if (cin) {
-      const float cv = __ldg(cin + (long long)row * ep.ldcin + col);
+      const float cv = ld_plain(cin + (long long)row * ep.ldcin + col);
       y = __fadd_rn(ep.beta == 1.f ? cv : __fmul_rn(ep.beta, cv), y);
     }
     if (ep.bias_n) {
-      const float bv = __ldg(ep.bias_n + col);
+      const float bv = ld_plain(ep.bias_n + col);
       y = __fadd_rn(y, ep.bias_scale == 1.f ? bv : __fmul_rn(ep.bias_scale, bv));
     }
     if (ep.bias_m) {
-      const float bv = __ldg(ep.bias_m + row);
+      const float bv = ld_plain(ep.bias_m + row);
       y = __fadd_rn(y, ep.bias_scale == 1.f ? bv : __fmul_rn(ep.bias_scale, bv));
     }
     y = apply_act(ep.act, y, ep.act_alpha, ep.act_beta);
-    if (res) y = __fadd_rn(y, __ldg(res + (long long)row * ep.ldres + col));
+    if (res) y = __fadd_rn(y, ld_plain(res + (long long)row * ep.ldres + col));
     if (c) c[(long long)row * ep.ldc + col] = y;
     y4[e] = y;
   }
@@ -551,9 +552,11 @@ __device__ __forceinline__ void fixup_apply(const TcEpilogue& ep, int row, int c
 }
 
 // Adds the K-slices of the tail tiles in slice order and applies the epilogue.
-__global__ void __launch_bounds__(256) gemm_tc_fixup_kernel(const float* __restrict__ ws, TcEpilogue ep, int bm,
+__global__ void __launch_bounds__(256) gemm_tc_fixup_kernel(const float* ws, TcEpilogue ep, int bm,
                                                             int bn, int dp_tiles, int parts, int tiles_m,
                                                             int tiles_n) {
+  pdl_trigger();
+  pdl_wait();
   const int tt = blockIdx.y;
   const int t = dp_tiles + tt;
   const int tn = t % tiles_n, tm = (t / tiles_n) % tiles_m, bz = t / (tiles_n * tiles_m);
@@ -565,7 +568,7 @@ __global__ void __launch_bounds__(256) gemm_tc_fixup_kernel(const float* __restr
   const float* src = ws + (size_t)tt * parts * bm * bn + (size_t)rl * bn + cl;
   // Slices are added in slice order; their loads are issued eight at a time so that the
   // chain of additions does not also serialise the L2 round trips.
-  float4 acc = __ldg(reinterpret_cast<const float4*>(src));
+  float4 acc = __ldcg(reinterpret_cast<const float4*>(src));
   auto add = [&](const float4& v) {
     acc.x = __fadd_rn(acc.x, v.x); acc.y = __fadd_rn(acc.y, v.y);
     acc.z = __fadd_rn(acc.z, v.z); acc.w = __fadd_rn(acc.w, v.w);
@@ -574,11 +577,11 @@ __global__ void __launch_bounds__(256) gemm_tc_fixup_kernel(const float* __restr
   for (; p + 8 <= parts; p += 8) {
     float4 v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __ldg(reinterpret_cast<const float4*>(src + (size_t)(p + j) * bm * bn));
+    for (int j = 0; j < 8; ++j) v[j] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(p + j) * bm * bn));
 #pragma unroll
     for (int j = 0; j < 8; ++j) add(v[j]);
   }
-  for (; p < parts; ++p) add(__ldg(reinterpret_cast<const float4*>(src + (size_t)p * bm * bn)));
+  for (; p < parts; ++p) add(__ldcg(reinterpret_cast<const float4*>(src + (size_t)p * bm * bn)));
   fixup_apply(ep, row, col0, bz, acc);
 }
 
@@ -706,6 +709,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();                         // behind the allocation: the next kernel's cannot come first
+  pdl_wait();
 
   if (warp == kTmaWarp) {
     // ---------------- TMA producer ----------------
@@ -873,7 +878,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
               float4 v = sb[i * kSplitThreads + t0];
               if (MODE == TC_3X_SPLIT_B_MN && rs) {
                 const int k = kb * KB + ((i * kSplitThreads + t0) % (KB * 8)) / 8;
-                const float f = k < ep.k_total ? __ldg(rs + k) : 1.f;
+                const float f = k < ep.k_total ? ld_plain(rs + k) : 1.f;
                 v.x = __fmul_rn(v.x, f); v.y = __fmul_rn(v.y, f); v.z = __fmul_rn(v.z, f); v.w = __fmul_rn(v.w, f);
               }
               tf32_split(v, hi, lo);
@@ -1038,7 +1043,7 @@ __device__ __forceinline__ void pair_stamp(int dbg, int slot) {
 // barriers, which is all the MMA thread waits for.
 template <int BN, bool PRE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-gemm_tc_pair_kernel(const float* __restrict__ a_ptr, long long lda, int k_total,
+gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
                     const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_alo,
                     const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_blo,
                     TcEpilogue ep, TcSched sc, int tiles_m, int tiles_n, float* workspace, int* err, int dbg) {
@@ -1094,6 +1099,8 @@ gemm_tc_pair_kernel(const float* __restrict__ a_ptr, long long lda, int k_total,
   cluster_sync_all();                    // barriers of both CTAs initialised before any remote arrival
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();                         // behind the allocation: the next kernel's cannot come first
+  pdl_wait();
   if (threadIdx.x == 0) pair_stamp(dbg, 1);
 
   if (warp == kTmaWarp) {
@@ -1235,7 +1242,7 @@ gemm_tc_pair_kernel(const float* __restrict__ a_ptr, long long lda, int k_total,
           const int item = i * kSplitThreads + t0;
           const int r = item >> 3, kcol = kb * KB + (item & 7) * 4;
           x[i] = (m0 + r < ep.m && kcol < k_total)
-                     ? __ldg(reinterpret_cast<const float4*>(a_tile + (long long)r * lda + kcol))
+                     ? ld_plain(reinterpret_cast<const float4*>(a_tile + (long long)r * lda + kcol))
                      : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         ok = mbar_wait(&empty[s], ph ^ 1);          // the pair's MMAs on the previous use of the stage are done
@@ -1375,7 +1382,7 @@ __global__ void tf32_split_kernel(const float* __restrict__ x, float* __restrict
                                   float* __restrict__ lo, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
-    const float v = __ldg(x + i);
+    const float v = ld_plain(x + i);
     const float h = round_tf32(v);
     hi[i] = h;
     lo[i] = round_tf32(__fsub_rn(v, h));
@@ -1386,7 +1393,7 @@ __global__ void tf32_split_kernel(const float* __restrict__ x, float* __restrict
 __global__ void absmax_kernel(const float* __restrict__ x, int64_t rows, int64_t k, int64_t ld, unsigned* out) {
   unsigned m = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * k; i += (int64_t)gridDim.x * blockDim.x) {
-    const unsigned ab = __float_as_uint(__ldg(x + (i / k) * ld + (i % k))) & 0x7FFFFFFFu;
+    const unsigned ab = __float_as_uint(ld_plain(x + (i / k) * ld + (i % k))) & 0x7FFFFFFFu;
     if (ab < 0x7F800000u) m = max(m, ab);
   }
   m = __reduce_max_sync(0xffffffffu, m);
@@ -1416,7 +1423,7 @@ __global__ void f16_split_kernel(const float* __restrict__ x, __half* __restrict
   if (i == 0 && inv_scale) *inv_scale = __fdiv_rn(1.f, sc);
   if (i >= rows * k8) return;
   const int64_t r = i / k8, c = i % k8;
-  const float v = c < k ? __fmul_rn(__ldg(x + r * ld + c), sc) : 0.f;
+  const float v = c < k ? __fmul_rn(ld_plain(x + r * ld + c), sc) : 0.f;
   const __half h = __float2half_rn(v);
   hi[i] = h;
   const float rest = __fsub_rn(v, __half2float(h));
@@ -1434,7 +1441,7 @@ __global__ void __launch_bounds__(256) f16_split_vec8_kernel(const float* __rest
   if (i < rows * k8th) {
     const int64_t r = i / k8th, c = i % k8th;
     const float4* src = reinterpret_cast<const float4*>(x + r * ld + c * 8);
-    const float4 v0 = __ldg(src), v1 = __ldg(src + 1);
+    const float4 v0 = ld_plain(src), v1 = ld_plain(src + 1);
     uint2 h0, l0, h1, l1;
     if (fixed) {
       f16_split_fixed(v0, h0, l0);
@@ -1555,15 +1562,13 @@ cudaError_t launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtens
   using L = TcSmem<BN, MT, MODE>;
   static unsigned long long attr_done = 0;
   if (cudaError_t e0 = ensure_dynamic_smem(gemm_tc_kernel<BN, MT, MODE>, L::kDynBytes, &attr_done)) return e0;
-  gemm_tc_kernel<BN, MT, MODE><<<pl.grid, kThreads, L::kDynBytes, st>>>(ma, mb, mbl, ep, pl.sc, a_batched, b_batched,
-                                                                    pl.tiles_m, pl.tiles_n, workspace, err);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pdl(gemm_tc_kernel<BN, MT, MODE>, dim3((unsigned)pl.grid), dim3(kThreads), L::kDynBytes, st, 1, ma, mb,
+                                   mbl, ep, pl.sc, a_batched, b_batched, pl.tiles_m, pl.tiles_n, workspace, err);
   if (e != cudaSuccess || pl.sc.tail_parts < 2) return e;
   const int tail = pl.sc.num_tiles - pl.sc.dp_tiles;
   dim3 grid((MT * BM * BN / 4 + 255) / 256, tail);
-  gemm_tc_fixup_kernel<<<grid, 256, 0, st>>>(workspace, ep, MT * BM, BN, pl.sc.dp_tiles, pl.sc.tail_parts, pl.tiles_m,
-                                             pl.tiles_n);
-  return cudaGetLastError();
+  return launch_pdl(gemm_tc_fixup_kernel, grid, dim3(256), 0, st, 1, workspace, ep, MT * BM, BN, pl.sc.dp_tiles, pl.sc.tail_parts,
+                    pl.tiles_m, pl.tiles_n);
 }
 
 template <int BN, bool PRE>
@@ -1575,8 +1580,8 @@ cudaError_t launch_pair(const float* a, long long lda, int k, const CUtensorMap&
   if (cudaError_t e0 = ensure_dynamic_smem(gemm_tc_pair_kernel<BN, PRE>, L::kDynBytes, &attr_done)) return e0;
   // pl.grid counts pairs; the cluster shape (2, 1, 1) is a compile-time attribute of the kernel.
   static const int dbg = std::getenv("ALTIUS_CUDA_TC_DBG") ? std::atoi(std::getenv("ALTIUS_CUDA_TC_DBG")) : 0;
-  gemm_tc_pair_kernel<BN, PRE><<<2 * pl.grid, kThreads, L::kDynBytes, st>>>(a, lda, k, ma, mal, mb, mbl, ep, pl.sc,
-                                                                          pl.tiles_m, pl.tiles_n, workspace, err, dbg);
+  const cudaError_t e = launch_pdl(gemm_tc_pair_kernel<BN, PRE>, dim3(2u * (unsigned)pl.grid), dim3(kThreads), L::kDynBytes, st, 1, a, lda,
+                                   k, ma, mal, mb, mbl, ep, pl.sc, pl.tiles_m, pl.tiles_n, workspace, err, dbg);
   if (dbg & 0x1000) {
     cudaStreamSynchronize(st);
     static long long h[160][24];
@@ -1593,13 +1598,11 @@ cudaError_t launch_pair(const float* a, long long lda, int k, const CUtensorMap&
       std::printf("\n");
     }
   }
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || pl.sc.tail_parts < 2) return e;
   const int tail = pl.sc.num_tiles - pl.sc.dp_tiles;
   dim3 grid((2 * BM * BN / 4 + 255) / 256, tail);
-  gemm_tc_fixup_kernel<<<grid, 256, 0, st>>>(workspace, ep, 2 * BM, BN, pl.sc.dp_tiles, pl.sc.tail_parts, pl.tiles_m,
-                                             pl.tiles_n);
-  return cudaGetLastError();
+  return launch_pdl(gemm_tc_fixup_kernel, grid, dim3(256), 0, st, 1, workspace, ep, 2 * BM, BN, pl.sc.dp_tiles, pl.sc.tail_parts,
+                    pl.tiles_m, pl.tiles_n);
 }
 
 }  // namespace

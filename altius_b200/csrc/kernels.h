@@ -116,6 +116,7 @@ struct LayerNormParams {
   float eps;
   int gelu;
   int residual_first;
+  bool constants;          // pre_bias, gamma and beta are constants of the graph
 };
 cudaError_t launch_layer_norm(const LayerNormParams& p, cudaStream_t st);
 
@@ -176,7 +177,7 @@ cudaError_t launch_im2col(const ConvParams& p, const float* x, float* col, cudaS
 cudaError_t launch_patchify(const ConvParams& p, const float* x, float* rows, cudaStream_t st);
 // Depthwise (group == c == oc) stencil with bias and activation fused.
 cudaError_t launch_depthwise_conv(const ConvParams& p, const float* x, const float* w,
-                                  const float* bias, float* out, cudaStream_t st);
+                                  const float* bias, float* out, bool constants, cudaStream_t st);
 
 // Small convolutions (group 1) on the CUDA cores without a column buffer (conv_simt.cu). `wt` is the
 // filter matrix transposed by launch_pack_filter: [k][conv_simt_ldw(oc)]. `gate`: [n][c] factors of

@@ -1199,19 +1199,20 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
   const int64_t kdim = (int64_t)icg * p.kh * p.kw;
   const double flops = 2.0 * p.n * p.oc * ohw * kdim;
 
+  // What the kernels may read while the one in front still runs.
+  const bool constants = em.c.val(w).is_const && (bias < 0 || em.c.val(bias).is_const);
+
   if (p.group == p.c && icg == 1 && ocg == 1 && ep.residual < 0) {  // depthwise stencil
     const double bytes = f32_bytes(xv) + f32_bytes(wv) + f32_bytes(ov);
     em.add("conv_depthwise", n.op, {x, w, bias}, {out}, bytes, flops, [=](cudaStream_t st) {
       return launch_depthwise_conv(p, s->fptr(x), s->fptr(w), bias >= 0 ? s->fptr(bias) : nullptr,
-                                   s->fptr_mut(out), st);
+                                   s->fptr_mut(out), constants, st);
     });
     return;
   }
   // GEMM form: out[n] (ocg x ohw) = W_g (ocg x k) * col[n, g] (k x ohw), bias per row.
   const bool pointwise = p.kh == 1 && p.kw == 1 && p.sh == 1 && p.sw == 1 && p.pad_t == 0 &&
                          p.pad_l == 0 && pads[2] == 0 && pads[3] == 0;
-  // What the kernels may read while the one in front still runs.
-  const bool constants = em.c.val(w).is_const && (bias < 0 || em.c.val(bias).is_const);
   if (tensor_conv_applies(*s, flops) && !(pointwise && ohw == 1) && conv_tc_supported(p)) {
     const int wt = new_value(em.c, conv_tc_filter_elems(p), em.c.val(w).is_const);
     em.add("filter_pack", n.op, {w}, {wt}, 4.0 * p.oc * kdim * 3, 0,
@@ -1661,6 +1662,7 @@ void lower_node(Emit& em, Plan& plan, int nid) {
         p.out16_lo = o16_lo >= 0 ? s->ptr(o16_lo) : nullptr;
         p.err_word = s->err_word;
         p.rows = rows; p.len = len; p.eps = eps; p.gelu = gelu;
+        p.constants = s->values[gamma].is_const && s->values[beta].is_const && (pb < 0 || s->values[pb].is_const);
         return launch_layer_norm(p, st);
       });
       return;

@@ -10,6 +10,7 @@
 #include <cstdlib>
 
 #include "kernels.h"
+#include "pdl.cuh"
 #include "ref_math.cuh"
 #include "tc_common.cuh"
 
@@ -161,7 +162,7 @@ struct LnDev {
 };
 
 __device__ __forceinline__ float ln_prologue(const LnDev& p, float v, int col, float res) {
-  if (p.pre_bias) v = __fadd_rn(v, __ldg(p.pre_bias + col));
+  if (p.pre_bias) v = __fadd_rn(v, ld_plain(p.pre_bias + col));
   if (p.gelu) v = gelu_ref(v);
   if (p.residual) v = __fadd_rn(v, res);
   return v;
@@ -180,8 +181,8 @@ __device__ __forceinline__ void ln_load_row(const LnDev& p, int64_t row, int lan
   for (int i = 0; i < NV; ++i) {
     const int c = lane + 32 * i;
     if (c < nvec) {
-      v[i] = __ldg(xr + c);
-      if (FUSED && rr) r[i] = __ldg(rr + c);
+      v[i] = ld_plain(xr + c);
+      if (FUSED && rr) r[i] = ld_plain(rr + c);
     }
   }
 }
@@ -199,6 +200,8 @@ __device__ __forceinline__ void ln_load_row(const LnDev& p, int64_t row, int lan
 // of resident blocks).
 template <int NV, bool FUSED, bool GELU, bool SPLIT, int RESX, bool PF = (!FUSED || RESX == 2)>
 __global__ void __launch_bounds__(kThreads, FUSED ? (RESX == 1 ? 4 : 3) : (PF ? 2 : 4)) layer_norm_vec(LnDev p) {
+  pdl_trigger();
+  pdl_wait();
   constexpr bool PREFETCH = PF;
   float seen_max = 0.f;           // largest magnitude written as fixed-scale halves
   const int lane = threadIdx.x & 31;
@@ -540,6 +543,8 @@ cudaError_t launch_layer_norm(const LayerNormParams& q, cudaStream_t st) {
   if (vec) {
     const int nv = (int)((q.len / 4 + 31) / 32);
     const bool fused = q.pre_bias || q.residual || q.gelu || q.sum_out;
+    const int overlap = q.constants ? 1 : 0;   // scale and shift are read through the read-only path
+    cudaError_t le = cudaSuccess;
     // Two blocks of 8 warps per SM: several rows per warp, so the prefetch of the next
     // row overlaps the stores of the current one.
     // The residual is the chain's own input (x + f(x)): variant 1 or 2 (debug toggle
@@ -556,13 +561,13 @@ cudaError_t launch_layer_norm(const LayerNormParams& q, cudaStream_t st) {
     const unsigned vblocks = blocks64 > vcap ? (unsigned)vcap : (unsigned)blocks64;
 #define AC_LN2(NVV, SP)                                                                     \
   do {                                                                                     \
-    if (fused && q.gelu && resx == 1) layer_norm_vec<NVV, true, true, SP, 1><<<vblocks, kThreads, 0, st>>>(p);  \
-    else if (fused && q.gelu && resx == 2) layer_norm_vec<NVV, true, true, SP, 2><<<vblocks, kThreads, 0, st>>>(p);  \
-    else if (fused && q.gelu) layer_norm_vec<NVV, true, true, SP, 0><<<vblocks, kThreads, 0, st>>>(p);  \
-    else if (fused && resx) layer_norm_vec<NVV, true, false, SP, 1><<<vblocks, kThreads, 0, st>>>(p);   \
-    else if (fused) layer_norm_vec<NVV, true, false, SP, 0><<<vblocks, kThreads, 0, st>>>(p);      \
-    else if (plain_pf) layer_norm_vec<NVV, false, false, SP, 0, true><<<vblocks, kThreads, 0, st>>>(p);     \
-    else layer_norm_vec<NVV, false, false, SP, 0, false><<<vblocks, kThreads, 0, st>>>(p);             \
+    if (fused && q.gelu && resx == 1) le = launch_pdl(layer_norm_vec<NVV, true, true, SP, 1>, dim3((unsigned)vblocks), dim3(kThreads), 0, st, overlap, p);  \
+    else if (fused && q.gelu && resx == 2) le = launch_pdl(layer_norm_vec<NVV, true, true, SP, 2>, dim3((unsigned)vblocks), dim3(kThreads), 0, st, overlap, p);  \
+    else if (fused && q.gelu) le = launch_pdl(layer_norm_vec<NVV, true, true, SP, 0>, dim3((unsigned)vblocks), dim3(kThreads), 0, st, overlap, p);  \
+    else if (fused && resx) le = launch_pdl(layer_norm_vec<NVV, true, false, SP, 1>, dim3((unsigned)vblocks), dim3(kThreads), 0, st, overlap, p);   \
+    else if (fused) le = launch_pdl(layer_norm_vec<NVV, true, false, SP, 0>, dim3((unsigned)vblocks), dim3(kThreads), 0, st, overlap, p);      \
+    else if (plain_pf) le = launch_pdl(layer_norm_vec<NVV, false, false, SP, 0, true>, dim3((unsigned)vblocks), dim3(kThreads), 0, st, overlap, p);     \
+    else le = launch_pdl(layer_norm_vec<NVV, false, false, SP, 0, false>, dim3((unsigned)vblocks), dim3(kThreads), 0, st, overlap, p);             \
   } while (0)
 #define AC_LN(NVV)                                                                         \
   do {                                                                                     \
@@ -577,6 +582,7 @@ cudaError_t launch_layer_norm(const LayerNormParams& q, cudaStream_t st) {
     else AC_LN(8);
 #undef AC_LN
 #undef AC_LN2
+    return le;
   } else {
     layer_norm_generic<<<blocks, kThreads, 0, st>>>(p);
   }

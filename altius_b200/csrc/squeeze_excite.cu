@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kThreads) squeeze_excite_kernel(const SqueezeE
       const float u = warp_sum(acc[g]);
       if (quarter == g) v = u;
     }
-    if (p.b1) v = __fadd_rn(v, __ldg(p.b1 + j));
+    if (p.b1) v = __fadd_rn(v, ld_plain(p.b1 + j));
     v = apply_act(p.act1, v, p.alpha1, p.beta1);
     if (quarter < G) cl.map_shared_rank(hid, sub)[quarter * s + j] = v;
   }
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kThreads) squeeze_excite_kernel(const SqueezeE
       if (sub == g) v = u;
     }
     if (ch < c1 && sub < G && n0 + sub < p.n) {
-      if (p.b2) v = __fadd_rn(v, __ldg(p.b2 + ch));
+      if (p.b2) v = __fadd_rn(v, ld_plain(p.b2 + ch));
       p.gate[(long long)(n0 + sub) * c + ch] = apply_act(p.act2, v, p.alpha2, p.beta2);
     }
   }
