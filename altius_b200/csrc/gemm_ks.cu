@@ -98,58 +98,20 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   if (warp == kTmaWarp && lane == 0)
     for (int it = 0; it < S && it < kbs; ++it) load_b(it);   // constants: ahead of pdl_wait
   __syncwarp();
-  pdl_wait();
-  if (parts > 1) cl.barrier_wait();           // every block of the cluster runs
-
-  if (warp == kTmaWarp) {
-    if (lane == 0) {
-      for (int it = 0; it < kbs; ++it) {
-        if (it >= S) {
-          if (!mbar_wait(&empty[it % S], (uint32_t)((it / S) & 1) ^ 1)) {
-            atomicExch(p.err, 61);
-            for (int s = 0; s < S; ++s) (void)mbar_wait(&full[s], (uint32_t)((it - 1) / S) & 1);   // copies in flight land
-            break;
-          }
-          load_b(it);
-        }
-        load_a(it);
-      }
-    }
-  } else if (warp == kMmaWarp) {
-    if (elect_one()) {
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-      for (int it = 0; it < kbs; ++it) {
-        const int s = it % S;
-        if (!mbar_wait(&full[s], (uint32_t)(it / S) & 1)) { atomicExch(p.err, 62); break; }
-        tc_fence_after();
-        const uint32_t a = smem_u32(smem + s * stage_bytes);
-        const uint64_t da = desc_sw128(a), dal = desc_sw128(a + kAHalf);
-        const uint64_t db = desc_sw128(a + 2 * kAHalf), dbl = desc_sw128(a + 2 * kAHalf + bhalf);
-        // Always four steps (what lies beyond K arrives as zeros): with a run-time count an instruction
-        // took 113 clocks to issue, unrolled 57 (96 columns).
-#pragma unroll
-        for (int kk = 0; kk < KB / 16; ++kk) {
-          const uint64_t off = (uint64_t)(kk * 32 >> 4);
-          tc_mma_f16(tmem, dal + off, db + off, idesc, (it > 0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
-          tc_mma_f16(tmem, da + off, dbl + off, idesc, 1u);                             // a_hi * b_lo
-          tc_mma_f16(tmem, da + off, db + off, idesc, 1u);                              // a_hi * b_hi
-        }
-        tc_commit(&empty[s]);
-      }
-      tc_commit(&acc_full);
-    }
-  }
   // ---- accumulator -> the blocks that finish its columns -> this block's columns of the tile ----
   // Columns are handled in float4s: `quads` of them per row and block, float4 q of row r of rank s at
   // [(s * quads + q) * (BM + 1) + r]: a warp's rows are neighbours when they are sent (512 bytes a
   // store) and its columns lie in different banks when they are read.
   const int quads = share / 4, total = BM * quads;
+  int live = 0;                                // of them this thread's block has to finish: none in the first pass
   constexpr int CH = 4;                        // float4s a thread has in work at once
   float4 rs[CH], bi[CH];
+#pragma unroll
+  for (int i = 0; i < CH; ++i) rs[i] = bi[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   auto place = [&](int e, int* row, int* q) {
     *row = (int)(((unsigned)e * (unsigned)p.inv) >> 20);
     *q = e - *row * quads;
-    return e < total && m0 + *row < p.m && n0 + rank * share + 4 * *q < p.n;   // n % 4 == 0: the four columns exist together
+    return e < live && m0 + *row < p.m && n0 + rank * share + 4 * *q < p.n;   // n % 4 == 0: the four columns exist together
   };
   auto fetch = [&](int e0) {
 #pragma unroll
@@ -162,49 +124,19 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       if (p.bias) bi[i] = ld_plain(reinterpret_cast<const float4*>(p.bias + col));
     }
   };
-  if (warp < 8) {
-    fetch(tid);                                // under the products
-    if (!warp_mbar_wait(&acc_full, 0, lane)) atomicExch(p.err, 63);
-    tc_fence_after();
-    const int row = (warp & 3) * 32 + lane;
-    const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    for (int c = (warp >> 2) * 16; c < bn; c += 64) {
-      uint32_t u[2][16];
-      const bool two = c + 32 < bn;
-      tc_ld_32x16_nowait(base + (uint32_t)c, u[0]);
-      if (two) tc_ld_32x16_nowait(base + (uint32_t)(c + 32), u[1]);
-      tc_wait_ld();
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (h == 1 && !two) break;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int cq = c / 4 + 8 * h + i, owner = (int)(((unsigned)cq * (unsigned)p.inv) >> 20);
-          float4* dst = part + ((rank * quads + cq - owner * quads) * (BM + 1) + row);
-          if (parts > 1) dst = cl.map_shared_rank(dst, owner);
-          *dst = make_float4(__uint_as_float(u[h][4 * i]), __uint_as_float(u[h][4 * i + 1]), __uint_as_float(u[h][4 * i + 2]),
-                             __uint_as_float(u[h][4 * i + 3]));
-        }
-      }
-    }
-    tc_fence_before();
-  }
-  __syncwarp();
-  if (parts > 1) cl.sync();
-  else __syncthreads();
-
-  if (warp < 8) {
-    const float sc = p.acc_scale ? __fmul_rn(ld_plain(p.acc_scale), kFixedUnscale) : kFixedUnscale;
+  const float sc = p.acc_scale ? __fmul_rn(ld_plain(p.acc_scale), kFixedUnscale) : kFixedUnscale;   // prepared with B: a constant
+  auto finish = [&] {
     float most = 0.f;
-    for (int e0 = tid; e0 < total; e0 += CH * kEpiThreads) {
+    for (int e0 = tid; e0 < max(live, kEpiThreads); e0 += CH * kEpiThreads) {
       if (e0 != tid) fetch(e0);
       float4 x[CH];
 #pragma unroll
       for (int i = 0; i < CH; ++i) {
         const int e = e0 + i * kEpiThreads;
         int row, q;
-        const bool ok = place(e, &row, &q);
-        const float4* src = part + (ok ? q * (BM + 1) + row : 0);
+        x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!place(e, &row, &q)) continue;
+        const float4* src = part + q * (BM + 1) + row;
         x[i] = src[0];
         for (int s = 1; s < parts; ++s) {
           const float4 u = src[s * quads * (BM + 1)];
@@ -243,10 +175,93 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
         }
       }
     }
-    if (p.c16_hi) {
+    if (p.c16_hi && live > 0) {
       const unsigned all = __reduce_or_sync(0xffffffffu, split_seen_fixed_of_max(most));
       if (lane == 0) atomicOr(&seen, all);
     }
+  };
+  auto produce = [&] {
+    pdl_wait();
+    if (parts > 1) cl.barrier_wait();           // every block of the cluster runs
+
+    if (warp == kTmaWarp) {
+      if (lane == 0) {
+        for (int it = 0; it < kbs; ++it) {
+          if (it >= S) {
+            if (!mbar_wait(&empty[it % S], (uint32_t)((it / S) & 1) ^ 1)) {
+              atomicExch(p.err, 61);
+              for (int s = 0; s < S; ++s) (void)mbar_wait(&full[s], (uint32_t)((it - 1) / S) & 1);   // copies in flight land
+              break;
+            }
+            load_b(it);
+          }
+          load_a(it);
+        }
+      }
+    } else if (warp == kMmaWarp) {
+      if (elect_one()) {
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        for (int it = 0; it < kbs; ++it) {
+          const int s = it % S;
+          if (!mbar_wait(&full[s], (uint32_t)(it / S) & 1)) { atomicExch(p.err, 62); break; }
+          tc_fence_after();
+          const uint32_t a = smem_u32(smem + s * stage_bytes);
+          const uint64_t da = desc_sw128(a), dal = desc_sw128(a + kAHalf);
+          const uint64_t db = desc_sw128(a + 2 * kAHalf), dbl = desc_sw128(a + 2 * kAHalf + bhalf);
+          // Always four steps (what lies beyond K arrives as zeros): with a run-time count an instruction
+          // took 113 clocks to issue, unrolled 57 (96 columns).
+#pragma unroll
+          for (int kk = 0; kk < KB / 16; ++kk) {
+            const uint64_t off = (uint64_t)(kk * 32 >> 4);
+            tc_mma_f16(tmem, dal + off, db + off, idesc, (it > 0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
+            tc_mma_f16(tmem, da + off, dbl + off, idesc, 1u);                             // a_hi * b_lo
+            tc_mma_f16(tmem, da + off, db + off, idesc, 1u);                              // a_hi * b_hi
+          }
+          tc_commit(&empty[s]);
+        }
+        tc_commit(&acc_full);
+      }
+    }
+    if (warp < 8) {
+      fetch(tid);                                // under the products
+      if (!warp_mbar_wait(&acc_full, 0, lane)) atomicExch(p.err, 63);
+      tc_fence_after();
+      const int row = (warp & 3) * 32 + lane;
+      const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+      for (int c = (warp >> 2) * 16; c < bn; c += 64) {
+        uint32_t u[2][16];
+        const bool two = c + 32 < bn;
+        tc_ld_32x16_nowait(base + (uint32_t)c, u[0]);
+        if (two) tc_ld_32x16_nowait(base + (uint32_t)(c + 32), u[1]);
+        tc_wait_ld();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (h == 1 && !two) break;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int cq = c / 4 + 8 * h + i, owner = (int)(((unsigned)cq * (unsigned)p.inv) >> 20);
+            float4* dst = part + ((rank * quads + cq - owner * quads) * (BM + 1) + row);
+            if (parts > 1) dst = cl.map_shared_rank(dst, owner);
+            *dst = make_float4(__uint_as_float(u[h][4 * i]), __uint_as_float(u[h][4 * i + 1]), __uint_as_float(u[h][4 * i + 2]),
+                               __uint_as_float(u[h][4 * i + 3]));
+          }
+        }
+      }
+      tc_fence_before();
+    }
+    __syncwarp();
+    if (parts > 1) cl.sync();
+    else __syncthreads();
+  };
+  // The first pass has nothing to finish: it brings the epilogue's code into the instruction cache while
+  // the kernel in front still runs (over cold code it took 5600 clocks for 1500 of work).
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    if (pass == 1) {
+      live = total;
+      produce();
+    }
+    if (warp < 8) finish();
   }
   __syncthreads();
   // Out of range, or nothing but tiny values in this block's 128 x share results.
