@@ -12,7 +12,7 @@
 // the result does not depend on timing; bias, activation, residual; whole-line stores). The weights
 // of the first stages are requested while the kernel in front still runs.
 //
-// Per block: warps 0-7 move the accumulator and run the epilogue, warp 8 issues TMA, warp 9 MMAs.
+// Per block: warps 0-15 move the accumulator and run the epilogue, warp 16 issues TMA, warp 17 MMAs.
 #include <cooperative_groups.h>
 #include <cuda.h>
 
@@ -31,7 +31,7 @@ namespace {
 
 using namespace tc;
 
-constexpr int BM = 128, KB = 64, kEpiThreads = 256, kTmaWarp = 8, kMmaWarp = 9, kThreads = 320, kMaxStages = 4;
+constexpr int BM = 128, KB = 64, kEpiThreads = 512, kTmaWarp = 16, kMmaWarp = 17, kThreads = 576, kMaxStages = 4;
 constexpr int kAHalf = BM * KB * 2;           // bytes of A's hi (or lo) tile
 
 struct KsDev {
@@ -104,7 +104,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   // store) and its columns lie in different banks when they are read.
   const int quads = share / 4, total = BM * quads;
   int live = 0;                                // of them this thread's block has to finish: none in the first pass
-  constexpr int CH = 4;                        // float4s a thread has in work at once
+  constexpr int CH = 3;                        // float4s a thread has in work at once
   float4 rs[CH], bi[CH];
 #pragma unroll
   for (int i = 0; i < CH; ++i) rs[i] = bi[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -222,29 +222,23 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
         tc_commit(&acc_full);
       }
     }
-    if (warp < 8) {
+    if (warp < kEpiThreads / 32) {
       fetch(tid);                                // under the products
       if (!warp_mbar_wait(&acc_full, 0, lane)) atomicExch(p.err, 63);
       tc_fence_after();
       const int row = (warp & 3) * 32 + lane;
       const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
       for (int c = (warp >> 2) * 16; c < bn; c += 64) {
-        uint32_t u[2][16];
-        const bool two = c + 32 < bn;
-        tc_ld_32x16_nowait(base + (uint32_t)c, u[0]);
-        if (two) tc_ld_32x16_nowait(base + (uint32_t)(c + 32), u[1]);
+        uint32_t u[16];
+        tc_ld_32x16_nowait(base + (uint32_t)c, u);
         tc_wait_ld();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (h == 1 && !two) break;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int cq = c / 4 + 8 * h + i, owner = (int)(((unsigned)cq * (unsigned)p.inv) >> 20);
-            float4* dst = part + ((rank * quads + cq - owner * quads) * (BM + 1) + row);
-            if (parts > 1) dst = cl.map_shared_rank(dst, owner);
-            *dst = make_float4(__uint_as_float(u[h][4 * i]), __uint_as_float(u[h][4 * i + 1]), __uint_as_float(u[h][4 * i + 2]),
-                               __uint_as_float(u[h][4 * i + 3]));
-          }
+        for (int i = 0; i < 4; ++i) {
+          const int cq = c / 4 + i, owner = (int)(((unsigned)cq * (unsigned)p.inv) >> 20);
+          float4* dst = part + ((rank * quads + cq - owner * quads) * (BM + 1) + row);
+          if (parts > 1) dst = cl.map_shared_rank(dst, owner);
+          *dst = make_float4(__uint_as_float(u[4 * i]), __uint_as_float(u[4 * i + 1]), __uint_as_float(u[4 * i + 2]),
+                             __uint_as_float(u[4 * i + 3]));
         }
       }
       tc_fence_before();
@@ -261,7 +255,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       live = total;
       produce();
     }
-    if (warp < 8) finish();
+    if (warp < kEpiThreads / 32) finish();
   }
   __syncthreads();
   // Out of range, or nothing but tiny values in this block's 128 x share results.
@@ -280,9 +274,9 @@ struct Shape {
   double clocks = 1e30;
 };
 
-// Tile width and K split by clocks: a K-block costs its twelve MMAs (about 110 clocks each up to 128
-// columns) or its bytes at 28 a clock, whichever is more; start, first loads, exchange and epilogue
-// about 5000 (and 250 per block of a cluster).
+// Tile width and K split by clocks, from stamps in the kernel: a K-block costs its twelve MMAs (45 to 65 clocks
+// each) or its bytes at 60 a clock, whichever is more; first loads and drain 2700; exchange 1600 and 18
+// per column; epilogue 1500 and 40 per column that a block finishes.
 Shape pick_shape(int64_t m, int64_t n, int64_t k, int sms) {
   Shape best;
   const int nkb = (int)((k + KB - 1) / KB);
@@ -296,8 +290,8 @@ Shape pick_shape(int64_t m, int64_t n, int64_t k, int sms) {
       const int stages = (int)std::min<size_t>(std::min(kper, kMaxStages), (kSmemMax - 1024 - ex) / stage);
       if (stages < std::min(2, kper)) continue;
       const double ctas = (double)mt * ((n + bn - 1) / bn) * split, waves = std::ceil(ctas / sms);
-      const double kb = std::max(12 * 110.0, (double)stage / 28.0);
-      const double t = waves * (kper * kb + 5000.0 + 250.0 * split + 10.0 * bn);
+      const double kb = std::max(12 * (32.0 + 0.26 * bn), (double)stage / 60.0);
+      const double t = waves * (kper * kb + 4200.0 + (split > 1 ? 1600.0 + 18.0 * bn : 0.0) + 40.0 * bn / split);
       if (t < best.clocks) {
         best.bn = bn; best.split = split; best.kper = kper; best.stages = stages; best.inv = ((1 << 20) + quads - 1) / quads;
         best.smem = stages * stage + ex + 1024;
