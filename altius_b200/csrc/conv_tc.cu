@@ -455,9 +455,8 @@ Shape pick_shape(const ConvParams& q, int sms) {
     for (int split = 1; split <= 8; split *= 2) {
       const int kper = (nkb + split - 1) / split;
       if ((split - 1) * kper >= nkb) continue;
-      const double ctas = (double)px * tiles * split;
       const double step = std::max(420.0, 12 * std::max(65.0, 0.8 * bn) * std::min(1.0, k / 32.0));
-      const double body = kper * step + 4.0 * bn, waves = std::ceil(ctas / sms);
+      const double body = kper * step + 4.0 * bn, waves = std::ceil((double)px * tiles / cluster_slots(split));
       const double t = waves * body + 2500 + (split > 1 ? 1500 : 0);
       if (t < best_t * 0.98) { best_t = t; best.bn = bn; best.tiles = tiles; best.split = split; best.kper = kper; }
     }

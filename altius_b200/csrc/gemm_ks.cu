@@ -17,6 +17,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "kernels.h"
 #include "pdl.cuh"
@@ -274,10 +275,43 @@ struct Shape {
   double clocks = 1e30;
 };
 
+}  // namespace
+
+// The parts of the chip that hold a cluster have 14 to 18 SMs each, so fewer blocks run at once than there
+// are SMs: 36 clusters of four took two rounds (18 us for 197 x 768 x 2304), 24 one.
+int cluster_slots(int split) {
+  if (split <= 1) return device_sm_count();
+  static std::atomic<int> known[64][4];
+  const int at = split <= 2 ? 1 : split <= 4 ? 2 : 3;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  if (const int v = known[dev][at].load(std::memory_order_relaxed)) return v;
+  static unsigned long long done = 0;
+  int slots = 0;
+  if (ensure_dynamic_smem(gemm_ks_kernel<ACT_NONE>, (int)kSmemMax, &done) == cudaSuccess) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(1, (unsigned)device_sm_count(), (unsigned)split);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemMax;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = (unsigned)split;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&slots, gemm_ks_kernel<ACT_NONE>, &cfg) != cudaSuccess) slots = 0;
+  }
+  (void)cudaGetLastError();
+  if (slots <= 0) slots = std::max(1, device_sm_count() * 7 / 8 / split);
+  known[dev][at].store(slots, std::memory_order_relaxed);
+  return slots;
+}
+
+namespace {
+
 // Tile width and K split by clocks, from stamps in the kernel: a K-block costs its twelve MMAs (45 to 65 clocks
 // each) or its bytes at 60 a clock, whichever is more; first loads and drain 2700; exchange 1600 and 18
 // per column; epilogue 1500 and 40 per column that a block finishes.
-Shape pick_shape(int64_t m, int64_t n, int64_t k, int sms) {
+Shape pick_shape(int64_t m, int64_t n, int64_t k) {
   Shape best;
   const int nkb = (int)((k + KB - 1) / KB);
   const long long mt = (m + BM - 1) / BM;
@@ -289,7 +323,7 @@ Shape pick_shape(int64_t m, int64_t n, int64_t k, int sms) {
       const size_t stage = 2 * (size_t)kAHalf + (size_t)bn * KB * 4, ex = (size_t)split * quads * (BM + 1) * 16;
       const int stages = (int)std::min<size_t>(std::min(kper, kMaxStages), (kSmemMax - 1024 - ex) / stage);
       if (stages < std::min(2, kper)) continue;
-      const double ctas = (double)mt * ((n + bn - 1) / bn) * split, waves = std::ceil(ctas / sms);
+      const double waves = std::ceil((double)mt * ((n + bn - 1) / bn) / cluster_slots(split));
       const double kb = std::max(12 * (32.0 + 0.26 * bn), (double)stage / 60.0);
       const double t = waves * (kper * kb + 4200.0 + (split > 1 ? 1600.0 + 18.0 * bn : 0.0) + 40.0 * bn / split);
       if (t < best.clocks) {
@@ -317,7 +351,7 @@ inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) =
 
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k) {
   if (m < 1 || n < 4 || (n % 4) || k < 64 || (k % 8) || m > (1 << 20) || n > (1 << 20)) return 1e30;
-  return pick_shape(m, n, k, device_sm_count()).clocks;
+  return pick_shape(m, n, k).clocks;
 }
 
 bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bias_scale) {
@@ -330,7 +364,7 @@ cudaError_t launch_gemm_ks(const GemmParams& q, int* err_word, cudaStream_t st) 
       (q.c && (!al16(q.c) || (q.ldc % 4))) || (q.residual && (!al16(q.residual) || (q.ld_res % 4))) || (q.bias_n && !al16(q.bias_n)) ||
       (q.c16_hi && (q.ldc16 % 4)) || !gemm_ks_epilogue_ok(q.act, q.bias_m != nullptr, q.beta != 0.f && q.c_in, q.alpha, q.bias_scale))
     return cudaErrorInvalidValue;
-  const Shape sh = pick_shape(q.m, q.n, q.k, device_sm_count());
+  const Shape sh = pick_shape(q.m, q.n, q.k);
   KsDev d{};
   d.m = (int)q.m; d.n = (int)q.n; d.k = (int)q.k;
   d.bn = sh.bn; d.stages = sh.stages; d.kper = sh.kper; d.inv = sh.inv;
