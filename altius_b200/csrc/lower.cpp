@@ -123,15 +123,19 @@ bool on_device(const AcSession& s) { return !s.opt.plan_only; }
 // gemm_mode 1 promises exact ascending chains and 2 its own precision: both keep their kernels.
 bool fp32_level_mode(const AcSession& s) { return s.opt.gemm_mode == 0 || s.opt.gemm_mode == 3; }
 
-// Convolutions below the size from which the tensor cores take them (2^23 operations) run on the
-// small-convolution kernel: at 28 K products per SM or fewer they are bound by latency.
-constexpr double kTensorConvFloor = double(1 << 23);
-bool small_conv_applies(const AcSession& s, double flops) {
-  return on_device(s) && fp32_level_mode(s) && flops < kTensorConvFloor;
+// Convolutions below 2^23 operations run on the CUDA-core kernel, and up to 2^25 those with few pixels, whose tiles
+// of 128 leave the tensor-core kernel a few blocks in clusters: at 110 K products per SM they are
+// bound by latency (49 pixels, 160 x 960: 7.4 us against 11.6; 196 pixels, 672 x 112: 9.6 against 14.4;
+// but 12544 pixels, 16 x 64: 8.0 against 5.8).
+bool tensor_size(double flops, int64_t columns) {
+  return flops >= double(1 << 23) && (flops >= double(1 << 25) || columns > 8192);
+}
+bool small_conv_applies(const AcSession& s, double flops, int64_t columns) {
+  return on_device(s) && fp32_level_mode(s) && !tensor_size(flops, columns);
 }
 // The larger ones on the tensor-core kernel that reads the planes itself.
-bool tensor_conv_applies(const AcSession& s, double flops) {
-  return on_device(s) && fp32_level_mode(s) && flops >= kTensorConvFloor;
+bool tensor_conv_applies(const AcSession& s, double flops, int64_t columns) {
+  return on_device(s) && fp32_level_mode(s) && tensor_size(flops, columns);
 }
 
 // Recognises `hs = HardSigmoid(t); m = Mul(t, hs)` hanging off value t whose only
@@ -552,7 +556,7 @@ void detect_se_gate(Ctx& c, Plan& plan) {
     const bool gelu = plan.epi.count(cn) && plan.epi[cn].act == ACT_GELU;
     const bool direct = on_device(c.s) && fp32_level_mode(c.s) && ch <= 4096 && ov.dims[1] <= 16384 && !gelu &&
                         xv.numel() < (1ll << 30);
-    const bool tensor = (hw % 4) == 0 && (ch % 4) == 0 && ch >= 8 && flops >= kTensorConvFloor;
+    const bool tensor = (hw % 4) == 0 && (ch % 4) == 0 && ch >= 8 && flops >= double(1 << 23);
     if (!pointwise || !nopad || !(tensor || direct) ||
         xv.dims[0] > 65535 || !c.val(conv.inputs[1]).is_const)
       continue;
@@ -1213,7 +1217,7 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
   // GEMM form: out[n] (ocg x ohw) = W_g (ocg x k) * col[n, g] (k x ohw), bias per row.
   const bool pointwise = p.kh == 1 && p.kw == 1 && p.sh == 1 && p.sw == 1 && p.pad_t == 0 &&
                          p.pad_l == 0 && pads[2] == 0 && pads[3] == 0;
-  if (tensor_conv_applies(*s, flops) && !(pointwise && ohw == 1) && conv_tc_supported(p)) {
+  if (tensor_conv_applies(*s, flops, p.n * ohw) && !(pointwise && ohw == 1) && conv_tc_supported(p)) {
     const int wt = new_value(em.c, conv_tc_filter_elems(p), em.c.val(w).is_const);
     em.add("filter_pack", n.op, {w}, {wt}, 4.0 * p.oc * kdim * 3, 0,
            [=](cudaStream_t st) { return launch_pack_filter_tc(p, s->fptr(w), s->fptr_mut(wt), st); });
@@ -1225,7 +1229,7 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
     });
     return;
   }
-  if (small_conv_applies(*s, flops) && !(pointwise && ohw == 1) && conv_simt_supported(p)) {
+  if (small_conv_applies(*s, flops, p.n * ohw) && !(pointwise && ohw == 1) && conv_simt_supported(p)) {
     const int wt = new_value(em.c, conv_simt_ldw(p.oc) * kdim, em.c.val(w).is_const);
     const int64_t oc = p.oc, kd = kdim;
     em.add("filter_pack", n.op, {w}, {wt}, 8.0 * oc * kd, 0,

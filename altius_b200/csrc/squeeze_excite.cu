@@ -6,8 +6,7 @@
 // latency: a cluster of eight blocks shares one to four images; every block pools its eighth of the
 // channels and leaves the means in the shared memory of all eight, computes an eighth of the hidden
 // units from them and exchanges those in the same way, then finishes its eighth of the gate.
-// Several images per cluster (from a batch of 17 on, when the clusters of one image no longer fit
-// the SMs at once) read the weights once for all of them.
+// Several images per cluster (when the clusters of one image no longer fit the SMs at once) read the weights once for all of them.
 #include <cooperative_groups.h>
 
 #include "kernels.h"
@@ -175,7 +174,9 @@ bool squeeze_excite_supported(const SqueezeExciteParams& p) {
 
 cudaError_t launch_squeeze_excite(const SqueezeExciteParams& p, cudaStream_t st) {
   if (!squeeze_excite_supported(p) || !al16(p.w1) || !al16(p.w2)) return cudaErrorInvalidValue;
-  const int per_wave = 16;            // clusters of eight that run at once: two in each part of the chip that can hold one
+  // Clusters that run at once (a block of 1024 threads fills an SM). One more takes a second round: 32 images
+  // as 16 clusters of two 19 to 26 us, as 8 clusters of four 12 to 21.
+  const int per_wave = cluster_slots(kCluster);
   if (p.n <= per_wave) return launch_g<1>(p, st);
   return p.n <= 2 * per_wave ? launch_g<2>(p, st) : launch_g<4>(p, st);
 }

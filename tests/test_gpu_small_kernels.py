@@ -102,9 +102,9 @@ def test_product_of_a_few_rows(cuda_lib, m, k, n):
 # Channel counts off the 16s, K off the 8s and 32s, planes of odd size, K cut over a cluster of
 # eight, several channel tiles, windows, a gate; residual and bias always.
 @pytest.mark.parametrize("n,c,h,oc,k,s,p,gate", [
-    (3, 21, 57, 27, 1, 1, 0, True), (2, 960, 7, 160, 1, 1, 0, True), (1, 672, 14, 112, 1, 1, 0, False),
-    (5, 40, 28, 241, 1, 1, 0, False), (2, 3, 97, 33, 3, 2, 1, False), (1, 72, 14, 80, 5, 1, 2, False),
-    (2, 1, 512, 16, 1, 1, 0, True), (1, 4096, 5, 300, 1, 1, 0, False), (32, 16, 40, 64, 1, 1, 0, False)])
+    (10, 21, 57, 27, 1, 1, 0, True), (3, 960, 7, 160, 1, 1, 0, True), (2, 672, 14, 112, 1, 1, 0, False),
+    (5, 40, 28, 241, 1, 1, 0, False), (8, 3, 97, 33, 3, 2, 1, False), (1, 72, 14, 80, 5, 1, 2, False),
+    (5, 1, 512, 16, 1, 1, 0, True), (1, 4096, 5, 300, 1, 1, 0, False), (32, 16, 40, 64, 1, 1, 0, False)])
 def test_tensor_core_convolution(cuda_lib, n, c, h, oc, k, s, p, gate):
     rng = np.random.default_rng(c * h + oc)
     x = rng.standard_normal((n, c, h, h)).astype(np.float32)
@@ -123,6 +123,21 @@ def test_tensor_core_convolution(cuda_lib, n, c, h, oc, k, s, p, gate):
     want = torch.relu(conv(xg, torch.from_numpy(w).double(), torch.from_numpy(b).double())).numpy() + r
     mass = conv(xg.abs(), torch.from_numpy(w).double().abs(), torch.from_numpy(b).double().abs()).numpy() + np.abs(r)
     assert (np.abs(got - want) <= 1e-5 * np.abs(want) + 5e-6 * mass).all()
+
+
+# Rows of whole float4s with the paddings of the vector form, other paddings and rows, results whose rows are not
+# whole float4s, planes smaller than the filter. K * K + 2 roundings of terms bounded by the sum of magnitudes.
+@pytest.mark.parametrize("n,c,h,w,k,s,p", [
+    (2, 5, 28, 28, 3, 1, 1), (1, 7, 56, 112, 3, 2, 1), (2, 3, 16, 20, 5, 1, 2), (3, 4, 28, 28, 5, 2, 2), (1, 9, 12, 8, 3, 1, 0),
+    (1, 3, 9, 4, 5, 2, 1), (2, 3, 14, 14, 3, 1, 1), (1, 2, 6, 12, 3, 2, 0), (1, 2, 8, 8, 3, 1, 2), (1, 3, 1, 4, 3, 1, 1)])
+def test_depthwise_convolution(cuda_lib, n, c, h, w, k, s, p):
+    rng = np.random.default_rng(h * w + k)
+    x, f, b = (rng.standard_normal(d).astype(np.float32) for d in ((n, c, h, w), (c, 1, k, k), (c,)))
+    got = _run(lambda g, xi: g.op("ReLU", g.op("Conv2d", xi, g.new_init(f), g.new_init(b), kernel_shape=[k, k], strides=[s, s],
+                                               padding=[p] * 4, dilations=[1, 1], group=c, auto_pad="")), [x], ["conv_depthwise"])
+    conv = lambda a, q, r: torch.nn.functional.conv2d(torch.from_numpy(a).double(), torch.from_numpy(q).double(),
+                                                      torch.from_numpy(r).double(), stride=s, padding=p, groups=c).numpy()
+    assert (np.abs(got - np.maximum(conv(x, f, b), 0)) <= (k * k + 2) * EPS * conv(np.abs(x), np.abs(f), np.abs(b))).all()
 
 
 # Filter and bias computed by the steps in front: nothing of them may be read before these have finished.
