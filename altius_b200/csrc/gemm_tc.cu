@@ -1656,9 +1656,6 @@ int pair_count() {
   return n;
 }
 
-// The kernel that adds up a tail's K slices: 5.7 to 12.9 us (33 to 66 tiles of 128 x 256).
-constexpr double kFixupClocks = 10000.0;
-
 // Tile shape by a cost model in SM clocks, fitted to measurements: TMA fills shared
 // memory at about 28 bytes per clock per SM (8 TB/s over the chip, the L2 -> SM
 // limit), and an MMA of 128 x BN x 32 bytes of K takes about (4096 + 32 BN) / 64 clocks
@@ -1692,7 +1689,6 @@ TcShape pick_shape(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, 
     const int acc_cols = (f16 ? 2 : 1) * c.mt * c.bn;
     const double epi_clk = 2 * acc_cols <= 512 ? 0.0 : c.mt * c.bn * (f16 ? 24.0 : 18.0);
     double cost = rounds * (pl.sc.num_kb * std::max(mma_clk, feed_clk) + epi_clk);
-    if (pl.sc.tail_parts >= 2) cost += kFixupClocks;
     if (pl.sc.num_tiles < sms) cost += 1.0;   // ties: prefer the shape with more tiles in flight
     if (cost < best_cost - 1e-9) { best_cost = cost; best = c; }
   }
@@ -1704,8 +1700,7 @@ TcShape pick_shape(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, 
     const TcPlan pl = make_plan(m, n, k, batch, 256, 2, pkb, pairs);
     double rounds = (double)(pl.sc.dp_tiles / pairs) + (pl.sc.dp_tiles % pairs ? 1.0 : 0.0);
     if (pl.sc.tail_parts >= 2) rounds += 1.0 / pl.sc.tail_parts + 0.05;
-    const double cost = rounds * (pl.sc.num_kb * (pkb / 32) * std::max(6.0 * 128.0, 32768.0 / 28.0) + 256 * 24.0) +
-                        (pl.sc.tail_parts >= 2 ? kFixupClocks : 0.0);
+    const double cost = rounds * (pl.sc.num_kb * (pkb / 32) * std::max(6.0 * 128.0, 32768.0 / 28.0) + 256 * 24.0);
     if (cost < best_cost - 1e-9) { best_cost = cost; best = {256, 2, true}; }
   }
   return best;
