@@ -1,7 +1,10 @@
 // fp16-split GEMM for few rows (a small batch of a transformer): C = epilogue(A * B^T) with both operands
 // as fp16 halves by TMA (A on the fixed scale, written by the kernel in front; B prepared once), three
-// kind::f16 MMAs per product into one accumulator -- the operand formats of the CTA-pair kernel
-// (gemm_tc.cu), which takes the larger problems.
+// kind::f16 MMAs per product -- the operand formats of the CTA-pair kernel (gemm_tc.cu), which takes
+// the larger problems. The tensor core truncates its sum at every instruction, an error that grows with the
+// number of instructions behind one another on an accumulator of full size; so the cross terms
+// (2^-11 of the result) have an accumulator of their own and the others are dealt to three
+// (197 x 768 x 2304: relative error against 64 bits 9.8e-7 in one accumulator, 1.6e-7 this way; the pair kernel 3.5e-7).
 //
 // What bounds it: 197 rows against 768 x 2304 are 2.1 GFLOP and 7 MB of weights, 1.2 us of either, so what
 // counts is latency. On 256 x 256 tiles such a product has 9 tiles for 74 pairs; cut along K its
@@ -66,7 +69,10 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   float4* part = reinterpret_cast<float4*>(smem + S * stage_bytes);   // [parts][quads][BM + 1]
   const int nkb = (p.k + KB - 1) / KB, kb0 = rank * p.kper, kbs = min(nkb, kb0 + p.kper) - kb0;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * bn;
-  const uint32_t cols = bn <= 32 ? 32 : bn <= 64 ? 64 : 128;
+  // Accumulators: the cross terms have one of their own, the products of the high halves up to three, K-block by
+  // K-block in turn.
+  const uint32_t set = bn <= 32 ? 32 : bn <= 64 ? 64 : 128, cols = 4 * set;
+  const int mains = min(3, kbs);
   cg::cluster_group cl = cg::this_cluster();
   if (parts > 1) cl.barrier_arrive();         // answered before the first write to another block's memory
   if (tid == 0) {
@@ -75,15 +81,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
     seen = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kMmaWarp) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(cols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
-  }
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_slot;
-  pdl_trigger();
 
   auto load_b = [&](int it) {
     uint8_t* b = smem + (it % S) * stage_bytes + 2 * kAHalf;
@@ -181,14 +179,29 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       if (lane == 0) atomicOr(&seen, all);
     }
   };
+  uint32_t tmem = 0;
   auto produce = [&] {
     pdl_wait();
     if (parts > 1) cl.barrier_wait();           // every block of the cluster runs
+    // Tensor memory only now: taken earlier, it would wait for the blocks of the kernel in front that share the SM;
+    // and the next kernel may start only behind it, or its allocation could come first.
+    if (warp == kTmaWarp && lane == 0)
+      for (int it = 0; it < S && it < kbs; ++it) load_a(it);
+    __syncwarp();
+    if (warp == kMmaWarp) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(cols));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    tmem = tmem_slot;
+    pdl_trigger();
 
     if (warp == kTmaWarp) {
       if (lane == 0) {
-        for (int it = 0; it < kbs; ++it) {
-          if (it >= S) {
+        for (int it = S; it < kbs; ++it) {
+          {
             if (!mbar_wait(&empty[it % S], (uint32_t)((it / S) & 1) ^ 1)) {
               atomicExch(p.err, 61);
               for (int s = 0; s < S; ++s) (void)mbar_wait(&full[s], (uint32_t)((it - 1) / S) & 1);   // copies in flight land
@@ -211,12 +224,13 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
           const uint64_t db = desc_sw128(a + 2 * kAHalf), dbl = desc_sw128(a + 2 * kAHalf + bhalf);
           // Always four steps (what lies beyond K arrives as zeros): with a run-time count an instruction
           // took 113 clocks to issue, unrolled 57 (96 columns).
+          const uint32_t cross = tmem, main = tmem + (uint32_t)(1 + it % mains) * set;
 #pragma unroll
           for (int kk = 0; kk < KB / 16; ++kk) {
             const uint64_t off = (uint64_t)(kk * 32 >> 4);
-            tc_mma_f16(tmem, dal + off, db + off, idesc, (it > 0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
-            tc_mma_f16(tmem, da + off, dbl + off, idesc, 1u);                             // a_hi * b_lo
-            tc_mma_f16(tmem, da + off, db + off, idesc, 1u);                              // a_hi * b_hi
+            tc_mma_f16(main, da + off, db + off, idesc, (it >= mains || kk > 0) ? 1u : 0u);        // a_hi * b_hi
+            tc_mma_f16(cross, dal + off, db + off, idesc, (it > 0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
+            tc_mma_f16(cross, da + off, dbl + off, idesc, 1u);             // a_hi * b_lo
           }
           tc_commit(&empty[s]);
         }
@@ -231,8 +245,19 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
       for (int c = (warp >> 2) * 16; c < bn; c += 64) {
         uint32_t u[16];
+        uint32_t v[3][16];
         tc_ld_32x16_nowait(base + (uint32_t)c, u);
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if (a < mains) tc_ld_32x16_nowait(base + (uint32_t)c + (uint32_t)(1 + a) * set, v[a]);
         tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float x = __uint_as_float(v[0][i]);
+          if (mains > 1) x = __fadd_rn(x, __uint_as_float(v[1][i]));
+          if (mains > 2) x = __fadd_rn(x, __uint_as_float(v[2][i]));
+          u[i] = __float_as_uint(__fadd_rn(x, __uint_as_float(u[i])));
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int cq = c / 4 + i, owner = (int)(((unsigned)cq * (unsigned)p.inv) >> 20);

@@ -123,12 +123,12 @@ bool on_device(const AcSession& s) { return !s.opt.plan_only; }
 // gemm_mode 1 promises exact ascending chains and 2 its own precision: both keep their kernels.
 bool fp32_level_mode(const AcSession& s) { return s.opt.gemm_mode == 0 || s.opt.gemm_mode == 3; }
 
-// Convolutions below 2^23 operations run on the CUDA-core kernel, and up to 2^25 those with few pixels, whose tiles
+// Convolutions below 2^23 operations run on the CUDA-core kernel, and up to 2^25 the pointwise ones with few pixels, whose tiles
 // of 128 leave the tensor-core kernel a few blocks in clusters: at 110 K products per SM they are
 // bound by latency (49 pixels, 160 x 960: 7.4 us against 11.6; 196 pixels, 672 x 112: 9.6 against 14.4;
-// but 12544 pixels, 16 x 64: 8.0 against 5.8).
+// but 12544 pixels, 16 x 64: 8.0 against 5.8; up to 3136 pixels within 1 us of each other).
 bool tensor_size(double flops, int64_t columns) {
-  return flops >= double(1 << 23) && (flops >= double(1 << 25) || columns > 8192);
+  return flops >= double(1 << 23) && (flops >= double(1 << 25) || columns > 1024);
 }
 bool small_conv_applies(const AcSession& s, double flops, int64_t columns) {
   return on_device(s) && fp32_level_mode(s) && !tensor_size(flops, columns);
@@ -1217,7 +1217,8 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
   // GEMM form: out[n] (ocg x ohw) = W_g (ocg x k) * col[n, g] (k x ohw), bias per row.
   const bool pointwise = p.kh == 1 && p.kw == 1 && p.sh == 1 && p.sw == 1 && p.pad_t == 0 &&
                          p.pad_l == 0 && pads[2] == 0 && pads[3] == 0;
-  if (tensor_conv_applies(*s, flops, p.n * ohw) && !(pointwise && ohw == 1) && conv_tc_supported(p)) {
+  const int64_t small_columns = pointwise ? p.n * ohw : int64_t(1) << 40;   // the rule is measured on 1 x 1 filters
+  if (tensor_conv_applies(*s, flops, small_columns) && !(pointwise && ohw == 1) && conv_tc_supported(p)) {
     const int wt = new_value(em.c, conv_tc_filter_elems(p), em.c.val(w).is_const);
     em.add("filter_pack", n.op, {w}, {wt}, 4.0 * p.oc * kdim * 3, 0,
            [=](cudaStream_t st) { return launch_pack_filter_tc(p, s->fptr(w), s->fptr_mut(wt), st); });
@@ -1229,7 +1230,7 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
     });
     return;
   }
-  if (small_conv_applies(*s, flops, p.n * ohw) && !(pointwise && ohw == 1) && conv_simt_supported(p)) {
+  if (small_conv_applies(*s, flops, small_columns) && !(pointwise && ohw == 1) && conv_simt_supported(p)) {
     const int wt = new_value(em.c, conv_simt_ldw(p.oc) * kdim, em.c.val(w).is_const);
     const int64_t oc = p.oc, kd = kdim;
     em.add("filter_pack", n.op, {w}, {wt}, 8.0 * oc * kd, 0,
