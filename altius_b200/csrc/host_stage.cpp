@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cstring>
 #include <map>
+#include <system_error>
 
 #if defined(__x86_64__)
 #include <immintrin.h>
@@ -63,7 +64,12 @@ bool HostStage::init() {
       return false;
     }
   const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
-  for (int i = 0; i < std::min(4, cores / 2); ++i) threads_.emplace_back([this] { worker(); });
+  // Without (all of) them the uploading thread copies what nobody else has taken; nothing may be thrown
+  // through the C interface.
+  try {
+    for (int i = 0; i < std::min(4, cores / 2); ++i) threads_.emplace_back([this] { worker(); });
+  } catch (const std::system_error&) {
+  }
   return true;
 }
 
