@@ -117,9 +117,6 @@ struct Plan {
   std::map<int, Squeeze> squeeze;   // GlobalAveragePool node -> the two 1 x 1 convolutions behind it
 };
 
-// Sessions on a device refine the schedule with kernels that a plan_only session does not list: its
-// schedule, arena plan and launch count are those of the general kernels, whatever the device.
-bool on_device(const AcSession& s) { return !s.opt.plan_only; }
 // gemm_mode 1 promises exact ascending chains and 2 its own precision: both keep their kernels.
 bool fp32_level_mode(const AcSession& s) { return s.opt.gemm_mode == 0 || s.opt.gemm_mode == 3; }
 
@@ -131,11 +128,11 @@ bool tensor_size(double flops, int64_t columns) {
   return flops >= double(1 << 23) && (flops >= double(1 << 25) || columns > 1024);
 }
 bool small_conv_applies(const AcSession& s, double flops, int64_t columns) {
-  return on_device(s) && fp32_level_mode(s) && !tensor_size(flops, columns);
+  return fp32_level_mode(s) && !tensor_size(flops, columns);
 }
 // The larger ones on the tensor-core kernel that reads the planes itself.
 bool tensor_conv_applies(const AcSession& s, double flops, int64_t columns) {
-  return on_device(s) && fp32_level_mode(s) && tensor_size(flops, columns);
+  return fp32_level_mode(s) && tensor_size(flops, columns);
 }
 
 // Recognises `hs = HardSigmoid(t); m = Mul(t, hs)` hanging off value t whose only
@@ -212,7 +209,7 @@ int effective_pairs(const AcSession& s) {
 }
 
 bool flash_attention_applies(const AcSession& s, const AttentionFusion& f) {
-  return on_device(s) && s.opt.gemm_mode == 0 && effective_pairs(s) == 2 && !std::getenv("ALTIUS_CUDA_NO_ATTENTION_TMA") &&
+  return s.opt.gemm_mode == 0 && effective_pairs(s) == 2 && !std::getenv("ALTIUS_CUDA_NO_ATTENTION_TMA") &&
          f.q.src == f.k.src && f.q.src == f.v.src && !s.values[f.q.src].is_const && s.values[f.q.src].elem_ty == AC_F32 &&
          attention_flash16_shape_ok((int)f.q.hd, (int)f.q.T, f.q.C, f.q.col, f.k.col, f.v.col, f.q.H * f.q.hd,
                                     f.q.T * f.q.H * f.q.hd);
@@ -551,10 +548,10 @@ void detect_se_gate(Ctx& c, Plan& plan) {
     for (int64_t k = 0; k < conv.ints[9]; ++k) nopad = nopad && conv.ints[10 + k] == 0;
     const double flops = 2.0 * xv.dims[0] * ov.dims[1] * hw * ch;
     // The conditions under which lower_conv / emit_gemm take the [K, N] tensor-core path.
-    // On a device the convolution kernels take a gate with any plane (lower_conv's conditions); the
+    // The convolution kernels take a gate with any plane (lower_conv's conditions); the
     // GEMM that reads the planes by TMA needs whole float4s and a size of its own.
     const bool gelu = plan.epi.count(cn) && plan.epi[cn].act == ACT_GELU;
-    const bool direct = on_device(c.s) && fp32_level_mode(c.s) && ch <= 4096 && ov.dims[1] <= 16384 && !gelu &&
+    const bool direct = fp32_level_mode(c.s) && ch <= 4096 && ov.dims[1] <= 16384 && !gelu &&
                         xv.numel() < (1ll << 30);
     const bool tensor = (hw % 4) == 0 && (ch % 4) == 0 && ch >= 8 && flops >= double(1 << 23);
     if (!pointwise || !nopad || !(tensor || direct) ||
@@ -568,7 +565,7 @@ void detect_se_gate(Ctx& c, Plan& plan) {
 // GlobalAveragePool -> pointwise Conv2d [+ act] -> pointwise Conv2d [+ act] on the 1 x 1 planes: the
 // squeeze-and-excite block up to its gate, one kernel.
 void detect_squeeze(Ctx& c, Plan& plan) {
-  if (!on_device(c.s) || !fp32_level_mode(c.s)) return;
+  if (!fp32_level_mode(c.s)) return;
   auto plain_1x1 = [&](int nid) {
     const Node& n = c.node(nid);
     if (c.absorbed[nid] || n.op != AC_OP_CONV2D || n.ints[0] != 1 || n.ints[1] != 1 || n.ints[2] != 1 || n.ints[3] != 1 ||
@@ -765,7 +762,7 @@ int new_value(Ctx& c, int64_t numel, bool is_const) {
 
 // Products of a few rows run in fp32 on the kernel that streams B (classifier heads at small batches).
 bool gemm_rows_applies(const AcSession& s, const GemmShape& g, bool b_const, int64_t a_off, int64_t b_off) {
-  return on_device(s) && fp32_level_mode(s) && g.batch == 1 && !g.ta && g.m <= kGemmRowsMax && g.k >= 4 && (g.k % 4) == 0 &&
+  return fp32_level_mode(s) && g.batch == 1 && !g.ta && g.m <= kGemmRowsMax && g.k >= 4 && (g.k % 4) == 0 &&
          (g.lda % 4) == 0 && (a_off % 4) == 0 &&
          (g.tb ? (g.ldb % 4) == 0 && (b_off % 4) == 0 : b_const && b_off == 0);
 }
@@ -787,7 +784,7 @@ bool presplit_applies(const AcSession& s, const GemmShape& g, bool b_const, int6
 // The same operands on the kernel for few rows, where it is the faster one (only for an A whose
 // producer writes the halves: a split kernel in front would cost what it saves).
 bool gemm_ks_applies(const AcSession& s, const GemmShape& g, bool b_const, int64_t a_off, int64_t b_off) {
-  if (!on_device(s) || s.opt.gemm_mode != 0 || effective_pairs(s) != 2 || !b_const || g.batch != 1 || g.ta || a_off != 0 ||
+  if (s.opt.gemm_mode != 0 || effective_pairs(s) != 2 || !b_const || g.batch != 1 || g.ta || a_off != 0 ||
       b_off != 0 || g.lda != g.k || gemm_rows_applies(s, g, b_const, a_off, b_off))
     return false;
   if (g.tb ? (g.ldb % 4) != 0 : (g.k % 4) != 0) return false;

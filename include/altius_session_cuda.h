@@ -153,8 +153,10 @@ typedef struct AcOptions {
                                 1 CUDA-core fp32 FMA only, 2 tcgen05 1xTF32,
                                 3 tcgen05 3xTF32 only                             */
   int32_t plan_only;         /* 1: infer shapes, lower and plan the arena without
-                                touching a GPU; run() then fails. For inspecting
-                                the schedule on a machine without a device.      */
+                                creating anything on a GPU; run() then fails. For
+                                inspecting the schedule on a machine without a
+                                device: the one a session on a B200 runs (on a
+                                machine with a device, on that device).          */
   int32_t gemm_pairs;        /* fp16-split GEMMs of 256 x 256 tiles on clusters of two CTAs
                                 (tcgen05 .cta_group::2, each SM stages its rows of A and half
                                 of the weight tile). 0 (default) and 2: where the cost model

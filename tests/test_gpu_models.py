@@ -35,6 +35,16 @@ def test_inference_session_by_name(cuda_lib):
         sess.run(None, {"wrong": feeds["Input3"]})
 
 
+@pytest.mark.parametrize("fn,kw", [(configs.mnist_cnn, {}), (configs.mobilenet_v3_large, dict(batch=2)),
+                                   (configs.vit_base_16, dict(batch=1, depth=1)), (configs.vit_base_16, dict(batch=32, depth=1))])
+def test_a_planned_schedule_is_the_one_that_runs(cuda_lib, fn, kw):
+    model, _ = fn(**kw)
+    built, planned = CudaSessionBuilder(model).build(), CudaSessionBuilder(model).with_plan_only(True).build()
+    assert planned.schedule() == built.schedule()
+    assert planned.arena_bytes == built.arena_bytes and planned.launches_per_run == built.launches_per_run
+    built.close()
+
+
 @pytest.mark.parametrize("batch", [3, 64])
 def test_micrograph(cuda_lib, batch):
     model, feeds = configs.micrograph(batch=batch)

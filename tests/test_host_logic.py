@@ -1,6 +1,6 @@
 """CPU-only tests of the session library's host side: the C ABI surface, shape
 inference, lowering / fusion and the arena plan (sessions built with
-`plan_only`, which touches no GPU), and error reporting at create time."""
+`plan_only`, which creates nothing on a GPU), and error reporting at create time."""
 import collections
 import os
 import re
@@ -65,11 +65,12 @@ def test_fusion_folds_the_expected_chains():
     kinds = collections.Counter(e["kind"] for e in plan(model).schedule())
     gemms = sum(v for k, v in kinds.items() if k.startswith("gemm"))
     assert gemms == 2 * 4 + 2          # per layer: qkv, proj, mlp1, mlp2; patch embed; head
-    # Split/Reshape/Transpose/QK^T/scale/Softmax/PV/merge in one kernel; at this batch the projection
-    # GEMM is too small for the CTA-pair kernel that would write its operands as fp16 halves
-    assert kinds["attention_tcgen05"] + kinds["attention_tma_tcgen05"] == 2
+    # Split/Reshape/Transpose/QK^T/scale/Softmax/PV/merge in one kernel: with few heads a block per tile of
+    # 128 queries, else a block per head
+    assert kinds["attention_flash_tcgen05"] == 2
+    assert kinds["gemm_fp32_rows"] == 1           # the head: two rows
     big = collections.Counter(e["kind"] for e in plan(configs.vit_base_16(batch=32, depth=2)[0]).schedule())
-    assert big["attention_tma_tcgen05"] == 2 and big["attention_tcgen05"] == 0
+    assert big["attention_tma_tcgen05"] == 2 and big["gemm_f16x3_pair_tcgen05"] == 2 * 4 + 1
     assert not any(k in kinds for k in ("split_copy", "transpose_copy", "softmax", "softmax_scaled"))
     unfused = collections.Counter(e["kind"] for e in plan(model, fuse=False).schedule())
     assert unfused["split_copy"] == 6 and unfused["softmax"] == 2
@@ -80,27 +81,21 @@ def test_fusion_folds_the_expected_chains():
     model, _ = configs.mobilenet_v3_large(batch=1)
     kinds = collections.Counter(e["kind"] for e in plan(model).schedule())
     assert "unary_hard_sigmoid" not in kinds and "unary_relu" not in kinds and "binary_Add" not in kinds
-    # Squeeze-excite gates: folded into the pointwise convolution that follows where that one
-    # runs on the tensor cores with the planes as its [K, N] operand (large enough, plane size a
-    # multiple of four floats); the rest stay broadcast Mul kernels.
-    assert kinds["binary_Mul"] == 6
+    # Squeeze-excite: pool and both products in one kernel, the gate in the operand loads of the
+    # pointwise convolution behind it.
+    assert kinds["binary_Mul"] == 0 and kinds["squeeze_excite"] == 8 and kinds["global_avg_pool"] == 1
     assert kinds["conv_depthwise"] == 15
+    assert kinds["gemm_fp32_rows"] == 2                # the 1 x 1 head convolution and the classifier
+    assert kinds["conv_fp32_simt"] + kinds["gemm_tf32x3_tcgen05"] == 31
 
-    # At the benchmark's batch the convolution GEMMs are large enough for the tensor cores:
-    # pointwise layers read the planes as a [K, N] rhs, the 7 x 7 layers through transposed planes,
-    # the first layer (3 x 3 x 3 = 27 taps) with zero-padded filter rows, the squeeze-excite
-    # layers (1 x 1 planes) as one product over the batch.
+    # At the benchmark's batch all convolutions run on the tensor cores with the planes read in place.
     model, _ = configs.mobilenet_v3_large(batch=32)
     steps = plan(model).schedule()
     kinds = collections.Counter(e["kind"] for e in steps)
-    assert kinds["im2col"] == 1 and kinds["transpose_copy"] == 6
-    assert kinds["binary_Mul"] == 3                    # gates of the three 7 x 7 blocks (transposed planes)
-    assert plan(model, fuse=False).schedule().count is not None
+    assert kinds["binary_Mul"] == 0 and kinds["im2col"] == 0 and kinds["transpose_copy"] == 0
+    assert kinds["gemm_tf32x3_tcgen05"] == 31 and kinds["squeeze_excite"] == 8
     assert collections.Counter(e["kind"] for e in plan(model, fuse=False).schedule())["binary_Mul"] >= 8
-    assert kinds["gemm_tf32x3_tcgen05"] == 31          # the first layer and the 30 pointwise layers on planes
-    assert kinds["gemm_f16x3_tcgen05"] == 12           # squeeze-excite, the 1 x 1 head convolution, the classifier
-    assert kinds["gemm_fp32_simt"] == 6                # the smallest squeeze-excite products
-    assert "weight_pad" not in kinds                   # prepared once at create, not per run
+    assert "filter_pack" not in kinds                  # prepared once at create, not per run
     cuda_cores = CudaSessionBuilder(model).with_plan_only(True).with_gemm_mode(1).build().schedule()
     assert sum(e["kind"] == "gemm_fp32_simt" for e in cuda_cores) == 49
     assert not any(e["kind"].endswith("tcgen05") for e in cuda_cores)
@@ -128,7 +123,19 @@ def test_arena_reuses_memory():
 def test_constant_only_nodes_are_not_in_the_per_run_schedule():
     model, _ = configs.mnist_cnn()
     kinds = [e["kind"] for e in plan(model).schedule()]
-    assert len(kinds) == 7     # 2x (im2col + conv gemm + maxpool) + the final matmul
+    assert kinds == ["conv_fp32_simt", "max_pool"] * 2 + ["gemm_fp32_rows"]
+
+
+def test_convolutions_beyond_the_direct_kernels_go_through_the_gemm():
+    """More than 4096 products per result: a column buffer, or planes read as they are / transposed."""
+    def conv(c, h, oc, k):
+        x, w = np.zeros((4, c, h, h), np.float32), np.zeros((oc, c, k, k), np.float32)
+        return [e["kind"] for e in plan(single_op_model("Conv2d", [x], [w, np.zeros(oc, np.float32)], kernel_shape=[k, k],
+                                                        strides=[1, 1], padding=[k // 2] * 4, dilations=[1, 1], group=1,
+                                                        auto_pad="")).schedule()]
+    assert conv(512, 14, 64, 3) == ["im2col", "gemm_tf32x3_tcgen05"]
+    assert conv(4100, 8, 64, 1) == ["gemm_tf32x3_tcgen05"]
+    assert conv(4100, 7, 64, 1) == ["transpose_copy", "gemm_tf32x3_tcgen05"]
 
 
 def test_errors_are_reported_at_create():
