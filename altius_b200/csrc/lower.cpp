@@ -767,6 +767,13 @@ bool gemm_rows_applies(const AcSession& s, const GemmShape& g, bool b_const, int
          (g.tb ? (g.ldb % 4) == 0 && (b_off % 4) == 0 : b_const && b_off == 0);
 }
 
+// Below about 8 MFLOP the CUDA-core kernel wins, except for few rows against a long K (the
+// squeeze-excite products, batch x channels): one or two of its blocks then walk K alone,
+// while the persistent kernel cuts K into slices over the idle SMs.
+double tensor_core_floor(const GemmShape& g) {
+  return g.batch == 1 && g.m <= 128 && g.k >= 64 ? double(1 << 19) : double(1 << 23);
+}
+
 // The static part of emit_gemm's decision to run a GEMM with a constant rhs on the CTA-pair
 // kernel that takes A pre-split (kept in one place: plan_presplit decides with it which
 // producers write split results before the GEMMs themselves are lowered).
@@ -775,8 +782,7 @@ bool presplit_applies(const AcSession& s, const GemmShape& g, bool b_const, int6
   if (gemm_rows_applies(s, g, b_const, a_off, b_off)) return false;
   if (mode != 0 || effective_pairs(s) != 2 || !b_const || g.batch != 1 || g.ta || b_off != 0) return false;
   const double flops = 2.0 * g.batch * g.m * g.n * g.k;
-  const double tc_floor = (g.batch == 1 && g.m <= 128 && g.k >= 64) ? double(1 << 19) : double(1 << 23);
-  if ((g.lda % 4) || (a_off % 4) || flops < tc_floor || g.k < 8 || (g.k % 8)) return false;
+  if ((g.lda % 4) || (a_off % 4) || flops < tensor_core_floor(g) || g.k < 8 || (g.k % 8)) return false;
   if (g.tb ? (g.ldb % 4) != 0 : (g.k % 4) != 0) return false;
   return gemm_tc_wants_presplit(g.m, g.n, g.k, g.batch);
 }
@@ -788,7 +794,7 @@ bool gemm_ks_applies(const AcSession& s, const GemmShape& g, bool b_const, int64
       b_off != 0 || g.lda != g.k || gemm_rows_applies(s, g, b_const, a_off, b_off))
     return false;
   if (g.tb ? (g.ldb % 4) != 0 : (g.k % 4) != 0) return false;
-  if (2.0 * g.m * g.n * g.k < double(1 << 20)) return false;
+  if (2.0 * g.m * g.n * g.k < std::max(double(1 << 20), tensor_core_floor(g))) return false;   // emit_gemm's floor, too
   return gemm_ks_clocks(g.m, g.n, g.k) < gemm_tc_pair_clocks(g.m, g.n, g.k);
 }
 
@@ -913,12 +919,8 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   // ---- tensor-core eligibility (static part; alignment is re-checked at launch) ----
   const int mode = s->opt.gemm_mode;
   const int pairs = effective_pairs(*s);
-  // Below about 8 MFLOP the CUDA-core kernel wins, except for few rows against a long K (the
-  // squeeze-excite products, batch x channels): one or two of its blocks then walk K alone,
-  // while the persistent kernel cuts K into slices over the idle SMs.
-  const double tc_floor = (g.batch == 1 && g.m <= 128 && g.k >= 64) ? double(1 << 19) : double(1 << 23);
   bool tc = mode != 1 && !g.ta && (g.lda % 4) == 0 && (a_off % 4) == 0 && (g.sa % 4) == 0 &&
-            flops >= tc_floor && g.k >= 8;
+            flops >= tensor_core_floor(g) && g.k >= 8;
   int b_use = b, b_lo = -1;
   const bool b_const = em.c.val(b).is_const;
   if (tc) {

@@ -138,6 +138,32 @@ def test_convolutions_beyond_the_direct_kernels_go_through_the_gemm():
     assert conv(4100, 7, 64, 1) == ["transpose_copy", "gemm_tf32x3_tcgen05"]
 
 
+def _mlp_behind_layer_norm(m, d, n):
+    g = ir.Graph()
+    f = lambda *shape: g.new_init(np.zeros(shape, np.float32))
+    h = g.op("LayerNormalization", g.add_input("x", (m, d)), f(d), f(d), axis=-1, epsilon=1e-6, stash_type=1)
+    h = g.op("Gelu", g.op("Add", g.op("MatMul", h, f(d, n)), f(n)))
+    g.outputs.append(g.op("Add", g.op("MatMul", h, f(n, d)), f(d)))
+    return ir.Model(g, 13)
+
+
+@pytest.mark.parametrize("m", [1, 32, 33, 65, 128, 129, 197, 577, 1386, 6304])
+def test_products_of_any_size_lower(m):
+    """Whoever writes an operand as halves and the product that takes it decide by one rule: around every
+    limit of it (operations, rows, K and N off the multiples) the graph lowers, the operand's producer included."""
+    for d in (64, 72, 100, 128, 200, 384, 1032):
+        for n in (32, 64, 66, 128, 256, 1024):
+            kinds = [e["kind"] for e in plan(_mlp_behind_layer_norm(m, d, n)).schedule()]
+            assert sum(k.startswith("gemm") for k in kinds) == 2, (m, d, n, kinds)
+
+
+@pytest.mark.parametrize("dim,heads", [(64, 1), (128, 2), (192, 3), (256, 4)])
+def test_narrow_transformers_lower(dim, heads):
+    for batch in (1, 2, 3, 4, 9):
+        for px in (48, 96, 224):
+            plan(configs.vision_transformer(batch, dim, 2, heads, 4 * dim, 1, img=px)[0])
+
+
 def test_errors_are_reported_at_create():
     a = np.zeros((1, 3, 28, 28), np.float32)
     b = np.zeros((3, 1, 2), np.float32)
