@@ -25,6 +25,7 @@
 
 #include <algorithm>
 
+#include "conv_tc_shape.h"
 #include "kernels.h"
 #include "pdl.cuh"
 #include "ref_math.cuh"
@@ -36,10 +37,9 @@ namespace ac {
 namespace {
 
 using namespace tc;
+using namespace conv_tc;
 
-constexpr int PX = 128, KB = 32;             // pixels per tile, floats of K per step (128-byte rows)
-constexpr int kLoaders = 256, kThreads = kLoaders + 32, kMaxStages = 3;
-constexpr int kABytes = PX * KB * 4;         // one of hi / lo
+constexpr int kLoaders = 256, kThreads = kLoaders + 32;
 
 struct ConvTcDev {
   const float* x;
@@ -431,59 +431,8 @@ __global__ void pack_filter_tc_kernel(const float* __restrict__ w, uint8_t* __re
   *reinterpret_cast<float4*>(blk + bn * KB * 4 + sw128(r, c)) = lo;
 }
 
-struct Shape {
-  int bn, tiles, split, kper, stages, resident, ctas;
-  size_t smem;
-};
-
-constexpr size_t kSmemSm = 233472;           // shared memory of an SM
-constexpr size_t kSmemMax = 231000;          // dynamic shared memory of one block
-
-// Picks channels per tile and K split. Times in clocks, from measurements of the kernel's parts: a K step
-// costs its loads and stores to shared memory (about 420 when blocks overlap) or its MMAs (12 per
-// full step at 65 or 0.8 per channel, whichever is more), the epilogue about 4 per channel, start
-// and end 2500 and a cluster's exchange 1500.
-Shape pick_shape(const ConvParams& q, int sms) {
-  const int k = q.c * q.kh * q.kw, nkb = (k + KB - 1) / KB;
-  const long long px = ((long long)q.n * q.oh * q.ow + PX - 1) / PX;
-  const bool window = q.kh != 1 || q.kw != 1 || q.sh != 1 || q.sw != 1 || q.pad_t || q.pad_l || q.oh != q.ih || q.ow != q.iw;
-  Shape best{};
-  double best_t = 1e30;
-  for (int tiles = (q.oc + 255) / 256; tiles <= (q.oc + 15) / 16; ++tiles) {
-    const int bn = ((q.oc + tiles - 1) / tiles + 15) / 16 * 16;
-    if ((bn * (tiles - 1)) >= q.oc) continue;
-    for (int split = 1; split <= 8; split *= 2) {
-      const int kper = (nkb + split - 1) / split;
-      if ((split - 1) * kper >= nkb) continue;
-      const double step = std::max(420.0, 12 * std::max(65.0, 0.8 * bn) * std::min(1.0, k / 32.0));
-      const double body = kper * step + 4.0 * bn, waves = std::ceil((double)px * tiles / cluster_slots(split));
-      const double t = waves * body + 2500 + (split > 1 ? 1500 : 0);
-      if (t < best_t * 0.98) { best_t = t; best.bn = bn; best.tiles = tiles; best.split = split; best.kper = kper; }
-    }
-    if (bn <= 32) break;
-  }
-  // Blocks walk tiles when there are more than two per SM (and nothing is cut over a cluster); then
-  // a block needs two accumulators, and those of two blocks fit tensor memory up to 128 channels.
-  const bool walk = best.split == 1 && px * best.tiles > 2 * sms;
-  if (walk && best.bn > 128) {
-    best.tiles = (q.oc + 127) / 128;
-    best.bn = ((q.oc + best.tiles - 1) / best.tiles + 15) / 16 * 16;
-  }
-  best.ctas = (int)(walk ? std::min<long long>(px, std::max(1, 2 * sms / best.tiles)) : px);
-  const size_t bb = (size_t)best.bn * KB * 8;
-  const size_t table = window ? (size_t)k * sizeof(int2) : 0, part = best.split > 1 ? (size_t)best.bn * PX * 4 : 0;
-  // A walking block keeps its filter tile in shared memory where that leaves room for two stages.
-  const size_t half = kSmemSm / 2 - 3072;
-  best.resident = walk && 2 * (2 * (size_t)kABytes) + best.kper * bb + table <= half;
-  const size_t stage = 2 * (size_t)kABytes + (best.resident ? 0 : bb);
-  best.stages = std::min(best.kper * (walk ? 2 : 1), kMaxStages);
-  auto need = [&](int st) { return st * stage + (best.resident ? best.kper * bb : 0) + part + table + 1024; };
-  // As many stages as leave room for a second block on the SM, at least two when there are two steps.
-  while (best.stages > 2 && need(best.stages) > half) --best.stages;
-  while (best.stages > 1 && need(best.stages) > kSmemMax) --best.stages;
-  const int set = best.bn <= 32 ? 32 : best.bn <= 64 ? 64 : best.bn <= 128 ? 128 : 256;
-  best.smem = std::max(need(best.stages), kSmemSm * (best.ctas < px ? 2 * set : set) / 512 - 2048);
-  return best;
+Shape shape_of(const ConvParams& q) {
+  return pick_shape(q, {device_sm_count(), cluster_slots(2), cluster_slots(4), cluster_slots(8)});
 }
 
 template <bool WINDOW, int ACT>
@@ -509,18 +458,18 @@ cudaError_t launch_one(const ConvTcDev& p, const Shape& sh, int act, cudaStream_
 
 bool conv_tc_supported(const ConvParams& q) {
   const int64_t k = (int64_t)q.c * q.kh * q.kw, cols = (int64_t)q.n * q.oh * q.ow;
-  return q.group == 1 && k >= 1 && k <= 4096 && cols < (1ll << 30) && (int64_t)q.c * q.ih * q.iw < (1ll << 30) &&
-         q.kh * q.dh < 32768 && q.kw * q.dw < 32768 && q.oc <= 16384 && q.act != ACT_GELU;
+  return q.group == 1 && k >= 1 && k <= 4096 && cols >= 1 && cols < (1ll << 30) && (int64_t)q.c * q.ih * q.iw < (1ll << 30) &&
+         q.kh * q.dh < 32768 && q.kw * q.dw < 32768 && q.oc >= 1 && q.oc <= 16384 && q.act != ACT_GELU && shape_of(q).bn > 0;
 }
 
 int64_t conv_tc_filter_elems(const ConvParams& q) {
-  const Shape sh = pick_shape(q, device_sm_count());
+  const Shape sh = shape_of(q);
   const int64_t nkb = ((int64_t)q.c * q.kh * q.kw + KB - 1) / KB;
   return (int64_t)sh.tiles * nkb * sh.bn * KB * 2;
 }
 
 cudaError_t launch_pack_filter_tc(const ConvParams& q, const float* w, float* packed, cudaStream_t st) {
-  const Shape sh = pick_shape(q, device_sm_count());
+  const Shape sh = shape_of(q);
   const int k = q.c * q.kh * q.kw;
   const long long chunks = (long long)sh.tiles * ((k + KB - 1) / KB) * sh.bn * 8;
   pack_filter_tc_kernel<<<(unsigned)((chunks + 255) / 256), 256, 0, st>>>(w, reinterpret_cast<uint8_t*>(packed), q.oc, k, sh.bn,
@@ -530,7 +479,7 @@ cudaError_t launch_pack_filter_tc(const ConvParams& q, const float* w, float* pa
 
 cudaError_t launch_conv_tc(const ConvParams& q, const float* x, const float* packed, const float* bias, const float* gate,
                            const float* residual, float* out, bool constants, int* err_word, cudaStream_t st) {
-  const Shape sh = pick_shape(q, device_sm_count());
+  const Shape sh = shape_of(q);
   ConvTcDev p{};
   p.x = x; p.w = packed; p.out = out; p.bias = bias; p.res = residual; p.gate = gate;
   p.m = q.oc; p.k = q.c * q.kh * q.kw; p.hw = q.oh * q.ow; p.n = q.n * p.hw;
