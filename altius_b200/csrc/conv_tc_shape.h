@@ -22,6 +22,7 @@ struct Shape {
 
 constexpr size_t kSmemSm = 233472;           // shared memory of an SM
 constexpr size_t kSmemMax = 231000;          // dynamic shared memory of one block
+constexpr size_t kSmemBeside = 2304;         // beside it: 1120 static bytes, 1024 of the system, rounding
 
 // Picks channels per tile and K split among those that fit a block's shared memory with two stages. Times in clocks, from measurements of the kernel's parts: a K step
 // costs its loads and stores to shared memory (about 420 when blocks overlap) or its MMAs (12 per
@@ -61,16 +62,20 @@ inline Shape pick_shape(const ConvParams& q, const std::array<int, 4>& slots) {
     best.tiles = (q.oc + 127) / 128;
     best.bn = ((q.oc + best.tiles - 1) / best.tiles + 15) / 16 * 16;
   }
-  best.ctas = (int)(walk ? std::min<long long>(px, std::max(1, 2 * sms / best.tiles)) : px);
   // A walking block keeps its filter tile in shared memory where that leaves room for two stages.
-  const size_t half = kSmemSm / 2 - 3072;
+  const size_t half = kSmemSm / 2 - kSmemBeside;
   best.resident = walk && bytes(best.bn, 1, best.kper, 2, true) <= half;
   best.stages = std::min(best.kper * (walk ? 2 : 1), kMaxStages);
   auto need = [&](int st) { return bytes(best.bn, best.split, best.kper, st, best.resident); };
   // As many stages as leave room for a second block on the SM, at least two when there are two steps.
   while (best.stages > 2 && need(best.stages) > half) --best.stages;
+  // Shared memory in proportion to the columns of tensor memory, so that whatever blocks share an SM find theirs.
+  // (With 2048 bytes for what lies beside it two blocks of 256 columns missed the SM by 192 bytes, and half of a
+  // grid of two blocks per SM started when the other half had finished.)
   const int set = best.bn <= 32 ? 32 : best.bn <= 64 ? 64 : best.bn <= 128 ? 128 : 256;
-  best.smem = std::max(need(best.stages), kSmemSm * (best.ctas < px ? 2 * set : set) / 512 - 2048);
+  best.smem = std::max(need(best.stages), kSmemSm * (walk ? 2 * set : set) / 512 - kSmemBeside);
+  const int resident_blocks = sms * (best.smem <= half ? 2 : 1);
+  best.ctas = (int)(walk ? std::min<long long>(px, std::max(1, resident_blocks / best.tiles)) : px);
   return best;
 }
 

@@ -1,5 +1,6 @@
 """Host arithmetic of the tensor-core convolution's tile choice (conv_tc_shape.h), compiled and swept
-over layers, batches and numbers of clusters that run at once: every shape it returns can be launched."""
+over layers, batches and numbers of clusters that run at once: every shape it returns can be launched, and
+the blocks that walk tiles run at once."""
 import os
 import subprocess
 
@@ -23,12 +24,18 @@ int main() {
               const conv_tc::Shape s = conv_tc::pick_shape(q, slots);
               const int k = c * kk * kk, nkb = (k + 31) / 32;
               ++tried;
-              const bool ok = s.bn >= 16 && s.bn <= 256 && s.bn % 16 == 0 && s.tiles >= 1 && s.tiles <= 65535 && (long long)s.tiles * s.bn >= oc &&
+              // What lives on an SM together: 1120 static bytes and 1024 of the system beside the dynamic ones.
+              const long long px = ((long long)n * h * h + 127) / 128;
+              const int per_sm = (int)std::min<size_t>(7, 233472 / ((s.smem + 1120 + 127) / 128 * 128 + 1024));
+              const int set = s.bn <= 32 ? 32 : s.bn <= 64 ? 64 : s.bn <= 128 ? 128 : 256, columns = s.ctas < px ? 2 * set : set;
+              const bool walks = s.ctas < px;
+              const bool fits = per_sm * columns <= 512 && (!walks || s.ctas == 1 || s.ctas * s.tiles <= per_sm * slots[0]);
+              const bool ok = fits && s.bn >= 16 && s.bn <= 256 && s.bn % 16 == 0 && s.tiles >= 1 && s.tiles <= 65535 && (long long)s.tiles * s.bn >= oc &&
                               s.split * s.kper >= nkb && (s.split - 1) * s.kper < nkb && s.ctas >= 1 &&
                               s.stages >= std::min(2, s.kper) && s.stages <= 3 && s.smem <= conv_tc::kSmemMax;
               if (!ok && ++bad <= 12)
-                std::printf("n %d c %d h %d oc %d filter %d slots %d: bn %d split %d stages %d smem %zu\n", n, c, h, oc, kk, slots[3],
-                            s.bn, s.split, s.stages, s.smem);
+                std::printf("n %d c %d h %d oc %d filter %d slots %d: bn %d split %d stages %d smem %zu blocks %d x %d, %d an SM\n", n, c, h, oc, kk,
+                            slots[3], s.bn, s.split, s.stages, s.smem, s.ctas, s.tiles, per_sm);
             }
   std::printf("%lld tried, %lld bad\n", tried, bad);
   return bad != 0;
