@@ -145,14 +145,18 @@ cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStre
     do {
       // Chunk allowed - kSlots is on its way (it is below c): once it has left, its slot is free.
       while (allowed < n && allowed - kSlots < c) {
-        if (cudaEventQuery(left_[allowed % kSlots]) != cudaSuccess) {
+        const cudaError_t left = cudaEventQuery(left_[allowed % kSlots]);
+        if (left != cudaSuccess) {
           (void)cudaGetLastError();
+          if (left != cudaErrorNotReady) err = left;   // a fault on the device: the slot never gets free
           break;
         }
         allowed_.store(++allowed, std::memory_order_release);
       }
+      if (err != cudaSuccess) break;
       if (!copy_next(c + 1)) relax();         // this chunk itself, if no worker has taken it yet
     } while (!done_[c].load(std::memory_order_acquire));
+    if (err != cudaSuccess) break;
     const size_t at = (size_t)c * kChunk;
     err = cudaMemcpyAsync(static_cast<char*>(dst) + at, ring_ + (size_t)(c % kSlots) * kChunk, std::min(kChunk, bytes - at),
                           cudaMemcpyHostToDevice, st);
