@@ -114,7 +114,9 @@ void HostStage::worker() {
 }
 
 cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-  std::lock_guard<std::mutex> use(use_);
+  // While another thread's upload holds the ring this one takes the driver's path: both then run at once.
+  std::unique_lock<std::mutex> use(use_, std::try_to_lock);
+  if (!use.owns_lock()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
   const int n = (int)((bytes + kChunk - 1) / kChunk);
   for (cudaEvent_t e : left_)                 // slots an earlier upload may still occupy
     if (cudaError_t err = cudaEventSynchronize(e)) return err;

@@ -5,7 +5,7 @@
 // link, so the upload runs at the link's rate after the first chunk.
 //
 // One stage per device, shared by the sessions that need it and freed with the last of them; one
-// upload at a time.
+// upload at a time, and those that find it taken are copied by the driver.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -83,6 +83,6 @@ def harness(tmp_path_factory):
     return str(d / "h")
 
 
-@pytest.mark.parametrize("what", ["copies", "fault"])
+@pytest.mark.parametrize("what", ["copies", "fault", "two"])
 def test_staged_upload(harness, what):
     assert subprocess.run([harness, what], timeout=30).returncode == 0
