@@ -2,8 +2,9 @@
 
 #include <algorithm>
 #include <cstring>
+#include <exception>
 #include <map>
-#include <system_error>
+#include <new>
 
 #if defined(__x86_64__)
 #include <immintrin.h>
@@ -44,12 +45,17 @@ inline void relax() {
 std::shared_ptr<HostStage> HostStage::of_device(int device) {
   static std::mutex m;
   static std::map<int, std::weak_ptr<HostStage>> made;
-  std::lock_guard<std::mutex> lock(m);
-  if (std::shared_ptr<HostStage> s = made[device].lock()) return s;
-  std::shared_ptr<HostStage> s(new HostStage());
-  if (!s->init()) return nullptr;
-  made[device] = s;
-  return s;
+  // Nothing may be thrown through the C interface: without memory for it the caller does without.
+  try {
+    std::lock_guard<std::mutex> lock(m);
+    if (std::shared_ptr<HostStage> s = made[device].lock()) return s;
+    std::shared_ptr<HostStage> s(new HostStage());
+    if (!s->init()) return nullptr;
+    made[device] = s;
+    return s;
+  } catch (const std::exception&) {
+    return nullptr;
+  }
 }
 
 bool HostStage::init() {
@@ -64,11 +70,10 @@ bool HostStage::init() {
       return false;
     }
   const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
-  // Without (all of) them the uploading thread copies what nobody else has taken; nothing may be thrown
-  // through the C interface.
+  // Without (all of) them the uploading thread copies what nobody else has taken.
   try {
     for (int i = 0; i < std::min(4, cores / 2); ++i) threads_.emplace_back([this] { worker(); });
-  } catch (const std::system_error&) {
+  } catch (const std::exception&) {
   }
   return true;
 }
@@ -118,6 +123,11 @@ cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStre
   std::unique_lock<std::mutex> use(use_, std::try_to_lock);
   if (!use.owns_lock()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
   const int n = (int)((bytes + kChunk - 1) / kChunk);
+  std::unique_ptr<std::atomic<char>[]> more;
+  if (done_size_ < n) {                       // only ever changed under use_
+    more.reset(new (std::nothrow) std::atomic<char>[n]);
+    if (!more) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  }
   for (cudaEvent_t e : left_)                 // slots an earlier upload may still occupy
     if (cudaError_t err = cudaEventSynchronize(e)) return err;
   {
@@ -128,8 +138,8 @@ cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStre
       relax();
       lock.lock();
     }
-    if (done_size_ < n) {
-      done_.reset(new std::atomic<char>[n]);
+    if (more) {
+      done_ = std::move(more);
       done_size_ = n;
     }
     for (int i = 0; i < n; ++i) done_[i].store(0, std::memory_order_relaxed);

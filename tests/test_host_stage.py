@@ -12,6 +12,7 @@ HARNESS = r"""
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -19,6 +20,19 @@ HARNESS = r"""
 
 static std::atomic<int> query_result{0}, whole_copies{0}, copies{0};
 static std::atomic<bool> held{false};       // copies have been handed over but do not finish
+static std::atomic<bool> no_memory{false};
+void* operator new(size_t n) {
+  void* p = no_memory ? nullptr : std::malloc(n);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void* operator new[](size_t n) { return operator new(n); }
+void* operator new(size_t n, const std::nothrow_t&) noexcept { return no_memory ? nullptr : std::malloc(n); }
+void* operator new[](size_t n, const std::nothrow_t& t) noexcept { return operator new(n, t); }
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete[](void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+void operator delete[](void* p, size_t) noexcept { std::free(p); }
 extern "C" {
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::malloc(n); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
@@ -40,6 +54,17 @@ static bool right(const std::vector<char>& a, const std::vector<char>& b) { retu
 
 int main(int argc, char** argv) {
   const std::string what = argv[1];
+  if (what == "memory") {                    // nothing to be had: no stage, nothing thrown; later: the driver's path
+    no_memory = true;
+    if (ac::HostStage::of_device(1)) return 1;
+    no_memory = false;
+    auto s = ac::HostStage::of_device(1);
+    std::vector<char> a(size_t(5) << 20, 7), b(size_t(5) << 20);
+    no_memory = true;
+    const bool ok = s->upload(b.data(), a.data(), a.size(), nullptr) == cudaSuccess && whole_copies == 1;
+    no_memory = false;
+    return ok && std::memcmp(a.data(), b.data(), a.size()) == 0 ? 0 : 2;
+  }
   auto stage = ac::HostStage::of_device(0);
   const size_t big = (size_t(40) << 20) + 12345;
   std::vector<char> src(big), dst(big), dst2(big);
@@ -83,6 +108,6 @@ def harness(tmp_path_factory):
     return str(d / "h")
 
 
-@pytest.mark.parametrize("what", ["copies", "fault", "two"])
+@pytest.mark.parametrize("what", ["copies", "fault", "two", "memory"])
 def test_staged_upload(harness, what):
     assert subprocess.run([harness, what], timeout=30).returncode == 0
