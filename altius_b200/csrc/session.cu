@@ -197,6 +197,11 @@ cudaError_t capture(AcSession* s, int first, int last, cudaGraph_t* graph, cudaG
 
 cudaError_t launch_all(AcSession* s) { return s->graph_exec ? cudaGraphLaunch(s->graph_exec, s->stream) : replay(s, s->stream); }
 
+void destroy_segment(Segment& g) {
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  if (g.graph) cudaGraphDestroy(g.graph);
+}
+
 // A run on device buffers need not copy them in and out of the arena (115 of the 200 us that the
 // tensor-op micrograph spent on the GPU): the kernels that read a graph input or write a graph
 // output take the caller's pointers. Their launches cannot be in a graph then, so this is done where
@@ -218,32 +223,16 @@ void plan_segments(AcSession& s) {
   for (const Step& st : s.init_steps)
     for (int w : st.writes)
       if (io[w]) return;
-  int direct = 0;
-  std::vector<Segment> segs;
-  for (int i = 0; i < (int)s.steps.size(); ++i) {
-    bool touches = false;
-    for (int r : s.steps[i].reads) touches = touches || io[r];
-    for (int w : s.steps[i].writes) touches = touches || io[w];
-    direct += touches;
-    // A graph segment is marked by last < 0 until its end is known.
-    if (segs.empty() || touches != (segs.back().graph == nullptr)) {
-      Segment g;
-      g.first = i;
-      g.graph = touches ? nullptr : reinterpret_cast<cudaGraph_t>(1);
-      segs.push_back(g);
-    }
-    segs.back().last = i + 1;
+  std::vector<char> touches(s.steps.size(), 0);
+  for (size_t i = 0; i < s.steps.size(); ++i) {
+    for (int r : s.steps[i].reads) touches[i] |= io[r];
+    for (int w : s.steps[i].writes) touches[i] |= io[w];
   }
-  if (segs.size() > 6 || direct > 8) return;
-  for (Segment& g : segs) {
-    if (!g.graph) continue;
-    g.graph = nullptr;
-    if (cudaError_t e = capture(&s, g.first, g.last, &g.graph, &g.exec)) {
-      s.segments = segs;               // destroyed with the session
-      fail(AC_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-    }
-  }
-  s.segments = segs;
+  std::vector<Segment> segs = split_segments(touches);
+  if (segs.size() > 6 || std::count(touches.begin(), touches.end(), 1) > 8) return;
+  capture_segments(segs, [&](Segment& g) { return capture(&s, g.first, g.last, &g.graph, &g.exec); }, destroy_segment);
+  (void)cudaGetLastError();
+  s.segments = std::move(segs);
 }
 
 // Kernels read and write with 16-byte accesses; a result may not land on a buffer that a later
@@ -282,7 +271,7 @@ cudaError_t launch_bound(AcSession* s, const void* const* ins, void* const* outs
   bind(true);
   cudaError_t e = cudaSuccess;
   for (const Segment& g : s->segments) {
-    e = g.exec ? cudaGraphLaunch(g.exec, s->stream) : replay(s, s->stream, g.first, g.last);
+    e = g.direct ? replay(s, s->stream, g.first, g.last) : cudaGraphLaunch(g.exec, s->stream);
     if (e != cudaSuccess) break;
   }
   bind(false);
@@ -805,10 +794,7 @@ void altius_cuda_destroy(AcSession* s) {
   if (s->graph) cudaGraphDestroy(s->graph);
   for (cudaEvent_t ev : s->events)
     if (ev) cudaEventDestroy(ev);
-  for (ac::Segment& g : s->segments) {
-    if (g.exec) cudaGraphExecDestroy(g.exec);
-    if (g.graph) cudaGraphDestroy(g.graph);
-  }
+  destroy_segments(s->segments, destroy_segment);
   if (s->sweep_buf) cudaFree(s->sweep_buf);
   for (int k = 0; k < 2; ++k) {
     for (void* p : s->staging[k])

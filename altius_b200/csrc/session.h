@@ -16,6 +16,7 @@
 #include "../../include/altius_session_cuda.h"
 #include "host_stage.h"
 #include "kernels.h"
+#include "segments.h"
 
 namespace ac {
 
@@ -63,14 +64,6 @@ struct Step {
   double bytes = 0, flops = 0;     // algorithmic work
   int launches = 1;
   bool const_only = false;         // all inputs constant: executed once at create()
-};
-
-// Consecutive steps of the schedule for runs on bound buffers: those that touch a graph input or
-// output are launched one by one on the caller's pointers, the others replay a graph.
-struct Segment {
-  int first = 0, last = 0;         // steps [first, last)
-  cudaGraph_t graph = nullptr;     // null: launched one by one
-  cudaGraphExec_t exec = nullptr;
 };
 
 struct ProfileAcc {
