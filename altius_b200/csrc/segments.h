@@ -1,7 +1,9 @@
 // Consecutive steps of a schedule for runs on bound buffers (session.cu): host logic only.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
+#include <utility>
 #include <vector>
 
 namespace ac {
@@ -42,6 +44,28 @@ template <typename Capture, typename Destroy>
 void capture_segments(std::vector<Segment>& segs, Capture capture, Destroy destroy) {
   for (Segment& g : segs)
     if (!g.direct && capture(g) != cudaSuccess) return destroy_segments(segs, destroy);
+}
+
+// Whether the schedule may run on these buffers, `in(i)` and `out(i)` being their addresses and sizes.
+// Kernels read and write with 16-byte accesses; a result may not land on a buffer that a later kernel
+// still reads; and `local(address)` says whether the memory is the device's own -- a copy also takes
+// page-locked host memory and another device's, which kernels cannot reach or reach over a link.
+template <typename In, typename Out, typename Local>
+bool can_bind_buffers(int n_in, In in, int n_out, Out out, Local local) {
+  auto usable = [&](std::pair<uintptr_t, size_t> b) { return (b.first & 15) == 0 && (b.second == 0 || local(b.first)); };
+  auto meet = [](std::pair<uintptr_t, size_t> a, std::pair<uintptr_t, size_t> b) {
+    return a.first < b.first + b.second && b.first < a.first + a.second;
+  };
+  for (int i = 0; i < n_in; ++i)
+    if (!usable(in(i))) return false;
+  for (int i = 0; i < n_out; ++i) {
+    if (!usable(out(i))) return false;
+    for (int j = 0; j < n_in; ++j)
+      if (meet(out(i), in(j))) return false;
+    for (int j = 0; j < i; ++j)
+      if (meet(out(i), out(j))) return false;
+  }
+  return true;
 }
 
 }  // namespace ac

@@ -235,28 +235,20 @@ void plan_segments(AcSession& s) {
   s.segments = std::move(segs);
 }
 
-// Kernels read and write with 16-byte accesses; a result may not land on a buffer that a later
-// kernel still reads.
 bool can_bind(const AcSession* s, const void* const* ins, void* const* outs) {
   if (s->segments.empty()) return false;
-  std::vector<std::pair<uintptr_t, uintptr_t>> in, out;
-  for (size_t i = 0; i < s->inputs.size(); ++i) {
-    const uintptr_t p = reinterpret_cast<uintptr_t>(ins[i]);
-    if (p & 15) return false;
-    in.push_back({p, p + s->values[s->inputs[i]].bytes()});
-  }
-  for (size_t i = 0; i < s->outputs.size(); ++i) {
-    const uintptr_t p = reinterpret_cast<uintptr_t>(outs[i]);
-    if (p & 15) return false;
-    out.push_back({p, p + s->values[s->outputs[i]].bytes()});
-  }
-  for (size_t i = 0; i < out.size(); ++i) {
-    for (auto& q : in)
-      if (out[i].first < q.second && q.first < out[i].second) return false;
-    for (size_t j = i + 1; j < out.size(); ++j)
-      if (out[i].first < out[j].second && out[j].first < out[i].second) return false;
-  }
-  return true;
+  auto local = [&](uintptr_t p) {
+    cudaPointerAttributes pa{};
+    if (cudaPointerGetAttributes(&pa, reinterpret_cast<const void*>(p)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    return pa.type == cudaMemoryTypeDevice && pa.device == s->device;
+  };
+  return can_bind_buffers(
+      (int)s->inputs.size(), [&](int i) { return std::make_pair(reinterpret_cast<uintptr_t>(ins[i]), s->values[s->inputs[i]].bytes()); },
+      (int)s->outputs.size(), [&](int i) { return std::make_pair(reinterpret_cast<uintptr_t>(outs[i]), s->values[s->outputs[i]].bytes()); },
+      local);
 }
 
 // The schedule with device buffers in place of the arena slots of the graph's inputs (and outputs,

@@ -35,6 +35,29 @@ def test_inference_session_by_name(cuda_lib):
         sess.run(None, {"wrong": feeds["Input3"]})
 
 
+def test_device_runs_on_buffers_of_any_kind(cuda_lib):
+    """Own device memory is used in place; page-locked memory and unaligned or overlapping buffers go through copies."""
+    import torch
+    model, feeds = configs.micrograph(batch=2)
+    want = run_oracle(model, feeds.values())
+    sess = CudaSessionBuilder(model).build()
+    ins = [torch.from_numpy(np.ascontiguousarray(a)) for a in feeds.values()]
+    shapes = [s for s, _ in sess.output_info]
+    def odd(t):                      # the same values 4 bytes off the alignment
+        buf = torch.empty(t.numel() + 1, device="cuda")
+        buf[1:].copy_(t.flatten())
+        return buf[1:]
+    for place_in, place_out in ((lambda t: t.cuda(), lambda s: torch.empty(s, device="cuda")), (odd, lambda s: torch.empty(s, device="cuda")),
+                                (lambda t: t.pin_memory(), lambda s: torch.empty(s).pin_memory())):
+        bufs, outs = [place_in(t) for t in ins], [place_out(s) for s in shapes]
+        torch.cuda.synchronize()
+        for _ in range(2):
+            sess.run_device([t.data_ptr() for t in bufs], [t.data_ptr() for t in outs])
+        for g, w in zip(outs, want):
+            np.testing.assert_allclose(g.cpu().numpy().reshape(w.shape), w, rtol=1e-5, atol=1e-6)
+    sess.close()
+
+
 @pytest.mark.parametrize("fn,kw", [(configs.mnist_cnn, {}), (configs.mobilenet_v3_large, dict(batch=2)),
                                    (configs.vit_base_16, dict(batch=1, depth=1)), (configs.vit_base_16, dict(batch=32, depth=1))])
 def test_a_planned_schedule_is_the_one_that_runs(cuda_lib, fn, kw):

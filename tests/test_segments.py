@@ -1,5 +1,5 @@
-"""The segments of a schedule that runs on the caller's device buffers (segments.h), with a stand-in for the
-capture that fails where the test says."""
+"""Runs on the caller's device buffers (segments.h): which buffers are taken, and the segments of the schedule,
+with a stand-in for the capture that fails where the test says."""
 import os
 import subprocess
 
@@ -42,9 +42,39 @@ int main() {
 """
 
 
-def test_a_capture_that_fails_leaves_no_segments(tmp_path):
-    (tmp_path / "h.cpp").write_text(HARNESS)
+BUFFERS = r"""
+#include "segments.h"
+using namespace ac;
+using B = std::pair<uintptr_t, size_t>;
+int main() {
+  // memory of this device from 0x10000 on, of another one from 0x20000 on, the host's from 0x30000 on
+  auto local = [](uintptr_t p) { return p >= 0x10000 && p < 0x20000; };
+  auto ok = [&](std::vector<B> in, std::vector<B> out) {
+    return can_bind_buffers((int)in.size(), [&](int i) { return in[i]; }, (int)out.size(), [&](int i) { return out[i]; }, local);
+  };
+  if (!ok({{0x10000, 64}}, {{0x10040, 64}, {0x10080, 4}})) return 1;
+  if (ok({{0x20000, 64}}, {{0x10040, 64}}) || ok({{0x10000, 64}}, {{0x20040, 64}})) return 2;      // another device's
+  if (ok({{0x30000, 64}}, {{0x10040, 64}}) || ok({{0x10000, 64}}, {{0x10040, 64}, {0x30000, 4}})) return 3;
+  if (ok({{0x10004, 60}}, {{0x10040, 64}}) || ok({{0x10000, 64}}, {{0x10048, 64}})) return 4;      // alignment
+  if (ok({{0x10000, 64}}, {{0x10030, 64}}) || ok({{0x10030, 64}}, {{0x10000, 64}})) return 5;      // an input under a result
+  if (ok({{0x10000, 64}}, {{0x10100, 64}, {0x10130, 64}}) || ok({{0x10000, 64}}, {{0x10000, 64}})) return 6;
+  if (!ok({{0, 0}}, {{0x10040, 64}})) return 7;                                                   // nothing to read
+  return 0;
+}
+"""
+
+
+def _run(tmp_path, text):
+    (tmp_path / "h.cpp").write_text(text)
     cuda = os.path.dirname(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")))
     subprocess.run(["g++", "-std=c++17", "-I", os.path.join(ROOT, "altius_b200", "csrc"), "-I", os.path.join(cuda, "include"),
                     str(tmp_path / "h.cpp"), "-o", str(tmp_path / "h")], check=True)
     assert subprocess.run([str(tmp_path / "h")]).returncode == 0
+
+
+def test_buffers_a_run_takes_in_place(tmp_path):
+    _run(tmp_path, BUFFERS)
+
+
+def test_a_capture_that_fails_leaves_no_segments(tmp_path):
+    _run(tmp_path, HARNESS)
