@@ -270,12 +270,6 @@ cudaError_t launch_bound(AcSession* s, const void* const* ins, void* const* outs
   return e;
 }
 
-cudaError_t use_device(int device) {
-  int cur = -1;
-  if (cudaGetDevice(&cur) == cudaSuccess && cur == device) return cudaSuccess;
-  return cudaSetDevice(device);
-}
-
 constexpr size_t kSmallIo = size_t(1) << 20;   // inputs (outputs) up to this go through the session's staging block
 
 // Host inputs into the arena. Small ones are gathered in the page-locked block first: the driver's own
@@ -407,7 +401,7 @@ int run_common(AcSession* s, const void* const* ins, void* const* outs, bool dev
     if (rc != AC_OK) s->err = s->fallback->err;
     return rc;
   }
-  cudaError_t e = use_device(s->device);
+  cudaError_t e = cudaSetDevice(s->device);
   if (e != cudaSuccess) return set_err(s, AC_ERR_CUDA, cudaGetErrorString(e));
   // An error after this point drains the stream before returning, for the same reason.
   auto fail_cuda = [&](const std::string& what, cudaError_t err) {
@@ -603,7 +597,7 @@ int altius_cuda_run_batches(AcSession* s, int32_t n_batches, const void* const* 
     }
     return AC_OK;
   }
-  cudaError_t e = use_device(s->device);
+  cudaError_t e = cudaSetDevice(s->device);
   if (e == cudaSuccess && !s->copy_stream) {
     e = cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking);
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
@@ -669,7 +663,7 @@ int altius_cuda_time_device_runs(AcSession* s, const void* const* d_ins, void* c
     if (rc != AC_OK) s->err = s->fallback->err;
     return rc;
   }
-  cudaError_t e = use_device(s->device);
+  cudaError_t e = cudaSetDevice(s->device);
   const bool bound = can_bind(s, d_ins, d_outs);
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   if (e == cudaSuccess) e = cudaEventCreate(&t0);

@@ -58,6 +58,31 @@ def test_device_runs_on_buffers_of_any_kind(cuda_lib):
     sess.close()
 
 
+def test_runs_from_a_thread_with_a_context_of_its_own(cuda_lib):
+    """A caller whose current context on the device is not the session's: the run makes the session's current."""
+    import ctypes
+    import torch
+    model, feeds = configs.micrograph(batch=2)
+    sess = CudaSessionBuilder(model).build()
+    want = sess.run(list(feeds.values()))
+    ins = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in feeds.values()]
+    outs = [torch.zeros(s, device="cuda") for s, _ in sess.output_info]
+    torch.cuda.synchronize()
+    cuda = ctypes.CDLL("libcuda.so.1")
+    ctx, dev = ctypes.c_void_p(), ctypes.c_int()
+    assert cuda.cuDeviceGet(ctypes.byref(dev), 0) == 0 and cuda.cuCtxCreate_v2(ctypes.byref(ctx), 0, dev) == 0
+    try:
+        for got, w in zip(sess.run(list(feeds.values())), want):
+            assert np.array_equal(got, w)
+        sess.run_device([t.data_ptr() for t in ins], [t.data_ptr() for t in outs])
+    finally:
+        cuda.cuCtxDestroy_v2(ctx)
+    torch.cuda.synchronize()
+    for got, w in zip(outs, want):
+        assert np.array_equal(got.cpu().numpy(), w)
+    sess.close()
+
+
 @pytest.mark.parametrize("fn,kw", [(configs.mnist_cnn, {}), (configs.mobilenet_v3_large, dict(batch=2)),
                                    (configs.vit_base_16, dict(batch=1, depth=1)), (configs.vit_base_16, dict(batch=32, depth=1))])
 def test_a_planned_schedule_is_the_one_that_runs(cuda_lib, fn, kw):
