@@ -209,7 +209,7 @@ int effective_pairs(const AcSession& s) {
 }
 
 bool flash_attention_applies(const AcSession& s, const AttentionFusion& f) {
-  return s.opt.gemm_mode == 0 && effective_pairs(s) == 2 && !std::getenv("ALTIUS_CUDA_NO_ATTENTION_TMA") &&
+  return s.opt.gemm_mode == 0 && !s.wide && effective_pairs(s) == 2 && !std::getenv("ALTIUS_CUDA_NO_ATTENTION_TMA") &&
          f.q.src == f.k.src && f.q.src == f.v.src && !s.values[f.q.src].is_const && s.values[f.q.src].elem_ty == AC_F32 &&
          attention_flash16_shape_ok((int)f.q.hd, (int)f.q.T, f.q.C, f.q.col, f.k.col, f.v.col, f.q.H * f.q.hd,
                                     f.q.T * f.q.H * f.q.hd);
@@ -790,7 +790,7 @@ bool presplit_applies(const AcSession& s, const GemmShape& g, bool b_const, int6
 // The same operands on the kernel for few rows, where it is the faster one (only for an A whose
 // producer writes the halves: a split kernel in front would cost what it saves).
 bool gemm_ks_applies(const AcSession& s, const GemmShape& g, bool b_const, int64_t a_off, int64_t b_off) {
-  if (s.opt.gemm_mode != 0 || effective_pairs(s) != 2 || !b_const || g.batch != 1 || g.ta || a_off != 0 ||
+  if (s.opt.gemm_mode != 0 || s.wide || effective_pairs(s) != 2 || !b_const || g.batch != 1 || g.ta || a_off != 0 ||
       b_off != 0 || g.lda != g.k || gemm_rows_applies(s, g, b_const, a_off, b_off))
     return false;
   if (g.tb ? (g.ldb % 4) != 0 : (g.k % 4) != 0) return false;
@@ -951,6 +951,7 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   const auto sp_a = em.c.split.find(a);
   const bool use_ks = b16_ok && sp_a != em.c.split.end() && sp_a->second.by_producer && b_row_scale < 0 && gemm_ks_applies(*s, g, true, a_off, b_off) &&
                       gemm_ks_epilogue_ok(act, bias_m >= 0, c_in >= 0, alpha, bias_scale) && c_off == 0 && g.ldc == g.n;
+  if (use_ks) s->narrow = true;
   const bool pre = b16_ok && (use_ks || presplit_applies(*s, g, true, a_off, b_off));
   if (b16_ok) {
     ldb16 = (g.k + 7) / 8 * 8;
@@ -1551,6 +1552,7 @@ void lower_node(Emit& em, Plan& plan, int nid) {
         std::vector<int> awrites;
         if (o_fp32) awrites.push_back(f.out);
         if (o16_hi >= 0) { awrites.push_back(o16_hi); awrites.push_back(o16_lo); }
+        if (flash) s->narrow = true;
         if (tc16 || flash) {
           const int in_hi = si->second.hi, in_lo = si->second.lo;
           em.add(tc16 ? "attention_tma_tcgen05" : "attention_flash_tcgen05", n.op, {in_hi, in_lo, f.scale}, awrites, bytes, flops,

@@ -335,10 +335,31 @@ std::unique_ptr<GraphCopy> copy_graph(const AcGraphDesc& g) {
   return c;
 }
 
-int create_session(const AcGraphDesc* graph, const AcOptions* options, AcSession** out);
+int create_session(const AcGraphDesc* graph, const AcOptions* options, AcSession** out, bool wide = false);
 
-// Second session on the 3xTF32 path, built from the kept description; its initializers
-// are read from this session's weight blob (or the host copies of the small ones).
+// What a session holds on the device for its runs.
+void release_runs(AcSession* s) {
+  if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
+  if (s->graph) cudaGraphDestroy(s->graph);
+  s->graph_exec = nullptr;
+  s->graph = nullptr;
+  destroy_segments(s->segments, destroy_segment);
+  for (int k = 0; k < 2; ++k) {
+    for (void*& p : s->staging[k]) {
+      if (p) cudaFree(p);
+      p = nullptr;
+    }
+  }
+  if (s->arena) cudaFree(s->arena);
+  if (s->weights) cudaFree(s->weights);
+  s->arena = s->weights = nullptr;
+}
+
+// The session that takes over when an operand has left the fp16 range, built from the kept description; its
+// initializers are read from this session's weight blob (or the host copies of the small ones). A plan with
+// operands on the fixed scale that could do without it (|x| <= 255: the cluster GEMM, attention in blocks
+// of keys) gives way to the same mode without these, whose range is 65504 there; only a plan that has left that
+// too, to the 3xTF32 one. The session that is left keeps no memory.
 int create_fallback(AcSession* s) {
   if (s->fallback) return AC_OK;
   if (!s->desc) return set_err(s, AC_ERR_CUDA, "an operand exceeds the fp16 range and no fallback description was kept");
@@ -364,9 +385,15 @@ int create_fallback(AcSession* s) {
   g.n_inputs = (int32_t)c.inputs.size(); g.inputs = c.inputs.data();
   g.n_outputs = (int32_t)c.outputs.size(); g.outputs = c.outputs.data();
   AcOptions o = s->opt;
-  o.gemm_mode = 3;
-  const int rc = create_session(&g, &o, &s->fallback);
-  if (rc != AC_OK) return set_err(s, rc, "building the 3xTF32 fallback failed: " + g_create_error);
+  const bool same_mode = s->narrow && !s->wide;
+  if (!same_mode) o.gemm_mode = 3;
+  int rc = create_session(&g, &o, &s->fallback, same_mode);
+  if (rc == -kGemmRangeCode) {
+    o.gemm_mode = 3;
+    rc = create_session(&g, &o, &s->fallback);
+  }
+  if (rc != AC_OK) return set_err(s, rc, "building the fallback failed: " + g_create_error);
+  release_runs(s);
   return AC_OK;
 }
 
@@ -480,13 +507,14 @@ int altius_cuda_device_count(void) {
 }  // extern "C"
 
 namespace {
-int create_session(const AcGraphDesc* graph, const AcOptions* options, AcSession** out) {
+int create_session(const AcGraphDesc* graph, const AcOptions* options, AcSession** out, bool wide) {
   if (!graph || !out) return set_err(nullptr, AC_ERR_INVALID, "null argument");
   *out = nullptr;
   AcSession* s = new AcSession();
   try {
     if (options) s->opt = *options;
     s->device = s->opt.device;
+    s->wide = wide;
     if (s->opt.plan_only) {
       parse_graph(*s, *graph);
       infer_shapes(*s);
@@ -716,16 +744,16 @@ int altius_cuda_value_info(const AcSession* s, int32_t value, AcValueDesc* out) 
 }
 
 int64_t altius_cuda_launches_per_run(const AcSession* s) {
-  if (s && s->use_fallback) s = s->fallback;
+  while (s && s->use_fallback) s = s->fallback;
   return s ? s->launches_per_run : -1;
 }
 uint64_t altius_cuda_arena_bytes(const AcSession* s) {
-  if (s && s->use_fallback) s = s->fallback;
+  while (s && s->use_fallback) s = s->fallback;
   return s ? s->arena_bytes : 0;
 }
 
 int altius_cuda_profile(AcSession* s, AcProfileEntry* entries, size_t* n) {
-  if (s && s->use_fallback) s = s->fallback;
+  while (s && s->use_fallback) s = s->fallback;
   if (!s || !n) return AC_ERR_INVALID;
   const size_t cap = *n;
   size_t i = 0;
@@ -746,7 +774,7 @@ int altius_cuda_profile(AcSession* s, AcProfileEntry* entries, size_t* n) {
 }
 
 int altius_cuda_schedule(const AcSession* s, AcProfileEntry* entries, size_t* n) {
-  if (s && s->use_fallback) s = s->fallback;
+  while (s && s->use_fallback) s = s->fallback;
   if (!s || !n) return AC_ERR_INVALID;
   const size_t cap = *n;
   for (size_t i = 0; i < s->steps.size() && entries && i < cap; ++i) {
@@ -762,7 +790,7 @@ int altius_cuda_schedule(const AcSession* s, AcProfileEntry* entries, size_t* n)
 }
 
 int altius_cuda_profile_reset(AcSession* s) {
-  if (s && s->use_fallback) s = s->fallback;
+  while (s && s->use_fallback) s = s->fallback;
   if (!s) return AC_ERR_INVALID;
   s->profile.clear();
   return AC_OK;
@@ -776,22 +804,16 @@ void altius_cuda_destroy(AcSession* s) {
   if (!s) return;
   if (s->fallback) altius_cuda_destroy(s->fallback);
   if (s->stream) cudaSetDevice(s->device);
-  if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
-  if (s->graph) cudaGraphDestroy(s->graph);
+  release_runs(s);
   for (cudaEvent_t ev : s->events)
     if (ev) cudaEventDestroy(ev);
-  destroy_segments(s->segments, destroy_segment);
   if (s->sweep_buf) cudaFree(s->sweep_buf);
   for (int k = 0; k < 2; ++k) {
-    for (void* p : s->staging[k])
-      if (p) cudaFree(p);
     if (s->staged[k]) cudaEventDestroy(s->staged[k]);
     if (s->consumed[k]) cudaEventDestroy(s->consumed[k]);
   }
   if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
   if (s->host_block) cudaFreeHost(s->host_block);
-  if (s->arena) cudaFree(s->arena);
-  if (s->weights) cudaFree(s->weights);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
 }

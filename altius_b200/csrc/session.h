@@ -126,16 +126,19 @@ struct AcSession {
   std::map<std::string, ac::ProfileAcc> profile;
   int64_t launches_per_run = 0;
   std::string err;
-  // gemm_mode 0 only: when an operand of an fp16-split GEMM turns out not to fit fp16,
-  // a second session lowered with gemm_mode 3 (3xTF32) takes over for good.
   // run_batches: second stream, two sets of device staging buffers for the inputs, events
   cudaStream_t copy_stream = nullptr;
   std::vector<void*> staging[2];
   cudaEvent_t staged[2] = {nullptr, nullptr};    // H2D of a staging set has landed
   cudaEvent_t consumed[2] = {nullptr, nullptr};  // the set has been copied into the arena
+  // gemm_mode 0 only: when an operand of an fp16-split product turns out not to fit its range, another session
+  // takes over for good: one lowered without the kernels that `narrow` stands for (`wide`), or with
+  // gemm_mode 3 (3xTF32).
   std::unique_ptr<ac::GraphCopy> desc;
   AcSession* fallback = nullptr;
   bool use_fallback = false;
+  bool wide = false;                   // no operands on the fixed scale but those of the CTA-pair GEMM and its attention
+  bool narrow = false;                 // lowered with some that a wide plan does without
   // run / run_device / run_batches / time_device_runs share the arena, the staging buffers, the
   // error word and the fallback switch: one caller at a time per session (recursive: a run
   // re-enters itself once when it switches to the fallback plan).

@@ -76,3 +76,28 @@ def test_flash_attention(cuda_lib, B, T, H, scale_op, projection, peaks):
     err = np.abs(got - want)
     print("largest share of the bound", (err / bound).max(), "rel", np.linalg.norm(got - want) / np.linalg.norm(want))
     assert (err <= bound).all()
+
+
+def test_values_beyond_the_fixed_scale_take_the_plan_without_it(cuda_lib):
+    """Values of up to 4000 leave the fixed scale (255): the session goes on with the operators one by one, in
+    the same mode; the products of constant weights stay on fp16 halves, which hold 65504."""
+    B, T, H = 2, 300, 2
+    D = 64 * H
+    rng = np.random.default_rng(1)
+    x = rng.standard_normal((B, T, D)).astype(np.float32)
+    w = (rng.standard_normal((D, 3 * D)) / np.sqrt(D)).astype(np.float32)
+    w[:, 2 * D:] *= 1000
+    b = np.zeros(3 * D, np.float32)
+    sess = CudaSessionBuilder(_model(B, T, H, w, b, "Mul", True)).build()
+    try:
+        assert "attention_flash_tcgen05" in [e["kind"] for e in sess.schedule()]
+        for _ in range(2):
+            got = sess.run([x])[0]
+        kinds = [e["kind"] for e in sess.schedule()]
+        assert "attention_flash_tcgen05" not in kinds and "softmax_scaled" in kinds
+        assert any(k.startswith("gemm_f16x3") for k in kinds), kinds
+    finally:
+        sess.close()
+    q, k, v = [u.reshape(B, T, H, 64).transpose(1, 2) for u in (torch.from_numpy(x).double() @ torch.from_numpy(w).double()).split(D, dim=2)]
+    want = (torch.softmax(0.125 * (q @ k.transpose(2, 3)), dim=-1) @ v).transpose(1, 2).reshape(B, T, D).numpy()
+    assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)

@@ -196,3 +196,34 @@ def test_few_row_products_on_clusters(cuda_lib, m, d, hidden):
     want = t(x) + a @ t(w2) + t(b2)
     bound = 1.13 * e1 @ t(w2).abs() + 1e-5 * want.abs() + 6e-6 * (a.abs() @ t(w2).abs())
     assert (np.abs(got - want.numpy()) <= bound.numpy()).all()
+
+
+def test_few_row_products_beyond_the_fixed_scale(cuda_lib):
+    """A hidden layer of magnitude 1000 leaves the fixed scale of the halves (255): the session goes on with the
+    kernels that split their operand themselves (65504), and only beyond that with 3xTF32."""
+    m, d, hidden = 197, 384, 1536
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal((m, d)).astype(np.float32)
+    w1 = (1000 * rng.standard_normal((d, hidden)) / np.sqrt(d)).astype(np.float32)
+    w2 = (rng.standard_normal((hidden, d)) / np.sqrt(hidden)).astype(np.float32)
+    w3 = (rng.standard_normal((d, d)) / np.sqrt(d)).astype(np.float32)
+    g = ir.Graph()
+    one, zero = g.new_init(np.ones(d, np.float32)), g.new_init(np.zeros(d, np.float32))
+    xi, scale = g.add_input("x", x.shape), g.add_input("scale", (1,))
+    h = g.op("LayerNormalization", xi, one, zero, axis=-1, epsilon=1e-6, stash_type=1)
+    g.outputs.append(g.op("MatMul", g.op("Gelu", g.op("MatMul", h, g.new_init(w1))), g.new_init(w2)))
+    g.outputs.append(g.op("MatMul", g.op("Mul", xi, scale), g.new_init(w3)))
+    sess = CudaSessionBuilder(ir.Model(g, 13)).build()
+    kinds = lambda: {e["kind"] for e in sess.schedule()}
+    t = lambda a: torch.from_numpy(a).double()
+    ln = lambda a: torch.nn.functional.layer_norm(a, (d,), None, None, 1e-6)
+    want = [torch.nn.functional.gelu(ln(t(x)) @ t(w1), approximate="tanh") @ t(w2), t(x) @ t(w3)]
+    try:
+        assert "gemm_f16x3_cluster_tcgen05" in kinds()
+        for factor, there in ((1.0, {"gemm_f16x3_tcgen05"}), (1.0, {"gemm_f16x3_tcgen05"}), (1e6, {"gemm_tf32x3_tcgen05"})):
+            got = sess.run([x, np.array([factor], np.float32)])
+            assert {k for k in kinds() if k.startswith("gemm")} == there, kinds()
+            for a, b in zip(got, (want[0], factor * want[1])):
+                assert np.linalg.norm(a - b.numpy()) <= 1e-5 * np.linalg.norm(b.numpy())
+    finally:
+        sess.close()
