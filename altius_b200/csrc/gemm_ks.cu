@@ -3,8 +3,9 @@
 // kind::f16 MMAs per product -- the operand formats of the CTA-pair kernel (gemm_tc.cu), which takes
 // the larger problems. The tensor core truncates its sum at every instruction, an error that grows with the
 // number of instructions behind one another on an accumulator of full size; so the cross terms
-// (2^-11 of the result) have an accumulator of their own and the others are dealt to three
-// (197 x 768 x 2304: relative error against 64 bits 9.8e-7 in one accumulator, 1.6e-7 this way; the pair kernel 3.5e-7).
+// (2^-11 of the result) have an accumulator of their own and the others are dealt to as many as
+// tensor memory holds beside it, K-block by K-block in turn
+// (197 x 768 x 2304: relative error against 64 bits 9.8e-7 in one accumulator, 1.2e-7 this way; the pair kernel 3.5e-7).
 //
 // What bounds it: 197 rows against 768 x 2304 are 2.1 GFLOP and 7 MB of weights, 1.2 us of either, so what
 // counts is latency. On 256 x 256 tiles such a product has 9 tiles for 74 pairs; cut along K its
@@ -69,10 +70,10 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   float4* part = reinterpret_cast<float4*>(smem + S * stage_bytes);   // [parts][quads][BM + 1]
   const int nkb = (p.k + KB - 1) / KB, kb0 = rank * p.kper, kbs = min(nkb, kb0 + p.kper) - kb0;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * bn;
-  // Accumulators: the cross terms have one of their own, the products of the high halves up to three, K-block by
-  // K-block in turn.
-  const uint32_t set = bn <= 32 ? 32 : bn <= 64 ? 64 : 128, cols = 4 * set;
-  const int mains = min(3, kbs);
+  // Accumulators of bn columns: the cross terms have the first, the products of the high halves the others. (Three
+  // at most, for any width, left 394 x 384 x 1152 at 1.66e-7 where the kernel it replaces has 1.42e-7.)
+  const int mains = min(512 / bn - 1, kbs);
+  const uint32_t cols = bn * (mains + 1) <= 64 ? 64 : bn * (mains + 1) <= 128 ? 128 : bn * (mains + 1) <= 256 ? 256 : 512;
   cg::cluster_group cl = cg::this_cluster();
   if (parts > 1) cl.barrier_arrive();         // answered before the first write to another block's memory
   if (tid == 0) {
@@ -224,7 +225,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
           const uint64_t db = desc_sw128(a + 2 * kAHalf), dbl = desc_sw128(a + 2 * kAHalf + bhalf);
           // Always four steps (what lies beyond K arrives as zeros): with a run-time count an instruction
           // took 113 clocks to issue, unrolled 57 (96 columns).
-          const uint32_t cross = tmem, main = tmem + (uint32_t)(1 + it % mains) * set;
+          const uint32_t cross = tmem, main = tmem + (uint32_t)((1 + it % mains) * bn);
 #pragma unroll
           for (int kk = 0; kk < KB / 16; ++kk) {
             const uint64_t off = (uint64_t)(kk * 32 >> 4);
@@ -244,20 +245,23 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       const int row = (warp & 3) * 32 + lane;
       const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
       for (int c = (warp >> 2) * 16; c < bn; c += 64) {
-        uint32_t u[16];
-        uint32_t v[3][16];
-        tc_ld_32x16_nowait(base + (uint32_t)c, u);
+        const uint32_t at = base + (uint32_t)c;
+        uint32_t u[16], x[16], y[16];
+        auto plus = [](uint32_t (&a)[16], const uint32_t (&b)[16]) {
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-          if (a < mains) tc_ld_32x16_nowait(base + (uint32_t)c + (uint32_t)(1 + a) * set, v[a]);
-        tc_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float x = __uint_as_float(v[0][i]);
-          if (mains > 1) x = __fadd_rn(x, __uint_as_float(v[1][i]));
-          if (mains > 2) x = __fadd_rn(x, __uint_as_float(v[2][i]));
-          u[i] = __float_as_uint(__fadd_rn(x, __uint_as_float(u[i])));
+          for (int i = 0; i < 16; ++i) a[i] = __float_as_uint(__fadd_rn(__uint_as_float(a[i]), __uint_as_float(b[i])));
+        };
+        tc_ld_32x16_nowait(at + (uint32_t)bn, u);
+        for (int a = 2; a <= mains; a += 2) {       // two accumulators on their way at once, added in order
+          tc_ld_32x16_nowait(at + (uint32_t)(a * bn), x);
+          if (a < mains) tc_ld_32x16_nowait(at + (uint32_t)((a + 1) * bn), y);
+          tc_wait_ld();
+          plus(u, x);
+          if (a < mains) plus(u, y);
         }
+        tc_ld_32x16_nowait(at, x);
+        tc_wait_ld();
+        plus(u, x);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int cq = c / 4 + i, owner = (int)(((unsigned)cq * (unsigned)p.inv) >> 20);
