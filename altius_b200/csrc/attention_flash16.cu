@@ -16,13 +16,19 @@
 //                 registers: block maximum (exchanged by the two), then P = 2^(t - m + 9) split
 //                 into fp16 hi / lo over the scores it came from.
 //
+// An accumulator takes the products of two blocks of keys; then the softmax threads add it, in fp32, to sums
+// of their own in memory (32 KB per group, in L2) and the next block starts it again: with all blocks of
+// 577 tokens on one the result was off by 8.8e-7 of it (fp32 products: 7.5e-7), this way by 4.9e-7.
+//
 // The rows' reference m follows the maximum lazily: as long as no row of a warp has exceeded its m by
 // more than 4 (in powers of two) nothing is rescaled and P stays below 2^13; otherwise the warp
 // waits for the last product and multiplies its part of O by 2^(m - m').
 //
 // P V as two instructions per 16 keys instead of three: V hi and V lo are neighbours along N, so
-// P_hi * [V_hi | V_lo] goes to 128 accumulator columns in one MMA and P_lo * V_hi adds to the first 64;
-// the two halves are added when O is read. An instruction costs 105 to 150 clocks whatever its width
+// P_hi * [V_hi | V_lo] goes to 128 accumulator columns in one MMA and P_lo * V_hi adds to the last 64;
+// the two halves are added when O is read. The tensor core truncates its sum at every instruction by
+// up to an ulp of the sum, so what is small is added where or while the sum is small: the cross terms of
+// P V have those 64 columns to themselves, and those of Q K^T come before its main terms. An instruction costs 105 to 150 clocks whatever its width
 // (attention_tc16.cu), so the count is what bounds the kernel: 28 per block of keys.
 //
 // Tensor memory: S / P of group g in columns [128 g, 128 g + 128), O in [256 + 128 g, ...). Every wait
@@ -47,6 +53,7 @@ constexpr int kMmaWarp = 16, kTmaWarp = 17, kLaunch = 18 * 32;
 constexpr int kTile = 128 * 128;                // bytes of one operand's hi (or lo): 128 rows of 128 bytes
 constexpr int kGroupBytes = 6 * kTile;          // Q, K, V, each hi and lo
 constexpr uint32_t kOCol = 256;
+constexpr int kRun = 2;                         // blocks of keys whose products share an accumulator
 constexpr uint32_t kPollLimit = 1u << 26;
 
 struct FlashDev {
@@ -55,6 +62,7 @@ struct FlashDev {
   int heads, tokens, tiles, items;
   int q_col, k_col, v_col;
   const float* scale; int scale_mode;
+  float* sums;                                  // [grid][group][64 columns][128 rows], with more than kRun blocks of keys
   int* err;
 };
 
@@ -201,10 +209,10 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
             const uint32_t id64 = (1u << 4) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(QM >> 4) << 24);
             const uint64_t v = desc_mn128(base + 4 * kTile);
             auto hi = [&](int c) {              // P_hi * [V_hi | V_lo]
-              mma_f16_ta(o_col, s_col + (uint32_t)(16 * c), v + (uint64_t)(c * 128), id128, (j > 0 || c > 0) ? 1u : 0u);
+              mma_f16_ta(o_col, s_col + (uint32_t)(16 * c), v + (uint64_t)(c * 128), id128, (j % kRun > 0 || c > 0) ? 1u : 0u);
             };
-            auto lo = [&](int c) {              // P_lo * V_hi
-              mma_f16_ta(o_col, s_col + (uint32_t)(16 * c + 8), v + (uint64_t)(c * 128), id64, 1u);
+            auto lo = [&](int c) {              // P_lo * V_hi, beside the other cross terms
+              mma_f16_ta(o_col + (uint32_t)HD, s_col + (uint32_t)(16 * c + 8), v + (uint64_t)(c * 128), id64, 1u);
             };
             if (chunks == KV / 16) {            // unrolled: half the time to issue an instruction
 #pragma unroll
@@ -230,10 +238,14 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
             const uint64_t q_hi = desc_k128(base), q_lo = desc_k128(base + kTile);
             const uint64_t k_hi = desc_k128(base + 2 * kTile), k_lo = desc_k128(base + 3 * kTile);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
+            for (int kk = 0; kk < 4; ++kk) {   // the cross terms, 2^-11 of the scores, while the sum is small
               const uint64_t off = (uint64_t)(kk * 32 >> 4);
               tc_mma_f16(s_col, q_lo + off, k_hi + off, idesc, kk ? 1u : 0u);
               tc_mma_f16(s_col, q_hi + off, k_lo + off, idesc, 1u);
+            }
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+              const uint64_t off = (uint64_t)(kk * 32 >> 4);
               tc_mma_f16(s_col, q_hi + off, k_hi + off, idesc, 1u);
             }
             tc_commit(&bar.s_full[g]);
@@ -253,6 +265,7 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
     const int row = q * 32 + lane;
     float(*xch)[QM] = xch_all[g];
     const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+    float* sums = p.sums + ((size_t)(2 * blockIdx.x + g) * HD + hf * 32) * QM + row;   // [column][row], written and read by this thread only
     const uint32_t scol = trow + (uint32_t)(g * 128 + hf * 64), ocol = trow + kOCol + (uint32_t)(g * 128 + hf * 32);
     // Scores arrive as (q * 2^8) . (k * 2^8); t = acc * c1 with c1 = 2^-16 * log2(e) (* | /) scale.
     const float kLog2e = 1.44269504088896341f;
@@ -265,7 +278,7 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
     const int my_items = items_of(g);
 #pragma unroll 1
     for (int k = 0; k < my_items; ++k) {
-      float ref = 0.f, sum = 0.f;
+      float ref = 0.f, sum = 0.f, since = 1.f;  // since: factor of the moves of ref since `sums` was written
 #pragma unroll 1
       for (int j = 0; j < blocks; ++j, ++nb) {
         const int left = T - j * KV - hf * 64;  // keys of this thread's half that exist
@@ -290,23 +303,46 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
         pair_sync(g, q);
         m = fmaxf(xch[0][row], xch[1][row]);
         pair_sync(g, q);
-        if (j == 0) {
-          ref = m;
-        } else if (__any_sync(0xffffffffu, m > ref + 4.f)) {   // the same rows, so the same vote, in both warps
+        const bool move = j > 0 && __any_sync(0xffffffffu, m > ref + 4.f);   // the same rows, so the same vote, in both warps
+        const bool flush = j > 0 && j % kRun == 0;             // this block's products start the accumulator again
+        if (j == 0) ref = m;
+        if (flush || move) {
+          // Free: the scores that have just been read came behind these products in the pipe.
+          if (ok && !warp_mbar_wait(&bar.pv_done[g], (uint32_t)((nb - 1) & 1), lane)) { atomicExch(p.err, 55); ok = false; }
+          tc_fence_after();
+        }
+        if (flush) {
+#pragma unroll
+          for (int part = 0; part < 2; ++part) {   // this warp's 32 columns
+            uint32_t o[16], ol[16];
+            tc_ld_32x16_nowait(ocol + (uint32_t)(part * 16), o);
+            tc_ld_32x16_nowait(ocol + (uint32_t)(HD + part * 16), ol);
+            tc_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              float* at = sums + (part * 16 + e) * QM;
+              const float x = __fadd_rn(__uint_as_float(o[e]), __uint_as_float(ol[e]));
+              *at = j == kRun ? x : fmaf(*at, since, x);
+            }
+          }
+          since = 1.f;
+        }
+        if (move) {
           const float next = fmaxf(ref, m), f = ex2(__fsub_rn(ref, next));
           ref = next;
           sum = __fmul_rn(sum, f);
-          if (ok && !warp_mbar_wait(&bar.pv_done[g], (uint32_t)((nb - 1) & 1), lane)) { atomicExch(p.err, 55); ok = false; }
-          tc_fence_after();
+          since = __fmul_rn(since, f);
+          if (!flush) {
 #pragma unroll
-          for (int part = 0; part < 4; ++part) {   // this warp's 32 columns of both halves of O
-            const uint32_t at = ocol + (uint32_t)((part >> 1) * 64 + (part & 1) * 16);
-            uint32_t o[16];
-            tc_ld_32x16_nowait(at, o);
-            tc_wait_ld();
+            for (int part = 0; part < 4; ++part) {   // this warp's 32 columns of both halves of O
+              const uint32_t at = ocol + (uint32_t)((part >> 1) * 64 + (part & 1) * 16);
+              uint32_t o[16];
+              tc_ld_32x16_nowait(at, o);
+              tc_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__fmul_rn(__uint_as_float(o[e]), f));
-            st16(at, o);
+              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__fmul_rn(__uint_as_float(o[e]), f));
+              st16(at, o);
+            }
           }
         }
         const float off = __fsub_rn(ref, 9.f);
@@ -360,8 +396,11 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
         for (int i = 0; i < 2; ++i) {
           float y[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
-            y[e] = __fmul_rn(__fadd_rn(__uint_as_float(o[8 * i + e]), __uint_as_float(ol[8 * i + e])), recip);
+          for (int e = 0; e < 8; ++e) {
+            y[e] = __fadd_rn(__uint_as_float(o[8 * i + e]), __uint_as_float(ol[8 * i + e]));
+            if (blocks > kRun) y[e] = fmaf(sums[(half * 16 + 8 * i + e) * QM], since, y[e]);
+            y[e] = __fmul_rn(y[e], recip);
+          }
           const float4 y0 = make_float4(y[0], y[1], y[2], y[3]), y1 = make_float4(y[4], y[5], y[6], y[7]);
           const long long at = ob + half * 16 + 8 * i;
           if (p.out) {
@@ -413,6 +452,11 @@ bool attention_flash16_shape_ok(int head_dim, int tokens, int64_t ld16, int64_t 
          (out_row_stride % 8) == 0 && (out_batch_stride % 8) == 0;
 }
 
+int64_t attention_flash16_workspace(int64_t batch, int64_t heads, int64_t tokens) {
+  const int64_t items = batch * heads * ((tokens + QM - 1) / QM);
+  return tokens > kRun * KV ? std::min<int64_t>(items, device_sm_count()) * 2 * HD * QM : 0;
+}
+
 cudaError_t launch_attention_flash16(const Attention16Params& p, cudaStream_t st) {
   auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if (!attention_flash16_shape_ok(p.head_dim, p.tokens, p.ld16, p.q_col, p.k_col, p.v_col, p.out_row_stride, p.out_batch_stride) ||
@@ -428,6 +472,8 @@ cudaError_t launch_attention_flash16(const Attention16Params& p, cudaStream_t st
   d.q_col = (int)p.q_col; d.k_col = (int)p.k_col; d.v_col = (int)p.v_col;
   d.scale = p.scale; d.scale_mode = p.scale ? p.scale_mode : 0;
   d.err = p.err_word;
+  d.sums = p.workspace;
+  if (p.tokens > kRun * KV && !p.workspace) return cudaErrorInvalidValue;
   if (d.scale_mode == 1) return launch_mode<1>(p, d, st);
   if (d.scale_mode == 2) return launch_mode<2>(p, d, st);
   return launch_mode<0>(p, d, st);

@@ -332,6 +332,7 @@ struct Attention16Params {
   int batch, heads, tokens, head_dim;
   const float* scale; int scale_mode;                     // device scalar or null; 1: multiply, 2: divide
   int* err_word;
+  float* workspace;                                       // attention_flash16_workspace floats
 };
 bool attention_tc16_shape_ok(int head_dim, int tokens, int64_t ld16, int64_t q_col, int64_t k_col, int64_t v_col,
                              int64_t out_row_stride, int64_t out_batch_stride);
@@ -340,6 +341,7 @@ cudaError_t launch_attention_tc16(const Attention16Params& p, cudaStream_t st);
 // The same operands and result for any number of tokens: keys in blocks with a running maximum.
 bool attention_flash16_shape_ok(int head_dim, int tokens, int64_t ld16, int64_t q_col, int64_t k_col, int64_t v_col,
                                 int64_t out_row_stride, int64_t out_batch_stride);
+int64_t attention_flash16_workspace(int64_t batch, int64_t heads, int64_t tokens);
 cudaError_t launch_attention_flash16(const Attention16Params& p, cudaStream_t st);
 
 }  // namespace ac

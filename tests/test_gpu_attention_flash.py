@@ -33,13 +33,15 @@ def _model(B, T, H, w, b, scale_op, projection):
     return ir.Model(g, 13)
 
 
-# Tokens: one block and its edges, several blocks with a last one of 1, 65 and 128 keys, tiles of one row;
+# Tokens: two blocks and their edges, several with a last one of 1, 65, 76 and 128 keys, tiles of one row, sums of
+# one and more runs of two blocks, in the last one a run of one block;
 # items: fewer than blocks, a second round for some groups; "peaks" makes the running maximum move by more
 # than the lazy threshold in every block.
 @pytest.mark.parametrize("B,T,H,scale_op,projection,peaks", [
-    (64, 37, 12, "Mul", True, False), (40, 64, 12, "Div", True, False), (12, 209, 12, "Mul", True, False),
+    (3, 129, 12, "Mul", True, False), (6, 200, 12, "Div", True, False), (12, 209, 12, "Mul", True, False),
     (9, 256, 12, "Mul", True, True), (2, 257, 2, "Mul", False, False), (1, 577, 12, "Mul", False, True),
-    (5, 577, 12, "Mul", True, False), (3, 321, 1, "Div", False, True), (1, 1024, 3, None, False, False)])
+    (5, 577, 12, "Mul", True, False), (3, 321, 1, "Div", False, True), (1, 1024, 3, None, False, False),
+    (2, 513, 3, "Mul", False, True), (3, 1100, 2, "Mul", False, True)])
 def test_flash_attention(cuda_lib, B, T, H, scale_op, projection, peaks):
     rng = np.random.default_rng(T + H)
     D = 64 * H

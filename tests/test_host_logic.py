@@ -164,6 +164,19 @@ def test_narrow_transformers_lower(dim, heads):
             plan(configs.vision_transformer(batch, dim, 2, heads, 4 * dim, 1, img=px)[0])
 
 
+@pytest.mark.parametrize("px,batch,kind", [(96, 1, "attention_fused"), (96, 32, "attention_fused"), (112, 8, "attention_fused"),
+                                           (128, 32, "attention_tma_tcgen05"), (224, 32, "attention_tma_tcgen05"),
+                                           (224, 1, "attention_flash_tcgen05"), (240, 1, "attention_flash_tcgen05"),
+                                           (240, 32, "attention_flash_tcgen05"), (384, 2, "attention_flash_tcgen05")])
+def test_attention_kernel_by_tokens_and_heads(px, batch, kind):
+    """fp32 up to 64 tokens; halves of the projection by TMA, a block per head up to 208 and per tile of queries
+    with few heads and beyond."""
+    model, _ = configs.vision_transformer(batch, 384, 1, 6, 1536, 1, img=px)
+    kinds = [e["kind"] for e in plan(model).schedule()]
+    assert [k for k in kinds if k.startswith("attention")] == [kind]
+    assert "softmax_scaled" not in kinds and "act_f16_split" not in kinds[kinds.index(kind):]
+
+
 def test_errors_are_reported_at_create():
     a = np.zeros((1, 3, 28, 28), np.float32)
     b = np.zeros((3, 1, 2), np.float32)
