@@ -208,10 +208,15 @@ int effective_pairs(const AcSession& s) {
   return s.opt.gemm_pairs == 0 ? 2 : (s.opt.gemm_pairs == 3 ? 0 : s.opt.gemm_pairs);
 }
 
+// Debug toggle: ALTIUS_CUDA_NO_FUSED_SPLIT=1 keeps a split kernel in front of every pair GEMM, and no operand is
+// planned as halves.
+bool fused_split() { return !std::getenv("ALTIUS_CUDA_NO_FUSED_SPLIT"); }
+
 // Up to 64 tokens the fp32 kernel: its error against 64 bits is the smaller one (8 images of 37 tokens behind their
 // projection 4.6e-7 of the result against 5.5e-7; from 129 on this kernel's is), and so is its time with few heads.
 bool flash_attention_applies(const AcSession& s, const AttentionFusion& f) {
-  return f.q.T > 64 && s.opt.gemm_mode == 0 && !s.wide && effective_pairs(s) == 2 && !std::getenv("ALTIUS_CUDA_NO_ATTENTION_TMA") &&
+  return f.q.T > 64 && f.q.B > 0 && s.opt.gemm_mode == 0 && !s.wide && effective_pairs(s) == 2 && fused_split() &&
+         !std::getenv("ALTIUS_CUDA_NO_ATTENTION_TMA") &&
          f.q.src == f.k.src && f.q.src == f.v.src && !s.values[f.q.src].is_const && s.values[f.q.src].elem_ty == AC_F32 &&
          attention_flash16_shape_ok((int)f.q.hd, (int)f.q.T, f.q.C, f.q.col, f.k.col, f.v.col, f.q.H * f.q.hd,
                                     f.q.T * f.q.H * f.q.hd);
@@ -2027,8 +2032,7 @@ void lower_graph(AcSession& s) {
       detect_se_gate(c, plan);
       detect_squeeze(c, plan);
       detect_reduce_siblings(c, plan);
-      // Debug toggle: ALTIUS_CUDA_NO_FUSED_SPLIT=1 keeps a split kernel in front of every pair GEMM.
-      if (!std::getenv("ALTIUS_CUDA_NO_FUSED_SPLIT")) plan_presplit(c, plan);
+      if (fused_split()) plan_presplit(c, plan);
     }
     Emit em(c);
     for (int nid : s.order)

@@ -177,6 +177,27 @@ def test_attention_kernel_by_tokens_and_heads(px, batch, kind):
     assert "softmax_scaled" not in kinds and "act_f16_split" not in kinds[kinds.index(kind):]
 
 
+@pytest.mark.parametrize("toggle,batch", [("ALTIUS_CUDA_NO_FUSED_SPLIT", 2), ("ALTIUS_CUDA_NO_ATTENTION_TMA", 2), (None, 0)])
+def test_long_attention_without_its_kernel_is_separate_operators(monkeypatch, toggle, batch):
+    """Beyond 256 tokens only the kernel on halves of the projection takes the fused chain; where these are not
+    planned, or there is nothing to compute, the operators stay."""
+    if toggle:
+        monkeypatch.setenv(toggle, "1")
+    B, T, H = batch, 300, 2
+    D = 64 * H
+    g = ir.Graph()
+    i64 = lambda v: g.new_init(np.asarray(v, np.int64))
+    qkv = g.op("MatMul", g.add_input("x", (B, T, D)), g.new_init(np.zeros((D, 3 * D), np.float32)))
+    q, k, v = g.add_node("Split", [qkv, i64([D, D, D])], 3, axis=2)
+    heads = lambda t: g.op("Reshape", g.op("Transpose", g.op("Reshape", t, i64([B, T, H, 64])), perm=[0, 2, 1, 3]), i64([B * H, T, 64]))
+    q, k, v = heads(q), heads(k), heads(v)
+    s = g.op("Softmax", g.op("MatMul", q, g.op("Transpose", k, perm=[0, 2, 1])), axis=-1)
+    o = g.op("Reshape", g.op("MatMul", s, v), i64([B, H, T, 64]))
+    g.outputs.append(g.op("Reshape", g.op("Transpose", o, perm=[0, 2, 1, 3]), i64([B, T, D])))
+    kinds = [e["kind"] for e in plan(ir.Model(g, 13)).schedule()]
+    assert "softmax" in kinds and not any(k.startswith("attention") for k in kinds), kinds
+
+
 def test_errors_are_reported_at_create():
     a = np.zeros((1, 3, 28, 28), np.float32)
     b = np.zeros((3, 1, 2), np.float32)
