@@ -218,7 +218,11 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
         const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
         for (int it = 0; it < kbs; ++it) {
           const int s = it % S;
-          if (!mbar_wait(&full[s], (uint32_t)(it / S) & 1)) { atomicExch(p.err, 62); break; }
+          if (!mbar_wait(&full[s], (uint32_t)(it / S) & 1)) {
+            atomicExch(p.err, 62);
+            for (int w = it; w < kbs && w < it + S; ++w) (void)mbar_wait(&full[w % S], (uint32_t)(w / S) & 1);   // copies in flight land
+            break;
+          }
           tc_fence_after();
           const uint32_t a = smem_u32(smem + s * stage_bytes);
           const uint64_t da = desc_sw128(a), dal = desc_sw128(a + kAHalf);
