@@ -17,7 +17,7 @@
 // What bounds it: the layers of the CNNs have K of 16 to 960 and move 0.5 to 100 FMAs per byte. The
 // wide planes are bound by HBM if loads, MMAs and stores of different tiles overlap: two blocks share
 // an SM and each walks tiles; the loads of the next tile are in flight, and its MMAs run into a second
-// accumulator, while a tile is finished and stored. The narrow planes (7 x 7, 14 x 14) have few tiles
+// buffer of accumulators where tensor memory has one, while a tile is finished and stored. The narrow planes (7 x 7, 14 x 14) have few tiles
 // and a long K and are bound by the MMA rate of one SM (about 110 clocks per instruction whatever its
 // width): there a cluster of up to eight blocks cuts K and adds its accumulators up through
 // distributed shared memory, in rank order.
@@ -51,6 +51,7 @@ struct ConvTcDev {
   int m, k, hw, n;          // n = batch * hw columns
   int bn, stages, kper;     // channels per tile, ring entries, K steps per block of the cluster
   int resident;             // the filter tile stays in shared memory (its K steps behind the ring)
+  int set, mains, bufs, cols;   // columns of an accumulator, accumulators of the main terms (0: one for all terms), buffers, columns in all
   long long x_batch, out_batch;
   int ih, iw, ow, kh, kw, sh, sw, dh, dw, pt, pl;
   float act_alpha, act_beta;
@@ -72,7 +73,8 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                : "memory");
 }
 
-template <bool WINDOW, int ACT>
+// ONE: one accumulator for all terms, two buffers (a block that does not walk uses the first).
+template <bool WINDOW, int ACT, bool ONE>
 __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -88,8 +90,10 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
   float* part = reinterpret_cast<float*>(wres + (p.resident ? p.kper * bbytes : 0));   // [parts][bn / parts][PX] sums of the cluster
   int2* tab = reinterpret_cast<int2*>(part + (parts > 1 ? bn * PX : 0));
   const int tiles = (p.n + PX - 1) / PX, mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  const uint32_t set = bn <= 32 ? 32 : bn <= 64 ? 64 : bn <= 128 ? 128 : 256;   // columns of an accumulator
-  const uint32_t cols = gridDim.x < tiles ? 2 * set : set;
+  // Accumulators of a tile: [cross terms | main terms of even | of odd K steps], or one for all.
+  const uint32_t set = p.set, cols = p.cols, span = (p.mains + 1) * set;
+  const int mains = ONE ? 0 : min(p.mains, kbs);   // in use
+  const int two = ONE ? 1 : p.bufs - 1;        // tile i has buffer i & two, for the (i >> two)-th time
   cg::cluster_group cl = cg::this_cluster();
   if (parts > 1) cl.barrier_arrive();          // answered before the first write to another block's memory
 
@@ -226,10 +230,10 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
     uint32_t use = 0, nuse = 0;
     int g = 0;                                 // running K step
     bool alive = true;
-    // Loads tile i (whose first step is already in v) into the ring; leaves the first step of
-    // tile i + 1 in v.
-    auto fill = [&](int i) {
-      for (int kb = 0; kb < kbs && alive; ++kb, ++g) {
+    // Loads steps [from, to) of tile i (the first of them is already in v) into the ring; leaves the step
+    // behind them in v.
+    auto fill = [&](int i, int from, int to) {
+      for (int kb = from; kb < to && alive; ++kb, ++g) {
         const float* gc = gcol;
         if (kb + 1 == kbs) place(i + 1);
         if (kb + 1 < kbs || i + 1 < mine) nuse = fetch(kb + 1 < kbs ? kb + 1 : 0, nx);
@@ -267,24 +271,35 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
     if (mine > 0) {
       place(0);
       use = fetch(0, v);
-      fill(0);
+      fill(0, 0, kbs);
     }
+    // With one buffer the products of tile i + 1 wait for this epilogue: only the ring is filled ahead of it.
+    const int ahead = ONE || two ? kbs : min(kbs, S);
     for (int i = 0; i < mine && alive; ++i) {
-      if (i + 1 < mine) fill(i + 1);
+      if (i + 1 < mine) fill(i + 1, 0, ahead);
       if (!alive) break;
       const int col = ((int)blockIdx.x + i * (int)gridDim.x) * PX + row;
       const bool col_ok = col < p.n;
       const int cc = min(col, p.n - 1), cb = cc / p.hw;
       const long long at = cb * p.out_batch + (cc - cb * p.hw) + (long long)m0 * p.hw;
-      if (!mbar_wait(&acc_full[i & 1], (i >> 1) & 1)) { atomicExch(p.err, 33); abort_flag = 1; break; }
+      if (!mbar_wait(&acc_full[i & two], (i >> two) & 1)) { atomicExch(p.err, 33); abort_flag = 1; break; }
       tc_fence_after();
       const int share = bn / parts;
-      const uint32_t base = tmem + (i & 1) * set + ((uint32_t)((warp & 3) * 32) << 16);
+      const uint32_t base = tmem + (i & two) * span + ((uint32_t)((warp & 3) * 32) << 16);
       for (int c = (warp >> 2) * 16; c < bn && c <= mlast; c += 32) {
         uint32_t u[16];
-        tc_ld_32x16_nowait(base + (uint32_t)c, u);
+        tc_ld_32x16_nowait(base + (uint32_t)c + (mains ? set : 0u), u);
+        auto add = [&](uint32_t from) {          // u += an accumulator, once both are there
+          uint32_t more[16];
+          tc_ld_32x16_nowait(base + (uint32_t)c + from, more);
+          tc_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(__fadd_rn(__uint_as_float(u[j]), __uint_as_float(more[j])));
+        };
         if (parts > 1) {
           // To the block that finishes these channels; no one waits for a remote load.
+          if (mains > 1) add(2 * set);
+          if (mains) add(0u);
           tc_wait_ld();
           int owner = c / share, left = share - c % share;
           for (int j = 0; j < 16;) {           // uniform: channels per owner are a multiple of two
@@ -304,6 +319,8 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) r[j] = *reinterpret_cast<const float*>(rs + (uint32_t)min(j, mlast - c) * hw4);
         }
+        if (mains > 1) add(2 * set);
+        if (mains) add(0u);
         tc_wait_ld();
         float y[16];
 #pragma unroll
@@ -330,7 +347,8 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[i & 1]);
+      if (lane == 0) mbar_arrive(&acc_empty[i & two]);
+      if (!ONE && i + 1 < mine) fill(i + 1, ahead, kbs);
     }
   } else if (elect_one()) {
     // Both operands TF32 (format 2), K-major, fp32 accumulator.
@@ -338,12 +356,12 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
     bool ok = !p.resident || mbar_wait(&w_full, 0);
     if (!ok) { atomicExch(p.err, 34); abort_flag = 1; }
     for (int i = 0, g = 0; i < mine && ok; ++i) {
-      if (i >= 2) {
-        ok = mbar_wait(&acc_empty[i & 1], ((i >> 1) & 1) ^ 1);
+      if (i > two) {
+        ok = mbar_wait(&acc_empty[i & two], ((i >> two) & 1) ^ 1);
         if (!ok) { atomicExch(p.err, 35); abort_flag = 1; break; }
         tc_fence_after();
       }
-      const uint32_t d = tmem + (i & 1) * set;
+      const uint32_t d = tmem + (i & two) * span;
       for (int kb = 0; kb < kbs; ++kb, ++g) {
         const int s = g % S;
         ok = mbar_wait(&full[s], (g / S) & 1);
@@ -353,25 +371,34 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
         const uint32_t b = p.resident ? smem_u32(wres + kb * bbytes) : a + 2 * kABytes;
         const uint64_t da = desc_sw128(a), dal = desc_sw128(a + kABytes);
         const uint64_t db = desc_sw128(b), dbl = desc_sw128(b + bbytes / 2);
+        const uint32_t dm = mains ? d + (uint32_t)(1 + (mains > 1 ? kb & 1 : 0)) * set : d;
         const int steps = min(4, (p.k - (kb0 + kb) * KB + 7) / 8);
-        auto step = [&](int kk) {
+        // The cross terms of a step first: 2^-11 of the result, they are added while its sum may still be small.
+        auto cross = [&](int kk) {
           const uint64_t off = (uint64_t)(kk * 32 >> 4);
           tc_mma_tf32(d, dal + off, db + off, idesc, (kb > 0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
           tc_mma_tf32(d, da + off, dbl + off, idesc, 1u);                             // a_hi * b_lo
-          tc_mma_tf32(d, da + off, db + off, idesc, 1u);                              // a_hi * b_hi
+        };
+        auto main = [&](int kk) {
+          const uint64_t off = (uint64_t)(kk * 32 >> 4);
+          tc_mma_tf32(dm, da + off, db + off, idesc, (ONE || kb >= mains || kk > 0) ? 1u : 0u);   // a_hi * b_hi
         };
         // Full steps unrolled: issuing an instruction took 113 clocks in a loop of run-time length, 40 to
         // 65 (up to 128 channels) this way.
         if (steps == 4) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) step(kk);
+          for (int kk = 0; kk < 4; ++kk) cross(kk);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) main(kk);
         } else {
 #pragma unroll 1
-          for (int kk = 0; kk < steps; ++kk) step(kk);
+          for (int kk = 0; kk < steps; ++kk) cross(kk);
+#pragma unroll 1
+          for (int kk = 0; kk < steps; ++kk) main(kk);
         }
         tc_commit(&empty[s]);
       }
-      if (ok) tc_commit(&acc_full[i & 1]);
+      if (ok) tc_commit(&acc_full[i & two]);
     }
   }
   __syncwarp();
@@ -435,12 +462,17 @@ Shape shape_of(const ConvParams& q) {
   return pick_shape(q, {device_sm_count(), cluster_slots(2), cluster_slots(4), cluster_slots(8)});
 }
 
+template <bool WINDOW, int ACT, bool ONE>
+cudaError_t launch_form(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
+  static unsigned long long done = 0;
+  if (cudaError_t e = ensure_dynamic_smem(conv_tc_kernel<WINDOW, ACT, ONE>, (int)kSmemMax, &done)) return e;
+  const dim3 grid((unsigned)sh.ctas, (unsigned)sh.tiles, (unsigned)sh.split);
+  return launch_pdl(conv_tc_kernel<WINDOW, ACT, ONE>, grid, dim3(kThreads), sh.smem, st, sh.split, p);
+}
+
 template <bool WINDOW, int ACT>
 cudaError_t launch_act(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
-  static unsigned long long done = 0;
-  if (cudaError_t e = ensure_dynamic_smem(conv_tc_kernel<WINDOW, ACT>, (int)kSmemMax, &done)) return e;
-  const dim3 grid((unsigned)sh.ctas, (unsigned)sh.tiles, (unsigned)sh.split);
-  return launch_pdl(conv_tc_kernel<WINDOW, ACT>, grid, dim3(kThreads), sh.smem, st, sh.split, p);
+  return sh.mains == 0 ? launch_form<WINDOW, ACT, true>(p, sh, st) : launch_form<WINDOW, ACT, false>(p, sh, st);
 }
 
 template <bool WINDOW>
@@ -485,6 +517,7 @@ cudaError_t launch_conv_tc(const ConvParams& q, const float* x, const float* pac
   p.m = q.oc; p.k = q.c * q.kh * q.kw; p.hw = q.oh * q.ow; p.n = q.n * p.hw;
   if (p.m == 0 || p.n == 0) return cudaSuccess;
   p.bn = sh.bn; p.stages = sh.stages; p.kper = sh.kper; p.resident = sh.resident;
+  p.set = sh.set; p.mains = sh.mains; p.bufs = sh.bufs; p.cols = sh.cols;
   p.x_batch = (long long)q.c * q.ih * q.iw; p.out_batch = (long long)p.m * p.hw;
   p.ih = q.ih; p.iw = q.iw; p.ow = q.ow; p.kh = q.kh; p.kw = q.kw; p.sh = q.sh; p.sw = q.sw; p.dh = q.dh; p.dw = q.dw;
   p.pt = q.pad_t; p.pl = q.pad_l;

@@ -17,6 +17,7 @@ constexpr int kABytes = PX * KB * 4;         // one of hi / lo
 
 struct Shape {
   int bn, tiles, split, kper, stages, resident, ctas;
+  int set, mains, bufs, cols;                // tensor memory: see the end of pick_shape
   size_t smem;
 };
 
@@ -55,8 +56,8 @@ inline Shape pick_shape(const ConvParams& q, const std::array<int, 4>& slots) {
     }
     if (bn <= 32) break;
   }
-  // Blocks walk tiles when there are more than two per SM (and nothing is cut over a cluster); then
-  // a block needs two accumulators, and those of two blocks fit tensor memory up to 128 channels.
+  // Blocks walk tiles when there are more than two per SM (and nothing is cut over a cluster), two blocks to an SM:
+  // each has half of tensor memory, which holds the accumulators of up to 128 channels.
   const bool walk = best.split == 1 && px * best.tiles > 2 * sms;
   if (walk && best.bn > 128) {
     best.tiles = (q.oc + 127) / 128;
@@ -69,11 +70,23 @@ inline Shape pick_shape(const ConvParams& q, const std::array<int, 4>& slots) {
   auto need = [&](int st) { return bytes(best.bn, best.split, best.kper, st, best.resident); };
   // As many stages as leave room for a second block on the SM, at least two when there are two steps.
   while (best.stages > 2 && need(best.stages) > half) --best.stages;
-  // Shared memory in proportion to the columns of tensor memory, so that whatever blocks share an SM find theirs.
-  // (With 2048 bytes for what lies beside it two blocks of 256 columns missed the SM by 192 bytes, and half of a
-  // grid of two blocks per SM started when the other half had finished.)
-  const int set = best.bn <= 32 ? 32 : best.bn <= 64 ? 64 : best.bn <= 128 ? 128 : 256;
-  best.smem = std::max(need(best.stages), kSmemSm * (walk ? 2 * set : set) / 512 - kSmemBeside);
+  // Accumulators: `set` columns each. The tensor core truncates its sum at every instruction by up to an ulp of
+  // the sum, an error that grows with the instructions behind one another: so the cross terms, 2^-11 of the
+  // result, have an accumulator of their own, and the main terms of narrow tiles, and of a K cut eight times, are
+  // dealt to two, K step by K step. (All on one: 1.3e-6 of the result at 2048 x 7 x 7 into 512, 5.9e-7 at
+  // 480 x 32 x 32 into 480; the GEMM on a column buffer, with its up to 32 slices of K, 3.4e-7 and 2.7e-7; this way
+  // 2.5e-7 and 2.3e-7.) One or two K steps need none of it, all terms are on one (mains 0): no slice of that GEMM
+  // is shorter. Walking blocks have a second buffer of accumulators, so that the products of the next tile run
+  // under the stores of a tile, as far as the columns go.
+  best.set = best.bn <= 32 ? 32 : best.bn <= 64 ? 64 : best.bn <= 128 ? 128 : 256;
+  best.mains = best.kper <= 2 ? 0 : walk || best.set == 256 || (best.set == 128 && best.split < 8) ? 1 : 2;
+  best.bufs = walk && best.set * (best.mains + 1) <= 128 ? 2 : 1;   // mains 0: always two
+  best.cols = 32;
+  while (best.cols < best.set * (best.mains + 1) * best.bufs) best.cols *= 2;
+  // Shared memory in proportion to the columns, so that whatever blocks share an SM find theirs. (With 2048 bytes
+  // for what lies beside it two blocks of 256 columns missed the SM by 192 bytes, and half of a grid of two
+  // blocks per SM started when the other half had finished.)
+  best.smem = std::max(need(best.stages), best.cols == 512 ? kSmemSm / 2 : kSmemSm * best.cols / 512 - kSmemBeside);
   const int resident_blocks = sms * (best.smem <= half ? 2 : 1);
   best.ctas = (int)(walk ? std::min<long long>(px, std::max(1, resident_blocks / best.tiles)) : px);
   return best;

@@ -27,9 +27,9 @@ int main() {
               // What lives on an SM together: 1120 static bytes and 1024 of the system beside the dynamic ones.
               const long long px = ((long long)n * h * h + 127) / 128;
               const int per_sm = (int)std::min<size_t>(7, 233472 / ((s.smem + 1120 + 127) / 128 * 128 + 1024));
-              const int set = s.bn <= 32 ? 32 : s.bn <= 64 ? 64 : s.bn <= 128 ? 128 : 256, columns = s.ctas < px ? 2 * set : set;
               const bool walks = s.ctas < px;
-              const bool fits = per_sm * columns <= 512 && (!walks || s.ctas == 1 || s.ctas * s.tiles <= per_sm * slots[0]);
+              const bool fits = per_sm * s.cols <= 512 && s.cols >= s.set * (s.mains + 1) * s.bufs && s.set >= s.bn && s.cols >= 32 &&
+                                (s.mains > 0 || (s.kper <= 2 && (!walks || s.bufs == 2))) && (!walks || s.ctas == 1 || s.ctas * s.tiles <= per_sm * slots[0]);
               const bool ok = fits && s.bn >= 16 && s.bn <= 256 && s.bn % 16 == 0 && s.tiles >= 1 && s.tiles <= 65535 && (long long)s.tiles * s.bn >= oc &&
                               s.split * s.kper >= nkb && (s.split - 1) * s.kper < nkb && s.ctas >= 1 &&
                               s.stages >= std::min(2, s.kper) && s.stages <= 3 && s.smem <= conv_tc::kSmemMax;
