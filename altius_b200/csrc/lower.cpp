@@ -767,9 +767,14 @@ int new_value(Ctx& c, int64_t numel, bool is_const) {
   return (int)c.s.values.size() - 1;
 }
 
-// Products of a few rows run in fp32 on the kernel that streams B (classifier heads at small batches).
+// Products of a few rows run in fp32 on the kernel that streams B (classifier heads at small batches): up to four
+// rows, and up to 32 while the operands are few, since each eight rows read B again and each pair of columns A.
+// Microseconds with operands in L2 / not, against the tensor-core kernel with its split of K: 32 x 768 x 1000 6 / 16
+// and 16 / 19, 24 x 768 x 3072 11 / 26 and 20 / 25, 16 x 2048 x 1000 12 / 31 and 20 / 24; but 9 x 1024 x 32000
+// 102 / 109 and 50 / 49, 16 x 4096 x 4096 57 / 91 and 36 / 38, 32 x 768 x 3072 16 / 29 and 20 / 24.
 bool gemm_rows_applies(const AcSession& s, const GemmShape& g, bool b_const, int64_t a_off, int64_t b_off) {
   return fp32_level_mode(s) && g.batch == 1 && !g.ta && g.m <= kGemmRowsMax && g.k >= 4 && (g.k % 4) == 0 &&
+         (g.m <= 4 || (double)g.m * g.n * g.k <= double(1 << 26)) &&
          (g.lda % 4) == 0 && (a_off % 4) == 0 &&
          (g.tb ? (g.ldb % 4) == 0 && (b_off % 4) == 0 : b_const && b_off == 0);
 }

@@ -198,6 +198,14 @@ def test_long_attention_without_its_kernel_is_separate_operators(monkeypatch, to
     assert "softmax" in kinds and not any(k.startswith("attention") for k in kinds), kinds
 
 
+@pytest.mark.parametrize("m,k,n,rows", [(1, 1024, 32000, True), (4, 4096, 4096, True), (32, 768, 1000, True), (24, 768, 3072, True),
+                                         (32, 768, 3072, False), (9, 1024, 32000, False), (16, 4096, 4096, False), (33, 768, 1000, False)])
+def test_few_rows_take_the_kernel_that_streams_the_weights_while_they_are_small(m, k, n, rows):
+    x, w = np.zeros((m, k), np.float32), np.zeros((n, k), np.float32)
+    kinds = [e["kind"] for e in plan(single_op_model("Gemm", [x], [w], alpha=1.0, beta=1.0, trans_a=False, trans_b=True)).schedule()]
+    assert kinds == (["gemm_fp32_rows"] if rows else ["gemm_f16x3_tcgen05"])
+
+
 def test_errors_are_reported_at_create():
     a = np.zeros((1, 3, 28, 28), np.float32)
     b = np.zeros((3, 1, 2), np.float32)
