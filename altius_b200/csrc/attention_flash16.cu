@@ -66,10 +66,6 @@ struct FlashDev {
   int* err;
 };
 
-__device__ __forceinline__ uint64_t desc_k128(uint32_t saddr) {      // K-major, 128-byte rows and swizzle
-  return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
-         (uint64_t)2 << 61;
-}
 // MN-major: 8 k-rows of 64 columns 1024 bytes apart, the next 64 columns (the lo tile) kTile further on.
 __device__ __forceinline__ uint64_t desc_mn128(uint32_t saddr) {
   return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)(kTile >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
@@ -235,8 +231,8 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
             tc_fence_after();
             const int j = sn[g] % blocks, ns = (min(KV, T - j * KV) + 15) / 16 * 16;
             const uint32_t idesc = (1u << 4) | ((uint32_t)(ns >> 3) << 17) | ((uint32_t)(QM >> 4) << 24);
-            const uint64_t q_hi = desc_k128(base), q_lo = desc_k128(base + kTile);
-            const uint64_t k_hi = desc_k128(base + 2 * kTile), k_lo = desc_k128(base + 3 * kTile);
+            const uint64_t q_hi = desc_sw128(base), q_lo = desc_sw128(base + kTile);
+            const uint64_t k_hi = desc_sw128(base + 2 * kTile), k_lo = desc_sw128(base + 3 * kTile);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {   // the cross terms, 2^-11 of the scores, while the sum is small
               const uint64_t off = (uint64_t)(kk * 32 >> 4);

@@ -65,16 +65,6 @@ __device__ long long g_attn16_stamps[80];   // [0]: kernel entry; [1 + 6 item + 
 #define AT16_MSTAMP(i, k) do { if (p.dbg && blockIdx.x == 0 && (i) < 6) p.dbg[40 + 6 * (i) + (k)] = clock64(); } while (0)
 #define AT16_STAMP(k) do { if (p.dbg && blockIdx.x == 0 && (warp & 7) == 0 && lane == 0 && i < 6) p.dbg[1 + 6 * i + (k)] = clock64(); } while (0)
 
-// K-major tile with rows of 128 bytes and the 128-byte swizzle: 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t desc_k128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;                   // leading byte offset (ignored for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;         // stride byte offset
-  d |= (uint64_t)1 << 46;                   // descriptor version for this architecture
-  d |= (uint64_t)2 << 61;                   // 128-byte swizzle
-  return d;
-}
 // MN-major tile of 64 fp16 columns (one 128-byte swizzle atom wide): k-rows of 128 bytes, 8-row
 // groups 1024 bytes apart (stride byte offset); a second atom along N does not exist here.
 __device__ __forceinline__ uint64_t desc_mn128(uint32_t saddr) {
@@ -245,8 +235,8 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
           const uint32_t qa = q_hi + kk * 32, ka = smem_u32(k_hi) + kk * 32;
-          const uint64_t a_hi = desc_k128(qa), a_lo = desc_k128(qa + kQHalfBytes);
-          const uint64_t b_hi = desc_k128(ka), b_lo = desc_k128(ka + kKvHalfBytes);
+          const uint64_t a_hi = desc_sw128(qa), a_lo = desc_sw128(qa + kQHalfBytes);
+          const uint64_t b_hi = desc_sw128(ka), b_lo = desc_sw128(ka + kKvHalfBytes);
           tc_mma_f16(d, a_lo, b_hi, idesc_s, kk ? 1u : 0u);
           tc_mma_f16(d, a_hi, b_lo, idesc_s, 1u);
           tc_mma_f16(d, a_hi, b_hi, idesc_s, 1u);

@@ -59,12 +59,7 @@ struct ConvTcDev {
   int* err;
 };
 
-// K-major tile of 128-byte rows with the 128-byte swizzle: 8-row groups are 1024 bytes apart.
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
-         (uint64_t)2 << 61;
-}
-// Byte offset of 16-byte chunk c of row r in such a tile.
+// Byte offset of 16-byte chunk c of row r in a K-major tile of 128-byte rows with the 128-byte swizzle.
 __host__ __device__ __forceinline__ uint32_t sw128(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {

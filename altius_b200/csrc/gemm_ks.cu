@@ -50,11 +50,6 @@ struct KsDev {
   int* err;
 };
 
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
-         (uint64_t)2 << 61;
-}
-
 template <int ACT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
@@ -346,7 +341,11 @@ namespace {
 
 // Tile width and K split by clocks, from stamps in the kernel: a K-block costs its twelve MMAs (45 to 65 clocks
 // each) or its bytes at 60 a clock, whichever is more; first loads and drain 2700; exchange 1600 and 18
-// per column; epilogue 1500 and 40 per column that a block finishes.
+// per column; epilogue 1500 and 40 per column that a block finishes. A launch as timed takes 1.4 to 2 times as long
+// (launch, cold code; operands arrive at 34 bytes a clock when all SMs load at once), the pair kernel 1.2 to 1.6 times
+// its clocks, so the comparison errs towards this kernel where both are close and K is long: the second product of
+// an MLP of 1182 to 2885 x 768 takes 4 us less to 6 more of 45, of 3152 x 768 and 12672 x 384 9 more of 67 (error
+// against 64 bits 1.2e-5 -> 2.4e-6 and 5.3e-6 -> 1.3e-6, so the choice stays); elsewhere it is the faster one.
 Shape pick_shape(int64_t m, int64_t n, int64_t k) {
   Shape best;
   const int nkb = (int)((k + KB - 1) / KB);

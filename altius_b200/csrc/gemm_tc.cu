@@ -107,17 +107,6 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
   return d;
 }
 
-// K-major tile whose rows are 128 bytes (64 halves) with the 128-byte swizzle: 8-row groups
-// are 1024 bytes apart. A K-step of 16 halves advances the start address by 32 bytes.
-__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;                        // leading byte offset (ignored for swizzled K-major)
-  d |= (uint64_t)((8 * 128) >> 4) << 32;         // stride byte offset: 8 rows
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;                        // 128-byte swizzle
-  return d;
-}
 
 // Descriptor of an MN-major tile of 4-byte elements. The one layout the tensor core accepts
 // for them is the 128-byte swizzle with 32-byte atoms: 32 columns (128 bytes) x 4 k-rows form
@@ -1167,8 +1156,8 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
             if (it == 0) pair_stamp(dbg, 2);
             tc_fence_after();
             const uint32_t ea = smem_u32(smem + sa * L::kStageBytes), eb = smem_u32(smem + sb * L::kStageBytes);
-            const uint64_t da = make_smem_desc_sw128(ea), dal = make_smem_desc_sw128(ea + L::kABytes);
-            const uint64_t db = make_smem_desc_sw128(eb), dbl = make_smem_desc_sw128(eb + L::kABytes);
+            const uint64_t da = desc_sw128(ea), dal = desc_sw128(ea + L::kABytes);
+            const uint64_t db = desc_sw128(eb), dbl = desc_sw128(eb + L::kABytes);
             // Operands on fixed scales: the cross terms go into the same accumulator.
 #pragma unroll
             for (int kk = 0; kk < KB / 16; ++kk) {          // K-steps of 16 halves (32 bytes of a row)
@@ -1712,7 +1701,8 @@ bool gemm_tc_wants_presplit(int64_t m, int64_t n, int64_t k, int64_t batch) {
 }
 
 // A K-block of a 256 x 256 tile takes 1950 clocks, launch, first operands and last epilogue 20000, the
-// K-slice pass behind it 9000 (ViT-B/16's four GEMMs at 1 to 96 images, within 15 %).
+// K-slice pass behind it 9000. (Products of 197 to 12672 rows against 384 to 768 x 384 to 2304 take 1.2 to 1.6 times
+// that: an epilogue of 11000 a tile runs only partly under the next tile's products.)
 double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k) {
   const int pairs = pair_count();
   if (pairs <= 0) return 1e30;

@@ -81,6 +81,18 @@ __device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, i
   return done != 0;
 }
 
+// Shared-memory descriptor of a K-major tile of 128-byte rows with the 128-byte swizzle: 8-row groups are 1024
+// bytes apart. A K-step of 32 bytes advances the start address by as much.
+__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)1 << 16;                   // leading byte offset (ignored for swizzled K-major)
+  d |= (uint64_t)(1024 >> 4) << 32;         // stride byte offset: 8 rows
+  d |= (uint64_t)1 << 46;                   // descriptor version for this architecture
+  d |= (uint64_t)2 << 61;                   // 128-byte swizzle
+  return d;
+}
+
 // One thread of a converged warp, in a form that lets ptxas keep the operands of the tensor-core
 // instructions behind it in uniform registers.
 __device__ __forceinline__ bool elect_one() {
