@@ -287,7 +287,10 @@ cudaError_t upload_inputs(AcSession* s, const void* const* ins) {
     } else {
       cudaPointerAttributes pa{};
       bool pageable = bytes > kSmallIo;
-      if (pageable && cudaPointerGetAttributes(&pa, ins[i]) == cudaSuccess) pageable = pa.type == cudaMemoryTypeUnregistered;
+      if (pageable) {
+        if (cudaPointerGetAttributes(&pa, ins[i]) == cudaSuccess) pageable = pa.type == cudaMemoryTypeUnregistered;
+        else (void)cudaGetLastError();       // not left for the next launch to report
+      }
       if (pageable && !s->host_stage) s->host_stage = HostStage::of_device(s->device);
       e = pageable && s->host_stage ? s->host_stage->upload(dst, ins[i], bytes, s->stream)
                                     : cudaMemcpyAsync(dst, ins[i], bytes, cudaMemcpyHostToDevice, s->stream);
