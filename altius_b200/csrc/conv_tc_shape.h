@@ -75,11 +75,12 @@ inline Shape pick_shape(const ConvParams& q, const std::array<int, 4>& slots) {
   // result, have an accumulator of their own, and the main terms of narrow tiles, and of a K cut eight times, are
   // dealt to two, K step by K step. (All on one: 1.3e-6 of the result at 2048 x 7 x 7 into 512, 5.9e-7 at
   // 480 x 32 x 32 into 480; the GEMM on a column buffer, with its up to 32 slices of K, 3.4e-7 and 2.7e-7; this way
-  // 2.5e-7 and 2.3e-7.) One or two K steps need none of it, all terms are on one (mains 0): no slice of that GEMM
-  // is shorter. Walking blocks have a second buffer of accumulators, so that the products of the next tile run
-  // under the stores of a tile, as far as the columns go.
+  // 2.5e-7 and 2.3e-7.) A single K step, or two of a block that walks, need none of it, all terms are on one
+  // (mains 0): that GEMM has no shorter slices, and cuts K only where it has few tiles (64 x 56 x 56 into 256, one
+  // image: two steps on one 2.6e-7, this way 1.1e-7, that GEMM 1.9e-7). Walking blocks have a second buffer of
+  // accumulators, so that the products of the next tile run under the stores of a tile, as far as the columns go.
   best.set = best.bn <= 32 ? 32 : best.bn <= 64 ? 64 : best.bn <= 128 ? 128 : 256;
-  best.mains = best.kper <= 2 ? 0 : walk || best.set == 256 || (best.set == 128 && best.split < 8) ? 1 : 2;
+  best.mains = best.kper == 1 || (walk && best.kper == 2) ? 0 : walk || best.set == 256 || (best.set == 128 && best.split < 8) ? 1 : 2;
   best.bufs = walk && best.set * (best.mains + 1) <= 128 ? 2 : 1;   // mains 0: always two
   best.cols = 32;
   while (best.cols < best.set * (best.mains + 1) * best.bufs) best.cols *= 2;

@@ -29,7 +29,7 @@ int main() {
               const int per_sm = (int)std::min<size_t>(7, 233472 / ((s.smem + 1120 + 127) / 128 * 128 + 1024));
               const bool walks = s.ctas < px;
               const bool fits = per_sm * s.cols <= 512 && s.cols >= s.set * (s.mains + 1) * s.bufs && s.set >= s.bn && s.cols >= 32 &&
-                                (s.mains > 0 || (s.kper <= 2 && (!walks || s.bufs == 2))) && (!walks || s.ctas == 1 || s.ctas * s.tiles <= per_sm * slots[0]);
+                                (s.mains > 0 || s.kper == 1 || (walks && s.kper == 2)) && (s.mains > 0 || !walks || s.bufs == 2) && (!walks || s.ctas == 1 || s.ctas * s.tiles <= per_sm * slots[0]);
               const bool ok = fits && s.bn >= 16 && s.bn <= 256 && s.bn % 16 == 0 && s.tiles >= 1 && s.tiles <= 65535 && (long long)s.tiles * s.bn >= oc &&
                               s.split * s.kper >= nkb && (s.split - 1) * s.kper < nkb && s.ctas >= 1 &&
                               s.stages >= std::min(2, s.kper) && s.stages <= 3 && s.smem <= conv_tc::kSmemMax;
