@@ -84,15 +84,25 @@ struct TcEpilogue {
   const float* bias_n; const float* bias_m; float bias_scale;
   int act; float act_alpha, act_beta;
   const float* res; long long ldres, sres;
-  uint2* c16_hi; uint2* c16_lo; long long ldc16;   // result as fp16 hi / lo halves (4 per uint2; ldc16 in halves), or null
-  int c16_fixed;            // the halves on the fixed scale (f16_split_fixed) instead of f16_split
+  uint2* c16_hi; uint2* c16_lo; long long ldc16;   // result as fp16 hi / lo halves on the fixed scale (4 per uint2; ldc16 in halves), or null
   const float* acc_scale;   // device scalar the accumulators are multiplied by (B was scaled by its inverse), or null
   float acc_scale_const;    // times this power of two (the inverse of the fixed scale of a pre-split A; else 1)
   const float* b_row_scale; long long b_row_scale_stride; int k_total;   // [K, N] operand: row k of B[bz] is multiplied by
                                                                        // b_row_scale[bz * stride + k] while it is split, or null
   int* err;                 // error word: range of the split output
-  int dbg;   // timing experiments only (0 in normal use)
 };
+
+// Which of the epilogues with compile-time options fits (alpha 1, no C input, one kind of bias, everything 16-byte
+// aligned, N a multiple of 4): bias per column 1, residual 2, activation << 2, bias per row 64; -1 none.
+__host__ __device__ __forceinline__ int epilogue_key(const TcEpilogue& ep) {
+  const bool simple = ep.alpha == 1.f && !(ep.cin && ep.beta != 0.f) && !(ep.bias_m && ep.bias_n) &&
+                      ep.bias_scale == 1.f && (ep.ldc % 4) == 0 && (ep.n % 4) == 0 && (ep.sc % 4) == 0 &&
+                      ((reinterpret_cast<uintptr_t>(ep.c) & 15) == 0) &&
+                      (!ep.res || ((ep.ldres % 4) == 0 && (ep.sres % 4) == 0 &&
+                                   (reinterpret_cast<uintptr_t>(ep.res) & 15) == 0)) &&
+                      (!ep.bias_n || (reinterpret_cast<uintptr_t>(ep.bias_n) & 15) == 0);
+  return !simple ? -1 : ((ep.bias_n ? 1 : 0) | (ep.res ? 2 : 0) | (ep.act << 2) | (ep.bias_m ? 64 : 0));
+}
 
 // Shared-memory matrix descriptor for a K-major tile whose rows are 64 bytes
 // (16 floats), stored row after row with the 64-byte swizzle: 8-row groups are
@@ -330,148 +340,6 @@ __device__ __forceinline__ bool epilogue_fast(const TcEpilogue& ep, float4* stag
   return released;
 }
 
-// The epilogue of the pair kernel that takes A pre-split: sixteen warps, a warp per tensor-memory
-// lane quarter and 64-column group, each with 4 KB of shared memory. Reading tensor memory
-// while MMAs write it is slow, so a warp first takes its whole 32 x 64 part out -- the second
-// 32-column chunk into its shared memory, the first into registers -- and hands tensor memory
-// back to the MMA warp; bias, activation, residual, the stores and the fp16 split for a
-// consuming kernel then run under the next tile's MMAs: the parked chunk first, then the one
-// from the registers through the same 4 KB. Shared memory is written a row per lane and read
-// eight lanes per row (the whole 128 bytes of a row of the chunk per instruction and row: the
-// global loads and stores that follow are whole 128-byte lines, or 64 bytes of each fp16 half);
-// the 16-byte slots of a row are XOR-swizzled by the row so that neither side has bank conflicts.
-__device__ long long g_epi_stamps[8];   // debug aid: clock64 inside the epilogue of CTA 0, warp 0, tiles 0 and 1
-__device__ __forceinline__ int epi_slot(int row, int j) { return j ^ (((row & 1) << 2) | ((row >> 1) & 3)); }
-
-template <int D2OFF, int ACT, int BIAS, bool HAS_RES, typename Release>
-__device__ __forceinline__ bool epilogue_parked(const TcEpilogue& ep, float4* buf, uint32_t tmem_base, int q,
-                                                int lane, int m0, int n0, int bz, int cc0, unsigned& seen,
-                                                Release&& release, int stamp = -1) {
-  const float sc = acc_scale_of(ep);
-  float* c = ep.c ? ep.c + (long long)bz * ep.sc : nullptr;
-  const float* res = HAS_RES ? ep.res + (long long)bz * ep.sres : nullptr;
-  const bool have0 = n0 + cc0 * 32 < ep.n, have1 = n0 + (cc0 + 1) * 32 < ep.n;   // uniform across the warp
-  const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16);
-  auto to_buf = [&](const uint32_t (&v)[32]) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      buf[lane * 8 + epi_slot(lane, j)] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                                      __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-  };
-  uint32_t v[32];
-  __syncwarp();                                     // the previous tile's reads of the buffer are over
-  if (D2OFF == 0 && have0 && have1 && !(ep.dbg & 128)) {
-    // One accumulator, both chunks there. A load of tensor memory issued behind the parking
-    // stores waited 2.7 K clocks where the first one took 0.4 K: the kept chunk and the first
-    // half of the parked one are requested together, the second half before the first is parked.
-    uint32_t w[16];
-    tc_ld_32x32_nowait(trow + (uint32_t)(cc0 * 32), v);
-    tc_ld_32x16_nowait(trow + (uint32_t)((cc0 + 1) * 32), w);
-    tc_wait_ld();
-    uint32_t w2[16];
-    tc_ld_32x16_nowait(trow + (uint32_t)((cc0 + 1) * 32 + 16), w2);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      buf[lane * 8 + epi_slot(lane, j)] =
-          make_float4(__fmul_rn(__uint_as_float(w[4 * j]), sc), __fmul_rn(__uint_as_float(w[4 * j + 1]), sc),
-                      __fmul_rn(__uint_as_float(w[4 * j + 2]), sc), __fmul_rn(__uint_as_float(w[4 * j + 3]), sc));
-    tc_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      buf[lane * 8 + epi_slot(lane, 4 + j)] =
-          make_float4(__fmul_rn(__uint_as_float(w2[4 * j]), sc), __fmul_rn(__uint_as_float(w2[4 * j + 1]), sc),
-                      __fmul_rn(__uint_as_float(w2[4 * j + 2]), sc), __fmul_rn(__uint_as_float(w2[4 * j + 3]), sc));
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fmul_rn(__uint_as_float(v[j]), sc));   // sc is a power of two
-  } else {
-    if (have1) {
-      load_acc<D2OFF>(trow + (uint32_t)((cc0 + 1) * 32), v, sc);
-      to_buf(v);
-    }
-    if (have0) load_acc<D2OFF>(trow + (uint32_t)(cc0 * 32), v, sc);
-  }
-  const bool released = release();                  // includes a __syncwarp: the buffer is written
-  if (stamp >= 0 && lane == 0) g_epi_stamps[stamp] = clock64();
-  // Eight lanes per row: 128 contiguous bytes of fp32 (64 of each fp16 half) per row and
-  // instruction, four rows per instruction, sixteen rows per pass.
-  const int c8 = lane & 7, r4 = lane >> 3;
-  float seen_max = 0.f;                             // largest magnitude written as fixed-scale halves
-  auto from_buf = [&](const int chunk) {            // bias, activation, residual, stores of one 32-column chunk
-    const int col = n0 + chunk * 32 + 4 * c8;
-    const bool col_ok = col < ep.n;                 // n % 4 == 0: the whole float4 is in range
-    float4 bn = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (BIAS == 1 && col_ok) bn = ld_plain(reinterpret_cast<const float4*>(ep.bias_n + col));
-#pragma unroll 1
-    for (int pass = 0; pass < 2; ++pass) {
-      const int row_base = m0 + q * 32 + 16 * pass + r4;
-      float4 a[4], r[4];
-      float bm[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int rl = 16 * pass + 4 * i + r4;
-        a[i] = buf[rl * 8 + epi_slot(rl, c8)];
-        const int row = row_base + 4 * i;
-        if (BIAS == 2) bm[i] = row < ep.m ? ld_plain(ep.bias_m + row) : 0.f;
-        if (HAS_RES) {
-          r[i] = (col_ok && row < ep.m)
-                     ? ld_plain(reinterpret_cast<const float4*>(res + (long long)row * ep.ldres + col))
-                     : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float4 x = a[i];
-        if (BIAS == 1) {
-          x.x = __fadd_rn(x.x, bn.x); x.y = __fadd_rn(x.y, bn.y);
-          x.z = __fadd_rn(x.z, bn.z); x.w = __fadd_rn(x.w, bn.w);
-        }
-        if (BIAS == 2) {
-          x.x = __fadd_rn(x.x, bm[i]); x.y = __fadd_rn(x.y, bm[i]);
-          x.z = __fadd_rn(x.z, bm[i]); x.w = __fadd_rn(x.w, bm[i]);
-        }
-        if (ACT == ACT_GELU) {
-          const float2 lo = gelu_ref2(make_float2(x.x, x.y)), hi = gelu_ref2(make_float2(x.z, x.w));
-          x = make_float4(lo.x, lo.y, hi.x, hi.y);
-        } else if (ACT != ACT_NONE) {
-          const float al = ep.act_alpha, be = ep.act_beta;
-          x.x = apply_act(ACT, x.x, al, be); x.y = apply_act(ACT, x.y, al, be);
-          x.z = apply_act(ACT, x.z, al, be); x.w = apply_act(ACT, x.w, al, be);
-        }
-        if (HAS_RES) {
-          x.x = __fadd_rn(x.x, r[i].x); x.y = __fadd_rn(x.y, r[i].y);
-          x.z = __fadd_rn(x.z, r[i].z); x.w = __fadd_rn(x.w, r[i].w);
-        }
-        const int row = row_base + 4 * i;
-        if (col_ok && row < ep.m) {
-          if (c) *reinterpret_cast<float4*>(c + (long long)row * ep.ldc + col) = x;
-          if (ep.c16_hi) {   // the kernel that consumes this result takes it split (batch 1)
-            uint2 h, l;
-            if (ep.c16_fixed) { f16_split_fixed(x, h, l); seen_max = split_track(seen_max, x); }
-            else { f16_split(x, h, l); seen |= split_seen(x); }
-            const long long o = ((long long)row * ep.ldc16 + col) >> 2;
-            ep.c16_hi[o] = h;
-            ep.c16_lo[o] = l;
-          }
-        }
-      }
-    }
-  };
-  if (have1) {
-    from_buf(cc0 + 1);
-    __syncwarp();                                   // everybody has read the parked chunk
-  }
-  if (stamp >= 0 && lane == 0) g_epi_stamps[stamp + 1] = clock64();
-  if (have0) {
-    to_buf(v);
-    __syncwarp();
-    if (stamp >= 0 && lane == 0) g_epi_stamps[stamp + 2] = clock64();
-    from_buf(cc0);
-  }
-  if (stamp >= 0 && lane == 0) g_epi_stamps[stamp + 3] = clock64();
-  seen |= split_seen_fixed_of_max(seen_max);
-  return released;
-}
-
 // Unreduced accumulator of a K-slice -> workspace tile [128][BN], same staging
 // as the real epilogues so that the stores are full lines.
 template <int BN, int D2OFF>
@@ -531,17 +399,138 @@ __device__ __forceinline__ void fixup_apply(const TcEpilogue& ep, int row, int c
   if (ep.c16_hi) {   // n is a multiple of 8 here: the whole float4 is in range
     uint2 h, l;
     const float4 yv = make_float4(y4[0], y4[1], y4[2], y4[3]);
-    if (ep.c16_fixed) f16_split_fixed(yv, h, l); else f16_split(yv, h, l);
+    f16_split_fixed(yv, h, l);
     const long long o = ((long long)row * ep.ldc16 + col0) >> 2;
     ep.c16_hi[o] = h;
     ep.c16_lo[o] = l;
     // A tile's few K-sliced elements say nothing about the tensor being tiny: overflow only.
-    if ((ep.c16_fixed ? split_seen_fixed(yv) : split_seen(yv)) & 1u) atomicCAS(ep.err, 0, kRangeCode);
+    if (split_seen_fixed(yv) & 1u) atomicCAS(ep.err, 0, kRangeCode);
+  }
+}
+
+// The epilogue of the pair kernel that takes A pre-split: sixteen warps, a warp per tensor-memory lane
+// quarter and 64-column group, in eight blocks of 16 rows x 16 columns that go from tensor memory to global
+// memory through registers alone. The fragment of tcgen05.ld.16x256b gives a lane two neighbouring columns
+// of two rows in each 8-column group; one exchange with the neighbouring lane makes them float4s (bias, residual and
+// fp32 stores are 64 contiguous bytes per row and instruction), and one more, with the lane two on, makes the
+// fp16 halves 16 bytes of one row per lane. The next block's accumulator, residual and bias are under way meanwhile.
+// What bounds it: shared memory. The tensor cores read 53 bytes of operands a clock and TMA
+// writes 42 at the full rate, of the 128 there are; parking the accumulator there (the earlier form, 256 KB per
+// tile and CTA there and back) made the epilogue of a tile as long as the main loop it runs under and that loop a
+// third longer. Blocks twice as wide spilled. Offsets inside the tile are 32-bit sums.
+//
+// All of a warp's loads of an accumulator have completed: one arrival on the leader's barrier.
+__device__ __forceinline__ void hand_back(uint32_t acc_empty_leader, int lane) {
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive_cluster(acc_empty_leader);
+}
+
+template <int ACT, int BIAS, bool HAS_RES>
+__device__ __forceinline__ unsigned epilogue_regs(const TcEpilogue& ep, uint32_t acc, int q, int lane, int m0, int n0,
+                                                  uint32_t acc_empty_leader) {
+  const float sc = acc_scale_of(ep);
+  const int odd = lane & 1, high = (lane >> 1) & 1;
+  const int rl = q * 32 + (lane >> 2), cl = 8 * odd + 4 * high;   // the lane's first row and column of block 0
+  const int rows = ep.m - m0 - rl, cols = ep.n - n0 - cl;          // how many there are from there on
+  const int blocks = 2 * min(4, (ep.n - n0 + 15) / 16);            // uniform across the warp
+  float seen_max = 0.f;                             // largest magnitude written as fixed-scale halves
+  uint32_t nx[8];
+  float4 nr[HAS_RES ? 2 : 1], nb = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto request = [&](int b) {
+    const int rb = 16 * (b & 1), cb = 16 * (b >> 1);
+    tc_ld_16x256_x2_nowait(acc + ((uint32_t)(q * 32 + rb) << 16) + (uint32_t)cb, nx);
+    if (BIAS == 1 && rb == 0 && cb < cols) nb = ld_plain(reinterpret_cast<const float4*>(ep.bias_n + n0 + cl + cb));   // n % 4 == 0
+    if (HAS_RES) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        nr[HAS_RES ? h : 0] = cb < cols && rb + 8 * h < rows
+                    ? ld_plain(reinterpret_cast<const float4*>(ep.res + (long long)m0 * ep.ldres + n0 + ((rl + rb + 8 * h) * (int)ep.ldres + cl + cb)))
+                    : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  if (blocks > 0) request(0);
+  else hand_back(acc_empty_leader, lane);
+#pragma unroll 1
+  for (int b = 0; b < blocks; ++b) {
+    const int rb = 16 * (b & 1), cb = 16 * (b >> 1);
+    tc_wait_ld(nx);
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(__uint_as_float(nx[j]), sc);   // sc is a power of two
+    const float4 bi = nb, r[2] = {nr[0], nr[HAS_RES ? 1 : 0]};
+    if (b + 1 < blocks) request(b + 1);
+    else hand_back(acc_empty_leader, lane);
+    uint2 hi[2], lo[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float4 x = quad_exchange(v[2 * h], v[2 * h + 1], v[4 + 2 * h], v[5 + 2 * h], odd);
+      if (BIAS == 1) {
+        x.x = __fadd_rn(x.x, bi.x); x.y = __fadd_rn(x.y, bi.y);
+        x.z = __fadd_rn(x.z, bi.z); x.w = __fadd_rn(x.w, bi.w);
+      }
+      if (ACT == ACT_GELU) {
+        const float2 g0 = gelu_ref2(make_float2(x.x, x.y)), g1 = gelu_ref2(make_float2(x.z, x.w));
+        x = make_float4(g0.x, g0.y, g1.x, g1.y);
+      } else if (ACT == ACT_RELU) {
+        x.x = fmaxf(x.x, 0.f); x.y = fmaxf(x.y, 0.f); x.z = fmaxf(x.z, 0.f); x.w = fmaxf(x.w, 0.f);
+      }
+      if (HAS_RES) {
+        x.x = __fadd_rn(x.x, r[h].x); x.y = __fadd_rn(x.y, r[h].y);
+        x.z = __fadd_rn(x.z, r[h].z); x.w = __fadd_rn(x.w, r[h].w);
+      }
+      const bool ok = rb + 8 * h < rows && cb < cols;
+      if (ep.c && ok)
+        *reinterpret_cast<float4*>(ep.c + (long long)m0 * ep.ldc + n0 + ((rl + rb + 8 * h) * (int)ep.ldc + cl + cb)) = x;
+      if (ep.c16_hi) {                              // the kernel that consumes this result takes it split
+        f16_split_fixed(x, hi[h], lo[h]);
+        if (ok) seen_max = split_track(seen_max, x);
+      }
+    }
+    if (ep.c16_hi) {
+      // Lanes two apart hold the halves of an 8-column group of both rows: each leaves with one row's.
+      auto join = [&](const uint2 (&w)[2]) {
+        const uint2 give = high ? w[0] : w[1], keep = high ? w[1] : w[0];
+        const uint2 got = make_uint2(__shfl_xor_sync(0xffffffffu, give.x, 2), __shfl_xor_sync(0xffffffffu, give.y, 2));
+        return high ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
+      };
+      const uint4 hh = join(hi), ll = join(lo);
+      if (rb + 8 * high < rows && cb < cols) {      // n % 8 == 0: the eight columns exist together
+        const long long o = ((long long)m0 * ep.ldc16 + n0 + ((rl + rb + 8 * high) * (int)ep.ldc16 + cb + 8 * odd)) >> 3;
+        reinterpret_cast<uint4*>(ep.c16_hi)[o] = hh;
+        reinterpret_cast<uint4*>(ep.c16_lo)[o] = ll;
+      }
+    }
+  }
+  return split_seen_fixed_of_max(seen_max);
+}
+
+// The same walk for what the common epilogues do not cover: the unreduced accumulator of a K-slice into its
+// workspace tile [128][ld] (ws), or any epilogue, element by element.
+__device__ __noinline__ void epilogue_regs_other(const TcEpilogue& ep, float* ws, int ld, uint32_t acc, int q, int lane, int m0, int n0,
+                                                 int cg, uint32_t acc_empty_leader) {
+  const float sc = acc_scale_of(ep);
+  const int odd = lane & 1, high = (lane >> 1) & 1;
+#pragma unroll 1
+  for (int b = 0; b < 8; ++b) {
+    uint32_t u[8];
+    tc_ld_16x256_x2_nowait(acc + ((uint32_t)(q * 32 + 16 * (b & 1)) << 16) + (uint32_t)(16 * (b >> 1)), u);
+    tc_wait_ld(u);
+    if (b == 7) hand_back(acc_empty_leader, lane);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float4 x = quad_exchange(__uint_as_float(u[2 * h]), __uint_as_float(u[2 * h + 1]), __uint_as_float(u[4 + 2 * h]),
+                               __uint_as_float(u[5 + 2 * h]), odd);
+      x.x = __fmul_rn(x.x, sc); x.y = __fmul_rn(x.y, sc); x.z = __fmul_rn(x.z, sc); x.w = __fmul_rn(x.w, sc);
+      const int row = q * 32 + 16 * (b & 1) + 8 * h + (lane >> 2), col = 16 * (b >> 1) + 8 * odd + 4 * high;
+      if (ws) *reinterpret_cast<float4*>(ws + (size_t)row * ld + cg + col) = x;
+      else if (m0 + row < ep.m && n0 + col < ep.n) fixup_apply(ep, m0 + row, n0 + col, 0, x);
+    }
   }
 }
 
 // Adds the K-slices of the tail tiles in slice order and applies the epilogue.
-__global__ void __launch_bounds__(256) gemm_tc_fixup_kernel(const float* ws, TcEpilogue ep, int bm,
+__global__ void __launch_bounds__(256) gemm_tc_fixup_kernel(const float* ws, const __grid_constant__ TcEpilogue ep, int bm,
                                                             int bn, int dp_tiles, int parts, int tiles_m,
                                                             int tiles_n) {
   pdl_trigger();
@@ -646,7 +635,7 @@ __device__ __forceinline__ bool tc_get_work(const TcSched& sc, int w, TcWork* ou
 template <int BN, int MT, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-               const __grid_constant__ CUtensorMap tm_blo, TcEpilogue ep, TcSched sc, int a_batched,
+               const __grid_constant__ CUtensorMap tm_blo, const __grid_constant__ TcEpilogue ep, const __grid_constant__ TcSched sc, int a_batched,
                int b_batched, int tiles_m, int tiles_n, float* workspace, int* err) {
   using L = TcSmem<BN, MT, MODE>;
   constexpr bool kBMN = MODE == TC_3X_SPLIT_B_MN;
@@ -888,13 +877,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     const int e = warp - kSplitWarps, q = e & 3;   // TMEM lane quarter (kSplitWarps is a multiple of 4)
     const int cc0 = (e >> 2) * (BN / 64), cc1 = cc0 + BN / 64;   // this warp's 32-column chunks
     float4* stage = reinterpret_cast<float4*>(epi_smem + e * 4096);
-    const bool simple = ep.alpha == 1.f && !(ep.cin && ep.beta != 0.f) && !(ep.bias_m && ep.bias_n) &&
-                        ep.bias_scale == 1.f && (ep.ldc % 4) == 0 && (ep.n % 4) == 0 && (ep.sc % 4) == 0 &&
-                        ((reinterpret_cast<uintptr_t>(ep.c) & 15) == 0) &&
-                        (!ep.res || ((ep.ldres % 4) == 0 && (ep.sres % 4) == 0 &&
-                                     (reinterpret_cast<uintptr_t>(ep.res) & 15) == 0)) &&
-                        (!ep.bias_n || (reinterpret_cast<uintptr_t>(ep.bias_n) & 15) == 0);
-    const int key = !simple ? -1 : ((ep.bias_n ? 1 : 0) | (ep.res ? 2 : 0) | (ep.act << 2) | (ep.bias_m ? 64 : 0));
+    const int key = epilogue_key(ep);
     int ti = 0;
     TcWork wk;
     for (int w = 0; tc_get_work(sc, w, &wk); ++w, ++ti) {
@@ -1008,10 +991,9 @@ struct PairSmem {
   static constexpr int kStageBytes = PRE ? 2 * kABytes : 2 * kABytes + 2 * kBBytes;
   // TMA brings B only (A goes global -> registers -> tiles); PRE: a whole entry
   static constexpr int kTxBytes = PRE ? 2 * kABytes : 2 * kBBytes;
-  // Epilogue memory: 4 KB per epilogue warp (PRE: sixteen of them; a parking place for half of
-  // the warp's accumulator part, or the staging tile of the general epilogues).
-  static constexpr int kEpiBytes = (PRE ? 16 : kEpiWarps) * 4096;
-  static constexpr int kStages = (227 * 1024 - kEpiBytes - 1536) / kStageBytes;   // BN 256: 5 entries with PRE, else 6 stages
+  // Epilogue memory: 4 KB per epilogue warp (none with PRE, whose epilogues work in registers).
+  static constexpr int kEpiBytes = PRE ? 0 : kEpiWarps * 4096;
+  static constexpr int kStages = (227 * 1024 - kEpiBytes - 1536) / kStageBytes;   // BN 256: 7 entries with PRE, else 6 stages
   static constexpr int kDynBytes = kStages * kStageBytes + kEpiBytes + 1024 /*alignment*/ + 512 /*barriers*/;
   // Without PRE: D1 and D2, one accumulator set. PRE: the operands are on fixed scales, the three
   // partial products share ONE accumulator, and two sets alternate between consecutive tiles, so
@@ -1029,13 +1011,17 @@ __device__ __forceinline__ void pair_stamp(int dbg, int slot) {
 
 // PRE runs 18 warps: sixteen epilogue warps (no thread has to touch the operand tiles), the TMA
 // producer and the MMA issuer. Both CTAs' loads count their bytes on the leader's `ready`
-// barriers, which is all the MMA thread waits for.
-template <int BN, bool PRE>
+// barriers, which is all the MMA thread waits for. Its `ready` and `empty` barriers belong to K-blocks (two
+// entries of the ring each; kFlight of them, no more are in flight): one wait and one commit per K-block.
+// KEY: the common epilogue (epilogue_key) that is compiled in with PRE, -1 any other; all of them in one kernel
+// spilled 540 bytes a thread.
+constexpr int kFlight = 4;
+template <int BN, bool PRE, int KEY>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
                     const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_alo,
                     const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_blo,
-                    TcEpilogue ep, TcSched sc, int tiles_m, int tiles_n, float* workspace, int* err, int dbg) {
+                    const __grid_constant__ TcEpilogue ep, const __grid_constant__ TcSched sc, int tiles_m, int tiles_n, float* workspace, int* err, int dbg) {
   using L = PairSmem<BN, PRE>;
   // Debug toggle: bits 16-19 of dbg, when set, use fewer stages of the ring.
   const int S = ((dbg >> 16) & 15) > 0 && ((dbg >> 16) & 15) < L::kStages ? ((dbg >> 16) & 15) : L::kStages;
@@ -1047,8 +1033,8 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
   uint8_t* epi_smem = smem + SM * L::kStageBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(epi_smem + L::kEpiBytes);
   uint64_t* full = bars;                 // this CTA's TMA bytes landed
-  uint64_t* ready = bars + SM;            // leader's: both CTAs' fp16 tiles written (2 x 4 warps arrive)
-  uint64_t* empty = bars + 2 * SM;        // this CTA's: the pair's MMAs that read the stage have completed
+  uint64_t* ready = bars + SM;            // leader's: both CTAs' fp16 tiles written (2 x 4 warps arrive; PRE: landed, K-block % kFlight)
+  uint64_t* empty = bars + 2 * SM;        // this CTA's: the pair's MMAs that read the stage (PRE: the K-block) have completed
   uint64_t* acc_full = bars + 3 * SM;     // [2] this CTA's: accumulator set complete (PRE uses both sets)
   uint64_t* acc_empty = bars + 3 * SM + 2;   // [2] leader's: set drained by the epilogue warps of the pair
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * SM + 4);
@@ -1066,7 +1052,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
   auto b_lo = [&](int s) { return smem + s * L::kStageBytes + L::kOffBLo; };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) {
+    for (int s = 0; s < SM; ++s) {
       mbar_init(&full[s], 1);
       // one arrival per splitter warp of the pair; PRE: the leader's producer, with the bytes of both CTAs
       mbar_init(&ready[s], PRE ? 1 : 2 * (kSplitThreads / 32));
@@ -1103,14 +1089,15 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         const int m0 = ((wk.tile / tiles_n) % tiles_m) * (2 * BM) + (int)rank * BM;
         if (PRE) {
           // Two ring entries per K-block of 64 halves: this CTA's 128 rows of A (hi, lo; rows past
-          // M are zero-filled), then its half of the B tile (hi, lo).
+          // M are zero-filled), then its half of the B tile (hi, lo). An entry is free when the K-block of its
+          // last use is.
           for (int kb = wk.k0; ok && kb < wk.k1; ++kb) {
+            const int q = (it >> 1) % kFlight;
+            const uint32_t rdy = map_to_cta(&ready[q], 0);         // the leader's barrier of this K-block
             for (int op = 0; op < 2; ++op, ++it) {
-              const int s = it % S;
-              const uint32_t ph = (it / S) & 1;
-              if (!pwait(&empty[s], ph ^ 1)) { atomicExch(err, 1); *abort_flag = 1; ok = false; break; }
-              const uint32_t rdy = map_to_cta(&ready[s], 0);       // the leader's barrier of this entry
-              if (leader) mbar_arrive_expect_tx(&ready[s], 2 * L::kTxBytes);
+              const int s = it % S, last = (it - S) >> 1;
+              if (it >= S && !pwait(&empty[last % kFlight], (last / kFlight) & 1)) { atomicExch(err, 1); *abort_flag = 1; ok = false; break; }
+              if (leader && op == 0) mbar_arrive_expect_tx(&ready[q], 4 * L::kTxBytes);
               uint8_t* e = smem + s * L::kStageBytes;
               if (op == 0) {
                 tma_load_3d_pair(e, &tm_a, rdy, kb * KB, m0, 0);
@@ -1135,7 +1122,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
     }
   } else if (warp == kMmaWarp) {
     // ---------------- MMA issuer (leader only) ----------------
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       // fp32 accumulators, fp16 A and B (format 0), both K-major, N = BN, M = 256 over the pair.
       const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
       int it = 0, ti = 0;
@@ -1150,8 +1137,8 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         const uint32_t d1 = tmem_base + (uint32_t)(set * BN);
         if (PRE) {
           for (int kb = wk.k0; kb < wk.k1; ++kb, it += 2) {
-            const int sa = it % S, sb = (it + 1) % S;          // the K-block's A entry and B entry
-            ok = pwait(&ready[sa], (it / S) & 1) && pwait(&ready[sb], ((it + 1) / S) & 1);
+            const int sa = it % S, sb = (it + 1) % S, kq = it >> 1;          // the K-block's A entry and B entry
+            ok = pwait(&ready[kq % kFlight], (kq / kFlight) & 1);
             if (!ok) { atomicExch(err, 2); *abort_flag = 1; break; }
             if (it == 0) pair_stamp(dbg, 2);
             tc_fence_after();
@@ -1163,13 +1150,10 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
             for (int kk = 0; kk < KB / 16; ++kk) {          // K-steps of 16 halves (32 bytes of a row)
               const uint64_t off = (uint64_t)(kk * 2);
               tc_mma_f16_pair(d1, dal + off, db + off, idesc, (kb > wk.k0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
-              tc_mma_f16_pair(d1, da + off, dbl + off, idesc, 1u);                                  // a_hi * b_lo
-              tc_mma_f16_pair(d1, da + off, db + off, idesc, 1u);                                   // a_hi * b_hi
+              tc_mma_f16_pair_fill(d1, da + off, dbl + off, idesc);                                 // a_hi * b_lo
+              tc_mma_f16_pair_lastuse(d1, da + off, db + off, idesc);                               // a_hi * b_hi
             }
-            tc_commit_pair(smem_u32(&empty[sa]));          // both entries are free again in this CTA ...
-            tc_commit_pair(map_to_cta(&empty[sa], 1));     // ... and in the peer
-            tc_commit_pair(smem_u32(&empty[sb]));
-            tc_commit_pair(map_to_cta(&empty[sb], 1));
+            tc_commit_pair_both(&empty[kq % kFlight]);     // both entries are free again in both CTAs
           }
         } else
         for (int kb = wk.k0; kb < wk.k1; ++kb, ++it) {
@@ -1193,13 +1177,9 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
               tc_mma_f16_pair(d1 + D2, da + (uint64_t)(kk * 2), dbl + (uint64_t)(kk * 2), idesc, 1u);
             }
           }
-          tc_commit_pair(smem_u32(&empty[s]));      // the stage is free again in this CTA ...
-          tc_commit_pair(map_to_cta(&empty[s], 1)); // ... and in the peer
+          tc_commit_pair_both(&empty[s]);          // the stage is free again in both CTAs
         }
-        if (ok) {
-          tc_commit_pair(smem_u32(&acc_full[set]));
-          tc_commit_pair(map_to_cta(&acc_full[set], 1));
-        }
+        if (ok) tc_commit_pair_both(&acc_full[set]);
         if (ti < 5) pair_stamp(dbg, 3 + ti);   // all MMAs of tile ti issued
       }
     }
@@ -1258,24 +1238,13 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
     split_report_warp(seen, err);
   } else if (!PRE || warp < 16) {
     // ---------------- epilogue (each CTA its own 128 rows) ----------------
-    // PRE: warps 0-15, a warp per lane quarter and quarter of the columns on the common
-    // epilogues (2 KB of staging each); the general and the K-slice epilogues are left to warps
-    // 8-15 with 4 KB each (the same 32 KB), the others only hand the accumulator back.
+    // PRE: warps 0-15, a warp per lane quarter and quarter of the columns, in registers; else eight warps, half of the
+    // columns each, through 4 KB of shared memory.
     const int e = PRE ? warp : warp - kSplitWarps, q = e & 3;
-    const int eo = PRE ? e - 8 : e;                                // index among the eight "old" warps
-    const int cc0 = (eo >> 2) * (BN / 64), cc1 = cc0 + BN / 64;   // their 32-column chunks
-    const int hc0 = (e >> 2) * (BN / 128);                        // PRE, common epilogues: 64 columns from chunk hc0
-    // 4 KB of shared memory per epilogue warp: the parking place of the common epilogues, the
-    // staging tile of the others.
+    const int cc0 = (e >> 2) * (BN / 64), cc1 = cc0 + BN / 64;    // 32-column chunks of the eight
+    const int cg = (e >> 2) * (BN / 4);                           // first column of the sixteen
     float4* stage = reinterpret_cast<float4*>(epi_smem + e * 4096);
-    float4* park = stage;
-    const bool simple = ep.alpha == 1.f && !(ep.cin && ep.beta != 0.f) && !(ep.bias_m && ep.bias_n) &&
-                        ep.bias_scale == 1.f && (ep.ldc % 4) == 0 && (ep.n % 4) == 0 && (ep.sc % 4) == 0 &&
-                        ((reinterpret_cast<uintptr_t>(ep.c) & 15) == 0) &&
-                        (!ep.res || ((ep.ldres % 4) == 0 && (ep.sres % 4) == 0 &&
-                                     (reinterpret_cast<uintptr_t>(ep.res) & 15) == 0)) &&
-                        (!ep.bias_n || (reinterpret_cast<uintptr_t>(ep.bias_n) & 15) == 0);
-    const int key = !simple ? -1 : ((ep.bias_n ? 1 : 0) | (ep.res ? 2 : 0) | (ep.act << 2) | (ep.bias_m ? 64 : 0));
+    const int key = PRE ? KEY : epilogue_key(ep);
     int ti = 0;
     unsigned seen_out = 0;   // what this warp has seen of the results it wrote split (ep.c16_hi)
     TcWork wk;
@@ -1291,40 +1260,36 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         // While the tile's MMAs run: pull this warp's 32 x 64 block of the residual into L2 -- but
         // not ahead of the kernel's first operand tiles (a thousand prefetches per SM issued at
         // kernel entry delayed those by 5 K clocks): wait until the first K-block has been used.
-        if (ti == 0) (void)mbar_wait(&empty[1], 0);
+        if (ti == 0) (void)mbar_wait(&empty[0], 0);
         const float* rp = ep.res + (long long)bz * ep.sres;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          const int row = m0 + q * 32 + (lane >> 1) + 16 * i, col = n0 + hc0 * 32 + (lane & 1) * 32;
+          const int row = m0 + q * 32 + (lane >> 1) + 16 * i, col = n0 + cg + (lane & 1) * 32;
           if (row < ep.m && col < ep.n)
             asm volatile("prefetch.global.L2 [%0];" ::"l"(rp + (long long)row * ep.ldres + col));
         }
       }
-      const bool wide = wk.raw >= 0 || key < 0 || (key & 64);
       if (!mbar_wait(&acc_full[set], use & 1)) { atomicExch(err, 4); *abort_flag = 1; break; }
       tc_fence_after();
       if (e == 0 && lane == 0 && ti < 3) pair_stamp(dbg, 8 + 2 * ti);     // accumulator of tile ti complete
       bool released = false;
-      const int estamp = ((dbg & 0x1000) && blockIdx.x == 0 && e == 0 && ti < 2) ? 4 * ti : -1;
       auto release = [&]() -> bool {     // all of this warp's tcgen05.ld have completed
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(acc_empty_leader);
         return true;
       };
-      if (PRE && BN == 256 && m0 < ep.m && !wide) {
-        switch (key) {
-          case 0: released = epilogue_parked<D2, ACT_NONE, 0, false>(ep, park, acc, q, lane, m0, n0, bz, hc0, seen_out, release, estamp); break;
-          case 1: released = epilogue_parked<D2, ACT_NONE, 1, false>(ep, park, acc, q, lane, m0, n0, bz, hc0, seen_out, release, estamp); break;
-          case 2: released = epilogue_parked<D2, ACT_NONE, 0, true>(ep, park, acc, q, lane, m0, n0, bz, hc0, seen_out, release, estamp); break;
-          case 3: released = epilogue_parked<D2, ACT_NONE, 1, true>(ep, park, acc, q, lane, m0, n0, bz, hc0, seen_out, release, estamp); break;
-          case (ACT_GELU << 2) | 1: released = epilogue_parked<D2, ACT_GELU, 1, false>(ep, park, acc, q, lane, m0, n0, bz, hc0, seen_out, release, estamp); break;
-          case (ACT_RELU << 2) | 1: released = epilogue_parked<D2, ACT_RELU, 1, false>(ep, park, acc, q, lane, m0, n0, bz, hc0, seen_out, release, estamp); break;
-          default:
-            if (eo >= 0) epilogue_generic<BN, D2>(ep, stage, acc, q, lane, m0, n0, bz, cc0, cc1);
-            break;
-        }
-      } else if (m0 < ep.m && eo >= 0) {
+      if (PRE) {
+        const int nw = n0 + cg;
+        const uint32_t part = acc + (uint32_t)cg;
+        if (m0 >= ep.m) hand_back(acc_empty_leader, lane);
+        else if (wk.raw >= 0)
+          epilogue_regs_other(ep, workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, BN, part, q, lane, m0, nw, cg, acc_empty_leader);
+        else if (KEY >= 0)
+          seen_out |= epilogue_regs<(KEY >= 0 ? KEY >> 2 : 0), KEY & 1, (KEY & 2) != 0>(ep, part, q, lane, m0, nw, acc_empty_leader);
+        else
+          epilogue_regs_other(ep, nullptr, 0, part, q, lane, m0, nw, cg, acc_empty_leader);
+      } else if (m0 < ep.m) {
         if (wk.raw >= 0) {
           epilogue_raw<BN, D2>(workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, stage, acc, q, lane, cc0, cc1, acc_scale_of(ep));
         } else
@@ -1342,7 +1307,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
           default: epilogue_generic<BN, D2>(ep, stage, acc, q, lane, m0, n0, bz, cc0, cc1); break;
         }
       }
-      if (!released) release();
+      if (!PRE && !released) release();
       if (e == 0 && lane == 0 && ti < 3) pair_stamp(dbg, 9 + 2 * ti);     // this warp's part of tile ti stored
     }
     if (PRE && ep.c16_hi) split_report_warp(seen_out, err);
@@ -1353,7 +1318,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
   tc_fence_before();
   __syncthreads();
   if (*abort_flag != 0 && warp == kTmaWarp && lane == 0) {
-    for (int s = 0; s < S; ++s) {        // copies that may still be in flight: a bounded time to land
+    for (int s = 0; s < (PRE ? kFlight : S); ++s) {        // copies that may still be in flight: a bounded time to land
       (void)mbar_wait(PRE ? &ready[s] : &full[s], 0);
       (void)mbar_wait(PRE ? &ready[s] : &full[s], 1);
     }
@@ -1560,26 +1525,21 @@ cudaError_t launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtens
                     pl.tiles_m, pl.tiles_n);
 }
 
-template <int BN, bool PRE>
+template <int BN, bool PRE, int KEY>
 cudaError_t launch_pair(const float* a, long long lda, int k, const CUtensorMap& ma, const CUtensorMap& mal,
                         const CUtensorMap& mb, const CUtensorMap& mbl, const TcEpilogue& ep, const TcPlan& pl,
                         float* workspace, int* err, cudaStream_t st) {
   using L = PairSmem<BN, PRE>;
   static unsigned long long attr_done = 0;
-  if (cudaError_t e0 = ensure_dynamic_smem(gemm_tc_pair_kernel<BN, PRE>, L::kDynBytes, &attr_done)) return e0;
+  if (cudaError_t e0 = ensure_dynamic_smem(gemm_tc_pair_kernel<BN, PRE, KEY>, L::kDynBytes, &attr_done)) return e0;
   // pl.grid counts pairs; the cluster shape (2, 1, 1) is a compile-time attribute of the kernel.
   static const int dbg = std::getenv("ALTIUS_CUDA_TC_DBG") ? std::atoi(std::getenv("ALTIUS_CUDA_TC_DBG")) : 0;
-  const cudaError_t e = launch_pdl(gemm_tc_pair_kernel<BN, PRE>, dim3(2u * (unsigned)pl.grid), dim3(kThreads), L::kDynBytes, st, 1, a, lda,
+  const cudaError_t e = launch_pdl(gemm_tc_pair_kernel<BN, PRE, KEY>, dim3(2u * (unsigned)pl.grid), dim3(kThreads), L::kDynBytes, st, 1, a, lda,
                                    k, ma, mal, mb, mbl, ep, pl.sc, pl.tiles_m, pl.tiles_n, workspace, err, dbg);
   if (dbg & 0x1000) {
     cudaStreamSynchronize(st);
     static long long h[160][24];
     cudaMemcpyFromSymbol(h, g_pair_stamps, sizeof(h));
-    long long eh[8];
-    cudaMemcpyFromSymbol(eh, g_epi_stamps, sizeof(eh));
-    std::printf("epi stamps:");
-    for (int i = 0; i < 8; ++i) std::printf(" %lld", eh[i] - h[0][0]);
-    std::printf("\n");
     for (int c : {0, 1, 64, 65, 146, 147}) {
       if (c >= 2 * pl.grid) continue;
       std::printf("pair cta %3d:", c);
@@ -1624,7 +1584,7 @@ int pair_count() {
     }
     {
       using L = PairSmem<256, false>;
-      if (cudaFuncSetAttribute(gemm_tc_pair_kernel<256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      if (cudaFuncSetAttribute(gemm_tc_pair_kernel<256, false, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                L::kDynBytes) == cudaSuccess) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(sm_count() & ~1);
@@ -1636,7 +1596,7 @@ int pair_count() {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<256, false>, &cfg) == cudaSuccess && clusters > 0)
+        if (cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<256, false, -1>, &cfg) == cudaSuccess && clusters > 0)
           n = std::min(clusters, sm_count() / 2);
       }
       (void)cudaGetLastError();
@@ -1778,7 +1738,6 @@ cudaError_t launch_gemm_tc(const GemmParams& q, int mode, int* err_word, cudaStr
   ep.act = q.act; ep.act_alpha = q.act_alpha; ep.act_beta = q.act_beta;
   ep.res = q.residual; ep.ldres = q.ld_res; ep.sres = q.stride_res;
   ep.c16_hi = static_cast<uint2*>(q.c16_hi); ep.c16_lo = static_cast<uint2*>(q.c16_lo); ep.ldc16 = q.ldc16;
-  ep.c16_fixed = q.c16_fixed;
   ep.acc_scale = kmode == TC_F16X3 ? q.b16_inv_scale : nullptr;
   ep.acc_scale_const = (kmode == TC_F16X3 && pre) ? kFixedUnscale : 1.f;   // A arrives on the fixed scale
   ep.b_row_scale = q.b_row_scale; ep.b_row_scale_stride = q.b_row_scale_stride; ep.k_total = (int)q.k;
@@ -1786,7 +1745,8 @@ cudaError_t launch_gemm_tc(const GemmParams& q, int mode, int* err_word, cudaStr
   ep.err = err_word;
   if (q.c16_hi) {
     // Only the pair kernel's common epilogues (and the tail fix-up) write the split result.
-    if (!(sh.pair && pre) || !q.c16_lo || q.batch != 1 || (q.n % 8) != 0 || (q.ldc16 % 8) != 0 ||
+    if (!(sh.pair && pre) || !q.c16_lo || !q.c16_fixed || q.batch != 1 || (q.n % 8) != 0 || (q.ldc16 % 8) != 0 ||
+        ((reinterpret_cast<uintptr_t>(q.c16_hi) | reinterpret_cast<uintptr_t>(q.c16_lo)) & 15) != 0 ||
         !gemm_tc_can_split_output(q.act, q.bias_n != nullptr, q.bias_m != nullptr, q.c_in && q.beta != 0.f, q.alpha, q.bias_scale) ||
         (q.c && ((q.ldc % 4) != 0 || (reinterpret_cast<uintptr_t>(q.c) & 15) != 0)) ||
         (q.residual && ((q.ld_res % 4) != 0 || (reinterpret_cast<uintptr_t>(q.residual) & 15) != 0)) ||
@@ -1795,7 +1755,6 @@ cudaError_t launch_gemm_tc(const GemmParams& q, int mode, int* err_word, cudaStr
   } else if (!q.c) {
     return cudaErrorInvalidValue;
   }
-  ep.dbg = std::getenv("ALTIUS_CUDA_TC_DBG") ? std::atoi(std::getenv("ALTIUS_CUDA_TC_DBG")) : 0;
   TcPlan pl = make_plan(q.m, q.n, q.k, q.batch, bn, sh.mt, (sh.pair && pre) ? 64 : (kmode == TC_F16X3 ? BK16 : BK),
                         sh.pair ? pair_count() : 0);
   if (pl.sc.tail_parts >= 2 && (!q.workspace || q.workspace_bytes < pl.workspace_bytes)) {
@@ -1804,8 +1763,20 @@ cudaError_t launch_gemm_tc(const GemmParams& q, int mode, int* err_word, cudaStr
     pl.sc.tail_parts = 0;
   }
   float* ws = q.workspace;
-  if (sh.pair && pre) return launch_pair<256, true>(q.a, q.lda, (int)q.k, ma, mal, mb, mbl, ep, pl, ws, err_word, st);
-  if (sh.pair) return launch_pair<256, false>(q.a, q.lda, (int)q.k, ma, ma, mb, mbl, ep, pl, ws, err_word, st);
+  if (sh.pair && pre) {
+    // Its offsets inside a tile are 32-bit.
+    const int key = std::max({ep.ldc, ep.ldres, ep.ldc16}) < (1ll << 24) ? epilogue_key(ep) : -1;
+#define AC_PAIR(KEYV) launch_pair<256, true, KEYV>(q.a, q.lda, (int)q.k, ma, mal, mb, mbl, ep, pl, ws, err_word, st)
+    if (key == 0) return AC_PAIR(0);
+    if (key == 1) return AC_PAIR(1);
+    if (key == 2) return AC_PAIR(2);
+    if (key == 3) return AC_PAIR(3);
+    if (key == ((ACT_GELU << 2) | 1)) return AC_PAIR((ACT_GELU << 2) | 1);
+    if (key == ((ACT_RELU << 2) | 1)) return AC_PAIR((ACT_RELU << 2) | 1);
+    return AC_PAIR(-1);
+#undef AC_PAIR
+  }
+  if (sh.pair) return launch_pair<256, false, -1>(q.a, q.lda, (int)q.k, ma, ma, mb, mbl, ep, pl, ws, err_word, st);
 #define AC_TC(BNV)                                                                                         \
   (kmode == TC_1X ? launch_tc<BNV, 1, TC_1X>(ma, mb, mbl, ep, pl, a_batched, b_batched, ws, err_word, st)     \
    : kmode == TC_F16X3                                                                                     \
@@ -1848,7 +1819,7 @@ cudaError_t launch_f16_split(const float* x, void* hi, void* lo, int64_t rows, i
 }
 
 bool gemm_tc_can_split_output(int act, bool bias_n, bool bias_m, bool c_in, float alpha, float bias_scale) {
-  // The epilogues the pair kernel has compiled in with the split store (epilogue_parked's callers).
+  // The epilogues the pair kernel has compiled in with the split store (epilogue_regs' callers).
   return !bias_m && !c_in && alpha == 1.f && bias_scale == 1.f && (act == ACT_NONE || (bias_n && (act == ACT_GELU || act == ACT_RELU)));
 }
 

@@ -193,6 +193,29 @@ __device__ __forceinline__ void tc_ld_32x16_nowait(uint32_t taddr, uint32_t (&v)
       : "memory");
 }
 
+// 16 lanes (from a lane of the warp's quarter that is a multiple of 16) x 16 columns: registers 4 j .. 4 j + 3 of
+// a lane are columns 8 j + 2 (lane % 4), + 1 of row lane / 4 and of row lane / 4 + 8. Without the wait.
+__device__ __forceinline__ void tc_ld_16x256_x2_nowait(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+// The wait, with the registers that the loads in front fill: no use of them moves ahead of it.
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&v)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
+               :
+               : "memory");
+}
+// Four neighbouring columns of a row from that fragment: (a0, a1) are the lane's of the first, (b0, b1) of the second
+// of two 8-column groups; even lanes get columns of the first (4 x (lane / 2 % 2) ..), odd ones of the second.
+__device__ __forceinline__ float4 quad_exchange(float a0, float a1, float b0, float b1, int odd) {
+  const float s0 = odd ? a0 : b0, s1 = odd ? a1 : b1;
+  const float g0 = __shfl_xor_sync(0xffffffffu, s0, 1), g1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+  return odd ? make_float4(g0, g1, b0, b1) : make_float4(a0, a1, g0, g1);
+}
+
 // Round to nearest (ties away from zero) to TF32's 10 mantissa bits, on the
 // integer ALU: cvt.rna.tf32.f32 gives the same bits but issues on the
 // quarter-rate conversion pipe.
@@ -332,21 +355,39 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // MMA of a CTA pair: M = 256 (128 rows per CTA), B rows split between the two CTAs; issued by
-// one thread of the leader CTA (rank 0). The eight zero words disable no output lane.
+// one thread of the leader CTA (rank 0).
 __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                 uint32_t accumulate) {
-  const uint32_t z = 0;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(z)
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Completion of the pair's MMAs issued so far -> one arrival on the mbarrier at a
-// shared::cluster address (own or peer CTA).
-__device__ __forceinline__ void tc_commit_pair(uint32_t cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr)
+// The same in a run of two instructions on one A: the first leaves it in the tensor core's operand
+// buffer, the second takes it from there instead of from shared memory.
+__device__ __forceinline__ void tc_mma_f16_pair_fill(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
+      : "memory");
+}
+__device__ __forceinline__ void tc_mma_f16_pair_lastuse(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16.collector::a::lastuse [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
+      : "memory");
+}
+// Completion of the pair's MMAs issued so far -> one arrival on the mbarrier at this shared-memory location in
+// both CTAs.
+__device__ __forceinline__ void tc_commit_pair_both(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3)
                : "memory");
 }
 

@@ -1,0 +1,80 @@
+"""Epilogues of the CTA-pair GEMM against float64 at the edges of its tiles (256 x 256; blocks of 16 x 16 within): a
+row or a few columns beyond whole tiles, columns that are whole float4s but not whole groups of eight, K-sliced
+last tiles. The bound is the one of all fp16-split products: 1e-5 of the result and 5e-6 of sum |a||b|."""
+import numpy as np
+import pytest
+import torch
+
+from altius_b200 import ir
+from altius_b200.session import CudaSessionBuilder
+
+pytestmark = pytest.mark.gpu
+
+
+def _t(a):
+    return torch.from_numpy(a).double().cuda()
+
+
+def _run(graph, inputs, kinds):
+    sess = CudaSessionBuilder(ir.Model(graph, 13)).build()
+    try:
+        assert [e["kind"] for e in sess.schedule()] == kinds
+        return torch.from_numpy(sess.run(inputs)[0]).double().cuda()
+    finally:
+        sess.close()
+
+
+@pytest.mark.parametrize("m,n,k", [(2817, 1544, 264), (6305, 772, 392), (2561, 2308, 384)])
+@pytest.mark.parametrize("act", [None, "ReLU", "Gelu", "HardSwish"])
+@pytest.mark.parametrize("bias,res", [(False, False), (True, False), (False, True), (True, True)])
+def test_pair_epilogues(cuda_lib, m, n, k, act, bias, res):
+    rng = np.random.default_rng(m + n)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    w = (rng.standard_normal((k, n)) / np.sqrt(k)).astype(np.float32)
+    b = rng.standard_normal(n).astype(np.float32)
+    r = rng.standard_normal((m, n)).astype(np.float32)
+    g = ir.Graph()
+    xi = g.add_input("x", x.shape)
+    ri = g.add_input("r", r.shape) if res else None
+    y = g.op("MatMul", xi, g.new_init(w))
+    y = g.op("Add", y, g.new_init(b)) if bias else y
+    y = g.op("Mul", y, g.op("HardSigmoid", y)) if act == "HardSwish" else g.op(act, y) if act else y
+    g.outputs.append(g.op("Add", y, ri) if res else y)
+    got = _run(g, [x] + ([r] if res else []), ["act_f16_split", "gemm_f16x3_pair_tcgen05"])
+    want, mass, slack = _t(x) @ _t(w), _t(x).abs() @ _t(w).abs(), 0
+    if bias:
+        want, mass = want + _t(b), mass + _t(b).abs()
+    if act == "HardSwish":
+        want = want * (0.2 * want + 0.5).clamp(0, 1)
+        mass = 2 * mass                             # its slope is at most 1.5
+    elif act:
+        slack = 1e-6 * want.abs() if act == "Gelu" else 0   # the rational tanh and its cancellation against 1
+        want = torch.relu(want) if act == "ReLU" else torch.nn.functional.gelu(want, approximate="tanh")
+    if res:
+        want, mass = want + _t(r), mass + _t(r).abs()
+    assert ((got - want).abs() <= 1e-5 * want.abs() + 5e-6 * mass + slack).all()
+
+
+@pytest.mark.parametrize("m,h,n", [(2817, 1544, 512), (2561, 2312, 768)])
+def test_pair_writes_split_results_with_ragged_columns(cuda_lib, m, h, n):
+    """The first product's result exists only as fp16 halves (16 bytes of a row per lane); columns end inside a
+    64-column group."""
+    rng = np.random.default_rng(h)
+    x = rng.standard_normal((m, 384)).astype(np.float32)
+    w1 = (rng.standard_normal((384, h)) / np.sqrt(384)).astype(np.float32)
+    b1 = rng.standard_normal(h).astype(np.float32)
+    w2 = (rng.standard_normal((h, n)) / np.sqrt(h)).astype(np.float32)
+    g = ir.Graph()
+    y = g.op("ReLU", g.op("Add", g.op("MatMul", g.add_input("x", x.shape), g.new_init(w1)), g.new_init(b1)))
+    g.outputs.append(g.op("MatMul", y, g.new_init(w2)))
+    sess = CudaSessionBuilder(ir.Model(g, 13)).build()
+    try:
+        assert [e["kind"] for e in sess.schedule()][:2] == ["act_f16_split", "gemm_f16x3_pair_tcgen05"]
+        got = torch.from_numpy(sess.run([x])[0]).double().cuda()
+    finally:
+        sess.close()
+    h64 = torch.relu(_t(x) @ _t(w1) + _t(b1))
+    h_err = 1e-5 * h64 + 5e-6 * (_t(x).abs() @ _t(w1).abs() + _t(b1).abs())
+    want = h64 @ _t(w2)
+    bound = 1e-5 * want.abs() + 5e-6 * (h64 @ _t(w2).abs()) + h_err @ _t(w2).abs()
+    assert ((got - want).abs() <= bound).all()
