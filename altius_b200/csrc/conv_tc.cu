@@ -69,8 +69,11 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 }
 
 // ONE: one accumulator for all terms, two buffers (a block that does not walk uses the first).
+// 96 registers: a quarter of an SM holds five such warps (16384 registers), so that two blocks of nine fit. With 112 it held four,
+// one block per SM, whatever the shared memory left (32 images of 16 x 112 x 112 into 64 channels: 9 warps active, issue 32 %,
+// 56 us; MobileNetV3-Large at 32 images 919 us, with two blocks 798).
 template <bool WINDOW, int ACT, bool ONE>
-__global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
+__global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], w_full;
@@ -94,7 +97,7 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], kLoaders + (p.resident ? 0 : 1));   // every loader once, and the bulk copy's bytes
+      mbar_init(&full[s], kLoaders / 32 + (p.resident ? 0 : 1));   // every loader warp once, and the bulk copy's bytes
       mbar_init(&empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -221,21 +224,18 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
       for (int j = 0; j < 16; ++j) d[j] = __fmul_rn(d[j], gv[j]);
     };
 
-    float v[16], nx[16];
-    uint32_t use = 0, nuse = 0;
+    float v[16];
+    uint32_t use = 0;
     int g = 0;                                 // running K step
     bool alive = true;
     // Loads steps [from, to) of tile i (the first of them is already in v) into the ring; leaves the step
     // behind them in v.
     auto fill = [&](int i, int from, int to) {
       for (int kb = from; kb < to && alive; ++kb, ++g) {
-        const float* gc = gcol;
-        if (kb + 1 == kbs) place(i + 1);
-        if (kb + 1 < kbs || i + 1 < mine) nuse = fetch(kb + 1 < kbs ? kb + 1 : 0, nx);
-        if (gc) apply_gate(kb, gc, v);
+        if (gcol) apply_gate(kb, gcol, v);
         const int s = g % S;
         if (g >= S) {
-          if (!mbar_wait(&empty[s], ((g / S) & 1) ^ 1)) { atomicExch(p.err, 31); abort_flag = 1; alive = false; return; }
+          if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((g / S) & 1) ^ 1))) { atomicExch(p.err, 31); abort_flag = 1; alive = false; return; }
           if (tid == 0 && !p.resident) load_filter(g);
         }
         uint8_t* hi_t = smem + s * stage_bytes;
@@ -256,10 +256,12 @@ __global__ void __maxnreg__(112) conv_tc_kernel(const ConvTcDev p) {
           }
         }
         fence_proxy_async();
-        mbar_arrive(&full[s]);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = nx[j];
-        use = nuse;
+        __syncwarp();                          // one arrival per warp: those of 256 threads took their turns at the barrier
+        if (lane == 0) mbar_arrive(&full[s]);
+        // The next step's loads, under way over the epilogue that may lie in front of it. (A second set of registers for
+        // them would leave one block per SM.)
+        if (kb + 1 == kbs) place(i + 1);
+        if (kb + 1 < kbs || i + 1 < mine) use = fetch(kb + 1 < kbs ? kb + 1 : 0, v);
       }
     };
 
