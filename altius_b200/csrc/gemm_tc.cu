@@ -667,7 +667,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&ready[s], kSplitThreads);
+      mbar_init(&ready[s], kSplitThreads / 32);
       mbar_init(&empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -721,7 +721,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     }
   } else if (warp == kMmaWarp) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       // Instruction descriptor: fp32 accumulator, A and B both TF32 (format 2) or both
       // fp16 (format 0), both K-major, N = BN, M = 128.
       constexpr uint32_t kFmt = MODE == TC_F16X3 ? 0u : 2u;
@@ -802,7 +802,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           if (it % kSplitGroups != group) continue;
           const int s = it % S;
           const uint32_t ph = (it / S) & 1;
-          ok = mbar_wait(&full[s], ph);
+          ok = __all_sync(0xffffffffu, mbar_wait(&full[s], ph));
           if (MODE != TC_F16X3 && !ok) { atomicExch(err, 3); *abort_flag = 1; break; }
           if (MODE == TC_F16X3) {
             // fp32 rows of 32 floats -> fp16 hi / lo tiles; one float4 (4 consecutive k) per item.
@@ -865,7 +865,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             }
           }
           fence_proxy_async();
-          mbar_arrive(&ready[s]);
+          __syncwarp();                        // one arrival per warp
+          if (lane == 0) mbar_arrive(&ready[s]);
         }
       }
       // An element of A too large for fp16, or nothing but tiny ones: the result is not to be
