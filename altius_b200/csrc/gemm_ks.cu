@@ -382,6 +382,19 @@ cudaError_t launch_act(const CUtensorMap& ah, const CUtensorMap& al, const CUten
 
 inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
 
+// Products whose tiles take this kernel more than a round go to CTA pairs on tiles of 256 x 192 that hand their
+// accumulators over to fp32 sums every `run` K-blocks (launch_gemm_pair_sums; 0: stay here). In this kernel's clocks
+// such a tile takes 1300 a K-block and 6000 around them (us with a LayerNormalization in front, here -> there: 3152 x 768 x 768
+// 31.6 -> 23.2, 12672 x 384 x 384 37.3 -> 30.4, 788 x 768 x 3072 30.6 -> 22.7; but 2885 x 768 x 768 20.5 -> 23.0,
+// 1576 x 512 x 512 14.2 -> 18.4). Relative error against 64 bits with runs of two 1.6e-7 for any K, of one 1.2e-7; here
+// 2.1e-7 at K = 768, 2.0e-7 at 576, 1.5e-7 at 384 and 512: one there.
+int pair_sums_run(const GemmParams& q, double clocks) {
+  if (q.c16_hi && ((q.n % 8) || (q.ldc16 % 8) || !al16(q.c16_hi) || !al16(q.c16_lo))) return 0;
+  const int64_t nkb = (q.k + KB - 1) / KB, tiles = ((q.m + 255) / 256) * ((q.n + 191) / 192);
+  const int64_t rounds = (tiles + cluster_slots(2) - 1) / cluster_slots(2);
+  return 4000.0 + rounds * (1300.0 * nkb + 6000.0) < 0.97 * clocks ? (q.k > 576 ? 2 : 1) : 0;
+}
+
 }  // namespace
 
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k) {
@@ -400,6 +413,7 @@ cudaError_t launch_gemm_ks(const GemmParams& q, int* err_word, cudaStream_t st) 
       (q.c16_hi && (q.ldc16 % 4)) || !gemm_ks_epilogue_ok(q.act, q.bias_m != nullptr, q.beta != 0.f && q.c_in, q.alpha, q.bias_scale))
     return cudaErrorInvalidValue;
   const Shape sh = pick_shape(q.m, q.n, q.k);
+  if (const int run = pair_sums_run(q, sh.clocks)) return launch_gemm_pair_sums(q, run, err_word, st);
   KsDev d{};
   d.m = (int)q.m; d.n = (int)q.n; d.k = (int)q.k;
   d.bn = sh.bn; d.stages = sh.stages; d.kper = sh.kper; d.inv = sh.inv;

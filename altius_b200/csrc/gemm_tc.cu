@@ -426,14 +426,14 @@ __device__ __forceinline__ void hand_back(uint32_t acc_empty_leader, int lane) {
   if (lane == 0) mbar_arrive_cluster(acc_empty_leader);
 }
 
-template <int ACT, int BIAS, bool HAS_RES>
+template <int GROUPS, int ACT, int BIAS, bool HAS_RES>   // GROUPS of 16 columns
 __device__ __forceinline__ unsigned epilogue_regs(const TcEpilogue& ep, uint32_t acc, int q, int lane, int m0, int n0,
                                                   uint32_t acc_empty_leader) {
   const float sc = acc_scale_of(ep);
   const int odd = lane & 1, high = (lane >> 1) & 1;
   const int rl = q * 32 + (lane >> 2), cl = 8 * odd + 4 * high;   // the lane's first row and column of block 0
   const int rows = ep.m - m0 - rl, cols = ep.n - n0 - cl;          // how many there are from there on
-  const int blocks = 2 * min(4, (ep.n - n0 + 15) / 16);            // uniform across the warp
+  const int blocks = 2 * min(GROUPS, (ep.n - n0 + 15) / 16);           // uniform across the warp
   float seen_max = 0.f;                             // largest magnitude written as fixed-scale halves
   uint32_t nx[8];
   float4 nr[HAS_RES ? 2 : 1], nb = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -507,16 +507,16 @@ __device__ __forceinline__ unsigned epilogue_regs(const TcEpilogue& ep, uint32_t
 
 // The same walk for what the common epilogues do not cover: the unreduced accumulator of a K-slice into its
 // workspace tile [128][ld] (ws), or any epilogue, element by element.
-__device__ __noinline__ void epilogue_regs_other(const TcEpilogue& ep, float* ws, int ld, uint32_t acc, int q, int lane, int m0, int n0,
-                                                 int cg, uint32_t acc_empty_leader) {
+__device__ __noinline__ void epilogue_regs_other(const TcEpilogue& ep, float* ws, int ld, int groups, uint32_t acc, int q, int lane, int m0,
+                                                 int n0, int cg, uint32_t acc_empty_leader) {
   const float sc = acc_scale_of(ep);
   const int odd = lane & 1, high = (lane >> 1) & 1;
 #pragma unroll 1
-  for (int b = 0; b < 8; ++b) {
+  for (int b = 0; b < 2 * groups; ++b) {
     uint32_t u[8];
     tc_ld_16x256_x2_nowait(acc + ((uint32_t)(q * 32 + 16 * (b & 1)) << 16) + (uint32_t)(16 * (b >> 1)), u);
     tc_wait_ld(u);
-    if (b == 7) hand_back(acc_empty_leader, lane);
+    if (b + 1 == 2 * groups) hand_back(acc_empty_leader, lane);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       float4 x = quad_exchange(__uint_as_float(u[2 * h]), __uint_as_float(u[2 * h + 1]), __uint_as_float(u[4 + 2 * h]),
@@ -602,6 +602,7 @@ struct TcSmem {
 // the epilogue. tail_parts < 2: no slicing, dp_tiles == num_tiles.
 struct TcSched {
   int num_tiles, dp_tiles, tail_parts, num_kb;
+  int run;                 // pair kernel with SUM: K-blocks on one accumulator
 };
 struct TcWork {
   int tile, k0, k1, raw;   // raw: workspace slot, or -1 for a whole tile with the real epilogue
@@ -988,10 +989,10 @@ struct PairSmem {
   static constexpr int kOffALo = kABytes;
   static constexpr int kOffBHi = 2 * kABytes;
   static constexpr int kOffBLo = kOffBHi + kBBytes;
-  static_assert(!PRE || kABytes == kBBytes, "entries of one size");
+  static_assert(!PRE || kABytes >= kBBytes, "entries of one size");
   static constexpr int kStageBytes = PRE ? 2 * kABytes : 2 * kABytes + 2 * kBBytes;
-  // TMA brings B only (A goes global -> registers -> tiles); PRE: a whole entry
-  static constexpr int kTxBytes = PRE ? 2 * kABytes : 2 * kBBytes;
+  // TMA brings B only (A goes global -> registers -> tiles); PRE: a K-block's two entries
+  static constexpr int kTxBytes = PRE ? 2 * kABytes + 2 * kBBytes : 2 * kBBytes;
   // Epilogue memory: 4 KB per epilogue warp (none with PRE, whose epilogues work in registers).
   static constexpr int kEpiBytes = PRE ? 0 : kEpiWarps * 4096;
   static constexpr int kStages = (227 * 1024 - kEpiBytes - 1536) / kStageBytes;   // BN 256: 7 entries with PRE, else 6 stages
@@ -999,7 +1000,8 @@ struct PairSmem {
   // Without PRE: D1 and D2, one accumulator set. PRE: the operands are on fixed scales, the three
   // partial products share ONE accumulator, and two sets alternate between consecutive tiles, so
   // that a tile's epilogue runs under the next tile's MMAs.
-  static constexpr int kTmemCols = 2 * BN;
+  static constexpr int kSetCols = BN <= 128 ? 128 : 256;   // columns from one set to the next
+  static constexpr int kTmemCols = 2 * kSetCols;
   static_assert(kDynBytes <= 227 * 1024, "shared memory per CTA");
   static_assert(kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "tensor memory");
 };
@@ -1016,14 +1018,18 @@ __device__ __forceinline__ void pair_stamp(int dbg, int slot) {
 // entries of the ring each; kFlight of them, no more are in flight): one wait and one commit per K-block.
 // KEY: the common epilogue (epilogue_key) that is compiled in with PRE, -1 any other; all of them in one kernel
 // spilled 540 bytes a thread.
+// SUM: the tensor core truncates its sum at every instruction by up to an ulp of it, an error that grows with the
+// instructions behind one another. So an accumulator is given up after sc.run K-blocks; the epilogue warps add it to fp32
+// sums in their registers under the products of the next, and put the sums in the place of the last one for the epilogue.
 constexpr int kFlight = 4;
-template <int BN, bool PRE, int KEY>
+template <int BN, bool PRE, int KEY, bool SUM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
                     const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_alo,
                     const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_blo,
                     const __grid_constant__ TcEpilogue ep, const __grid_constant__ TcSched sc, int tiles_m, int tiles_n, float* workspace, int* err, int dbg) {
   using L = PairSmem<BN, PRE>;
+  static_assert(!SUM || kFlight * (2 * L::kABytes + 2 * L::kBBytes) <= L::kStages * L::kStageBytes, "ring");
   // Debug toggle: bits 16-19 of dbg, when set, use fewer stages of the ring.
   const int S = ((dbg >> 16) & 15) > 0 && ((dbg >> 16) & 15) < L::kStages ? ((dbg >> 16) & 15) : L::kStages;
   constexpr int KB = L::kKb;
@@ -1047,6 +1053,11 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
   if (threadIdx.x == 0) pair_stamp(dbg, 0);
 
   auto pwait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity); };
+  // PRE: entry i of the ring, A's (even) or B's of K-block i / 2. SUM: whole K-blocks, as many as are in flight, since two at
+  // a time stay until their cross terms are issued (in entries of one size there were three and a half).
+  auto entry = [&](int i) {
+    return smem + (SUM ? ((i >> 1) % kFlight) * (2 * L::kABytes + 2 * L::kBBytes) + (i & 1) * 2 * L::kABytes : (i % S) * L::kStageBytes);
+  };
   auto a_raw = [&](int s) { return smem + s * L::kStageBytes; };    // fp16 hi tile of A
   auto a_lo = [&](int s) { return smem + s * L::kStageBytes + L::kOffALo; };
   auto b_hi = [&](int s) { return smem + s * L::kStageBytes + L::kOffBHi; };
@@ -1096,16 +1107,16 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
             const int q = (it >> 1) % kFlight;
             const uint32_t rdy = map_to_cta(&ready[q], 0);         // the leader's barrier of this K-block
             for (int op = 0; op < 2; ++op, ++it) {
-              const int s = it % S, last = (it - S) >> 1;
-              if (it >= S && !pwait(&empty[last % kFlight], (last / kFlight) & 1)) { atomicExch(err, 1); *abort_flag = 1; ok = false; break; }
-              if (leader && op == 0) mbar_arrive_expect_tx(&ready[q], 4 * L::kTxBytes);
-              uint8_t* e = smem + s * L::kStageBytes;
+              const int last = SUM ? (it >> 1) - kFlight : (it - S) >> 1;
+              if (it >= (SUM ? 2 * kFlight : S) && !pwait(&empty[last % kFlight], (last / kFlight) & 1)) { atomicExch(err, 1); *abort_flag = 1; ok = false; break; }
+              if (leader && op == 0) mbar_arrive_expect_tx(&ready[q], 2 * L::kTxBytes);
+              uint8_t* e = entry(it);
               if (op == 0) {
                 tma_load_3d_pair(e, &tm_a, rdy, kb * KB, m0, 0);
                 tma_load_3d_pair(e + L::kABytes, &tm_alo, rdy, kb * KB, m0, 0);
               } else {
                 tma_load_3d_pair(e, &tm_b, rdy, kb * KB, tn * BN + (int)rank * (BN / 2), 0);
-                tma_load_3d_pair(e + L::kABytes, &tm_blo, rdy, kb * KB, tn * BN + (int)rank * (BN / 2), 0);
+                tma_load_3d_pair(e + L::kBBytes, &tm_blo, rdy, kb * KB, tn * BN + (int)rank * (BN / 2), 0);
               }
             }
           }
@@ -1129,32 +1140,60 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
       int it = 0, ti = 0;
       bool ok = true;
       TcWork wk;
-      for (int w = 0; ok && pair_get_work(sc, w, &wk); ++w, ++ti) {
-        // The epilogue warps must have drained this accumulator set (PRE: the tile before last).
+      for (int w = 0; ok && pair_get_work(sc, w, &wk); ++w)
+      for (int first = wk.k0, end; ok && first < wk.k1; first = end, ++ti) {
+        end = SUM ? min(first + sc.run, wk.k1) : wk.k1;        // K-blocks [first, end) on one accumulator
+        // The epilogue warps must have drained this accumulator set (PRE: the one before last).
         const bool two_sets = PRE && !(dbg & 1024);
         const int set = two_sets ? (ti & 1) : 0, use = two_sets ? (ti >> 1) : ti;
-        if (!mbar_wait(&acc_empty[set], (use & 1) ^ 1)) { atomicExch(err, 5); *abort_flag = 1; break; }
+        if (!mbar_wait(&acc_empty[set], (use & 1) ^ 1)) { atomicExch(err, 5); *abort_flag = 1; ok = false; break; }
         tc_fence_after();
-        const uint32_t d1 = tmem_base + (uint32_t)(set * BN);
+        const uint32_t d1 = tmem_base + (uint32_t)(set * L::kSetCols);
         if (PRE) {
-          for (int kb = wk.k0; kb < wk.k1; ++kb, it += 2) {
-            const int sa = it % S, sb = (it + 1) % S, kq = it >> 1;          // the K-block's A entry and B entry
+          // Operands on fixed scales: the cross terms go into the same accumulator.
+          struct Descs { uint64_t a, al, b, bl; };
+          auto descs = [&](int i) {
+            const uint32_t ea = smem_u32(entry(i)), eb = smem_u32(entry(i + 1));
+            return Descs{desc_sw128(ea), desc_sw128(ea + L::kABytes), desc_sw128(eb), desc_sw128(eb + L::kBBytes)};
+          };
+          auto landed = [&](int i) {                         // the K-block whose entries are i and i + 1
+            const int kq = i >> 1;
             ok = pwait(&ready[kq % kFlight], (kq / kFlight) & 1);
-            if (!ok) { atomicExch(err, 2); *abort_flag = 1; break; }
-            if (it == 0) pair_stamp(dbg, 2);
+            if (!ok) { atomicExch(err, 2); *abort_flag = 1; }
+            else if (i == 0) pair_stamp(dbg, 2);
             tc_fence_after();
-            const uint32_t ea = smem_u32(smem + sa * L::kStageBytes), eb = smem_u32(smem + sb * L::kStageBytes);
-            const uint64_t da = desc_sw128(ea), dal = desc_sw128(ea + L::kABytes);
-            const uint64_t db = desc_sw128(eb), dbl = desc_sw128(eb + L::kABytes);
-            // Operands on fixed scales: the cross terms go into the same accumulator.
+            return ok;
+          };
+          if (SUM) {
+            // The cross terms of a run first: 2^-11 of the result, they are added while the sum is small.
+            for (int kb = first, i = it; kb < end; ++kb, i += 2) {
+              if (!landed(i)) break;
+              const Descs d = descs(i);
+#pragma unroll
+              for (int kk = 0; kk < KB / 16; ++kk) {
+                const uint64_t off = (uint64_t)(kk * 2);
+                tc_mma_f16_pair(d1, d.al + off, d.b + off, idesc, (kb > first || kk > 0) ? 1u : 0u);
+                tc_mma_f16_pair(d1, d.a + off, d.bl + off, idesc, 1u);
+              }
+            }
+            for (int kb = first; ok && kb < end; ++kb, it += 2) {
+              const Descs d = descs(it);
+#pragma unroll
+              for (int kk = 0; kk < KB / 16; ++kk) tc_mma_f16_pair(d1, d.a + (uint64_t)(kk * 2), d.b + (uint64_t)(kk * 2), idesc, 1u);
+              tc_commit_pair_both(&empty[(it >> 1) % kFlight]);
+            }
+          } else
+          for (int kb = first; kb < end; ++kb, it += 2) {
+            if (!landed(it)) break;
+            const Descs d = descs(it);
 #pragma unroll
             for (int kk = 0; kk < KB / 16; ++kk) {          // K-steps of 16 halves (32 bytes of a row)
               const uint64_t off = (uint64_t)(kk * 2);
-              tc_mma_f16_pair(d1, dal + off, db + off, idesc, (kb > wk.k0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
-              tc_mma_f16_pair_fill(d1, da + off, dbl + off, idesc);                                 // a_hi * b_lo
-              tc_mma_f16_pair_lastuse(d1, da + off, db + off, idesc);                               // a_hi * b_hi
+              tc_mma_f16_pair(d1, d.al + off, d.b + off, idesc, (kb > first || kk > 0) ? 1u : 0u);   // a_lo * b_hi
+              tc_mma_f16_pair_fill(d1, d.a + off, d.bl + off, idesc);                                 // a_hi * b_lo
+              tc_mma_f16_pair_lastuse(d1, d.a + off, d.b + off, idesc);                               // a_hi * b_hi
             }
-            tc_commit_pair_both(&empty[kq % kFlight]);     // both entries are free again in both CTAs
+            tc_commit_pair_both(&empty[(it >> 1) % kFlight]);     // both entries are free again in both CTAs
           }
         } else
         for (int kb = wk.k0; kb < wk.k1; ++kb, ++it) {
@@ -1253,10 +1292,16 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
       const int t = wk.tile;
       const int tn = t % tiles_n, tm = (t / tiles_n) % tiles_m, bz = t / (tiles_n * tiles_m);
       const int m0 = tm * (2 * BM) + (int)rank * BM, n0 = tn * BN;
-      const bool two_sets = PRE && !(dbg & 1024);
-      const int set = two_sets ? (ti & 1) : 0, use = two_sets ? (ti >> 1) : ti;
-      const uint32_t acc = tmem_base + (uint32_t)(set * BN);
-      const uint32_t acc_empty_leader = map_to_cta(&acc_empty[set], 0);
+      uint32_t acc = 0, acc_empty_leader = 0;
+      auto next_acc = [&]() -> bool {    // waits for accumulator ti
+        const bool two_sets = PRE && !(dbg & 1024);
+        const int set = two_sets ? (ti & 1) : 0, use = two_sets ? (ti >> 1) : ti;
+        acc = tmem_base + (uint32_t)(set * L::kSetCols);
+        acc_empty_leader = map_to_cta(&acc_empty[set], 0);
+        const bool there = mbar_wait(&acc_full[set], use & 1);
+        tc_fence_after();
+        return there;
+      };
       if (PRE && ep.res && key >= 0 && wk.raw < 0) {
         // While the tile's MMAs run: pull this warp's 32 x 64 block of the residual into L2 -- but
         // not ahead of the kernel's first operand tiles (a thousand prefetches per SM issued at
@@ -1270,8 +1315,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
             asm volatile("prefetch.global.L2 [%0];" ::"l"(rp + (long long)row * ep.ldres + col));
         }
       }
-      if (!mbar_wait(&acc_full[set], use & 1)) { atomicExch(err, 4); *abort_flag = 1; break; }
-      tc_fence_after();
+      if (!next_acc()) { atomicExch(err, 4); *abort_flag = 1; break; }
       if (e == 0 && lane == 0 && ti < 3) pair_stamp(dbg, 8 + 2 * ti);     // accumulator of tile ti complete
       bool released = false;
       auto release = [&]() -> bool {     // all of this warp's tcgen05.ld have completed
@@ -1281,15 +1325,49 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         return true;
       };
       if (PRE) {
+        if (SUM && wk.k0 + sc.run < wk.k1) {
+          constexpr int NS = SUM ? BN / 64 : 1;
+          float sums[16 * NS];
+#pragma unroll
+          for (int j = 0; j < 16 * NS; ++j) sums[j] = 0.f;
+          bool there = true;
+#pragma unroll 1
+          for (int first = wk.k0;; first += sc.run) {
+            const bool last = first + sc.run >= wk.k1;
+            const uint32_t from = acc + (uint32_t)cg + ((uint32_t)(q * 32) << 16);
+            uint32_t u[2][16];
+            tc_ld_32x16_nowait(from, u[0]);
+            tc_ld_32x16_nowait(from + 16u, u[1]);
+            tc_wait_ld();
+#pragma unroll
+            for (int c = 0; c < NS; ++c) {            // two loads under way ahead of the sums
+#pragma unroll
+              for (int j = 0; j < 16; ++j) sums[16 * c + j] = __fadd_rn(sums[16 * c + j], __uint_as_float(u[c & 1][j]));
+              if (c + 2 < NS) tc_ld_32x16_nowait(from + (uint32_t)(16 * (c + 2)), u[c & 1]);
+              if (c >= 1 && c + 1 < NS) tc_wait_ld();
+            }
+            if (last) {
+#pragma unroll
+              for (int c = 0; c < NS; ++c) tc_st_32x16(from + (uint32_t)(16 * c), &sums[16 * c]);
+              asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+              break;
+            }
+            hand_back(acc_empty_leader, lane);
+            ++ti;
+            there = next_acc();
+            if (!there) break;
+          }
+          if (!there) { atomicExch(err, 4); *abort_flag = 1; break; }
+        }
         const int nw = n0 + cg;
         const uint32_t part = acc + (uint32_t)cg;
         if (m0 >= ep.m) hand_back(acc_empty_leader, lane);
         else if (wk.raw >= 0)
-          epilogue_regs_other(ep, workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, BN, part, q, lane, m0, nw, cg, acc_empty_leader);
+          epilogue_regs_other(ep, workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, BN, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
         else if (KEY >= 0)
-          seen_out |= epilogue_regs<(KEY >= 0 ? KEY >> 2 : 0), KEY & 1, (KEY & 2) != 0>(ep, part, q, lane, m0, nw, acc_empty_leader);
+          seen_out |= epilogue_regs<BN / 64, (KEY >= 0 ? KEY >> 2 : 0), KEY & 1, (KEY & 2) != 0>(ep, part, q, lane, m0, nw, acc_empty_leader);
         else
-          epilogue_regs_other(ep, nullptr, 0, part, q, lane, m0, nw, cg, acc_empty_leader);
+          epilogue_regs_other(ep, nullptr, 0, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
       } else if (m0 < ep.m) {
         if (wk.raw >= 0) {
           epilogue_raw<BN, D2>(workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, stage, acc, q, lane, cc0, cc1, acc_scale_of(ep));
@@ -1526,16 +1604,16 @@ cudaError_t launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtens
                     pl.tiles_m, pl.tiles_n);
 }
 
-template <int BN, bool PRE, int KEY>
+template <int BN, bool PRE, int KEY, bool SUM>
 cudaError_t launch_pair(const float* a, long long lda, int k, const CUtensorMap& ma, const CUtensorMap& mal,
                         const CUtensorMap& mb, const CUtensorMap& mbl, const TcEpilogue& ep, const TcPlan& pl,
                         float* workspace, int* err, cudaStream_t st) {
   using L = PairSmem<BN, PRE>;
   static unsigned long long attr_done = 0;
-  if (cudaError_t e0 = ensure_dynamic_smem(gemm_tc_pair_kernel<BN, PRE, KEY>, L::kDynBytes, &attr_done)) return e0;
+  if (cudaError_t e0 = ensure_dynamic_smem(gemm_tc_pair_kernel<BN, PRE, KEY, SUM>, L::kDynBytes, &attr_done)) return e0;
   // pl.grid counts pairs; the cluster shape (2, 1, 1) is a compile-time attribute of the kernel.
   static const int dbg = std::getenv("ALTIUS_CUDA_TC_DBG") ? std::atoi(std::getenv("ALTIUS_CUDA_TC_DBG")) : 0;
-  const cudaError_t e = launch_pdl(gemm_tc_pair_kernel<BN, PRE, KEY>, dim3(2u * (unsigned)pl.grid), dim3(kThreads), L::kDynBytes, st, 1, a, lda,
+  const cudaError_t e = launch_pdl(gemm_tc_pair_kernel<BN, PRE, KEY, SUM>, dim3(2u * (unsigned)pl.grid), dim3(kThreads), L::kDynBytes, st, 1, a, lda,
                                    k, ma, mal, mb, mbl, ep, pl.sc, pl.tiles_m, pl.tiles_n, workspace, err, dbg);
   if (dbg & 0x1000) {
     cudaStreamSynchronize(st);
@@ -1553,6 +1631,42 @@ cudaError_t launch_pair(const float* a, long long lda, int k, const CUtensorMap&
   dim3 grid((2 * BM * BN / 4 + 255) / 256, tail);
   return launch_pdl(gemm_tc_fixup_kernel, grid, dim3(256), 0, st, 1, workspace, ep, 2 * BM, BN, pl.sc.dp_tiles, pl.sc.tail_parts,
                     pl.tiles_m, pl.tiles_n);
+}
+
+// A arrives as fp16 halves: by the epilogue that is compiled in.
+template <int BN, bool SUM>
+cudaError_t launch_pair_key(const GemmParams& q, const CUtensorMap& ma, const CUtensorMap& mal, const CUtensorMap& mb, const CUtensorMap& mbl,
+                            const TcEpilogue& ep, const TcPlan& pl, float* ws, int* err, cudaStream_t st) {
+  // Its offsets inside a tile are 32-bit.
+  const int key = std::max({ep.ldc, ep.ldres, ep.ldc16}) < (1ll << 24) ? epilogue_key(ep) : -1;
+  switch (key) {
+#define AC_PAIR(KEYV) case KEYV: return launch_pair<BN, true, KEYV, SUM>(q.a, q.lda, (int)q.k, ma, mal, mb, mbl, ep, pl, ws, err, st)
+    AC_PAIR(0);
+    AC_PAIR(1);
+    AC_PAIR(2);
+    AC_PAIR(3);
+    AC_PAIR((ACT_GELU << 2) | 1);
+    AC_PAIR((ACT_RELU << 2) | 1);
+#undef AC_PAIR
+    default: return launch_pair<BN, true, -1, SUM>(q.a, q.lda, (int)q.k, ma, mal, mb, mbl, ep, pl, ws, err, st);
+  }
+}
+
+TcEpilogue epilogue_of(const GemmParams& q, int* err_word) {
+  TcEpilogue ep;
+  ep.m = (int)q.m; ep.n = (int)q.n;
+  ep.c = q.c; ep.ldc = q.ldc; ep.sc = q.stride_c;
+  ep.alpha = q.alpha; ep.beta = q.beta;
+  ep.cin = q.beta != 0.f ? q.c_in : nullptr; ep.ldcin = q.ldc_in; ep.scin = q.stride_c_in;
+  ep.bias_n = q.bias_n; ep.bias_m = q.bias_m; ep.bias_scale = q.bias_scale;
+  ep.act = q.act; ep.act_alpha = q.act_alpha; ep.act_beta = q.act_beta;
+  ep.res = q.residual; ep.ldres = q.ld_res; ep.sres = q.stride_res;
+  ep.c16_hi = static_cast<uint2*>(q.c16_hi); ep.c16_lo = static_cast<uint2*>(q.c16_lo); ep.ldc16 = q.ldc16;
+  ep.acc_scale = nullptr;
+  ep.acc_scale_const = 1.f;
+  ep.b_row_scale = nullptr; ep.b_row_scale_stride = 0; ep.k_total = (int)q.k;
+  ep.err = err_word;
+  return ep;
 }
 
 }  // namespace
@@ -1585,7 +1699,7 @@ int pair_count() {
     }
     {
       using L = PairSmem<256, false>;
-      if (cudaFuncSetAttribute(gemm_tc_pair_kernel<256, false, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      if (cudaFuncSetAttribute(gemm_tc_pair_kernel<256, false, -1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                L::kDynBytes) == cudaSuccess) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(sm_count() & ~1);
@@ -1597,7 +1711,7 @@ int pair_count() {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<256, false, -1>, &cfg) == cudaSuccess && clusters > 0)
+        if (cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<256, false, -1, false>, &cfg) == cudaSuccess && clusters > 0)
           n = std::min(clusters, sm_count() / 2);
       }
       (void)cudaGetLastError();
@@ -1730,20 +1844,11 @@ cudaError_t launch_gemm_tc(const GemmParams& q, int mode, int* err_word, cudaStr
       mbl = mb;
     }
   }
-  TcEpilogue ep;
-  ep.m = (int)q.m; ep.n = (int)q.n;
-  ep.c = q.c; ep.ldc = q.ldc; ep.sc = q.stride_c;
-  ep.alpha = q.alpha; ep.beta = q.beta;
-  ep.cin = q.beta != 0.f ? q.c_in : nullptr; ep.ldcin = q.ldc_in; ep.scin = q.stride_c_in;
-  ep.bias_n = q.bias_n; ep.bias_m = q.bias_m; ep.bias_scale = q.bias_scale;
-  ep.act = q.act; ep.act_alpha = q.act_alpha; ep.act_beta = q.act_beta;
-  ep.res = q.residual; ep.ldres = q.ld_res; ep.sres = q.stride_res;
-  ep.c16_hi = static_cast<uint2*>(q.c16_hi); ep.c16_lo = static_cast<uint2*>(q.c16_lo); ep.ldc16 = q.ldc16;
+  TcEpilogue ep = epilogue_of(q, err_word);
   ep.acc_scale = kmode == TC_F16X3 ? q.b16_inv_scale : nullptr;
   ep.acc_scale_const = (kmode == TC_F16X3 && pre) ? kFixedUnscale : 1.f;   // A arrives on the fixed scale
-  ep.b_row_scale = q.b_row_scale; ep.b_row_scale_stride = q.b_row_scale_stride; ep.k_total = (int)q.k;
+  ep.b_row_scale = q.b_row_scale; ep.b_row_scale_stride = q.b_row_scale_stride;
   if (q.b_row_scale && kmode != TC_3X_SPLIT_B_MN) return cudaErrorInvalidValue;   // exists for the [K, N] operand only
-  ep.err = err_word;
   if (q.c16_hi) {
     // Only the pair kernel's common epilogues (and the tail fix-up) write the split result.
     if (!(sh.pair && pre) || !q.c16_lo || !q.c16_fixed || q.batch != 1 || (q.n % 8) != 0 || (q.ldc16 % 8) != 0 ||
@@ -1764,20 +1869,8 @@ cudaError_t launch_gemm_tc(const GemmParams& q, int mode, int* err_word, cudaStr
     pl.sc.tail_parts = 0;
   }
   float* ws = q.workspace;
-  if (sh.pair && pre) {
-    // Its offsets inside a tile are 32-bit.
-    const int key = std::max({ep.ldc, ep.ldres, ep.ldc16}) < (1ll << 24) ? epilogue_key(ep) : -1;
-#define AC_PAIR(KEYV) launch_pair<256, true, KEYV>(q.a, q.lda, (int)q.k, ma, mal, mb, mbl, ep, pl, ws, err_word, st)
-    if (key == 0) return AC_PAIR(0);
-    if (key == 1) return AC_PAIR(1);
-    if (key == 2) return AC_PAIR(2);
-    if (key == 3) return AC_PAIR(3);
-    if (key == ((ACT_GELU << 2) | 1)) return AC_PAIR((ACT_GELU << 2) | 1);
-    if (key == ((ACT_RELU << 2) | 1)) return AC_PAIR((ACT_RELU << 2) | 1);
-    return AC_PAIR(-1);
-#undef AC_PAIR
-  }
-  if (sh.pair) return launch_pair<256, false, -1>(q.a, q.lda, (int)q.k, ma, ma, mb, mbl, ep, pl, ws, err_word, st);
+  if (sh.pair && pre) return launch_pair_key<256, false>(q, ma, mal, mb, mbl, ep, pl, ws, err_word, st);
+  if (sh.pair) return launch_pair<256, false, -1, false>(q.a, q.lda, (int)q.k, ma, ma, mb, mbl, ep, pl, ws, err_word, st);
 #define AC_TC(BNV)                                                                                         \
   (kmode == TC_1X ? launch_tc<BNV, 1, TC_1X>(ma, mb, mbl, ep, pl, a_batched, b_batched, ws, err_word, st)     \
    : kmode == TC_F16X3                                                                                     \
@@ -1791,6 +1884,26 @@ cudaError_t launch_gemm_tc(const GemmParams& q, int mode, int* err_word, cudaStr
   if (bn == 128) return AC_TC(128);
   return AC_TC(64);
 #undef AC_TC
+}
+
+// Whole tiles of 256 x 192, `run` K-blocks on one accumulator.
+cudaError_t launch_gemm_pair_sums(const GemmParams& q, int run, int* err_word, cudaStream_t st) {
+  constexpr int bn = 192;                      // 256 columns took 15 % more: half of the sums spill
+  const int pairs = pair_count();
+  if (pairs <= 0 || run < 1 || run > 2 || encode_fn() == nullptr) return cudaErrorInvalidValue;
+  CUtensorMap ma, mal, mb, mbl;
+  if (!make_map(&ma, q.a16_hi, 2, q.k, q.m, 1, q.lda16, 0, 64, BM, 1128) || !make_map(&mal, q.a16_lo, 2, q.k, q.m, 1, q.lda16, 0, 64, BM, 1128) ||
+      !make_map(&mb, q.b16_hi, 2, q.k, q.n, 1, q.ldb16, 0, 64, bn / 2, 1128) || !make_map(&mbl, q.b16_lo, 2, q.k, q.n, 1, q.ldb16, 0, 64, bn / 2, 1128))
+    return cudaErrorInvalidValue;
+  TcEpilogue ep = epilogue_of(q, err_word);
+  ep.acc_scale = q.b16_inv_scale;
+  ep.acc_scale_const = kFixedUnscale;
+  TcPlan pl = make_plan(q.m, q.n, q.k, 1, bn, 2, 64, pairs);
+  pl.sc.dp_tiles = pl.sc.num_tiles;            // no K-slices: they would need a workspace and a second kernel
+  pl.sc.tail_parts = 0;
+  pl.grid = std::min(pl.sc.num_tiles, pairs);
+  pl.sc.run = run;
+  return launch_pair_key<192, true>(q, ma, mal, mb, mbl, ep, pl, nullptr, err_word, st);
 }
 
 cudaError_t launch_f16_split(const float* x, void* hi, void* lo, int64_t rows, int64_t k, int64_t ld, int64_t k8,

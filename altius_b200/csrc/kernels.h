@@ -282,6 +282,8 @@ int cluster_slots(int split);
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k);
 bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bias_scale);
 cudaError_t launch_gemm_ks(const GemmParams& p, int* err_word, cudaStream_t st);
+// The same operands and epilogues on CTA pairs, `run` K-blocks of 64 on one accumulator (gemm_tc.cu).
+cudaError_t launch_gemm_pair_sums(const GemmParams& p, int run, int* err_word, cudaStream_t st);
 // fp16 split of a constant [rows, k] operand (row stride ld) into [rows, k8] halves
 // (k8 >= k, a multiple of 8, padding zero); leaves kGemmRangeCode in *err_word when an
 // element exceeds the fp16 range.

@@ -208,6 +208,14 @@ __device__ __forceinline__ void tc_wait_ld(uint32_t (&v)[8]) {
                :
                : "memory");
 }
+// Sixteen columns of the warp's 32 lanes, back to tensor memory.
+__device__ __forceinline__ void tc_st_32x16(uint32_t taddr, const float* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]),
+      "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
+      : "memory");
+}
 // Four neighbouring columns of a row from that fragment: (a0, a1) are the lane's of the first, (b0, b1) of the second
 // of two 8-column groups; even lanes get columns of the first (4 x (lane / 2 % 2) ..), odd ones of the second.
 __device__ __forceinline__ float4 quad_exchange(float a0, float a1, float b0, float b1, int odd) {

@@ -78,3 +78,31 @@ def test_pair_writes_split_results_with_ragged_columns(cuda_lib, m, h, n):
     want = h64 @ _t(w2)
     bound = 1e-5 * want.abs() + 5e-6 * (h64 @ _t(w2).abs()) + h_err @ _t(w2).abs()
     assert ((got - want).abs() <= bound).all()
+
+
+# Products that the kernel for few rows would take more than a round for: CTA pairs on 256 x 192 tiles whose accumulators
+# are given up every one or two K-blocks. Bound: what that kernel measured on these inputs. The last two have ragged rows, columns
+# and K.
+@pytest.mark.parametrize("m,d,n,bound", [(3152, 768, 768, 2.09e-7), (12672, 384, 384, 1.51e-7), (788, 768, 3072, 2.11e-7),
+                                         (6304, 384, 384, 1.53e-7), (3081, 840, 780, 2.35e-7), (8001, 520, 324, 1.62e-7)])
+@pytest.mark.parametrize("act,res", [(None, False), ("ReLU", True)])
+def test_pairs_with_short_accumulators(cuda_lib, m, d, n, bound, act, res):
+    rng = np.random.default_rng(m + n)
+    x = rng.standard_normal((m, d)).astype(np.float32)
+    w = (rng.standard_normal((d, n)) / np.sqrt(d)).astype(np.float32)
+    b = rng.standard_normal(n).astype(np.float32)
+    r = rng.standard_normal((m, n)).astype(np.float32)
+    g = ir.Graph()
+    xi = g.add_input("x", x.shape)
+    ri = g.add_input("r", r.shape) if res else None
+    h = g.op("LayerNormalization", xi, g.new_init(np.ones(d, np.float32)), g.new_init(np.zeros(d, np.float32)), axis=-1, epsilon=1e-6,
+             stash_type=1)
+    y = g.op("Add", g.op("MatMul", h, g.new_init(w)), g.new_init(b))
+    y = g.op(act, y) if act else y
+    g.outputs.append(g.op("Add", y, ri) if res else y)
+    got = _run(g, [x] + ([r] if res else []), ["layer_norm", "gemm_f16x3_cluster_tcgen05"])
+    y = torch.nn.functional.layer_norm(_t(x), (d,), None, None, 1e-6) @ _t(w) + _t(b)
+    y = torch.relu(y) if act else y
+    want = y + _t(r) if res else y
+    assert ((got - want).norm() / want.norm()).item() <= bound
+    assert ((got - want).abs() <= 1e-5 * want.abs() + 2e-5).all()
