@@ -366,6 +366,17 @@ __device__ __forceinline__ void epilogue_raw(float* ws_tile, float4* stage, uint
   }
 }
 
+// Four results as fp16 halves (n is a multiple of 8 then: the four columns exist together).
+__device__ __forceinline__ void fixup_split(const TcEpilogue& ep, int row, int col0, float4 y) {
+  uint2 h, l;
+  f16_split_fixed(y, h, l);
+  const long long o = ((long long)row * ep.ldc16 + col0) >> 2;
+  ep.c16_hi[o] = h;
+  ep.c16_lo[o] = l;
+  // A tile's few K-sliced elements say nothing about the tensor being tiny: overflow only.
+  if (split_seen_fixed(y) & 1u) atomicCAS(ep.err, 0, kRangeCode);
+}
+
 // The epilogue of four consecutive elements of row `row` from column `col0` on (n % 4 == 0 when
 // the split result is written): what the tail fix-up applies to the summed K-slices.
 __device__ __forceinline__ void fixup_apply(const TcEpilogue& ep, int row, int col0, int bz, float4 acc) {
@@ -396,16 +407,7 @@ __device__ __forceinline__ void fixup_apply(const TcEpilogue& ep, int row, int c
     if (c) c[(long long)row * ep.ldc + col] = y;
     y4[e] = y;
   }
-  if (ep.c16_hi) {   // n is a multiple of 8 here: the whole float4 is in range
-    uint2 h, l;
-    const float4 yv = make_float4(y4[0], y4[1], y4[2], y4[3]);
-    f16_split_fixed(yv, h, l);
-    const long long o = ((long long)row * ep.ldc16 + col0) >> 2;
-    ep.c16_hi[o] = h;
-    ep.c16_lo[o] = l;
-    // A tile's few K-sliced elements say nothing about the tensor being tiny: overflow only.
-    if (split_seen_fixed(yv) & 1u) atomicCAS(ep.err, 0, kRangeCode);
-  }
+  if (ep.c16_hi) fixup_split(ep, row, col0, make_float4(y4[0], y4[1], y4[2], y4[3]));
 }
 
 // The epilogue of the pair kernel that takes A pre-split: sixteen warps, a warp per tensor-memory lane
@@ -529,38 +531,69 @@ __device__ __noinline__ void epilogue_regs_other(const TcEpilogue& ep, float* ws
   }
 }
 
-// Adds the K-slices of the tail tiles in slice order and applies the epilogue.
-__global__ void __launch_bounds__(256) gemm_tc_fixup_kernel(const float* ws, const __grid_constant__ TcEpilogue ep, int bm,
-                                                            int bn, int dp_tiles, int parts, int tiles_m,
-                                                            int tiles_n) {
+// Adds the K-slices of the tail tiles and applies the epilogue. What bounds it is latency (a tile of 256 x 256 in 24 slices is
+// 6 MB): all loads are under way at once, bias and residual with the slices'. With many slices eight groups of four lanes take
+// one in eight each and add up through the warp, so that no lane has more than four (a thread for all slices, eight loads a
+// round: 7.1 us behind the products of ViT-B/16 at 32 images). The order of the sum is fixed: slices g, g + GROUPS, .. of each
+// group, then the groups. 64 registers, 128 threads and no shared memory: a block fits beside one of the kernel in front.
+constexpr int kFixThreads = 128;
+template <int GROUPS>
+__global__ void __maxnreg__(64) gemm_tc_fixup_kernel(const float* ws, const __grid_constant__ TcEpilogue ep, int bm,
+                                                     int bn, int dp_tiles, int parts, int tiles_m, int tiles_n) {
+  constexpr int PER = kFixThreads / GROUPS, LANES = 32 / GROUPS, LOADS = GROUPS == 1 ? 6 : 4;   // slices a lane has under way
   pdl_trigger();
-  pdl_wait();
-  const int tt = blockIdx.y;
-  const int t = dp_tiles + tt;
+  const int tt = blockIdx.y, t = dp_tiles + tt;
   const int tn = t % tiles_n, tm = (t / tiles_n) % tiles_m, bz = t / (tiles_n * tiles_m);
-  const int e4 = blockIdx.x * 256 + threadIdx.x;          // float4 index inside the tile
-  if (e4 >= bm * bn / 4) return;
+  const int lane = threadIdx.x & 31, group = lane / LANES;
+  const int e4 = blockIdx.x * PER + (threadIdx.x >> 5) * LANES + lane % LANES;   // float4 index inside the tile
   const int rl = e4 / (bn / 4), cl = (e4 % (bn / 4)) * 4;
   const int row = tm * bm + rl, col0 = tn * bn + cl;
-  if (row >= ep.m || col0 >= ep.n) return;
-  const float* src = ws + (size_t)tt * parts * bm * bn + (size_t)rl * bn + cl;
-  // Slices are added in slice order; their loads are issued eight at a time so that the
-  // chain of additions does not also serialise the L2 round trips.
-  float4 acc = __ldcg(reinterpret_cast<const float4*>(src));
-  auto add = [&](const float4& v) {
-    acc.x = __fadd_rn(acc.x, v.x); acc.y = __fadd_rn(acc.y, v.y);
-    acc.z = __fadd_rn(acc.z, v.z); acc.w = __fadd_rn(acc.w, v.w);
-  };
-  int p = 1;
-  for (; p + 8 <= parts; p += 8) {
-    float4 v[8];
+  const bool live = e4 < bm * bn / 4 && row < ep.m && col0 < ep.n, mine = live && group == 0;
+  const int key = epilogue_key(ep);
+  const bool common = key >= 0 && !(key & 64);            // n % 4 == 0: the four columns exist together
+  float4 b = make_float4(0.f, 0.f, 0.f, 0.f), r = b, acc = b;
+  pdl_wait();
+  if (live) {
+    const size_t step = (size_t)bm * bn;
+    const float* src = ws + (size_t)tt * parts * step + (size_t)rl * bn + cl;
+    for (int p0 = group; p0 < parts; p0 += LOADS * GROUPS) {
+      float4 v[LOADS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(p + j) * bm * bn));
+      for (int j = 0; j < LOADS; ++j)
+        v[j] = p0 + j * GROUPS < parts ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)(p0 + j * GROUPS) * step)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p0 == 0 && common) {
+        if (ep.bias_n) b = ld_plain(reinterpret_cast<const float4*>(ep.bias_n + col0));
+        if (ep.res) r = ld_plain(reinterpret_cast<const float4*>(ep.res + (long long)bz * ep.sres + (long long)row * ep.ldres + col0));
+      }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) add(v[j]);
+      for (int j = 0; j < LOADS; ++j) {
+        acc.x = __fadd_rn(acc.x, v[j].x); acc.y = __fadd_rn(acc.y, v[j].y);
+        acc.z = __fadd_rn(acc.z, v[j].z); acc.w = __fadd_rn(acc.w, v[j].w);
+      }
+    }
   }
-  for (; p < parts; ++p) add(__ldcg(reinterpret_cast<const float4*>(src + (size_t)p * bm * bn)));
-  fixup_apply(ep, row, col0, bz, acc);
+#pragma unroll
+  for (int o = LANES; o < 32; o *= 2) {
+    acc.x = __fadd_rn(acc.x, __shfl_xor_sync(0xffffffffu, acc.x, o)); acc.y = __fadd_rn(acc.y, __shfl_xor_sync(0xffffffffu, acc.y, o));
+    acc.z = __fadd_rn(acc.z, __shfl_xor_sync(0xffffffffu, acc.z, o)); acc.w = __fadd_rn(acc.w, __shfl_xor_sync(0xffffffffu, acc.w, o));
+  }
+  if (!mine) return;
+  if (!common) {
+    fixup_apply(ep, row, col0, bz, acc);
+    return;
+  }
+  if (ep.bias_n) acc = make_float4(__fadd_rn(acc.x, b.x), __fadd_rn(acc.y, b.y), __fadd_rn(acc.z, b.z), __fadd_rn(acc.w, b.w));
+  if (ep.act == ACT_GELU) {
+    const float2 g0 = gelu_ref2(make_float2(acc.x, acc.y)), g1 = gelu_ref2(make_float2(acc.z, acc.w));
+    acc = make_float4(g0.x, g0.y, g1.x, g1.y);
+  } else if (ep.act != ACT_NONE) {
+    const float al = ep.act_alpha, be = ep.act_beta;
+    acc = make_float4(apply_act(ep.act, acc.x, al, be), apply_act(ep.act, acc.y, al, be), apply_act(ep.act, acc.z, al, be),
+                      apply_act(ep.act, acc.w, al, be));
+  }
+  if (ep.res) acc = make_float4(__fadd_rn(acc.x, r.x), __fadd_rn(acc.y, r.y), __fadd_rn(acc.z, r.z), __fadd_rn(acc.w, r.w));
+  if (ep.c) *reinterpret_cast<float4*>(ep.c + (long long)bz * ep.sc + (long long)row * ep.ldc + col0) = acc;
+  if (ep.c16_hi) fixup_split(ep, row, col0, acc);
 }
 
 // Shared-memory stage of the main loop. MT = 128-row sub-tiles per CTA tile.
@@ -1588,6 +1621,16 @@ TcPlan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int bn, int mt,
   return pl;
 }
 
+cudaError_t launch_fixup(const float* ws, const TcEpilogue& ep, int bm, int bn, const TcPlan& pl, cudaStream_t st) {
+  // Eight groups make eight times as many blocks: for one tile they are 1024. (For eight tiles in six slices, ViT-B/16 at 16
+  // images, they took 3.5 us more than one group.)
+  const int tail = pl.sc.num_tiles - pl.sc.dp_tiles;
+  const int groups = pl.sc.tail_parts > 4 && (long long)tail * bm * bn <= 256 * 256 ? 8 : 1, per = kFixThreads / groups;
+  const dim3 grid((bm * bn / 4 + per - 1) / per, tail);
+  return launch_pdl(groups == 8 ? gemm_tc_fixup_kernel<8> : gemm_tc_fixup_kernel<1>, grid, dim3(kFixThreads), 0, st, 1, ws, ep, bm, bn,
+                    pl.sc.dp_tiles, pl.sc.tail_parts, pl.tiles_m, pl.tiles_n);
+}
+
 template <int BN, int MT, int MODE>
 cudaError_t launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mbl,
                       const TcEpilogue& ep, const TcPlan& pl, int a_batched, int b_batched, float* workspace,
@@ -1598,10 +1641,7 @@ cudaError_t launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtens
   const cudaError_t e = launch_pdl(gemm_tc_kernel<BN, MT, MODE>, dim3((unsigned)pl.grid), dim3(kThreads), L::kDynBytes, st, 1, ma, mb,
                                    mbl, ep, pl.sc, a_batched, b_batched, pl.tiles_m, pl.tiles_n, workspace, err);
   if (e != cudaSuccess || pl.sc.tail_parts < 2) return e;
-  const int tail = pl.sc.num_tiles - pl.sc.dp_tiles;
-  dim3 grid((MT * BM * BN / 4 + 255) / 256, tail);
-  return launch_pdl(gemm_tc_fixup_kernel, grid, dim3(256), 0, st, 1, workspace, ep, MT * BM, BN, pl.sc.dp_tiles, pl.sc.tail_parts,
-                    pl.tiles_m, pl.tiles_n);
+  return launch_fixup(workspace, ep, MT * BM, BN, pl, st);
 }
 
 template <int BN, bool PRE, int KEY, bool SUM>
@@ -1627,10 +1667,7 @@ cudaError_t launch_pair(const float* a, long long lda, int k, const CUtensorMap&
     }
   }
   if (e != cudaSuccess || pl.sc.tail_parts < 2) return e;
-  const int tail = pl.sc.num_tiles - pl.sc.dp_tiles;
-  dim3 grid((2 * BM * BN / 4 + 255) / 256, tail);
-  return launch_pdl(gemm_tc_fixup_kernel, grid, dim3(256), 0, st, 1, workspace, ep, 2 * BM, BN, pl.sc.dp_tiles, pl.sc.tail_parts,
-                    pl.tiles_m, pl.tiles_n);
+  return launch_fixup(workspace, ep, 2 * BM, BN, pl, st);
 }
 
 // A arrives as fp16 halves: by the epilogue that is compiled in.
