@@ -90,14 +90,16 @@ HostStage::~HostStage() {
   if (ring_) cudaFreeHost(ring_);
 }
 
-// Copies the next chunk below `limit` whose slot is free; false if there is none now.
+// Copies the next piece of a chunk below `limit` whose slot is free; false if there is none now.
 bool HostStage::copy_next(int limit) {
-  int c = next_.load(std::memory_order_relaxed);
+  int i = next_.load(std::memory_order_relaxed);
+  const int c = i / kPieces;
   if (c >= limit || c >= allowed_.load(std::memory_order_acquire)) return false;
-  if (!next_.compare_exchange_strong(c, c + 1)) return false;
-  const size_t at = (size_t)c * kChunk;
-  copy_past_caches(ring_ + (size_t)(c % kSlots) * kChunk, src_ + at, std::min(kChunk, bytes_ - at));
-  done_[c].store(1, std::memory_order_release);
+  if (!next_.compare_exchange_strong(i, i + 1)) return false;
+  constexpr size_t kPiece = kChunk / kPieces;
+  const size_t in = (size_t)(i % kPieces) * kPiece, at = (size_t)c * kChunk + in;
+  if (at < bytes_) copy_past_caches(ring_ + (size_t)(c % kSlots) * kChunk + in, src_ + at, std::min(kPiece, bytes_ - at));
+  done_[c].fetch_add(1, std::memory_order_release);
   return true;
 }
 
@@ -111,7 +113,7 @@ void HostStage::worker() {
       seen = job_;
       ++busy_;
     }
-    while (next_.load(std::memory_order_relaxed) < chunks_)
+    while (next_.load(std::memory_order_relaxed) < chunks_ * kPieces)
       if (!copy_next(chunks_)) relax();
     std::lock_guard<std::mutex> lock(m_);
     --busy_;
@@ -167,7 +169,7 @@ cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStre
       }
       if (err != cudaSuccess) break;
       if (!copy_next(c + 1)) relax();         // this chunk itself, if no worker has taken it yet
-    } while (!done_[c].load(std::memory_order_acquire));
+    } while (done_[c].load(std::memory_order_acquire) < kPieces);
     if (err != cudaSuccess) break;
     const size_t at = (size_t)c * kChunk;
     err = cudaMemcpyAsync(static_cast<char*>(dst) + at, ring_ + (size_t)(c % kSlots) * kChunk, std::min(kChunk, bytes - at),
@@ -175,7 +177,7 @@ cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStre
     if (err == cudaSuccess) err = cudaEventRecord(left_[c % kSlots], st);
   }
   if (err != cudaSuccess) {                   // nobody may go on reading the caller's memory
-    next_.store(n);
+    next_.store(n * kPieces);
     for (;;) {
       std::lock_guard<std::mutex> lock(m_);
       if (busy_ == 0) break;

@@ -29,6 +29,8 @@ class HostStage {
 
  private:
   static constexpr size_t kChunk = size_t(1) << 20;
+  static constexpr int kPieces = 4;           // a chunk is copied by several threads, so that the first is on its way after 25 us
+                                              // (whole chunks: 38 MB 980 us behind the device time, this way 860)
   static constexpr int kSlots = 12;
   HostStage() = default;
   bool init();
@@ -47,8 +49,8 @@ class HostStage {
   const char* src_ = nullptr;
   size_t bytes_ = 0;
   int chunks_ = 0;
-  std::atomic<int> next_{0}, allowed_{0};     // next chunk to copy; chunks below `allowed_` have a free slot
-  std::unique_ptr<std::atomic<char>[]> done_;
+  std::atomic<int> next_{0}, allowed_{0};     // next piece to copy; chunks below `allowed_` have a free slot
+  std::unique_ptr<std::atomic<char>[]> done_;   // pieces of a chunk that have been copied
   int done_size_ = 0;
 };
 
