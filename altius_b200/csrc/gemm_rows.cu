@@ -13,16 +13,66 @@
 namespace ac {
 namespace {
 
-constexpr int kWarps = 8;
+constexpr int kWarps = 8, KC = 1024;
+
+// Eight rows of A are more than a lane can have under way beside B: the block brings them to shared memory, KC
+// floats of K at a time, while each lane already loads its part of B for the next four steps. 80 registers, so that
+// three blocks share an SM. (Rows from L1, two steps at a time, two blocks: 16.8 of 20 issue slots waited for a load;
+// 32 x 960 x 1280 19 us.)
+__device__ __forceinline__ void cp16(float4* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
 
 template <int MT, int NW>
-__global__ void __launch_bounds__(kWarps * 32) gemm_rows_kernel(const GemmParams p) {
+__device__ __forceinline__ void staged_products(const float* const (&a)[MT], const float* const (&b)[NW], int K, int lane, float (&acc)[NW][MT]) {
+  __shared__ float4 as[MT * (KC / 4)];
+  for (int kc = 0; kc < K; kc += KC) {
+    const int kn = min(KC, K - kc), quads = kn / 4;
+    if (kc) __syncthreads();                   // everybody is through with the part before
+    for (int i = threadIdx.x; i < MT * (KC / 4); i += kWarps * 32) {
+      const int r = i / (KC / 4), q = i % (KC / 4);
+      const float* row = a[0];
+#pragma unroll
+      for (int e = 1; e < MT; ++e) row = r == e ? a[e] : row;
+      if (q < quads) cp16(&as[i], row + kc + 4 * q);
+    }
+    float4 bv[4][NW];
+    auto request = [&](int u, int k) {
+#pragma unroll
+      for (int j = 0; j < NW; ++j)
+        bv[u][j] = k < kn ? ld_plain(reinterpret_cast<const float4*>(b[j] + kc + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+#pragma unroll
+    for (int u = 0; u < 4; ++u) request(u, lane * 4 + 128 * u);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int k0 = lane * 4; k0 < kn; k0 += 512) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int k = k0 + 128 * u;
+        if (k < kn) {
+#pragma unroll
+          for (int i = 0; i < MT; ++i) {
+            const float4 av = as[i * (KC / 4) + k / 4];
+#pragma unroll
+            for (int j = 0; j < NW; ++j)
+              acc[j][i] = fmaf(av.x, bv[u][j].x, fmaf(av.y, bv[u][j].y, fmaf(av.z, bv[u][j].z, fmaf(av.w, bv[u][j].w, acc[j][i]))));
+          }
+        }
+        request(u, k + 512);
+      }
+    }
+  }
+}
+
+template <int MT, int NW>
+__global__ void __launch_bounds__(kWarps * 32, MT == 8 ? 3 : 1) gemm_rows_kernel(const GemmParams p) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n0 = (blockIdx.x * kWarps + warp) * NW, m0 = blockIdx.y * MT;
   const int N = (int)p.n, M = (int)p.m, K = (int)p.k;
   pdl_trigger();
   pdl_wait();
-  if (n0 >= N) return;
+  if (MT < 8 && n0 >= N) return;
   const float* a[MT];
   const float* b[NW];
 #pragma unroll
@@ -34,6 +84,8 @@ __global__ void __launch_bounds__(kWarps * 32) gemm_rows_kernel(const GemmParams
   for (int j = 0; j < NW; ++j)
 #pragma unroll
     for (int i = 0; i < MT; ++i) acc[j][i] = 0.f;
+  if (MT == 8) staged_products<MT, NW>(a, b, K, lane, acc);
+  else
 #pragma unroll (MT <= 2 ? 4 : 2)
   for (int k = lane * 4; k < K; k += 128) {
     float4 bv[NW];

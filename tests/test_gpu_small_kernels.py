@@ -227,3 +227,19 @@ def test_few_row_products_beyond_the_fixed_scale(cuda_lib):
                 assert np.linalg.norm(a - b.numpy()) <= 1e-5 * np.linalg.norm(b.numpy())
     finally:
         sess.close()
+
+
+# eight rows a block, in parts of 1024 floats of K: one part, a whole and a ragged second one, fewer quads than lanes, rows and
+# columns off the tile; a row of A without finite values stays in its row
+@pytest.mark.parametrize("m,k,n", [(5, 1024, 33), (8, 1028, 16), (13, 2048, 17), (31, 2564, 40), (6, 20, 5)])
+def test_product_of_eight_rows_in_parts_of_k(cuda_lib, m, k, n):
+    rng = np.random.default_rng(m * k + n)
+    a = rng.standard_normal((m, k)).astype(np.float32)
+    w = rng.standard_normal((n, k)).astype(np.float32)
+    a[1, k - 1] = np.inf
+    got = _run(lambda g, x: g.op("Gemm", x, g.new_init(w), g.new_init(np.zeros(n, np.float32)), alpha=1.0, beta=1.0, trans_a=False,
+                                 trans_b=True), [a], ["gemm_fp32_rows"])
+    assert np.isinf(got[1]).all()
+    rest = np.arange(m) != 1
+    a64, w64 = a[rest].astype(np.float64), w.astype(np.float64)
+    assert (np.abs(got[rest] - a64 @ w64.T) <= (k + 8) * EPS * (np.abs(a64) @ np.abs(w64).T)).all()
