@@ -178,7 +178,8 @@ cudaError_t launch_squeeze_excite(const SqueezeExciteParams& p, cudaStream_t st)
   // as 16 clusters of two 19 to 26 us, as 8 clusters of four 12 to 21.
   const int per_wave = cluster_slots(kCluster);
   if (p.n <= per_wave) return launch_g<1>(p, st);
-  return p.n <= 2 * per_wave ? launch_g<2>(p, st) : launch_g<4>(p, st);
+  if (p.n <= 2 * per_wave) return launch_g<2>(p, st);
+  return p.n <= 3 * per_wave ? launch_g<3>(p, st) : launch_g<4>(p, st);
 }
 
 }  // namespace ac

@@ -243,3 +243,7 @@ def test_product_of_eight_rows_in_parts_of_k(cuda_lib, m, k, n):
     rest = np.arange(m) != 1
     a64, w64 = a[rest].astype(np.float64), w.astype(np.float64)
     assert (np.abs(got[rest] - a64 @ w64.T) <= (k + 8) * EPS * (np.abs(a64) @ np.abs(w64).T)).all()
+
+
+def test_squeeze_excite_block_with_four_images_a_cluster(cuda_lib):
+    test_squeeze_excite_block(cuda_lib, 47, 36, 5, 4)   # 31 to 45 images are three a cluster
