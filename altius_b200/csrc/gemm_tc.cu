@@ -1096,6 +1096,13 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
   auto b_hi = [&](int s) { return smem + s * L::kStageBytes + L::kOffBHi; };
   auto b_lo = [&](int s) { return smem + s * L::kStageBytes + L::kOffBLo; };
 
+  auto load_b = [&](int i, int kb, int tn) {    // PRE: this CTA's half of B's K-block kb into entry i
+    uint8_t* e = entry(i);
+    const uint32_t rdy = map_to_cta(&ready[(i >> 1) % kFlight], 0);
+    tma_load_3d_pair(e, &tm_b, rdy, kb * KB, tn * BN + (int)rank * (BN / 2), 0);
+    tma_load_3d_pair(e + L::kBBytes, &tm_blo, rdy, kb * KB, tn * BN + (int)rank * (BN / 2), 0);
+  };
+
   if (threadIdx.x == 0) {
     for (int s = 0; s < SM; ++s) {
       mbar_init(&full[s], 1);
@@ -1119,6 +1126,19 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
   cluster_sync_all();                    // barriers of both CTAs initialised before any remote arrival
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // The first K-blocks' part of B, a constant, is requested ahead of the wait for the kernel in front (ViT-B/16 at 96
+  // images 9690 -> 9585 us).
+  int early = 0;
+  if (PRE && warp == kTmaWarp && lane == 0) {
+    TcWork wk;
+    if (pair_get_work(sc, 0, &wk)) early = min(min(3, S / 2), wk.k1 - wk.k0);
+    for (int q = 0; q < early; ++q) {
+      if (leader) mbar_arrive_expect_tx(&ready[q], 2 * L::kTxBytes);
+      load_b(2 * q + 1, wk.k0 + q, wk.tile % tiles_n);
+    }
+    prefetch_map(&tm_a);
+    prefetch_map(&tm_alo);
+  }
   pdl_trigger();                         // behind the allocation: the next kernel's cannot come first
   pdl_wait();
   if (threadIdx.x == 0) pair_stamp(dbg, 1);
@@ -1142,14 +1162,14 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
             for (int op = 0; op < 2; ++op, ++it) {
               const int last = SUM ? (it >> 1) - kFlight : (it - S) >> 1;
               if (it >= (SUM ? 2 * kFlight : S) && !pwait(&empty[last % kFlight], (last / kFlight) & 1)) { atomicExch(err, 1); *abort_flag = 1; ok = false; break; }
-              if (leader && op == 0) mbar_arrive_expect_tx(&ready[q], 2 * L::kTxBytes);
+              const bool asked = it < 2 * early;             // ahead of the wait
+              if (leader && op == 0 && !asked) mbar_arrive_expect_tx(&ready[q], 2 * L::kTxBytes);
               uint8_t* e = entry(it);
               if (op == 0) {
                 tma_load_3d_pair(e, &tm_a, rdy, kb * KB, m0, 0);
                 tma_load_3d_pair(e + L::kABytes, &tm_alo, rdy, kb * KB, m0, 0);
-              } else {
-                tma_load_3d_pair(e, &tm_b, rdy, kb * KB, tn * BN + (int)rank * (BN / 2), 0);
-                tma_load_3d_pair(e + L::kBBytes, &tm_blo, rdy, kb * KB, tn * BN + (int)rank * (BN / 2), 0);
+              } else if (!asked) {
+                load_b(it, kb, tn);
               }
             }
           }

@@ -101,6 +101,10 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
+// A kernel's first load through a map waits for the map itself: it is asked for ahead of the wait for the kernel in front.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x,
                                             int y, int z) {
   asm volatile(
