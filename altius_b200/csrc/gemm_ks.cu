@@ -342,10 +342,7 @@ namespace {
 // Tile width and K split by clocks, from stamps in the kernel: a K-block costs its twelve MMAs (45 to 65 clocks
 // each) or its bytes at 60 a clock, whichever is more; first loads and drain 2700; exchange 1600 and 18
 // per column; epilogue 1500 and 40 per column that a block finishes. A launch as timed takes 1.4 to 2 times as long
-// (launch, cold code; operands arrive at 34 bytes a clock when all SMs load at once), the pair kernel 1.2 to 1.6 times
-// its clocks, so the comparison errs towards this kernel where both are close and K is long: the second product of
-// an MLP of 1182 to 2885 x 768 takes 4 us less to 6 more of 45, of 3152 x 768 and 12672 x 384 9 more of 67 (error
-// against 64 bits 1.2e-5 -> 2.4e-6 and 5.3e-6 -> 1.3e-6, so the choice stays); elsewhere it is the faster one.
+// (launch, cold code; operands arrive at 34 bytes a clock when all SMs load at once).
 Shape pick_shape(int64_t m, int64_t n, int64_t k) {
   Shape best;
   const int nkb = (int)((k + KB - 1) / KB);

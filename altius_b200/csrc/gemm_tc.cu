@@ -1832,9 +1832,10 @@ bool gemm_tc_wants_presplit(int64_t m, int64_t n, int64_t k, int64_t batch) {
   return pick_shape(m, n, k, batch, 2, 2).pair;
 }
 
-// A K-block of a 256 x 256 tile takes 1950 clocks, launch, first operands and last epilogue 20000, the
-// K-slice pass behind it 9000. (Products of 197 to 12672 rows against 384 to 768 x 384 to 2304 take 1.2 to 1.6 times
-// that: an epilogue of 11000 a tile runs only partly under the next tile's products.)
+// What the choice between this kernel and the more exact ones (gemm_ks_clocks) counts: 1950 clocks a K-block of a
+// 256 x 256 tile, 20000 for launch, first operands and last epilogue, 9000 for the K-slice pass. These are the figures of an
+// epilogue through shared memory; the kernel takes 1540, 18000 and 7500 now. They stay, because with those products
+// would move from errors of 2e-7 to 1e-6 for a few us (2885 x 768 x 768, 1576 x 512 x 512).
 double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k) {
   const int pairs = pair_count();
   if (pairs <= 0) return 1e30;
