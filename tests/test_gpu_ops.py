@@ -77,6 +77,15 @@ def test_unary_bit_exact(cuda_lib, op, attrs, shape):
     assert_bit_exact(got[0], want[0])
 
 
+def test_gelu_over_all_magnitudes(cuda_lib):
+    # The vectorised kernel divides by an estimate and its residual; every 1021st float, both signs, NaN and infinity.
+    x = np.arange(0, 1 << 32, 1021, dtype=np.uint64).astype(np.uint32).view(np.float32)
+    x = np.append(x[: x.size // 4 * 4 - 4], np.float32([np.inf, -np.inf, np.nan, 3.4e38]))
+    with np.errstate(all="ignore"):
+        got, want = both(single_op_model("Gelu", [x]), [x])
+    assert_bit_exact(got[0], want[0])
+
+
 def test_erf_unpinned_tolerance(cuda_lib):
     # The reference's Erf lives in an un-vendored crate and is tested to atol 1e-1 only.
     x = RNG.standard_normal((3, 1, 28, 28)).astype(np.float32)
