@@ -367,19 +367,17 @@ __device__ __forceinline__ void epilogue_raw(float* ws_tile, float4* stage, uint
 }
 
 // Four results as fp16 halves (n is a multiple of 8 then: the four columns exist together).
-__device__ __forceinline__ void fixup_split(const TcEpilogue& ep, int row, int col0, float4 y) {
+__device__ __forceinline__ void store_halves(const TcEpilogue& ep, int row, int col0, float4 y) {
   uint2 h, l;
   f16_split_fixed(y, h, l);
   const long long o = ((long long)row * ep.ldc16 + col0) >> 2;
   ep.c16_hi[o] = h;
   ep.c16_lo[o] = l;
-  // A tile's few K-sliced elements say nothing about the tensor being tiny: overflow only.
-  if (split_seen_fixed(y) & 1u) atomicCAS(ep.err, 0, kRangeCode);
 }
 
-// The epilogue of four consecutive elements of row `row` from column `col0` on (n % 4 == 0 when
-// the split result is written): what the tail fix-up applies to the summed K-slices.
-__device__ __forceinline__ void fixup_apply(const TcEpilogue& ep, int row, int col0, int bz, float4 acc) {
+// Any epilogue of four consecutive elements of row `row` from column `col0` on (n % 4 == 0 when the split
+// result is written); returns them, so that the caller can report the range of what was split.
+__device__ __forceinline__ float4 apply_any(const TcEpilogue& ep, int row, int col0, int bz, float4 acc) {
   float* c = ep.c ? ep.c + (long long)bz * ep.sc : nullptr;
   const float* cin = (ep.cin && ep.beta != 0.f) ? ep.cin + (long long)bz * ep.scin : nullptr;
   const float* res = ep.res ? ep.res + (long long)bz * ep.sres : nullptr;
@@ -407,7 +405,9 @@ __device__ __forceinline__ void fixup_apply(const TcEpilogue& ep, int row, int c
     if (c) c[(long long)row * ep.ldc + col] = y;
     y4[e] = y;
   }
-  if (ep.c16_hi) fixup_split(ep, row, col0, make_float4(y4[0], y4[1], y4[2], y4[3]));
+  const float4 y = make_float4(y4[0], y4[1], y4[2], y4[3]);
+  if (ep.c16_hi) store_halves(ep, row, col0, y);
+  return y;
 }
 
 // The epilogue of the pair kernel that takes A pre-split: sixteen warps, a warp per tensor-memory lane
@@ -509,10 +509,11 @@ __device__ __forceinline__ unsigned epilogue_regs(const TcEpilogue& ep, uint32_t
 
 // The same walk for what the common epilogues do not cover: the unreduced accumulator of a K-slice into its
 // workspace tile [128][ld] (ws), or any epilogue, element by element.
-__device__ __noinline__ void epilogue_regs_other(const TcEpilogue& ep, float* ws, int ld, int groups, uint32_t acc, int q, int lane, int m0,
+__device__ __noinline__ unsigned epilogue_regs_other(const TcEpilogue& ep, float* ws, int ld, int groups, uint32_t acc, int q, int lane, int m0,
                                                  int n0, int cg, uint32_t acc_empty_leader) {
   const float sc = acc_scale_of(ep);
   const int odd = lane & 1, high = (lane >> 1) & 1;
+  float seen_max = 0.f;                             // largest magnitude written as fixed-scale halves
 #pragma unroll 1
   for (int b = 0; b < 2 * groups; ++b) {
     uint32_t u[8];
@@ -526,9 +527,13 @@ __device__ __noinline__ void epilogue_regs_other(const TcEpilogue& ep, float* ws
       x.x = __fmul_rn(x.x, sc); x.y = __fmul_rn(x.y, sc); x.z = __fmul_rn(x.z, sc); x.w = __fmul_rn(x.w, sc);
       const int row = q * 32 + 16 * (b & 1) + 8 * h + (lane >> 2), col = 16 * (b >> 1) + 8 * odd + 4 * high;
       if (ws) *reinterpret_cast<float4*>(ws + (size_t)row * ld + cg + col) = x;
-      else if (m0 + row < ep.m && n0 + col < ep.n) fixup_apply(ep, m0 + row, n0 + col, 0, x);
+      else if (m0 + row < ep.m && n0 + col < ep.n) {
+        x = apply_any(ep, m0 + row, n0 + col, 0, x);
+        if (ep.c16_hi) seen_max = split_track(seen_max, x);
+      }
     }
   }
+  return split_seen_fixed_of_max(seen_max);
 }
 
 // Adds the K-slices of the tail tiles and applies the epilogue. What bounds it is latency (a tile of 256 x 256 in 24 slices is
@@ -578,8 +583,12 @@ __global__ void __maxnreg__(64) gemm_tc_fixup_kernel(const float* ws, const __gr
     acc.z = __fadd_rn(acc.z, __shfl_xor_sync(0xffffffffu, acc.z, o)); acc.w = __fadd_rn(acc.w, __shfl_xor_sync(0xffffffffu, acc.w, o));
   }
   if (!mine) return;
+  // A tile's few K-sliced elements say nothing about the tensor being tiny: overflow only.
+  auto report = [&](float4 y) {
+    if (ep.c16_hi && (split_seen_fixed(y) & 1u)) atomicCAS(ep.err, 0, kRangeCode);
+  };
   if (!common) {
-    fixup_apply(ep, row, col0, bz, acc);
+    report(apply_any(ep, row, col0, bz, acc));
     return;
   }
   if (ep.bias_n) acc = make_float4(__fadd_rn(acc.x, b.x), __fadd_rn(acc.y, b.y), __fadd_rn(acc.z, b.z), __fadd_rn(acc.w, b.w));
@@ -593,7 +602,8 @@ __global__ void __maxnreg__(64) gemm_tc_fixup_kernel(const float* ws, const __gr
   }
   if (ep.res) acc = make_float4(__fadd_rn(acc.x, r.x), __fadd_rn(acc.y, r.y), __fadd_rn(acc.z, r.z), __fadd_rn(acc.w, r.w));
   if (ep.c) *reinterpret_cast<float4*>(ep.c + (long long)bz * ep.sc + (long long)row * ep.ldc + col0) = acc;
-  if (ep.c16_hi) fixup_split(ep, row, col0, acc);
+  if (ep.c16_hi) store_halves(ep, row, col0, acc);
+  report(acc);
 }
 
 // Shared-memory stage of the main loop. MT = 128-row sub-tiles per CTA tile.
@@ -1416,11 +1426,11 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         const uint32_t part = acc + (uint32_t)cg;
         if (m0 >= ep.m) hand_back(acc_empty_leader, lane);
         else if (wk.raw >= 0)
-          epilogue_regs_other(ep, workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, BN, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
+          (void)epilogue_regs_other(ep, workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, BN, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
         else if (KEY >= 0)
           seen_out |= epilogue_regs<BN / 64, (KEY >= 0 ? KEY >> 2 : 0), KEY & 1, (KEY & 2) != 0>(ep, part, q, lane, m0, nw, acc_empty_leader);
         else
-          epilogue_regs_other(ep, nullptr, 0, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
+          seen_out |= epilogue_regs_other(ep, nullptr, 0, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
       } else if (m0 < ep.m) {
         if (wk.raw >= 0) {
           epilogue_raw<BN, D2>(workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, stage, acc, q, lane, cc0, cc1, acc_scale_of(ep));

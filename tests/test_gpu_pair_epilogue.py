@@ -106,3 +106,56 @@ def test_pairs_with_short_accumulators(cuda_lib, m, d, n, bound, act, res):
     want = y + _t(r) if res else y
     assert ((got - want).norm() / want.norm()).item() <= bound
     assert ((got - want).abs() <= 1e-5 * want.abs() + 2e-5).all()
+
+
+# ---- range of the halves a product writes for the next one --------------------------------------
+# Reported (and repeated on another plan): anything beyond 255, and a warp's part of a tile with nothing of 2^-11 or more.
+def _mlp(x, w1, w2, b1=None, act=None, r=None, norm=True):
+    g = ir.Graph()
+    h = g.add_input("x", x.shape)
+    ri = g.add_input("r", r.shape) if r is not None else None
+    if norm:
+        h = g.op("LayerNormalization", h, g.new_init(np.ones(x.shape[1], np.float32)), g.new_init(np.zeros(x.shape[1], np.float32)), axis=-1,
+                 epsilon=1e-6, stash_type=1)
+    h = g.op("MatMul", h, g.new_init(w1))
+    h = g.op("Add", h, g.new_init(b1)) if b1 is not None else h
+    h = g.op(act, h) if act else h
+    h = g.op("Add", h, ri) if r is not None else h
+    g.outputs.append(g.op("MatMul", h, g.new_init(w2)))
+    sess = CudaSessionBuilder(ir.Model(g, 13)).build()
+    try:
+        before = [e["kind"] for e in sess.schedule()]
+        got = torch.from_numpy(sess.run([x] + ([r] if r is not None else []))[0]).double().cuda()
+        after = [e["kind"] for e in sess.schedule()]
+    finally:
+        sess.close()
+    y = torch.nn.functional.layer_norm(_t(x), x.shape[1:], None, None, 1e-6) if norm else _t(x)
+    y = y @ _t(w1)
+    y = y + _t(b1) if b1 is not None else y
+    y = {None: lambda v: v, "ReLU": torch.relu, "Gelu": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[act](y)
+    y = y + _t(r) if r is not None else y
+    return got, y @ _t(w2), before, after
+
+
+def _weights(rng, d, h, n):
+    return ((rng.standard_normal((d, h)) / np.sqrt(d)).astype(np.float32), (rng.standard_normal((h, n)) / np.sqrt(h)).astype(np.float32))
+
+
+def _rel(got, want):
+    return ((got - want).norm() / want.norm()).item()
+
+
+# Short accumulators behind a LayerNormalization, tiles of 256 x 256 without one; the epilogues that are compiled in and those that are not.
+@pytest.mark.parametrize("m,d,h,n,norm", [(3152, 768, 768, 768, True), (1576, 384, 1536, 384, True), (6304, 384, 1536, 384, False)])
+@pytest.mark.parametrize("act,bias,res", [(None, True, False), ("ReLU", True, False), ("ReLU", False, False), ("Gelu", False, False),
+                                          ("ReLU", True, True), ("Gelu", True, True)])
+def test_tiny_results_are_reported(cuda_lib, m, d, h, n, norm, act, bias, res):
+    rng = np.random.default_rng(m + h)
+    w1, w2 = _weights(rng, d, h, n)
+    tiny = np.float32(1e-8)
+    b1 = tiny * rng.standard_normal(h).astype(np.float32) if bias else None
+    r = tiny * rng.standard_normal((m, h)).astype(np.float32) if res else None
+    x = rng.standard_normal((m, d)).astype(np.float32)
+    got, want, before, after = _mlp(x, tiny * w1, w2, b1, act, r, norm)
+    assert before != after
+    assert _rel(got, want) <= 3e-5                   # 3xTF32, of positive values: 1.3e-5; as halves 6e-3
