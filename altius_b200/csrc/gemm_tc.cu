@@ -366,6 +366,15 @@ __device__ __forceinline__ void epilogue_raw(float* ws_tile, float4* stage, uint
   }
 }
 
+// Verdict of a warp on the `count` elements of a tile that it split. By tile: its next one lies elsewhere and says nothing about
+// these. A corner of a few elements says nothing about them being tiny, either (of eight results behind ReLU one group in 256 is
+// without a large one), and counts with the warp's tile before it.
+__device__ __forceinline__ unsigned report_tile(unsigned seen, int count, unsigned before, int* err) {
+  if (count < 256) seen |= before;
+  split_report_warp(seen, err);
+  return seen;
+}
+
 // Four results as fp16 halves (n is a multiple of 8 then: the four columns exist together).
 __device__ __forceinline__ void store_halves(const TcEpilogue& ep, int row, int col0, float4 y) {
   uint2 h, l;
@@ -839,9 +848,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
       const int group = threadIdx.x / kSplitThreads;   // takes the K-blocks with it % kSplitGroups == group
       int it = 0;
       bool ok = true;
-      unsigned seen = 0;
+      unsigned seen_before = 0;
       TcWork wk;
       for (int w = 0; ok && tc_get_work(sc, w, &wk); ++w) {
+        unsigned seen = 0;
         for (int kb = wk.k0; kb < wk.k1; ++kb, ++it) {
           if (it % kSplitGroups != group) continue;
           const int s = it % S;
@@ -912,10 +922,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           __syncwarp();                        // one arrival per warp
           if (lane == 0) mbar_arrive(&ready[s]);
         }
+        // An element of A too large for fp16, or nothing but tiny ones in this warp's quarter of the rows: the result
+        // is not to be used (the host re-runs on the TF32 path); a code from a timed-out wait takes precedence.
+        if (MODE == TC_F16X3)
+          seen_before = report_tile(seen, min(32, ep.m - (wk.tile / tiles_n) % tiles_m * (MT * BM)) * (wk.k1 - wk.k0) * (KB / kSplitGroups), seen_before, err);
       }
-      // An element of A too large for fp16, or nothing but tiny ones: the result is not to be
-      // used (the host re-runs on the TF32 path); a code from a timed-out wait takes precedence.
-      if (MODE == TC_F16X3) split_report_warp(seen, err);
     }
   } else {
     // ---------------- epilogue ----------------
@@ -1297,9 +1308,10 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
     constexpr int kItems = BM * KB / 4 / kSplitThreads;   // 8
     int it = 0;
     bool ok = true;
-    unsigned seen = 0;
+    unsigned seen_before = 0;
     TcWork wk;
     for (int w = 0; ok && pair_get_work(sc, w, &wk); ++w) {
+      unsigned seen = 0;
       const int t = wk.tile;
       const int tm = (t / tiles_n) % tiles_m;
       const int m0 = tm * (2 * BM) + (int)rank * BM;
@@ -1337,8 +1349,8 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         __syncwarp();                               // one remote arrival per warp, not per thread
         if (lane == 0) mbar_arrive_cluster(map_to_cta(&ready[s], 0));
       }
+      seen_before = report_tile(seen, min(32, ep.m - m0) * (wk.k1 - wk.k0) * (KB / kSplitGroups), seen_before, err);
     }
-    split_report_warp(seen, err);
   } else if (!PRE || warp < 16) {
     // ---------------- epilogue (each CTA its own 128 rows) ----------------
     // PRE: warps 0-15, a warp per lane quarter and quarter of the columns, in registers; else eight warps, half of the
@@ -1349,7 +1361,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
     float4* stage = reinterpret_cast<float4*>(epi_smem + e * 4096);
     const int key = PRE ? KEY : epilogue_key(ep);
     int ti = 0;
-    unsigned seen_out = 0;   // what this warp has seen of the results it wrote split (ep.c16_hi)
+    unsigned seen_before = 0;   // verdict on the halves of this warp's tile before
     TcWork wk;
     for (int w = 0; pair_get_work(sc, w, &wk); ++w, ++ti) {
       const int t = wk.tile;
@@ -1424,13 +1436,15 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         }
         const int nw = n0 + cg;
         const uint32_t part = acc + (uint32_t)cg;
+        unsigned seen = 0;               // of this warp's part of the tile, as far as it was written as halves
         if (m0 >= ep.m) hand_back(acc_empty_leader, lane);
         else if (wk.raw >= 0)
           (void)epilogue_regs_other(ep, workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, BN, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
         else if (KEY >= 0)
-          seen_out |= epilogue_regs<BN / 64, (KEY >= 0 ? KEY >> 2 : 0), KEY & 1, (KEY & 2) != 0>(ep, part, q, lane, m0, nw, acc_empty_leader);
+          seen = epilogue_regs<BN / 64, (KEY >= 0 ? KEY >> 2 : 0), KEY & 1, (KEY & 2) != 0>(ep, part, q, lane, m0, nw, acc_empty_leader);
         else
-          seen_out |= epilogue_regs_other(ep, nullptr, 0, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
+          seen = epilogue_regs_other(ep, nullptr, 0, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
+        if (ep.c16_hi) seen_before = report_tile(seen, min(32, ep.m - m0 - q * 32) * min(BN / 4, ep.n - nw), seen_before, err);
       } else if (m0 < ep.m) {
         if (wk.raw >= 0) {
           epilogue_raw<BN, D2>(workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, stage, acc, q, lane, cc0, cc1, acc_scale_of(ep));
@@ -1452,7 +1466,6 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
       if (!PRE && !released) release();
       if (e == 0 && lane == 0 && ti < 3) pair_stamp(dbg, 9 + 2 * ti);     // this warp's part of tile ti stored
     }
-    if (PRE && ep.c16_hi) split_report_warp(seen_out, err);
   }
 
   // ---------------- teardown ----------------

@@ -159,3 +159,17 @@ def test_tiny_results_are_reported(cuda_lib, m, d, h, n, norm, act, bias, res):
     got, want, before, after = _mlp(x, tiny * w1, w2, b1, act, r, norm)
     assert before != after
     assert _rel(got, want) <= 3e-5                   # 3xTF32, of positive values: 1.3e-5; as halves 6e-3
+
+
+# One tile of tiny rows, whose warps have a tile of normal ones, too: its rows live on K positions where the weights are small.
+@pytest.mark.parametrize("m,d,h,n,norm", [(12672, 384, 384, 384, True), (12672, 384, 1536, 384, False)])
+def test_a_tile_of_tiny_results_is_reported(cuda_lib, m, d, h, n, norm):
+    rng = np.random.default_rng(m + h)
+    w1, w2 = _weights(rng, d, h, n)
+    w1[:d // 2] *= np.float32(1e-7)
+    x = rng.standard_normal((m, d)).astype(np.float32)
+    x[:256] = 0
+    x[:256, :d // 2] = rng.permuted(np.tile(np.float32([1, -1]), (256, d // 4)), axis=1)     # a mean of zero, whatever the order
+    got, want, before, after = _mlp(x, w1, w2, norm=norm)
+    assert before != after
+    assert _rel(got[:256], want[:256]) <= 3e-5       # as halves 7e-4
