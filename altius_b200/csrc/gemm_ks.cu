@@ -387,8 +387,9 @@ inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) =
 // 2.1e-7 at K = 768, 2.0e-7 at 576, 1.5e-7 at 384 and 512: one there.
 int pair_sums_run(const GemmParams& q, double clocks) {
   if (q.c16_hi && ((q.n % 8) || (q.ldc16 % 8) || !al16(q.c16_hi) || !al16(q.c16_lo))) return 0;
-  const int64_t nkb = (q.k + KB - 1) / KB, tiles = ((q.m + 255) / 256) * ((q.n + 191) / 192);
-  const int64_t rounds = (tiles + cluster_slots(2) - 1) / cluster_slots(2);
+  const int64_t pairs = gemm_tc_pairs();
+  if (pairs <= 0) return 0;
+  const int64_t nkb = (q.k + KB - 1) / KB, tiles = ((q.m + 255) / 256) * ((q.n + 191) / 192), rounds = (tiles + pairs - 1) / pairs;
   return 4000.0 + rounds * (1300.0 * nkb + 6000.0) < 0.97 * clocks ? (q.k > 576 ? 2 : 1) : 0;
 }
 

@@ -1,6 +1,10 @@
 """Epilogues of the CTA-pair GEMM against float64 at the edges of its tiles (256 x 256; blocks of 16 x 16 within): a
 row or a few columns beyond whole tiles, columns that are whole float4s but not whole groups of eight, K-sliced
 last tiles. The bound is the one of all fp16-split products: 1e-5 of the result and 5e-6 of sum |a||b|."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -106,6 +110,32 @@ def test_pairs_with_short_accumulators(cuda_lib, m, d, n, bound, act, res):
     want = y + _t(r) if res else y
     assert ((got - want).norm() / want.norm()).item() <= bound
     assert ((got - want).abs() <= 1e-5 * want.abs() + 2e-5).all()
+
+
+_NO_PAIRS = """
+import numpy as np
+from altius_b200 import ir
+from altius_b200.session import CudaSessionBuilder
+x = np.random.default_rng(0).standard_normal((3152, 768)).astype(np.float32)
+g = ir.Graph()
+h = g.op("LayerNormalization", g.add_input("x", x.shape), g.new_init(np.ones(768, np.float32)), g.new_init(np.zeros(768, np.float32)),
+         axis=-1, epsilon=1e-6, stash_type=1)
+g.outputs.append(g.op("MatMul", h, g.new_init(2 * np.eye(768, dtype=np.float32))))
+sess = CudaSessionBuilder(ir.Model(g, 13)).build()
+assert [e["kind"] for e in sess.schedule()] == ["layer_norm", "gemm_f16x3_cluster_tcgen05"]
+y = sess.run([x])[0].astype(np.float64)
+x = x.astype(np.float64)
+want = 2 * (x - x.mean(1, keepdims=True)) / np.sqrt(x.var(1, keepdims=True) + 1e-6)
+assert np.linalg.norm(y - want) <= 1e-6 * np.linalg.norm(want)
+"""
+
+
+def test_without_room_for_a_pair_the_few_row_kernel_stays(cuda_lib):
+    """One SM for the persistent kernels: no CTA pair fits, and the product is not handed to them."""
+    env = dict(os.environ, ALTIUS_CUDA_TC_SMS="1")
+    r = subprocess.run([sys.executable, "-c", _NO_PAIRS], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), env=env,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 # ---- range of the halves a product writes for the next one --------------------------------------
