@@ -282,8 +282,8 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
         tc_fence_after();
         uint32_t s[64];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tc_ld_32x16_nowait(scol + (uint32_t)(16 * c), *reinterpret_cast<uint32_t(*)[16]>(&s[16 * c]));
-        tc_wait_ld();
+        for (int c = 0; c < 4; ++c) tc_ld_32x16(scol + (uint32_t)(16 * c), *reinterpret_cast<uint32_t(*)[16]>(&s[16 * c]));
+        tc_wait_ld(s);
         float m = -CUDART_INF_F;
         if (left >= 64) {
           float m4[4] = {m, m, m, m};
@@ -311,9 +311,9 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
 #pragma unroll
           for (int part = 0; part < 2; ++part) {   // this warp's 32 columns
             uint32_t o[16], ol[16];
-            tc_ld_32x16_nowait(ocol + (uint32_t)(part * 16), o);
-            tc_ld_32x16_nowait(ocol + (uint32_t)(HD + part * 16), ol);
-            tc_wait_ld();
+            tc_ld_32x16(ocol + (uint32_t)(part * 16), o);
+            tc_ld_32x16(ocol + (uint32_t)(HD + part * 16), ol);
+            tc_wait_ld(o, ol);
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
               float* at = sums + (part * 16 + e) * QM;
@@ -333,8 +333,8 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
             for (int part = 0; part < 4; ++part) {   // this warp's 32 columns of both halves of O
               const uint32_t at = ocol + (uint32_t)((part >> 1) * 64 + (part & 1) * 16);
               uint32_t o[16];
-              tc_ld_32x16_nowait(at, o);
-              tc_wait_ld();
+              tc_ld_32x16(at, o);
+              tc_wait_ld(o);
 #pragma unroll
               for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__fmul_rn(__uint_as_float(o[e]), f));
               st16(at, o);
@@ -384,9 +384,9 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         uint32_t o[16], ol[16];
-        tc_ld_32x16_nowait(ocol + (uint32_t)(half * 16), o);
-        tc_ld_32x16_nowait(ocol + (uint32_t)(64 + half * 16), ol);
-        tc_wait_ld();
+        tc_ld_32x16(ocol + (uint32_t)(half * 16), o);
+        tc_ld_32x16(ocol + (uint32_t)(64 + half * 16), ol);
+        tc_wait_ld(o, ol);
         if (!ok || r >= T) continue;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {

@@ -93,31 +93,6 @@ __device__ __forceinline__ uint64_t desc_sw64(uint32_t saddr) {
   return d;
 }
 
-// The load alone: several may be in flight before one tc_ld_wait().
-__device__ __forceinline__ void tc_ld_32x16_issue(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-        "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-        "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -369,9 +344,9 @@ __global__ void __launch_bounds__(kAtLaunch, 1) attention_tc_kernel(AttnTcDev p)
       for (int i = 0; i < b_count; ++i) {
         const int c0 = (b_begin + i) * 32;       // 32 columns per step; columns past NS read junk that is masked
         uint32_t v[2][16];
-        tc_ld_32x16_issue(trow + (uint32_t)c0, v[0]);
-        tc_ld_32x16_issue(trow + (uint32_t)(c0 + 16), v[1]);
-        tc_ld_wait();
+        tc_ld_32x16(trow + (uint32_t)c0, v[0]);
+        tc_ld_32x16(trow + (uint32_t)(c0 + 16), v[1]);
+        tc_wait_ld(v[0], v[1]);
         // Columns past T (exact zeros up to NS, junk beyond) are kept out of the maximum
         // by a select, not a branch, so that the chains stay interleaved.
         float m0 = CUDART_NAN_F, m1 = CUDART_NAN_F;
@@ -403,6 +378,7 @@ __global__ void __launch_bounds__(kAtLaunch, 1) attention_tc_kernel(AttnTcDev p)
           const int c0 = blk * 32 + h16 * 16;
           uint32_t v[16];
           tc_ld_32x16(trow + (uint32_t)c0, v);
+          tc_wait_ld(v);
           float e[16];
 #pragma unroll
           for (int u = 0; u < 16; ++u) {
@@ -446,6 +422,7 @@ __global__ void __launch_bounds__(kAtLaunch, 1) attention_tc_kernel(AttnTcDev p)
       uint32_t o[32], o2[32];
       tc_ld_32x32(trow + kOCol + (uint32_t)(hf * 32), o);
       tc_ld_32x32(trow + kOCol + (uint32_t)(HD + hf * 32), o2);
+      tc_wait_ld(o, o2);
       float4* stage = reinterpret_cast<float4*>(qp + warp * 4096);
       auto fin = [&](int j) {
         const float y = fmaf(__uint_as_float(o2[j]), kLoUnscale, __uint_as_float(o[j]));

@@ -76,16 +76,6 @@ __device__ __forceinline__ uint64_t desc_mn128(uint32_t saddr) {
   d |= (uint64_t)2 << 61;
   return d;
 }
-__device__ __forceinline__ void ld16_issue(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-        "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-}
 
 // The three partial products of one 16-key chunk (lo * hi, hi * lo, hi * hi) in one statement:
 // tcgen05.mma with the A operand in tensor memory (row r of A in lane r, 16 fp16 values of K in
@@ -341,9 +331,9 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
       for (int ci = 0; ci < c_count; ci += 2) {
         const int c0 = (c_begin + ci) * 16;
         uint32_t v[2][16];
-        ld16_issue(srow + (uint32_t)c0, v[0]);
-        ld16_issue(srow + (uint32_t)(c0 + 16), v[1]);
-        tc_wait_ld();
+        tc_ld_32x16(srow + (uint32_t)c0, v[0]);
+        tc_ld_32x16(srow + (uint32_t)(c0 + 16), v[1]);
+        tc_wait_ld(v[0], v[1]);
         float m0 = CUDART_NAN_F, m1 = CUDART_NAN_F;
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
@@ -366,8 +356,8 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
       for (int ci = 0; ci < c_count; ++ci) {
         const int c0 = (c_begin + ci) * 16;
         uint32_t v[16];
-        ld16_issue(srow + (uint32_t)c0, v);
-        tc_wait_ld();
+        tc_ld_32x16(srow + (uint32_t)c0, v);
+        tc_wait_ld(v);
         float e[16];
 #pragma unroll
         for (int x = 0; x < 16; ++x) {
@@ -403,6 +393,7 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
       AT16_STAMP(4);
       uint32_t o[32];
       tc_ld_32x32(trow + kOCol + (uint32_t)(hf * 32), o);
+      tc_wait_ld(o);
       tc_fence_before();
       __syncwarp();
       if (ok && lane == 0) mbar_arrive(&o_free[g]);

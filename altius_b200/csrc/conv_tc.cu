@@ -285,11 +285,11 @@ __global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
       const uint32_t base = tmem + (i & two) * span + ((uint32_t)((warp & 3) * 32) << 16);
       for (int c = (warp >> 2) * 16; c < bn && c <= mlast; c += 32) {
         uint32_t u[16];
-        tc_ld_32x16_nowait(base + (uint32_t)c + (mains ? set : 0u), u);
+        tc_ld_32x16(base + (uint32_t)c + (mains ? set : 0u), u);
         auto add = [&](uint32_t from) {          // u += an accumulator, once both are there
           uint32_t more[16];
-          tc_ld_32x16_nowait(base + (uint32_t)c + from, more);
-          tc_wait_ld();
+          tc_ld_32x16(base + (uint32_t)c + from, more);
+          tc_wait_ld(u, more);
 #pragma unroll
           for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(__fadd_rn(__uint_as_float(u[j]), __uint_as_float(more[j])));
         };
@@ -297,7 +297,7 @@ __global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
           // To the block that finishes these channels; no one waits for a remote load.
           if (mains > 1) add(2 * set);
           if (mains) add(0u);
-          tc_wait_ld();
+          else tc_wait_ld(u);
           int owner = c / share, left = share - c % share;
           for (int j = 0; j < 16;) {           // uniform: channels per owner are a multiple of two
             float* dst = cl.map_shared_rank(part, owner) + ((int)blockIdx.z * share + (share - left)) * PX + row;
@@ -318,7 +318,7 @@ __global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
         }
         if (mains > 1) add(2 * set);
         if (mains) add(0u);
-        tc_wait_ld();
+        else tc_wait_ld(u);
         float y[16];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {

@@ -250,16 +250,19 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 16; ++i) a[i] = __float_as_uint(__fadd_rn(__uint_as_float(a[i]), __uint_as_float(b[i])));
         };
-        tc_ld_32x16_nowait(at + (uint32_t)bn, u);
+        tc_ld_32x16(at + (uint32_t)bn, u);
         for (int a = 2; a <= mains; a += 2) {       // two accumulators on their way at once, added in order
-          tc_ld_32x16_nowait(at + (uint32_t)(a * bn), x);
-          if (a < mains) tc_ld_32x16_nowait(at + (uint32_t)((a + 1) * bn), y);
-          tc_wait_ld();
+          tc_ld_32x16(at + (uint32_t)(a * bn), x);
+          if (a < mains) tc_ld_32x16(at + (uint32_t)((a + 1) * bn), y);
+          tc_wait_ld(u, x);
           plus(u, x);
-          if (a < mains) plus(u, y);
+          if (a < mains) {
+            tc_landed(y);
+            plus(u, y);
+          }
         }
-        tc_ld_32x16_nowait(at, x);
-        tc_wait_ld();
+        tc_ld_32x16(at, x);
+        tc_wait_ld(u, x);
         plus(u, x);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {

@@ -139,16 +139,16 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr, uint32_t c
 // `sc`: power of two that undoes the scaling of a constant B (1 when there is none).
 template <int D2OFF>
 __device__ __forceinline__ void load_acc(uint32_t taddr, uint32_t (&v)[32], float sc) {
-  tc_ld_32x32_nowait(taddr, v);
+  tc_ld_32x32(taddr, v);
   if (D2OFF != 0) {
     uint32_t w[32];
-    tc_ld_32x32_nowait(taddr + (uint32_t)D2OFF, w);
-    tc_wait_ld();
+    tc_ld_32x32(taddr + (uint32_t)D2OFF, w);
+    tc_wait_ld(v, w);
 #pragma unroll
     for (int j = 0; j < 32; ++j)
       v[j] = __float_as_uint(__fmul_rn(fmaf(__uint_as_float(w[j]), kLoUnscale, __uint_as_float(v[j])), sc));
   } else {
-    tc_wait_ld();
+    tc_wait_ld(v);
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fmul_rn(__uint_as_float(v[j]), sc));   // sc is a power of two
   }
@@ -450,7 +450,7 @@ __device__ __forceinline__ unsigned epilogue_regs(const TcEpilogue& ep, uint32_t
   float4 nr[HAS_RES ? 2 : 1], nb = make_float4(0.f, 0.f, 0.f, 0.f);
   auto request = [&](int b) {
     const int rb = 16 * (b & 1), cb = 16 * (b >> 1);
-    tc_ld_16x256_x2_nowait(acc + ((uint32_t)(q * 32 + rb) << 16) + (uint32_t)cb, nx);
+    tc_ld_16x256_x2(acc + ((uint32_t)(q * 32 + rb) << 16) + (uint32_t)cb, nx);
     if (BIAS == 1 && rb == 0 && cb < cols) nb = ld_plain(reinterpret_cast<const float4*>(ep.bias_n + n0 + cl + cb));   // n % 4 == 0
     if (HAS_RES) {
 #pragma unroll
@@ -526,7 +526,7 @@ __device__ __noinline__ unsigned epilogue_regs_other(const TcEpilogue& ep, float
 #pragma unroll 1
   for (int b = 0; b < 2 * groups; ++b) {
     uint32_t u[8];
-    tc_ld_16x256_x2_nowait(acc + ((uint32_t)(q * 32 + 16 * (b & 1)) << 16) + (uint32_t)(16 * (b >> 1)), u);
+    tc_ld_16x256_x2(acc + ((uint32_t)(q * 32 + 16 * (b & 1)) << 16) + (uint32_t)(16 * (b >> 1)), u);
     tc_wait_ld(u);
     if (b + 1 == 2 * groups) hand_back(acc_empty_leader, lane);
 #pragma unroll
@@ -1411,15 +1411,15 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
             const bool last = first + sc.run >= wk.k1;
             const uint32_t from = acc + (uint32_t)cg + ((uint32_t)(q * 32) << 16);
             uint32_t u[2][16];
-            tc_ld_32x16_nowait(from, u[0]);
-            tc_ld_32x16_nowait(from + 16u, u[1]);
-            tc_wait_ld();
+            tc_ld_32x16(from, u[0]);
+            tc_ld_32x16(from + 16u, u[1]);
+            tc_wait_ld(u[0], u[1]);
 #pragma unroll
             for (int c = 0; c < NS; ++c) {            // two loads under way ahead of the sums
 #pragma unroll
               for (int j = 0; j < 16; ++j) sums[16 * c + j] = __fadd_rn(sums[16 * c + j], __uint_as_float(u[c & 1][j]));
-              if (c + 2 < NS) tc_ld_32x16_nowait(from + (uint32_t)(16 * (c + 2)), u[c & 1]);
-              if (c >= 1 && c + 1 < NS) tc_wait_ld();
+              if (c + 2 < NS) tc_ld_32x16(from + (uint32_t)(16 * (c + 2)), u[c & 1]);
+              if (c >= 1 && c + 1 < NS) tc_wait_ld(u[(c + 1) & 1]);
             }
             if (last) {
 #pragma unroll

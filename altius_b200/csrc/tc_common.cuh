@@ -155,6 +155,20 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uin
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Loads from tensor memory only start here: several may be under way before one tc_wait_ld. The registers are
+// outputs of the load for the compiler, so the wait takes them as operands: no use of them moves ahead of it.
+template <int N>
+__device__ __forceinline__ void tc_landed(uint32_t (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(v[i]));
+}
+template <int N, typename... More>
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&v)[N], More&... more) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  tc_landed(v);
+  (tc_landed(more), ...);
+}
+// 32 columns of the warp's 32 lanes.
 __device__ __forceinline__ void tc_ld_32x32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -167,26 +181,9 @@ __device__ __forceinline__ void tc_ld_32x32(uint32_t taddr, uint32_t (&v)[32]) {
         "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(taddr)
       : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-
-// The same load without the wait: several loads can be in flight before one tc_wait_ld().
-__device__ __forceinline__ void tc_ld_32x32_nowait(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-        "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
-        "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
-        "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// Sixteen columns of the warp's 32 lanes, without the wait.
-__device__ __forceinline__ void tc_ld_32x16_nowait(uint32_t taddr, uint32_t (&v)[16]) {
+// Sixteen columns of the warp's 32 lanes.
+__device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -198,18 +195,11 @@ __device__ __forceinline__ void tc_ld_32x16_nowait(uint32_t taddr, uint32_t (&v)
 }
 
 // 16 lanes (from a lane of the warp's quarter that is a multiple of 16) x 16 columns: registers 4 j .. 4 j + 3 of
-// a lane are columns 8 j + 2 (lane % 4), + 1 of row lane / 4 and of row lane / 4 + 8. Without the wait.
-__device__ __forceinline__ void tc_ld_16x256_x2_nowait(uint32_t taddr, uint32_t (&v)[8]) {
+// a lane are columns 8 j + 2 (lane % 4), + 1 of row lane / 4 and of row lane / 4 + 8.
+__device__ __forceinline__ void tc_ld_16x256_x2(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "r"(taddr)
-               : "memory");
-}
-// The wait, with the registers that the loads in front fill: no use of them moves ahead of it.
-__device__ __forceinline__ void tc_wait_ld(uint32_t (&v)[8]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
-               :
                : "memory");
 }
 // Sixteen columns of the warp's 32 lanes, back to tensor memory.
