@@ -235,7 +235,7 @@ __global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
         if (gcol) apply_gate(kb, gcol, v);
         const int s = g % S;
         if (g >= S) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((g / S) & 1) ^ 1))) { atomicExch(p.err, 31); abort_flag = 1; alive = false; return; }
+          if (!mbar_wait_all(&empty[s], ((g / S) & 1) ^ 1)) { atomicExch(p.err, 31); abort_flag = 1; alive = false; return; }
           if (tid == 0 && !p.resident) load_filter(g);
         }
         uint8_t* hi_t = smem + s * stage_bytes;
@@ -279,7 +279,7 @@ __global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
       const bool col_ok = col < p.n;
       const int cc = min(col, p.n - 1), cb = cc / p.hw;
       const long long at = cb * p.out_batch + (cc - cb * p.hw) + (long long)m0 * p.hw;
-      if (!mbar_wait(&acc_full[i & two], (i >> two) & 1)) { atomicExch(p.err, 33); abort_flag = 1; break; }
+      if (!mbar_wait_all(&acc_full[i & two], (i >> two) & 1)) { atomicExch(p.err, 33); abort_flag = 1; break; }
       tc_fence_after();
       const int share = bn / parts;
       const uint32_t base = tmem + (i & two) * span + ((uint32_t)((warp & 3) * 32) << 16);

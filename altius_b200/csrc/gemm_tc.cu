@@ -856,7 +856,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           if (it % kSplitGroups != group) continue;
           const int s = it % S;
           const uint32_t ph = (it / S) & 1;
-          ok = __all_sync(0xffffffffu, mbar_wait(&full[s], ph));
+          ok = mbar_wait_all(&full[s], ph);
           if (MODE != TC_F16X3 && !ok) { atomicExch(err, 3); *abort_flag = 1; break; }
           if (MODE == TC_F16X3) {
             // fp32 rows of 32 floats -> fp16 hi / lo tiles; one float4 (4 consecutive k) per item.
@@ -940,7 +940,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
       const int t = wk.tile;
       const int tn = t % tiles_n, tm = (t / tiles_n) % tiles_m, bz = t / (tiles_n * tiles_m);
       const int ab = ti % NACC;
-      if (!mbar_wait(&acc_full[ab], (ti / NACC) & 1)) { atomicExch(err, 4); *abort_flag = 1; break; }
+      if (!mbar_wait_all(&acc_full[ab], (ti / NACC) & 1)) { atomicExch(err, 4); *abort_flag = 1; break; }
       tc_fence_after();
       // Every tcgen05.ld of this warp has completed (each is followed by wait::ld) when the
       // accumulator is handed back to the MMA warp.
@@ -1329,7 +1329,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
                      ? ld_plain(reinterpret_cast<const float4*>(a_tile + (long long)r * lda + kcol))
                      : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        ok = mbar_wait(&empty[s], ph ^ 1);          // the pair's MMAs on the previous use of the stage are done
+        ok = mbar_wait_all(&empty[s], ph ^ 1);      // the pair's MMAs on the previous use of the stage are done
         if (!ok) { atomicExch(err, 3); *abort_flag = 1; break; }
         uint8_t* hi_t = a_raw(s);
         uint8_t* lo_t = a_lo(s);
@@ -1344,7 +1344,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
           *reinterpret_cast<uint2*>(lo_t + off) = lo;
         }
         fence_proxy_async();
-        ok = mbar_wait(&full[s], ph);               // this CTA's half of B has landed too
+        ok = mbar_wait_all(&full[s], ph);           // this CTA's half of B has landed too
         if (!ok) { atomicExch(err, 3); *abort_flag = 1; break; }
         __syncwarp();                               // one remote arrival per warp, not per thread
         if (lane == 0) mbar_arrive_cluster(map_to_cta(&ready[s], 0));
@@ -1373,7 +1373,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         const int set = two_sets ? (ti & 1) : 0, use = two_sets ? (ti >> 1) : ti;
         acc = tmem_base + (uint32_t)(set * L::kSetCols);
         acc_empty_leader = map_to_cta(&acc_empty[set], 0);
-        const bool there = mbar_wait(&acc_full[set], use & 1);
+        const bool there = mbar_wait_all(&acc_full[set], use & 1);
         tc_fence_after();
         return there;
       };

@@ -72,6 +72,8 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity) {
   }
   return false;
 }
+// A whole warp waits, every lane polls: one verdict, so that no lane leaves ahead of the warp's next .sync instruction.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
 // A whole warp waits on an mbarrier phase: one lane polls (fewer probes of shared memory
 // while the tensor core fetches its operands from it), the others get the result by shuffle.
 __device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, int lane) {
