@@ -384,39 +384,66 @@ __device__ __forceinline__ void store_halves(const TcEpilogue& ep, int row, int 
   ep.c16_lo[o] = l;
 }
 
-// Any epilogue of four consecutive elements of row `row` from column `col0` on (n % 4 == 0 when the split
-// result is written); returns them, so that the caller can report the range of what was split.
-__device__ __forceinline__ float4 apply_any(const TcEpilogue& ep, int row, int col0, int bz, float4 acc) {
-  float* c = ep.c ? ep.c + (long long)bz * ep.sc : nullptr;
-  const float* cin = (ep.cin && ep.beta != 0.f) ? ep.cin + (long long)bz * ep.scin : nullptr;
-  const float* res = ep.res ? ep.res + (long long)bz * ep.sres : nullptr;
-  const float x[4] = {acc.x, acc.y, acc.z, acc.w};
-  float y4[4] = {0.f, 0.f, 0.f, 0.f};
+// Any epilogue of four consecutive elements of row `row` from column `col0` on (n % 4 == 0 when the split result is
+// written): its operands, so that several can be under way at once, then the arithmetic and the stores. It returns the
+// results, so that the caller can report the range of what was split. vec: float4s (epilogue_vec), else element by element.
+__device__ __forceinline__ bool epilogue_vec(const TcEpilogue& ep) {
+  auto al = [](const void* p, long long ld, long long stride) {
+    return !p || ((reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ld % 4) == 0 && (stride % 4) == 0);
+  };
+  return (ep.n % 4) == 0 && al(ep.c, ep.ldc, ep.sc) && al(ep.cin, ep.ldcin, ep.scin) && al(ep.res, ep.ldres, ep.sres) && al(ep.bias_n, 0, 0);
+}
+struct AnyOperands { float cin[4], bias[4], res[4], bias_m; };
+__device__ __forceinline__ AnyOperands fetch_any(const TcEpilogue& ep, int row, int col0, int bz, bool vec) {
+  AnyOperands o;
+  auto four = [&](const float* p, float (&v)[4]) {
+    if (vec) {
+      const float4 t = p ? ld_plain(reinterpret_cast<const float4*>(p + col0)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = p && col0 + e < ep.n ? ld_plain(p + col0 + e) : 0.f;
+    }
+  };
+  four(ep.cin && ep.beta != 0.f ? ep.cin + (long long)bz * ep.scin + (long long)row * ep.ldcin : nullptr, o.cin);
+  four(ep.bias_n, o.bias);
+  four(ep.res ? ep.res + (long long)bz * ep.sres + (long long)row * ep.ldres : nullptr, o.res);
+  o.bias_m = ep.bias_m ? ld_plain(ep.bias_m + row) : 0.f;
+  return o;
+}
+__device__ __forceinline__ float4 apply_any(const TcEpilogue& ep, int row, int col0, int bz, float4 acc, bool vec, const AnyOperands& o) {
+  float y[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
   for (int e = 0; e < 4; ++e) {
-    const int col = col0 + e;
-    if (col >= ep.n) break;
-    float y = x[e];
-    if (ep.alpha != 1.f) y = __fmul_rn(ep.alpha, y);
-    if (cin) {
-      const float cv = ld_plain(cin + (long long)row * ep.ldcin + col);
-      y = __fadd_rn(ep.beta == 1.f ? cv : __fmul_rn(ep.beta, cv), y);
-    }
-    if (ep.bias_n) {
-      const float bv = ld_plain(ep.bias_n + col);
-      y = __fadd_rn(y, ep.bias_scale == 1.f ? bv : __fmul_rn(ep.bias_scale, bv));
-    }
-    if (ep.bias_m) {
-      const float bv = ld_plain(ep.bias_m + row);
-      y = __fadd_rn(y, ep.bias_scale == 1.f ? bv : __fmul_rn(ep.bias_scale, bv));
-    }
-    y = apply_act(ep.act, y, ep.act_alpha, ep.act_beta);
-    if (res) y = __fadd_rn(y, ld_plain(res + (long long)row * ep.ldres + col));
-    if (c) c[(long long)row * ep.ldc + col] = y;
-    y4[e] = y;
+    if (ep.alpha != 1.f) y[e] = __fmul_rn(ep.alpha, y[e]);
+    if (ep.cin && ep.beta != 0.f) y[e] = __fadd_rn(ep.beta == 1.f ? o.cin[e] : __fmul_rn(ep.beta, o.cin[e]), y[e]);
+    if (ep.bias_n) y[e] = __fadd_rn(y[e], ep.bias_scale == 1.f ? o.bias[e] : __fmul_rn(ep.bias_scale, o.bias[e]));
+    if (ep.bias_m) y[e] = __fadd_rn(y[e], ep.bias_scale == 1.f ? o.bias_m : __fmul_rn(ep.bias_scale, o.bias_m));
   }
-  const float4 y = make_float4(y4[0], y4[1], y4[2], y4[3]);
-  if (ep.c16_hi) store_halves(ep, row, col0, y);
-  return y;
+  if (ep.act == ACT_GELU) {
+    const float2 g0 = gelu_ref2(make_float2(y[0], y[1])), g1 = gelu_ref2(make_float2(y[2], y[3]));
+    y[0] = g0.x; y[1] = g0.y; y[2] = g1.x; y[3] = g1.y;
+  } else if (ep.act != ACT_NONE) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[e] = apply_act(ep.act, y[e], ep.act_alpha, ep.act_beta);
+  }
+  if (ep.res) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[e] = __fadd_rn(y[e], o.res[e]);
+  }
+  const float4 r = make_float4(y[0], y[1], y[2], y[3]);
+  if (ep.c) {
+    float* c = ep.c + (long long)bz * ep.sc + (long long)row * ep.ldc + col0;
+    if (vec) {
+      *reinterpret_cast<float4*>(c) = r;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (col0 + e < ep.n) c[e] = y[e];
+    }
+  }
+  if (ep.c16_hi) store_halves(ep, row, col0, r);
+  return r;
 }
 
 // The epilogue of the pair kernel that takes A pre-split: sixteen warps, a warp per tensor-memory lane
@@ -516,13 +543,18 @@ __device__ __forceinline__ unsigned epilogue_regs(const TcEpilogue& ep, uint32_t
   return split_seen_fixed_of_max(seen_max);
 }
 
-// The same walk for what the common epilogues do not cover: the unreduced accumulator of a K-slice into its
-// workspace tile [128][ld] (ws), or any epilogue, element by element.
-__device__ __noinline__ unsigned epilogue_regs_other(const TcEpilogue& ep, float* ws, int ld, int groups, uint32_t acc, int q, int lane, int m0,
-                                                 int n0, int cg, uint32_t acc_empty_leader) {
+// Four neighbouring columns of row lane / 4 (h 0) or that + 8 (h 1) from a loaded 16 x 16 block, scaled.
+__device__ __forceinline__ float4 block_quad(const uint32_t (&u)[8], int h, int odd, float sc) {
+  const float4 x = quad_exchange(__uint_as_float(u[2 * h]), __uint_as_float(u[2 * h + 1]), __uint_as_float(u[4 + 2 * h]),
+                                 __uint_as_float(u[5 + 2 * h]), odd);
+  return make_float4(__fmul_rn(x.x, sc), __fmul_rn(x.y, sc), __fmul_rn(x.z, sc), __fmul_rn(x.w, sc));
+}
+
+// The same walk for the unreduced accumulator of a K-slice into its workspace tile [128][ld].
+__device__ __noinline__ void epilogue_regs_raw(const TcEpilogue& ep, float* ws, int ld, int groups, uint32_t acc, int q, int lane, int cg,
+                                               uint32_t acc_empty_leader) {
   const float sc = acc_scale_of(ep);
   const int odd = lane & 1, high = (lane >> 1) & 1;
-  float seen_max = 0.f;                             // largest magnitude written as fixed-scale halves
 #pragma unroll 1
   for (int b = 0; b < 2 * groups; ++b) {
     uint32_t u[8];
@@ -531,13 +563,38 @@ __device__ __noinline__ unsigned epilogue_regs_other(const TcEpilogue& ep, float
     if (b + 1 == 2 * groups) hand_back(acc_empty_leader, lane);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      float4 x = quad_exchange(__uint_as_float(u[2 * h]), __uint_as_float(u[2 * h + 1]), __uint_as_float(u[4 + 2 * h]),
-                               __uint_as_float(u[5 + 2 * h]), odd);
-      x.x = __fmul_rn(x.x, sc); x.y = __fmul_rn(x.y, sc); x.z = __fmul_rn(x.z, sc); x.w = __fmul_rn(x.w, sc);
-      const int row = q * 32 + 16 * (b & 1) + 8 * h + (lane >> 2), col = 16 * (b >> 1) + 8 * odd + 4 * high;
-      if (ws) *reinterpret_cast<float4*>(ws + (size_t)row * ld + cg + col) = x;
-      else if (m0 + row < ep.m && n0 + col < ep.n) {
-        x = apply_any(ep, m0 + row, n0 + col, 0, x);
+      const int row = q * 32 + 16 * (b & 1) + 8 * h + (lane >> 2), col = cg + 16 * (b >> 1) + 8 * odd + 4 * high;
+      *reinterpret_cast<float4*>(ws + (size_t)row * ld + col) = block_quad(u, h, odd, sc);
+    }
+  }
+}
+
+// And for any epilogue by its run-time options, float4s where everything is aligned, both rows' operands under way at once.
+// Inlined, so that the options are constants of the launch and not memory that every store may have changed (6304 x 768 x 2304
+// with HardSwish, with alpha, beta and a C matrix, and 2306 columns: element by element and not inlined 147, 214 and 166 us,
+// float4s 124, 138 and 155, inlined 87, 82 and 101).
+__device__ __forceinline__ unsigned epilogue_regs_any(const TcEpilogue& ep, int groups, uint32_t acc, int q, int lane, int m0, int n0,
+                                                   uint32_t acc_empty_leader) {
+  const float sc = acc_scale_of(ep);
+  const int odd = lane & 1, high = (lane >> 1) & 1;
+  const bool vec = epilogue_vec(ep);
+  float seen_max = 0.f;                             // largest magnitude written as fixed-scale halves
+#pragma unroll 1
+  for (int b = 0; b < 2 * groups; ++b) {
+    const int row = m0 + q * 32 + 16 * (b & 1) + (lane >> 2), col = n0 + 16 * (b >> 1) + 8 * odd + 4 * high;   // and row + 8
+    uint32_t u[8];
+    tc_ld_16x256_x2(acc + ((uint32_t)(q * 32 + 16 * (b & 1)) << 16) + (uint32_t)(16 * (b >> 1)), u);
+    AnyOperands o[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (col < ep.n && row + 8 * h < ep.m) o[h] = fetch_any(ep, row + 8 * h, col, 0, vec);
+    tc_wait_ld(u);
+    if (b + 1 == 2 * groups) hand_back(acc_empty_leader, lane);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float4 x = block_quad(u, h, odd, sc);
+      if (col < ep.n && row + 8 * h < ep.m) {
+        x = apply_any(ep, row + 8 * h, col, 0, x, vec, o[h]);
         if (ep.c16_hi) seen_max = split_track(seen_max, x);
       }
     }
@@ -597,7 +654,8 @@ __global__ void __maxnreg__(64) gemm_tc_fixup_kernel(const float* ws, const __gr
     if (ep.c16_hi && (split_seen_fixed(y) & 1u)) atomicCAS(ep.err, 0, kRangeCode);
   };
   if (!common) {
-    report(apply_any(ep, row, col0, bz, acc));
+    const bool vec = epilogue_vec(ep);
+    report(apply_any(ep, row, col0, bz, acc, vec, fetch_any(ep, row, col0, bz, vec)));
     return;
   }
   if (ep.bias_n) acc = make_float4(__fadd_rn(acc.x, b.x), __fadd_rn(acc.y, b.y), __fadd_rn(acc.z, b.z), __fadd_rn(acc.w, b.w));
@@ -1377,7 +1435,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         tc_fence_after();
         return there;
       };
-      if (PRE && ep.res && key >= 0 && wk.raw < 0) {
+      if (PRE && ep.res && wk.raw < 0) {
         // While the tile's MMAs run: pull this warp's 32 x 64 block of the residual into L2 -- but
         // not ahead of the kernel's first operand tiles (a thousand prefetches per SM issued at
         // kernel entry delayed those by 5 K clocks): wait until the first K-block has been used.
@@ -1438,12 +1496,12 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         const uint32_t part = acc + (uint32_t)cg;
         unsigned seen = 0;               // of this warp's part of the tile, as far as it was written as halves
         if (m0 >= ep.m) hand_back(acc_empty_leader, lane);
-        else if (wk.raw >= 0)
-          (void)epilogue_regs_other(ep, workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, BN, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
+        else if (!SUM && wk.raw >= 0)
+          epilogue_regs_raw(ep, workspace + ((size_t)wk.raw * 2 + rank) * BM * BN, BN, BN / 64, part, q, lane, cg, acc_empty_leader);
         else if (KEY >= 0)
           seen = epilogue_regs<BN / 64, (KEY >= 0 ? KEY >> 2 : 0), KEY & 1, (KEY & 2) != 0>(ep, part, q, lane, m0, nw, acc_empty_leader);
         else
-          seen = epilogue_regs_other(ep, nullptr, 0, BN / 64, part, q, lane, m0, nw, cg, acc_empty_leader);
+          seen = epilogue_regs_any(ep, BN / 64, part, q, lane, m0, nw, acc_empty_leader);
         if (ep.c16_hi) seen_before = report_tile(seen, min(32, ep.m - m0 - q * 32) * min(BN / 4, ep.n - nw), seen_before, err);
       } else if (m0 < ep.m) {
         if (wk.raw >= 0) {
@@ -1713,7 +1771,9 @@ cudaError_t launch_pair(const float* a, long long lda, int k, const CUtensorMap&
   return launch_fixup(workspace, ep, 2 * BM, BN, pl, st);
 }
 
-// A arrives as fp16 halves: by the epilogue that is compiled in.
+// A arrives as fp16 halves: by the epilogue that is compiled in. With short accumulators that is every one that
+// gemm_ks_epilogue_ok allows (LayerNormalization -> 12672 x 384 x 384 -> ReLU, and with a bias and a residual: 36 and 46 us; by
+// the run-time options 73 and 87, in gemm_ks.cu 47 and 48); elsewhere the others take epilogue_regs_any.
 template <int BN, bool SUM>
 cudaError_t launch_pair_key(const GemmParams& q, const CUtensorMap& ma, const CUtensorMap& mal, const CUtensorMap& mb, const CUtensorMap& mbl,
                             const TcEpilogue& ep, const TcPlan& pl, float* ws, int* err, cudaStream_t st) {
@@ -1728,8 +1788,19 @@ cudaError_t launch_pair_key(const GemmParams& q, const CUtensorMap& ma, const CU
     AC_PAIR((ACT_GELU << 2) | 1);
     AC_PAIR((ACT_RELU << 2) | 1);
 #undef AC_PAIR
-    default: return launch_pair<BN, true, -1, SUM>(q.a, q.lda, (int)q.k, ma, mal, mb, mbl, ep, pl, ws, err, st);
+#define AC_PAIR(KEYV) \
+  case KEYV: if constexpr (SUM) return launch_pair<BN, true, KEYV, SUM>(q.a, q.lda, (int)q.k, ma, mal, mb, mbl, ep, pl, ws, err, st); else break
+    AC_PAIR(ACT_GELU << 2);
+    AC_PAIR((ACT_GELU << 2) | 2);
+    AC_PAIR((ACT_GELU << 2) | 3);
+    AC_PAIR(ACT_RELU << 2);
+    AC_PAIR((ACT_RELU << 2) | 2);
+    AC_PAIR((ACT_RELU << 2) | 3);
+#undef AC_PAIR
   }
+  // With short accumulators these are all there are (gemm_ks_epilogue_ok, n at most 2^20).
+  if constexpr (SUM) return cudaErrorInvalidValue;
+  else return launch_pair<BN, true, -1, SUM>(q.a, q.lda, (int)q.k, ma, mal, mb, mbl, ep, pl, ws, err, st);
 }
 
 TcEpilogue epilogue_of(const GemmParams& q, int* err_word) {

@@ -59,6 +59,24 @@ def test_pair_epilogues(cuda_lib, m, n, k, act, bias, res):
     assert ((got - want).abs() <= 1e-5 * want.abs() + 5e-6 * mass + slack).all()
 
 
+# alpha, beta and C beside the product: whole float4s and single elements, a tile cut along K (k 1544), too.
+@pytest.mark.parametrize("m,n,k", [(2817, 1540, 264), (6305, 2306, 392), (2561, 1284, 1544)])
+@pytest.mark.parametrize("alpha,beta,full", [(0.5, 1.0, False), (1.0, -2.0, False), (0.5, 2.0, True), (1.0, 1.0, True)])
+def test_pair_epilogues_with_factors(cuda_lib, m, n, k, alpha, beta, full):
+    rng = np.random.default_rng(m + n)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    w = (rng.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32)
+    c = rng.standard_normal((m, n) if full else n).astype(np.float32)
+    g = ir.Graph()
+    xi = g.add_input("x", x.shape)
+    ci = g.add_input("c", c.shape) if full else g.new_init(c)
+    g.outputs.append(g.op("Gemm", xi, g.new_init(w), ci, alpha=alpha, beta=beta, trans_a=False, trans_b=True))
+    got = _run(g, [x] + ([c] if full else []), ["act_f16_split", "gemm_f16x3_pair_tcgen05"])
+    want = alpha * (_t(x) @ _t(w).T) + beta * _t(c)
+    mass = alpha * (_t(x).abs() @ _t(w).abs().T) + abs(beta) * _t(c).abs()
+    assert ((got - want).abs() <= 1e-5 * want.abs() + 5e-6 * mass).all()
+
+
 @pytest.mark.parametrize("m,h,n", [(2817, 1544, 512), (2561, 2312, 768)])
 def test_pair_writes_split_results_with_ragged_columns(cuda_lib, m, h, n):
     """The first product's result exists only as fp16 halves (16 bytes of a row per lane); columns end inside a
@@ -109,6 +127,32 @@ def test_pairs_with_short_accumulators(cuda_lib, m, d, n, bound, act, res):
     y = torch.relu(y) if act else y
     want = y + _t(r) if res else y
     assert ((got - want).norm() / want.norm()).item() <= bound
+    assert ((got - want).abs() <= 1e-5 * want.abs() + 2e-5).all()
+
+
+@pytest.mark.parametrize("act", [None, "ReLU", "Gelu"])
+@pytest.mark.parametrize("bias,res", [(False, False), (True, False), (False, True), (True, True)])
+def test_every_epilogue_with_short_accumulators(cuda_lib, act, bias, res):
+    rng = np.random.default_rng(5)
+    m, d, n = 3081, 840, 780
+    x = rng.standard_normal((m, d)).astype(np.float32)
+    w = (rng.standard_normal((d, n)) / np.sqrt(d)).astype(np.float32)
+    b, r = rng.standard_normal(n).astype(np.float32), rng.standard_normal((m, n)).astype(np.float32)
+    g = ir.Graph()
+    xi = g.add_input("x", x.shape)
+    ri = g.add_input("r", r.shape) if res else None
+    y = g.op("LayerNormalization", xi, g.new_init(np.ones(d, np.float32)), g.new_init(np.zeros(d, np.float32)), axis=-1, epsilon=1e-6,
+             stash_type=1)
+    y = g.op("MatMul", y, g.new_init(w))
+    y = g.op("Add", y, g.new_init(b)) if bias else y
+    y = g.op(act, y) if act else y
+    g.outputs.append(g.op("Add", y, ri) if res else y)
+    got = _run(g, [x] + ([r] if res else []), ["layer_norm", "gemm_f16x3_cluster_tcgen05"])
+    y = torch.nn.functional.layer_norm(_t(x), (d,), None, None, 1e-6) @ _t(w)
+    y = y + _t(b) if bias else y
+    y = {None: lambda v: v, "ReLU": torch.relu, "Gelu": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[act](y)
+    want = y + _t(r) if res else y
+    assert ((got - want).norm() / want.norm()).item() <= 2.35e-7 * (2 if act == "Gelu" else 1)   # of the product; Gelu's own 2e-7
     assert ((got - want).abs() <= 1e-5 * want.abs() + 2e-5).all()
 
 
