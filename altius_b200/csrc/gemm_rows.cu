@@ -2,8 +2,8 @@
 // crates/session_interpreter/src/gemm.rs:36-110, session.rs:684-734):
 //   C[m, n] = act(alpha * A[m, :] . B[n, :] + beta * Cin[m, n] + bias[n]) + residual[m, n]
 // in fp32. Bound by reading B once (1000 x 768 floats: 3 MB, 0.5 us of HBM) and by latency: one warp
-// per one or two columns n, its lanes along K with 16-byte loads, up to eight rows of A per warp (from
-// L1: all warps of a block read the same ones). A tile kernel gives such a product 8 to 16 blocks
+// per one or two columns n, its lanes along K with 16-byte loads, up to eight rows of A per warp (all
+// warps of a block read the same ones: from L1, eight rows of more than 256 floats from shared memory). A tile kernel gives such a product 8 to 16 blocks
 // with a split of the operands and a second pass behind it: 15 us for one row of 768 into 1000
 // columns, here 3.
 #include "kernels.h"
@@ -65,14 +65,14 @@ __device__ __forceinline__ void staged_products(const float* const (&a)[MT], con
   }
 }
 
-template <int MT, int NW>
-__global__ void __launch_bounds__(kWarps * 32, MT == 8 ? 3 : 1) gemm_rows_kernel(const GemmParams p) {
+template <int MT, int NW, bool STAGED>
+__global__ void __launch_bounds__(kWarps * 32, STAGED ? 3 : 1) gemm_rows_kernel(const GemmParams p) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n0 = (blockIdx.x * kWarps + warp) * NW, m0 = blockIdx.y * MT;
   const int N = (int)p.n, M = (int)p.m, K = (int)p.k;
   pdl_trigger();
   pdl_wait();
-  if (MT < 8 && n0 >= N) return;
+  if (!STAGED && n0 >= N) return;
   const float* a[MT];
   const float* b[NW];
 #pragma unroll
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kWarps * 32, MT == 8 ? 3 : 1) gemm_rows_kernel
   for (int j = 0; j < NW; ++j)
 #pragma unroll
     for (int i = 0; i < MT; ++i) acc[j][i] = 0.f;
-  if (MT == 8) staged_products<MT, NW>(a, b, K, lane, acc);
+  if (STAGED) staged_products<MT, NW>(a, b, K, lane, acc);
   else
 #pragma unroll (MT <= 2 ? 4 : 2)
   for (int k = lane * 4; k < K; k += 128) {
@@ -123,10 +123,10 @@ __global__ void __launch_bounds__(kWarps * 32, MT == 8 ? 3 : 1) gemm_rows_kernel
   p.c[(long long)m * p.ldc + n] = v;
 }
 
-template <int MT, int NW>
+template <int MT, int NW, bool STAGED = false>
 cudaError_t launch_t(const GemmParams& p, cudaStream_t st) {
   const dim3 grid((unsigned)((p.n + kWarps * NW - 1) / (kWarps * NW)), (unsigned)((p.m + MT - 1) / MT));
-  return launch_pdl(gemm_rows_kernel<MT, NW>, grid, dim3(kWarps * 32), 0, st, 1, p);
+  return launch_pdl(gemm_rows_kernel<MT, NW, STAGED>, grid, dim3(kWarps * 32), 0, st, 1, p);
 }
 
 inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
@@ -143,7 +143,9 @@ cudaError_t launch_gemm_rows(const GemmParams& p, cudaStream_t st) {
   if (p.m == 1) return launch_t<1, 1>(p, st);
   if (p.m == 2) return launch_t<2, 1>(p, st);
   if (p.m <= 4) return launch_t<4, 2>(p, st);
-  return launch_t<8, 2>(p, st);
+  // A lane's two steps of K are under way at once without a detour: with them alone, shared memory only costs its barrier (5 to 32
+  // rows, 40 and 1000 columns, call times: K = 32 to 128 0.7 us longer, 192 and 256 the same, 320 to 768 0.2 to 1.7 us shorter).
+  return p.k > 256 ? launch_t<8, 2, true>(p, st) : launch_t<8, 2>(p, st);
 }
 
 }  // namespace ac

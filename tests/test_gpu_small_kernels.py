@@ -231,7 +231,8 @@ def test_few_row_products_beyond_the_fixed_scale(cuda_lib):
 
 # eight rows a block, in parts of 1024 floats of K: one part, a whole and a ragged second one, fewer quads than lanes, rows and
 # columns off the tile; a row of A without finite values stays in its row
-@pytest.mark.parametrize("m,k,n", [(5, 1024, 33), (8, 1028, 16), (13, 2048, 17), (31, 2564, 40), (6, 20, 5)])
+# (up to 256 floats of K it is not staged)
+@pytest.mark.parametrize("m,k,n", [(5, 1024, 33), (8, 1028, 16), (13, 2048, 17), (31, 2564, 40), (6, 20, 5), (7, 256, 19), (17, 260, 19)])
 def test_product_of_eight_rows_in_parts_of_k(cuda_lib, m, k, n):
     rng = np.random.default_rng(m * k + n)
     a = rng.standard_normal((m, k)).astype(np.float32)
