@@ -69,11 +69,12 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 }
 
 // ONE: one accumulator for all terms, two buffers (a block that does not walk uses the first).
-// 96 registers: a quarter of an SM holds five such warps (16384 registers), so that two blocks of nine fit. With 112 it held four,
-// one block per SM, whatever the shared memory left (32 images of 16 x 112 x 112 into 64 channels: 9 warps active, issue 32 %,
+// ALONE: no second block fits the SM. Then a second set of registers takes the next step's loads while this one is split. Else 96
+// registers: a quarter of an SM holds five such warps (16384 registers), so that two blocks of nine fit. With 112 it holds four,
+// one block per SM, whatever the shared memory leaves (32 images of 16 x 112 x 112 into 64 channels: 9 warps active, issue 37 %,
 // 56 us; MobileNetV3-Large at 32 images 919 us, with two blocks 798).
-template <bool WINDOW, int ACT, bool ONE>
-__global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
+template <bool WINDOW, int ACT, bool ONE, bool ALONE>
+__global__ void __maxnreg__(ALONE ? 112 : 96) conv_tc_kernel(const ConvTcDev p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], w_full;
@@ -224,7 +225,7 @@ __global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
       for (int j = 0; j < 16; ++j) d[j] = __fmul_rn(d[j], gv[j]);
     };
 
-    float v[16];
+    float v[16], ahead_v[ALONE ? 16 : 1];
     uint32_t use = 0;
     int g = 0;                                 // running K step
     bool alive = true;
@@ -232,7 +233,14 @@ __global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
     // behind them in v.
     auto fill = [&](int i, int from, int to) {
       for (int kb = from; kb < to && alive; ++kb, ++g) {
-        if (gcol) apply_gate(kb, gcol, v);
+        const float* gc = gcol;
+        auto next = [&](float (&d)[16]) -> uint32_t {
+          if (kb + 1 == kbs) place(i + 1);
+          return kb + 1 < kbs || i + 1 < mine ? fetch(kb + 1 < kbs ? kb + 1 : 0, d) : 0u;
+        };
+        uint32_t ahead_use = 0;
+        if constexpr (ALONE) ahead_use = next(ahead_v);
+        if (gc) apply_gate(kb, gc, v);
         const int s = g % S;
         if (g >= S) {
           if (!mbar_wait_all(&empty[s], ((g / S) & 1) ^ 1)) { atomicExch(p.err, 31); abort_flag = 1; alive = false; return; }
@@ -258,10 +266,13 @@ __global__ void __maxnreg__(96) conv_tc_kernel(const ConvTcDev p) {
         fence_proxy_async();
         __syncwarp();                          // one arrival per warp: those of 256 threads took their turns at the barrier
         if (lane == 0) mbar_arrive(&full[s]);
-        // The next step's loads, under way over the epilogue that may lie in front of it. (A second set of registers for
-        // them would leave one block per SM.)
-        if (kb + 1 == kbs) place(i + 1);
-        if (kb + 1 < kbs || i + 1 < mine) use = fetch(kb + 1 < kbs ? kb + 1 : 0, v);
+        if constexpr (ALONE) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = ahead_v[j];
+          use = ahead_use;
+        } else {
+          use = next(v);                       // under way over the epilogue that may lie in front of the next step
+        }
       }
     };
 
@@ -459,17 +470,23 @@ Shape shape_of(const ConvParams& q) {
   return pick_shape(q, {device_sm_count(), cluster_slots(2), cluster_slots(4), cluster_slots(8)});
 }
 
-template <bool WINDOW, int ACT, bool ONE>
+template <bool WINDOW, int ACT, bool ONE, bool ALONE>
 cudaError_t launch_form(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
   static unsigned long long done = 0;
-  if (cudaError_t e = ensure_dynamic_smem(conv_tc_kernel<WINDOW, ACT, ONE>, (int)kSmemMax, &done)) return e;
+  if (cudaError_t e = ensure_dynamic_smem(conv_tc_kernel<WINDOW, ACT, ONE, ALONE>, (int)kSmemMax, &done)) return e;
   const dim3 grid((unsigned)sh.ctas, (unsigned)sh.tiles, (unsigned)sh.split);
-  return launch_pdl(conv_tc_kernel<WINDOW, ACT, ONE>, grid, dim3(kThreads), sh.smem, st, sh.split, p);
+  return launch_pdl(conv_tc_kernel<WINDOW, ACT, ONE, ALONE>, grid, dim3(kThreads), sh.smem, st, sh.split, p);
 }
 
 template <bool WINDOW, int ACT>
 cudaError_t launch_act(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
-  return sh.mains == 0 ? launch_form<WINDOW, ACT, true>(p, sh, st) : launch_form<WINDOW, ACT, false>(p, sh, st);
+  // Blocks of more than half of an SM's shared memory (calls of 32 x 117 x 57 x 57 into 216: with the second set 93 us, without 99;
+  // 13 x 326 x 57 x 57 into 170: 79 and 80). Where there are only too few blocks for two on an SM, and with a window, the second set
+  // gains on some shapes what it loses on others (1.01 of the time over 26 shapes, 1.00 over 45 with a window).
+  const bool alone = sh.smem > kSmemSm / 2 - kSmemBeside;
+  if constexpr (!WINDOW)
+    if (alone) return sh.mains == 0 ? launch_form<WINDOW, ACT, true, true>(p, sh, st) : launch_form<WINDOW, ACT, false, true>(p, sh, st);
+  return sh.mains == 0 ? launch_form<WINDOW, ACT, true, false>(p, sh, st) : launch_form<WINDOW, ACT, false, false>(p, sh, st);
 }
 
 template <bool WINDOW>

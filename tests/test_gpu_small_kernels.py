@@ -107,7 +107,9 @@ def test_product_of_a_few_rows(cuda_lib, m, k, n):
     (5, 1, 512, 16, 1, 1, 0, True), (1, 4096, 5, 300, 1, 1, 0, False), (32, 16, 40, 64, 1, 1, 0, False),
     # wide channel tiles with a table and a cluster's exchange beside the ring
     (8, 256, 14, 256, 3, 1, 1, False), (1, 256, 28, 512, 3, 1, 1, False), (1, 256, 32, 480, 3, 1, 1, False),
-    (16, 128, 14, 256, 3, 1, 1, False), (2, 448, 14, 250, 3, 1, 1, False)])
+    (16, 128, 14, 256, 3, 1, 1, False), (2, 448, 14, 250, 3, 1, 1, False),
+    # walking blocks that have an SM to themselves
+    (6, 117, 57, 216, 1, 1, 0, True), (6, 117, 57, 215, 1, 1, 0, False)])
 def test_tensor_core_convolution(cuda_lib, n, c, h, oc, k, s, p, gate):
     rng = np.random.default_rng(c * h + oc)
     x = rng.standard_normal((n, c, h, h)).astype(np.float32)
