@@ -382,21 +382,20 @@ cudaError_t launch_act(const CUtensorMap& ah, const CUtensorMap& al, const CUten
 
 inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
 
+}  // namespace
+
 // Products whose tiles take this kernel more than a round go to CTA pairs on tiles of 256 x 192 that hand their
-// accumulators over to fp32 sums every `run` K-blocks (launch_gemm_pair_sums; 0: stay here). In this kernel's clocks
-// such a tile takes 1300 a K-block and 6000 around them (us with a LayerNormalization in front, here -> there: 3152 x 768 x 768
-// 31.6 -> 23.2, 12672 x 384 x 384 37.3 -> 30.4, 788 x 768 x 3072 30.6 -> 22.7; but 2885 x 768 x 768 20.5 -> 23.0,
-// 1576 x 512 x 512 14.2 -> 18.4). Relative error against 64 bits with runs of two 1.6e-7 for any K, of one 1.2e-7; here
-// 2.1e-7 at K = 768, 2.0e-7 at 576, 1.5e-7 at 384 and 512: one there.
-int pair_sums_run(const GemmParams& q, double clocks) {
-  if (q.c16_hi && ((q.n % 8) || (q.ldc16 % 8) || !al16(q.c16_hi) || !al16(q.c16_lo))) return 0;
+// accumulators over to fp32 sums every `run` K-blocks (launch_gemm_pair_sums; 0: stay here). Fitted in this kernel's clocks,
+// launch and ends included as in pick_shape: 1300 a K-block of such a tile and 6000 around them (us with a LayerNormalization
+// in front, here -> there: 3152 x 768 x 768 31.6 -> 23.2, 12672 x 384 x 384 37.3 -> 30.4, 788 x 768 x 3072 30.6 -> 22.7; but
+// 2885 x 768 x 768 20.5 -> 23.0, 1576 x 512 x 512 14.2 -> 18.4). Relative error against 64 bits with runs of two 1.6e-7 for
+// any K, of one 1.2e-7; here 2.1e-7 at K = 768, 2.0e-7 at 576, 1.5e-7 at 384 and 512: one there.
+int gemm_ks_pair_run(int64_t m, int64_t n, int64_t k) {
   const int64_t pairs = gemm_tc_pairs();
   if (pairs <= 0) return 0;
-  const int64_t nkb = (q.k + KB - 1) / KB, tiles = ((q.m + 255) / 256) * ((q.n + 191) / 192), rounds = (tiles + pairs - 1) / pairs;
-  return 4000.0 + rounds * (1300.0 * nkb + 6000.0) < 0.97 * clocks ? (q.k > 576 ? 2 : 1) : 0;
+  const int64_t nkb = (k + KB - 1) / KB, tiles = ((m + 255) / 256) * ((n + 191) / 192), rounds = (tiles + pairs - 1) / pairs;
+  return 4000.0 + rounds * (1300.0 * nkb + 6000.0) < 0.97 * gemm_ks_clocks(m, n, k) ? (k > 576 ? 2 : 1) : 0;
 }
-
-}  // namespace
 
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k) {
   if (m < 1 || n < 4 || (n % 4) || k < 64 || (k % 8) || m > (1 << 20) || n > (1 << 20)) return 1e30;
@@ -407,14 +406,17 @@ bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bia
   return (act == ACT_NONE || act == ACT_GELU || act == ACT_RELU) && !bias_m && !c_in && alpha == 1.f && bias_scale == 1.f;
 }
 
-cudaError_t launch_gemm_ks(const GemmParams& q, int* err_word, cudaStream_t st) {
+cudaError_t launch_gemm_ks(const GemmParams& q, int pair_run, int* err_word, cudaStream_t st) {
   if (!q.a16_hi || !q.a16_lo || !q.b16_hi || !q.b16_lo || !q.a16_fixed || !q.b16_plain || q.batch != 1 || (q.n % 4) ||
       (q.k % 8) || (q.lda16 % 8) || (q.ldb16 % 8) || !al16(q.a16_hi) || !al16(q.a16_lo) || !al16(q.b16_hi) || !al16(q.b16_lo) ||
       (q.c && (!al16(q.c) || (q.ldc % 4))) || (q.residual && (!al16(q.residual) || (q.ld_res % 4))) || (q.bias_n && !al16(q.bias_n)) ||
       (q.c16_hi && (q.ldc16 % 4)) || !gemm_ks_epilogue_ok(q.act, q.bias_m != nullptr, q.beta != 0.f && q.c_in, q.alpha, q.bias_scale))
     return cudaErrorInvalidValue;
+  if (pair_run) {
+    if (q.c16_hi && ((q.n % 8) || (q.ldc16 % 8) || !al16(q.c16_hi) || !al16(q.c16_lo))) return cudaErrorInvalidValue;   // 16 bytes of a row at once
+    return launch_gemm_pair_sums(q, pair_run, err_word, st);
+  }
   const Shape sh = pick_shape(q.m, q.n, q.k);
-  if (const int run = pair_sums_run(q, sh.clocks)) return launch_gemm_pair_sums(q, run, err_word, st);
   KsDev d{};
   d.m = (int)q.m; d.n = (int)q.n; d.k = (int)q.k;
   d.bn = sh.bn; d.stages = sh.stages; d.kper = sh.kper; d.inv = sh.inv;

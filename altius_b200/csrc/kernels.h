@@ -283,7 +283,10 @@ int gemm_tc_pairs();
 int cluster_slots(int split);
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k);
 bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bias_scale);
-cudaError_t launch_gemm_ks(const GemmParams& p, int* err_word, cudaStream_t st);
+// K-blocks of 64 on one accumulator where such a product is better off on CTA pairs, or 0 for the few-row kernel itself; the
+// lowering asks, so that the schedule names the kernel that runs, and hands the answer to the launch.
+int gemm_ks_pair_run(int64_t m, int64_t n, int64_t k);
+cudaError_t launch_gemm_ks(const GemmParams& p, int pair_run, int* err_word, cudaStream_t st);
 // The same operands and epilogues on CTA pairs, `run` K-blocks of 64 on one accumulator (gemm_tc.cu).
 cudaError_t launch_gemm_pair_sums(const GemmParams& p, int run, int* err_word, cudaStream_t st);
 // fp16 split of a constant [rows, k] operand (row stride ld) into [rows, k8] halves

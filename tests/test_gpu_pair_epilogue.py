@@ -103,8 +103,8 @@ def test_pair_writes_split_results_with_ragged_columns(cuda_lib, m, h, n):
 
 
 # Products that the kernel for few rows would take more than a round for: CTA pairs on 256 x 192 tiles whose accumulators
-# are given up every one or two K-blocks. Bound: what that kernel measured on these inputs. The last two have ragged rows, columns
-# and K.
+# are given up every one or two K-blocks. Bound: what the few-row kernel measured on these inputs. The last two have ragged rows,
+# columns and K.
 @pytest.mark.parametrize("m,d,n,bound", [(3152, 768, 768, 2.09e-7), (12672, 384, 384, 1.51e-7), (788, 768, 3072, 2.11e-7),
                                          (6304, 384, 384, 1.53e-7), (3081, 840, 780, 2.35e-7), (8001, 520, 324, 1.62e-7)])
 @pytest.mark.parametrize("act,res", [(None, False), ("ReLU", True)])
@@ -122,7 +122,7 @@ def test_pairs_with_short_accumulators(cuda_lib, m, d, n, bound, act, res):
     y = g.op("Add", g.op("MatMul", h, g.new_init(w)), g.new_init(b))
     y = g.op(act, y) if act else y
     g.outputs.append(g.op("Add", y, ri) if res else y)
-    got = _run(g, [x] + ([r] if res else []), ["layer_norm", "gemm_f16x3_cluster_tcgen05"])
+    got = _run(g, [x] + ([r] if res else []), ["layer_norm", "gemm_f16x3_pair_sums_tcgen05"])
     y = torch.nn.functional.layer_norm(_t(x), (d,), None, None, 1e-6) @ _t(w) + _t(b)
     y = torch.relu(y) if act else y
     want = y + _t(r) if res else y
@@ -147,7 +147,7 @@ def test_every_epilogue_with_short_accumulators(cuda_lib, act, bias, res):
     y = g.op("Add", y, g.new_init(b)) if bias else y
     y = g.op(act, y) if act else y
     g.outputs.append(g.op("Add", y, ri) if res else y)
-    got = _run(g, [x] + ([r] if res else []), ["layer_norm", "gemm_f16x3_cluster_tcgen05"])
+    got = _run(g, [x] + ([r] if res else []), ["layer_norm", "gemm_f16x3_pair_sums_tcgen05"])
     y = torch.nn.functional.layer_norm(_t(x), (d,), None, None, 1e-6) @ _t(w)
     y = y + _t(b) if bias else y
     y = {None: lambda v: v, "ReLU": torch.relu, "Gelu": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[act](y)
@@ -231,7 +231,7 @@ def test_tiny_results_are_reported(cuda_lib, m, d, h, n, norm, act, bias, res):
     r = tiny * rng.standard_normal((m, h)).astype(np.float32) if res else None
     x = rng.standard_normal((m, d)).astype(np.float32)
     got, want, before, after = _mlp(x, tiny * w1, w2, b1, act, r, norm)
-    assert before != after
+    assert before[1] == ("gemm_f16x3_pair_sums_tcgen05" if norm else "gemm_f16x3_pair_tcgen05") and before != after
     assert _rel(got, want) <= 3e-5                   # 3xTF32, of positive values: 1.3e-5; as halves 6e-3
 
 
@@ -247,3 +247,21 @@ def test_a_tile_of_tiny_results_is_reported(cuda_lib, m, d, h, n, norm):
     got, want, before, after = _mlp(x, w1, w2, norm=norm)
     assert before != after
     assert _rel(got[:256], want[:256]) <= 3e-5       # as halves 7e-4
+
+
+# In range the halves stay: M, N and K off the tiles, N a multiple of 8 but not of 16; one value beyond 255 goes to another plan.
+@pytest.mark.parametrize("m,d,h,n,norm", [(1577, 392, 1544, 384, True), (3081, 776, 776, 520, True), (6305, 392, 1544, 384, False)])
+@pytest.mark.parametrize("act,bias,res", [(None, False, False), ("Gelu", True, False), ("ReLU", False, False), ("Gelu", True, True)])
+@pytest.mark.parametrize("beyond", [False, True])
+def test_results_as_halves(cuda_lib, m, d, h, n, norm, act, bias, res, beyond):
+    rng = np.random.default_rng(m + h)
+    w1, w2 = _weights(rng, d, h, n)
+    b1 = rng.standard_normal(h).astype(np.float32) if bias or beyond else None
+    if beyond:
+        b1[h - 1] = 300
+    r = rng.standard_normal((m, h)).astype(np.float32) if res else None
+    x = rng.standard_normal((m, d)).astype(np.float32)
+    got, want, before, after = _mlp(x, w1, w2, b1, act, r, norm)
+    assert before[1] == ("gemm_f16x3_pair_sums_tcgen05" if norm else "gemm_f16x3_pair_tcgen05")
+    assert (before != after) == beyond
+    assert _rel(got, want) <= 2e-6

@@ -101,6 +101,19 @@ def test_fusion_folds_the_expected_chains():
     assert not any(e["kind"].endswith("tcgen05") for e in cuda_cores)
 
 
+def test_the_schedule_names_the_kernel_of_a_product():
+    """Behind a LayerNormalization: the few-row kernel, beyond a round of it CTA pairs with short accumulators, or long ones."""
+    def kind(m, d, n):
+        g = ir.Graph()
+        one, zero = g.new_init(np.ones(d, np.float32)), g.new_init(np.zeros(d, np.float32))
+        h = g.op("LayerNormalization", g.add_input("x", (m, d)), one, zero, axis=-1, epsilon=1e-6, stash_type=1)
+        g.outputs.append(g.op("MatMul", h, g.new_init(np.zeros((d, n), np.float32))))
+        return plan(ir.Model(g, 13)).schedule()[-1]["kind"]
+    assert kind(197, 768, 2304) == kind(2885, 768, 768) == "gemm_f16x3_cluster_tcgen05"
+    assert kind(3152, 768, 768) == kind(12672, 384, 384) == "gemm_f16x3_pair_sums_tcgen05"
+    assert kind(6304, 768, 2304) == "gemm_f16x3_pair_tcgen05"
+
+
 def test_flops_of_vit_match_the_published_count():
     model, _ = configs.vit_base_16(batch=1, depth=12)
     flops = sum(e["flops"] for e in plan(model).schedule())
