@@ -447,7 +447,7 @@ __device__ __forceinline__ float4 apply_any(const TcEpilogue& ep, int row, int c
 }
 
 // The epilogue of the pair kernel that takes A pre-split: sixteen warps, a warp per tensor-memory lane
-// quarter and 64-column group, in eight blocks of 16 rows x 16 columns that go from tensor memory to global
+// quarter and 64 columns (48 of 192), in eight (six) blocks of 16 rows x 16 columns that go from tensor memory to global
 // memory through registers alone. The fragment of tcgen05.ld.16x256b gives a lane two neighbouring columns
 // of two rows in each 8-column group; one exchange with the neighbouring lane makes them float4s (bias, residual and
 // fp32 stores are 64 contiguous bytes per row and instruction), and one more, with the lane two on, makes the
@@ -1436,9 +1436,10 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         return there;
       };
       if (PRE && ep.res && wk.raw < 0) {
-        // While the tile's MMAs run: pull this warp's 32 x 64 block of the residual into L2 -- but
-        // not ahead of the kernel's first operand tiles (a thousand prefetches per SM issued at
-        // kernel entry delayed those by 5 K clocks): wait until the first K-block has been used.
+        // While the tile's MMAs run: pull this warp's 32 x 64 block of the residual into L2 (whole 128-byte lines: of
+        // 192 columns a warp has 48, and the rest of the last line is its neighbour's) -- but not ahead of the kernel's
+        // first operand tiles (a thousand prefetches per SM issued at kernel entry delayed those by 5 K clocks): wait
+        // until the first K-block has been used.
         if (ti == 0) (void)mbar_wait(&empty[0], 0);
         const float* rp = ep.res + (long long)bz * ep.sres;
 #pragma unroll
@@ -1908,7 +1909,9 @@ TcShape pick_shape(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, 
     if (cost < best_cost - 1e-9) { best_cost = cost; best = c; }
   }
   // CTA pairs (fp16 split, one GEMM, BN 256): 256 x 256 tiles, each SM pulls its A rows and
-  // half of B (32 KB per stage), the pair's MMAs cost 128 clocks per SM; single accumulator set.
+  // half of B (32 KB per stage), the pair's MMAs cost 128 clocks per SM; single accumulator set. That is the kernel that
+  // stages A through registers. The one that takes A split is faster (1540 clocks for 64 of K, here 2340; its epilogue
+  // under the next tile), so near the line it is left aside where it would win: products stay where their errors were measured.
   const int pairs = allow_pairs ? pair_count() : 0;
   if (f16 && batch == 1 && (k % (allow_pairs == 2 ? 8 : 4)) == 0 && pairs > 0 && (!fbn || fbn == 256)) {
     const int pkb = kbf;
@@ -1928,17 +1931,19 @@ bool gemm_tc_wants_presplit(int64_t m, int64_t n, int64_t k, int64_t batch) {
   return pick_shape(m, n, k, batch, 2, 2).pair;
 }
 
-// What the choice between this kernel and the more exact ones (gemm_ks_clocks) counts: 1950 clocks a K-block of a
-// 256 x 256 tile, 20000 for launch, first operands and last epilogue, 9000 for the K-slice pass. These are the figures of an
-// epilogue through shared memory; the kernel takes 1540, 18000 and 7500 now. They stay, because with those products
-// would move from errors of 2e-7 to 1e-6 for a few us (2885 x 768 x 768, 1576 x 512 x 512).
+// What the choice between this kernel and the more exact ones (gemm_ks_clocks) counts: the kernel's clocks for a K-block of a
+// 256 x 256 tile, for launch, first operands and last epilogue, and for the K-slice pass; and what the smaller error of the
+// others is worth beside each: without that products would move from errors of 2e-7 to 1e-6 for a few us (2885 x 768 x 768,
+// 1576 x 512 x 512).
+constexpr double kPairBlock = 1540, kPairEnds = 18000, kPairSlices = 7500;
+constexpr double kExactBlock = 410, kExactEnds = 2000, kExactSlices = 1500;
 double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k) {
   const int pairs = pair_count();
   if (pairs <= 0) return 1e30;
   const TcPlan pl = make_plan(m, n, k, 1, 256, 2, 64, pairs);
   double blocks = (double)((pl.sc.dp_tiles + pairs - 1) / pairs) * pl.sc.num_kb;
   if (pl.sc.tail_parts >= 2) blocks += (double)pl.sc.num_kb / pl.sc.tail_parts;
-  return blocks * 1950.0 + 20000.0 + (pl.sc.tail_parts >= 2 ? 9000.0 : 0.0);
+  return blocks * (kPairBlock + kExactBlock) + kPairEnds + kExactEnds + (pl.sc.tail_parts >= 2 ? kPairSlices + kExactSlices : 0.0);
 }
 
 size_t gemm_tc_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, int allow_pairs) {
@@ -2004,8 +2009,8 @@ cudaError_t launch_gemm_tc(const GemmParams& q, int mode, int* err_word, cudaStr
   ep.b_row_scale = q.b_row_scale; ep.b_row_scale_stride = q.b_row_scale_stride;
   if (q.b_row_scale && kmode != TC_3X_SPLIT_B_MN) return cudaErrorInvalidValue;   // exists for the [K, N] operand only
   if (q.c16_hi) {
-    // Only the pair kernel's common epilogues (and the tail fix-up) write the split result.
-    if (!(sh.pair && pre) || !q.c16_lo || !q.c16_fixed || q.batch != 1 || (q.n % 8) != 0 || (q.ldc16 % 8) != 0 ||
+    // Only the pair kernel's epilogues (and the tail fix-up) write the split result.
+    if (!(sh.pair && pre) || !q.c16_lo || q.batch != 1 || (q.n % 8) != 0 || (q.ldc16 % 8) != 0 ||
         ((reinterpret_cast<uintptr_t>(q.c16_hi) | reinterpret_cast<uintptr_t>(q.c16_lo)) & 15) != 0 ||
         !gemm_tc_can_split_output(q.act, q.bias_n != nullptr, q.bias_m != nullptr, q.c_in && q.beta != 0.f, q.alpha, q.bias_scale) ||
         (q.c && ((q.ldc % 4) != 0 || (reinterpret_cast<uintptr_t>(q.c) & 15) != 0)) ||
@@ -2087,7 +2092,7 @@ cudaError_t launch_f16_split(const float* x, void* hi, void* lo, int64_t rows, i
 }
 
 bool gemm_tc_can_split_output(int act, bool bias_n, bool bias_m, bool c_in, float alpha, float bias_scale) {
-  // The epilogues the pair kernel has compiled in with the split store (epilogue_regs' callers).
+  // Those of the 256-column pair kernel, with or without a residual (behind an activation that is an epilogue by run-time options).
   return !bias_m && !c_in && alpha == 1.f && bias_scale == 1.f && (act == ACT_NONE || (bias_n && (act == ACT_GELU || act == ACT_RELU)));
 }
 

@@ -230,9 +230,7 @@ struct GemmParams {
   float* c; int64_t ldc; int64_t stride_c;   // c may be null when c16_hi / c16_lo are given
   void* c16_hi;             // tensor-core pair kernel only: the result also (or only) as fp16 hi / lo
   void* c16_lo;             // halves [m, ldc16], for the GEMM that takes it as its pre-split A; or null
-  int64_t ldc16;
-  int c16_fixed;            // 0: hi / lo as f16_split (lo scaled by 2^11); 1: both on the fixed scale 2^8
-                            // (f16_split_fixed): what the kernels that take their operands by TMA read
+  int64_t ldc16;            // both on the fixed scale 2^8 (f16_split_fixed): what the kernels that take their operands by TMA read
   int a16_fixed;            // a16_hi / a16_lo are on the fixed scale (required by the pair kernel that takes them)
   int b16_plain;            // b16_lo = rn(v - hi) on the scale of b16_hi (the same kernel's format for B)
   const float* b16_inv_scale;  // device scalar 2^-e when b16_hi / b16_lo hold B * 2^e; or null
@@ -329,7 +327,7 @@ bool attention_tc_supported(const AttentionParams& p);
 cudaError_t launch_attention_tc(const AttentionParams& p, cudaStream_t st);
 
 // tcgen05 kernel fed by TMA: Q, K and V are column ranges of one [B, T, ld16] projection that its
-// GEMM wrote as two fp16 arrays on the fixed scale (GemmParams::c16_fixed); head_dim 64,
+// GEMM wrote as two fp16 arrays on the fixed scale (GemmParams::c16_hi); head_dim 64,
 // 64 < tokens <= 208. Head h of an operand starts at column col + 64 h.
 struct Attention16Params {
   const void* qkv16_hi; const void* qkv16_lo;

@@ -1032,14 +1032,13 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   // This GEMM's own result, when a later GEMM takes it pre-split and this one runs on the pair
   // kernel with an epilogue that can write the halves.
   int c16_hi = -1, c16_lo = -1;
-  bool c_fp32 = true, c16_fixed = false;
+  bool c_fp32 = true;
   {
     auto so = em.c.split.find(out);
     if (so != em.c.split.end() && !so->second.produced && a16_hi >= 0 && c_off == 0 && g.ldc == g.n && (g.n % 8) == 0 &&
         (use_ks || gemm_tc_can_split_output(act, bias_n >= 0, bias_m >= 0, c_in >= 0, alpha, bias_scale))) {
       c16_hi = so->second.hi; c16_lo = so->second.lo;
       c_fp32 = so->second.fp32_needed;
-      c16_fixed = true;
       so->second.produced = true;
     }
   }
@@ -1084,7 +1083,6 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
     p.c16_hi = c16_hi >= 0 ? s->ptr(c16_hi) : nullptr;
     p.c16_lo = c16_lo >= 0 ? s->ptr(c16_lo) : nullptr;
     p.ldc16 = g.n;
-    p.c16_fixed = c16_fixed ? 1 : 0;
     p.b16_inv_scale = b16_scale >= 0 ? s->fptr(b16_scale) : nullptr;
     p.b_row_scale = b_row_scale >= 0 ? s->fptr(b_row_scale) : nullptr;
     p.b_row_scale_stride = g.k;

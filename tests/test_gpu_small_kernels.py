@@ -57,7 +57,7 @@ def test_small_convolution(cuda_lib, n, c, h, oc, k, s, p, gate):
     assert (np.abs(got - want) <= (c * k * k + 8) * EPS * mass).all()
 
 
-# one, two and four images per cluster, with a remainder; planes with and without whole float4s
+# one, two and three images per cluster, with a remainder; planes with and without whole float4s
 @pytest.mark.parametrize("n,c,h,s", [(1, 72, 28, 24), (3, 960, 7, 240), (19, 120, 14, 32), (41, 36, 5, 4), (1, 8, 1, 8)])
 def test_squeeze_excite_block(cuda_lib, n, c, h, s):
     rng = np.random.default_rng(c + h)
