@@ -1439,8 +1439,9 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         // While the tile's MMAs run: pull this warp's 32 x 64 block of the residual into L2 (whole 128-byte lines: of
         // 192 columns a warp has 48, and the rest of the last line is its neighbour's) -- but not ahead of the kernel's
         // first operand tiles (a thousand prefetches per SM issued at kernel entry delayed those by 5 K clocks): wait
-        // until the first K-block has been used.
-        if (ti == 0) (void)mbar_wait(&empty[0], 0);
+        // until the first K-block has been used, but not for long: for a warp that comes later than the K-blocks behind
+        // it, the barrier's parity has turned.
+        for (int i = 0; ti == 0 && i < 256 && !mbar_test(&empty[0], 0); ++i) __nanosleep(64);
         const float* rp = ep.res + (long long)bz * ep.sres;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
