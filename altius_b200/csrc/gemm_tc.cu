@@ -1435,7 +1435,7 @@ gemm_tc_pair_kernel(const float* a_ptr, long long lda, int k_total,
         tc_fence_after();
         return there;
       };
-      if (PRE && ep.res && wk.raw < 0) {
+      if (PRE && ep.res && wk.raw < 0 && (KEY >= 0 || epilogue_vec(ep))) {   // (an aligned residual)
         // While the tile's MMAs run: pull this warp's 32 x 64 block of the residual into L2 (whole 128-byte lines: of
         // 192 columns a warp has 48, and the rest of the last line is its neighbour's) -- but not ahead of the kernel's
         // first operand tiles (a thousand prefetches per SM issued at kernel entry delayed those by 5 K clocks): wait

@@ -1,6 +1,7 @@
 """Epilogues of the CTA-pair GEMM against float64 at the edges of its tiles (256 x 256; blocks of 16 x 16 within): a
 row or a few columns beyond whole tiles, columns that are whole float4s but not whole groups of eight, K-sliced
-last tiles. The bound is the one of all fp16-split products: 1e-5 of the result and 5e-6 of sum |a||b|."""
+last tiles. The bound is the one of all fp16-split products: 1e-5 of the result and 5e-6 of sum |a||b|. Then its form with
+short accumulators, and the range of the halves that both write for a next product."""
 import os
 import subprocess
 import sys
