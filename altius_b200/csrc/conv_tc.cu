@@ -480,10 +480,11 @@ cudaError_t launch_form(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
 
 template <bool WINDOW, int ACT>
 cudaError_t launch_act(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
-  // Blocks of more than half of an SM's shared memory (calls of 32 x 117 x 57 x 57 into 216: with the second set 93 us, without 99;
-  // 13 x 326 x 57 x 57 into 170: 79 and 80). Where there are only too few blocks for two on an SM, and with a window, the second set
-  // gains on some shapes what it loses on others (1.01 of the time over 26 shapes, 1.00 over 45 with a window).
-  const bool alone = sh.smem > kSmemSm / 2 - kSmemBeside;
+  // Walking blocks of more than half of an SM's shared memory (calls of 32 x 117 x 57 x 57 into 216: with the second set 94 us,
+  // without 101; 13 x 326 x 57 x 57 into 170: 79 and 78). Blocks of that size with a tile each lose by it (MobileNetV3-Large, 56
+  // images of 192 x 192: 925 us, without 912); where only the grid is too small for two on an SM, and with a window, it gains on
+  // some shapes what it loses on others.
+  const bool alone = sh.smem > kSmemSm / 2 - kSmemBeside && sh.ctas < (p.n + PX - 1) / PX;
   if constexpr (!WINDOW)
     if (alone) return sh.mains == 0 ? launch_form<WINDOW, ACT, true, true>(p, sh, st) : launch_form<WINDOW, ACT, false, true>(p, sh, st);
   return sh.mains == 0 ? launch_form<WINDOW, ACT, true, false>(p, sh, st) : launch_form<WINDOW, ACT, false, false>(p, sh, st);
