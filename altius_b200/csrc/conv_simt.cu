@@ -13,14 +13,21 @@
 // or written as a column buffer first: planes of any size and filters with a window (their
 // addresses come from a table in shared memory) take the same loop.
 //
-// Shape: a group of 128 threads (8 x 16) owns a tile of 8 TM output channels x 64 columns, TM x 4
-// in registers. A block has four such groups, which share the tile and take interleaved slices of
-// every K step of 32; a cluster of up to eight blocks shares the tile in the same way over ranges
-// of K. Partial sums meet in (distributed) shared memory in a fixed order, so results do not
-// depend on timing. Operands arrive by cp.async in a ring of four stages; the filter's part of
-// the first stages is requested before the kernel in front has finished.
+// Shape: a tile is 16 output channels x 64 columns. Each of a block's eight warps holds all of it in registers (4 x 8 a
+// thread) and takes four rows of every K step of 32, loaded by itself: no barrier between loads and sums. A
+// cluster of up to eight blocks shares the tile over ranges of K. Partial sums meet in (distributed)
+// shared memory in a fixed order, so results do not depend on timing; the blocks of a cluster send
+// theirs with stores that count on the receiver's mbarrier. The filter's part of the first stages is
+// requested, and the code run once without effect, before the kernel in front has finished.
+//
+// Measured, per launch in a MobileNetV3-Large at batch one, from the end of the kernel in front: 40 -> 120 at 28 x 28 4.8 us
+// -> 3.1; 672 -> 112 at 14 x 14 with a gate 10.7 -> 6.1; 960 -> 160 at 7 x 7 with a gate 12.7 -> 5.2. Before that: four groups of 128
+// threads on 2 x 4 results each with a barrier of the block in every K step (1100 clocks a step against 800: shared memory
+// hands a warp 128 bytes a clock, so the bytes loaded per product count), planes by 4-byte cp.async, the gate fetched one step
+// ahead, remote partial sums read block by block, the residual behind them.
 #include <cooperative_groups.h>
 
+#include "cluster_send.cuh"
 #include "kernels.h"
 #include "pdl.cuh"
 #include "ref_math.cuh"
@@ -30,7 +37,6 @@ namespace cg = cooperative_groups;
 namespace ac {
 namespace {
 
-constexpr int GROUP = 128;
 enum Load { LOAD_VEC = 0, LOAD_SCALAR, LOAD_WINDOW };
 
 struct ConvDev {
@@ -46,34 +52,23 @@ struct ConvDev {
   int act;
   float act_alpha, act_beta;
   int kper;                 // K steps per block of the cluster
-  int early;                // the filter is a constant: read ahead of pdl_wait
+  int early;                // the filter and the bias are constants: read ahead of pdl_wait
+  int cold;                 // nothing runs in front: no pass ahead of the first
+  int* err;
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-// Copies 16 / 4 bytes, or writes zeros when !ok (the source is then not read).
+// Copies 16 bytes, or writes zeros when !ok (the source is then not read).
 __device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
   const int n = ok ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp4(float* dst, const float* src, bool ok) {
-  const int n = ok ? 4 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// A thread's TM rows are neighbours (TM 2 or 4): one aligned load.
-template <int TM>
-__device__ __forceinline__ void load_a(const float* row, int ty, float (&a)[TM]) {
-  static_assert(TM == 2 || TM == 4, "rows per thread");
-  if (TM == 4) {
-    const float4 v = *reinterpret_cast<const float4*>(row + ty * 4);
-    a[0] = v.x; a[1] = v.y; a[TM - 2] = v.z; a[TM - 1] = v.w;
-  } else {
-    const float2 v = *reinterpret_cast<const float2*>(row + ty * 2);
-    a[0] = v.x; a[1] = v.y;
-  }
+__device__ __forceinline__ void add4(float4& s, float4 v) {
+  s.x = __fadd_rn(s.x, v.x); s.y = __fadd_rn(s.y, v.y); s.z = __fadd_rn(s.z, v.z); s.w = __fadd_rn(s.w, v.w);
 }
 
 __device__ __forceinline__ float finish(const ConvDev& p, float v, float bias) {
@@ -84,224 +79,281 @@ __device__ __forceinline__ float finish(const ConvDev& p, float v, float bias) {
   return apply_act(p.act, v, p.act_alpha, p.act_beta);
 }
 
-// Four neighbouring columns of one output row.
+// Four neighbouring columns of one output row: where they lie, and what is added behind the activation.
 template <int LOAD>
-__device__ __forceinline__ void store_quad(const ConvDev& p, int row, int col, float4 v) {
-  if (row >= p.m || col >= p.n) return;
-  const float bias = p.bias ? ld_plain(p.bias + row) : 0.f;
-  v.x = finish(p, v.x, bias); v.y = finish(p, v.y, bias); v.z = finish(p, v.z, bias); v.w = finish(p, v.w, bias);
-  if (LOAD == LOAD_VEC) {   // planes are whole float4s: the four columns lie in one image
-    const int b = col / p.hw;
-    const long long at = b * p.out_batch + (long long)row * p.hw + (col - b * p.hw);
-    if (p.res) {
-      const float4 r = *reinterpret_cast<const float4*>(p.res + at);
-      v.x = __fadd_rn(v.x, r.x); v.y = __fadd_rn(v.y, r.y); v.z = __fadd_rn(v.z, r.z); v.w = __fadd_rn(v.w, r.w);
-    }
-    *reinterpret_cast<float4*>(p.out + at) = v;
-    return;
-  }
-  const float e[4] = {v.x, v.y, v.z, v.w};
-  int b = col / p.hw, px = col - b * p.hw;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (col + j >= p.n) return;
-    const long long at = b * p.out_batch + (long long)row * p.hw + px;
-    p.out[at] = p.res ? __fadd_rn(e[j], p.res[at]) : e[j];
-    if (++px == p.hw) { px = 0; ++b; }
-  }
-}
+struct Quad {
+  long long at = 0;
+  int live = 0;                            // columns that exist; LOAD_VEC: planes are whole float4s, all four or none
+  int left = 0;                            // pixels up to the end of the first column's plane
+  float res[4] = {0.f, 0.f, 0.f, 0.f};
+  float bias = 0.f;
 
-constexpr int TN = 4, WK = 4;
-constexpr int BN = 16 * TN, BK = 32, T = GROUP * WK, S = 4;
-template <int TM>
-struct Cfg {
-  static constexpr int BM = 8 * TM;
-  static constexpr int STAGE = BK * (BM + BN);                 // floats
-  static constexpr int QUADS = TM * TN / 4;                    // float4s of results per thread
-  static constexpr int PARTS = WK * GROUP * TM * TN;           // floats of partial sums
-  static constexpr int FLOATS = S * STAGE > PARTS ? S * STAGE : PARTS;
+  __device__ __forceinline__ void place(const ConvDev& p, bool mine, int row, int col) {
+    if (!mine || row >= p.m || col >= p.n) return;
+    const int b = col / p.hw, px = col - b * p.hw;
+    at = b * p.out_batch + (long long)row * p.hw + px;
+    live = LOAD == LOAD_VEC ? 4 : min(4, p.n - col);
+    left = p.hw - px;
+    if (p.bias) bias = ld_plain(p.bias + row);
+  }
+  // The j-th column's element; the last pixel of an image's plane is followed by the next image's first.
+  template <typename F>
+  __device__ __forceinline__ void each(const ConvDev& p, F f) const {
+    long long a = at;
+    int l = left;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (j < live) f(j, a);
+      ++a;
+      if (--l == 0) { l = p.hw; a += p.out_batch - p.hw; }
+    }
+  }
+  __device__ __forceinline__ void fetch(const ConvDev& p) {
+    if (!p.res) return;
+    if (LOAD == LOAD_VEC) {
+      if (!live) return;
+      const float4 r = *reinterpret_cast<const float4*>(p.res + at);
+      res[0] = r.x; res[1] = r.y; res[2] = r.z; res[3] = r.w;
+    } else {
+      each(p, [&](int j, long long a) { res[j] = p.res[a]; });
+    }
+  }
+  __device__ __forceinline__ void store(const ConvDev& p, float4 v, bool now) const {
+    float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      e[j] = finish(p, e[j], bias);
+      if (p.res) e[j] = __fadd_rn(e[j], res[j]);
+    }
+    if (!now) return;
+    if (LOAD == LOAD_VEC) {
+      if (live) *reinterpret_cast<float4*>(p.out + at) = make_float4(e[0], e[1], e[2], e[3]);
+    } else {
+      each(p, [&](int j, long long a) { p.out[a] = e[j]; });
+    }
+  }
 };
 
-template <int TM, int LOAD>
-__global__ void __launch_bounds__(T) conv_simt_kernel(const ConvDev p) {
-  using C = Cfg<TM>;
-  constexpr int BM = C::BM, QUADS = C::QUADS;
+constexpr int BM = 16, BN = 64, BK = 32, WARPS = 8, T = 32 * WARPS, KW = BK / WARPS, S = 4;
+constexpr int SLICE = KW * (BM + BN);                      // floats: a warp's rows of a K step
+constexpr int QUADS = BM * BN / 4;                         // float4s of the tile
+constexpr int RING = WARPS * S * SLICE, PARTS = WARPS * QUADS * 4;
+constexpr int FLOATS = (RING > PARTS ? RING : PARTS) + QUADS * 4;
+static_assert(QUADS == T, "a thread adds one float4 of the result up");
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+template <int LOAD>
+__global__ void __launch_bounds__(T, 2) conv_simt_kernel(const ConvDev p) {
   extern __shared__ __align__(16) float smem[];
-  const int tid = threadIdx.x, g = tid / GROUP, t = tid % GROUP, lane = t & 31, warp = t >> 5;
-  // A warp covers 4 x 8 threads of the group's 8 x 16: one wavefront per shared-memory load.
-  const int ty = (warp >> 1) * 4 + (lane >> 3), tx = (warp & 1) * 8 + (lane & 7);
+  __shared__ __align__(8) uint64_t sent;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ty = lane >> 3, tx = lane & 7;          // 4 rows x (2 x 4) columns a thread, the tile a warp
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int nkt = (p.k + BK - 1) / BK;
   const int kt0 = blockIdx.z * p.kper, kt1 = min(nkt, kt0 + p.kper), kts = kt1 - kt0;
+  const int parts = gridDim.z, rank = blockIdx.z;   // blocks of the cluster
+  const int share = QUADS / parts;                  // float4s of the result that a block finishes
 
   // k -> (offset of the tap inside an image, its row and column) for filters with a window.
-  int2* tab = reinterpret_cast<int2*>(smem + C::FLOATS);
+  int2* tab = reinterpret_cast<int2*>(smem + FLOATS);
   if (LOAD == LOAD_WINDOW) {
     const int taps = p.kh * p.kw;
     for (int k = tid; k < p.k; k += T) {
       const int c = k / taps, r = k - c * taps, fy = r / p.kw * p.dh, fx = (r % p.kw) * p.dw;
       tab[k] = make_int2(c * p.ih * p.iw + fy * p.iw + fx, fy << 16 | fx);
     }
-    __syncthreads();
   }
+  if (tid == 0 && parts > 1) {
+    tc::mbar_init(&sent, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tc::mbar_arrive_expect_tx(&sent, (uint32_t)(parts * share * 16));
+  }
+  __syncthreads();
   pdl_trigger();
+  cg::cluster_group cl = cg::this_cluster();
+  if (parts > 1) cl.barrier_arrive();
 
-  // The column(s) this thread loads are the same in every K step.
-  constexpr int CPR = LOAD == LOAD_VEC ? BN / 4 : BN, RPP = T / CPR, ROWS = BK / RPP;   // columns a row, rows a pass
-  static_assert(T % CPR == 0 && BK % RPP == 0, "loader shape");
-  const int lc = tid % CPR, lr = tid / CPR;
-  const int col = n0 + (LOAD == LOAD_VEC ? 4 * lc : lc);
-  const bool col_ok = col < p.n;
-  const int cb = col_ok ? col / p.hw : 0, px = col_ok ? col - cb * p.hw : 0;
-  const float* xcol = p.x + cb * p.x_batch;
-  int iy0 = 0, ix0 = 0;
-  if (LOAD == LOAD_WINDOW) {
-    const int oy = px / p.ow;
-    iy0 = oy * p.sh - p.pt;
-    ix0 = (px - oy * p.ow) * p.sw - p.pl;
-    xcol += (long long)iy0 * p.iw + ix0;
-  } else {
-    xcol += px;
+  // The column(s) this lane loads are the same in every row: one float4 of every second row, or columns lane and lane + 32.
+  constexpr int COLS = LOAD == LOAD_VEC ? 1 : 2, ROWS = LOAD == LOAD_VEC ? KW / 2 : KW, FL = LOAD == LOAD_VEC ? 4 : 1;
+  const int lr = LOAD == LOAD_VEC ? lane >> 4 : 0, lc = LOAD == LOAD_VEC ? (lane & 15) * 4 : lane;
+  constexpr int RSTEP = LOAD == LOAD_VEC ? 2 : 1;
+  const float *xcol[COLS], *gcol[COLS];
+  int iy0[COLS], ix0[COLS];
+  bool col_ok[COLS];
+#pragma unroll
+  for (int c = 0; c < COLS; ++c) {
+    const int col = n0 + lc + 32 * c;
+    col_ok[c] = col < p.n;
+    const int b = col_ok[c] ? col / p.hw : 0, px = col_ok[c] ? col - b * p.hw : 0;
+    xcol[c] = p.x + b * p.x_batch;
+    iy0[c] = ix0[c] = 0;
+    if (LOAD == LOAD_WINDOW) {
+      const int oy = px / p.ow;
+      iy0[c] = oy * p.sh - p.pt;
+      ix0[c] = (px - oy * p.ow) * p.sw - p.pl;
+      xcol[c] += (long long)iy0[c] * p.iw + ix0[c];
+    } else {
+      xcol[c] += px;
+    }
+    gcol[c] = p.gate ? p.gate + (long long)b * p.k : nullptr;
   }
-  const float* gcol = p.gate ? p.gate + (long long)cb * p.k : nullptr;
 
+  // Everything a warp multiplies it has loaded itself: rows [4 warp, 4 warp + 4) of every K step, so no barrier of
+  // the block stands between the loads and the sums.
+  float* mine = smem + warp * (S * SLICE);
   auto load_w = [&](int s, int kt) {
-    float* As = smem + s * C::STAGE;
-    const int k0 = kt * BK;
-#pragma unroll
-    for (int i = tid; i < BK * (BM / 4); i += T) {
-      const int r = i / (BM / 4), c4 = (i % (BM / 4)) * 4;
-      const bool ok = k0 + r < p.k && m0 + c4 < p.ldw;
-      cp16(As + r * BM + c4, ok ? p.wt + (long long)(k0 + r) * p.ldw + m0 + c4 : p.wt, ok);
+    const int r = lane >> 2, c4 = (lane & 3) * 4, k = kt * BK + warp * KW + r;
+    if (lane < KW * (BM / 4)) {
+      const bool ok = k < p.k && m0 + c4 < p.ldw;
+      cp16(mine + s * SLICE + r * BM + c4, ok ? p.wt + (long long)k * p.ldw + m0 + c4 : p.wt, ok);
     }
   };
-  auto load_x = [&](int s, int kt) {
-    float* Bs = smem + s * C::STAGE + BK * BM;
-    const int k0 = kt * BK;
+  // The planes' part of a K step goes through registers: a warp's cp.async of 4 bytes a lane took 15 clocks of the SM to
+  // issue whatever its width, 24 of them in front of the first step 5600 clocks.
+  struct Piece { float x[ROWS][COLS][FL], gate[LOAD == LOAD_WINDOW ? 1 : ROWS][COLS]; };   // no gate with a window
+  auto fetch = [&](Piece& u, int kt, bool go) {
 #pragma unroll
-    for (int i = 0; i < ROWS; ++i) {
-      const int r = lr + i * RPP, k = k0 + r;
-      if (LOAD == LOAD_VEC) {
-        const bool ok = col_ok && k < p.k;
-        cp16(Bs + r * BN + 4 * lc, ok ? xcol + (long long)k * p.hw : p.x, ok);
-      } else if (LOAD == LOAD_SCALAR) {
-        const bool ok = col_ok && k < p.k;
-        cp4(Bs + r * BN + lc, ok ? xcol + (long long)k * p.hw : p.x, ok);
-      } else {
-        bool ok = col_ok && k < p.k;
-        const int2 e = ok ? tab[k] : make_int2(0, 0);
-        const int iy = iy0 + (e.y >> 16), ix = ix0 + (e.y & 0xffff);
-        ok = ok && (unsigned)iy < (unsigned)p.ih && (unsigned)ix < (unsigned)p.iw;
-        cp4(Bs + r * BN + lc, ok ? xcol + e.x : p.x, ok);
-      }
-    }
-  };
-  float gv[ROWS];                          // factors of the elements this thread loads next
-  auto fetch_gate = [&](int kt) {
+    for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-    for (int i = 0; i < ROWS; ++i) {
-      const int k = kt * BK + lr + i * RPP;
-      gv[i] = col_ok && k < p.k ? gcol[k] : 0.f;
-    }
-  };
-
-  if (!p.early) pdl_wait();                // packed by a step in front
-#pragma unroll
-  for (int s = 0; s < S - 1; ++s)
-    if (s < kts) load_w(s, kt0 + s);
-  pdl_wait();
-#pragma unroll
-  for (int s = 0; s < S - 1; ++s) {
-    if (s < kts) load_x(s, kt0 + s);
-    cp_commit();
-  }
-  if (p.gate && kts > 0) fetch_gate(kt0);
-
-  float acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-
-  for (int it = 0; it < kts; ++it) {
-    const int s = it % S;
-    cp_wait<S - 2>();
-    if (p.gate) {                          // own elements only: visible without a barrier
-      float* Bs = smem + s * C::STAGE + BK * BM;
-#pragma unroll
-      for (int i = 0; i < ROWS; ++i) {
-        float* e = Bs + (lr + i * RPP) * BN + (LOAD == LOAD_VEC ? 4 * lc : lc);
+      for (int c = 0; c < COLS; ++c) {
+        const int k = kt * BK + warp * KW + lr + i * RSTEP;
+        bool ok = go && col_ok[c] && k < p.k;
+        if (LOAD != LOAD_WINDOW) u.gate[i][c] = p.gate && ok ? gcol[c][k] : 1.f;
         if (LOAD == LOAD_VEC) {
-          float4 v = *reinterpret_cast<float4*>(e);
-          v.x = __fmul_rn(v.x, gv[i]); v.y = __fmul_rn(v.y, gv[i]); v.z = __fmul_rn(v.z, gv[i]); v.w = __fmul_rn(v.w, gv[i]);
-          *reinterpret_cast<float4*>(e) = v;
+          const float4 v = ok ? *reinterpret_cast<const float4*>(xcol[c] + (long long)k * p.hw) : make_float4(0.f, 0.f, 0.f, 0.f);
+          u.x[i][c][0] = v.x; u.x[i][c][FL > 1 ? 1 : 0] = v.y; u.x[i][c][FL > 1 ? 2 : 0] = v.z; u.x[i][c][FL > 1 ? 3 : 0] = v.w;
+        } else if (LOAD == LOAD_SCALAR) {
+          u.x[i][c][0] = ok ? xcol[c][(long long)k * p.hw] : 0.f;
         } else {
-          *e = __fmul_rn(*e, gv[i]);
+          const int2 e = ok ? tab[k] : make_int2(0, 0);
+          const int iy = iy0[c] + (e.y >> 16), ix = ix0[c] + (e.y & 0xffff);
+          ok = ok && (unsigned)iy < (unsigned)p.ih && (unsigned)ix < (unsigned)p.iw;
+          u.x[i][c][0] = ok ? xcol[c][e.x] : 0.f;
         }
       }
-      if (it + 1 < kts) fetch_gate(kt0 + it + 1);
-    }
-    __syncthreads();                       // stage s complete for all; stage of step it - 1 is free
-    if (it + S - 1 < kts) {
-      load_w((it + S - 1) % S, kt0 + it + S - 1);
-      load_x((it + S - 1) % S, kt0 + it + S - 1);
-    }
-    cp_commit();
-    const float* As = smem + s * C::STAGE + g * (BK / WK) * BM;
-    const float* Bs = smem + s * C::STAGE + BK * BM + g * (BK / WK) * BN;
+  };
+  auto put = [&](int s, const Piece& u) {
+    float* Bs = mine + s * SLICE + KW * BM;
 #pragma unroll
-    for (int kk = 0; kk < BK / WK; ++kk) {
-      float a[TM], b[TN];
-      load_a<TM>(As + kk * BM, ty, a);
-      const float4 v = *reinterpret_cast<const float4*>(Bs + kk * BN + tx * 4);
-      b[0] = v.x; b[1] = v.y; b[2] = v.z; b[3] = v.w;
+    for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+      for (int c = 0; c < COLS; ++c) {
+        float v[FL];
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-  }
-  cp_wait<0>();
+        for (int j = 0; j < FL; ++j)
+          v[j] = LOAD != LOAD_WINDOW && p.gate ? __fmul_rn(u.x[i][c][j], u.gate[LOAD == LOAD_WINDOW ? 0 : i][c]) : u.x[i][c][j];
+        float* at = Bs + (lr + i * RSTEP) * BN + lc + 32 * c;
+        if (LOAD == LOAD_VEC) *reinterpret_cast<float4*>(at) = make_float4(v[0], v[FL > 1 ? 1 : 0], v[FL > 1 ? 2 : 0], v[FL > 1 ? 3 : 0]);
+        else *at = v[0];
+      }
+  };
 
-  const int parts = gridDim.z;             // blocks of the cluster
-  // Partial sums: row i of thread t of group g at [(g * TM + i) * 128 + t].
-  float4* part = reinterpret_cast<float4*>(smem);
-  __syncthreads();
+  // Float4 e of the tile: row (e / 8 % 4) * 4 + e / 64, columns from e / 32 % 2 * 32 + e % 8 * 4.
+  Quad<LOAD> quad;                                                 // what this thread finishes
+  float4* part = reinterpret_cast<float4*>(smem);                  // [warps][QUADS], over the ring
+  float4* recv = reinterpret_cast<float4*>(smem + FLOATS) - QUADS; // [parts][share], written by the cluster's blocks
+
+  if (!p.early) pdl_wait();                // filter or bias come from a step in front
+#pragma unroll 1
+  for (int s = 0; s < S - 1; ++s)
+    if (s < kts) load_w(s, kt0 + s);
+  cp_commit();
+  {
+    const int e = rank * share + tid;
+    quad.place(p, tid < share, m0 + (e >> 3 & 3) * 4 + (e >> 6), n0 + (e >> 5 & 1) * 32 + (e & 7) * 4);
+  }
+
+  // The first pass reads and writes nothing outside the block: it brings the code into the instruction cache while
+  // the kernel in front still runs. One K step, of zeros.
+#pragma unroll 1
+  for (int pass = p.cold; pass < 2; ++pass) {
+    const bool now = pass == 1;
+    if (now) pdl_wait();
+    {
+      Piece u[S - 1];
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
-    part[(g * TM + i) * GROUP + t] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-  cg::cluster_group cl = cg::this_cluster();
-  if (parts > 1) cl.sync();
-  else __syncthreads();
-  // Each block of the cluster finishes its share of the quads.
-  const int share = QUADS * GROUP / parts, base = blockIdx.z * share;
-  for (int v = tid; v < share; v += T) {
-    const int e = base + v, q = e / GROUP, tt = e % GROUP;
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int r = 0; r < parts; ++r) {
-      const float4* src = parts > 1 ? cl.map_shared_rank(part, r) : part;
+      for (int s = 0; s < S - 1; ++s)
+        if (LOAD != LOAD_WINDOW || !now || s < kts) fetch(u[s], kt0 + s, now && s < kts);
+      if (now) quad.fetch(p);
 #pragma unroll
-      for (int w = 0; w < WK; ++w) {
-        const float4 u = src[w * QUADS * GROUP + e];
-        sum.x = __fadd_rn(sum.x, u.x); sum.y = __fadd_rn(sum.y, u.y);
-        sum.z = __fadd_rn(sum.z, u.z); sum.w = __fadd_rn(sum.w, u.w);
+      for (int s = 0; s < S - 1; ++s)
+        if (LOAD != LOAD_WINDOW || !now || s < kts) put(s, u[s]);
+    }
+
+    float2 acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
+
+    const int steps = now ? kts : 1;
+    for (int it = 0; it < steps; ++it) {
+      const int s = it % S;
+      if (it == 0) cp_wait<0>();           // the filter's part of the first stages
+      else cp_wait<S - 2>();
+      __syncwarp();                        // stage s complete for the warp; stage of step it - 1 is free
+      Piece u;
+      const bool more = now && it + S - 1 < kts;
+      if (more) load_w((it + S - 1) % S, kt0 + it + S - 1);
+      cp_commit();
+      fetch(u, kt0 + it + S - 1, more);
+      const float* As = mine + s * SLICE;
+      const float* Bs = As + KW * BM;
+#pragma unroll
+      for (int kk = 0; kk < KW; ++kk) {
+        const float4 a4 = *reinterpret_cast<const float4*>(As + kk * BM + ty * 4);
+        const float4 b0 = *reinterpret_cast<const float4*>(Bs + kk * BN + tx * 4);
+        const float4 b1 = *reinterpret_cast<const float4*>(Bs + kk * BN + 32 + tx * 4);
+        const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 aa = make_float2(a[i], a[i]);
+          acc[i][0] = fma2(aa, make_float2(b0.x, b0.y), acc[i][0]);
+          acc[i][1] = fma2(aa, make_float2(b0.z, b0.w), acc[i][1]);
+          acc[i][2] = fma2(aa, make_float2(b1.x, b1.y), acc[i][2]);
+          acc[i][3] = fma2(aa, make_float2(b1.z, b1.w), acc[i][3]);
+        }
+      }
+      if (more) put((it + S - 1) % S, u);
+    }
+
+    // The warps' sums, then the blocks': both in order. A block sends each other one its share.
+    __syncthreads();
+    if (now) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          part[warp * QUADS + (2 * i + h) * 32 + lane] = make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
+    }
+    __syncthreads();
+    float4 sum = part[tid];
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w) add4(sum, part[w * QUADS + tid]);
+    if (parts > 1) {
+      if (now) {
+        cl.barrier_wait();                 // every block of the cluster runs and has announced what it waits for
+        const int owner = tid / share;
+        send4(cluster_addr(recv + rank * share + tid - owner * share, owner), cluster_addr(&sent, owner), sum);
+        if (tid < share && !wait_sent(&sent, 0)) atomicExch(p.err, 71);
+      }
+      if (tid < share) {
+        sum = recv[tid];
+        for (int r = 1; r < parts; ++r) add4(sum, recv[r * share + tid]);
       }
     }
-    const int ll = tt & 31, ww = tt >> 5;
-    const int yy = (ww >> 1) * 4 + (ll >> 3), xx = (ww & 1) * 8 + (ll & 7);
-    store_quad<LOAD>(p, m0 + yy * TM + q, n0 + xx * 4, sum);
+    quad.store(p, sum, now);
   }
-  if (parts > 1) cl.sync();                // no block leaves while others read its sums
 }
 
-template <int TM, int LOAD>
+template <int LOAD>
 cudaError_t launch_one(const ConvDev& p, int split, cudaStream_t st) {
-  using C = Cfg<TM>;
   static unsigned long long done = 0;
-  const size_t smem = C::FLOATS * sizeof(float) + (LOAD == LOAD_WINDOW ? (size_t)p.k * sizeof(int2) : 0);
-  if (cudaError_t e = ensure_dynamic_smem(conv_simt_kernel<TM, LOAD>, 96 << 10, &done)) return e;
-  const dim3 grid((unsigned)((p.n + BN - 1) / BN), (unsigned)((p.m + C::BM - 1) / C::BM), (unsigned)split);
-  return launch_pdl(conv_simt_kernel<TM, LOAD>, grid, dim3(T), smem, st, split, p);
+  const size_t smem = FLOATS * sizeof(float) + (LOAD == LOAD_WINDOW ? (size_t)p.k * sizeof(int2) : 0);
+  if (cudaError_t e = ensure_dynamic_smem(conv_simt_kernel<LOAD>, 96 << 10, &done)) return e;
+  const dim3 grid((unsigned)((p.n + BN - 1) / BN), (unsigned)((p.m + BM - 1) / BM), (unsigned)split);
+  return launch_pdl(conv_simt_kernel<LOAD>, grid, dim3(T), smem, st, split, p);
 }
 
 __global__ void pack_filter_kernel(const float* __restrict__ w, float* __restrict__ wt, int m, int k, int ldw) {
@@ -329,7 +381,7 @@ bool conv_simt_supported(const ConvParams& q) {
 }
 
 cudaError_t launch_conv_simt(const ConvParams& q, const float* x, const float* wt, const float* bias, const float* gate,
-                             const float* residual, float* out, bool constants, cudaStream_t st) {
+                             const float* residual, float* out, bool constants, bool first, int* err_word, cudaStream_t st) {
   ConvDev p{};
   p.x = x; p.wt = wt; p.out = out; p.bias = bias; p.res = residual; p.gate = gate;
   p.ldw = (int)conv_simt_ldw(q.oc); p.m = q.oc; p.k = q.c * q.kh * q.kw; p.hw = q.oh * q.ow; p.n = q.n * p.hw;
@@ -338,24 +390,20 @@ cudaError_t launch_conv_simt(const ConvParams& q, const float* x, const float* w
   p.ih = q.ih; p.iw = q.iw; p.ow = q.ow; p.kh = q.kh; p.kw = q.kw; p.sh = q.sh; p.sw = q.sw; p.dh = q.dh; p.dw = q.dw;
   p.pt = q.pad_t; p.pl = q.pad_l;
   p.early = constants;
+  p.cold = first;
+  p.err = err_word;
   p.act = q.act; p.act_alpha = q.act_alpha; p.act_beta = q.act_beta;
   const bool window = q.kh != 1 || q.kw != 1 || q.sh != 1 || q.sw != 1 || q.pad_t || q.pad_l || q.oh != q.ih || q.ow != q.iw;
   if (window && gate) return cudaErrorInvalidValue;
   const bool vec = !window && (p.hw % 4) == 0 && al16(x) && al16(out) && (!residual || al16(residual));
-  // Tiles of 32 channels when they already give every SM one; else of 16, and K cut over the
-  // blocks of a cluster (at least one K step each) until the SMs have about one block each.
+  // K is cut over the blocks of a cluster (at least one K step each) until the SMs have about one block each.
   const int sms = device_sm_count(), nkt = (p.k + BK - 1) / BK;
-  auto tiles = [&](int bm) { return (long long)((p.n + BN - 1) / BN) * ((p.m + bm - 1) / bm); };
-  const bool tall = tiles(32) >= sms;
+  const long long tiles = (long long)((p.n + BN - 1) / BN) * ((p.m + BM - 1) / BM);
   int split = 1;
-  while (split < 8 && 2 * split <= nkt && 2 * split * tiles(tall ? 32 : 16) <= sms + sms / 4) split *= 2;
+  while (split < 8 && 2 * split <= nkt && 2 * split * tiles <= sms + sms / 4) split *= 2;
   p.kper = (nkt + split - 1) / split;
-  if (tall) {
-    if (window) return launch_one<4, LOAD_WINDOW>(p, split, st);
-    return vec ? launch_one<4, LOAD_VEC>(p, split, st) : launch_one<4, LOAD_SCALAR>(p, split, st);
-  }
-  if (window) return launch_one<2, LOAD_WINDOW>(p, split, st);
-  return vec ? launch_one<2, LOAD_VEC>(p, split, st) : launch_one<2, LOAD_SCALAR>(p, split, st);
+  if (window) return launch_one<LOAD_WINDOW>(p, split, st);
+  return vec ? launch_one<LOAD_VEC>(p, split, st) : launch_one<LOAD_SCALAR>(p, split, st);
 }
 
 }  // namespace ac

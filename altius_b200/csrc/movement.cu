@@ -2,16 +2,19 @@
 // Split, Gather, Concat pieces), batched 2-D transpose through shared memory,
 // im2col. Pure copies are bit-exact by construction.
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace ac {
 namespace {
 
 // compute_max_pool, crates/session_interpreter/src/session.rs:325-382:
 // f32::MIN start value; a window that saw no element yields 0.0.
-__global__ void max_pool_kernel(const float* __restrict__ x, float* __restrict__ out,
+__global__ void max_pool_kernel(const float* x, float* out,
                                 int64_t total, int ih, int iw, int oh, int ow, int kh, int kw,
                                 int sh, int sw, int pad_t, int pad_l) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (i >= total) return;
   const int ox = (int)(i % ow);
   const int oy = (int)((i / ow) % oh);
@@ -23,7 +26,7 @@ __global__ void max_pool_kernel(const float* __restrict__ x, float* __restrict__
   const int fy0 = max(-y0, 0), fy1 = min(kh, ih - y0);
   const int fx0 = max(-x0, 0), fx1 = min(kw, iw - x0);
   for (int fy = fy0; fy < fy1; ++fy)
-    for (int fx = fx0; fx < fx1; ++fx) m = fmaxf(__ldg(in + (y0 + fy) * iw + (x0 + fx)), m);
+    for (int fx = fx0; fx < fx1; ++fx) m = fmaxf(ld_plain(in + (y0 + fy) * iw + (x0 + fx)), m);
   out[i] = (m == FMIN) ? 0.0f : m;
 }
 
@@ -168,9 +171,8 @@ cudaError_t launch_max_pool(const float* x, float* out, int64_t planes, int ih, 
                             cudaStream_t st) {
   const int64_t total = planes * oh * ow;
   if (total == 0) return cudaSuccess;
-  max_pool_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(x, out, total, ih, iw, oh, ow,
-                                                                  kh, kw, sh, sw, pad_t, pad_l);
-  return cudaGetLastError();
+  return launch_pdl(max_pool_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st, 1, x, out, total, ih, iw, oh, ow, kh, kw, sh,
+                    sw, pad_t, pad_l);
 }
 
 cudaError_t launch_strided_copy(const CopyParams& q, const void* in, void* out, cudaStream_t st) {

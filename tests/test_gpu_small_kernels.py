@@ -57,6 +57,28 @@ def test_small_convolution(cuda_lib, n, c, h, oc, k, s, p, gate):
     assert (np.abs(got - want) <= (c * k * k + 8) * EPS * mass).all()
 
 
+# The same kernel behind another one, where it makes a pass over zeros ahead of its first: a block of the cluster
+# without a K step, K steps beyond the ring, tiles over many images, a single K step, a window.
+@pytest.mark.parametrize("n,c,h,oc,k,p,gate", [
+    (1, 160, 7, 80, 1, 0, True), (1, 2048, 5, 20, 1, 0, True), (1, 1600, 4, 33, 1, 0, True), (40, 36, 2, 17, 1, 0, False),
+    (33, 40, 3, 7, 1, 0, True), (1, 8, 14, 16, 5, 2, False), (3, 31, 6, 18, 3, 1, False)])
+def test_small_convolution_behind_a_kernel(cuda_lib, n, c, h, oc, k, p, gate):
+    rng = np.random.default_rng(c * h + oc)
+    x, gt, r = (rng.standard_normal(d).astype(np.float32) for d in ((n, c, h, h), (n, c, 1, 1), (n, oc, h, h)))
+    w, b = rng.standard_normal((oc, c, k, k)).astype(np.float32), rng.standard_normal(oc).astype(np.float32)
+
+    def build(g, xi, ri, gi=None):
+        xi = g.op("Sqrt", g.op("ReLU", xi))
+        return g.op("Add", g.op("ReLU", _conv(g, g.op("Mul", xi, gi) if gate else xi, w, b, k, 1, p)), ri)
+    got = _run(build, [x, r] + ([gt] if gate else []))
+    xs = np.sqrt(np.maximum(x, 0))
+    xg = torch.from_numpy(xs * gt if gate else xs).double()
+    conv = lambda a, f, bias: torch.nn.functional.conv2d(a, f, bias, padding=p)
+    want = torch.relu(conv(xg, torch.from_numpy(w).double(), torch.from_numpy(b).double())).numpy() + r
+    mass = conv(xg.abs(), torch.from_numpy(w).double().abs(), torch.from_numpy(b).double().abs()).numpy() + np.abs(r)
+    assert (np.abs(got - want) <= (c * k * k + 8) * EPS * mass).all()
+
+
 # one, two and three images per cluster, with a remainder; planes with and without whole float4s
 @pytest.mark.parametrize("n,c,h,s", [(1, 72, 28, 24), (3, 960, 7, 240), (19, 120, 14, 32), (41, 36, 5, 4), (1, 8, 1, 8)])
 def test_squeeze_excite_block(cuda_lib, n, c, h, s):
