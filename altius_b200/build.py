@@ -24,7 +24,7 @@ COMMON = (["-DAC_TC_BK=" + os.environ["AC_TC_BK"]] if "AC_TC_BK" in os.environ e
           "-Xcudafe", "--diag_suppress=177"]
 
 SOURCES = ["session.cu", "host_stage.cpp", "shapes.cpp", "lower.cpp", "eltwise.cu", "rowops.cu", "movement.cu",
-           "gemm_simt.cu", "gemm_rows.cu", "conv_simt.cu", "conv_tc.cu", "squeeze_excite.cu", "gemm_tc.cu", "gemm_ks.cu", "attention.cu", "attention_tc.cu", "attention_tc16.cu", "attention_flash16.cu", "noalloc.cu",
+           "gemm_simt.cu", "gemm_rows.cu", "conv_simt.cu", "conv_tc.cu", "squeeze_excite.cu", "depthwise_planes.cu", "gemm_tc.cu", "gemm_ks.cu", "attention.cu", "attention_tc.cu", "attention_tc16.cu", "attention_flash16.cu", "noalloc.cu",
            "model.cpp", "onnx_load.cpp", "passes.cpp"]
 
 

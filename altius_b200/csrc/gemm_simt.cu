@@ -14,6 +14,7 @@
 // with the next K step prefetched into registers during the math.
 #include "kernels.h"
 #include "pdl.cuh"
+#include "plane_means.cuh"
 #include "ref_math.cuh"
 
 namespace ac {
@@ -251,14 +252,15 @@ __global__ void __launch_bounds__(256) depthwise_kernel(const float* __restrict_
 // OFF >= 0: rows are whole float4s and x0 % 4 == OFF for every thread (it follows from the padding): the
 // segment comes as the aligned float4s around it, half as many requests of neighbouring threads
 // per line (32 x 64 planes of 112 x 112, stride 2: 28.5 us against 54.4); OFF < 0: any row, element by element.
-template <int K, int S, int ACT, int OFF>
+template <int K, int S, int ACT, int OFF, bool MEANS>
 __global__ void __launch_bounds__(256) depthwise_rows_kernel(const float* x,
                                                              const float* __restrict__ w,
                                                              const float* __restrict__ bias,
-                                                             float* out, ConvParams p,
-                                                             unsigned owg, unsigned items) {
-  const unsigned item = blockIdx.x * 256u + threadIdx.x;
-  const bool live = item < items;
+                                                             float* out, float* means, ConvParams p,
+                                                             unsigned owg, unsigned items, unsigned span) {
+  // `span` items a block: whole planes of them where means are asked for.
+  const unsigned item = blockIdx.x * (MEANS ? span : 256u) + threadIdx.x;
+  const bool live = (!MEANS || threadIdx.x < span) && item < items;
   const unsigned xg = item % owg, t = (live ? item : 0u) / owg;
   const unsigned oy = t % (unsigned)p.oh, plane = t / (unsigned)p.oh;   // plane = n * c + ch
   const int ch = (int)(plane % (unsigned)p.c);
@@ -269,7 +271,7 @@ __global__ void __launch_bounds__(256) depthwise_rows_kernel(const float* x,
   const float bv = bias ? __ldg(bias + ch) : 0.f;
   pdl_trigger();
   pdl_wait();
-  if (!live) return;
+  if (!MEANS && !live) return;
   constexpr int SEG = 3 * S + K;
   const int ox0 = (int)xg * 4;
   const int y0 = (int)oy * S - p.pad_t, x0 = ox0 * S - p.pad_l;
@@ -277,7 +279,7 @@ __global__ void __launch_bounds__(256) depthwise_rows_kernel(const float* x,
 #pragma unroll
   for (int fy = 0; fy < K; ++fy) {
     const int iy = y0 + fy;
-    if (iy < 0 || iy >= p.ih) continue;            // uniform per thread: all four pixels skip the row
+    if (iy < 0 || iy >= p.ih || (MEANS && !live)) continue;   // uniform per thread: all four pixels skip the row
     const float* row = in + iy * p.iw;
     float seg[SEG];
     if (OFF >= 0) {
@@ -315,34 +317,43 @@ __global__ void __launch_bounds__(256) depthwise_rows_kernel(const float* x,
     acc[o] = apply_act(ACT, acc[o], p.act_alpha, p.act_beta);
   }
   if (OFF >= 0 && (p.ow & 3) == 0) {
-    *reinterpret_cast<float4*>(dst) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    if (!MEANS || live) *reinterpret_cast<float4*>(dst) = make_float4(acc[0], acc[1], acc[2], acc[3]);
   } else {
 #pragma unroll
-    for (int o = 0; o < 4; ++o)
-      if (ox0 + o < p.ow) dst[o] = acc[o];
+    for (int o = 0; o < 4; ++o) {
+      if ((MEANS && !live) || ox0 + o >= p.ow) acc[o] = 0.f;
+      else dst[o] = acc[o];
+    }
   }
+  if (!MEANS) return;
+  __shared__ float sums[MEANS ? 256 : 1];
+  sums[threadIdx.x] = __fadd_rn(__fadd_rn(acc[0], acc[1]), __fadd_rn(acc[2], acc[3]));
+  __syncthreads();
+  const unsigned per_plane = owg * (unsigned)p.oh;
+  plane_means(sums, span / per_plane, per_plane, means, blockIdx.x * (span / per_plane), items / per_plane, p.oh * p.ow);
 }
 
 template <int K, int S, int OFF>
-bool launch_depthwise_rows(const ConvParams& p, const float* x, const float* w, const float* bias, float* out,
+bool launch_depthwise_rows(const ConvParams& p, const float* x, const float* w, const float* bias, float* out, float* means,
                            unsigned owg, unsigned items, int overlap, cudaError_t* e, cudaStream_t st) {
-  const dim3 blocks((items + 255u) / 256u), block(256);
+  const unsigned per_plane = owg * (unsigned)p.oh, span = means ? 256u / per_plane * per_plane : 256u;
+  const dim3 blocks((items + span - 1u) / span), block((span + 31u) / 32u * 32u);
   switch (p.act) {
-    case ACT_NONE: *e = launch_pdl(depthwise_rows_kernel<K, S, ACT_NONE, OFF>, blocks, block, 0, st, overlap, x, w, bias, out, p, owg, items); return true;
-    case ACT_RELU: *e = launch_pdl(depthwise_rows_kernel<K, S, ACT_RELU, OFF>, blocks, block, 0, st, overlap, x, w, bias, out, p, owg, items); return true;
-    case ACT_HARDSWISH: *e = launch_pdl(depthwise_rows_kernel<K, S, ACT_HARDSWISH, OFF>, blocks, block, 0, st, overlap, x, w, bias, out, p, owg, items); return true;
+    case ACT_NONE: *e = launch_pdl(means ? depthwise_rows_kernel<K, S, ACT_NONE, OFF, true> : depthwise_rows_kernel<K, S, ACT_NONE, OFF, false>, blocks, block, 0, st, overlap, x, w, bias, out, means, p, owg, items, span); return true;
+    case ACT_RELU: *e = launch_pdl(means ? depthwise_rows_kernel<K, S, ACT_RELU, OFF, true> : depthwise_rows_kernel<K, S, ACT_RELU, OFF, false>, blocks, block, 0, st, overlap, x, w, bias, out, means, p, owg, items, span); return true;
+    case ACT_HARDSWISH: *e = launch_pdl(means ? depthwise_rows_kernel<K, S, ACT_HARDSWISH, OFF, true> : depthwise_rows_kernel<K, S, ACT_HARDSWISH, OFF, false>, blocks, block, 0, st, overlap, x, w, bias, out, means, p, owg, items, span); return true;
     default: return false;
   }
 }
 
 // PA, PB: the paddings on the left that the vector form exists for.
 template <int K, int S, int PA, int PB>
-bool launch_depthwise_shape(const ConvParams& p, const float* x, const float* w, const float* bias, float* out,
+bool launch_depthwise_shape(const ConvParams& p, const float* x, const float* w, const float* bias, float* out, float* means,
                             unsigned owg, unsigned items, int overlap, cudaError_t* e, cudaStream_t st) {
   const bool vec = (p.iw % 4) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  if (vec && p.pad_l == PA) return launch_depthwise_rows<K, S, (4 - PA) % 4>(p, x, w, bias, out, owg, items, overlap, e, st);
-  if (vec && p.pad_l == PB) return launch_depthwise_rows<K, S, (4 - PB) % 4>(p, x, w, bias, out, owg, items, overlap, e, st);
-  return launch_depthwise_rows<K, S, -1>(p, x, w, bias, out, owg, items, overlap, e, st);
+  if (vec && p.pad_l == PA) return launch_depthwise_rows<K, S, (4 - PA) % 4>(p, x, w, bias, out, means, owg, items, overlap, e, st);
+  if (vec && p.pad_l == PB) return launch_depthwise_rows<K, S, (4 - PB) % 4>(p, x, w, bias, out, means, owg, items, overlap, e, st);
+  return launch_depthwise_rows<K, S, -1>(p, x, w, bias, out, means, owg, items, overlap, e, st);
 }
 
 inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
@@ -370,20 +381,42 @@ cudaError_t launch_gemm_simt(const GemmParams& q, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_depthwise_conv(const ConvParams& p, const float* x, const float* w,
-                                  const float* bias, float* out, bool constants, cudaStream_t st) {
+// The shapes that the rows kernel takes.
+static bool depthwise_rows_ok(const ConvParams& p) {
+  return p.kh == p.kw && p.sh == p.sw && p.dh == 1 && p.dw == 1 && (p.kh == 3 || p.kh == 5) && (p.sh == 1 || p.sh == 2) &&
+         (long long)p.n * p.oc * p.oh * ((p.ow + 3) / 4) < (1ll << 31) && (long long)p.ih * p.iw < (1ll << 31) &&
+         (p.act == ACT_NONE || p.act == ACT_RELU || p.act == ACT_HARDSWISH);
+}
+
+// Planes in shared memory (depthwise_planes.cu) for rows that are no whole float4s: a load per value here (32 images, 960
+// planes of 7 x 7, 5 x 5: 14.1 us against 9.2, 672 of 14 x 14, 3 x 3: 18.2 against 12.5; one image within 3 %). With whole
+// float4s, and at stride two, the rows kernel is the faster one (32 images, 240 of 28 x 28, 3 x 3, stride two: 7.3 against 9.3).
+static bool depthwise_planes_wins(const ConvParams& p) { return (p.iw & 3) && depthwise_planes_supported(p); }
+
+// The rows kernel's blocks add their planes up behind a barrier, which costs more than the squeeze-and-excite block saves once the
+// blocks take several rounds (120 planes of 28 x 28, 5 x 5, then the squeeze: 32 images 16.1 + 9.0 us -> 22.0 + 6.1; 13 of
+// 24 x 24: 6.2 + 8.2 -> 7.8 + 5.2).
+bool depthwise_conv_pools(const ConvParams& p) {
+  const long long per_plane = (long long)p.oh * ((p.ow + 3) / 4);
+  return depthwise_rows_ok(p) && per_plane >= 1 && per_plane <= 256 &&
+         (depthwise_planes_wins(p) || (long long)p.n * p.oc * per_plane <= 2048ll * device_sm_count());
+}
+
+cudaError_t launch_depthwise_conv(const ConvParams& p, const float* x, const float* w, const float* bias, float* out, float* means,
+                                  bool constants, cudaStream_t st) {
   const long long total = (long long)p.n * p.oc * p.oh * p.ow;
   if (total == 0) return cudaSuccess;
+  if (means && !depthwise_conv_pools(p)) return cudaErrorInvalidValue;
+  if (depthwise_planes_wins(p) && al16(x)) return launch_depthwise_planes(p, x, w, bias, out, means, constants, st);
   const long long owg = (p.ow + 3) / 4, items = (long long)p.n * p.oc * p.oh * owg;
-  if (p.kh == p.kw && p.sh == p.sw && p.dh == 1 && p.dw == 1 && items < (1ll << 31) &&
-      (long long)p.ih * p.iw < (1ll << 31)) {
+  if (depthwise_rows_ok(p)) {
     bool done = false;
     cudaError_t e = cudaSuccess;
     const int overlap = constants ? 1 : 0;
-    if (p.kh == 3 && p.sh == 1) done = launch_depthwise_shape<3, 1, 0, 1>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, overlap, &e, st);
-    else if (p.kh == 3 && p.sh == 2) done = launch_depthwise_shape<3, 2, 0, 1>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, overlap, &e, st);
-    else if (p.kh == 5 && p.sh == 1) done = launch_depthwise_shape<5, 1, 1, 2>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, overlap, &e, st);
-    else if (p.kh == 5 && p.sh == 2) done = launch_depthwise_shape<5, 2, 1, 2>(p, x, w, bias, out, (unsigned)owg, (unsigned)items, overlap, &e, st);
+    if (p.kh == 3 && p.sh == 1) done = launch_depthwise_shape<3, 1, 0, 1>(p, x, w, bias, out, means, (unsigned)owg, (unsigned)items, overlap, &e, st);
+    else if (p.kh == 3 && p.sh == 2) done = launch_depthwise_shape<3, 2, 0, 1>(p, x, w, bias, out, means, (unsigned)owg, (unsigned)items, overlap, &e, st);
+    else if (p.kh == 5 && p.sh == 1) done = launch_depthwise_shape<5, 1, 1, 2>(p, x, w, bias, out, means, (unsigned)owg, (unsigned)items, overlap, &e, st);
+    else if (p.kh == 5 && p.sh == 2) done = launch_depthwise_shape<5, 2, 1, 2>(p, x, w, bias, out, means, (unsigned)owg, (unsigned)items, overlap, &e, st);
     if (done) return e;
   }
   depthwise_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(x, w, bias, out, p, total);

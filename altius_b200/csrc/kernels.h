@@ -175,9 +175,15 @@ cudaError_t launch_im2col(const ConvParams& p, const float* x, float* col, cudaS
 // Non-overlapping patches (kernel == stride, no padding): rows[n * oh * ow, c * kh * kw] <- x,
 // one row per patch with the (c, fy, fx) order of the weight's K axis. kw % 4 == 0.
 cudaError_t launch_patchify(const ConvParams& p, const float* x, float* rows, cudaStream_t st);
-// Depthwise (group == c == oc) stencil with bias and activation fused.
-cudaError_t launch_depthwise_conv(const ConvParams& p, const float* x, const float* w,
-                                  const float* bias, float* out, bool constants, cudaStream_t st);
+// Depthwise (group == c == oc) stencil with bias and activation fused. `means`: [n][c] means of the resulting planes, written
+// too where depthwise_conv_pools says so, or null.
+bool depthwise_conv_pools(const ConvParams& p);
+cudaError_t launch_depthwise_conv(const ConvParams& p, const float* x, const float* w, const float* bias, float* out, float* means,
+                                  bool constants, cudaStream_t st);
+// The same over whole planes in shared memory (depthwise_planes.cu), stride 1; x 16-byte aligned.
+bool depthwise_planes_supported(const ConvParams& p);
+cudaError_t launch_depthwise_planes(const ConvParams& p, const float* x, const float* w, const float* bias, float* out, float* means,
+                                    bool constants, cudaStream_t st);
 
 // Small convolutions (group 1) on the CUDA cores without a column buffer (conv_simt.cu). `wt` is the
 // filter matrix transposed by launch_pack_filter: [k][conv_simt_ldw(oc)]. `gate`: [n][c] factors of
@@ -200,6 +206,7 @@ cudaError_t launch_conv_tc(const ConvParams& p, const float* x, const float* pac
 //   gate[n, :] = act2(W2 * act1(W1 * mean(x[n, :, plane]) + b1) + b2),  W1 [s, c], W2 [c, s].
 struct SqueezeExciteParams {
   const float* x;
+  const float* mean;                  // mean(x) where the kernel in front has made it, or null
   const float* w1; const float* b1;   // biases may be null
   const float* w2; const float* b2;
   float* gate;
@@ -207,6 +214,7 @@ struct SqueezeExciteParams {
   int64_t hw;
   int act1, act2;
   float alpha1, beta1, alpha2, beta2;
+  int* err;
 };
 bool squeeze_excite_supported(const SqueezeExciteParams& p);
 cudaError_t launch_squeeze_excite(const SqueezeExciteParams& p, cudaStream_t st);

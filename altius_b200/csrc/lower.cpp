@@ -115,6 +115,7 @@ struct Plan {
   std::map<int, SeGate> se_gate;    // pointwise Conv2d node -> squeeze-excite Mul folded into its input
   struct Squeeze { int conv1, conv2, b1, b2, act1, act2, out; float alpha1, beta1, alpha2, beta2; };
   std::map<int, Squeeze> squeeze;   // GlobalAveragePool node -> the two 1 x 1 convolutions behind it
+  std::map<int, int> means;         // value that a squeeze-excite block pools -> its planes' means once a kernel writes them, or -1
 };
 
 // gemm_mode 1 promises exact ascending chains and 2 its own precision: both keep their kernels.
@@ -608,6 +609,7 @@ void detect_squeeze(Ctx& c, Plan& plan) {
     if (c.val(c.node(q.conv2).inputs[1]).dims[0] != p.c || c.val(n.inputs[0]).is_const || !squeeze_excite_supported(p)) continue;
     c.absorbed[q.conv1] = c.absorbed[q.conv2] = 1;
     plan.squeeze[nid] = q;
+    plan.means[n.inputs[0]] = -1;
   }
 }
 
@@ -1144,7 +1146,7 @@ void lower_gemm(Emit& em, int nid, const Epilogue* e) {
   emit_gemm(em, n.op, g, a, b, out, c_in, bias_n, -1, alpha, beta, beta, e);
 }
 
-void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate = nullptr) {
+void lower_conv(Emit& em, Plan& plan, int nid, const Epilogue* e, const Plan::SeGate* gate = nullptr) {
   Node& n = em.c.node(nid);
   AcSession* s = em.s;
   // With a folded squeeze-excite gate the convolution reads the un-gated planes.
@@ -1220,10 +1222,15 @@ void lower_conv(Emit& em, int nid, const Epilogue* e, const Plan::SeGate* gate =
 
   if (p.group == p.c && icg == 1 && ocg == 1 && ep.residual < 0) {  // depthwise stencil
     const double bytes = f32_bytes(xv) + f32_bytes(wv) + f32_bytes(ov);
-    em.add("conv_depthwise", n.op, {x, w, bias}, {out}, bytes, flops, [=](cudaStream_t st) {
-      return launch_depthwise_conv(p, s->fptr(x), s->fptr(w), bias >= 0 ? s->fptr(bias) : nullptr,
-                                   s->fptr_mut(out), constants, st);
-    });
+    // A squeeze-excite block behind it starts from the means of the planes that this kernel has in hand.
+    int means = -1;
+    if (auto m = plan.means.find(out); m != plan.means.end() && depthwise_conv_pools(p))
+      m->second = means = new_value(em.c, (int64_t)p.n * p.c, false);
+    em.add("conv_depthwise", n.op, {x, w, bias}, means >= 0 ? std::vector<int>{out, means} : std::vector<int>{out}, bytes, flops,
+           [=](cudaStream_t st) {
+             return launch_depthwise_conv(p, s->fptr(x), s->fptr(w), bias >= 0 ? s->fptr(bias) : nullptr, s->fptr_mut(out),
+                                          means >= 0 ? s->fptr_mut(means) : nullptr, constants, st);
+           });
     return;
   }
   // GEMM form: out[n] (ocg x ohw) = W_g (ocg x k) * col[n, g] (k x ohw), bias per row.
@@ -1744,10 +1751,13 @@ void lower_node(Emit& em, Plan& plan, int nid) {
         const Plan::Squeeze q = sq->second;
         const int w1 = c.node(q.conv1).inputs[1], w2 = c.node(q.conv2).inputs[1];
         const int64_t ch = xv.dims[1], hid = V(w1).dims[0], nb = xv.dims[0];
-        const double bytes = f32_bytes(xv) + f32_bytes(V(w1)) + f32_bytes(V(w2)) + 4.0 * planes;
-        em.add("squeeze_excite", n.op, {x, w1, q.b1, w2, q.b2}, {q.out}, bytes, 4.0 * nb * ch * hid, [=](cudaStream_t st) {
+        const int mean = plan.means[x];
+        const double bytes = (mean >= 0 ? 4.0 * planes : f32_bytes(xv)) + f32_bytes(V(w1)) + f32_bytes(V(w2)) + 4.0 * planes;
+        em.add("squeeze_excite", n.op, {mean >= 0 ? mean : x, w1, q.b1, w2, q.b2}, {q.out}, bytes, 4.0 * nb * ch * hid, [=](cudaStream_t st) {
           SqueezeExciteParams p{};
           p.x = s->fptr(x);
+          p.mean = mean >= 0 ? s->fptr(mean) : nullptr;
+          p.err = s->err_word;
           p.w1 = s->fptr(w1); p.b1 = q.b1 >= 0 ? s->fptr(q.b1) : nullptr;
           p.w2 = s->fptr(w2); p.b2 = q.b2 >= 0 ? s->fptr(q.b2) : nullptr;
           p.gate = s->fptr_mut(q.out);
@@ -1916,7 +1926,7 @@ void lower_node(Emit& em, Plan& plan, int nid) {
     case AC_OP_CONV2D: {
       auto it = plan.epi.find(nid);
       auto sg = plan.se_gate.find(nid);
-      return lower_conv(em, nid, it == plan.epi.end() ? nullptr : &it->second,
+      return lower_conv(em, plan, nid, it == plan.epi.end() ? nullptr : &it->second,
                         sg == plan.se_gate.end() ? nullptr : &sg->second);
     }
     default:

@@ -102,6 +102,53 @@ def test_squeeze_excite_block(cuda_lib, n, c, h, s):
     assert (np.abs(got - np.clip(0.2 * z + 0.5, 0, 1)) <= 0.2 * e_z + 4 * EPS).all()
 
 
+# Depthwise convolution, activation, squeeze-and-excite block: means from the convolution's kernel (rows of whole float4s
+# and others, several planes a block with a remainder, stride two, one image and clusters of two) or, where its planes
+# are too large for that, from the block itself. The convolution's own result is held to its taps' rounding.
+@pytest.mark.parametrize("n,c,h,k,st,s,pooled", [
+    (1, 72, 28, 5, 2, 24, True), (2, 120, 28, 5, 1, 32, True), (3, 36, 7, 5, 1, 12, True), (19, 40, 14, 3, 1, 8, True),
+    (1, 44, 9, 3, 1, 4, True), (2, 24, 14, 5, 2, 8, True), (1, 8, 5, 5, 1, 8, True), (1, 16, 40, 3, 1, 8, False), (2, 12, 61, 3, 1, 4, False)])
+@pytest.mark.parametrize("act", ["ReLU", "HardSwish"])
+def test_depthwise_in_front_of_squeeze_excite(cuda_lib, n, c, h, k, st, s, pooled, act):
+    rng = np.random.default_rng(c + h)
+    x = rng.standard_normal((n, c, h, h)).astype(np.float32)
+    f, fb = rng.standard_normal((c, 1, k, k)).astype(np.float32), rng.standard_normal(c).astype(np.float32)
+    w1, w2 = (rng.standard_normal(d).astype(np.float32) / 4 for d in ((s, c, 1, 1), (c, s, 1, 1)))
+    b1, b2 = rng.standard_normal(s).astype(np.float32), rng.standard_normal(c).astype(np.float32)
+    g = ir.Graph()
+    y = g.op("Conv2d", g.add_input("x", x.shape), g.new_init(f), g.new_init(fb), kernel_shape=[k, k], strides=[st, st],
+             padding=[k // 2] * 4, dilations=[1, 1], group=c, auto_pad="")
+    y = g.op("Mul", y, g.op("HardSigmoid", y)) if act == "HardSwish" else g.op(act, y)
+    z = g.op("ReLU", _conv(g, g.op("GlobalAveragePool", y), w1, b1))
+    g.outputs += [y, g.op("HardSigmoid", _conv(g, z, w2, b2), alpha=0.2, beta=0.5)]
+    sess = CudaSessionBuilder(ir.Model(g, 13)).build()
+    try:
+        plan = sess.schedule()
+        assert [e["kind"] for e in plan] == ["conv_depthwise", "squeeze_excite"]
+        planes = 4.0 * n * c * ((h - 1) // st + 1) ** 2
+        assert (plan[1]["bytes"] < planes + 4 * (2 * c * s)) == pooled
+        got_y, got = sess.run([x])
+    finally:
+        sess.close()
+    conv = lambda a, b: torch.nn.functional.conv2d(torch.from_numpy(a).double(), torch.from_numpy(b).double(), None, stride=st, padding=k // 2,
+                                                   groups=c).numpy()
+    y64 = conv(x, f) + fb[:, None, None]
+    e_y = (k * k + 2) * EPS * (conv(np.abs(x), np.abs(f)) + np.abs(fb)[:, None, None])
+    if act == "HardSwish":                             # slope at most 1.5, four roundings
+        y64, e_y = y64 * np.clip(0.2 * y64 + 0.5, 0, 1), 1.5 * e_y + 4 * EPS * np.abs(y64)
+    else:
+        y64 = np.maximum(y64, 0)
+    assert (np.abs(got_y - y64) <= e_y).all()
+    hw, a1, a2 = y64.shape[2] * y64.shape[3], w1[:, :, 0, 0].astype(np.float64), w2[:, :, 0, 0].astype(np.float64)
+    mean = y64.mean((2, 3))
+    hid = np.maximum(mean @ a1.T + b1, 0)
+    e_mean = (hw + 8) * EPS * np.abs(y64).mean((2, 3)) + e_y.mean((2, 3))
+    e_hid = e_mean @ np.abs(a1).T + (c + 8) * EPS * (np.abs(mean) @ np.abs(a1).T + np.abs(b1))
+    e_z = e_hid @ np.abs(a2).T + (s + 8) * EPS * (hid @ np.abs(a2).T + np.abs(b2))
+    want = np.clip(0.2 * (hid @ a2.T + b2) + 0.5, 0, 1)
+    assert (np.abs(got[:, :, 0, 0] - want) <= 0.2 * e_z + 4 * EPS).all()
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 4, 3), (1, 768, 1000), (2, 132, 17), (3, 256, 10), (4, 60, 33), (9, 1280, 65), (32, 960, 1280)])
 def test_product_of_a_few_rows(cuda_lib, m, k, n):
     rng = np.random.default_rng(m + k + n)
