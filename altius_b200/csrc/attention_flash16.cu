@@ -288,8 +288,9 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
         if (left >= 64) {
           float m4[4] = {m, m, m, m};
 #pragma unroll
-          for (int e = 0; e < 64; ++e) m4[e & 3] = fmaxf(m4[e & 3], __fmul_rn(__uint_as_float(s[e]), c1));
-          m = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+          for (int e = 0; e < 64; e += 2)
+            m4[e / 2 & 3] = fmax3(m4[e / 2 & 3], __fmul_rn(__uint_as_float(s[e]), c1), __fmul_rn(__uint_as_float(s[e + 1]), c1));
+          m = fmaxf(fmax3(m4[0], m4[1], m4[2]), m4[3]);
         } else {
 #pragma unroll
           for (int e = 0; e < 64; ++e)
@@ -380,14 +381,15 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
       place(g, k, &tile, &h, &b);
       const float recip = __fmul_rn(__fdiv_rn(1.f, sum), kFixedUnscale);
       const int r = tile * QM + row;
-      const long long ob = (long long)b * p.out_batch_stride + (long long)r * p.out_row_stride + h * HD + hf * 32;
+      const bool mine = ok && r < T;
+      const long long ob = (long long)b * p.out_batch_stride + h * HD + hf * 32;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         uint32_t o[16], ol[16];
         tc_ld_32x16(ocol + (uint32_t)(half * 16), o);
         tc_ld_32x16(ocol + (uint32_t)(64 + half * 16), ol);
         tc_wait_ld(o, ol);
-        if (!ok || r >= T) continue;
+        uint4 yh[2], yl[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           float y[8];
@@ -398,18 +400,28 @@ attention_flash16_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid
             y[e] = __fmul_rn(y[e], recip);
           }
           const float4 y0 = make_float4(y[0], y[1], y[2], y[3]), y1 = make_float4(y[4], y[5], y[6], y[7]);
-          const long long at = ob + half * 16 + 8 * i;
-          if (p.out) {
-            *reinterpret_cast<float4*>(p.out + at) = y0;
-            *reinterpret_cast<float4*>(p.out + at + 4) = y1;
+          if (p.out && mine) {
+            float* at = p.out + ob + (long long)r * p.out_row_stride + half * 16 + 8 * i;
+            *reinterpret_cast<float4*>(at) = y0;
+            *reinterpret_cast<float4*>(at + 4) = y1;
           }
-          if (p.o16_hi) {
-            uint2 h0, l0, h1, l1;
-            f16_split_fixed(y0, h0, l0);
-            f16_split_fixed(y1, h1, l1);
-            *reinterpret_cast<uint4*>(p.o16_hi + (at >> 2)) = make_uint4(h0.x, h0.y, h1.x, h1.y);
-            *reinterpret_cast<uint4*>(p.o16_lo + (at >> 2)) = make_uint4(l0.x, l0.y, l1.x, l1.y);
-            seen_max = split_track(split_track(seen_max, y0), y1);
+          uint2 h0, l0, h1, l1;
+          f16_split_fixed(y0, h0, l0);
+          f16_split_fixed(y1, h1, l1);
+          yh[i] = make_uint4(h0.x, h0.y, h1.x, h1.y);
+          yl[i] = make_uint4(l0.x, l0.y, l1.x, l1.y);
+          if (mine) seen_max = split_track(split_track(seen_max, y0), y1);
+        }
+        if (p.o16_hi) {   // two lanes write 32 bytes of one row and then of the other: whole sectors
+          lane_swap(yh[0], yh[1], lane & 1, 1);
+          lane_swap(yl[0], yl[1], lane & 1, 1);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int ri = tile * QM + q * 32 + (lane & ~1) + i;
+            if (!ok || ri >= T) continue;
+            const long long at = (ob + (long long)ri * p.out_row_stride + half * 16 + 8 * (lane & 1)) >> 2;
+            *reinterpret_cast<uint4*>(p.o16_hi + at) = yh[i];
+            *reinterpret_cast<uint4*>(p.o16_lo + at) = yl[i];
           }
         }
       }

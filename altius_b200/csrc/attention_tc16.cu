@@ -29,6 +29,14 @@
 // contiguous: the B operand of P V is MN-major (128-byte swizzle, 8-key groups 1024 bytes
 // apart). Every mbarrier wait is bounded; on expiry the kernel records a code in the error
 // word and runs to its end without waiting again.
+//
+// What bounds it (clock stamps, 197 tokens): 5450 clocks an item. A group takes 10.9 K from its scores to its next ones: pass 1
+// 1200, pass 2 5000 (tensor memory is read and written beside the MMAs), 600 until the last product is done,
+// then 3900 for the next scores, under which the output (3000) is written. The MMAs take 4200 an item. Before (7200 an item): the
+// output stored a row per lane, 32 lines with every store (4300 clocks; 3000 with 64 bytes of a row at a time), the
+// products of a stage issued in a loop (twice the time an instruction), a mask on every score, and a wait for
+// products that are in front in the pipe anyway. 32 images of 12 heads 31 -> 25 us, 96 images 104 -> 85, 64 of 6 heads 30 -> 24.
+// Not kept: chunks of pass 2 loaded one ahead (pass 2 6000 to 7000 clocks), two chunks at a time (5100).
 #include <cuda.h>
 
 #include <cstdio>
@@ -133,17 +141,14 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
   uint8_t* q_base = v_base + 4 * kKvHalfBytes; // two buffers of Q hi, Q lo
   uint64_t* bars = reinterpret_cast<uint64_t*>(q_base + 4 * kQHalfBytes);
   uint64_t* q_full = bars;                     // [2] TMA: Q of an item has landed in buffer i & 1
-  uint64_t* q_free = bars + 2;                 // [2] the scores of the item are complete
   uint64_t* k_full = bars + 4;
-  uint64_t* k_free = bars + 5;                 // the scores of a unit's last item are complete
   uint64_t* v_full = bars + 6;                 // [2] V of a unit has landed in buffer u & 1
   uint64_t* v_free = bars + 8;                 // [2] the last P V product of the unit is complete
   // One barrier per group wherever a group waits: a parity wait is only right for a waiter at
   // most one phase ahead, and a group may be a whole item ahead of the other.
   uint64_t* o_full = bars + 10;                // [2] the output accumulator of an item of group g is complete
   uint64_t* o_free = bars + 12;                // [2] ... has been read by the 8 warps of the group
-  uint64_t* s_full = bars + 14;                // [2] scores complete in buffer j
-  uint64_t* s_free = bars + 16;                // [2] the products that read P from buffer j are complete
+  uint64_t* s_full = bars + 14;                // [2] scores complete in buffer j: Q of the item, and with a unit's last item K, are free
   uint64_t* ready = bars + 18;                 // [2 groups][2 halves][4 stages] P written (4 warps)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 34);
   float* xch_all = reinterpret_cast<float*>(bars + 40);   // [2 groups][2 halves][128] row maxima, then row sums
@@ -161,7 +166,6 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
     for (int j = 0; j < 2; ++j) {
       mbar_init(&o_free[j], 8);
       mbar_init(&s_full[j], 1);
-      mbar_init(&s_free[j], 1);
     }
     for (int i = 0; i < 16; ++i) mbar_init(&ready[i], 4);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -183,7 +187,7 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
     if (lane == 0) {
       auto load_q = [&](int i, int tile, int h, int b) {
         const int qb = i & 1;
-        if (i >= 2 && !mbar_wait(&q_free[qb], (uint32_t)(((i >> 1) - 1) & 1))) { atomicExch(p.err, 32); ok = false; return; }
+        if (i >= 2 && !mbar_wait(&s_full[qb], (uint32_t)(((i >> 1) - 1) & 1))) { atomicExch(p.err, 32); ok = false; return; }
         uint8_t* dst = q_base + qb * 2 * kQHalfBytes;
         mbar_arrive_expect_tx(&q_full[qb], 2 * kQHalfBytes);
         tma_load_3d(dst, &tm_q_hi, &q_full[qb], p.q_col + h * HD, tile * QM, b);
@@ -195,7 +199,8 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
         const int vb = u & 1;
         load_q(u * n_tiles, 0, h, b);
         if (!ok) break;
-        if (u >= 1 && !mbar_wait(k_free, (uint32_t)((u - 1) & 1))) { atomicExch(p.err, 31); ok = false; break; }
+        const int last = u * n_tiles - 1;        // item in front of the unit
+        if (u >= 1 && !mbar_wait(&s_full[last & 1], (uint32_t)((last >> 1) & 1))) { atomicExch(p.err, 31); ok = false; break; }
         mbar_arrive_expect_tx(k_full, 2 * kKvHalfBytes);
         tma_load_3d(k_hi, &tm_kv_hi, k_full, p.k_col + h * HD, 0, b);
         tma_load_3d(k_hi + kKvHalfBytes, &tm_kv_lo, k_full, p.k_col + h * HD, 0, b);
@@ -217,7 +222,7 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
         AT16_MSTAMP(i, 0);
         if (!mbar_wait(&q_full[j], (uint32_t)((i >> 1) & 1))) { atomicExch(p.err, 34); ok = false; return; }
         if (tile == 0 && !mbar_wait(k_full, (uint32_t)(u & 1))) { atomicExch(p.err, 35); ok = false; return; }
-        if (i >= 2 && !mbar_wait(&s_free[j], (uint32_t)(((i >> 1) - 1) & 1))) { atomicExch(p.err, 36); ok = false; return; }
+        // P of item i - 2 lies where these scores go: the products that read it are in front in the pipe.
         tc_fence_after();
         AT16_MSTAMP(i, 1);
         const uint32_t d = tmem_base + (j ? kS1Col : 0u);
@@ -232,8 +237,6 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
           tc_mma_f16(d, a_hi, b_hi, idesc_s, 1u);
         }
         tc_commit(&s_full[j]);
-        tc_commit(&q_free[j]);
-        if (tile == n_tiles - 1) tc_commit(k_free);
       };
       auto issue_pv = [&](int i) {
         const int u = i / n_tiles, tile = i - u * n_tiles, g = i & 1, vb = u & 1;
@@ -249,42 +252,27 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
         const bool all_there = mbar_test(&ready[(g * 2) * 4 + (NB0 + 1) / 2 - 1], rpar) &&
                                mbar_test(&ready[(g * 2 + 1) * 4 + (NB - NB0 + 1) / 2 - 1], rpar);
         if (all_there) tc_fence_after();
-        bool first = true;
-        if (all_there) {
-          // The same order, unrolled: issuing an instruction takes half the time of the loop below.
-          AT16_MSTAMP(i, 4);
+        AT16_MSTAMP(i, 4);
+        // Unrolled, waits and all: in a loop an instruction took twice the time to issue, and the products of an item
+        // ended 1700 clocks behind its softmax.
 #pragma unroll
-          for (int n = 0; n < 2 * kStages; ++n) {
-            const int st = n >> 1, hf = n & 1, cnt = hf ? NB - NB0 : NB0;
-#pragma unroll
-            for (int c = 2 * st; c < (2 * st + 2 < cnt ? 2 * st + 2 : cnt); ++c) {
-              const int chunk = (hf ? NB0 : 0) + c;
-              const uint32_t a_hi = pcol + (uint32_t)(16 * chunk);
-              const uint64_t b_hi = v_desc + (uint64_t)(chunk * 128);
-              tc_mma3_f16_ta(tmem_base + kOCol, a_hi, a_hi + 8u, b_hi, b_hi + (uint64_t)(kKvHalfBytes >> 4), idesc_o, n + c ? 1u : 0u);
-            }
-          }
-        } else
-#pragma unroll 1
         for (int n = 0; n < 2 * kStages; ++n) {
-          const int st = n >> 1, hf = n & 1;
-          const int cnt = hf ? NB - NB0 : NB0;
+          const int st = n >> 1, half = n & 1, cnt = half ? NB - NB0 : NB0;
           if (2 * st >= cnt) continue;
-          if (!mbar_wait(&ready[(g * 2 + hf) * 4 + st], rpar)) { atomicExch(p.err, 39); ok = false; return; }
-          tc_fence_after();
-          if (n == 0) AT16_MSTAMP(i, 4);
-          const int c_end = 2 * st + 2 < cnt ? 2 * st + 2 : cnt;
-          for (int c = 2 * st; c < c_end; ++c) {
-            const int chunk = (hf ? NB0 : 0) + c;
-            const uint32_t a_hi = pcol + (uint32_t)(16 * chunk), a_lo = a_hi + 8u;
-            const uint64_t b_hi = v_desc + (uint64_t)(chunk * 128), b_lo = b_hi + (uint64_t)(kKvHalfBytes >> 4);
-            tc_mma3_f16_ta(tmem_base + kOCol, a_hi, a_lo, b_hi, b_lo, idesc_o, first ? 0u : 1u);
-            first = false;
+          if (!all_there) {
+            if (!mbar_wait(&ready[(g * 2 + half) * 4 + st], rpar)) { atomicExch(p.err, 39); ok = false; return; }
+            tc_fence_after();
+          }
+#pragma unroll
+          for (int c = 2 * st; c < (2 * st + 2 < cnt ? 2 * st + 2 : cnt); ++c) {
+            const int at = (half ? NB0 : 0) + c;
+            const uint32_t a_hi = pcol + (uint32_t)(16 * at);
+            const uint64_t b_hi = v_desc + (uint64_t)(at * 128);
+            tc_mma3_f16_ta(tmem_base + kOCol, a_hi, a_hi + 8u, b_hi, b_hi + (uint64_t)(kKvHalfBytes >> 4), idesc_o, n + c ? 1u : 0u);
           }
         }
         AT16_MSTAMP(i, 5);
         tc_commit(&o_full[g]);
-        tc_commit(&s_free[g]);
         if (tile == n_tiles - 1) tc_commit(&v_free[vb]);
       };
       if (n_items > 0) issue_s(0);
@@ -335,13 +323,19 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
         tc_ld_32x16(srow + (uint32_t)(c0 + 16), v[1]);
         tc_wait_ld(v[0], v[1]);
         float m0 = CUDART_NAN_F, m1 = CUDART_NAN_F;
+        if (c0 + 32 > T) {                       // few of the chunks, the same for all lanes
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const float t0 = __fmul_rn(__uint_as_float(v[0][e]), c1), t1 = __fmul_rn(__uint_as_float(v[1][e]), c1);
-          m0 = fmaxf(c0 + e < T ? t0 : CUDART_NAN_F, m0);
-          m1 = fmaxf(c0 + 16 + e < T ? t1 : CUDART_NAN_F, m1);
+          for (int e = 0; e < 16; ++e) {
+            if (c0 + e >= T) v[0][e] = 0x7fc00000u;
+            if (c0 + 16 + e >= T) v[1][e] = 0x7fc00000u;
+          }
         }
-        m = fmaxf(fmaxf(m0, m1), m);
+#pragma unroll
+        for (int e = 0; e < 16; e += 2) {
+          m0 = fmax3(m0, __fmul_rn(__uint_as_float(v[0][e]), c1), __fmul_rn(__uint_as_float(v[0][e + 1]), c1));
+          m1 = fmax3(m1, __fmul_rn(__uint_as_float(v[1][e]), c1), __fmul_rn(__uint_as_float(v[1][e + 1]), c1));
+        }
+        m = fmax3(m, m0, m1);
       }
       xch[hf * QM + row] = m;
       pair_sync(g, q);
@@ -352,17 +346,15 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
       float sum = 0.f;
       AT16_STAMP(1);
       AT16_STAMP(2);
-#pragma unroll 1
-      for (int ci = 0; ci < c_count; ++ci) {
+      auto chunk = [&](int ci, uint32_t (&v)[16]) {
         const int c0 = (c_begin + ci) * 16;
-        uint32_t v[16];
-        tc_ld_32x16(srow + (uint32_t)c0, v);
-        tc_wait_ld(v);
         float e[16];
 #pragma unroll
-        for (int x = 0; x < 16; ++x) {
-          const float ev = ex2_approx(fmaf(__uint_as_float(v[x]), c1, -m13));
-          e[x] = c0 + x < T ? ev : 0.f;
+        for (int x = 0; x < 16; ++x) e[x] = ex2_approx(fmaf(__uint_as_float(v[x]), c1, -m13));
+        if (c0 + 16 > T) {                       // one chunk of the row, or those behind it: the same for all lanes
+#pragma unroll
+          for (int x = 0; x < 16; ++x)
+            if (c0 + x >= T) e[x] = 0.f;
         }
 #pragma unroll
         for (int x = 0; x < 16; ++x) sum = __fadd_rn(sum, e[x]);   // + 0 for masked columns: exact
@@ -381,6 +373,13 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
           __syncwarp();
           if (ok && lane == 0) mbar_arrive(&my_ready[ci >> 1]);
         }
+      };
+#pragma unroll 1
+      for (int ci = 0; ci < c_count; ++ci) {
+        uint32_t v[16];
+        tc_ld_32x16(srow + (uint32_t)((c_begin + ci) * 16), v);
+        tc_wait_ld(v);
+        chunk(ci, v);
       }
       AT16_STAMP(3);
       xch[hf * QM + row] = sum;
@@ -399,27 +398,41 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
       if (ok && lane == 0) mbar_arrive(&o_free[g]);
       const float recip = __fmul_rn(__fdiv_rn(1.f, sum), kFixedUnscale);
       const int r = q0 + row;
-      if (ok && r < T) {
-        const long long ob = (long long)b * p.out_batch_stride + (long long)r * p.out_row_stride + h * HD + hf * 32;
+      const bool mine = ok && r < T;
+      const long long ob = (long long)b * p.out_batch_stride + h * HD + hf * 32;
+      uint4 yh[4], yl[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 y0 = make_float4(__fmul_rn(__uint_as_float(o[8 * j]), recip), __fmul_rn(__uint_as_float(o[8 * j + 1]), recip),
-                                        __fmul_rn(__uint_as_float(o[8 * j + 2]), recip), __fmul_rn(__uint_as_float(o[8 * j + 3]), recip));
-          const float4 y1 = make_float4(__fmul_rn(__uint_as_float(o[8 * j + 4]), recip), __fmul_rn(__uint_as_float(o[8 * j + 5]), recip),
-                                        __fmul_rn(__uint_as_float(o[8 * j + 6]), recip), __fmul_rn(__uint_as_float(o[8 * j + 7]), recip));
-          if (p.out) {
-            *reinterpret_cast<float4*>(p.out + ob + 8 * j) = y0;
-            *reinterpret_cast<float4*>(p.out + ob + 8 * j + 4) = y1;
-          }
-          if (p.o16_hi) {   // for the projection GEMM that takes this result as its pre-split A
-            uint2 h0, l0, h1, l1;
-            f16_split_fixed(y0, h0, l0);
-            f16_split_fixed(y1, h1, l1);
-            const long long o4 = (ob + 8 * j) >> 2;      // uint2 index; even: 16-byte aligned
-            *reinterpret_cast<uint4*>(p.o16_hi + o4) = make_uint4(h0.x, h0.y, h1.x, h1.y);
-            *reinterpret_cast<uint4*>(p.o16_lo + o4) = make_uint4(l0.x, l0.y, l1.x, l1.y);
-            seen_max = split_track(split_track(seen_max, y0), y1);
-          }
+      for (int j = 0; j < 4; ++j) {
+        const float4 y0 = make_float4(__fmul_rn(__uint_as_float(o[8 * j]), recip), __fmul_rn(__uint_as_float(o[8 * j + 1]), recip),
+                                      __fmul_rn(__uint_as_float(o[8 * j + 2]), recip), __fmul_rn(__uint_as_float(o[8 * j + 3]), recip));
+        const float4 y1 = make_float4(__fmul_rn(__uint_as_float(o[8 * j + 4]), recip), __fmul_rn(__uint_as_float(o[8 * j + 5]), recip),
+                                      __fmul_rn(__uint_as_float(o[8 * j + 6]), recip), __fmul_rn(__uint_as_float(o[8 * j + 7]), recip));
+        if (p.out && mine) {
+          float* at = p.out + ob + (long long)r * p.out_row_stride + 8 * j;
+          *reinterpret_cast<float4*>(at) = y0;
+          *reinterpret_cast<float4*>(at + 4) = y1;
+        }
+        if (p.o16_hi) {   // for the projection GEMM that takes this result as its pre-split A
+          uint2 h0, l0, h1, l1;
+          f16_split_fixed(y0, h0, l0);
+          f16_split_fixed(y1, h1, l1);
+          yh[j] = make_uint4(h0.x, h0.y, h1.x, h1.y);
+          yl[j] = make_uint4(l0.x, l0.y, l1.x, l1.y);
+          if (mine) seen_max = split_track(split_track(seen_max, y0), y1);
+        }
+      }
+      if (p.o16_hi) {
+        // A lane per row would touch 32 lines with every store (4300 clocks an item); four lanes exchange their rows'
+        // quarters and write 64 bytes of one row at a time.
+        quad_transpose(yh, lane);
+        quad_transpose(yl, lane);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int rk = q0 + q * 32 + (lane & ~3) + k;
+          if (!ok || rk >= T) continue;
+          const long long o4 = (ob + (long long)rk * p.out_row_stride + 8 * (lane & 3)) >> 2;   // uint2 index; even: 16-byte aligned
+          *reinterpret_cast<uint4*>(p.o16_hi + o4) = yh[k];
+          *reinterpret_cast<uint4*>(p.o16_lo + o4) = yl[k];
         }
       }
       AT16_STAMP(5);

@@ -157,6 +157,31 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uin
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Max of three; like fmaxf it ignores NaN.
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// The lower lane's y against the upper lane's x, `with` lanes apart.
+__device__ __forceinline__ void lane_swap(uint4& x, uint4& y, bool upper, int with) {
+  const uint4 out = upper ? x : y;
+  uint4 in;
+  in.x = __shfl_xor_sync(0xffffffffu, out.x, with);
+  in.y = __shfl_xor_sync(0xffffffffu, out.y, with);
+  in.z = __shfl_xor_sync(0xffffffffu, out.z, with);
+  in.w = __shfl_xor_sync(0xffffffffu, out.w, with);
+  if (upper) x = in;
+  else y = in;
+}
+// Four neighbouring lanes, four values each: lane l ends up with value l of the four lanes in order.
+__device__ __forceinline__ void quad_transpose(uint4 (&a)[4], int lane) {
+  lane_swap(a[0], a[1], lane & 1, 1);
+  lane_swap(a[2], a[3], lane & 1, 1);
+  lane_swap(a[0], a[2], lane & 2, 2);
+  lane_swap(a[1], a[3], lane & 2, 2);
+}
+
 // Loads from tensor memory only start here: several may be under way before one tc_wait_ld. The registers are
 // outputs of the load for the compiler, so the wait takes them as operands: no use of them moves ahead of it.
 template <int N>
