@@ -49,45 +49,50 @@ struct SoftmaxMask {
 };
 
 template <int VPT, int MODE, bool MASK>
-__global__ void __launch_bounds__(kThreads) softmax_warp(const float* __restrict__ x,
-                                                         float* __restrict__ out, int64_t rows,
-                                                         int len, const float* __restrict__ scale, SoftmaxMask mk) {
+__global__ void __launch_bounds__(kThreads) softmax_warp(const float* x, float* out, int64_t rows, int len, const float* scale,
+                                                         SoftmaxMask mk) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-  const float s = MODE ? __ldg(scale) : 1.f;
-  const float other = MASK ? __ldg(mk.other) : 0.f;
+  const float s = MODE ? ld_plain(scale) : 1.f;
+  const float other = MASK ? ld_plain(mk.other) : 0.f;
+  constexpr int PAIRS = (VPT + 1) / 2;         // columns lane + 64 i and lane + 64 i + 32: two at a time in packed instructions
   for (int64_t row = warp; row < rows; row += nwarps) {
     const float* xr = x + row * len;
     const uint8_t* mr = MASK ? mk.mask + (row % mk.mask_rows) * len : nullptr;
-    float v[VPT];
+    float2 v[PAIRS];
     float m = CUDART_NAN_F;
+    auto load = [&](int c) {                   // columns that do not exist change neither maximum nor sum
+      if (c >= len) return CUDART_NAN_F;
+      const float e = pre_scale<MODE>(ld_plain(xr + c), s);
+      return MASK ? (mr[c] ? e : other) : e;   // Where(mask, x, other): a selection, exact
+    };
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = lane + 32 * i;
-      if (c < len) {
-        v[i] = pre_scale<MODE>(__ldg(xr + c), s);
-        if (MASK) v[i] = mr[c] ? v[i] : other;     // Where(mask, x, other): a selection, exact
-        m = fmaxf(v[i], m);
-      }
+    for (int i = 0; i < PAIRS; ++i) {
+      v[i].x = load(lane + 64 * i);
+      v[i].y = 2 * i + 1 < VPT ? load(lane + 64 * i + 32) : CUDART_NAN_F;
     }
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) m = fmaxf(v[i].y, fmaxf(v[i].x, m));
     m = warp_max(m);
     float sum = 0.f;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = lane + 32 * i;
-      if (c < len) {
-        v[i] = exp_poly_softmax(__fsub_rn(v[i], m));
-        sum = __fadd_rn(sum, v[i]);
-      }
+    for (int i = 0; i < PAIRS; ++i) {
+      // x - m, as a multiplication by one and an addition: nothing for the compiler to contract.
+      v[i] = exp_poly_softmax2(__ffma2_rn(v[i], make_float2(1.f, 1.f), make_float2(-m, -m)));
+      sum = __fadd_rn(sum, lane + 64 * i < len ? v[i].x : 0.f);
+      if (2 * i + 1 < VPT) sum = __fadd_rn(sum, lane + 64 * i + 32 < len ? v[i].y : 0.f);
     }
     sum = warp_sum(sum);
     const float recip = __fdiv_rn(1.f, sum);
     float* orow = out + row * len;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = lane + 32 * i;
-      if (c < len) orow[c] = __fmul_rn(v[i], recip);
+    for (int i = 0; i < PAIRS; ++i) {
+      const int c = lane + 64 * i;
+      if (c < len) orow[c] = __fmul_rn(v[i].x, recip);
+      if (2 * i + 1 < VPT && c + 32 < len) orow[c + 32] = __fmul_rn(v[i].y, recip);
     }
   }
 }
@@ -134,7 +139,7 @@ cudaError_t softmax_dispatch(const float* x, float* out, int64_t rows, int64_t l
   const unsigned blocks = (unsigned)(blocks64 > device_sm_count() * 64 ? device_sm_count() * 64 : blocks64);
   const int vpt = (int)((len + 31) / 32);
 #define AC_SM(V)                                                                         \
-  softmax_warp<V, MODE, MASK><<<blocks, kThreads, 0, st>>>(x, out, rows, (int)len, scale, mk)
+  return launch_pdl(softmax_warp<V, MODE, MASK>, dim3(blocks), dim3(kThreads), 0, st, 1, x, out, rows, (int)len, scale, mk)
   if (vpt <= 1) AC_SM(1);
   else if (vpt <= 2) AC_SM(2);
   else if (vpt <= 4) AC_SM(4);
@@ -167,6 +172,24 @@ __device__ __forceinline__ float ln_prologue(const LnDev& p, float v, int col, f
   if (p.gelu) v = gelu_ref(v);
   if (p.residual) v = __fadd_rn(v, res);
   return v;
+}
+
+// Four elements in two packed instructions, each rounded as its scalar counterpart (bit for bit). The sum is a
+// multiplication by one and an addition, which leaves the compiler nothing to contract with a product in front.
+__device__ __forceinline__ float4 fma4(float4 a, float4 b, float4 c) {
+  const float2 l = __ffma2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y), make_float2(c.x, c.y));
+  const float2 h = __ffma2_rn(make_float2(a.z, a.w), make_float2(b.z, b.w), make_float2(c.z, c.w));
+  return make_float4(l.x, l.y, h.x, h.y);
+}
+// Behind Gelu's last product the packed form was contracted all the same (a quarter of the results off by an ulp).
+__device__ __forceinline__ float4 add4_scalar(float4 a, float4 b) {
+  return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return fma4(a, make_float4(1.f, 1.f, 1.f, 1.f), b); }
+__device__ __forceinline__ float4 mul4(float4 a, float4 b) {
+  const float2 l = __fmul2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  const float2 h = __fmul2_rn(make_float2(a.z, a.w), make_float2(b.z, b.w));
+  return make_float4(l.x, l.y, h.x, h.y);
 }
 
 // Vector path: len % 4 == 0, all pointers 16-byte aligned. NV float4 per lane.
@@ -245,8 +268,7 @@ __global__ void __launch_bounds__(kThreads, FUSED ? (RESX == 1 ? 4 : 3) : (PF ? 
           const float4 orig = v[i];
           if (p.pre_bias) {
             const float4 bv = __ldg(reinterpret_cast<const float4*>(p.pre_bias) + c);
-            v[i].x = __fadd_rn(v[i].x, bv.x); v[i].y = __fadd_rn(v[i].y, bv.y);
-            v[i].z = __fadd_rn(v[i].z, bv.z); v[i].w = __fadd_rn(v[i].w, bv.w);
+            v[i] = add4(v[i], bv);
           }
           if (GELU) {
             const float2 lo = gelu_ref2(make_float2(v[i].x, v[i].y));
@@ -254,11 +276,9 @@ __global__ void __launch_bounds__(kThreads, FUSED ? (RESX == 1 ? 4 : 3) : (PF ? 
             v[i] = make_float4(lo.x, lo.y, hi.x, hi.y);
           }
           if (RESX != 0) {
-            v[i].x = __fadd_rn(v[i].x, orig.x); v[i].y = __fadd_rn(v[i].y, orig.y);
-            v[i].z = __fadd_rn(v[i].z, orig.z); v[i].w = __fadd_rn(v[i].w, orig.w);
+            v[i] = add4_scalar(v[i], orig);
           } else if (p.residual) {
-            v[i].x = __fadd_rn(v[i].x, r[LOAD_RES ? i : 0].x); v[i].y = __fadd_rn(v[i].y, r[LOAD_RES ? i : 0].y);
-            v[i].z = __fadd_rn(v[i].z, r[LOAD_RES ? i : 0].z); v[i].w = __fadd_rn(v[i].w, r[LOAD_RES ? i : 0].w);
+            v[i] = add4_scalar(v[i], r[LOAD_RES ? i : 0]);
           }
           if (p.sum_out && !dry) reinterpret_cast<float4*>(p.sum_out + row * p.len)[c] = v[i];
         }
@@ -271,12 +291,9 @@ __global__ void __launch_bounds__(kThreads, FUSED ? (RESX == 1 ? 4 : 3) : (PF ? 
     for (int i = 0; i < NV; ++i) {
       const int c = lane + 32 * i;
       if (c < nvec) {
-        v[i].x = __fsub_rn(v[i].x, mean);
-        v[i].y = __fsub_rn(v[i].y, mean);
-        v[i].z = __fsub_rn(v[i].z, mean);
-        v[i].w = __fsub_rn(v[i].w, mean);
-        sq = __fadd_rn(sq, __fadd_rn(__fadd_rn(__fmul_rn(v[i].x, v[i].x), __fmul_rn(v[i].y, v[i].y)),
-                                     __fadd_rn(__fmul_rn(v[i].z, v[i].z), __fmul_rn(v[i].w, v[i].w))));
+        v[i] = add4(v[i], make_float4(-mean, -mean, -mean, -mean));
+        const float4 q = mul4(v[i], v[i]);
+        sq = __fadd_rn(sq, __fadd_rn(__fadd_rn(q.x, q.y), __fadd_rn(q.z, q.w)));
       }
     }
     const float var = fmaf(warp_sum(sq), inv_n, p.eps);
@@ -288,11 +305,7 @@ __global__ void __launch_bounds__(kThreads, FUSED ? (RESX == 1 ? 4 : 3) : (PF ? 
       if (c < nvec) {
         const float4 g = __ldg(reinterpret_cast<const float4*>(p.gamma) + c);
         const float4 b = __ldg(reinterpret_cast<const float4*>(p.beta) + c);
-        float4 o;
-        o.x = fmaf(__fmul_rn(v[i].x, inv), g.x, b.x);
-        o.y = fmaf(__fmul_rn(v[i].y, inv), g.y, b.y);
-        o.z = fmaf(__fmul_rn(v[i].z, inv), g.z, b.z);
-        o.w = fmaf(__fmul_rn(v[i].w, inv), g.w, b.w);
+        const float4 o = fma4(mul4(v[i], make_float4(inv, inv, inv, inv)), g, b);
         if ((!SPLIT || p.out) && !dry) orow[c] = o;
         if (SPLIT && !dry) {
           uint2 h, l;
@@ -441,8 +454,9 @@ __global__ void __launch_bounds__(kThreads) reduce_last_vec(const float* __restr
 // ReduceMean and ReduceMax of the same rows in one pass over them (the two are siblings in
 // the tensor-op micrograph): same loads, same order of additions as reduce_last_vec.
 template <int NV>
-__global__ void __launch_bounds__(kThreads) reduce_mean_max_vec(const float* __restrict__ x, float* __restrict__ mean_out,
-                                                                float* __restrict__ max_out, int64_t rows) {
+__global__ void __launch_bounds__(kThreads) reduce_mean_max_vec(const float* x, float* mean_out, float* max_out, int64_t rows) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
@@ -454,9 +468,9 @@ __global__ void __launch_bounds__(kThreads) reduce_mean_max_vec(const float* __r
     const float4* x1 = reinterpret_cast<const float4*>(x + (two ? row + 1 : row) * len);
     float4 a[NV], b[NV];
 #pragma unroll
-    for (int j = 0; j < NV; ++j) a[j] = __ldg(x0 + lane + 32 * j);
+    for (int j = 0; j < NV; ++j) a[j] = ld_plain(x0 + lane + 32 * j);
 #pragma unroll
-    for (int j = 0; j < NV; ++j) b[j] = __ldg(x1 + lane + 32 * j);
+    for (int j = 0; j < NV; ++j) b[j] = ld_plain(x1 + lane + 32 * j);
     float s0 = 0.f, s1 = 0.f, m0 = -CUDART_INF_F, m1 = -CUDART_INF_F;
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
@@ -625,16 +639,15 @@ cudaError_t launch_reduce_mean_max_last(const float* x, float* mean_out, float* 
     const int64_t cap = (int64_t)device_sm_count() * 6;
     const unsigned vb = (unsigned)(want > cap ? cap : want);
     switch (len / 128) {
-      case 1: reduce_mean_max_vec<1><<<vb, kThreads, 0, st>>>(x, mean_out, max_out, rows); break;
-      case 2: reduce_mean_max_vec<2><<<vb, kThreads, 0, st>>>(x, mean_out, max_out, rows); break;
-      case 3: reduce_mean_max_vec<3><<<vb, kThreads, 0, st>>>(x, mean_out, max_out, rows); break;
-      case 4: reduce_mean_max_vec<4><<<vb, kThreads, 0, st>>>(x, mean_out, max_out, rows); break;
-      case 5: reduce_mean_max_vec<5><<<vb, kThreads, 0, st>>>(x, mean_out, max_out, rows); break;
-      case 6: reduce_mean_max_vec<6><<<vb, kThreads, 0, st>>>(x, mean_out, max_out, rows); break;
-      case 7: reduce_mean_max_vec<7><<<vb, kThreads, 0, st>>>(x, mean_out, max_out, rows); break;
-      default: reduce_mean_max_vec<8><<<vb, kThreads, 0, st>>>(x, mean_out, max_out, rows); break;
+      case 1: return launch_pdl(reduce_mean_max_vec<1>, dim3(vb), dim3(kThreads), 0, st, 1, x, mean_out, max_out, rows);
+      case 2: return launch_pdl(reduce_mean_max_vec<2>, dim3(vb), dim3(kThreads), 0, st, 1, x, mean_out, max_out, rows);
+      case 3: return launch_pdl(reduce_mean_max_vec<3>, dim3(vb), dim3(kThreads), 0, st, 1, x, mean_out, max_out, rows);
+      case 4: return launch_pdl(reduce_mean_max_vec<4>, dim3(vb), dim3(kThreads), 0, st, 1, x, mean_out, max_out, rows);
+      case 5: return launch_pdl(reduce_mean_max_vec<5>, dim3(vb), dim3(kThreads), 0, st, 1, x, mean_out, max_out, rows);
+      case 6: return launch_pdl(reduce_mean_max_vec<6>, dim3(vb), dim3(kThreads), 0, st, 1, x, mean_out, max_out, rows);
+      case 7: return launch_pdl(reduce_mean_max_vec<7>, dim3(vb), dim3(kThreads), 0, st, 1, x, mean_out, max_out, rows);
+      default: return launch_pdl(reduce_mean_max_vec<8>, dim3(vb), dim3(kThreads), 0, st, 1, x, mean_out, max_out, rows);
     }
-    return cudaGetLastError();
   }
   cudaError_t e = reduce_last_dispatch<0>(x, mean_out, rows, len, st);
   return e != cudaSuccess ? e : reduce_last_dispatch<1>(x, max_out, rows, len, st);
