@@ -17,6 +17,10 @@
 // of the first stages are requested while the kernel in front still runs.
 //
 // Per block: warps 0-15 move the accumulator and run the epilogue, warp 16 issues TMA, warp 17 MMAs.
+//
+// The full-range products (3xTF32) of few rows run here too, from fp32 operands (WIDE): one kernel without K-slices through
+// memory (a second kernel of 6 us behind each product), cross terms apart, so errors against 64 bits two to five times
+// smaller: 1386 x 384 x 1152 21.2 -> 14.1 us, 4.9e-7 -> 1.2e-7; 12 layers of DeiT-S at 7 images 1186 -> 972 us.
 #include <cooperative_groups.h>
 #include <cuda.h>
 
@@ -37,7 +41,7 @@ namespace {
 using namespace tc;
 
 constexpr int BM = 128, KB = 64, kEpiThreads = 512, kTmaWarp = 16, kMmaWarp = 17, kThreads = 576, kMaxStages = 4;
-constexpr int kAHalf = BM * KB * 2;           // bytes of A's hi (or lo) tile
+constexpr int kAHalf = BM * KB * 2;           // bytes of A's hi (or lo) tile: rows of 128 bytes
 
 struct KsDev {
   int m, n, k;
@@ -50,29 +54,53 @@ struct KsDev {
   int* err;
 };
 
-template <int ACT>
+// Eight 32-bit columns of the warp's 32 lanes.
+__device__ __forceinline__ void st8(uint32_t taddr, const float (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(__float_as_uint(v[0])),
+               "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])),
+               "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+               : "memory");
+}
+// A in tensor memory: row r in lane r, eight values of K in eight columns.
+__device__ __forceinline__ void mma_tf32_ta(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// WIDE: fp32 operands of any range as 3xTF32, K-blocks of 32 floats. B comes prepared; A arrives as it is, and the sixteen warps split it
+// into tensor memory, from where the products take it (written back beside it in shared memory the halves cost 7 % more).
+template <int ACT, bool WIDE>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
                const __grid_constant__ CUtensorMap tb_hi, const __grid_constant__ CUtensorMap tb_lo, const KsDev p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full;
+  __shared__ __align__(8) uint64_t full[kMaxStages], ready[kMaxStages], empty[kMaxStages], acc_full;
   __shared__ uint32_t tmem_slot;
   __shared__ unsigned seen;                   // what the block has seen of the values it split
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bn = p.bn, S = p.stages, parts = gridDim.z, share = bn / parts, rank = blockIdx.z;
-  const int bhalf = bn * KB * 2, stage_bytes = 2 * kAHalf + 2 * bhalf;
-  float4* part = reinterpret_cast<float4*>(smem + S * stage_bytes);   // [parts][quads][BM + 1]
-  const int nkb = (p.k + KB - 1) / KB, kb0 = rank * p.kper, kbs = min(nkb, kb0 + p.kper) - kb0;
+  const int bhalf = bn * KB * 2;
+  constexpr int kABytes = WIDE ? kAHalf : 2 * kAHalf;
+  const int stage_bytes = kABytes + 2 * bhalf;
+  // [parts][quads][BM + 1]: behind the ring, or over it where no other block writes there.
+  float4* part = reinterpret_cast<float4*>(smem + (parts > 1 ? S * stage_bytes : 0));
+  constexpr int kStep = WIDE ? KB / 2 : KB;   // of K in a block
+  const int nkb = (p.k + kStep - 1) / kStep, kb0 = rank * p.kper, kbs = min(nkb, kb0 + p.kper) - kb0;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * bn;
   // Accumulators of bn columns: the cross terms have the first, the products of the high halves the others. (Three
   // at most, for any width, left 394 x 384 x 1152 at 1.66e-7 where the kernel it replaces has 1.42e-7.)
-  const int mains = min(512 / bn - 1, kbs);
-  const uint32_t cols = bn * (mains + 1) <= 64 ? 64 : bn * (mains + 1) <= 128 ? 128 : bn * (mains + 1) <= 256 ? 256 : 512;
+  // Wide: behind them two buffers for A's hi and lo halves of a K-block, 32 columns each. (Three or four gave nothing: 1190 clocks
+  // a K-block whatever the columns up to 96, which is the issue of its twelve products.)
+  constexpr int kACols = WIDE ? 128 : 0;
+  const int mains = min((512 - kACols) / bn - 1, kbs), used = bn * (mains + 1) + kACols;
+  const uint32_t cols = used <= 64 ? 64 : used <= 128 ? 128 : used <= 256 ? 256 : 512;
   cg::cluster_group cl = cg::this_cluster();
   if (parts > 1) cl.barrier_arrive();         // answered before the first write to another block's memory
   if (tid == 0) {
-    for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&ready[s], kEpiThreads / 32); mbar_init(&empty[s], 1); }
     mbar_init(&acc_full, 1);
     seen = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -80,15 +108,15 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   __syncthreads();
 
   auto load_b = [&](int it) {
-    uint8_t* b = smem + (it % S) * stage_bytes + 2 * kAHalf;
+    uint8_t* b = smem + (it % S) * stage_bytes + kABytes;
     mbar_arrive_expect_tx(&full[it % S], (uint32_t)stage_bytes);
-    tma_load_3d(b, &tb_hi, &full[it % S], (kb0 + it) * KB, n0, 0);
-    tma_load_3d(b + bhalf, &tb_lo, &full[it % S], (kb0 + it) * KB, n0, 0);
+    tma_load_3d(b, &tb_hi, &full[it % S], (kb0 + it) * kStep, n0, 0);
+    tma_load_3d(b + bhalf, &tb_lo, &full[it % S], (kb0 + it) * kStep, n0, 0);
   };
   auto load_a = [&](int it) {
     uint8_t* a = smem + (it % S) * stage_bytes;
-    tma_load_3d(a, &ta_hi, &full[it % S], (kb0 + it) * KB, m0, 0);
-    tma_load_3d(a + kAHalf, &ta_lo, &full[it % S], (kb0 + it) * KB, m0, 0);
+    tma_load_3d(a, &ta_hi, &full[it % S], (kb0 + it) * kStep, m0, 0);
+    if (!WIDE) tma_load_3d(a + kAHalf, &ta_lo, &full[it % S], (kb0 + it) * kStep, m0, 0);
   };
   if (warp == kTmaWarp && lane == 0)
     for (int it = 0; it < S && it < kbs; ++it) load_b(it);   // constants: ahead of pdl_wait
@@ -119,7 +147,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       if (p.bias) bi[i] = ld_plain(reinterpret_cast<const float4*>(p.bias + col));
     }
   };
-  const float sc = p.acc_scale ? __fmul_rn(ld_plain(p.acc_scale), kFixedUnscale) : kFixedUnscale;   // prepared with B: a constant
+  const float sc = WIDE ? 1.f : p.acc_scale ? __fmul_rn(ld_plain(p.acc_scale), kFixedUnscale) : kFixedUnscale;   // prepared with B: a constant
   auto finish = [&] {
     float most = 0.f;
     for (int e0 = tid; e0 < max(live, kEpiThreads); e0 += CH * kEpiThreads) {
@@ -142,7 +170,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       for (int i = 0; i < CH; ++i) {
         const float4 b = bi[i], r = rs[i];
         float4 y = x[i];
-        y.x = __fmul_rn(y.x, sc); y.y = __fmul_rn(y.y, sc); y.z = __fmul_rn(y.z, sc); y.w = __fmul_rn(y.w, sc);
+        if (!WIDE) { y.x = __fmul_rn(y.x, sc); y.y = __fmul_rn(y.y, sc); y.z = __fmul_rn(y.z, sc); y.w = __fmul_rn(y.w, sc); }
         if (p.bias) { y.x = __fadd_rn(y.x, b.x); y.y = __fadd_rn(y.y, b.y); y.z = __fadd_rn(y.z, b.z); y.w = __fadd_rn(y.w, b.w); }
         if (ACT == ACT_GELU) {
           const float2 lo = gelu_ref2(make_float2(y.x, y.y)), hi = gelu_ref2(make_float2(y.z, y.w));
@@ -160,7 +188,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
         const long long r = m0 + row;
         const int col = n0 + rank * share + 4 * q;
         if (p.c) *reinterpret_cast<float4*>(p.c + r * p.ldc + col) = x[i];
-        if (p.c16_hi) {
+        if (!WIDE && p.c16_hi) {
           uint2 h, l;
           f16_split_fixed(x[i], h, l);
           const long long at = (r * p.ldc16 + col) >> 2;
@@ -170,7 +198,7 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
         }
       }
     }
-    if (p.c16_hi && live > 0) {
+    if (!WIDE && p.c16_hi && live > 0) {
       const unsigned all = __reduce_or_sync(0xffffffffu, split_seen_fixed_of_max(most));
       if (lane == 0) atomicOr(&seen, all);
     }
@@ -210,10 +238,11 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
       }
     } else if (warp == kMmaWarp) {
       if (elect_one()) {
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        constexpr uint32_t kFmt = WIDE ? 2u : 0u;   // TF32 or fp16
+        const uint32_t idesc = (1u << 4) | (kFmt << 7) | (kFmt << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
         for (int it = 0; it < kbs; ++it) {
           const int s = it % S;
-          if (!mbar_wait(&full[s], (uint32_t)(it / S) & 1)) {
+          if (!mbar_wait(WIDE ? &ready[s] : &full[s], (uint32_t)(it / S) & 1)) {
             atomicExch(p.err, 62);
             for (int w = it; w < kbs && w < it + S; ++w) (void)mbar_wait(&full[w % S], (uint32_t)(w / S) & 1);   // copies in flight land
             break;
@@ -221,16 +250,21 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
           tc_fence_after();
           const uint32_t a = smem_u32(smem + s * stage_bytes);
           const uint64_t da = desc_sw128(a), dal = desc_sw128(a + kAHalf);
-          const uint64_t db = desc_sw128(a + 2 * kAHalf), dbl = desc_sw128(a + 2 * kAHalf + bhalf);
+          const uint64_t db = desc_sw128(a + kABytes), dbl = desc_sw128(a + kABytes + bhalf);
+          const uint32_t ta = tmem + (uint32_t)(bn * (mains + 1) + (it & 1) * 64);   // wide: A's halves
           // Always four steps (what lies beyond K arrives as zeros): with a run-time count an instruction
           // took 113 clocks to issue, unrolled 57 (96 columns).
           const uint32_t cross = tmem, main = tmem + (uint32_t)((1 + it % mains) * bn);
 #pragma unroll
-          for (int kk = 0; kk < KB / 16; ++kk) {
+          for (int kk = 0; kk < 4; ++kk) {
             const uint64_t off = (uint64_t)(kk * 32 >> 4);
-            tc_mma_f16(main, da + off, db + off, idesc, (it >= mains || kk > 0) ? 1u : 0u);        // a_hi * b_hi
-            tc_mma_f16(cross, dal + off, db + off, idesc, (it > 0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
-            tc_mma_f16(cross, da + off, dbl + off, idesc, 1u);             // a_hi * b_lo
+            auto mma = [&](uint32_t d, bool lo, uint64_t b, uint32_t accumulate) {
+              if (WIDE) mma_tf32_ta(d, ta + (uint32_t)(8 * kk + (lo ? 32 : 0)), b + off, idesc, accumulate);
+              else tc_mma_f16(d, (lo ? dal : da) + off, b + off, idesc, accumulate);
+            };
+            mma(main, false, db, (it >= mains || kk > 0) ? 1u : 0u);        // a_hi * b_hi
+            mma(cross, true, db, (it > 0 || kk > 0) ? 1u : 0u);   // a_lo * b_hi
+            mma(cross, false, dbl, 1u);                           // a_hi * b_lo
           }
           tc_commit(&empty[s]);
         }
@@ -239,6 +273,34 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
     }
     if (warp < kEpiThreads / 32) {
       fetch(tid);                                // under the products
+      if (WIDE) {
+        for (int it = 0; it < kbs; ++it) {
+          const int s = it % S;
+          if (!mbar_wait_all(&full[s], (uint32_t)(it / S) & 1)) { atomicExch(p.err, 65); break; }
+          // This warp's 32 rows, 8 of their 32 values: two 16-byte chunks, which the swizzle spreads over the banks.
+          const int row = (warp & 3) * 32 + lane, part8 = warp >> 2;
+          const uint8_t* at = smem + s * stage_bytes + row * 128;
+          float h[8], l[8];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            float4 hi, lo;
+            tf32_split(*reinterpret_cast<const float4*>(at + (((2 * part8 + c) ^ (row & 7)) << 4)), hi, lo);
+            h[4 * c] = hi.x; h[4 * c + 1] = hi.y; h[4 * c + 2] = hi.z; h[4 * c + 3] = hi.w;
+            l[4 * c] = lo.x; l[4 * c + 1] = lo.y; l[4 * c + 2] = lo.z; l[4 * c + 3] = lo.w;
+          }
+          // The products that took the buffer's last contents are complete (with a ring of two or fewer the entry could not
+          // have been loaded before).
+          if (S > 2 && it >= 2 && !mbar_wait_all(&empty[(it - 2) % S], (uint32_t)((it - 2) / S) & 1)) { atomicExch(p.err, 66); break; }
+          tc_fence_after();
+          const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(bn * (mains + 1) + (it & 1) * 64 + 8 * part8);
+          st8(ta, h);
+          st8(ta + 32u, l);
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ready[s]);
+        }
+      }
       if (!warp_mbar_wait(&acc_full, 0, lane)) atomicExch(p.err, 63);
       tc_fence_after();
       const int row = (warp & 3) * 32 + lane;
@@ -319,7 +381,7 @@ int cluster_slots(int split) {
   if (const int v = known[dev][at].load(std::memory_order_relaxed)) return v;
   static unsigned long long done = 0;
   int slots = 0;
-  if (ensure_dynamic_smem(gemm_ks_kernel<ACT_NONE>, (int)kSmemMax, &done) == cudaSuccess) {
+  if (ensure_dynamic_smem(gemm_ks_kernel<ACT_NONE, false>, (int)kSmemMax, &done) == cudaSuccess) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(1, (unsigned)device_sm_count(), (unsigned)split);
     cfg.blockDim = dim3(kThreads);
@@ -329,7 +391,7 @@ int cluster_slots(int split) {
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = (unsigned)split;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&slots, gemm_ks_kernel<ACT_NONE>, &cfg) != cudaSuccess) slots = 0;
+    if (cudaOccupancyMaxActiveClusters(&slots, gemm_ks_kernel<ACT_NONE, false>, &cfg) != cudaSuccess) slots = 0;
   }
   (void)cudaGetLastError();
   if (slots <= 0) {            // no device: the counts of a B200
@@ -346,24 +408,27 @@ namespace {
 // each) or its bytes at 60 a clock, whichever is more; first loads and drain 2700; exchange 1600 and 18
 // per column; epilogue 1500 and 40 per column that a block finishes. A launch as timed takes 1.4 to 2 times as long
 // (launch, cold code; operands arrive at 34 bytes a clock when all SMs load at once).
-Shape pick_shape(int64_t m, int64_t n, int64_t k) {
+//
+// Fp32 operands: a K-block of 32 costs 1190 clocks up to 96 columns, 1370 with 128.
+Shape pick_shape(int64_t m, int64_t n, int64_t k, bool wide) {
   Shape best;
-  const int nkb = (int)((k + KB - 1) / KB);
+  const int step = wide ? KB / 2 : KB, nkb = (int)((k + step - 1) / step);
   const long long mt = (m + BM - 1) / BM;
   for (int bn : {32, 64, 96, 128}) {
     for (int split : {1, 2, 4, 8}) {
       const int kper = (nkb + split - 1) / split;
       if ((split - 1) * kper >= nkb || (bn % (4 * split)) != 0) continue;
       const int quads = bn / split / 4;
-      const size_t stage = 2 * (size_t)kAHalf + (size_t)bn * KB * 4, ex = (size_t)split * quads * (BM + 1) * 16;
-      const int stages = (int)std::min<size_t>(std::min(kper, kMaxStages), (kSmemMax - 1024 - ex) / stage);
+      const size_t stage = (wide ? 1 : 2) * (size_t)kAHalf + (size_t)bn * KB * 4, ex = (size_t)split * quads * (BM + 1) * 16;
+      const int stages = (int)std::min<size_t>(std::min(kper, kMaxStages), (kSmemMax - 1024 - (split > 1 ? ex : 0)) / stage);
       if (stages < std::min(2, kper)) continue;
       const double waves = std::ceil((double)mt * ((n + bn - 1) / bn) / cluster_slots(split));
-      const double kb = std::max(12 * (32.0 + 0.26 * bn), (double)stage / 60.0);
+      const double kb = wide ? (bn > 96 ? 1370.0 : 1190.0)
+                             : std::max(12 * (32.0 + 0.26 * bn), (double)stage / 60.0);
       const double t = waves * (kper * kb + 4200.0 + (split > 1 ? 1600.0 + 18.0 * bn : 0.0) + 40.0 * bn / split);
       if (t < best.clocks) {
         best.bn = bn; best.split = split; best.kper = kper; best.stages = stages; best.inv = ((1 << 20) + quads - 1) / quads;
-        best.smem = stages * stage + ex + 1024;
+        best.smem = std::max(stages * stage + (split > 1 ? ex : 0), ex) + 1024;
         best.clocks = t;
       }
     }
@@ -371,16 +436,33 @@ Shape pick_shape(int64_t m, int64_t n, int64_t k) {
   return best;
 }
 
-template <int ACT>
+template <int ACT, bool WIDE>
 cudaError_t launch_act(const CUtensorMap& ah, const CUtensorMap& al, const CUtensorMap& bh, const CUtensorMap& bl,
                        const KsDev& d, const Shape& sh, cudaStream_t st) {
   static unsigned long long done = 0;
-  if (cudaError_t e = ensure_dynamic_smem(gemm_ks_kernel<ACT>, (int)kSmemMax, &done)) return e;
+  if (cudaError_t e = ensure_dynamic_smem(gemm_ks_kernel<ACT, WIDE>, (int)kSmemMax, &done)) return e;
   const dim3 grid((unsigned)((d.n + sh.bn - 1) / sh.bn), (unsigned)((d.m + BM - 1) / BM), (unsigned)sh.split);
-  return launch_pdl(gemm_ks_kernel<ACT>, grid, dim3(kThreads), sh.smem, st, sh.split, ah, al, bh, bl, d);
+  return launch_pdl(gemm_ks_kernel<ACT, WIDE>, grid, dim3(kThreads), sh.smem, st, sh.split, ah, al, bh, bl, d);
+}
+template <bool WIDE>
+cudaError_t launch_any(int act, const CUtensorMap& ah, const CUtensorMap& al, const CUtensorMap& bh, const CUtensorMap& bl, const KsDev& d,
+                       const Shape& sh, cudaStream_t st) {
+  if (act == ACT_GELU) return launch_act<ACT_GELU, WIDE>(ah, al, bh, bl, d, sh, st);
+  if (act == ACT_RELU) return launch_act<ACT_RELU, WIDE>(ah, al, bh, bl, d, sh, st);
+  return launch_act<ACT_NONE, WIDE>(ah, al, bh, bl, d, sh, st);
 }
 
 inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
+
+KsDev device_params(const GemmParams& q, const Shape& sh, int* err_word) {
+  KsDev d{};
+  d.m = (int)q.m; d.n = (int)q.n; d.k = (int)q.k;
+  d.bn = sh.bn; d.stages = sh.stages; d.kper = sh.kper; d.inv = sh.inv;
+  d.c = q.c; d.ldc = q.ldc;
+  d.bias = q.bias_n; d.res = q.residual; d.ldres = q.ld_res;
+  d.err = err_word;
+  return d;
+}
 
 }  // namespace
 
@@ -399,7 +481,7 @@ int gemm_ks_pair_run(int64_t m, int64_t n, int64_t k) {
 
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k) {
   if (m < 1 || n < 4 || (n % 4) || k < 64 || (k % 8) || m > (1 << 20) || n > (1 << 20)) return 1e30;
-  return pick_shape(m, n, k).clocks;
+  return pick_shape(m, n, k, false).clocks;
 }
 
 bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bias_scale) {
@@ -416,22 +498,37 @@ cudaError_t launch_gemm_ks(const GemmParams& q, int pair_run, int* err_word, cud
     if (q.c16_hi && ((q.n % 8) || (q.ldc16 % 8) || !al16(q.c16_hi) || !al16(q.c16_lo))) return cudaErrorInvalidValue;   // 16 bytes of a row at once
     return launch_gemm_pair_sums(q, pair_run, err_word, st);
   }
-  const Shape sh = pick_shape(q.m, q.n, q.k);
-  KsDev d{};
-  d.m = (int)q.m; d.n = (int)q.n; d.k = (int)q.k;
-  d.bn = sh.bn; d.stages = sh.stages; d.kper = sh.kper; d.inv = sh.inv;
-  d.c = q.c; d.ldc = q.ldc;
+  const Shape sh = pick_shape(q.m, q.n, q.k, false);
+  KsDev d = device_params(q, sh, err_word);
   d.c16_hi = static_cast<uint2*>(q.c16_hi); d.c16_lo = static_cast<uint2*>(q.c16_lo); d.ldc16 = q.ldc16;
-  d.bias = q.bias_n; d.res = q.residual; d.ldres = q.ld_res;
   d.acc_scale = q.b16_inv_scale;
-  d.err = err_word;
   CUtensorMap ah, al, bh, bl;
   if (!make_map16(&ah, q.a16_hi, q.k, q.m, 1, q.lda16, q.m * q.lda16, BM) || !make_map16(&al, q.a16_lo, q.k, q.m, 1, q.lda16, q.m * q.lda16, BM) ||
       !make_map16(&bh, q.b16_hi, q.k, q.n, 1, q.ldb16, q.n * q.ldb16, sh.bn) || !make_map16(&bl, q.b16_lo, q.k, q.n, 1, q.ldb16, q.n * q.ldb16, sh.bn))
     return cudaErrorInvalidValue;
-  if (q.act == ACT_GELU) return launch_act<ACT_GELU>(ah, al, bh, bl, d, sh, st);
-  if (q.act == ACT_RELU) return launch_act<ACT_RELU>(ah, al, bh, bl, d, sh, st);
-  return launch_act<ACT_NONE>(ah, al, bh, bl, d, sh, st);
+  return launch_any<false>(q.act, ah, al, bh, bl, d, sh, st);
+}
+
+double gemm_ks_wide_clocks(int64_t m, int64_t n, int64_t k) {
+  if (m < 1 || n < 4 || (n % 4) || k < 32 || (k % 4) || m > (1 << 20) || n > (1 << 20)) return 1e30;
+  // Long K: the other kernel's slices fill the SMs better than either estimate says (1386 x 3072 x 768 38.4 us, here 42.4; 394 x 2048 x 512
+  // 15.5, 15.9; but 198 x 3072 x 768 17.0, 16.0).
+  return pick_shape(m, n, k, true).clocks * (k > 1536 ? 1.15 : 1.0);
+}
+
+cudaError_t launch_gemm_ks_wide(const GemmParams& q, int* err_word, cudaStream_t st) {
+  if (!q.a || !q.b || !q.b_lo || !q.c || !q.trans_b || q.trans_a || q.batch != 1 || q.c16_hi || gemm_ks_wide_clocks(q.m, q.n, q.k) >= 1e30 ||
+      (q.lda % 4) || (q.ldb % 4) || (q.ldc % 4) || !al16(q.a) || !al16(q.b) || !al16(q.b_lo) || !al16(q.c) ||
+      (q.residual && (!al16(q.residual) || (q.ld_res % 4))) || (q.bias_n && !al16(q.bias_n)) ||
+      !gemm_ks_epilogue_ok(q.act, q.bias_m != nullptr, q.beta != 0.f && q.c_in, q.alpha, q.bias_scale))
+    return cudaErrorInvalidValue;
+  const Shape sh = pick_shape(q.m, q.n, q.k, true);
+  const KsDev d = device_params(q, sh, err_word);
+  CUtensorMap a, bh, bl;
+  if (!make_map128(&a, q.a, 4, q.k, q.m, 1, q.lda, q.m * q.lda, BM) || !make_map128(&bh, q.b, 4, q.k, q.n, 1, q.ldb, q.n * q.ldb, sh.bn) ||
+      !make_map128(&bl, q.b_lo, 4, q.k, q.n, 1, q.ldb, q.n * q.ldb, sh.bn))
+    return cudaErrorInvalidValue;
+  return launch_any<true>(q.act, a, a, bh, bl, d, sh, st);
 }
 
 }  // namespace ac

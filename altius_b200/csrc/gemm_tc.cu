@@ -1883,7 +1883,7 @@ int pair_count() {
 // 1 TF32 with one B copy, 2 fp16 split.
 // allow_pairs: 0 no CTA pairs, 1 pairs that stage A through registers, 2 pairs whose A arrives
 // already split by TMA (each SM then pulls 32 KB per stage and no thread touches a tile).
-TcShape pick_shape(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, int allow_pairs) {
+TcShape pick_shape(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, int allow_pairs, double* clocks = nullptr) {
   static const TcShape cands[3] = {{256, 1, false}, {128, 1, false}, {64, 1, false}};
   // Debug toggle: ALTIUS_CUDA_TC_BN=64|128|256 forces the tile width.
   const char* ebn = std::getenv("ALTIUS_CUDA_TC_BN");
@@ -1922,6 +1922,7 @@ TcShape pick_shape(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, 
     const double cost = rounds * (pl.sc.num_kb * (pkb / 32) * std::max(6.0 * 128.0, 32768.0 / 28.0) + 256 * 24.0);
     if (cost < best_cost - 1e-9) { best_cost = cost; best = {256, 2, true}; }
   }
+  if (clocks) *clocks = best_cost;
   return best;
 }
 }  // namespace
@@ -1945,6 +1946,15 @@ double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k) {
   double blocks = (double)((pl.sc.dp_tiles + pairs - 1) / pairs) * pl.sc.num_kb;
   if (pl.sc.tail_parts >= 2) blocks += (double)pl.sc.num_kb / pl.sc.tail_parts;
   return blocks * (kPairBlock + kExactBlock) + kPairEnds + kExactEnds + (pl.sc.tail_parts >= 2 ? kPairSlices + kExactSlices : 0.0);
+}
+
+// The same for 3xTF32 products with a prepared B, beside gemm_ks_wide_clocks: fitted over 150 products of 64 to 9456 rows by 192 to
+// 3072 (us here, there: 1386 x 384 x 1152 21.2, 14.1; 1386 x 384 x 384 11.3, 9.7; 198 x 768 x 768 11.6, 9.7; but 1386 x 768 x 2304
+// 36.0, 43.1 and 2956 x 384 x 1536 22.5, 31.4). K-slices and their second kernel count 6000.
+double gemm_tc_wide_clocks(int64_t m, int64_t n, int64_t k) {
+  double clocks = 0;
+  const TcShape sh = pick_shape(m, n, k, 1, 0, 0, &clocks);
+  return 8100.0 + 0.74 * clocks + (make_plan(m, n, k, 1, sh.bn, sh.mt, BK).sc.tail_parts >= 2 ? 6000.0 : 0.0);
 }
 
 size_t gemm_tc_workspace_bytes(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, int allow_pairs) {

@@ -282,6 +282,7 @@ constexpr int kGemmRangeCode = 21;
 // Clocks of the pre-split GEMM of this shape on CTA pairs (its K-slice pass included), by the same plan the
 // launch uses; and of the kernel for few rows (gemm_ks.cu: clusters that share a tile along K; 1e30
 // where it does not apply), which takes the operands of the pair kernel.
+double gemm_tc_wide_clocks(int64_t m, int64_t n, int64_t k);
 double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k);
 // CTA pairs that can run at once (0: none, their kernels cannot be launched).
 int gemm_tc_pairs();
@@ -293,6 +294,9 @@ bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bia
 // lowering asks, so that the schedule names the kernel that runs, and hands the answer to the launch.
 int gemm_ks_pair_run(int64_t m, int64_t n, int64_t k);
 cudaError_t launch_gemm_ks(const GemmParams& p, int pair_run, int* err_word, cudaStream_t st);
+// The same kernel on fp32 operands as 3xTF32 (a; b and b_lo as for launch_gemm_tc), the epilogues of gemm_ks_epilogue_ok; 1e30: not for it.
+double gemm_ks_wide_clocks(int64_t m, int64_t n, int64_t k);
+cudaError_t launch_gemm_ks_wide(const GemmParams& p, int* err_word, cudaStream_t st);
 // The same operands and epilogues on CTA pairs, `run` K-blocks of 64 on one accumulator (gemm_tc.cu).
 cudaError_t launch_gemm_pair_sums(const GemmParams& p, int run, int* err_word, cudaStream_t st);
 // fp16 split of a constant [rows, k] operand (row stride ld) into [rows, k8] halves

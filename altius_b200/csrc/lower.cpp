@@ -998,6 +998,10 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
     b_use = hi;
   }
   const int bsrc = b_use;
+  // Products of few rows in full range, from fp32 operands.
+  const bool ks_wide = b_lo >= 0 && g.batch == 1 && a_off == 0 && b_off == 0 && c_off == 0 && g.lda == g.k && g.ldb == g.k && g.ldc == g.n &&
+                       b_row_scale < 0 && gemm_ks_epilogue_ok(act, bias_m >= 0, c_in >= 0, alpha, bias_scale) &&
+                       gemm_ks_wide_clocks(g.m, g.n, g.k) < gemm_tc_wide_clocks(g.m, g.n, g.k);
   // CTA pairs that take A by TMA want it already split into fp16 hi / lo halves (rows of K
   // halves): written by the kernel that produced A when plan_presplit arranged that, else by a
   // split kernel in front of the GEMM.
@@ -1047,7 +1051,7 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   // Scratch for the K-sliced tail tiles of the persistent kernel (lives for this step only).
   int ws = -1;
   size_t ws_bytes = 0;
-  if (tc && !use_ks) {
+  if (tc && !use_ks && !ks_wide) {
     ws_bytes = gemm_tc_workspace_bytes(g.m, g.n, g.k, g.batch, b16_hi >= 0 ? 2 : (b_lo >= 0 ? 0 : 1), pairs);
     if (ws_bytes) ws = new_value(em.c, (int64_t)(ws_bytes / 4), false);
   }
@@ -1096,6 +1100,7 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
     p.act = act; p.act_alpha = aa; p.act_beta = ab;
     p.residual = res >= 0 ? s->fptr(res) + c_off : nullptr; p.ld_res = g.ldc; p.stride_res = g.sc;
     if (use_ks) return launch_gemm_ks(p, pair_run, s->err_word, st);
+    if (ks_wide) return launch_gemm_ks_wide(p, s->err_word, st);
     if (tc && gemm_tc_supported(p)) return launch_gemm_tc(p, mode, s->err_word, st);
     if (!p.a || !p.c || p.c16_hi || p.b_row_scale) return cudaErrorInvalidValue;   // operands exist for the tensor-core kernel only
     // The CUDA-core kernel multiplies the operand as given, not a TF32-rounded copy of it.

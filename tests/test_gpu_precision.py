@@ -60,6 +60,37 @@ def test_few_row_product(cuda_lib, m, d, n, bound):
     assert _rel(g, x, want, "gemm_f16x3_cluster_tcgen05") <= bound
 
 
+# Full-range products (gemm_mode 3) of few rows: the one-CTA kernel's error on these inputs. Ragged rows, columns and K, K over a
+# cluster of two to eight, a single K-block; with each epilogue. Scaled inputs, which the fp16 formats could not hold.
+@pytest.mark.parametrize("m,d,n,bound", [(198, 768, 2304, 4.91e-7), (394, 384, 1152, 4.94e-7), (1386, 384, 384, 4.71e-7),
+                                         (198, 1536, 384, 6.4e-7), (788, 192, 576, 2.54e-7), (333, 520, 332, 1.84e-7),
+                                         (1001, 100, 516, 2.75e-7), (129, 36, 1028, 2.75e-7), (515, 32, 2052, 2.75e-7)])
+@pytest.mark.parametrize("act,res,scale", [(None, False, 1.0), ("Gelu", False, 1.0), ("ReLU", True, 1e6)])
+def test_full_range_product(cuda_lib, m, d, n, bound, act, res, scale):
+    rng = np.random.default_rng(m + n)
+    x = (scale * rng.standard_normal((m, d))).astype(np.float32)
+    w = (rng.standard_normal((d, n)) / np.sqrt(d)).astype(np.float32)
+    b = (scale * rng.standard_normal(n)).astype(np.float32)
+    r = (scale * rng.standard_normal((m, n))).astype(np.float32)
+    g = ir.Graph()
+    xi = g.add_input("x", x.shape)
+    ri = g.add_input("r", r.shape) if res else None
+    y = g.op("Add", g.op("MatMul", xi, g.new_init(w)), g.new_init(b))
+    y = g.op(act, y) if act else y
+    g.outputs.append(g.op("Add", y, ri) if res else y)
+    sess = CudaSessionBuilder(ir.Model(g, 13)).with_gemm_mode(3).build()
+    try:
+        assert [(e["kind"], e["launches"]) for e in sess.schedule()] == [("gemm_tf32x3_tcgen05", 1)]   # no second kernel for slices
+        got = torch.from_numpy(sess.run([x] + ([r] if res else []))[0]).double().cuda()
+    finally:
+        sess.close()
+    want = _t(x) @ _t(w) + _t(b)
+    want = torch.relu(want) if act == "ReLU" else torch.nn.functional.gelu(want, approximate="tanh") if act else want
+    want = want + _t(r) if res else want
+    # Gelu's slope is at most 1.13, its rational tanh is off by 1e-7 of the result
+    assert ((got - want).norm() / want.norm()).item() <= bound * (1.0 if not act else 2.0 if act == "Gelu" else 1.0)
+
+
 # beyond 256 tokens separate 3xTF32 and fp32 products, up to 256 the kernel on operands from fp32; on a given
 # projection (one of 577 tokens) and behind its GEMM
 @pytest.mark.parametrize("B,T,H,projection,bound", [
