@@ -524,13 +524,14 @@ cudaError_t launch_pack_filter_tc(const ConvParams& q, const float* w, float* pa
   return cudaGetLastError();
 }
 
-cudaError_t launch_conv_tc(const ConvParams& q, const float* x, const float* packed, const float* bias, const float* gate,
+cudaError_t launch_conv_tc(const ConvParams& q, int images, const float* x, const float* packed, const float* bias, const float* gate,
                            const float* residual, float* out, bool constants, int* err_word, cudaStream_t st) {
-  const Shape sh = shape_of(q);
+  Shape sh = shape_of(q);
   ConvTcDev p{};
   p.x = x; p.w = packed; p.out = out; p.bias = bias; p.res = residual; p.gate = gate;
-  p.m = q.oc; p.k = q.c * q.kh * q.kw; p.hw = q.oh * q.ow; p.n = q.n * p.hw;
+  p.m = q.oc; p.k = q.c * q.kh * q.kw; p.hw = q.oh * q.ow; p.n = images * p.hw;
   if (p.m == 0 || p.n == 0) return cudaSuccess;
+  sh.ctas = std::min(sh.ctas, (p.n + PX - 1) / PX);
   p.bn = sh.bn; p.stages = sh.stages; p.kper = sh.kper; p.resident = sh.resident;
   p.set = sh.set; p.mains = sh.mains; p.bufs = sh.bufs; p.cols = sh.cols;
   p.x_batch = (long long)q.c * q.ih * q.iw; p.out_batch = (long long)p.m * p.hw;

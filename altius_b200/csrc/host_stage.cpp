@@ -120,15 +120,19 @@ void HostStage::worker() {
   }
 }
 
-cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStream_t st, const std::function<cudaError_t(size_t)>& sent) {
+  auto whole = [&] {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess && sent ? sent(bytes) : e;
+  };
   // While another thread's upload holds the ring this one takes the driver's path: both then run at once.
   std::unique_lock<std::mutex> use(use_, std::try_to_lock);
-  if (!use.owns_lock()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  if (!use.owns_lock()) return whole();
   const int n = (int)((bytes + kChunk - 1) / kChunk);
   std::unique_ptr<std::atomic<char>[]> more;
   if (done_size_ < n) {                       // only ever changed under use_
     more.reset(new (std::nothrow) std::atomic<char>[n]);
-    if (!more) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    if (!more) return whole();
   }
   for (cudaEvent_t e : left_)                 // slots an earlier upload may still occupy
     if (cudaError_t err = cudaEventSynchronize(e)) return err;
@@ -175,6 +179,7 @@ cudaError_t HostStage::upload(void* dst, const void* src, size_t bytes, cudaStre
     err = cudaMemcpyAsync(static_cast<char*>(dst) + at, ring_ + (size_t)(c % kSlots) * kChunk, std::min(kChunk, bytes - at),
                           cudaMemcpyHostToDevice, st);
     if (err == cudaSuccess) err = cudaEventRecord(left_[c % kSlots], st);
+    if (err == cudaSuccess && sent) err = sent(std::min(bytes, at + kChunk));
   }
   if (err != cudaSuccess) {                   // nobody may go on reading the caller's memory
     next_.store(n * kPieces);

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <functional>
 #include <condition_variable>
 #include <memory>
 #include <mutex>
@@ -24,8 +25,9 @@ class HostStage {
   // cannot be had (the caller then lets the driver copy).
   static std::shared_ptr<HostStage> of_device(int device);
   ~HostStage();
-  // Enqueues dst (device) <- src (pageable host) on `st`; src has been read when this returns.
-  cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st);
+  // Enqueues dst (device) <- src (pageable host) on `st`; src has been read when this returns. `sent(n)` is called when
+  // the first n bytes have been enqueued, n growing to `bytes`; an error it returns ends the upload.
+  cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st, const std::function<cudaError_t(size_t)>& sent = nullptr);
 
  private:
   static constexpr size_t kChunk = size_t(1) << 20;

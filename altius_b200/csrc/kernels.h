@@ -199,7 +199,8 @@ cudaError_t launch_conv_simt(const ConvParams& p, const float* x, const float* w
 bool conv_tc_supported(const ConvParams& p);
 int64_t conv_tc_filter_elems(const ConvParams& p);
 cudaError_t launch_pack_filter_tc(const ConvParams& p, const float* w, float* packed, cudaStream_t st);
-cudaError_t launch_conv_tc(const ConvParams& p, const float* x, const float* packed, const float* bias, const float* gate,
+// `images`: of the p.n that the tile shape is chosen for, from the given pointers on.
+cudaError_t launch_conv_tc(const ConvParams& p, int images, const float* x, const float* packed, const float* bias, const float* gate,
                            const float* residual, float* out, bool constants, int* err_word, cudaStream_t st);
 
 // Squeeze-and-excite gate in one kernel (squeeze_excite.cu):

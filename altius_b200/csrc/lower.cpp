@@ -1231,11 +1231,17 @@ void lower_conv(Emit& em, Plan& plan, int nid, const Epilogue* e, const Plan::Se
     int means = -1;
     if (auto m = plan.means.find(out); m != plan.means.end() && depthwise_conv_pools(p))
       m->second = means = new_value(em.c, (int64_t)p.n * p.c, false);
-    em.add("conv_depthwise", n.op, {x, w, bias}, means >= 0 ? std::vector<int>{out, means} : std::vector<int>{out}, bytes, flops,
-           [=](cudaStream_t st) {
-             return launch_depthwise_conv(p, s->fptr(x), s->fptr(w), bias >= 0 ? s->fptr(bias) : nullptr, s->fptr_mut(out),
-                                          means >= 0 ? s->fptr_mut(means) : nullptr, constants, st);
-           });
+    auto part = [=](cudaStream_t st, int first, int count) {
+      ConvParams q = p;
+      q.n = count;
+      return launch_depthwise_conv(q, s->fptr(x) + (size_t)first * p.c * p.ih * p.iw, s->fptr(w), bias >= 0 ? s->fptr(bias) : nullptr,
+                                   s->fptr_mut(out) + (size_t)first * p.oc * ohw, means >= 0 ? s->fptr_mut(means) + (size_t)first * p.oc : nullptr,
+                                   constants, st);
+    };
+    Step& step = em.add("conv_depthwise", n.op, {x, w, bias}, means >= 0 ? std::vector<int>{out, means} : std::vector<int>{out}, bytes, flops,
+                        [=](cudaStream_t st) { return part(st, 0, p.n); });
+    step.part = part;
+    step.images = p.n;
     return;
   }
   // GEMM form: out[n] (ocg x ohw) = W_g (ocg x k) * col[n, g] (k x ohw), bias per row.
@@ -1248,10 +1254,16 @@ void lower_conv(Emit& em, Plan& plan, int nid, const Epilogue* e, const Plan::Se
            [=](cudaStream_t st) { return launch_pack_filter_tc(p, s->fptr(w), s->fptr_mut(wt), st); });
     const int res = ep.residual, gv = gate ? gate->gate : -1;
     const double bytes = f32_bytes(xv) + f32_bytes(wv) + f32_bytes(ov) * (res >= 0 ? 2 : 1);
-    em.add("gemm_tf32x3_tcgen05", n.op, {x, wt, bias, gv, res}, {out}, bytes, flops, [=](cudaStream_t st) {
-      return launch_conv_tc(p, s->fptr(x), s->fptr(wt), bias >= 0 ? s->fptr(bias) : nullptr,
-                            gv >= 0 ? s->fptr(gv) : nullptr, res >= 0 ? s->fptr(res) : nullptr, s->fptr_mut(out), constants, s->err_word, st);
-    });
+    auto part = [=](cudaStream_t st, int first, int count) {
+      const size_t o = (size_t)first * p.oc * ohw;
+      return launch_conv_tc(p, count, s->fptr(x) + (size_t)first * p.c * p.ih * p.iw, s->fptr(wt), bias >= 0 ? s->fptr(bias) : nullptr,
+                            gv >= 0 ? s->fptr(gv) + (size_t)first * p.c : nullptr, res >= 0 ? s->fptr(res) + o : nullptr,
+                            s->fptr_mut(out) + o, constants, s->err_word, st);
+    };
+    Step& step = em.add("gemm_tf32x3_tcgen05", n.op, {x, wt, bias, gv, res}, {out}, bytes, flops,
+                        [=](cudaStream_t st) { return part(st, 0, p.n); });
+    step.part = part;
+    step.images = p.n;
     return;
   }
   if (small_conv_applies(*s, flops, small_columns) && !(pointwise && ohw == 1) && conv_simt_supported(p)) {

@@ -16,6 +16,7 @@
 #include "../../include/altius_session_cuda.h"
 #include "host_stage.h"
 #include "kernels.h"
+#include "pieces.h"
 #include "segments.h"
 
 namespace ac {
@@ -64,6 +65,9 @@ struct Step {
   double bytes = 0, flops = 0;     // algorithmic work
   int launches = 1;
   bool const_only = false;         // all inputs constant: executed once at create()
+  // The step on images [first, first + count) of its batch of `images`, where its kernel takes them one by one.
+  std::function<cudaError_t(cudaStream_t, int first, int count)> part;
+  int images = 0;
 };
 
 struct ProfileAcc {
@@ -118,6 +122,11 @@ struct AcSession {
   char* stage_out = nullptr;
   std::shared_ptr<ac::HostStage> host_stage;   // uploads of large pageable inputs, from the first one on
   std::vector<ac::Segment> segments;   // empty: this schedule does not run on bound buffers
+  // Runs from large host inputs: the front of the schedule per piece of the batch, the rest behind it.
+  ac::PiecePlan pieces;
+  std::vector<ac::Segment> piece_graphs;   // one a piece and one for the rest; empty: not used
+  std::vector<cudaEvent_t> piece_up;       // a piece's images are on the device
+  cudaStream_t up_stream = nullptr;
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;

@@ -92,6 +92,16 @@ int main(int argc, char** argv) {
     t.join();
     return ok && right(dst, src) ? 0 : 1;
   }
+  if (what == "sent") {                      // told of what has been handed over, in order; an error ends the upload and is passed on
+    size_t last = 0;
+    int calls = 0;
+    auto told = [&](size_t n) { const bool ok = n > last && std::memcmp(dst.data(), src.data(), n) == 0; last = n; ++calls; return ok ? cudaSuccess : cudaErrorUnknown; };
+    if (stage->upload(dst.data(), src.data(), big, nullptr, std::ref(told)) != cudaSuccess || last != big || calls != 41) return 1;
+    copies = 0;
+    auto stop = [&](size_t n) { return n < (size_t(4) << 20) ? cudaSuccess : cudaErrorLaunchFailure; };
+    if (stage->upload(dst.data(), src.data(), big, nullptr, std::ref(stop)) != cudaErrorLaunchFailure || copies != 4) return 2;
+    return stage->upload(dst.data(), src.data(), big, nullptr) == cudaSuccess && right(dst, src) ? 0 : 3;
+  }
   return 9;
 }
 """
@@ -108,6 +118,6 @@ def harness(tmp_path_factory):
     return str(d / "h")
 
 
-@pytest.mark.parametrize("what", ["copies", "fault", "two", "memory"])
+@pytest.mark.parametrize("what", ["copies", "fault", "two", "memory", "sent"])
 def test_staged_upload(harness, what):
     assert subprocess.run([harness, what], timeout=30).returncode == 0

@@ -1,0 +1,70 @@
+"""The split of a batch into pieces whose first steps run while the others' images are still on their way (pieces.h): the
+plan, the arena's part in it, and runs from host memory against runs on device buffers."""
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from altius_b200 import configs
+from altius_b200.session import CudaSessionBuilder
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+HARNESS = r"""
+#include <cstdio>
+#include "pieces.h"
+int main() {
+  for (int front = 0; front < 6; ++front)
+    for (int images = 1; images < 200; ++images)
+      for (size_t image : {size_t(12), size_t(40000), size_t(602112), size_t(3) << 20}) {
+        const ac::PiecePlan p = ac::plan_pieces(front, images, image * images);
+        if (!p.steps) { if (p.count()) return 1; continue; }
+        if (p.steps != front || front < 3 || image * images < (size_t(8) << 20) || p.per % 4 || p.count() < 2 || p.count() > 4) return 2;
+        if ((size_t)p.per * image < (size_t(2) << 20) || p.begin(0) != 0 || p.end(p.count() - 1) != images) return 3;
+        for (int k = 0; k + 1 < p.count(); ++k) if (p.end(k) != p.begin(k + 1) || p.end(k) <= p.begin(k)) return 4;
+        if (p.end(p.count() - 1) <= p.begin(p.count() - 1)) return 5;
+      }
+  std::puts("ok");
+}
+"""
+
+
+def test_plan(tmp_path):
+    src = tmp_path / "p.cpp"
+    src.write_text(HARNESS)
+    subprocess.run(["g++", "-std=c++17", "-I", os.path.join(ROOT, "altius_b200", "csrc"), "-o", str(tmp_path / "p"), str(src)], check=True)
+    assert subprocess.run([str(tmp_path / "p")], capture_output=True, text=True).stdout == "ok\n"
+
+
+def test_a_large_batch_keeps_its_front_values_apart():
+    """11 convolutions up to the first squeeze-and-excite block: no two of their values may share memory."""
+    small, large = (CudaSessionBuilder(configs.mobilenet_v3_large(batch=b, img=224)[0]).with_plan_only(True).build() for b in (4, 32))
+    front = [e["kind"] for e in large.schedule()].index("squeeze_excite")
+    assert front == 11
+    per_image = 4 * (3 * 224 ** 2 + 3 * 16 * 112 ** 2 + 64 * 112 ** 2 + 64 * 56 ** 2 + 2 * 24 * 56 ** 2 + 3 * 72 * 56 ** 2 + 72 * 28 ** 2)
+    assert large.arena_bytes >= 32 * per_image > 8 * small.arena_bytes
+
+
+# three pieces of which the last has one image, pieces of an odd plane, four even ones
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,px", [(17, 224), (21, 193), (32, 224)])
+def test_runs_in_pieces(cuda_lib, batch, px):
+    import torch
+    sess = CudaSessionBuilder(configs.mobilenet_v3_large(batch=batch, img=px)[0]).build()
+    try:
+        rng = np.random.default_rng(batch)
+        for _ in range(3):
+            x = rng.standard_normal((batch, 3, px, px)).astype(np.float32)
+            want = torch.empty(sess.output_info[0][0], device="cuda")
+            xd = torch.from_numpy(x).cuda()
+            torch.cuda.synchronize()
+            sess.run_device([xd.data_ptr()], [want.data_ptr()])
+            want = want.cpu().numpy()
+            assert np.array_equal(sess.run([x])[0], want)
+            pinned, out = torch.from_numpy(x).pin_memory(), torch.empty(want.shape).pin_memory()
+            assert np.array_equal(sess.run([pinned.numpy()], [out.numpy()])[0], want)
+            outs = [[np.empty_like(want)], [np.empty_like(want)]]
+            sess.run_batches([[x], [x]], outs)
+            assert np.array_equal(outs[0][0], want) and np.array_equal(outs[1][0], want)
+    finally:
+        sess.close()
