@@ -2056,9 +2056,9 @@ cudaError_t launch_gemm_tc(const GemmParams& q, int mode, int* err_word, cudaStr
 #undef AC_TC
 }
 
-// Whole tiles of 256 x 192, `run` K-blocks on one accumulator.
-cudaError_t launch_gemm_pair_sums(const GemmParams& q, int run, int* err_word, cudaStream_t st) {
-  constexpr int bn = 192;                      // 256 columns took 15 % more: half of the sums spill
+// Whole tiles of 256 x bn (192 or 128), `run` K-blocks on one accumulator. (256 columns took 15 % more: half of the sums spill.)
+template <int bn>
+static cudaError_t launch_pair_sums(const GemmParams& q, int run, int* err_word, cudaStream_t st) {
   const int pairs = pair_count();
   if (pairs <= 0 || run < 1 || run > 2 || encode_fn() == nullptr) return cudaErrorInvalidValue;
   CUtensorMap ma, mal, mb, mbl;
@@ -2073,7 +2073,12 @@ cudaError_t launch_gemm_pair_sums(const GemmParams& q, int run, int* err_word, c
   pl.sc.tail_parts = 0;
   pl.grid = std::min(pl.sc.num_tiles, pairs);
   pl.sc.run = run;
-  return launch_pair_key<192, true>(q, ma, mal, mb, mbl, ep, pl, nullptr, err_word, st);
+  return launch_pair_key<bn, true>(q, ma, mal, mb, mbl, ep, pl, nullptr, err_word, st);
+}
+
+cudaError_t launch_gemm_pair_sums(const GemmParams& q, PairSums t, int* err_word, cudaStream_t st) {
+  if (t.bn == 128) return launch_pair_sums<128>(q, t.run, err_word, st);
+  return t.bn == 192 ? launch_pair_sums<192>(q, t.run, err_word, st) : cudaErrorInvalidValue;
 }
 
 cudaError_t launch_f16_split(const float* x, void* hi, void* lo, int64_t rows, int64_t k, int64_t ld, int64_t k8,

@@ -291,15 +291,16 @@ int gemm_tc_pairs();
 int cluster_slots(int split);
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k);
 bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bias_scale);
-// K-blocks of 64 on one accumulator where such a product is better off on CTA pairs, or 0 for the few-row kernel itself; the
-// lowering asks, so that the schedule names the kernel that runs, and hands the answer to the launch.
-int gemm_ks_pair_run(int64_t m, int64_t n, int64_t k);
-cudaError_t launch_gemm_ks(const GemmParams& p, int pair_run, int* err_word, cudaStream_t st);
+struct PairSums { int bn = 0, run = 0; };   // tiles of 256 x bn (192 or 128); run 0: not there
+// The tiles where such a product is better off on CTA pairs, run 0 for the few-row kernel itself; the lowering asks, so that
+// the schedule names the kernel that runs, and hands the answer to the launch.
+PairSums gemm_ks_pairs(int64_t m, int64_t n, int64_t k);
+cudaError_t launch_gemm_ks(const GemmParams& p, PairSums pairs, int* err_word, cudaStream_t st);
 // The same kernel on fp32 operands as 3xTF32 (a; b and b_lo as for launch_gemm_tc), the epilogues of gemm_ks_epilogue_ok; 1e30: not for it.
 double gemm_ks_wide_clocks(int64_t m, int64_t n, int64_t k);
 cudaError_t launch_gemm_ks_wide(const GemmParams& p, int* err_word, cudaStream_t st);
 // The same operands and epilogues on CTA pairs, `run` K-blocks of 64 on one accumulator (gemm_tc.cu).
-cudaError_t launch_gemm_pair_sums(const GemmParams& p, int run, int* err_word, cudaStream_t st);
+cudaError_t launch_gemm_pair_sums(const GemmParams& p, PairSums t, int* err_word, cudaStream_t st);
 // fp16 split of a constant [rows, k] operand (row stride ld) into [rows, k8] halves
 // (k8 >= k, a multiple of 8, padding zero); leaves kGemmRangeCode in *err_word when an
 // element exceeds the fp16 range.

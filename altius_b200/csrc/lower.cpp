@@ -966,7 +966,7 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   const auto sp_a = em.c.split.find(a);
   const bool use_ks = b16_ok && sp_a != em.c.split.end() && sp_a->second.by_producer && b_row_scale < 0 && gemm_ks_applies(*s, g, true, a_off, b_off) &&
                       gemm_ks_epilogue_ok(act, bias_m >= 0, c_in >= 0, alpha, bias_scale) && c_off == 0 && g.ldc == g.n;
-  const int pair_run = use_ks ? gemm_ks_pair_run(g.m, g.n, g.k) : 0;
+  const PairSums ks_pairs = use_ks ? gemm_ks_pairs(g.m, g.n, g.k) : PairSums{};
   if (use_ks) s->narrow = true;
   const bool pre = b16_ok && (use_ks || presplit_applies(*s, g, true, a_off, b_off));
   if (b16_ok) {
@@ -1061,7 +1061,7 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
                             c_in, bias_n, bias_m, res, b_row_scale};
   const char* kind = !tc ? "gemm_fp32_simt"
                      : (mode == 2 ? "gemm_tf32x1_tcgen05"
-                                  : (b16_hi >= 0 ? (use_ks ? (pair_run ? "gemm_f16x3_pair_sums_tcgen05" : "gemm_f16x3_cluster_tcgen05")
+                                  : (b16_hi >= 0 ? (use_ks ? (ks_pairs.run ? "gemm_f16x3_pair_sums_tcgen05" : "gemm_f16x3_cluster_tcgen05")
                                                     : a16_hi >= 0 ? "gemm_f16x3_pair_tcgen05" : "gemm_f16x3_tcgen05")
                                                  : "gemm_tf32x3_tcgen05"));
   std::vector<int> writes;
@@ -1099,7 +1099,7 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
     p.bias_scale = bias_scale;
     p.act = act; p.act_alpha = aa; p.act_beta = ab;
     p.residual = res >= 0 ? s->fptr(res) + c_off : nullptr; p.ld_res = g.ldc; p.stride_res = g.sc;
-    if (use_ks) return launch_gemm_ks(p, pair_run, s->err_word, st);
+    if (use_ks) return launch_gemm_ks(p, ks_pairs, s->err_word, st);
     if (ks_wide) return launch_gemm_ks_wide(p, s->err_word, st);
     if (tc && gemm_tc_supported(p)) return launch_gemm_tc(p, mode, s->err_word, st);
     if (!p.a || !p.c || p.c16_hi || p.b_row_scale) return cudaErrorInvalidValue;   // operands exist for the tensor-core kernel only

@@ -131,6 +131,34 @@ def test_pairs_with_short_accumulators(cuda_lib, m, d, n, bound, act, res):
     assert ((got - want).abs() <= 1e-5 * want.abs() + 2e-5).all()
 
 
+# The same with a long K, behind a product that leaves the halves: tiles of 128 columns, and (last) of 192. Bound: what the few-row
+# kernel measured on these inputs (at K = 1096 and 1992 on the line between), the error of the operand, 1.5e-7, included.
+@pytest.mark.parametrize("m,d,n,bound", [(1576, 3072, 768, 5.79e-7), (1182, 4096, 1024, 7.80e-7), (2177, 1096, 772, 2.6e-7),
+                                         (2100, 1992, 900, 4.1e-7), (1970, 1280, 1280, 2.86e-7)])
+@pytest.mark.parametrize("act,res", [(None, False), ("ReLU", True)])
+def test_pairs_with_short_accumulators_and_long_k(cuda_lib, m, d, n, bound, act, res):
+    rng = np.random.default_rng(m + n)
+    x = rng.standard_normal((m, 256)).astype(np.float32)
+    w0 = (rng.standard_normal((256, d)) / 16).astype(np.float32)
+    w = (rng.standard_normal((d, n)) / np.sqrt(d)).astype(np.float32)
+    b = rng.standard_normal(n).astype(np.float32)
+    r = rng.standard_normal((m, n)).astype(np.float32)
+    g = ir.Graph()
+    xi = g.add_input("x", x.shape)
+    ri = g.add_input("r", r.shape) if res else None
+    h = g.op("LayerNormalization", xi, g.new_init(np.ones(256, np.float32)), g.new_init(np.zeros(256, np.float32)), axis=-1,
+             epsilon=1e-6, stash_type=1)
+    y = g.op("Add", g.op("MatMul", g.op("ReLU", g.op("MatMul", h, g.new_init(w0))), g.new_init(w)), g.new_init(b))
+    y = g.op(act, y) if act else y
+    g.outputs.append(g.op("Add", y, ri) if res else y)
+    got = _run(g, [x] + ([r] if res else []), ["layer_norm"] + 2 * ["gemm_f16x3_pair_sums_tcgen05"])
+    y = torch.relu(torch.nn.functional.layer_norm(_t(x), (256,), None, None, 1e-6) @ _t(w0)) @ _t(w) + _t(b)
+    y = torch.relu(y) if act else y
+    want = y + _t(r) if res else y
+    assert ((got - want).norm() / want.norm()).item() <= bound
+    assert ((got - want).abs() <= 1e-5 * want.abs() + 2e-5).all()
+
+
 @pytest.mark.parametrize("act", [None, "ReLU", "Gelu"])
 @pytest.mark.parametrize("bias,res", [(False, False), (True, False), (False, True), (True, True)])
 def test_every_epilogue_with_short_accumulators(cuda_lib, act, bias, res):
