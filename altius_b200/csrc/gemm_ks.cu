@@ -466,30 +466,25 @@ KsDev device_params(const GemmParams& q, const Shape& sh, int* err_word) {
 
 }  // namespace
 
-// Products that this kernel has more tiles than SMs for may go to CTA pairs on tiles of 256 x 192 or 256 x 128 that hand their
-// accumulators over to fp32 sums every `run` K-blocks (launch_gemm_pair_sums; run 0: stay here). Fitted in this kernel's clocks,
-// launch and ends included as in pick_shape: 1300 a K-block of such a tile and 6000 around them (us with a LayerNormalization
-// in front, here -> there: 3152 x 768 x 768 31.6 -> 23.2, 12672 x 384 x 384 37.3 -> 30.4, 788 x 768 x 3072 30.6 -> 22.7; but
-// 2885 x 768 x 768 20.5 -> 23.0, 1576 x 512 x 512 14.2 -> 18.4). Relative error against 64 bits with runs of two 1.6e-7 for
-// any K, of one 1.2e-7; here 2.1e-7 at K = 768, 2.0e-7 at 576, 1.5e-7 at 384 and 512: one there.
-// Beyond K = 1024, where this kernel takes a tenth longer than its estimate and its error grows (5.8e-7 at 3072), tiles of 128
-// columns as well: an MMA of a pair reads 4 KB of A and 16 bytes a column of B from each shared memory, 1000 clocks a K-block.
-// They fill the pairs in one round where 192 columns leave a third of them idle (us, m x k x n with a quarter of the product
+// Products that this kernel has more tiles than SMs for go to CTA pairs with short accumulators where these are faster; fitted in
+// this kernel's clocks, launch and ends included as in pick_shape (us with a LayerNormalization in front, here -> there: 3152 x
+// 768 x 768 31.6 -> 23.2, 12672 x 384 x 384 37.3 -> 30.4, 788 x 768 x 3072 30.6 -> 22.7; but 2885 x 768 x 768 20.5 -> 23.0, 1576 x
+// 512 x 512 14.2 -> 18.4). Relative error against 64 bits there 1.6e-7, to K = 576 1.2e-7; here 2.1e-7 at K = 768, 1.5e-7 at 384.
+// Tiles of 128 columns fill the pairs in one round where 192 leave a third of them idle (us, m x k x n with a quarter of the product
 // that makes the operand, here -> 128 | 192: 2885 x 3072 x 768 50.6 -> 46.2 | 53.9, 1576 x 3072 x 768 42.5 -> 39.0 | 46.6,
-// 1182 x 4096 x 1024 51.8 -> 48.0 | 57.0, 4000 x 2048 x 512 41.0 -> 37.4 | 43.2; two rounds: 3152 x 3072 x 768 77.9 -> 71.8 |
-// 55.3; few rows: 788 x 3072 x 768 26.7 -> 36.1 | 43.6). Runs of one took a tenth more there.
+// 1182 x 4096 x 1024 51.8 -> 48.0 | 57.0, 4000 x 2048 x 512 41.0 -> 37.4 | 43.2; two rounds: 9838 x 384 x 384 24.1 -> 18.6 | 21.6,
+// 3152 x 3072 x 768 77.9 -> 71.8 | 55.3; few rows: 788 x 3072 x 768 26.7 -> 36.1 | 43.6). From K = 1024 on this kernel takes a
+// tenth longer than its estimate, and its error grows (5.8e-7 at 3072).
 PairSums gemm_ks_pairs(int64_t m, int64_t n, int64_t k) {
-  const int64_t pairs = gemm_tc_pairs();
-  if (pairs <= 0) return {};
-  const int64_t nkb = (k + KB - 1) / KB;
-  auto clocks = [&](int64_t bn, double per) {
-    const int64_t tiles = ((m + 255) / 256) * ((n + bn - 1) / bn);
-    return 4000.0 + (double)((tiles + pairs - 1) / pairs) * (per * (double)nkb + 6000.0);
-  };
-  const double here = gemm_ks_clocks(m, n, k) * (k > 1024 ? 1.08 : 0.97);
-  const double wide = clocks(192, 1300.0), slim = k > 1024 ? clocks(128, 1000.0) : 1e30;
-  if (std::min(wide, slim) >= here) return {};
-  return {slim < wide ? 128 : 192, k > 576 ? 2 : 1};
+  const double here = gemm_ks_clocks(m, n, k);
+  double there;
+  const PairSums t = gemm_pair_sums_tiles(m, n, k, &there);
+  return here >= gemm_tc_pair_clocks(m, n, k) || there < here * (k >= 1024 ? 1.08 : 0.97) ? t : PairSums{};
+}
+
+bool gemm_ks_wins(int64_t m, int64_t n, int64_t k) {
+  const double here = gemm_ks_clocks(m, n, k);
+  return here < gemm_tc_pair_clocks(m, n, k) || (here < 1e30 && gemm_pair_sums_wins(m, n, k));
 }
 
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k) {

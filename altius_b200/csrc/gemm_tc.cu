@@ -1933,9 +1933,9 @@ bool gemm_tc_wants_presplit(int64_t m, int64_t n, int64_t k, int64_t batch) {
   return pick_shape(m, n, k, batch, 2, 2).pair;
 }
 
-// What the choice between this kernel and the more exact ones (gemm_ks_clocks) counts: the kernel's clocks for a K-block of a
-// 256 x 256 tile, for launch, first operands and last epilogue, and for the K-slice pass; and what the smaller error of the
-// others is worth beside each: without that products would move from errors of 2e-7 to 1e-6 for a few us (2885 x 768 x 768,
+// What the choice between this kernel and the more exact one for few rows (gemm_ks_clocks) counts: the kernel's clocks for a
+// K-block of a 256 x 256 tile, for launch, first operands and last epilogue, and for the K-slice pass; and what the smaller error
+// of the other is worth beside each: without that products would move from errors of 2e-7 to 1e-6 for a few us (2885 x 768 x 768,
 // 1576 x 512 x 512).
 constexpr double kPairBlock = 1540, kPairEnds = 18000, kPairSlices = 7500;
 constexpr double kExactBlock = 410, kExactEnds = 2000, kExactSlices = 1500;
@@ -1946,6 +1946,40 @@ double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k) {
   double blocks = (double)((pl.sc.dp_tiles + pairs - 1) / pairs) * pl.sc.num_kb;
   if (pl.sc.tail_parts >= 2) blocks += (double)pl.sc.num_kb / pl.sc.tail_parts;
   return blocks * (kPairBlock + kExactBlock) + kPairEnds + kExactEnds + (pl.sc.tail_parts >= 2 ? kPairSlices + kExactSlices : 0.0);
+}
+
+// The two forms of the pair kernel beside one another: long accumulators on tiles of 256 x 256, or short ones on 256 x 192 and
+// 256 x 128 (launch_gemm_pair_sums), whose MMAs take longer for a column, but which have no K-slices to add up in a second kernel
+// and leave a tenth of the error. Fitted over 70 products of 400 to 20000 rows by 384 to 3072 columns (us with a quarter of a
+// LayerNormalization, long -> chosen: 2885 x 768 x 2304 35.0 -> 29.4, 9456 x 768 x 768 39.0 -> 32.3, 4554 x 384 x 1536 28.6 -> 22.2,
+// 2148 x 1024 x 1024 28.1 -> 18.3, 457 x 768 x 3072 20.3 -> 14.1; stay: 5742 x 384 x 1152 20.1, there 22.6; 5443 x 768 x 768
+// 22.1, 24.0; 18062 x 768 x 2304 137, 177).
+// An MMA of a pair reads 4 KB of A and 16 bytes a column of B from each shared memory: 1300 clocks for a K-block of 192 columns,
+// 1000 of 128.
+PairSums gemm_pair_sums_tiles(int64_t m, int64_t n, int64_t k, double* clocks) {
+  const int64_t pairs = pair_count(), nkb = (k + 63) / 64;
+  *clocks = 1e30;
+  if (pairs <= 0) return {};
+  const int run = k > 576 ? 2 : 1;           // K-blocks on one accumulator: errors of 1.6e-7 for any K, of 1.2e-7
+  auto tiled = [&](int64_t bn, double per) {
+    const int64_t tiles = ((m + 255) / 256) * ((n + bn - 1) / bn);
+    return 4000.0 + (double)((tiles + pairs - 1) / pairs) * ((per + (run == 1 ? 100.0 : 0.0)) * (double)nkb + 6000.0);
+  };
+  const double c192 = tiled(192, 1300.0), c128 = tiled(128, 1000.0);
+  *clocks = std::min(c192, c128);
+  return {c128 < c192 ? 128 : 192, run};
+}
+
+bool gemm_pair_sums_wins(int64_t m, int64_t n, int64_t k) {
+  const int pairs = pair_count();
+  double there;
+  if (gemm_pair_sums_tiles(m, n, k, &there).run == 0) return false;
+  const TcPlan pl = make_plan(m, n, k, 1, 256, 2, 64, pairs);
+  const bool slices = pl.sc.tail_parts >= 2;
+  double blocks = (double)((pl.sc.dp_tiles + pairs - 1) / pairs) * pl.sc.num_kb;
+  if (slices) blocks += (double)pl.sc.num_kb / pl.sc.tail_parts;
+  const double sliced = slices ? 8000.0 + 80.0 * (pl.sc.num_tiles - pl.sc.dp_tiles) * pl.sc.tail_parts : 0.0;
+  return there < 0.97 * (kPairBlock * blocks + 12000.0 + sliced);
 }
 
 // The same for 3xTF32 products with a prepared B, beside gemm_ks_wide_clocks: fitted over 150 products of 64 to 9456 rows by 192 to

@@ -291,15 +291,21 @@ int gemm_tc_pairs();
 int cluster_slots(int split);
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k);
 bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bias_scale);
-struct PairSums { int bn = 0, run = 0; };   // tiles of 256 x bn (192 or 128); run 0: not there
-// The tiles where such a product is better off on CTA pairs, run 0 for the few-row kernel itself; the lowering asks, so that
-// the schedule names the kernel that runs, and hands the answer to the launch.
+struct PairSums { int bn = 0, run = 0; };   // tiles of 256 x bn (192 or 128), `run` K-blocks of 64 on one accumulator; run 0: not there
+// The pair kernel with short accumulators: its tiles and clocks, and whether it is
+// better off than the one with long ones.
+PairSums gemm_pair_sums_tiles(int64_t m, int64_t n, int64_t k, double* clocks);
+bool gemm_pair_sums_wins(int64_t m, int64_t n, int64_t k);
+// Whether a product is better off on the kernel for few rows or on pairs with short accumulators than with long ones, and the
+// tiles if it is the pairs, run 0 for the kernel itself; the lowering asks, so that the schedule names the kernel that runs, and
+// hands the answer to the launch.
+bool gemm_ks_wins(int64_t m, int64_t n, int64_t k);
 PairSums gemm_ks_pairs(int64_t m, int64_t n, int64_t k);
 cudaError_t launch_gemm_ks(const GemmParams& p, PairSums pairs, int* err_word, cudaStream_t st);
 // The same kernel on fp32 operands as 3xTF32 (a; b and b_lo as for launch_gemm_tc), the epilogues of gemm_ks_epilogue_ok; 1e30: not for it.
 double gemm_ks_wide_clocks(int64_t m, int64_t n, int64_t k);
 cudaError_t launch_gemm_ks_wide(const GemmParams& p, int* err_word, cudaStream_t st);
-// The same operands and epilogues on CTA pairs, `run` K-blocks of 64 on one accumulator (gemm_tc.cu).
+// The same operands and epilogues on CTA pairs with short accumulators (gemm_tc.cu).
 cudaError_t launch_gemm_pair_sums(const GemmParams& p, PairSums t, int* err_word, cudaStream_t st);
 // fp16 split of a constant [rows, k] operand (row stride ld) into [rows, k8] halves
 // (k8 >= k, a multiple of 8, padding zero); leaves kGemmRangeCode in *err_word when an

@@ -809,7 +809,7 @@ bool gemm_ks_applies(const AcSession& s, const GemmShape& g, bool b_const, int64
     return false;
   if (g.tb ? (g.ldb % 4) != 0 : (g.k % 4) != 0) return false;
   if (2.0 * g.m * g.n * g.k < std::max(double(1 << 20), tensor_core_floor(g))) return false;   // emit_gemm's floor, too
-  return gemm_ks_clocks(g.m, g.n, g.k) < gemm_tc_pair_clocks(g.m, g.n, g.k);
+  return gemm_ks_wins(g.m, g.n, g.k);
 }
 
 GemmShape matmul_shape(Ctx& c, const Node& n, bool trans_b_folded) {
