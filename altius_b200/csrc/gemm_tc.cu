@@ -1954,8 +1954,8 @@ double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k) {
 // LayerNormalization, long -> chosen: 2885 x 768 x 2304 35.0 -> 29.4, 9456 x 768 x 768 39.0 -> 32.3, 4554 x 384 x 1536 28.6 -> 22.2,
 // 2148 x 1024 x 1024 28.1 -> 18.3, 457 x 768 x 3072 20.3 -> 14.1; stay: 5742 x 384 x 1152 20.1, there 22.6; 5443 x 768 x 768
 // 22.1, 24.0; 18062 x 768 x 2304 137, 177).
-// An MMA of a pair reads 4 KB of A and 16 bytes a column of B from each shared memory: 1300 clocks for a K-block of 192 columns,
-// 1000 of 128.
+// An SM takes 32 KB of A and 128 bytes a column of B from L2 for a K-block: 1300 clocks with 192 columns, 1000 with 128, 43 to 48
+// bytes a clock.
 PairSums gemm_pair_sums_tiles(int64_t m, int64_t n, int64_t k, double* clocks) {
   const int64_t pairs = pair_count(), nkb = (k + 63) / 64;
   *clocks = 1e30;

@@ -967,8 +967,11 @@ void emit_gemm(Emit& em, int op, const GemmShape& g_in, int a, int b, int out, i
   const bool use_ks = b16_ok && sp_a != em.c.split.end() && sp_a->second.by_producer && b_row_scale < 0 && gemm_ks_applies(*s, g, true, a_off, b_off) &&
                       gemm_ks_epilogue_ok(act, bias_m >= 0, c_in >= 0, alpha, bias_scale) && c_off == 0 && g.ldc == g.n;
   const PairSums ks_pairs = use_ks ? gemm_ks_pairs(g.m, g.n, g.k) : PairSums{};
-  if (use_ks) s->narrow = true;
-  const bool pre = b16_ok && (use_ks || presplit_applies(*s, g, true, a_off, b_off));
+  const bool on_pairs = b16_ok && presplit_applies(*s, g, true, a_off, b_off);
+  // (The pairs with long accumulators take operands on the same scale: where they are next in line, a plan without the others would
+  // leave its range as well.)
+  if (use_ks && (!on_pairs || gemm_ks_clocks(g.m, g.n, g.k) < gemm_tc_pair_clocks(g.m, g.n, g.k))) s->narrow = true;
+  const bool pre = use_ks || on_pairs;
   if (b16_ok) {
     ldb16 = (g.k + 7) / 8 * 8;
     const int64_t floats = g.n * ldb16 / 2;     // two halves per float of scratch
