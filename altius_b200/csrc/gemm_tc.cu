@@ -1954,7 +1954,7 @@ double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k) {
 // LayerNormalization, long -> chosen: 2885 x 768 x 2304 35.0 -> 29.4, 9456 x 768 x 768 39.0 -> 32.3, 4554 x 384 x 1536 28.6 -> 22.2,
 // 2148 x 1024 x 1024 28.1 -> 18.3, 457 x 768 x 3072 20.3 -> 14.1; stay: 5742 x 384 x 1152 20.1, there 22.6; 5443 x 768 x 768
 // 22.1, 24.0; 18062 x 768 x 2304 137, 177). With a Gelu or a residual, which only the long ones have under the next tile's
-products, what is chosen is still 0 to 20 % faster (9306 x 384 x 1152 45.6 -> 45.1 with a residual, 2885 x 768 x 2304 37.3 -> 33.3 with a Gelu).
+// products, what is chosen is still 0 to 20 % faster (9306 x 384 x 1152 45.6 -> 45.1 with a residual, 2885 x 768 x 2304 37.3 -> 33.3 with a Gelu).
 // An SM takes 32 KB of A and 128 bytes a column of B from L2 for a K-block: 1300 clocks with 192 columns, 1000 with 128, 43 to 48
 // bytes a clock.
 PairSums gemm_pair_sums_tiles(int64_t m, int64_t n, int64_t k, double* clocks) {
