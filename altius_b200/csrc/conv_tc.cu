@@ -73,7 +73,12 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 // registers: a quarter of an SM holds five such warps (16384 registers), so that two blocks of nine fit. With 112 it holds four,
 // one block per SM, whatever the shared memory leaves (32 images of 16 x 112 x 112 into 64 channels: 9 warps active, issue 37 %,
 // 56 us; MobileNetV3-Large at 32 images 919 us, with two blocks 798).
-template <bool WINDOW, int ACT, bool ONE, bool ALONE>
+// CUT: a pointwise product whose K is cut over a cluster, with the exchange unrolled: stores to one owner without a test per value, eight
+// channels of the final sum under way at once (one behind the other they took 310 clocks each, and of 37000 clocks of 32 images of
+// 672 x 14 x 14 into 112 the exchange had 13000): 18.4 -> 15.4 us, 8 of 512 x 28 x 28 into 128 16.9 -> 13.3, 32 of 960 x 7 x 7 into
+// 160 12.9 -> 12.3. A kernel of its own, without the code for a block that cuts nothing (with it 1 us more); unrolled in the others it
+// cost those that cut nothing 0.9 us, taken out of them 0.3 to 0.7. Windows keep the plain form.
+template <bool WINDOW, int ACT, bool ONE, bool ALONE, bool CUT>
 __global__ void __maxnreg__(ALONE ? 112 : 96) conv_tc_kernel(const ConvTcDev p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -87,14 +92,14 @@ __global__ void __maxnreg__(ALONE ? 112 : 96) conv_tc_kernel(const ConvTcDev p) 
   const int bbytes = bn * KB * 8, stage_bytes = 2 * kABytes + (p.resident ? 0 : bbytes);
   uint8_t* wres = smem + S * stage_bytes;      // the resident filter tile
   float* part = reinterpret_cast<float*>(wres + (p.resident ? p.kper * bbytes : 0));   // [parts][bn / parts][PX] sums of the cluster
-  int2* tab = reinterpret_cast<int2*>(part + (parts > 1 ? bn * PX : 0));
+  int2* tab = reinterpret_cast<int2*>(part + (CUT || parts > 1 ? bn * PX : 0));
   const int tiles = (p.n + PX - 1) / PX, mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   // Accumulators of a tile: [cross terms | main terms of even | of odd K steps], or one for all.
   const uint32_t set = p.set, cols = p.cols, span = (p.mains + 1) * set;
   const int mains = ONE ? 0 : min(p.mains, kbs);   // in use
   const int two = ONE ? 1 : p.bufs - 1;        // tile i has buffer i & two, for the (i >> two)-th time
   cg::cluster_group cl = cg::this_cluster();
-  if (parts > 1) cl.barrier_arrive();          // answered before the first write to another block's memory
+  if (CUT || parts > 1) cl.barrier_arrive();          // answered before the first write to another block's memory
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -147,7 +152,7 @@ __global__ void __maxnreg__(ALONE ? 112 : 96) conv_tc_kernel(const ConvTcDev p) 
     }
   }
   pdl_wait();
-  if (parts > 1) cl.barrier_wait();
+  if (CUT || parts > 1) cl.barrier_wait();
 
   auto finish = [&](float v, float bias) { return apply_act(ACT, __fadd_rn(v, bias), p.act_alpha, p.act_beta); };
   const size_t hw4 = (size_t)p.hw * 4;         // bytes between channels
@@ -304,12 +309,18 @@ __global__ void __maxnreg__(ALONE ? 112 : 96) conv_tc_kernel(const ConvTcDev p) 
 #pragma unroll
           for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(__fadd_rn(__uint_as_float(u[j]), __uint_as_float(more[j])));
         };
-        if (parts > 1) {
+        if (CUT || parts > 1) {
           // To the block that finishes these channels; no one waits for a remote load.
           if (mains > 1) add(2 * set);
           if (mains) add(0u);
           else tc_wait_ld(u);
           int owner = c / share, left = share - c % share;
+          if (CUT && left >= 16) {
+            float* dst = cl.map_shared_rank(part, owner) + ((int)blockIdx.z * share + (share - left)) * PX + row;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) dst[e * PX] = __uint_as_float(u[e]);
+            continue;
+          }
           for (int j = 0; j < 16;) {           // uniform: channels per owner are a multiple of two
             float* dst = cl.map_shared_rank(part, owner) + ((int)blockIdx.z * share + (share - left)) * PX + row;
             const int run = min(left, 16 - j);
@@ -411,22 +422,50 @@ __global__ void __maxnreg__(ALONE ? 112 : 96) conv_tc_kernel(const ConvTcDev p) 
   }
   __syncwarp();
 
-  if (parts > 1) {
+  if (CUT || parts > 1) {
     // Every block of the cluster finishes its share of the channels of the one tile.
     cl.sync();
     const int share = bn / parts, c0 = blockIdx.z * share, row = tid & (PX - 1), col = blockIdx.x * PX + row;
     if (warp < kLoaders / 32 && col < p.n) {
       const int cb = col / p.hw;
       const long long at = cb * p.out_batch + (col - cb * p.hw) + (long long)m0 * p.hw;
+      if constexpr (CUT) {
+        constexpr int G = 8;
+        char* o = reinterpret_cast<char*>(p.out + at) + c0 * hw4;
+        const char* rs = p.res ? reinterpret_cast<const char*>(p.res + at) + c0 * hw4 : nullptr;
+        const int last = min(share - 1, mlast - c0);
+#pragma unroll 1
+        for (int c1 = tid >> 7; c1 <= last; c1 += 2 * G) {
+          float r[G], sum[G];
+#pragma unroll
+          for (int i = 0; i < G; ++i) {
+            r[i] = sum[i] = 0.f;
+            if (rs) r[i] = *reinterpret_cast<const float*>(rs + (uint32_t)min(c1 + 2 * i, last) * hw4);
+          }
+          for (int q = 0; q < parts; ++q) {
+            const float* from = part + q * share * PX + row;
+#pragma unroll
+            for (int i = 0; i < G; ++i) sum[i] = __fadd_rn(sum[i], from[min(c1 + 2 * i, last) * PX]);
+          }
+#pragma unroll
+          for (int i = 0; i < G; ++i) {
+            const int c = c1 + 2 * i;
+            float y = finish(sum[i], bias_s[c0 + min(c, last)]);
+            if (rs) y = __fadd_rn(y, r[i]);
+            if (c <= last) *reinterpret_cast<float*>(o + (uint32_t)c * hw4) = y;
+          }
+        }
+      } else {
 #pragma unroll 2
-      for (int c = tid >> 7; c < share; c += 2) {
-        if (c0 + c > mlast) break;
-        const float r = p.res ? p.res[at + (long long)(c0 + c) * p.hw] : 0.f;
-        float sum = 0.f;
-        for (int q = 0; q < parts; ++q) sum = __fadd_rn(sum, part[(q * share + c) * PX + row]);
-        float y = finish(sum, bias_s[c0 + c]);
-        if (p.res) y = __fadd_rn(y, r);
-        p.out[at + (long long)(c0 + c) * p.hw] = y;
+        for (int c = tid >> 7; c < share; c += 2) {
+          if (c0 + c > mlast) break;
+          const float r = p.res ? p.res[at + (long long)(c0 + c) * p.hw] : 0.f;
+          float sum = 0.f;
+          for (int q = 0; q < parts; ++q) sum = __fadd_rn(sum, part[(q * share + c) * PX + row]);
+          float y = finish(sum, bias_s[c0 + c]);
+          if (p.res) y = __fadd_rn(y, r);
+          p.out[at + (long long)(c0 + c) * p.hw] = y;
+        }
       }
     }
   }
@@ -470,12 +509,12 @@ Shape shape_of(const ConvParams& q) {
   return pick_shape(q, {device_sm_count(), cluster_slots(2), cluster_slots(4), cluster_slots(8)});
 }
 
-template <bool WINDOW, int ACT, bool ONE, bool ALONE>
+template <bool WINDOW, int ACT, bool ONE, bool ALONE, bool CUT>
 cudaError_t launch_form(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
   static unsigned long long done = 0;
-  if (cudaError_t e = ensure_dynamic_smem(conv_tc_kernel<WINDOW, ACT, ONE, ALONE>, (int)kSmemMax, &done)) return e;
+  if (cudaError_t e = ensure_dynamic_smem(conv_tc_kernel<WINDOW, ACT, ONE, ALONE, CUT>, (int)kSmemMax, &done)) return e;
   const dim3 grid((unsigned)sh.ctas, (unsigned)sh.tiles, (unsigned)sh.split);
-  return launch_pdl(conv_tc_kernel<WINDOW, ACT, ONE, ALONE>, grid, dim3(kThreads), sh.smem, st, sh.split, p);
+  return launch_pdl(conv_tc_kernel<WINDOW, ACT, ONE, ALONE, CUT>, grid, dim3(kThreads), sh.smem, st, sh.split, p);
 }
 
 template <bool WINDOW, int ACT>
@@ -485,9 +524,12 @@ cudaError_t launch_act(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
   // images of 192 x 192: 925 us, without 912); where only the grid is too small for two on an SM, and with a window, it gains on
   // some shapes what it loses on others.
   const bool alone = sh.smem > kSmemSm / 2 - kSmemBeside && sh.ctas < (p.n + PX - 1) / PX;
-  if constexpr (!WINDOW)
-    if (alone) return sh.mains == 0 ? launch_form<WINDOW, ACT, true, true>(p, sh, st) : launch_form<WINDOW, ACT, false, true>(p, sh, st);
-  return sh.mains == 0 ? launch_form<WINDOW, ACT, true, false>(p, sh, st) : launch_form<WINDOW, ACT, false, false>(p, sh, st);
+  if constexpr (!WINDOW) {
+    if (alone) return sh.mains == 0 ? launch_form<WINDOW, ACT, true, true, false>(p, sh, st) : launch_form<WINDOW, ACT, false, true, false>(p, sh, st);
+    if (sh.split > 1)
+      return sh.mains == 0 ? launch_form<WINDOW, ACT, true, false, true>(p, sh, st) : launch_form<WINDOW, ACT, false, false, true>(p, sh, st);
+  }
+  return sh.mains == 0 ? launch_form<WINDOW, ACT, true, false, false>(p, sh, st) : launch_form<WINDOW, ACT, false, false, false>(p, sh, st);
 }
 
 template <bool WINDOW>

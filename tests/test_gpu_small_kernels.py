@@ -79,6 +79,29 @@ def test_small_convolution_behind_a_kernel(cuda_lib, n, c, h, oc, k, p, gate):
     assert (np.abs(got - want) <= (c * k * k + 8) * EPS * mass).all()
 
 
+# Pointwise on the tensor cores with K cut over a cluster of two, four or eight: channels of a block that are no multiple of sixteen
+# or of the eight under way at once, a last tile with channels that do not exist, ragged pixels. Bound: that of the split products.
+@pytest.mark.parametrize("n,c,h,oc", [(4, 672, 14, 112), (5, 512, 9, 130), (1, 2048, 7, 500), (8, 1024, 8, 47), (32, 240, 14, 80), (13, 960, 6, 161)])
+@pytest.mark.parametrize("act,res,gate", [(None, False, False), ("ReLU", True, False), (None, True, True)])
+def test_pointwise_convolution_cut_over_a_cluster(cuda_lib, n, c, h, oc, act, res, gate):
+    rng = np.random.default_rng(c + oc)
+    x, r = rng.standard_normal((n, c, h, h)).astype(np.float32), rng.standard_normal((n, oc, h, h)).astype(np.float32)
+    w, b, gt = rng.standard_normal((oc, c, 1, 1)).astype(np.float32), rng.standard_normal(oc).astype(np.float32), rng.random((n, c, 1, 1)).astype(np.float32)
+
+    def build(g, xi, *more):
+        y = _conv(g, g.op("Mul", xi, more[-1]) if gate else xi, w, b)
+        y = g.op(act, y) if act else y
+        return g.op("Add", y, more[0]) if res else y
+    got = _run(build, [x] + ([r] if res else []) + ([gt] if gate else []), ["gemm_tf32x3_tcgen05"])
+    xg = (x * gt if gate else x).astype(np.float64).transpose(0, 2, 3, 1)
+    back = lambda a: a.transpose(0, 3, 1, 2)
+    want = back(xg @ w[:, :, 0, 0].T.astype(np.float64) + b)
+    mass = back(np.abs(xg) @ np.abs(w[:, :, 0, 0].T).astype(np.float64) + np.abs(b))
+    want = np.maximum(want, 0) if act else want
+    want = want + r if res else want
+    assert (np.abs(got - want) <= 1e-5 * np.abs(want) + 5e-6 * mass).all()
+
+
 # one, two and three images per cluster, with a remainder; planes with and without whole float4s
 @pytest.mark.parametrize("n,c,h,s", [(1, 72, 28, 24), (3, 960, 7, 240), (19, 120, 14, 32), (41, 36, 5, 4), (1, 8, 1, 8)])
 def test_squeeze_excite_block(cuda_lib, n, c, h, s):
