@@ -18,8 +18,8 @@
 // wide planes are bound by HBM if loads, MMAs and stores of different tiles overlap: two blocks share
 // an SM and each walks tiles; the loads of the next tile are in flight, and its MMAs run into a second
 // buffer of accumulators where tensor memory has one, while a tile is finished and stored. The narrow planes (7 x 7, 14 x 14) have few tiles
-// and a long K and are bound by the MMA rate of one SM (about 110 clocks per instruction whatever its
-// width): there a cluster of up to eight blocks cuts K and adds its accumulators up through
+// and a long K and are bound by the K steps of one SM (1500 to 2000 clocks each: loads, split, stores and
+// barrier one behind the other): there a cluster of up to eight blocks cuts K and adds its accumulators up through
 // distributed shared memory, in rank order.
 #include <cooperative_groups.h>
 
