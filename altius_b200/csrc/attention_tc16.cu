@@ -30,12 +30,13 @@
 // apart). Every mbarrier wait is bounded; on expiry the kernel records a code in the error
 // word and runs to its end without waiting again.
 //
-// What bounds it (clock stamps, 197 tokens): 5450 clocks an item. A group takes 10.9 K from its scores to its next ones: pass 1
+// What bounds it (clock stamps, 197 tokens): about 5500 clocks an item. A group takes 10.9 K from its scores to its next ones: pass 1
 // 1200, pass 2 5000 (tensor memory is read and written beside the MMAs), 600 until the last product is done,
 // then 3900 for the next scores, under which the output (3000) is written. The MMAs take 4200 an item. Before (7200 an item): the
 // output stored a row per lane, 32 lines with every store (4300 clocks; 3000 with 64 bytes of a row at a time), the
-// products of a stage issued in a loop (twice the time an instruction), a mask on every score, and a wait for
-// products that are in front in the pipe anyway. 32 images of 12 heads 31 -> 25 us, 96 images 104 -> 85, 64 of 6 heads 30 -> 24.
+// products of a stage issued in a loop (twice the time an instruction) and a mask on every score. 32 images of 12 heads
+// 31 -> 25.5 us, 96 images 104 -> 85, 64 of 6 heads 30 -> 24.5; 0.4 of these us are the wait between the products that read
+// P and the scores that overwrite it.
 // Not kept: chunks of pass 2 loaded one ahead (pass 2 6000 to 7000 clocks), two chunks at a time (5100).
 #include <cuda.h>
 
@@ -222,7 +223,9 @@ attention_tc16_kernel(const __grid_constant__ CUtensorMap tm_q_hi, const __grid_
         AT16_MSTAMP(i, 0);
         if (!mbar_wait(&q_full[j], (uint32_t)((i >> 1) & 1))) { atomicExch(p.err, 34); ok = false; return; }
         if (tile == 0 && !mbar_wait(k_full, (uint32_t)(u & 1))) { atomicExch(p.err, 35); ok = false; return; }
-        // P of item i - 2 lies where these scores go: the products that read it are in front in the pipe.
+        // P of item i - 2 lies where these scores go: the products that read it must be complete (MMAs of another shape and
+        // accumulator are not among those that PTX keeps in order).
+        if (i >= 2 && !mbar_wait(&o_full[j], (uint32_t)(((i >> 1) - 1) & 1))) { atomicExch(p.err, 36); ok = false; return; }
         tc_fence_after();
         AT16_MSTAMP(i, 1);
         const uint32_t d = tmem_base + (j ? kS1Col : 0u);

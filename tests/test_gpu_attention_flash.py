@@ -41,7 +41,7 @@ def _model(B, T, H, w, b, scale_op, projection):
     (3, 129, 12, "Mul", True, False), (6, 200, 12, "Div", True, False), (12, 209, 12, "Mul", True, False),
     (9, 256, 12, "Mul", True, True), (2, 257, 2, "Mul", False, False), (1, 577, 12, "Mul", False, True),
     (5, 577, 12, "Mul", True, False), (3, 321, 1, "Div", False, True), (1, 1024, 3, None, False, False),
-    (2, 513, 3, "Mul", False, True), (3, 1100, 2, "Mul", False, True)])
+    (2, 513, 3, "Mul", False, True), (3, 1100, 2, "Mul", False, True), (20, 300, 12, "Mul", True, True)])
 def test_flash_attention(cuda_lib, B, T, H, scale_op, projection, peaks):
     rng = np.random.default_rng(T + H)
     D = 64 * H
