@@ -187,15 +187,23 @@ __global__ void __launch_bounds__(kThreads) squeeze_excite_kernel(const SqueezeE
   }
 }
 
+constexpr int kMaxVector = 3072;      // c + s
+
+template <int G, bool POOL, bool WARM>
+cudaError_t launch_form(const SqueezeExciteParams& p, cudaStream_t st) {
+  // Four images' vectors are 48 KB, which a kernel may use unasked only without the barrier beside them.
+  static unsigned long long done = 0;
+  if (cudaError_t e = ensure_dynamic_smem(squeeze_excite_kernel<G, POOL, WARM>, G * kMaxVector * (int)sizeof(float), &done)) return e;
+  return launch_pdl(squeeze_excite_kernel<G, POOL, WARM>, dim3((unsigned)((p.n + G - 1) / G), 1, kCluster), dim3(kThreads),
+                    (size_t)G * (p.c + p.s) * sizeof(float), st, kCluster, p);
+}
+
 template <int G>
 cudaError_t launch_g(const SqueezeExciteParams& p, cudaStream_t st) {
-  const dim3 grid((unsigned)((p.n + G - 1) / G), 1, kCluster);
-  const size_t smem = (size_t)G * (p.c + p.s) * sizeof(float);
   // A block fills an SM: it starts under the kernel in front, and has the time for a pass ahead, only while most SMs are free.
-  if (!p.mean) return launch_pdl(squeeze_excite_kernel<G, true, false>, grid, dim3(kThreads), smem, st, kCluster, p);
-  if (G == 1 && 2 * (int)grid.x * kCluster <= device_sm_count())
-    return launch_pdl(squeeze_excite_kernel<1, false, true>, grid, dim3(kThreads), smem, st, kCluster, p);
-  return launch_pdl(squeeze_excite_kernel<G, false, false>, grid, dim3(kThreads), smem, st, kCluster, p);
+  if (!p.mean) return launch_form<G, true, false>(p, st);
+  if (G == 1 && 2 * p.n * kCluster <= device_sm_count()) return launch_form<1, false, true>(p, st);
+  return launch_form<G, false, false>(p, st);
 }
 
 inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
@@ -203,9 +211,8 @@ inline bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) =
 }  // namespace
 
 bool squeeze_excite_supported(const SqueezeExciteParams& p) {
-  // Rows of the weights (and of the vectors in shared memory) are read as float4s; four images'
-  // vectors fit the 48 KB every kernel may use.
-  return p.c >= 8 && (p.c % 4) == 0 && p.s >= 4 && (p.s % 4) == 0 && p.c + p.s <= 3072 && p.n >= 1 && p.hw >= 1 &&
+  // Rows of the weights (and of the vectors in shared memory) are read as float4s.
+  return p.c >= 8 && (p.c % 4) == 0 && p.s >= 4 && (p.s % 4) == 0 && p.c + p.s <= kMaxVector && p.n >= 1 && p.hw >= 1 &&
          p.hw < (1 << 28);
 }
 

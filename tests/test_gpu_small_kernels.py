@@ -340,5 +340,12 @@ def test_product_of_eight_rows_in_parts_of_k(cuda_lib, m, k, n):
     assert (np.abs(got[rest] - a64 @ w64.T) <= (k + 8) * EPS * (np.abs(a64) @ np.abs(w64).T)).all()
 
 
-def test_squeeze_excite_block_with_four_images_a_cluster(cuda_lib):
-    test_squeeze_excite_block(cuda_lib, 47, 36, 5, 4)   # 31 to 45 images are three a cluster
+# 31 to 45 images are three a cluster; the widest vectors that the block takes, one image and four a cluster
+@pytest.mark.parametrize("n,c,h,s", [(47, 36, 5, 4), (2, 2560, 2, 512), (61, 3056, 1, 16), (47, 2560, 2, 512)])
+def test_squeeze_excite_block_with_four_images_a_cluster(cuda_lib, n, c, h, s):
+    test_squeeze_excite_block(cuda_lib, n, c, h, s)
+
+
+# ... and behind a depthwise convolution that leaves the means
+def test_squeeze_excite_block_with_four_images_a_cluster_from_means(cuda_lib):
+    test_depthwise_in_front_of_squeeze_excite(cuda_lib, 47, 2688, 2, 3, 1, 384, True, "ReLU")
