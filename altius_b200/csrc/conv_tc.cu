@@ -518,12 +518,12 @@ cudaError_t launch_form(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
 }
 
 template <bool WINDOW, int ACT>
-cudaError_t launch_act(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
+cudaError_t launch_act(const ConvTcDev& p, const Shape& sh, bool walks, cudaStream_t st) {
   // Walking blocks of more than half of an SM's shared memory (calls of 32 x 117 x 57 x 57 into 216: with the second set 94 us,
   // without 101; 13 x 326 x 57 x 57 into 170: 79 and 78). Blocks of that size with a tile each lose by it (MobileNetV3-Large, 56
   // images of 192 x 192: 925 us, without 912); where only the grid is too small for two on an SM, and with a window, it gains on
   // some shapes what it loses on others.
-  const bool alone = sh.smem > kSmemSm / 2 - kSmemBeside && sh.ctas < (p.n + PX - 1) / PX;
+  const bool alone = sh.smem > kSmemSm / 2 - kSmemBeside && walks;
   if constexpr (!WINDOW) {
     if (alone) return sh.mains == 0 ? launch_form<WINDOW, ACT, true, true, false>(p, sh, st) : launch_form<WINDOW, ACT, false, true, false>(p, sh, st);
     if (sh.split > 1)
@@ -533,12 +533,12 @@ cudaError_t launch_act(const ConvTcDev& p, const Shape& sh, cudaStream_t st) {
 }
 
 template <bool WINDOW>
-cudaError_t launch_one(const ConvTcDev& p, const Shape& sh, int act, cudaStream_t st) {
+cudaError_t launch_one(const ConvTcDev& p, const Shape& sh, bool walks, int act, cudaStream_t st) {
   switch (act) {
-    case ACT_NONE: return launch_act<WINDOW, ACT_NONE>(p, sh, st);
-    case ACT_RELU: return launch_act<WINDOW, ACT_RELU>(p, sh, st);
-    case ACT_HARDSWISH: return launch_act<WINDOW, ACT_HARDSWISH>(p, sh, st);
-    case ACT_HARDSIGMOID: return launch_act<WINDOW, ACT_HARDSIGMOID>(p, sh, st);
+    case ACT_NONE: return launch_act<WINDOW, ACT_NONE>(p, sh, walks, st);
+    case ACT_RELU: return launch_act<WINDOW, ACT_RELU>(p, sh, walks, st);
+    case ACT_HARDSWISH: return launch_act<WINDOW, ACT_HARDSWISH>(p, sh, walks, st);
+    case ACT_HARDSIGMOID: return launch_act<WINDOW, ACT_HARDSIGMOID>(p, sh, walks, st);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -573,6 +573,7 @@ cudaError_t launch_conv_tc(const ConvParams& q, int images, const float* x, cons
   p.x = x; p.w = packed; p.out = out; p.bias = bias; p.res = residual; p.gate = gate;
   p.m = q.oc; p.k = q.c * q.kh * q.kw; p.hw = q.oh * q.ow; p.n = images * p.hw;
   if (p.m == 0 || p.n == 0) return cudaSuccess;
+  const bool walks = sh.ctas < (q.n * p.hw + PX - 1) / PX;   // in the whole batch: a part takes the whole's kernel
   sh.ctas = std::min(sh.ctas, (p.n + PX - 1) / PX);
   p.bn = sh.bn; p.stages = sh.stages; p.kper = sh.kper; p.resident = sh.resident;
   p.set = sh.set; p.mains = sh.mains; p.bufs = sh.bufs; p.cols = sh.cols;
@@ -584,7 +585,7 @@ cudaError_t launch_conv_tc(const ConvParams& q, int images, const float* x, cons
   p.err = err_word;
   const bool window = q.kh != 1 || q.kw != 1 || q.sh != 1 || q.sw != 1 || q.pad_t || q.pad_l || q.oh != q.ih || q.ow != q.iw;
   if (window && gate) return cudaErrorInvalidValue;
-  return window ? launch_one<true>(p, sh, q.act, st) : launch_one<false>(p, sh, q.act, st);
+  return window ? launch_one<true>(p, sh, walks, q.act, st) : launch_one<false>(p, sh, walks, q.act, st);
 }
 
 }  // namespace ac

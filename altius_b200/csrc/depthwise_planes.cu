@@ -9,8 +9,7 @@
 // row contributes to in registers: K shared-memory loads and K * K products a pixel, the filter in registers. The
 // taps of a result are added in the order of the generic kernel and those outside the plane are
 // skipped, so the results are the same bits.
-#include <algorithm>
-
+#include "depthwise_planes_shape.h"
 #include "kernels.h"
 #include "pdl.cuh"
 #include "plane_means.cuh"
@@ -19,15 +18,12 @@
 namespace ac {
 namespace {
 
-constexpr int kMaxThreads = 512;
-constexpr size_t kMaxSmem = 100 << 10;      // two blocks an SM
+using namespace depthwise_planes;
 
 struct PlanesDev {
   const float* x; const float* w; const float* bias; float* out; float* means;
   int planes, c, ih, iw, oh, ow, pad_t, pad_l;
-  int per;                   // planes a block
-  int stride;                // floats from plane to plane in shared memory
-  int rows, segs;            // output rows a thread, threads down a column
+  int per, stride, rows, segs;   // see Shape
   float act_alpha, act_beta;
 };
 
@@ -140,43 +136,19 @@ cudaError_t launch_act(const PlanesDev& d, int act, int threads, size_t smem, in
 
 }  // namespace
 
-bool depthwise_planes_supported(const ConvParams& p) {
-  const long long ihw = (long long)p.ih * p.iw;
-  return p.kh == p.kw && (p.kh == 3 || p.kh == 5) && p.sh == 1 && p.sw == 1 && p.dh == 1 && p.dw == 1 &&
-         (p.act == ACT_NONE || p.act == ACT_RELU || p.act == ACT_HARDSWISH) && p.ow <= kMaxThreads / 4 &&
-         (ihw + 32) * (long long)sizeof(float) * ((ihw & 3) ? 4 : 1) <= (long long)kMaxSmem && (long long)p.n * p.c < (1ll << 30) &&
-         p.oh >= 1 && p.ow >= 1;
-}
+bool depthwise_planes_supported(const ConvParams& p) { return supported(p); }
 
-cudaError_t launch_depthwise_planes(const ConvParams& q, const float* x, const float* w, const float* bias, float* out, float* means,
-                                    bool constants, cudaStream_t st) {
-  if (!depthwise_planes_supported(q) || (reinterpret_cast<uintptr_t>(x) & 15)) return cudaErrorInvalidValue;
+cudaError_t launch_depthwise_planes(const ConvParams& q, int images, const float* x, const float* w, const float* bias, float* out,
+                                    float* means, bool constants, cudaStream_t st) {
+  if (!supported(q) || (reinterpret_cast<uintptr_t>(x) & 15)) return cudaErrorInvalidValue;
+  const Shape sh = pick_shape(q, device_sm_count());
   PlanesDev d{};
   d.x = x; d.w = w; d.bias = bias; d.out = out; d.means = means;
-  d.planes = q.n * q.c; d.c = q.c; d.ih = q.ih; d.iw = q.iw; d.oh = q.oh; d.ow = q.ow; d.pad_t = q.pad_t; d.pad_l = q.pad_l;
+  d.planes = images * q.c; d.c = q.c; d.ih = q.ih; d.iw = q.iw; d.oh = q.oh; d.ow = q.ow; d.pad_t = q.pad_t; d.pad_l = q.pad_l;
+  d.per = sh.per; d.stride = sh.stride; d.rows = sh.rows; d.segs = sh.segs;
   d.act_alpha = q.act_alpha; d.act_beta = q.act_beta;
-  const int ihw = q.ih * q.iw, unit = (ihw & 3) ? 4 : 1, sms = device_sm_count();
-  // Neighbouring lanes walk neighbouring columns, then the next plane's: its banks follow on those of the row (in
-  // whole float4s where the copies are).
-  const int step = (ihw & 3) ? 1 : 4;
-  d.stride = ihw;
-  while ((((d.stride - q.iw) % 32) + 32) % 32 >= step) d.stride += step;
-  // About 14 rows a thread and 256 threads a block; fewer planes and shorter columns while the SMs hold more threads
-  // than that gives (32 images, 200 planes of 14 x 14: 8.7 us with 600 threads an SM, 6.1 with 1200).
-  d.segs = std::max(1, std::min((q.oh + 13) / 14, kMaxThreads / (unit * q.ow)));
-  const int fit = std::max(1, (int)(kMaxSmem / 2 / sizeof(float)) / (d.stride * unit));
-  int units = std::max(1, std::min(256 / (d.segs * q.ow * unit), fit));
-  while (units > 1 && (d.planes + units * unit - 1) / (units * unit) < 2 * sms) units /= 2;
-  d.per = units * unit;
-  while ((q.oh + d.segs - 1) / d.segs > 4 && (long long)d.planes * d.segs * q.ow < (long long)sms * 1024 &&
-         2 * d.per * d.segs * q.ow <= kMaxThreads)
-    d.segs *= 2;
-  d.rows = (q.oh + d.segs - 1) / d.segs;
-  d.segs = (q.oh + d.rows - 1) / d.rows;
-  const int threads = (d.per * d.segs * q.ow + 31) / 32 * 32;
-  const size_t smem = (size_t)d.per * d.stride * sizeof(float);
   const int overlap = constants ? 1 : 0;
-  return q.kh == 3 ? launch_act<3>(d, q.act, threads, smem, overlap, st) : launch_act<5>(d, q.act, threads, smem, overlap, st);
+  return q.kh == 3 ? launch_act<3>(d, q.act, sh.threads, sh.smem, overlap, st) : launch_act<5>(d, q.act, sh.threads, sh.smem, overlap, st);
 }
 
 }  // namespace ac

@@ -402,13 +402,13 @@ bool depthwise_conv_pools(const ConvParams& p) {
          (depthwise_planes_wins(p) || (long long)p.n * p.oc * per_plane <= 2048ll * device_sm_count());
 }
 
-cudaError_t launch_depthwise_conv(const ConvParams& p, const float* x, const float* w, const float* bias, float* out, float* means,
-                                  bool constants, cudaStream_t st) {
-  const long long total = (long long)p.n * p.oc * p.oh * p.ow;
+cudaError_t launch_depthwise_conv(const ConvParams& p, int images, const float* x, const float* w, const float* bias, float* out,
+                                  float* means, bool constants, cudaStream_t st) {
+  const long long total = (long long)images * p.oc * p.oh * p.ow;
   if (total == 0) return cudaSuccess;
   if (means && !depthwise_conv_pools(p)) return cudaErrorInvalidValue;
-  if (depthwise_planes_wins(p) && al16(x)) return launch_depthwise_planes(p, x, w, bias, out, means, constants, st);
-  const long long owg = (p.ow + 3) / 4, items = (long long)p.n * p.oc * p.oh * owg;
+  if (depthwise_planes_wins(p) && al16(x)) return launch_depthwise_planes(p, images, x, w, bias, out, means, constants, st);
+  const long long owg = (p.ow + 3) / 4, items = (long long)images * p.oc * p.oh * owg;
   if (depthwise_rows_ok(p)) {
     bool done = false;
     cudaError_t e = cudaSuccess;

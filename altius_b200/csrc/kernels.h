@@ -176,13 +176,14 @@ cudaError_t launch_im2col(const ConvParams& p, const float* x, float* col, cudaS
 // one row per patch with the (c, fy, fx) order of the weight's K axis. kw % 4 == 0.
 cudaError_t launch_patchify(const ConvParams& p, const float* x, float* rows, cudaStream_t st);
 // Depthwise (group == c == oc) stencil with bias and activation fused. `means`: [n][c] means of the resulting planes, written
-// too where depthwise_conv_pools says so, or null.
+// too where depthwise_conv_pools says so, or null. `images`: of the p.n that kernel and split are chosen for, from the given
+// pointers on (the order of a mean's sum follows from the split).
 bool depthwise_conv_pools(const ConvParams& p);
-cudaError_t launch_depthwise_conv(const ConvParams& p, const float* x, const float* w, const float* bias, float* out, float* means,
+cudaError_t launch_depthwise_conv(const ConvParams& p, int images, const float* x, const float* w, const float* bias, float* out, float* means,
                                   bool constants, cudaStream_t st);
 // The same over whole planes in shared memory (depthwise_planes.cu), stride 1; x 16-byte aligned.
 bool depthwise_planes_supported(const ConvParams& p);
-cudaError_t launch_depthwise_planes(const ConvParams& p, const float* x, const float* w, const float* bias, float* out, float* means,
+cudaError_t launch_depthwise_planes(const ConvParams& p, int images, const float* x, const float* w, const float* bias, float* out, float* means,
                                     bool constants, cudaStream_t st);
 
 // Small convolutions (group 1) on the CUDA cores without a column buffer (conv_simt.cu). `wt` is the

@@ -1235,9 +1235,7 @@ void lower_conv(Emit& em, Plan& plan, int nid, const Epilogue* e, const Plan::Se
     if (auto m = plan.means.find(out); m != plan.means.end() && depthwise_conv_pools(p))
       m->second = means = new_value(em.c, (int64_t)p.n * p.c, false);
     auto part = [=](cudaStream_t st, int first, int count) {
-      ConvParams q = p;
-      q.n = count;
-      return launch_depthwise_conv(q, s->fptr(x) + (size_t)first * p.c * p.ih * p.iw, s->fptr(w), bias >= 0 ? s->fptr(bias) : nullptr,
+      return launch_depthwise_conv(p, count, s->fptr(x) + (size_t)first * p.c * p.ih * p.iw, s->fptr(w), bias >= 0 ? s->fptr(bias) : nullptr,
                                    s->fptr_mut(out) + (size_t)first * p.oc * ohw, means >= 0 ? s->fptr_mut(means) + (size_t)first * p.oc : nullptr,
                                    constants, st);
     };

@@ -6,7 +6,7 @@ import subprocess
 import numpy as np
 import pytest
 
-from altius_b200 import configs
+from altius_b200 import configs, ir
 from altius_b200.session import CudaSessionBuilder
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -66,5 +66,39 @@ def test_runs_in_pieces(cuda_lib, batch, px):
             outs = [[np.empty_like(want)], [np.empty_like(want)]]
             sess.run_batches([[x], [x]], outs)
             assert np.array_equal(outs[0][0], want) and np.array_equal(outs[1][0], want)
+    finally:
+        sess.close()
+
+
+# A front whose last layers leave means of narrow planes: their sums follow the split over the whole batch, not a piece's.
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,c,px,k", [(32, 200, 14, 3), (26, 200, 15, 5)])
+def test_pieces_give_the_bits_of_the_whole(cuda_lib, batch, c, px, k):
+    import torch
+    rng = np.random.default_rng(c)
+    f = lambda *sh: (rng.standard_normal(sh) / np.sqrt(np.prod(sh[1:]))).astype(np.float32)
+    g = ir.Graph()
+
+    def conv(x, w, group=1):
+        return g.op("Conv2d", x, g.new_init(w), kernel_shape=list(w.shape[2:]), strides=[1, 1], padding=[w.shape[2] // 2] * 4,
+                    dilations=[1, 1], group=group, auto_pad="")
+    y = conv(g.add_input("x", (batch, 2 * c, px, px)), f(c, 2 * c, 1, 1))
+    y = g.op("ReLU", conv(y, f(c, 1, 3, 3), c))
+    y = g.op("ReLU", conv(conv(y, f(c, c, 1, 1)), f(c, 1, k, k), c))
+    z = conv(g.op("ReLU", conv(g.op("GlobalAveragePool", y), f(48, c, 1, 1))), f(c, 48, 1, 1))
+    gate = g.op("HardSigmoid", z, alpha=0.2, beta=0.5)
+    g.outputs += [gate, conv(g.op("Mul", y, gate), f(c, c, 1, 1))]
+    sess = CudaSessionBuilder(ir.Model(g, 13)).build()
+    try:
+        kinds = [e["kind"] for e in sess.schedule()]
+        assert kinds == ["gemm_tf32x3_tcgen05", "conv_depthwise", "gemm_tf32x3_tcgen05", "conv_depthwise", "squeeze_excite",
+                         "gemm_tf32x3_tcgen05"]
+        x = rng.standard_normal((batch, 2 * c, px, px)).astype(np.float32)
+        outs = [torch.empty(s, device="cuda") for s, _ in sess.output_info]
+        xd = torch.from_numpy(x).cuda()
+        torch.cuda.synchronize()
+        sess.run_device([xd.data_ptr()], [o.data_ptr() for o in outs])
+        for got, want in zip(sess.run([x]), outs):
+            assert np.array_equal(got, want.cpu().numpy())
     finally:
         sess.close()
