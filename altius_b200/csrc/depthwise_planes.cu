@@ -136,8 +136,6 @@ cudaError_t launch_act(const PlanesDev& d, int act, int threads, size_t smem, in
 
 }  // namespace
 
-bool depthwise_planes_supported(const ConvParams& p) { return supported(p); }
-
 cudaError_t launch_depthwise_planes(const ConvParams& q, int images, const float* x, const float* w, const float* bias, float* out,
                                     float* means, bool constants, cudaStream_t st) {
   if (!supported(q) || (reinterpret_cast<uintptr_t>(x) & 15)) return cudaErrorInvalidValue;

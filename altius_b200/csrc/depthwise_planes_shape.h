@@ -1,4 +1,4 @@
-// Split of the depthwise kernel that works on whole planes (depthwise_planes.cu): host arithmetic only.
+// Split of the depthwise kernel that works on whole planes (depthwise_planes.cu), and where it is taken: host arithmetic only.
 #pragma once
 #include <stddef.h>
 
@@ -53,6 +53,31 @@ inline Shape pick_shape(const ConvParams& q, int sms) {
   s.threads = (s.per * s.segs * q.ow + 31) / 32 * 32;
   s.smem = (size_t)s.per * s.stride * sizeof(float);
   return s;
+}
+
+// Microseconds of a launch behind another one: this kernel's (a column's chain of rows, or the instructions of all threads, whichever is
+// more, and most of the other), and those of the kernel that reads global memory (depthwise_rows_kernel, four pixels a thread).
+// Fitted over 630 layers of 1 to 64 images, 16 to 960 planes, rows of 3 to 126 that are no whole float4s.
+inline double planes_us(const ConvParams& q, int sms) {
+  const Shape s = pick_shape(q, sms);
+  const bool wide = q.kh == 5;
+  const double steps = s.rows + q.kh - 1, blocks = (double)(((long long)q.n * q.c + s.per - 1) / s.per);
+  const double chain = steps * (wide ? 0.16 : 0.115), issue = blocks * s.threads * steps * (wide ? 0.46 : 0.36) / (1000.0 * sms);
+  return 2.5 + std::max(chain, issue) + 0.6 * std::min(chain, issue);
+}
+inline double rows_us(const ConvParams& q, int sms) {
+  const double quads = (double)q.n * q.c * q.oh * ((q.ow + 3) / 4);
+  return std::max(2.8, 2.6 + quads * (q.kh == 5 ? 27.7e-6 : 12.9e-6) * 148 / sms);
+}
+
+// Whether this kernel is the faster one. Only for rows that are no whole float4s: of those the other takes a value a load, but with them,
+// and at stride two, it is the faster one (32 images, 240 planes of 28 x 28, 3 x 3, stride two: 7.3 us against 9.3). Few or large
+// planes leave a thread a long column and most SMs idle (us, rows -> planes: one image, 16 planes of 75 x 75, 3 x 3 3.1 -> 16.5, 72 of
+// 61 x 61, 5 x 5 4.3 -> 11.3; 32 images, 72 of 61 x 61, 5 x 5 63.9 -> 34.5, 960 of 7 x 7 14.1 -> 9.3, 480 of 14 x 14, 3 x 3 13.7 -> 10.0,
+// 16 of 75 x 75 12.2 -> 19.2). Over the 630 the choice takes 5 % less than the other kernel alone, 0.7 % more than the better one each
+// time would. `gain`: us that the means of the planes are worth where only this kernel leaves them.
+inline bool wins(const ConvParams& q, int sms, double gain = 0.0) {
+  return (q.iw & 3) != 0 && supported(q) && planes_us(q, sms) < 0.95 * rows_us(q, sms) + gain;
 }
 
 }  // namespace depthwise_planes

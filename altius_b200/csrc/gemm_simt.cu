@@ -12,6 +12,7 @@
 // 8x8 register block (two 4-wide halves 64 apart so shared-memory reads are
 // conflict-free float4), operands staged through double-buffered shared memory
 // with the next K step prefetched into registers during the math.
+#include "depthwise_planes_shape.h"
 #include "kernels.h"
 #include "pdl.cuh"
 #include "plane_means.cuh"
@@ -388,18 +389,22 @@ static bool depthwise_rows_ok(const ConvParams& p) {
          (p.act == ACT_NONE || p.act == ACT_RELU || p.act == ACT_HARDSWISH);
 }
 
-// Planes in shared memory (depthwise_planes.cu) for rows that are no whole float4s: a load per value here (32 images, 960
-// planes of 7 x 7, 5 x 5: 14.1 us against 9.2, 672 of 14 x 14, 3 x 3: 18.2 against 12.5; one image within 3 %). With whole
-// float4s, and at stride two, the rows kernel is the faster one (32 images, 240 of 28 x 28, 3 x 3, stride two: 7.3 against 9.3).
-static bool depthwise_planes_wins(const ConvParams& p) { return (p.iw & 3) && depthwise_planes_supported(p); }
-
 // The rows kernel's blocks add their planes up behind a barrier, which costs more than the squeeze-and-excite block saves once the
 // blocks take several rounds (120 planes of 28 x 28, 5 x 5, then the squeeze: 32 images 16.1 + 9.0 us -> 22.0 + 6.1; 13 of
 // 24 x 24: 6.2 + 8.2 -> 7.8 + 5.2).
+static bool depthwise_rows_pool(const ConvParams& p) {
+  return (long long)p.n * p.oc * p.oh * ((p.ow + 3) / 4) <= 2048ll * device_sm_count();
+}
+
+// Planes in shared memory (depthwise_planes.cu). Where only they leave means, these save the squeeze-and-excite block its pool: 3 us of
+// 8 to 11.
+static bool depthwise_planes_wins(const ConvParams& p, bool means) {
+  return depthwise_planes::wins(p, device_sm_count(), means && !depthwise_rows_pool(p) ? 3.0 : 0.0);
+}
+
 bool depthwise_conv_pools(const ConvParams& p) {
   const long long per_plane = (long long)p.oh * ((p.ow + 3) / 4);
-  return depthwise_rows_ok(p) && per_plane >= 1 && per_plane <= 256 &&
-         (depthwise_planes_wins(p) || (long long)p.n * p.oc * per_plane <= 2048ll * device_sm_count());
+  return depthwise_rows_ok(p) && per_plane >= 1 && per_plane <= 256 && (depthwise_rows_pool(p) || depthwise_planes_wins(p, true));
 }
 
 cudaError_t launch_depthwise_conv(const ConvParams& p, int images, const float* x, const float* w, const float* bias, float* out,
@@ -407,7 +412,7 @@ cudaError_t launch_depthwise_conv(const ConvParams& p, int images, const float* 
   const long long total = (long long)images * p.oc * p.oh * p.ow;
   if (total == 0) return cudaSuccess;
   if (means && !depthwise_conv_pools(p)) return cudaErrorInvalidValue;
-  if (depthwise_planes_wins(p) && al16(x)) return launch_depthwise_planes(p, images, x, w, bias, out, means, constants, st);
+  if (depthwise_planes_wins(p, means != nullptr) && al16(x)) return launch_depthwise_planes(p, images, x, w, bias, out, means, constants, st);
   const long long owg = (p.ow + 3) / 4, items = (long long)images * p.oc * p.oh * owg;
   if (depthwise_rows_ok(p)) {
     bool done = false;

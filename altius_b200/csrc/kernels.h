@@ -182,7 +182,6 @@ bool depthwise_conv_pools(const ConvParams& p);
 cudaError_t launch_depthwise_conv(const ConvParams& p, int images, const float* x, const float* w, const float* bias, float* out, float* means,
                                   bool constants, cudaStream_t st);
 // The same over whole planes in shared memory (depthwise_planes.cu), stride 1; x 16-byte aligned.
-bool depthwise_planes_supported(const ConvParams& p);
 cudaError_t launch_depthwise_planes(const ConvParams& p, int images, const float* x, const float* w, const float* bias, float* out, float* means,
                                     bool constants, cudaStream_t st);
 
