@@ -18,13 +18,15 @@
 // cluster of up to eight blocks shares the tile over ranges of K. Partial sums meet in (distributed)
 // shared memory in a fixed order, so results do not depend on timing; the blocks of a cluster send
 // theirs with stores that count on the receiver's mbarrier. The filter's part of the first stages is
-// requested, and the code run once without effect, before the kernel in front has finished.
+// requested before the kernel in front has finished.
 //
 // Measured, per launch in a MobileNetV3-Large at batch one, from the end of the kernel in front: 40 -> 120 at 28 x 28 4.8 us
 // -> 3.1; 672 -> 112 at 14 x 14 with a gate 10.7 -> 6.1; 960 -> 160 at 7 x 7 with a gate 12.7 -> 5.2. Before that: four groups of 128
 // threads on 2 x 4 results each with a barrier of the block in every K step (1100 clocks a step against 800: shared memory
 // hands a warp 128 bytes a clock, so the bytes loaded per product count), planes by 4-byte cp.async, the gate fetched one step
-// ahead, remote partial sums read block by block, the residual behind them.
+// ahead, remote partial sums read block by block, the residual behind them. (A pass over zeros ahead of the wait, to have the code in
+// the instruction cache, gave a MobileNetV3-Large nothing, 312.8 us with it and 312.0 without, and cost 0.5 us of a launch behind
+// another of these and 2 us behind a kernel that lets nothing start early.)
 #include <cooperative_groups.h>
 
 #include "cluster_send.cuh"
@@ -53,7 +55,6 @@ struct ConvDev {
   float act_alpha, act_beta;
   int kper;                 // K steps per block of the cluster
   int early;                // the filter and the bias are constants: read ahead of pdl_wait
-  int cold;                 // nothing runs in front: no pass ahead of the first
   int* err;
 };
 
@@ -118,14 +119,13 @@ struct Quad {
       each(p, [&](int j, long long a) { res[j] = p.res[a]; });
     }
   }
-  __device__ __forceinline__ void store(const ConvDev& p, float4 v, bool now) const {
+  __device__ __forceinline__ void store(const ConvDev& p, float4 v) const {
     float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       e[j] = finish(p, e[j], bias);
       if (p.res) e[j] = __fadd_rn(e[j], res[j]);
     }
-    if (!now) return;
     if (LOAD == LOAD_VEC) {
       if (live) *reinterpret_cast<float4*>(p.out + at) = make_float4(e[0], e[1], e[2], e[3]);
     } else {
@@ -264,87 +264,76 @@ __global__ void __launch_bounds__(T, 2) conv_simt_kernel(const ConvDev p) {
     quad.place(p, tid < share, m0 + (e >> 3 & 3) * 4 + (e >> 6), n0 + (e >> 5 & 1) * 32 + (e & 7) * 4);
   }
 
-  // The first pass reads and writes nothing outside the block: it brings the code into the instruction cache while
-  // the kernel in front still runs. One K step, of zeros.
-#pragma unroll 1
-  for (int pass = p.cold; pass < 2; ++pass) {
-    const bool now = pass == 1;
-    if (now) pdl_wait();
-    {
-      Piece u[S - 1];
+  pdl_wait();
+  {
+    Piece u[S - 1];
 #pragma unroll
-      for (int s = 0; s < S - 1; ++s)
-        if (LOAD != LOAD_WINDOW || !now || s < kts) fetch(u[s], kt0 + s, now && s < kts);
-      if (now) quad.fetch(p);
+    for (int s = 0; s < S - 1; ++s)
+      if (LOAD != LOAD_WINDOW || s < kts) fetch(u[s], kt0 + s, s < kts);
+    quad.fetch(p);
 #pragma unroll
-      for (int s = 0; s < S - 1; ++s)
-        if (LOAD != LOAD_WINDOW || !now || s < kts) put(s, u[s]);
-    }
-
-    float2 acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
-
-    const int steps = now ? kts : 1;
-    for (int it = 0; it < steps; ++it) {
-      const int s = it % S;
-      if (it == 0) cp_wait<0>();           // the filter's part of the first stages
-      else cp_wait<S - 2>();
-      __syncwarp();                        // stage s complete for the warp; stage of step it - 1 is free
-      Piece u;
-      const bool more = now && it + S - 1 < kts;
-      if (more) load_w((it + S - 1) % S, kt0 + it + S - 1);
-      cp_commit();
-      fetch(u, kt0 + it + S - 1, more);
-      const float* As = mine + s * SLICE;
-      const float* Bs = As + KW * BM;
-#pragma unroll
-      for (int kk = 0; kk < KW; ++kk) {
-        const float4 a4 = *reinterpret_cast<const float4*>(As + kk * BM + ty * 4);
-        const float4 b0 = *reinterpret_cast<const float4*>(Bs + kk * BN + tx * 4);
-        const float4 b1 = *reinterpret_cast<const float4*>(Bs + kk * BN + 32 + tx * 4);
-        const float a[4] = {a4.x, a4.y, a4.z, a4.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 aa = make_float2(a[i], a[i]);
-          acc[i][0] = fma2(aa, make_float2(b0.x, b0.y), acc[i][0]);
-          acc[i][1] = fma2(aa, make_float2(b0.z, b0.w), acc[i][1]);
-          acc[i][2] = fma2(aa, make_float2(b1.x, b1.y), acc[i][2]);
-          acc[i][3] = fma2(aa, make_float2(b1.z, b1.w), acc[i][3]);
-        }
-      }
-      if (more) put((it + S - 1) % S, u);
-    }
-
-    // The warps' sums, then the blocks': both in order. A block sends each other one its share.
-    __syncthreads();
-    if (now) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          part[warp * QUADS + (2 * i + h) * 32 + lane] = make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
-    }
-    __syncthreads();
-    float4 sum = part[tid];
-#pragma unroll
-    for (int w = 1; w < WARPS; ++w) add4(sum, part[w * QUADS + tid]);
-    if (parts > 1) {
-      if (now) {
-        cl.barrier_wait();                 // every block of the cluster runs and has announced what it waits for
-        const int owner = tid / share;
-        send4(cluster_addr(recv + rank * share + tid - owner * share, owner), cluster_addr(&sent, owner), sum);
-        if (tid < share && !wait_sent(&sent, 0)) atomicExch(p.err, 71);
-      }
-      if (tid < share) {
-        sum = recv[tid];
-        for (int r = 1; r < parts; ++r) add4(sum, recv[r * share + tid]);
-      }
-    }
-    quad.store(p, sum, now);
+    for (int s = 0; s < S - 1; ++s)
+      if (LOAD != LOAD_WINDOW || s < kts) put(s, u[s]);
   }
+
+  float2 acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
+
+  for (int it = 0; it < kts; ++it) {
+    const int s = it % S;
+    if (it == 0) cp_wait<0>();             // the filter's part of the first stages
+    else cp_wait<S - 2>();
+    __syncwarp();                          // stage s complete for the warp; stage of step it - 1 is free
+    Piece u;
+    const bool more = it + S - 1 < kts;
+    if (more) load_w((it + S - 1) % S, kt0 + it + S - 1);
+    cp_commit();
+    fetch(u, kt0 + it + S - 1, more);
+    const float* As = mine + s * SLICE;
+    const float* Bs = As + KW * BM;
+#pragma unroll
+    for (int kk = 0; kk < KW; ++kk) {
+      const float4 a4 = *reinterpret_cast<const float4*>(As + kk * BM + ty * 4);
+      const float4 b0 = *reinterpret_cast<const float4*>(Bs + kk * BN + tx * 4);
+      const float4 b1 = *reinterpret_cast<const float4*>(Bs + kk * BN + 32 + tx * 4);
+      const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 aa = make_float2(a[i], a[i]);
+        acc[i][0] = fma2(aa, make_float2(b0.x, b0.y), acc[i][0]);
+        acc[i][1] = fma2(aa, make_float2(b0.z, b0.w), acc[i][1]);
+        acc[i][2] = fma2(aa, make_float2(b1.x, b1.y), acc[i][2]);
+        acc[i][3] = fma2(aa, make_float2(b1.z, b1.w), acc[i][3]);
+      }
+    }
+    if (more) put((it + S - 1) % S, u);
+  }
+
+  // The warps' sums, then the blocks': both in order. A block sends each other one its share.
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      part[warp * QUADS + (2 * i + h) * 32 + lane] = make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
+  __syncthreads();
+  float4 sum = part[tid];
+#pragma unroll
+  for (int w = 1; w < WARPS; ++w) add4(sum, part[w * QUADS + tid]);
+  if (parts > 1) {
+    cl.barrier_wait();                     // every block of the cluster runs and has announced what it waits for
+    const int owner = tid / share;
+    send4(cluster_addr(recv + rank * share + tid - owner * share, owner), cluster_addr(&sent, owner), sum);
+    if (tid < share) {
+      if (!wait_sent(&sent, 0)) atomicExch(p.err, 71);
+      sum = recv[tid];
+      for (int r = 1; r < parts; ++r) add4(sum, recv[r * share + tid]);
+    }
+  }
+  quad.store(p, sum);
 }
 
 template <int LOAD>
@@ -381,7 +370,7 @@ bool conv_simt_supported(const ConvParams& q) {
 }
 
 cudaError_t launch_conv_simt(const ConvParams& q, const float* x, const float* wt, const float* bias, const float* gate,
-                             const float* residual, float* out, bool constants, bool first, int* err_word, cudaStream_t st) {
+                             const float* residual, float* out, bool constants, int* err_word, cudaStream_t st) {
   ConvDev p{};
   p.x = x; p.wt = wt; p.out = out; p.bias = bias; p.res = residual; p.gate = gate;
   p.ldw = (int)conv_simt_ldw(q.oc); p.m = q.oc; p.k = q.c * q.kh * q.kw; p.hw = q.oh * q.ow; p.n = q.n * p.hw;
@@ -390,7 +379,6 @@ cudaError_t launch_conv_simt(const ConvParams& q, const float* x, const float* w
   p.ih = q.ih; p.iw = q.iw; p.ow = q.ow; p.kh = q.kh; p.kw = q.kw; p.sh = q.sh; p.sw = q.sw; p.dh = q.dh; p.dw = q.dw;
   p.pt = q.pad_t; p.pl = q.pad_l;
   p.early = constants;
-  p.cold = first;
   p.err = err_word;
   p.act = q.act; p.act_alpha = q.act_alpha; p.act_beta = q.act_beta;
   const bool window = q.kh != 1 || q.kw != 1 || q.sh != 1 || q.sw != 1 || q.pad_t || q.pad_l || q.oh != q.ih || q.ow != q.iw;

@@ -187,12 +187,12 @@ cudaError_t launch_depthwise_planes(const ConvParams& p, int images, const float
 
 // Small convolutions (group 1) on the CUDA cores without a column buffer (conv_simt.cu). `wt` is the
 // filter matrix transposed by launch_pack_filter: [k][conv_simt_ldw(oc)]. `gate`: [n][c] factors of
-// the input channels (pointwise convolutions only), or null; `residual`: added last, or null; `first`: no kernel runs in front.
+// the input channels (pointwise convolutions only), or null; `residual`: added last, or null.
 inline int64_t conv_simt_ldw(int64_t oc) { return (oc + 3) / 4 * 4; }
 bool conv_simt_supported(const ConvParams& p);
 cudaError_t launch_pack_filter(const float* w, float* wt, int64_t oc, int64_t k, cudaStream_t st);
 cudaError_t launch_conv_simt(const ConvParams& p, const float* x, const float* wt, const float* bias, const float* gate,
-                             const float* residual, float* out, bool constants, bool first, int* err_word, cudaStream_t st);
+                             const float* residual, float* out, bool constants, int* err_word, cudaStream_t st);
 // Larger convolutions (group 1, no Gelu behind) on the tensor cores, 3xTF32, planes read in place
 // (conv_tc.cu). The filter is split and blocked once by launch_pack_filter_tc into
 // conv_tc_filter_elems floats; the other operands as above.

@@ -1274,10 +1274,9 @@ void lower_conv(Emit& em, Plan& plan, int nid, const Epilogue* e, const Plan::Se
            [=](cudaStream_t st) { return launch_pack_filter(s->fptr(w), s->fptr_mut(wt), oc, kd, st); });
     const int res = ep.residual, gv = gate ? gate->gate : -1;
     const double bytes = f32_bytes(xv) + f32_bytes(wv) + f32_bytes(ov) * (res >= 0 ? 2 : 1);
-    const bool first = std::find(s->inputs.begin(), s->inputs.end(), x) != s->inputs.end();
     em.add("conv_fp32_simt", n.op, {x, wt, bias, gv, res}, {out}, bytes, flops, [=](cudaStream_t st) {
       return launch_conv_simt(p, s->fptr(x), s->fptr(wt), bias >= 0 ? s->fptr(bias) : nullptr,
-                              gv >= 0 ? s->fptr(gv) : nullptr, res >= 0 ? s->fptr(res) : nullptr, s->fptr_mut(out), constants, first, s->err_word, st);
+                              gv >= 0 ? s->fptr(gv) : nullptr, res >= 0 ? s->fptr(res) : nullptr, s->fptr_mut(out), constants, s->err_word, st);
     });
     return;
   }
