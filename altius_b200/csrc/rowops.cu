@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, FUSED ? (RESX == 1 ? 4 : 3) : (PF ? 
 
 // Any length / alignment: one warp per row, values recomputed from global
 // memory in each pass (served by L1/L2 after the first).
-__global__ void __launch_bounds__(kThreads) layer_norm_generic(LnDev p) {
+__global__ void __launch_bounds__(kThreads, 5) layer_norm_generic(LnDev p) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
