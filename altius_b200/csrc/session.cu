@@ -102,8 +102,6 @@ void parse_graph(AcSession& s, const AcGraphDesc& g) {
   if (s.outputs.empty()) fail(AC_ERR_INVALID, "graph without outputs");
 }
 
-// Lifetimes by step index, then first-fit placement of the largest buffers
-// first: two storages may share bytes only if their live ranges are disjoint.
 // The steps at the front that follow one another on the batch of the one input, image by image.
 void plan_front(AcSession& s) {
   s.pieces = PiecePlan{};
@@ -115,9 +113,33 @@ void plan_front(AcSession& s) {
   s.pieces = plan_pieces(front, (int)std::min<int64_t>(in.dims[0], 1 << 30), in.bytes());
 }
 
+// Where a piece's steps put the values that none but they read: a piece runs behind the one before it, so such a value needs
+// the room of one piece, in what the arena has free beside the input and the values that the rest reads, which
+// collect the whole batch. The arena does not grow for it; if it would have to, there are no pieces.
+void plan_piece_slots(AcSession& s) {
+  s.piece_slots.clear();
+  if (!s.pieces.steps) return;
+  const int last_front = s.pieces.steps - 1;
+  std::vector<Slot> fixed, own;
+  for (int i = 0; i < (int)s.storages.size(); ++i) {
+    const Storage& st = s.storages[i];
+    if (st.weight || st.last < 0 || st.first > last_front) continue;
+    if (st.first < 0 || st.last > last_front) {
+      fixed.push_back({st.bytes, 0, last_front, st.offset});
+    } else {
+      if (st.bytes % (size_t)s.pieces.images) { s.pieces = PiecePlan{}; s.piece_slots.clear(); return; }
+      own.push_back({st.bytes / (size_t)s.pieces.images * (size_t)s.pieces.per, st.first, st.last, 0});
+      s.piece_slots.push_back({i, 0});
+    }
+  }
+  const size_t top = place_slots(own, fixed);
+  for (size_t i = 0; i < own.size(); ++i) s.piece_slots[i].second = own[i].offset;
+  if (top > s.arena_bytes) { s.pieces = PiecePlan{}; s.piece_slots.clear(); }
+}
+
+// Lifetimes by step index, then the placement.
 void plan_arena(AcSession& s) {
   const int nsteps = (int)s.steps.size();
-  plan_front(s);
   for (Storage& st : s.storages) { st.first = 1 << 30; st.last = -1; }
   auto touch = [&](int sid, int step) {
     Storage& st = s.storages[sid];
@@ -134,6 +156,7 @@ void plan_arena(AcSession& s) {
   }
   size_t woff = 0;
   std::vector<int> live;
+  std::vector<Slot> slots;
   for (int i = 0; i < (int)s.storages.size(); ++i) {
     Storage& st = s.storages[i];
     if (st.weight) {
@@ -143,36 +166,14 @@ void plan_arena(AcSession& s) {
     }
     if (st.pinned_live) { st.first = -1; st.last = nsteps; }
     if (st.last < 0) continue;  // never touched
-    // A piece's steps run in front of the next piece's: no two values of theirs may share memory.
-    if (st.first < s.pieces.steps) { st.first = std::min(st.first, 0); st.last = std::max(st.last, s.pieces.steps - 1); }
     live.push_back(i);
+    slots.push_back({st.bytes, st.first, st.last, 0});
   }
   s.weight_bytes = woff;
-  std::sort(live.begin(), live.end(), [&](int a, int b) {
-    if (s.storages[a].bytes != s.storages[b].bytes) return s.storages[a].bytes > s.storages[b].bytes;
-    return a < b;
-  });
-  std::vector<int> placed;
-  size_t top = 0;
-  for (int id : live) {
-    Storage& st = s.storages[id];
-    const size_t need = align_up(st.bytes, 256);
-    std::vector<std::pair<size_t, size_t>> busy;
-    for (int o : placed) {
-      const Storage& q = s.storages[o];
-      if (q.first <= st.last && st.first <= q.last) busy.push_back({q.offset, q.offset + align_up(q.bytes, 256)});
-    }
-    std::sort(busy.begin(), busy.end());
-    size_t off = 0;
-    for (auto& b : busy) {
-      if (off + need <= b.first) break;
-      off = std::max(off, b.second);
-    }
-    st.offset = off;
-    top = std::max(top, off + need);
-    placed.push_back(id);
-  }
-  s.arena_bytes = std::max<size_t>(top, 256);
+  s.arena_bytes = std::max<size_t>(place_slots(slots), 256);
+  for (size_t i = 0; i < live.size(); ++i) s.storages[live[i]].offset = slots[i].offset;
+  plan_front(s);
+  plan_piece_slots(s);
 }
 
 void upload_weights(AcSession& s, const AcGraphDesc& g) {
@@ -273,7 +274,13 @@ void capture_pieces(AcSession& s) {
         for (int i = 0; i < p.steps && l == cudaSuccess; ++i) l = s.steps[i].part(s.stream, p.begin(k), p.end(k) - p.begin(k));
         return l;
       };
+      // The steps count from the batch's first image: that far in front of its slot a value of the piece's own begins.
+      for (auto& [id, offset] : s.piece_slots) {
+        const size_t image = s.storages[id].bytes / (size_t)p.images;
+        s.storages[id].bound = reinterpret_cast<void*>(reinterpret_cast<uintptr_t>(s.arena) + offset - (size_t)p.begin(k) * image);
+      }
       if (e == cudaSuccess) e = capture(&s, launches, &g.graph, &g.exec);
+      for (auto& slot : s.piece_slots) s.storages[slot.first].bound = nullptr;
     }
     s.piece_graphs.push_back(g);
   }

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/altius_session_cuda.h"
+#include "arena.h"
 #include "host_stage.h"
 #include "kernels.h"
 #include "pieces.h"
@@ -54,7 +55,7 @@ struct Storage {
   bool weight = false;   // lives in the weight blob, not the arena
   bool pinned_live = false;  // graph input/output or constant: live for the whole run
   size_t offset = 0;     // byte offset inside its region
-  void* bound = nullptr; // set while steps are enqueued on a caller's device buffer in place of the arena slot
+  void* bound = nullptr; // set while steps are enqueued on another buffer in place of the arena slot (a caller's, a piece's)
 };
 
 struct Step {
@@ -124,6 +125,7 @@ struct AcSession {
   std::vector<ac::Segment> segments;   // empty: this schedule does not run on bound buffers
   // Runs from large host inputs: the front of the schedule per piece of the batch, the rest behind it.
   ac::PiecePlan pieces;
+  std::vector<std::pair<int, size_t>> piece_slots;   // storages that only the front touches, and their place while a piece runs
   std::vector<ac::Segment> piece_graphs;   // one a piece and one for the rest; empty: not used
   std::vector<cudaEvent_t> piece_up;       // a piece's images are on the device
   cudaStream_t up_stream = nullptr;

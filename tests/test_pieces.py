@@ -36,13 +36,72 @@ def test_plan(tmp_path):
     assert subprocess.run([str(tmp_path / "p")], capture_output=True, text=True).stdout == "ok\n"
 
 
-def test_a_large_batch_keeps_its_front_values_apart():
-    """11 convolutions up to the first squeeze-and-excite block: no two of their values may share memory."""
-    small, large = (CudaSessionBuilder(configs.mobilenet_v3_large(batch=b, img=224)[0]).with_plan_only(True).build() for b in (4, 32))
-    front = [e["kind"] for e in large.schedule()].index("squeeze_excite")
-    assert front == 11
-    per_image = 4 * (3 * 224 ** 2 + 3 * 16 * 112 ** 2 + 64 * 112 ** 2 + 64 * 56 ** 2 + 2 * 24 * 56 ** 2 + 3 * 72 * 56 ** 2 + 72 * 28 ** 2)
-    assert large.arena_bytes >= 32 * per_image > 8 * small.arena_bytes
+ARENA = r"""
+#include <cstdio>
+#include <random>
+#include "arena.h"
+using ac::Slot;
+int main() {
+  std::mt19937 rng(1);
+  auto at = [&](int lo, int hi) { return lo + (int)(rng() % (unsigned)(hi - lo + 1)); };
+  for (int round = 0; round < 2000; ++round) {
+    std::vector<Slot> fixed, slots;
+    const int steps = at(1, 30), n = at(1, 40);
+    size_t sum = 0;
+    for (int i = 0; i < n; ++i) {
+      const int a = at(0, steps - 1), b = at(a, steps - 1);
+      slots.push_back({(size_t)at(0, 5000), a, b, 0});
+      sum += (slots.back().bytes + 255) / 256 * 256;
+    }
+    for (int i = at(0, 5), o = at(0, 4) * 256; i > 0; --i, o += at(0, 9) * 256) {
+      fixed.push_back({(size_t)at(1, 3000), 0, steps - 1, (size_t)o});
+      o = (int)fixed.back().end();
+    }
+    const std::vector<Slot> before = slots;
+    const size_t top = ac::place_slots(slots, fixed), gap = fixed.empty() ? 0 : fixed.back().end();
+    size_t end = 0;
+    for (size_t i = 0; i < slots.size(); ++i) {
+      const Slot& s = slots[i];
+      end = std::max(end, s.end());
+      if (s.bytes != before[i].bytes || s.first != before[i].first || s.last != before[i].last || s.offset % 256) return 1;
+      for (size_t j = 0; j < i; ++j)
+        if (s.bytes && slots[j].bytes && s.meets(slots[j]) && s.offset < slots[j].end() && slots[j].offset < s.end()) return 2;
+      for (const Slot& f : fixed)
+        if (s.bytes && s.offset < f.end() && f.offset < s.end()) return 3;
+    }
+    if (end != top || top > sum + gap) return 4;
+  }
+  std::puts("ok");
+}
+"""
+
+
+def test_slots_with_common_steps_do_not_overlap(tmp_path):
+    src = tmp_path / "a.cpp"
+    src.write_text(ARENA)
+    subprocess.run(["g++", "-std=c++17", "-I", os.path.join(ROOT, "altius_b200", "csrc"), "-o", str(tmp_path / "a"), str(src)], check=True)
+    r = subprocess.run([str(tmp_path / "a")], capture_output=True, text=True)
+    assert r.stdout == "ok\n", r.returncode
+
+
+def _convolutions(batch, layers=24, c=64, px=56):
+    """A net that is all front: with every value in a place of its own it would take `layers` times its input."""
+    g = ir.Graph()
+    x = g.add_input("x", (batch, c, px, px))
+    w = g.new_init(np.full((c, c, 1, 1), 1 / c, np.float32))
+    for _ in range(layers):
+        x = g.op("ReLU", g.op("Conv2d", x, w, kernel_shape=[1, 1], strides=[1, 1], padding=[0] * 4, dilations=[1, 1], group=1, auto_pad=""))
+    g.outputs.append(x)
+    return ir.Model(g, 13)
+
+
+@pytest.mark.parametrize("model,batch,most", [
+    (lambda b: configs.mobilenet_v3_large(batch=b, img=224)[0], 14, 73.5 * 2 ** 20), (lambda b: configs.mobilenet_v3_large(batch=b, img=224)[0], 32, 152.5 * 2 ** 20),
+    (_convolutions, 32, 4.1 * 32 * 4 * 64 * 56 ** 2)])
+def test_pieces_need_no_memory_of_their_own(model, batch, most):
+    m = model(batch)
+    pieces, whole = (CudaSessionBuilder(m).with_plan_only(True).with_cuda_graph(on).build() for on in (True, False))
+    assert pieces.arena_bytes == whole.arena_bytes <= most
 
 
 # three pieces of which the last has one image, pieces of an odd plane, four even ones
