@@ -397,9 +397,14 @@ static bool depthwise_rows_pool(const ConvParams& p) {
 }
 
 // Planes in shared memory (depthwise_planes.cu). Where only they leave means, these save the squeeze-and-excite block its pool: 3 us of
-// 8 to 11.
+// 8 to 11. Where both do, those of a few small planes cost the rows kernel more (us of the layer with its block, rows -> planes:
+// 960 planes of 7 x 7, 5 x 5 20.9 -> 20.5, three images 26.3 -> 25.6, 672 of 9 x 9 20.0 -> 19.1; but eleven images of 960 of 7 x 7
+// 35.8 -> 37.5, eight of 672 of 9 x 9 28.3 -> 29.2, one of 120 of 25 x 25 12.0 -> 13.6; with 3 x 3 a few tenths the other way).
 static bool depthwise_planes_wins(const ConvParams& p, bool means) {
-  return depthwise_planes::wins(p, device_sm_count(), means && !depthwise_rows_pool(p) ? 3.0 : 0.0);
+  double gain = 0.0;
+  if (means && !depthwise_rows_pool(p)) gain = 3.0;
+  else if (means && p.kh == 5 && p.oh <= 10 && (long long)p.n * p.oc * p.oh * p.ow <= 300000) gain = 1.3;
+  return depthwise_planes::wins(p, device_sm_count(), gain);
 }
 
 bool depthwise_conv_pools(const ConvParams& p) {
