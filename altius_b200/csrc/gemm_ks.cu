@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "gemm_ks_shape.h"
 #include "kernels.h"
 #include "pdl.cuh"
 #include "ref_math.cuh"
@@ -39,9 +40,9 @@ namespace ac {
 namespace {
 
 using namespace tc;
+using namespace gemm_ks;
 
-constexpr int BM = 128, KB = 64, kEpiThreads = 512, kTmaWarp = 16, kMmaWarp = 17, kThreads = 576, kMaxStages = 4;
-constexpr int kAHalf = BM * KB * 2;           // bytes of A's hi (or lo) tile: rows of 128 bytes
+constexpr int kEpiThreads = 512, kTmaWarp = 16, kMmaWarp = 17, kThreads = 576;
 
 struct KsDev {
   int m, n, k;
@@ -360,14 +361,6 @@ gemm_ks_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant_
   }
 }
 
-constexpr size_t kSmemMax = 231000;
-
-struct Shape {
-  int bn = 0, split = 0, kper = 0, stages = 0, inv = 0;
-  size_t smem = 0;
-  double clocks = 1e30;
-};
-
 }  // namespace
 
 // The parts of the chip that hold a cluster have 14 to 18 SMs each, so fewer blocks run at once than there
@@ -404,41 +397,18 @@ int cluster_slots(int split) {
 
 namespace {
 
-// Tile width and K split by clocks, from stamps in the kernel: a K-block costs its twelve MMAs (45 to 65 clocks
-// each) or its bytes at 60 a clock, whichever is more; first loads and drain 2700; exchange 1600 and 18
-// per column; epilogue 1500 and 40 per column that a block finishes. A launch as timed takes 1.4 to 2 times as long
-// (launch, cold code; operands arrive at 34 bytes a clock when all SMs load at once).
-//
-// Fp32 operands: a K-block of 32 costs 1190 clocks up to 96 columns, 1370 with 128.
-Shape pick_shape(int64_t m, int64_t n, int64_t k, bool wide) {
-  Shape best;
-  const int step = wide ? KB / 2 : KB, nkb = (int)((k + step - 1) / step);
-  const long long mt = (m + BM - 1) / BM;
-  for (int bn : {32, 64, 96, 128}) {
-    for (int split : {1, 2, 4, 8}) {
-      const int kper = (nkb + split - 1) / split;
-      if ((split - 1) * kper >= nkb || (bn % (4 * split)) != 0) continue;
-      const int quads = bn / split / 4;
-      const size_t stage = (wide ? 1 : 2) * (size_t)kAHalf + (size_t)bn * KB * 4, ex = (size_t)split * quads * (BM + 1) * 16;
-      const int stages = (int)std::min<size_t>(std::min(kper, kMaxStages), (kSmemMax - 1024 - (split > 1 ? ex : 0)) / stage);
-      if (stages < std::min(2, kper)) continue;
-      const double waves = std::ceil((double)mt * ((n + bn - 1) / bn) / cluster_slots(split));
-      const double kb = wide ? (bn > 96 ? 1370.0 : 1190.0)
-                             : std::max(12 * (32.0 + 0.26 * bn), (double)stage / 60.0);
-      const double t = waves * (kper * kb + 4200.0 + (split > 1 ? 1600.0 + 18.0 * bn : 0.0) + 40.0 * bn / split);
-      if (t < best.clocks) {
-        best.bn = bn; best.split = split; best.kper = kper; best.stages = stages; best.inv = ((1 << 20) + quads - 1) / quads;
-        best.smem = std::max(stages * stage + (split > 1 ? ex : 0), ex) + 1024;
-        best.clocks = t;
-      }
-    }
-  }
-  return best;
+Shape shape_of(int64_t m, int64_t n, int64_t k, bool wide) {
+  return pick_shape(m, n, k, wide, [](int split) { return cluster_slots(split); });
 }
 
 template <int ACT, bool WIDE>
 cudaError_t launch_act(const CUtensorMap& ah, const CUtensorMap& al, const CUtensorMap& bh, const CUtensorMap& bl,
                        const KsDev& d, const Shape& sh, cudaStream_t st) {
+  // The kernel takes its addresses in shared memory, its cluster's included, from these numbers without a check of its own.
+  Shape whole;
+  if (!make_shape(sh.bn, sh.split, d.k, WIDE, &whole) || d.bn != sh.bn || d.kper != whole.kper || d.stages != whole.stages || d.inv != whole.inv ||
+      sh.smem != whole.smem)
+    return cudaErrorInvalidValue;
   static unsigned long long done = 0;
   if (cudaError_t e = ensure_dynamic_smem(gemm_ks_kernel<ACT, WIDE>, (int)kSmemMax, &done)) return e;
   const dim3 grid((unsigned)((d.n + sh.bn - 1) / sh.bn), (unsigned)((d.m + BM - 1) / BM), (unsigned)sh.split);
@@ -489,7 +459,7 @@ bool gemm_ks_wins(int64_t m, int64_t n, int64_t k) {
 
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k) {
   if (m < 1 || n < 4 || (n % 4) || k < 64 || (k % 8) || m > (1 << 20) || n > (1 << 20)) return 1e30;
-  return pick_shape(m, n, k, false).clocks;
+  return shape_of(m, n, k, false).clocks;
 }
 
 bool gemm_ks_epilogue_ok(int act, bool bias_m, bool c_in, float alpha, float bias_scale) {
@@ -506,7 +476,8 @@ cudaError_t launch_gemm_ks(const GemmParams& q, PairSums pairs, int* err_word, c
     if (q.c16_hi && ((q.n % 8) || (q.ldc16 % 8) || !al16(q.c16_hi) || !al16(q.c16_lo))) return cudaErrorInvalidValue;   // 16 bytes of a row at once
     return launch_gemm_pair_sums(q, pairs, err_word, st);
   }
-  const Shape sh = pick_shape(q.m, q.n, q.k, false);
+  const Shape sh = shape_of(q.m, q.n, q.k, false);
+  if (!sh.bn) return cudaErrorInvalidValue;
   KsDev d = device_params(q, sh, err_word);
   d.c16_hi = static_cast<uint2*>(q.c16_hi); d.c16_lo = static_cast<uint2*>(q.c16_lo); d.ldc16 = q.ldc16;
   d.acc_scale = q.b16_inv_scale;
@@ -521,7 +492,7 @@ double gemm_ks_wide_clocks(int64_t m, int64_t n, int64_t k) {
   if (m < 1 || n < 4 || (n % 4) || k < 32 || (k % 4) || m > (1 << 20) || n > (1 << 20)) return 1e30;
   // Long K: the other kernel's slices fill the SMs better than either estimate says (1386 x 3072 x 768 38.4 us, here 42.4; 394 x 2048 x 512
   // 15.5, 15.9; but 198 x 3072 x 768 17.0, 16.0).
-  return pick_shape(m, n, k, true).clocks * (k > 1536 ? 1.15 : 1.0);
+  return shape_of(m, n, k, true).clocks * (k > 1536 ? 1.15 : 1.0);
 }
 
 cudaError_t launch_gemm_ks_wide(const GemmParams& q, int* err_word, cudaStream_t st) {
@@ -530,7 +501,7 @@ cudaError_t launch_gemm_ks_wide(const GemmParams& q, int* err_word, cudaStream_t
       (q.residual && (!al16(q.residual) || (q.ld_res % 4))) || (q.bias_n && !al16(q.bias_n)) ||
       !gemm_ks_epilogue_ok(q.act, q.bias_m != nullptr, q.beta != 0.f && q.c_in, q.alpha, q.bias_scale))
     return cudaErrorInvalidValue;
-  const Shape sh = pick_shape(q.m, q.n, q.k, true);
+  const Shape sh = shape_of(q.m, q.n, q.k, true);
   const KsDev d = device_params(q, sh, err_word);
   CUtensorMap a, bh, bl;
   if (!make_map128(&a, q.a, 4, q.k, q.m, 1, q.lda, q.m * q.lda, BM) || !make_map128(&bh, q.b, 4, q.k, q.n, 1, q.ldb, q.n * q.ldb, sh.bn) ||
