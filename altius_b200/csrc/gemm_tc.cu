@@ -1927,8 +1927,6 @@ TcShape pick_shape(int64_t m, int64_t n, int64_t k, int64_t batch, int variant, 
 }
 }  // namespace
 
-int gemm_tc_pairs() { return pair_count(); }
-
 bool gemm_tc_wants_presplit(int64_t m, int64_t n, int64_t k, int64_t batch) {
   return pick_shape(m, n, k, batch, 2, 2).pair;
 }

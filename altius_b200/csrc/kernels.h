@@ -285,8 +285,6 @@ constexpr int kGemmRangeCode = 21;
 // where it does not apply), which takes the operands of the pair kernel.
 double gemm_tc_wide_clocks(int64_t m, int64_t n, int64_t k);
 double gemm_tc_pair_clocks(int64_t m, int64_t n, int64_t k);
-// CTA pairs that can run at once (0: none, their kernels cannot be launched).
-int gemm_tc_pairs();
 // Clusters of `split` blocks that can run at once, one block per SM.
 int cluster_slots(int split);
 double gemm_ks_clocks(int64_t m, int64_t n, int64_t k);
