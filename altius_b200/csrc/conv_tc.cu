@@ -551,6 +551,8 @@ bool conv_tc_supported(const ConvParams& q) {
          q.kh * q.dh < 32768 && q.kw * q.dw < 32768 && q.oc >= 1 && q.oc <= 16384 && q.act != ACT_GELU && shape_of(q).bn > 0;
 }
 
+double conv_tc_rounds(const ConvParams& q) { return shape_of(q).rounds; }
+
 int64_t conv_tc_filter_elems(const ConvParams& q) {
   const Shape sh = shape_of(q);
   const int64_t nkb = ((int64_t)q.c * q.kh * q.kw + KB - 1) / KB;

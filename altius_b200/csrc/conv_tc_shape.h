@@ -19,6 +19,7 @@ struct Shape {
   int bn, tiles, split, kper, stages, resident, ctas;
   int set, mains, bufs, cols;                // tensor memory: see the end of pick_shape
   size_t smem;
+  double rounds;                             // of the blocks (clusters) that run at once
 };
 
 constexpr size_t kSmemSm = 233472;           // shared memory of an SM
@@ -89,6 +90,7 @@ inline Shape pick_shape(const ConvParams& q, const std::array<int, 4>& slots) {
   // blocks per SM started when the other half had finished.)
   best.smem = std::max(need(best.stages), best.cols == 512 ? kSmemSm / 2 : kSmemSm * best.cols / 512 - kSmemBeside);
   const int resident_blocks = sms * (best.smem <= half ? 2 : 1);
+  best.rounds = (double)px * best.tiles / (best.split == 1 ? resident_blocks : slots[best.split == 2 ? 1 : best.split == 4 ? 2 : 3]);
   best.ctas = (int)(walk ? std::min<long long>(px, std::max(1, resident_blocks / best.tiles)) : px);
   return best;
 }

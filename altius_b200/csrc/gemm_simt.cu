@@ -412,6 +412,10 @@ bool depthwise_conv_pools(const ConvParams& p) {
   return depthwise_rows_ok(p) && per_plane >= 1 && per_plane <= 256 && (depthwise_rows_pool(p) || depthwise_planes_wins(p, true));
 }
 
+double depthwise_conv_rounds(const ConvParams& p) {
+  return (double)p.n * p.oc * p.oh * ((p.ow + 3) / 4) / (1536.0 * device_sm_count());   // 40 registers a thread; four pixels each
+}
+
 cudaError_t launch_depthwise_conv(const ConvParams& p, int images, const float* x, const float* w, const float* bias, float* out,
                                   float* means, bool constants, cudaStream_t st) {
   const long long total = (long long)images * p.oc * p.oh * p.ow;

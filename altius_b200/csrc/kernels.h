@@ -179,6 +179,7 @@ cudaError_t launch_patchify(const ConvParams& p, const float* x, float* rows, cu
 // too where depthwise_conv_pools says so, or null. `images`: of the p.n that kernel and split are chosen for, from the given
 // pointers on (the order of a mean's sum follows from the split).
 bool depthwise_conv_pools(const ConvParams& p);
+double depthwise_conv_rounds(const ConvParams& p);   // of the threads that run at once
 cudaError_t launch_depthwise_conv(const ConvParams& p, int images, const float* x, const float* w, const float* bias, float* out, float* means,
                                   bool constants, cudaStream_t st);
 // The same over whole planes in shared memory (depthwise_planes.cu), stride 1; x 16-byte aligned.
@@ -198,6 +199,7 @@ cudaError_t launch_conv_simt(const ConvParams& p, const float* x, const float* w
 // conv_tc_filter_elems floats; the other operands as above.
 bool conv_tc_supported(const ConvParams& p);
 int64_t conv_tc_filter_elems(const ConvParams& p);
+double conv_tc_rounds(const ConvParams& p);   // of the blocks that run at once
 cudaError_t launch_pack_filter_tc(const ConvParams& p, const float* w, float* packed, cudaStream_t st);
 // `images`: of the p.n that the tile shape is chosen for, from the given pointers on.
 cudaError_t launch_conv_tc(const ConvParams& p, int images, const float* x, const float* packed, const float* bias, const float* gate,

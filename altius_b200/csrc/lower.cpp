@@ -1243,6 +1243,7 @@ void lower_conv(Emit& em, Plan& plan, int nid, const Epilogue* e, const Plan::Se
                         [=](cudaStream_t st) { return part(st, 0, p.n); });
     step.part = part;
     step.images = p.n;
+    step.rounds = depthwise_conv_rounds(p);
     return;
   }
   // GEMM form: out[n] (ocg x ohw) = W_g (ocg x k) * col[n, g] (k x ohw), bias per row.
@@ -1265,6 +1266,7 @@ void lower_conv(Emit& em, Plan& plan, int nid, const Epilogue* e, const Plan::Se
                         [=](cudaStream_t st) { return part(st, 0, p.n); });
     step.part = part;
     step.images = p.n;
+    step.rounds = conv_tc_rounds(p);
     return;
   }
   if (small_conv_applies(*s, flops, small_columns) && !(pointwise && ohw == 1) && conv_simt_supported(p)) {

@@ -108,8 +108,12 @@ void plan_front(AcSession& s) {
   if (s.opt.disable_cuda_graph || s.opt.enable_profiling || s.inputs.size() != 1) return;
   const Value& in = s.values[s.inputs[0]];
   if (in.rank < 1 || s.storages[in.storage].weight) return;
-  int front = 0;
-  while (front < (int)s.steps.size() && s.steps[front].part && s.steps[front].images == in.dims[0]) ++front;
+  std::vector<FrontStep> front;
+  for (const Step& st : s.steps) {
+    if (!st.part || st.images != in.dims[0]) break;
+    // Convolutions: 4 TB/s, or 80 TFLOP/s of the products.
+    front.push_back({FrontStep::kLaunch + std::max(st.bytes / 4e6, st.flops / 80e6), st.rounds});
+  }
   s.pieces = plan_pieces(front, (int)std::min<int64_t>(in.dims[0], 1 << 30), in.bytes());
 }
 

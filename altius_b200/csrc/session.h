@@ -69,6 +69,7 @@ struct Step {
   // The step on images [first, first + count) of its batch of `images`, where its kernel takes them one by one.
   std::function<cudaError_t(cudaStream_t, int first, int count)> part;
   int images = 0;
+  double rounds = 1;               // of the blocks that run at once, for the whole batch
 };
 
 struct ProfileAcc {
