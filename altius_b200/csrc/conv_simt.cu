@@ -269,11 +269,11 @@ __global__ void __launch_bounds__(T, 2) conv_simt_kernel(const ConvDev p) {
     Piece u[S - 1];
 #pragma unroll
     for (int s = 0; s < S - 1; ++s)
-      if (LOAD != LOAD_WINDOW || s < kts) fetch(u[s], kt0 + s, s < kts);
+      if (s < kts) fetch(u[s], kt0 + s, true);
     quad.fetch(p);
 #pragma unroll
     for (int s = 0; s < S - 1; ++s)
-      if (LOAD != LOAD_WINDOW || s < kts) put(s, u[s]);
+      if (s < kts) put(s, u[s]);
   }
 
   float2 acc[4][4];
